@@ -482,57 +482,84 @@ __global__ void __launch_bounds__(128) gemm_bf16_kernel(const bf16* __restrict__
         }
 }
 
-// Matrix product for very few rows (decoding): WPC warps per output column (each a 1/WPC interleaved share of K, the
-// shares added in a fixed order), lanes cut K into 16-byte pieces; the weights are streamed once, the MR activation
-// rows come from L1/L2.  WPC follows from N alone (narrow products get more warps per column so that the grid still
-// covers the SMs).  Needs K % 8 == 0 and 16-byte aligned operands.
-template <int MR, int WPC>
-__global__ void __launch_bounds__(256) gemv_bf16_kernel(const bf16* __restrict__ a, const bf16* __restrict__ w, float* __restrict__ y,
-                                                        int M, int N, int K) {
-    __shared__ float part[8][MR];
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, kw = warp % WPC;
-    const int n = blockIdx.x * (8 / WPC) + warp / WPC;
-    const bool valid = n < N;
-    float acc[MR];
+// Matrix product for few rows (decoding): bound by reading the weights once.  A block owns NR weight rows, its warps share K in
+// interleaved steps of 32: a lane reads whole 16-byte pieces -- 8 neighbouring k of a weight row and of an activation row -- and hands
+// them to m16n8k16 MMAs.  Both operands use the same assignment of k to fragment places, so the sum over k is the plain one in
+// another order; the warps' shares are added in warp order.
+// NR 16: the weights are the 16-row operand, a tile of activations its 8 columns.  NR 8 (narrow products, whose blocks of 16 would not
+// reach every SM): the weights are the 8 columns, a tile of activations the 16 rows.
+// On the CUDA cores (one warp per column) five rows cost 40 conversions and multiply-adds per 16 bytes of weights: 18.9 us per product
+// over a decode step of width 1536 (17 MB each, 0.9 TB/s) against 6.8 us here; one row of 768 x 4608 takes 8.2 us with NR 16 and 6.4
+// with NR 8.
+// WARPS follows from K, NR from N.  Needs K % 8 == 0 and 16-byte aligned operands.
+template <int NR, int MT, int WARPS>
+__global__ void __launch_bounds__(WARPS * 32) gemm_few_kernel(const bf16* __restrict__ a, const bf16* __restrict__ w, float* __restrict__ y,
+                                                              int M, int N, int K) {
+    constexpr int WT = NR / 8, AT = NR == 16 ? MT : 2 * MT;      // 8-row pieces of weights and of activations per step
+    constexpr int U = WT + AT <= 3 ? 4 : 2;                      // steps of 32 whose loads are in flight together
+    constexpr int OUT = NR * (NR == 16 ? 8 : 16) * MT;           // outputs of the block
+    __shared__ float part[WARPS][OUT];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, tq = lane & 3;
+    const int n0 = blockIdx.x * NR;
+    const bf16* wr[WT];
 #pragma unroll
-    for (int m = 0; m < MR; ++m) acc[m] = 0.0f;
-    if (valid) {
-        const bf16* wr = w + (size_t)n * K;
-        for (int k = (kw * 32 + lane) * 8; k < K; k += 256 * WPC) {
-            const uint4 wv = ldg_stream(wr + k);
-            const float w0 = bf_lo(wv.x), w1 = bf_hi(wv.x), w2 = bf_lo(wv.y), w3 = bf_hi(wv.y), w4 = bf_lo(wv.z), w5 = bf_hi(wv.z),
-                        w6 = bf_lo(wv.w), w7 = bf_hi(wv.w);
+    for (int i = 0; i < WT; ++i) wr[i] = w + (size_t)min(n0 + i * 8 + g, N - 1) * K + tq * 8;
+    float acc[MT][4];
 #pragma unroll
-            for (int m = 0; m < MR; ++m) {
-                if (m < M) {
-                    const uint4 av = ldg_v4(a + (size_t)m * K + k);
-                    float t = acc[m];
-                    t = fmaf(bf_lo(av.x), w0, t); t = fmaf(bf_hi(av.x), w1, t); t = fmaf(bf_lo(av.y), w2, t); t = fmaf(bf_hi(av.y), w3, t);
-                    t = fmaf(bf_lo(av.z), w4, t); t = fmaf(bf_hi(av.z), w5, t); t = fmaf(bf_lo(av.w), w6, t); t = fmaf(bf_hi(av.w), w7, t);
-                    acc[m] = t;
-                }
+    for (int i = 0; i < MT; ++i)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) acc[i][e] = 0.0f;
+    const uint4 zero = make_uint4(0, 0, 0, 0);
+    for (int k0 = warp * 32; k0 < K; k0 += WARPS * 32 * U) {
+        uint4 p[U][WT], x[U][AT];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const int k = k0 + u * WARPS * 32;
+#pragma unroll
+            for (int i = 0; i < WT; ++i) p[u][i] = k + tq * 8 < K ? ldg_stream(wr[i] + k) : zero;
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const int k = k0 + u * WARPS * 32 + tq * 8;
+#pragma unroll
+            for (int i = 0; i < AT; ++i) {
+                const int m = i * 8 + g;
+                x[u][i] = (m < M && k < K) ? ldg_v4(a + (size_t)m * K + k) : zero;
             }
         }
-    }
 #pragma unroll
-    for (int m = 0; m < MR; ++m) {
-        const float t = warp_sum(acc[m]);
-        if (WPC == 1) {
-            if (lane == 0 && valid && m < M) y[(size_t)m * N + n] = t;
-        } else if (lane == 0) {
-            part[warp][m] = t;
-        }
-    }
-    if (WPC > 1) {
-        __syncthreads();
-        if (kw == 0 && lane < MR && lane < M && valid) {
-            float t = part[warp][lane];
+        for (int u = 0; u < U; ++u)
 #pragma unroll
-            for (int x = 1; x < WPC; ++x) t += part[warp + x][lane];
-            y[(size_t)lane * N + n] = t;
+            for (int i = 0; i < MT; ++i) {
+                if constexpr (NR == 16) {
+                    mma_bf16_16816(acc[i], p[u][0].x, p[u][1].x, p[u][0].y, p[u][1].y, x[u][i].x, x[u][i].y);
+                    mma_bf16_16816(acc[i], p[u][0].z, p[u][1].z, p[u][0].w, p[u][1].w, x[u][i].z, x[u][i].w);
+                } else {
+                    mma_bf16_16816(acc[i], x[u][2 * i].x, x[u][2 * i + 1].x, x[u][2 * i].y, x[u][2 * i + 1].y, p[u][0].x, p[u][0].y);
+                    mma_bf16_16816(acc[i], x[u][2 * i].z, x[u][2 * i + 1].z, x[u][2 * i].w, x[u][2 * i + 1].w, p[u][0].z, p[u][0].w);
+                }
+            }
+    }
+    // part[warp][m * NR + n]: neighbouring outputs of a row side by side.  acc[.][e]: tile row g + (e / 2) * 8, tile column 2 tq + e % 2
+#pragma unroll
+    for (int i = 0; i < MT; ++i)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            const int r = g + (e >> 1) * 8, c = tq * 2 + (e & 1);
+            part[warp][NR == 16 ? (i * 8 + c) * NR + r : (i * 16 + r) * NR + c] = acc[i][e];
         }
+    __syncthreads();
+    for (int o = threadIdx.x; o < OUT; o += WARPS * 32) {
+        const int m = o / NR, n = n0 + o % NR;
+        float t = part[0][o];
+#pragma unroll
+        for (int x = 1; x < WARPS; ++x) t += part[x][o];
+        if (m < M && n < N) y[(size_t)m * N + n] = t;
     }
 }
+constexpr int kFewRows = 32;             // most rows of gemm_few_kernel
+constexpr int kFewLongK = 2048;          // from this K on 16 warps share it
+constexpr int kFewWideN = 16 * 148;      // from this N on blocks of 16 weight rows give every SM one
 
 // Matrix product for many rows (prompt portions), bf16 on the 5th-generation tensor cores: the library's tcgen05 tile
 // (umma.cuh: TMA loads into a 128-byte-swizzled ring, accumulators in tensor memory) over 128 rows x kTcTileN columns,
@@ -2373,21 +2400,20 @@ cudaError_t linear<bf16>(SmolLm* m, const bf16* a, const bf16* w, float* y, int 
             return cudaGetLastError();
         }
     }
-    if (M <= 8 && K % 8 == 0 && (reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(w)) % 16 == 0) {
-        // warps per column by N alone: a row's result must not depend on what else the step holds
-        const int wpc = N >= 1184 ? 1 : N >= 592 ? 2 : 4;
-        const int grid = (N * wpc + 7) / 8;
-#define SMOL_GEMV(MR)                                                                                   \
-        do {                                                                                            \
-            if (wpc == 1) gemv_bf16_kernel<MR, 1><<<grid, 256, 0, st>>>(a, w, y, M, N, K);              \
-            else if (wpc == 2) gemv_bf16_kernel<MR, 2><<<grid, 256, 0, st>>>(a, w, y, M, N, K);         \
-            else gemv_bf16_kernel<MR, 4><<<grid, 256, 0, st>>>(a, w, y, M, N, K);                       \
+    if (M <= kFewRows && aligned) {
+        // the block's shape by N and K alone: a row's result must not depend on what else the step holds beyond its number of rows
+#define SMOL_FEW(NR, MT)                                                                                          \
+        do {                                                                                                      \
+            if (K >= kFewLongK) gemm_few_kernel<NR, MT, 16><<<(N + NR - 1) / NR, 512, 0, st>>>(a, w, y, M, N, K); \
+            else gemm_few_kernel<NR, MT, 8><<<(N + NR - 1) / NR, 256, 0, st>>>(a, w, y, M, N, K);                 \
         } while (0)
-        if (M == 1) SMOL_GEMV(1);
-        else if (M == 2) SMOL_GEMV(2);
-        else if (M <= 4) SMOL_GEMV(4);
-        else SMOL_GEMV(8);
-#undef SMOL_GEMV
+        if (N < kFewWideN) {
+            if (M <= 16) SMOL_FEW(8, 1);
+            else SMOL_FEW(8, 2);
+        } else if (M <= 8) SMOL_FEW(16, 1);
+        else if (M <= 16) SMOL_FEW(16, 2);
+        else SMOL_FEW(16, 4);
+#undef SMOL_FEW
     } else {
         return linear_ex<bf16>(m, a, w, y, M, N, K, plain_io(K, N), 1, 0, st);
     }

@@ -1,0 +1,28 @@
+"""Kernels at the sizes where their tiles end: edges, remainders, the smallest and largest of a dispatch's range."""
+from __future__ import annotations
+
+import pytest
+import torch
+
+from pamasun_util import attn, config, engine_and_oracle
+
+pytestmark = pytest.mark.gpu
+
+
+def product_bound(a, w):
+    """|error| of an fp32 sum of K products, any order, each addition off by at most 2^-23 of the sum of absolute products."""
+    return (a.double().abs() @ w.double().abs().T) * (a.shape[1] * 2.0 ** -23)
+
+
+FEW_ROWS = ((1, 1, 8), (1, 16, 24), (7, 17, 40), (8, 771, 2040), (9, 15, 2048), (16, 33, 2056), (17, 64, 264), (31, 50, 4104), (32, 8, 1528), (33, 48, 64),
+            (2, 8192, 1536), (5, 2369, 4096), (8, 2367, 264), (13, 2368, 72), (25, 2400, 2072))
+
+
+@pytest.mark.parametrize("M,N,K", FEW_ROWS)
+def test_products_of_few_rows(M, N, K):
+    """At most 32 rows; blocks of 8 weight rows (16 from 2368 columns on), K shared by 8 or 16 warps in steps of 32."""
+    model, _, _ = engine_and_oracle(config([attn(ff=0)]), seed=9, dtype=torch.bfloat16)
+    g = torch.Generator(device="cuda").manual_seed(M * 31 + K)
+    a, w = (torch.randn(r, K, device="cuda", generator=g).bfloat16() for r in (M, N))
+    err = (model.linear(a, w).double() - a.double() @ w.double().T).abs()
+    assert bool((err <= product_bound(a, w)).all())

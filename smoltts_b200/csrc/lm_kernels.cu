@@ -1499,35 +1499,56 @@ struct DeltaArgs {
 };
 
 // Per token and channel: decay w = exp(-coef * sigmoid(w2 tanh(inner) + bias)), unit key u, removal vector a * u.
-__global__ void delta_prep_kernel(const DeltaArgs A, float* __restrict__ decay, float* __restrict__ ukey, float* __restrict__ aukey) {
-    extern __shared__ float th[];   // tanh(inner) [rank], then per-head 1/|k|
-    const int t = blockIdx.x, HD = A.H * A.d;      // blockIdx.y: a slice of blockDim.x channels
-    const float* row = A.proj + (size_t)t * A.n_in;
-    float* inv = th + A.rank;
-    for (int r = threadIdx.x; r < A.rank; r += blockDim.x) th[r] = tanhf(row[5 * HD + r]);
+// A block takes TT tokens and blockDim.x channels: the second decay matrix (rank x HD fp32, from L2) is read once per TT tokens.
+// One token per block made 2048 tokens of 12 x 64 channels and rank 64 read 400 MB of it: 84 us; eight: 27 us.
+template <int TT>
+__global__ void __launch_bounds__(128) delta_prep_kernel(const DeltaArgs A, float* __restrict__ decay, float* __restrict__ ukey, float* __restrict__ aukey) {
+    extern __shared__ float th[];   // tanh(inner) [rank][TT], then 1/|k| [TT][H]
+    const int t0 = blockIdx.x * TT, nt = min(TT, A.n_tokens - t0), HD = A.H * A.d;      // blockIdx.y: a slice of blockDim.x channels
+    float* inv = th + A.rank * TT;
+    for (int i = threadIdx.x; i < A.rank * TT; i += blockDim.x) {
+        const int tt = i / A.rank, r = i - tt * A.rank;
+        th[r * TT + tt] = tt < nt ? tanhf(A.proj[(size_t)(t0 + tt) * A.n_in + 5 * HD + r]) : 0.0f;
+    }
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
     const int c_lo = blockIdx.y * blockDim.x, c_hi = min(HD, c_lo + blockDim.x);      // this block's channels (gridDim.y slices cover HD)
     if (c_lo >= c_hi) return;
-    for (int h = c_lo / A.d + warp; h <= (c_hi - 1) / A.d; h += nw) {
-        const float* k = row + HD + h * A.d;
+    const int h_lo = c_lo / A.d, nh = (c_hi - 1) / A.d - h_lo + 1;
+    for (int x = warp; x < nh * nt; x += nw) {
+        const int tt = x / nh, h = h_lo + x - tt * nh;
+        const float* k = A.proj + (size_t)(t0 + tt) * A.n_in + HD + h * A.d;
         float ss = 0.0f;
         for (int c = lane; c < A.d; c += 32) ss += k[c] * k[c];
         ss = warp_sum(ss);
-        if (lane == 0) inv[h] = 1.0f / sqrtf(ss + A.unit_eps);
+        if (lane == 0) inv[tt * A.H + h] = 1.0f / sqrtf(ss + A.unit_eps);
     }
     __syncthreads();
     const int c = c_lo + threadIdx.x;
-    if (c < c_hi) {
-        float lo = A.decay_bias[c];
+    if (c >= c_hi) return;
+    float lo[TT];
+    const float bias = A.decay_bias[c];
+#pragma unroll
+    for (int tt = 0; tt < TT; ++tt) lo[tt] = bias;
 #pragma unroll 8
-        for (int r = 0; r < A.rank; ++r) lo = fmaf(A.decay_w2[(size_t)r * HD + c], th[r], lo);
-        const float u = row[HD + c] * inv[c / A.d];
-        const float a = sigmoidf_(row[4 * HD + c] + A.rate_bias[c]);
-        decay[(size_t)t * HD + c] = expf(-A.decay_coef * sigmoidf_(lo));
-        ukey[(size_t)t * HD + c] = u;
-        aukey[(size_t)t * HD + c] = a * u;
+    for (int r = 0; r < A.rank; ++r) {
+        const float wv = A.decay_w2[(size_t)r * HD + c];
+#pragma unroll
+        for (int tt = 0; tt < TT; ++tt) lo[tt] = fmaf(wv, th[r * TT + tt], lo[tt]);
     }
+    const float rb = A.rate_bias[c];
+#pragma unroll
+    for (int tt = 0; tt < TT; ++tt)
+        if (tt < nt) {
+            const float* row = A.proj + (size_t)(t0 + tt) * A.n_in;
+            const size_t at = (size_t)(t0 + tt) * HD + c;
+            const float u = row[HD + c] * inv[tt * A.H + c / A.d];
+            decay[at] = expf(-A.decay_coef * sigmoidf_(lo[tt]));
+            ukey[at] = u;
+            aukey[at] = sigmoidf_(row[4 * HD + c] + rb) * u;
+        }
 }
+constexpr int kDecayTokens = 8;          // tokens per block of the decay kernels
+constexpr int kDecayMinTokens = 128;     // fewer: a token per block (more blocks than the reuse is worth)
 
 // The recurrence.  The value columns of a head's state never mix: column j follows
 //   seen = sum_i u_i S_ij;   S_ij <- w_i S_ij - (a u)_i seen + k_i v_j;   o_j = sum_i S_ij r_i
@@ -3147,7 +3168,10 @@ static int step_impl(SmolLm* m, const SmolLmStep* s, cudaStream_t st) {
             A.seq_start = s->seq_start; A.seq_pos0 = s->seq_pos0; A.seq_slot = s->seq_slot;
             A.slot_floats = m->slot_floats; A.state_off = R.state_off; A.n_slots = m->n_slots; A.err = err;
             gla_sources_from_proj(A);
-            gla_prep_kernel<<<dim3(Tn, (L.heads * L.dim + 127) / 128), 128, L.rank * sizeof(float), st>>>(A, dec);
+            const int slices = (L.heads * L.dim + 127) / 128;
+            if (Tn >= kDecayMinTokens && kDecayTokens * L.rank * sizeof(float) <= 48 * 1024)
+                gla_prep_kernel<kDecayTokens><<<dim3((Tn + kDecayTokens - 1) / kDecayTokens, slices), 128, kDecayTokens * L.rank * sizeof(float), st>>>(A, dec);
+            else gla_prep_kernel<1><<<dim3(Tn, slices), 128, L.rank * sizeof(float), st>>>(A, dec);
             CU(launch_gla_scan_any(A, s->n_seqs, dec, m->slots, oraw, st));
             gla_out_kernel<T><<<(Tn * L.heads + 3) / 4, 128, 0, st>>>(A, oraw, mix);
             m->launches += 3;
@@ -3159,7 +3183,11 @@ static int step_impl(SmolLm* m, const SmolLmStep* s, cudaStream_t st) {
             A.rate_bias = L.rate_bias; A.decay_w2 = L.decay_w2; A.decay_bias = L.decay_bias; A.out_norm = L.out_norm;
             A.seq_start = s->seq_start; A.seq_pos0 = s->seq_pos0; A.seq_slot = s->seq_slot;
             A.slot_floats = m->slot_floats; A.state_off = R.state_off; A.n_slots = m->n_slots; A.err = err;
-            delta_prep_kernel<<<dim3(Tn, (L.heads * L.dim + 127) / 128), 128, (L.rank + L.heads) * sizeof(float), st>>>(A, dec, uk, auk);
+            const size_t prep_smem = (size_t)(L.rank + L.heads) * sizeof(float);
+            const int slices = (L.heads * L.dim + 127) / 128;
+            if (Tn >= kDecayMinTokens && kDecayTokens * prep_smem <= 48 * 1024)
+                delta_prep_kernel<kDecayTokens><<<dim3((Tn + kDecayTokens - 1) / kDecayTokens, slices), 128, kDecayTokens * prep_smem, st>>>(A, dec, uk, auk);
+            else delta_prep_kernel<1><<<dim3(Tn, slices), 128, prep_smem, st>>>(A, dec, uk, auk);
             cudaError_t e;
             if (L.dim <= 16) e = launch_scan<16>(A, s->n_seqs, dec, uk, auk, m->slots, oraw, st);
             else if (L.dim <= 32) e = launch_scan<32>(A, s->n_seqs, dec, uk, auk, m->slots, oraw, st);

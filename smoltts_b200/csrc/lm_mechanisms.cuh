@@ -340,19 +340,32 @@ __host__ __device__ inline void gla_sources_from_proj(GlaArgs& A) {
     A.out_scale = 1.0f;
 }
 
-// decay[t][c] for the H*d key channels; blockIdx.y: a slice of blockDim.x channels
-__global__ void gla_prep_kernel(const GlaArgs A, float* __restrict__ decay) {
-    extern __shared__ float inner[];
-    const int t = blockIdx.x, HD = A.H * A.d;
-    const float* row = A.proj + (size_t)t * A.n_in + 2 * HD + 2 * A.H * A.dv;
-    for (int r = threadIdx.x; r < A.rank; r += blockDim.x) inner[r] = row[r];
+// decay[t][c] for the H*d key channels; a block takes TT tokens and blockDim.x channels (as delta_prep_kernel, for its reason)
+template <int TT>
+__global__ void __launch_bounds__(128) gla_prep_kernel(const GlaArgs A, float* __restrict__ decay) {
+    extern __shared__ float inner[];      // [rank][TT]
+    const int t0 = blockIdx.x * TT, nt = min(TT, A.n_tokens - t0), HD = A.H * A.d;
+    const size_t at = 2 * HD + 2 * A.H * A.dv;
+    for (int i = threadIdx.x; i < A.rank * TT; i += blockDim.x) {
+        const int tt = i / A.rank, r = i - tt * A.rank;
+        inner[r * TT + tt] = tt < nt ? A.proj[(size_t)(t0 + tt) * A.n_in + at + r] : 0.0f;
+    }
     __syncthreads();
     const int c = blockIdx.y * blockDim.x + threadIdx.x;
     if (c >= HD) return;
-    float z = A.decay_bias[c];
+    float z[TT];
+    const float bias = A.decay_bias[c];
+#pragma unroll
+    for (int tt = 0; tt < TT; ++tt) z[tt] = bias;
 #pragma unroll 8
-    for (int r = 0; r < A.rank; ++r) z = fmaf(A.decay_w2[(size_t)r * HD + c], inner[r], z);
-    decay[(size_t)t * HD + c] = expf(log_sigmoid_(z) / A.tau);
+    for (int r = 0; r < A.rank; ++r) {
+        const float wv = A.decay_w2[(size_t)r * HD + c];
+#pragma unroll
+        for (int tt = 0; tt < TT; ++tt) z[tt] = fmaf(wv, inner[r * TT + tt], z[tt]);
+    }
+#pragma unroll
+    for (int tt = 0; tt < TT; ++tt)
+        if (tt < nt) decay[(size_t)(t0 + tt) * HD + c] = expf(log_sigmoid_(z[tt]) / A.tau);
 }
 
 // The scan.  Value columns never mix, so a head is cut into groups of CB columns, one block per (sequence, head, group);

@@ -4,7 +4,7 @@ from __future__ import annotations
 import pytest
 import torch
 
-from pamasun_util import attn, config, engine_and_oracle
+from pamasun_util import TOL, attn, config, delta, engine_and_oracle, rel_err, tokens
 
 pytestmark = pytest.mark.gpu
 
@@ -26,3 +26,15 @@ def test_products_of_few_rows(M, N, K):
     a, w = (torch.randn(r, K, device="cuda", generator=g).bfloat16() for r in (M, N))
     err = (model.linear(a, w).double() - a.double() @ w.double().T).abs()
     assert bool((err <= product_bound(a, w)).all())
+
+
+@pytest.mark.parametrize("n", [127, 128, 129, 135, 136])
+def test_decay_preparation_over_groups_of_tokens(n):
+    """128 tokens and more: eight tokens per block share the decay's second matrix; odd ranks, a last group of any size."""
+    cfg = config([delta(heads=3, dim=24, ff=0, rank=5)], vocab=61, width=48)
+    model, orc, _ = engine_and_oracle(cfg, seed=3, max_step_tokens=256)
+    toks = tokens(n, 61, n)
+    seq = model.open_sequence()
+    got = model.forward([(seq, toks, list(range(n)))]).clone()
+    model.close_sequence(seq)
+    assert rel_err(got, orc.forward(toks)) < TOL[torch.float32]

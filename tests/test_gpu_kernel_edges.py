@@ -28,6 +28,19 @@ def test_products_of_few_rows(M, N, K):
     assert bool((err <= product_bound(a, w)).all())
 
 
+F32_TILES = ((1, 1, 4), (16, 65, 36), (17, 64, 128), (64, 63, 132), (65, 130, 260), (300, 768, 1028), (31, 70, 2048), (512, 4700, 20), (640, 3841, 52))
+
+
+@pytest.mark.parametrize("M,N,K", F32_TILES)
+def test_float32_products(M, N, K):
+    """16-, 64- and 128-row tiles, steps of 16 k with a ragged last one, K shared by 1 to 8 thread blocks."""
+    model, _, _ = engine_and_oracle(config([attn(ff=0)]), seed=9)
+    g = torch.Generator(device="cuda").manual_seed(M * 31 + K)
+    a, w = (torch.randn(r, K, device="cuda", generator=g) for r in (M, N))
+    err = (model.linear(a, w).double() - a.double() @ w.double().T).abs()
+    assert bool((err <= product_bound(a, w)).all())
+
+
 @pytest.mark.parametrize("n", [127, 128, 129, 135, 136])
 def test_decay_preparation_over_groups_of_tokens(n):
     """128 tokens and more: eight tokens per block share the decay's second matrix; odd ranks, a last group of any size."""

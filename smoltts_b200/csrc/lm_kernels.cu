@@ -600,58 +600,13 @@ constexpr int kFewRows = 32;             // most rows of gemm_few_kernel
 constexpr int kFewLongK = 2048;          // from this K on 16 warps share it
 constexpr int kFewWideN = 16 * 148;      // from this N on blocks of 16 weight rows give every SM one
 
-// Matrix product for many rows (prompt portions), bf16 on the 5th-generation tensor cores: the library's tcgen05 tile
-// (umma.cuh: TMA loads into a 128-byte-swizzled ring, accumulators in tensor memory) over 128 rows x kTcTileN columns,
-// one persistent CTA per SM walking the tiles; row tiles that share a weight tile run on neighbouring CTAs.  Rows and
-// columns outside the matrices are zero-filled by TMA (a partial last K stage adds zeros); rows past M of the activation
-// buffer hold stale values whose accumulator lanes are never stored.
-constexpr int kTcTileN = umma::kMaxN;
-constexpr int kTcThreads = 512;
-constexpr int kTcSmemBytes = umma::kRingBytes + 1024;
-constexpr int kTcMinRows = 257;          // below this the mma.sync tiles fill the GPU better than 128-row tiles
+}  // namespace lm
+}  // namespace smol
 
-// Grouped rows (io.tile_group != nullptr): the row tiles come from the device-built table (128 rows each, group g's rows end
-// at seg[g + 1]; rows of the tile beyond that belong to the next group and are computed but not stored), and group g's
-// weights are rows g * N .. of the weight map.
-__global__ void __launch_bounds__(kTcThreads, 1) gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CUtensorMap tm_w,
-                                                                float* __restrict__ y, int M, int N, int K, const GemmIo io) {
-    extern __shared__ unsigned char tc_smem[];
-    __shared__ umma::Bars bars;
-    unsigned char* ring = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(tc_smem) + 1023) & ~(uintptr_t)1023);
-    umma::Pipe pipe;
-    umma::setup(&bars, pipe, (uint32_t)umma::kAcc, 2u);
-    const int m_tiles = io.tile_group ? *io.n_tiles : (M + umma::kM - 1) / umma::kM, n_tiles = (N + kTcTileN - 1) / kTcTileN;
-    const int k_pad = (K + umma::kBK - 1) / umma::kBK * umma::kBK;
-    const bool vec = N % 4 == 0;
-    for (int u = blockIdx.x; u < m_tiles * n_tiles; u += gridDim.x) {
-        int m0 = (u % m_tiles) * umma::kM, w_row = 0;
-        const int n0 = (u / m_tiles) * kTcTileN;
-        if (io.tile_group) {
-            const int g = io.tile_group[u % m_tiles];
-            m0 = io.tile_row0[u % m_tiles];
-            M = io.seg[g + 1];
-            w_row = g * N;
-        }
-        umma::BSrc b0, b1;
-        b0.tm = &tm_w; b0.row0 = w_row + n0; b0.n = kTcTileN; b0.box = kTcTileN;
-        b1.tm = nullptr; b1.row0 = 0; b1.n = 0; b1.box = kTcTileN;
-        umma::tile_mma_tma<kTcThreads>(ring, &bars, pipe, k_pad, &tm_a, m0, b0, b1);
-        umma::tile_epilogue(&bars, kTcTileN, [&](int row, int c0, const float (&acc)[8]) {
-            const int m = m0 + row, n = n0 + c0;
-            if (m >= M || n >= N) return;
-            float* out = y + (size_t)m * N + n;
-            if (vec && n + 8 <= N) {
-                *reinterpret_cast<float4*>(out) = make_float4(acc[0], acc[1], acc[2], acc[3]);
-                *reinterpret_cast<float4*>(out + 4) = make_float4(acc[4], acc[5], acc[6], acc[7]);
-            } else {
-#pragma unroll
-                for (int e = 0; e < 8; ++e)
-                    if (n + e < N) out[e] = acc[e];
-            }
-        }, kTcTileN);
-    }
-    umma::teardown(&bars);
-}
+#include "lm_gemm_tc.cuh"
+
+namespace smol {
+namespace lm {
 
 // ---------------------------------------------------------------------------------------------------------------------
 // Softmax attention over the paged pool.  A cached position holds, per key/value head, a key row of d elements (row
@@ -2337,6 +2292,14 @@ static cudaError_t set_kernel_attributes() {
     return e;
 }
 
+template <int BN>
+static cudaError_t gemm_tc_prepare_sized() { return cudaFuncSetAttribute(gemm_tc_kernel<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, gemm_tc_smem<BN>()); }
+static cudaError_t gemm_tc_prepare() {
+    for (cudaError_t e : {gemm_tc_prepare_sized<64>(), gemm_tc_prepare_sized<96>(), gemm_tc_prepare_sized<128>(), gemm_tc_prepare_sized<192>(), gemm_tc_prepare_sized<256>()})
+        if (e != cudaSuccess) return e;
+    return cudaSuccess;
+}
+
 extern "C" int smol_lm_bind(SmolLm* m, const SmolLmGlobals* g, void* d_workspace, size_t workspace_bytes, void* d_pages, int32_t n_pages,
                             void* d_slots, int32_t n_slots) {
     if (!m || !g || !d_workspace || !d_pages || !d_slots) return fail(SMOL_ERR_INVALID, "smol_lm_bind: null argument");
@@ -2350,7 +2313,7 @@ extern "C" int smol_lm_bind(SmolLm* m, const SmolLmGlobals* g, void* d_workspace
     int dev = 0;
     CU(cudaGetDevice(&dev));
     CU(cudaDeviceGetAttribute(&m->n_sms, cudaDevAttrMultiProcessorCount, dev));
-    CU(cudaFuncSetAttribute(gemm_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kTcSmemBytes));
+    CU(gemm_tc_prepare());
     m->tc_ready = smol::tensor_map_encoder() != nullptr && m->n_sms > 0;
     m->g = *g;
     m->ws = static_cast<char*>(d_workspace);
@@ -2478,18 +2441,50 @@ cudaError_t linear_ex<bf16>(SmolLm* m, const bf16* a, const bf16* w, float* y, i
     return cudaGetLastError();
 }
 
+// Width of the tcgen05 tiles: the one whose waves over the SMs take the fewest clocks.  A stage of a tile costs its bytes through the
+// SM's 64 bytes per clock from L2 (more than its MMAs cost at every width); the last epilogue follows the width.
+static int gemm_tc_pick(int row_tiles, int N, int K, int n_sms) {
+    static const int widths[] = {256, 192, 128, 96, 64};
+    const int nk = (K + smol::umma::kBK - 1) / smol::umma::kBK;
+    int best = 128;
+    double least = 1e30;
+    for (int bn : widths) {
+        const long long tiles = (long long)row_tiles * ((N + bn - 1) / bn), waves = (tiles + n_sms - 1) / n_sms;
+        const double clocks = (double)waves * nk * 2 * (smol::umma::kM + bn) + 6.0 * bn;
+        if (clocks < least) { least = clocks; best = bn; }
+    }
+    return best;
+}
+template <int BN>
+static bool launch_gemm_tc_sized(const bf16* a, const bf16* w, float* y, int M, int N, int row_tiles, int groups, int K, const GemmIo& io, int n_sms,
+                                 cudaStream_t st) {
+    CUtensorMap ta, tw;
+    if (!smol::make_tensor_map_2d(&ta, a, (uint64_t)M, (uint64_t)K, (uint64_t)K, (uint32_t)smol::umma::kM) ||
+        !smol::make_tensor_map_2d(&tw, w, (uint64_t)groups * N, (uint64_t)K, (uint64_t)K, (uint32_t)BN))
+        return false;
+    const long long tiles = (long long)row_tiles * ((N + BN - 1) / BN);
+    const int grid = io.tile_group ? n_sms : (int)std::min<long long>(tiles, n_sms);
+    gemm_tc_kernel<BN><<<grid, kTcThreads, gemm_tc_smem<BN>(), st>>>(ta, tw, y, M, N, K, io);
+    return true;
+}
+// false: the driver refused a tensor map (the caller takes another form)
+static bool launch_gemm_tc(const bf16* a, const bf16* w, float* y, int M, int N, int row_tiles, int groups, int K, const GemmIo& io, int n_sms, cudaStream_t st) {
+    switch (gemm_tc_pick(row_tiles, N, K, n_sms)) {
+        case 256: return launch_gemm_tc_sized<256>(a, w, y, M, N, row_tiles, groups, K, io, n_sms, st);
+        case 192: return launch_gemm_tc_sized<192>(a, w, y, M, N, row_tiles, groups, K, io, n_sms, st);
+        case 128: return launch_gemm_tc_sized<128>(a, w, y, M, N, row_tiles, groups, K, io, n_sms, st);
+        case 96: return launch_gemm_tc_sized<96>(a, w, y, M, N, row_tiles, groups, K, io, n_sms, st);
+        default: return launch_gemm_tc_sized<64>(a, w, y, M, N, row_tiles, groups, K, io, n_sms, st);
+    }
+}
+
 template <>
 cudaError_t linear<bf16>(SmolLm* m, const bf16* a, const bf16* w, float* y, int M, int N, int K, cudaStream_t st) {
     const bool aligned = K % 8 == 0 && (reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(w)) % 16 == 0;
-    if (M >= kTcMinRows && N >= kTcTileN && K >= smol::umma::kBK && aligned && m->tc_ready && reinterpret_cast<uintptr_t>(y) % 16 == 0) {
-        CUtensorMap ta, tw;
-        if (smol::make_tensor_map_2d(&ta, a, (uint64_t)M, (uint64_t)K, (uint64_t)K, (uint32_t)smol::umma::kM) &&
-            smol::make_tensor_map_2d(&tw, w, (uint64_t)N, (uint64_t)K, (uint64_t)K, (uint32_t)kTcTileN)) {
-            const int tiles = ((M + smol::umma::kM - 1) / smol::umma::kM) * ((N + kTcTileN - 1) / kTcTileN);
-            gemm_tc_kernel<<<std::min(tiles, m->n_sms), kTcThreads, kTcSmemBytes, st>>>(ta, tw, y, M, N, K, plain_io(K, N));
-            m->launches++;
-            return cudaGetLastError();
-        }
+    if (M >= kTcMinRows && N >= kTcMinCols && K >= smol::umma::kBK && aligned && m->tc_ready &&
+        launch_gemm_tc(a, w, y, M, N, (M + smol::umma::kM - 1) / smol::umma::kM, 1, K, plain_io(K, N), m->n_sms, st)) {
+        m->launches++;
+        return cudaGetLastError();
     }
     if (M <= kFewRows && aligned) {
         // the block's shape by N and K alone: a row's result must not depend on what else the step holds beyond its number of rows
@@ -2517,12 +2512,8 @@ cudaError_t linear<bf16>(SmolLm* m, const bf16* a, const bf16* w, float* y, int 
 static bool linear_grouped_tc(SmolLm* m, const bf16* a, const bf16* w, float* y, int rows, int groups, int N, int K, const GemmIo& io,
                               cudaStream_t st) {
     const bool aligned = K % 8 == 0 && (reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(w)) % 16 == 0;
-    if (!(N >= kTcTileN && K >= smol::umma::kBK && aligned && m->tc_ready && reinterpret_cast<uintptr_t>(y) % 16 == 0)) return false;
-    CUtensorMap ta, tw;
-    if (!smol::make_tensor_map_2d(&ta, a, (uint64_t)rows, (uint64_t)K, (uint64_t)K, (uint32_t)smol::umma::kM) ||
-        !smol::make_tensor_map_2d(&tw, w, (uint64_t)groups * N, (uint64_t)K, (uint64_t)K, (uint32_t)kTcTileN))
-        return false;
-    gemm_tc_kernel<<<m->n_sms, kTcThreads, kTcSmemBytes, st>>>(ta, tw, y, rows, N, K, io);
+    if (!(N >= kTcMinCols && K >= smol::umma::kBK && aligned && m->tc_ready)) return false;
+    if (!launch_gemm_tc(a, w, y, rows, N, rows / smol::umma::kM + groups / 2 + 1, groups, K, io, m->n_sms, st)) return false;
     m->launches++;
     return true;
 }
@@ -3068,7 +3059,7 @@ static int step_impl(SmolLm* m, const SmolLmStep* s, cudaStream_t st) {
                     // a handful of pairs (decoding), 32-row mma.sync tiles, 128-row tcgen05 tiles over rows copied into sorted order
                     const int NF = L.ff_plain ? L.ff : 2 * L.ff;          // rows of an expert's first matrix
                     const bool big = !kIsF32 && !few && m->tc_ready && pairs / L.n_experts >= 64 && D % 8 == 0 && L.ff % 8 == 0 &&
-                                     NF >= kTcTileN && D >= kTcTileN && D >= smol::umma::kBK && L.ff >= smol::umma::kBK;
+                                     NF >= kTcMinCols && D >= kTcMinCols && D >= smol::umma::kBK && L.ff >= smol::umma::kBK;
                     const int tile_rows = big ? smol::umma::kM : kGroupTile;
                     if (!direct) {
                         moe_index_kernel<<<1, 256, 0, st>>>(sel_id, pairs, L.n_experts, tile_rows, seg, perm, slot_of, tile_g, tile_r, n_tiles);

@@ -28,6 +28,20 @@ def test_products_of_few_rows(M, N, K):
     assert bool((err <= product_bound(a, w)).all())
 
 
+MANY_ROWS = ((257, 96, 64), (257, 4800, 72), (383, 97, 128), (384, 9600, 200), (512, 255, 72), (640, 257, 1000), (1025, 770, 520), (2048, 2049, 264),
+             (300, 6400, 4608))
+
+
+@pytest.mark.parametrize("M,N,K", MANY_ROWS)
+def test_products_of_many_rows(M, N, K):
+    """tcgen05 tiles of 64 to 256 columns: ragged rows, columns and last K stage, one tile per SM and several."""
+    model, _, _ = engine_and_oracle(config([attn(ff=0)]), seed=9, dtype=torch.bfloat16)
+    g = torch.Generator(device="cuda").manual_seed(M * 31 + K)
+    a, w = (torch.randn(r, K, device="cuda", generator=g).bfloat16() for r in (M, N))
+    err = (model.linear(a, w).double() - a.double() @ w.double().T).abs()
+    assert bool((err <= product_bound(a, w)).all())
+
+
 F32_TILES = ((1, 1, 4), (16, 65, 36), (17, 64, 128), (64, 63, 132), (65, 130, 260), (300, 768, 1028), (31, 70, 2048), (512, 4700, 20), (640, 3841, 52))
 
 

@@ -1493,6 +1493,7 @@ struct DeltaArgs {
 };
 
 // Per token and channel: decay w = exp(-coef * sigmoid(w2 tanh(inner) + bias)), unit key u, removal vector a * u.
+// ukey nullptr: the decay alone (the four-token scan takes the rest from the projection).
 // A block takes TT tokens and blockDim.x channels: the second decay matrix (rank x HD fp32, from L2) is read once per TT tokens.
 // One token per block made 2048 tokens of 12 x 64 channels and rank 64 read 400 MB of it: 84 us; eight: 27 us.
 template <int TT>
@@ -1508,7 +1509,7 @@ __global__ void __launch_bounds__(128) delta_prep_kernel(const DeltaArgs A, floa
     const int c_lo = blockIdx.y * blockDim.x, c_hi = min(HD, c_lo + blockDim.x);      // this block's channels (gridDim.y slices cover HD)
     if (c_lo >= c_hi) return;
     const int h_lo = c_lo / A.d, nh = (c_hi - 1) / A.d - h_lo + 1;
-    for (int x = warp; x < nh * nt; x += nw) {
+    for (int x = warp; ukey && x < nh * nt; x += nw) {
         const int tt = x / nh, h = h_lo + x - tt * nh;
         const float* k = A.proj + (size_t)(t0 + tt) * A.n_in + HD + h * A.d;
         float ss = 0.0f;
@@ -1535,8 +1536,9 @@ __global__ void __launch_bounds__(128) delta_prep_kernel(const DeltaArgs A, floa
         if (tt < nt) {
             const float* row = A.proj + (size_t)(t0 + tt) * A.n_in;
             const size_t at = (size_t)(t0 + tt) * HD + c;
-            const float u = row[HD + c] * inv[tt * A.H + c / A.d];
             decay[at] = expf(-A.decay_coef * sigmoidf_(lo[tt]));
+            if (!ukey) continue;
+            const float u = row[HD + c] * inv[tt * A.H + c / A.d];
             ukey[at] = u;
             aukey[at] = sigmoidf_(row[4 * HD + c] + rb) * u;
         }
@@ -1768,6 +1770,7 @@ __global__ void __launch_bounds__(kThreads) lm_sample_kernel(const float* __rest
 #include "lm_mechanisms.cuh"
 #include "lm_sigmoid_linear.cuh"
 #include "lm_delta_mlstm.cuh"
+#include "lm_quad_scan.cuh"
 
 // =====================================================================================================================
 // Host side
@@ -1803,6 +1806,7 @@ struct SmolLm {
     std::vector<RunInfo> side_runs;       // the cache / state placement of a run's side mixer
     size_t o_conv = 0, o_head = 0;        // state-space: convolved channels [T][channels], per-head decay and step [2][T][heads]
     int max_conv = 0, max_ssd_heads = 0;
+    size_t o_rec = 0, max_rec = 0;        // prompts' four-token scan: records of a group over all heads [floats]
     size_t o_pairs = 0;                   // four-token scan: products between a group's queries and keys
     int max_pair_heads = 0;
     SmolLmGlobals g{};
@@ -2205,6 +2209,17 @@ extern "C" int smol_lm_create(const SmolLmConfig* cfg, const SmolLmLayer* layers
         m->o_conv = carve(T * (size_t)m->max_conv * 4);
         m->o_head = carve(2 * T * (size_t)m->max_ssd_heads * 4);
     }
+    for (const RunInfo& r : m->runs)
+        for (const SmolLmLayer* L : {(const SmolLmLayer*)&m->layers[r.layer], m->layers[r.layer].side}) {
+            if (!L) continue;
+            const bool ssd = L->mixer == SMOL_LM_MIX_STATE_SPACE;
+            int form = -1;
+            if (L->mixer == SMOL_LM_MIX_GENERAL_DELTA) form = kFormGeneral;
+            else if (ssd || L->mixer == SMOL_LM_MIX_GATED_LINEAR || L->mixer == SMOL_LM_MIX_LIGHTNING || L->mixer == SMOL_LM_MIX_HGRN2 ||
+                     L->mixer == SMOL_LM_MIX_RETENTION) form = kFormAdd;
+            if (form >= 0) m->max_rec = std::max(m->max_rec, (size_t)L->heads * quad_record(form, quad_pad(ssd ? L->n_state : L->dim)));
+        }
+    if (m->max_rec > 0 && cfg->max_step_tokens >= kQuadMinTokens) m->o_rec = carve((T / kQuad + cfg->max_step_seqs + 1) * m->max_rec * 4);
     if (m->max_pair_heads > 0) m->o_pairs = carve(T * (size_t)m->max_pair_heads * kPairFloats * 4);
     if (m->max_top > 0) {
         const size_t pairs = T * (size_t)m->max_top;
@@ -2249,6 +2264,12 @@ static cudaError_t scan_attribute() {
     if (e == cudaSuccess) e = cudaFuncSetAttribute(gla_scan_kernel<DK, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, std::max(kScanSpread, (int)(2 * gla_buf_floats(DK) * sizeof(float))));
     return e;
 }
+template <int DK>
+static cudaError_t quad_attribute() {
+    cudaError_t e = cudaFuncSetAttribute(quad_scan_kernel<DK, kFormAdd>, cudaFuncAttributeMaxDynamicSharedMemorySize, std::max(kScanSpread, (int)quad_smem(kFormAdd, DK)));
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(quad_scan_kernel<DK, kFormGeneral>, cudaFuncAttributeMaxDynamicSharedMemorySize, std::max(kScanSpread, (int)quad_smem(kFormGeneral, DK)));
+    return e;
+}
 static constexpr int flash_smem_bytes(int DK, int DV, bool vk, int maps = 1) { return 2 * 64 * (maps * (DK + 8) + (vk ? 0 : DV + 8)) * (int)sizeof(bf16); }
 
 template <int DK, int HPW>
@@ -2265,6 +2286,10 @@ static cudaError_t set_kernel_attributes() {
     if (e == cudaSuccess) e = scan_attribute<64>();
     if (e == cudaSuccess) e = scan_attribute<128>();
     if (e == cudaSuccess) e = scan_attribute<256>();
+    if (e == cudaSuccess) e = quad_attribute<32>();
+    if (e == cudaSuccess) e = quad_attribute<64>();
+    if (e == cudaSuccess) e = quad_attribute<128>();
+    if (e == cudaSuccess) e = quad_attribute<256>();
     if (e == cudaSuccess) e = cudaFuncSetAttribute(attn_split_kernel<T, 8, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, kAttnSplitSmemMax);
     if (e == cudaSuccess) e = cudaFuncSetAttribute(attn_split_kernel<T, 8, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, kAttnSplitWideSmem);
     if (e == cudaSuccess) e = cudaFuncSetAttribute(attn_split_kernel<T, 16, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, kAttnSplitSmemMax);
@@ -2526,6 +2551,30 @@ static cudaError_t launch_scan(const DeltaArgs& A, int n_seqs, const float* dec,
     return cudaGetLastError();
 }
 
+// The four-token scan over a step in which some sequence brings at least kQuadMinTokens tokens (fewer: its two launches cost more than
+// the chain they shorten).
+template <int KIND, int DK>
+static cudaError_t launch_quad_sized(SmolLm* m, QuadSource Q, QuadArgs A, int n_seqs, int max_n, float* o_raw, cudaStream_t st, size_t min_smem) {
+    constexpr int FORM = quad_form(KIND);
+    float* rec = reinterpret_cast<float*>(m->ws + m->o_rec);
+    Q.cap = A.cap = m->cfg.max_step_tokens / kQuad + m->cfg.max_step_seqs + 1;
+    quad_prep_kernel<KIND, DK><<<dim3((max_n + kQuad - 1) / kQuad, n_seqs, (Q.H + 3) / 4), 128, 0, st>>>(Q, rec);
+    A.rec = rec;
+    const int parts = (A.dv + kQuadCols - 1) / kQuadCols;
+    quad_scan_kernel<DK, FORM><<<n_seqs * A.H * parts, kQuadThreads, std::max(quad_smem(FORM, DK), min_smem), st>>>(A, m->slots, o_raw);
+    m->launches += 1;
+    return cudaGetLastError();
+}
+template <int KIND>
+static cudaError_t launch_quad(SmolLm* m, const QuadSource& Q, const QuadArgs& A, int n_seqs, int max_n, float* o_raw, cudaStream_t st, size_t min_smem = 0) {
+    switch (quad_pad(A.d)) {
+        case 32: return launch_quad_sized<KIND, 32>(m, Q, A, n_seqs, max_n, o_raw, st, min_smem);
+        case 64: return launch_quad_sized<KIND, 64>(m, Q, A, n_seqs, max_n, o_raw, st, min_smem);
+        case 128: return launch_quad_sized<KIND, 128>(m, Q, A, n_seqs, max_n, o_raw, st, min_smem);
+        default: return launch_quad_sized<KIND, 256>(m, Q, A, n_seqs, max_n, o_raw, st, min_smem);
+    }
+}
+
 template <int DK>
 static cudaError_t launch_gla_scan(const GlaArgs& A, int n_seqs, const float* dec, float* pool, float* o_raw, cudaStream_t st, size_t min_smem) {
     constexpr int CB = gla_block_cols(DK), threads = CB * gla_lanes(DK);
@@ -2536,8 +2585,14 @@ static cudaError_t launch_gla_scan(const GlaArgs& A, int n_seqs, const float* de
     return cudaGetLastError();
 }
 // the scan over key sizes up to 256: the smallest built size that holds A.d
-static cudaError_t launch_gla_scan_any(const GlaArgs& A, int n_seqs, const float* dec, float* pool, float* o_raw, cudaStream_t st,
+static cudaError_t launch_gla_scan_any(SmolLm* m, const GlaArgs& A, int n_seqs, int max_n, const float* dec, float* pool, float* o_raw, cudaStream_t st,
                                         size_t min_smem = 0) {
+    if (max_n >= kQuadMinTokens) {
+        QuadSource Q{A.H, A.qk_share, A.d, A.q_src, A.k_src, A.q_ld, A.k_ld, dec, A.head_decay, A.head_step, A.head_ld, 1, nullptr, nullptr, 0.0f, A.seq_start, 0};
+        QuadArgs S{A.H, A.d, A.dv, nullptr, 0, A.v_src, A.v_ld, A.q_scale, A.seq_start, A.seq_pos0, A.seq_slot, A.slot_floats, A.state_off, A.n_slots, A.err};
+        if (A.head_decay) return launch_quad<kQuadHeadDecay>(m, Q, S, n_seqs, max_n, o_raw, st, min_smem);
+        return launch_quad<kQuadChannelDecay>(m, Q, S, n_seqs, max_n, o_raw, st, min_smem);
+    }
     if (A.d <= 16) return launch_gla_scan<16>(A, n_seqs, dec, pool, o_raw, st, min_smem);
     if (A.d <= 32) return launch_gla_scan<32>(A, n_seqs, dec, pool, o_raw, st, min_smem);
     if (A.d <= 64) return launch_gla_scan<64>(A, n_seqs, dec, pool, o_raw, st, min_smem);
@@ -2729,6 +2784,7 @@ static int step_impl(SmolLm* m, const SmolLmStep* s, cudaStream_t st) {
     auto norm_of = [&](const float* w, const float* shift, const float* alpha) { return NormSpec{c.norm_kind, w, shift, alpha, c.norm_eps}; };
     const NormSpec no_norm{c.norm_kind, nullptr, nullptr, nullptr, c.norm_eps}, copy_row{kNormCopy, nullptr, nullptr, nullptr, c.norm_eps};
     const size_t hist_stride = (size_t)Tn * D;
+    const int max_n = s->max_seq_tokens > 0 ? s->max_seq_tokens : Tn;      // most tokens a sequence brings
     constexpr bool kIsF32 = sizeof(T) == 4;
     const float woff = c.norm_plain ? 0.0f : 1.0f;
     float* conv = reinterpret_cast<float*>(m->ws + m->o_conv);
@@ -2827,7 +2883,7 @@ static int step_impl(SmolLm* m, const SmolLmStep* s, cudaStream_t st) {
             A.qk_share = M.heads / M.bc_groups;
             A.head_decay = head; A.head_step = head + (size_t)Tn * M.heads; A.head_ld = M.heads;
             A.out_ld = out_ld_now; A.out_scale = 1.0f;
-            CU(launch_gla_scan_any(A, s->n_seqs, nullptr, m->slots, oraw, ms));
+            CU(launch_gla_scan_any(m, A, s->n_seqs, max_n, nullptr, m->slots, oraw, ms));
             ssd_out_kernel<T><<<dim3(Tn, M.norm_parts), 256, 0, ms>>>(P, oraw, conv, mix_at, m->slots);
             m->launches += 3;
             return SMOL_OK;
@@ -2857,7 +2913,6 @@ static int step_impl(SmolLm* m, const SmolLmStep* s, cudaStream_t st) {
             sigmoid_prep_kernel<T><<<(units + 3) / 4, 128, 0, ms>>>(S, qbuf, pool);
             m->launches += 1;
             const int min_n = s->min_seq_tokens > 0 ? s->min_seq_tokens : 1;
-            const int max_n = s->max_seq_tokens > 0 ? s->max_seq_tokens : Tn;
             // sequences that bring more than a few tokens take the tiled tensor-core form (bf16), the others a warp per head
             const bool tiled = max_n > kShortSeq && launch_sigmoid_flash(m, s, S, max_n, reinterpret_cast<const bf16*>(qbuf), reinterpret_cast<const bf16*>(pool),
                                                                          reinterpret_cast<bf16*>(mix_at), sizeof(T) == 2, ms);
@@ -2909,7 +2964,7 @@ static int step_impl(SmolLm* m, const SmolLmStep* s, cudaStream_t st) {
             A.q_src = conv; A.k_src = conv + hd; A.v_src = conv + 2 * hd;
             A.q_ld = A.k_ld = A.v_ld = na;
             A.head_decay = head; A.head_step = head + (size_t)Tn * M.heads;
-            CU(launch_gla_scan_any(A, s->n_seqs, nullptr, m->slots, oraw, ms));
+            CU(launch_gla_scan_any(m, A, s->n_seqs, max_n, nullptr, m->slots, oraw, ms));
             LinOutArgs O{pj, n_in, hv, hv, hv, 1, ld, (size_t)2 * hd + hv, c.norm_eps, 1.0f, M.out_norm};
             lin_attn_out_kernel<T><<<dim3(Tn, 1), 256, 0, ms>>>(O, oraw, mix_at);
             m->launches += 3;
@@ -2924,14 +2979,13 @@ static int step_impl(SmolLm* m, const SmolLmStep* s, cudaStream_t st) {
             A.q_src = conv; A.k_src = conv + hd; A.v_src = pj + 2 * hd;
             A.q_ld = A.k_ld = 2 * hd; A.v_ld = n_in;
             A.head_decay = M.head_decay; A.head_ld = 0;
-            CU(launch_gla_scan_any(A, s->n_seqs, nullptr, m->slots, oraw, ms, parallel && Tn > kGraphMaxTokens ? kScanSpread : 0));
+            CU(launch_gla_scan_any(m, A, s->n_seqs, max_n, nullptr, m->slots, oraw, ms, parallel && Tn > kGraphMaxTokens ? kScanSpread : 0));
             A.out_ld = ld; A.out_scale = M.mix_scale;
             gla_out_kernel<T><<<(Tn * M.heads + 3) / 4, 128, 0, ms>>>(A, oraw, mix_at);
             m->launches += 3;
             return SMOL_OK;
         };
         // The four-token scan's arguments for a state [dim, vdim] per head in the slot.
-        const int max_n = s->max_seq_tokens > 0 ? s->max_seq_tokens : Tn;
         float* pairs = reinterpret_cast<float*>(m->ws + m->o_pairs);
         auto group_args = [&](const SmolLmLayer& M, const RunInfo& Ri, int G) {
             GroupScanArgs A;
@@ -3167,7 +3221,7 @@ static int step_impl(SmolLm* m, const SmolLmStep* s, cudaStream_t st) {
             GlaArgs A = scan_args(L, R, proj);
             A.q_src = uk; A.k_src = auk; A.v_src = proj + 2 * hd;
             A.q_ld = A.k_ld = hd; A.v_ld = n_in;
-            CU(launch_gla_scan_any(A, s->n_seqs, dec, m->slots, oraw, st));
+            CU(launch_gla_scan_any(m, A, s->n_seqs, max_n, dec, m->slots, oraw, st));
             LinOutArgs O{proj, n_in, hv, L.vdim, L.vdim, 0, hv, 0, c.norm_eps, 1.0f, L.out_norm};
             lin_attn_out_kernel<T><<<dim3(Tn, L.heads), 128, 0, st>>>(O, oraw, mix);
             m->launches += 3;
@@ -3233,7 +3287,7 @@ static int step_impl(SmolLm* m, const SmolLmStep* s, cudaStream_t st) {
             if (Tn >= kDecayMinTokens && kDecayTokens * L.rank * sizeof(float) <= 48 * 1024)
                 gla_prep_kernel<kDecayTokens><<<dim3((Tn + kDecayTokens - 1) / kDecayTokens, slices), 128, kDecayTokens * L.rank * sizeof(float), st>>>(A, dec);
             else gla_prep_kernel<1><<<dim3(Tn, slices), 128, L.rank * sizeof(float), st>>>(A, dec);
-            CU(launch_gla_scan_any(A, s->n_seqs, dec, m->slots, oraw, st));
+            CU(launch_gla_scan_any(m, A, s->n_seqs, max_n, dec, m->slots, oraw, st));
             gla_out_kernel<T><<<(Tn * L.heads + 3) / 4, 128, 0, st>>>(A, oraw, mix);
             m->launches += 3;
             mix_cols = L.heads * L.vdim;
@@ -3244,13 +3298,20 @@ static int step_impl(SmolLm* m, const SmolLmStep* s, cudaStream_t st) {
             A.rate_bias = L.rate_bias; A.decay_w2 = L.decay_w2; A.decay_bias = L.decay_bias; A.out_norm = L.out_norm;
             A.seq_start = s->seq_start; A.seq_pos0 = s->seq_pos0; A.seq_slot = s->seq_slot;
             A.slot_floats = m->slot_floats; A.state_off = R.state_off; A.n_slots = m->n_slots; A.err = err;
+            const bool quad = max_n >= kQuadMinTokens;
+            float *u_to = quad ? nullptr : uk, *au_to = quad ? nullptr : auk;
             const size_t prep_smem = (size_t)(L.rank + L.heads) * sizeof(float);
             const int slices = (L.heads * L.dim + 127) / 128;
             if (Tn >= kDecayMinTokens && kDecayTokens * prep_smem <= 48 * 1024)
-                delta_prep_kernel<kDecayTokens><<<dim3((Tn + kDecayTokens - 1) / kDecayTokens, slices), 128, kDecayTokens * prep_smem, st>>>(A, dec, uk, auk);
-            else delta_prep_kernel<1><<<dim3(Tn, slices), 128, prep_smem, st>>>(A, dec, uk, auk);
+                delta_prep_kernel<kDecayTokens><<<dim3((Tn + kDecayTokens - 1) / kDecayTokens, slices), 128, kDecayTokens * prep_smem, st>>>(A, dec, u_to, au_to);
+            else delta_prep_kernel<1><<<dim3(Tn, slices), 128, prep_smem, st>>>(A, dec, u_to, au_to);
             cudaError_t e;
-            if (L.dim <= 16) e = launch_scan<16>(A, s->n_seqs, dec, uk, auk, m->slots, oraw, st);
+            if (quad) {
+                const int HD = L.heads * L.dim;
+                QuadSource Q{L.heads, 1, L.dim, proj, proj + HD, n_in, n_in, dec, nullptr, nullptr, 0, 0, proj + 4 * HD, L.rate_bias, L.unit_eps, s->seq_start, 0};
+                QuadArgs S{L.heads, L.dim, L.dim, nullptr, 0, proj + 2 * HD, n_in, 1.0f, s->seq_start, s->seq_pos0, s->seq_slot, m->slot_floats, R.state_off, m->n_slots, err};
+                e = launch_quad<kQuadGeneralDelta>(m, Q, S, s->n_seqs, max_n, oraw, st);
+            } else if (L.dim <= 16) e = launch_scan<16>(A, s->n_seqs, dec, uk, auk, m->slots, oraw, st);
             else if (L.dim <= 32) e = launch_scan<32>(A, s->n_seqs, dec, uk, auk, m->slots, oraw, st);
             else if (L.dim <= 64) e = launch_scan<64>(A, s->n_seqs, dec, uk, auk, m->slots, oraw, st);
             else if (L.dim <= 128) e = launch_scan<128>(A, s->n_seqs, dec, uk, auk, m->slots, oraw, st);

@@ -65,3 +65,32 @@ def test_decay_preparation_over_groups_of_tokens(n):
     got = model.forward([(seq, toks, list(range(n)))]).clone()
     model.close_sequence(seq)
     assert rel_err(got, orc.forward(toks)) < TOL[torch.float32]
+
+
+@pytest.mark.parametrize("dim", [5, 32, 33, 64, 96, 200])
+def test_four_token_scan_of_prompts(dim):
+    """Every form of the recurrence, padded key channels, groups and chunks that end anywhere: sequences of 16 to 67 tokens beside a
+    single token, continued by a second portion, against the oracles."""
+    import maferax_util as mu
+    import virusun_util as vu
+
+    lens = (67, 16, 19, 1)
+    cases = [(config([delta(heads=3, dim=dim, ff=0, rank=5)], vocab=61, width=48), engine_and_oracle),
+             (mu.config([mu.gla(heads=2, dim=dim, vdim=11)], vocab=61, width=48), mu.engine_and_oracle),
+             (vu.config([vu.delta(heads=4, kv_heads=2, dim=dim, vdim=9, conv=3)], vocab=61, width=48), vu.engine_and_oracle),
+             (vu.config([vu.par(b=vu.right(heads=2, dim=dim, vdim=8))], vocab=61, width=48), vu.engine_and_oracle)]
+    for cfg, make in cases:
+        model, orc, _ = make(cfg, seed=4, max_tokens=2048, max_seqs=4, page_size=16, max_step_tokens=256)
+        toks = [tokens(n + 18, 61, n) for n in lens]
+        want = [orc.forward(t) for t in toks]
+        seqs = [model.open_sequence() for _ in lens]
+        first = model.forward([(s, t[:n], list(range(n))) for s, t, n in zip(seqs, toks, lens)]).clone()
+        then = model.forward([(s, t[n:], list(range(18))) for s, t, n in zip(seqs, toks, lens)]).clone()
+        for s in seqs:
+            model.close_sequence(s)
+        at = 0
+        for i, n in enumerate(lens):
+            if n > 1:
+                assert rel_err(first[at:at + n], want[i][:n]) < TOL[torch.float32]
+            assert rel_err(then[18 * i:18 * i + 18], want[i][n:]) < TOL[torch.float32]
+            at += n

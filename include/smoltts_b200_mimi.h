@@ -96,6 +96,15 @@ int smol_mimi_reset(SmolMimi* m, const int32_t* d_slots, int32_t n, void* stream
 int smol_mimi_decode_step(SmolMimi* m, const int32_t* d_codes, const int32_t* d_slots, int32_t batch, float* d_pcm,
                           void* stream);
 
+/* A run of `frames` decode_step calls at once, for utterances whose codes are all there (weights are then read once per run): d_codes
+ * int32 [batch][frames][n_q], d_pcm fp32 [batch][frames * samples_per_frame].  1 <= frames <= smol_mimi_max_frames(m, batch), which is 1
+ * unless smol_mimi_set_max_frames (1 .. 8; after create, before smol_mimi_workspace_bytes) has made room for more: 3 MB of workspace per
+ * stream and frame. */
+int smol_mimi_set_max_frames(SmolMimi* m, int32_t frames);
+int32_t smol_mimi_max_frames(const SmolMimi* m, int32_t batch);
+int smol_mimi_decode_frames(SmolMimi* m, const int32_t* d_codes, const int32_t* d_slots, int32_t batch, int32_t frames, float* d_pcm,
+                            void* stream);
+
 /* Test / profiling hooks: intermediate buffers by name ("emb": upsampled embeddings, "xf": transformer output; slot-major),
  * kernel launches per step, device-side error word (nonzero: a stream ran past max_positions). */
 void* smol_mimi_debug_buffer(SmolMimi* m, const char* name, int64_t* slot_stride_floats);

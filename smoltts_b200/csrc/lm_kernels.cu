@@ -301,11 +301,18 @@ __global__ void __launch_bounds__(f32t::Tile<BM, BN, TM, TN>::NT) gemm_f32_tile_
     int k_lo, k_hi;
     T::range(K, k_lo, k_hi);
     float out[TM][TN];
-    T::template product<false>(f32_sm, k_lo, k_hi, [&](int r, int k) { return arow[r] >= 0 ? a + arow[r] + k : nullptr; },
-                               [&](int r, int k) { return n0 + r < N ? w + (size_t)(n0 + r) * K + k : nullptr; },
+    T::template product<false>(f32_sm, k_lo, k_hi, [&](int r) { return arow[r] >= 0 ? a + arow[r] : nullptr; }, [](int k) -> long long { return k; },
+                               [&](int r) { return n0 + r < N ? w + (size_t)(n0 + r) * K : nullptr; },
                                [](float4 v, int, int) { return v; }, [] {}, out);
-    T::finish(f32_sm, out, [&](int r, int c, float v) {
-        if (m0 + r < M && n0 + c < N) y[(size_t)(m0 + r) * io.ldy + n0 + c] = v;
+    const bool whole = io.ldy % 4 == 0 && reinterpret_cast<uintptr_t>(y) % 16 == 0;
+    T::finish(f32_sm, out, [&](int r, int c, float4 v) {
+        if (m0 + r >= M) return;
+        float* to = y + (size_t)(m0 + r) * io.ldy + n0 + c;
+        if (whole && n0 + c + 4 <= N) { *reinterpret_cast<float4*>(to) = v; return; }
+        if (n0 + c < N) to[0] = v.x;
+        if (n0 + c + 1 < N) to[1] = v.y;
+        if (n0 + c + 2 < N) to[2] = v.z;
+        if (n0 + c + 3 < N) to[3] = v.w;
     });
 }
 
@@ -2390,9 +2397,10 @@ template <int BM, int BN, int TM, int TN>
 static cudaError_t launch_f32_tile(const float* a, const float* w, float* y, int M, int N, int K, const GemmIo& io, int batch, int row_tiles, cudaStream_t st) {
     using T = smol::f32t::Tile<BM, BN, TM, TN>;
     const int cols = (N + BN - 1) / BN;
-    // CTAs per tile: as many as bring the grid to two per SM, each with at least 128 k
+    // CTAs per tile: as many as bring the grid to about six per SM (four of a 64 x 64 tile's run side by side; fewer leave its FMAs waiting
+    // for loads and some SMs with a third more work than others), each with at least 128 k
     int S = 1;
-    while (S < 8 && (long long)cols * row_tiles * batch * S < 2 * 148 && K / (2 * S) >= 128) S *= 2;
+    while (S < 8 && (long long)cols * row_tiles * batch * S < 4 * 148 && K / (2 * S) >= 128) S *= 2;
     if (T::kSmemBytes > 48 * 1024)
         if (const cudaError_t e = cudaFuncSetAttribute(gemm_f32_tile_kernel<BM, BN, TM, TN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)T::kSmemBytes)) return e;
     cudaLaunchConfig_t cfg{};
@@ -2414,12 +2422,9 @@ cudaError_t linear_ex<float>(SmolLm* m, const float* a, const float* w, float* y
     m->launches++;
     // whole 16-byte pieces in every row of both operands
     if (K % 4 == 0 && io.lda % 4 == 0 && io.sa % 4 == 0 && io.sw % 4 == 0 && (reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(w)) % 16 == 0) {
-        if (io.tile_group) return launch_f32_tile<kGroupTile, 64, 4, 4>(a, w, y, M, N, K, io, 1, tiles, st);
-        if (M <= 16) return launch_f32_tile<16, 64, 4, 2>(a, w, y, M, N, K, io, batch, (M + 15) / 16, st);
-        // 128 x 128 tiles (16 loads feed 128 FMAs, against 12 for 64) where they fill the SMs and waste little of the last row tile
-        const long long big = (long long)((M + 127) / 128) * ((N + 127) / 128) * batch;
-        if (big >= 148 && M >= 512) return launch_f32_tile<128, 128, 8, 8>(a, w, y, M, N, K, io, batch, (M + 127) / 128, st);
-        return launch_f32_tile<64, 64, 8, 4>(a, w, y, M, N, K, io, batch, (M + 63) / 64, st);
+        if (io.tile_group) return launch_f32_tile<kGroupTile, 64, 8, 8>(a, w, y, M, N, K, io, 1, tiles, st);
+        if (M <= 16) return launch_f32_tile<16, 64, 4, 4>(a, w, y, M, N, K, io, batch, (M + 15) / 16, st);
+        return launch_f32_tile<64, 64, 8, 8>(a, w, y, M, N, K, io, batch, (M + 63) / 64, st);
     }
     if (io.tile_group) {
         dim3 grid((N + 63) / 64, tiles, 1);

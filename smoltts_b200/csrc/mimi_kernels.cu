@@ -9,12 +9,12 @@
 // At streaming batch sizes every stage is a handful of rows (2 .. 1920 per stream) against a weight matrix that is read
 // once: weight-streaming "row" products.  ONE kernel shape carries them all (rows_kernel): a CTA stages up to 16 input
 // rows in shared memory -- gathered straight from the producer's buffer, im2col of a causal convolution = a contiguous run
-// of (kernel x channels) floats that begins in the carried history rows; ELU or LayerNorm applied while staging -- and every
-// warp streams one weight row (four from 64 rows on) with 16-byte loads against all staged rows, finishing with a shuffle
-// reduction and a fused epilogue (bias, GELU, layer scale + residual, residual, or the upsampler).  Transposed convolutions
+// of (kernel x channels) floats that begins in the carried history rows; LayerNorm applied while staging -- and every
+// warp streams one weight row with 16-byte loads against all staged rows, finishing with a shuffle reduction and a fused
+// epilogue (bias, GELU, layer scale + residual, residual, the upsampler, the ELU of what reads the result).  Transposed convolutions
 // (kernel = 2 stride) are the same product with K = (previous | current input row) x channels and N = (phase, channel): their
-// outputs land contiguously.  From 12 streams on the SEANet's many-row stages run as 64 x 64 register tiles (tile_kernel) and
-// the one-channel last convolution as one thread per sample (rowdot_kernel).  Attention: one CTA per (stream, head, split
+// outputs land contiguously.  The SEANet's stages of 16 and more rows per frame, and from 12 streams on everything, run as register
+// tiles on packed FMAs (tile_kernel), the one-channel last convolution from shared memory (rowdot_kernel).  Attention: one CTA per (stream, head, split
 // of 512 cached positions), partial softmaxes combined in split order.  Everything a stream carries (convolution history
 // rows, the upsampler's previous embedding, KV cache, position) lives in per-slot arenas of the caller's workspace; a step is
 // a program of 57 operations, one launch each, replayed as one CUDA graph.
@@ -33,6 +33,7 @@
 
 #include "../../include/smoltts_b200.h"
 #include "../../include/smoltts_b200_mimi.h"
+#include "f32_tile.cuh"
 
 namespace smol {
 int capi_fail(int code, const std::string& msg);              // capi.cu: sets smol_last_error()
@@ -43,9 +44,9 @@ namespace mimi {
 constexpr int kThreads = 256;
 constexpr int kWarps = kThreads / 32;
 constexpr int kStageFloats = 8192;   // shared-memory staging area of rows_kernel: R rows x (8192 / R) floats
-constexpr int kMaxBufs = 24;
+constexpr int kMaxBufs = 32;
 
-enum { PRO_NONE = 0, PRO_ELU = 1, PRO_LN = 2 };
+enum { PRO_NONE = 0, PRO_LN = 1 };
 enum { EPI_BIAS = 0, EPI_GELU = 1, EPI_SCALE_RES = 2, EPI_RES = 3, EPI_UPSAMPLE = 4 };
 
 struct RowOp {
@@ -56,10 +57,13 @@ struct RowOp {
     float* out; long long out_stride; int out_off0, out_by_row;
     const float* res; long long res_stride; int res_off0;
     int pro, epi;
+    int elu;                                       // the output is stored through an ELU (what reads it wants nothing else) ...
+    float* raw; long long raw_stride; int raw_off0;   // ... and as it is here (nullptr: nowhere): the residual of the block that follows
     const float* ln_w; const float* ln_b; float eps;
+    float* norm_at;                                // slot arena: where the rows go after their LayerNorm when the product runs on tiles
     const float* scale;
     const float* wup; float* up_prev; int carry;   // EPI_UPSAMPLE
-    const int32_t* slots; int batch;
+    const int32_t* slots; int batch, frames;       // T: rows of all `frames` frames of the call
 };
 
 __device__ __forceinline__ float warp_sum(float v) {
@@ -78,6 +82,55 @@ __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;"
 __device__ __forceinline__ void pdl_go() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
 
+// The epilogue of output n of row (slot, t), batch row b.
+__device__ __forceinline__ void store_row(const RowOp& op, int b, int slot, int t, int n, float y) {
+    if (op.epi == EPI_UPSAMPLE) {
+        // grouped transposed convolution, kernel 4, stride 2 (conv.py:271-282): outputs 2 t + j take tap j of this frame
+        // and, with `carry`, tap 2 + j of the previous one (one frame per call then); decode_step upsamples every frame alone (carry = 0)
+        const float4 wu = *reinterpret_cast<const float4*>(op.wup + 4 * n);
+        float o0 = y * wu.x, o1 = y * wu.y;
+        if (op.carry) {
+            float* pp = op.up_prev + (long long)slot * op.N + n;
+            const float pv = *pp;
+            o0 = fmaf(pv, wu.z, o0); o1 = fmaf(pv, wu.w, o1);
+            *pp = y;
+        }
+        float* o = op.out + (long long)slot * op.out_stride + op.out_off0 + (long long)(2 * t) * op.N + n;
+        o[0] = o0; o[op.N] = o1;
+        return;
+    }
+    const long long e = (long long)t * op.N + n;
+    if (op.epi == EPI_GELU) y = gelu_erf(y);
+    else if (op.epi == EPI_SCALE_RES) y = op.res[(long long)slot * op.res_stride + op.res_off0 + e] + y * op.scale[n];
+    else if (op.epi == EPI_RES) y = op.res[(long long)slot * op.res_stride + op.res_off0 + e] + y;
+    if (op.raw) op.raw[(long long)slot * op.raw_stride + op.raw_off0 + e] = y;
+    op.out[(long long)(op.out_by_row ? b : slot) * op.out_stride + op.out_off0 + e] = op.elu ? elu1(y) : y;
+}
+
+// Outputs n .. n + 3 (n, N and bias_mod multiples of 4), bias included.
+__device__ __forceinline__ void store_row4(const RowOp& op, int b, int slot, int t, int n, float4 y) {
+    if (op.bias) {
+        const float4 w = *reinterpret_cast<const float4*>(op.bias + n % op.bias_mod);
+        y.x += w.x; y.y += w.y; y.z += w.z; y.w += w.w;
+    }
+    if (op.epi == EPI_UPSAMPLE) {
+        store_row(op, b, slot, t, n, y.x); store_row(op, b, slot, t, n + 1, y.y);
+        store_row(op, b, slot, t, n + 2, y.z); store_row(op, b, slot, t, n + 3, y.w);
+        return;
+    }
+    const long long e = (long long)t * op.N + n;
+    if (op.epi == EPI_GELU) {
+        y = make_float4(gelu_erf(y.x), gelu_erf(y.y), gelu_erf(y.z), gelu_erf(y.w));
+    } else if (op.epi == EPI_SCALE_RES || op.epi == EPI_RES) {
+        const float4 r = *reinterpret_cast<const float4*>(op.res + (long long)slot * op.res_stride + op.res_off0 + e);
+        const float4 w = op.epi == EPI_RES ? make_float4(1.f, 1.f, 1.f, 1.f) : *reinterpret_cast<const float4*>(op.scale + n);
+        y = make_float4(r.x + y.x * w.x, r.y + y.y * w.y, r.z + y.z * w.z, r.w + y.w * w.w);
+    }
+    if (op.raw) *reinterpret_cast<float4*>(op.raw + (long long)slot * op.raw_stride + op.raw_off0 + e) = y;
+    if (op.elu) y = make_float4(elu1(y.x), elu1(y.y), elu1(y.z), elu1(y.w));
+    *reinterpret_cast<float4*>(op.out + (long long)(op.out_by_row ? b : slot) * op.out_stride + op.out_off0 + e) = y;
+}
+
 // Y[row][n] = epilogue( sum_k A(row, k) W[n][k] ): R staged rows per CTA, one weight row per warp (8 per CTA).
 // Work item (bx, by) = (group of 8 weight rows, chunk of R input rows).
 struct RowsSmem {
@@ -86,18 +139,14 @@ struct RowsSmem {
     int slot[16], t[16], b[16];   // slot, row inside the step and batch row of every staged row
 };
 
-// CPW weight rows per warp: 1 at streaming batch sizes; 4 from 64 rows on, where an operation is many CTAs deep and every
-// CTA pays the same latency chain -- four rows per warp reuse the staged input rows (16 FMAs per shared-memory load instead of 4)
-// and cut the CTA count by four.  A column's arithmetic (lane-interleaved sums, shuffle tree) is the same for any CPW.
-template <int R, bool kPdl, int CPW>
+template <int R>
 __device__ __forceinline__ void rows_body(const RowOp& op, int bx, int by, RowsSmem& S) {
     constexpr int KC = kStageFloats / R;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int rows = op.batch * op.T;
     const int row0 = by * R;
-    const int n0 = (bx * kWarps + warp) * CPW;         // first of this warp's CPW weight rows
-    const bool n_ok = n0 < op.N;
-    const int n = n0;
+    const int n = bx * kWarps + warp;                  // this warp's weight row
+    const bool n_ok = n < op.N;
     if (tid < R) {   // (the slot table is constant during a step: read before the dependency wait)
         const int row = row0 + tid;
         int b = 0, t = 0, slot = -1;
@@ -107,13 +156,13 @@ __device__ __forceinline__ void rows_body(const RowOp& op, int bx, int by, RowsS
     // weights do not depend on the previous kernel / phase: the first four 16-byte pieces of this lane go straight into
     // registers (their latency overlaps the wait and the staging of the input rows) and the warp pulls its whole weight
     // row into L2
-    if (kPdl && n_ok && by == 0) {
+    if (n_ok && by == 0) {
         const char* wr = reinterpret_cast<const char*>(op.W + (long long)n * op.K);
-        const int lines = (min(CPW, op.N - n) * op.K * 4 + 127) >> 7;     // (the warp's rows are contiguous)
+        const int lines = (op.K * 4 + 127) >> 7;
         for (int l = lane; l < lines; l += 32) prefetch_l2(wr + ((long long)l << 7));
     }
-    constexpr int kPre = CPW == 1 ? 4 : 0;
-    float4 wpre[kPre > 0 ? kPre : 1];
+    constexpr int kPre = 4;
+    float4 wpre[kPre];
     {
         const int k0 = min(KC, op.K);
 #pragma unroll
@@ -124,12 +173,11 @@ __device__ __forceinline__ void rows_body(const RowOp& op, int bx, int by, RowsS
         }
     }
     __syncthreads();
-    if (kPdl) { pdl_wait(); pdl_go(); }
-    float acc[CPW][R];
+    pdl_wait();
+    pdl_go();
+    float acc[R];
 #pragma unroll
-    for (int c = 0; c < CPW; ++c)
-#pragma unroll
-        for (int r = 0; r < R; ++r) acc[c][r] = 0.f;
+    for (int r = 0; r < R; ++r) acc[r] = 0.f;
 
     for (int kc = 0; kc < op.K; kc += KC) {
         const int kcur = min(KC, op.K - kc);
@@ -145,7 +193,6 @@ __device__ __forceinline__ void rows_body(const RowOp& op, int bx, int by, RowsS
                 const int j = k / op.in_c, c = k - j * op.in_c;
                 const float* src = op.in + (long long)slot * op.in_stride + (long long)(op.in_hs + t + op.tap0 + j * op.tapstep) * op.in_c + c;
                 v = *reinterpret_cast<const float4*>(src);
-                if (op.pro == PRO_ELU) { v.x = elu1(v.x); v.y = elu1(v.y); v.z = elu1(v.z); v.w = elu1(v.w); }
             }
             *reinterpret_cast<float4*>(&S.As[r * KC + ((idx - r * q4) << 2)]) = v;
         }
@@ -179,91 +226,60 @@ __device__ __forceinline__ void rows_body(const RowOp& op, int bx, int by, RowsS
 #pragma unroll
                         for (int r = 0; r < R; ++r) {
                             const float4 a = *reinterpret_cast<const float4*>(&S.As[r * KC + k4]);
-                            acc[0][r] = fmaf(a.x, wpre[i].x, acc[0][r]); acc[0][r] = fmaf(a.y, wpre[i].y, acc[0][r]);
-                            acc[0][r] = fmaf(a.z, wpre[i].z, acc[0][r]); acc[0][r] = fmaf(a.w, wpre[i].w, acc[0][r]);
+                            acc[r] = fmaf(a.x, wpre[i].x, acc[r]); acc[r] = fmaf(a.y, wpre[i].y, acc[r]);
+                            acc[r] = fmaf(a.z, wpre[i].z, acc[r]); acc[r] = fmaf(a.w, wpre[i].w, acc[r]);
                         }
                         k4 += 128;
                     }
                 }
             }
-#pragma unroll(CPW == 1 ? 4 : 1)
+#pragma unroll 4
             for (; k4 < kcur; k4 += 128) {
-                float4 w[CPW];
-#pragma unroll
-                for (int c = 0; c < CPW; ++c)
-                    w[c] = (n + c < op.N) ? __ldg(reinterpret_cast<const float4*>(wrow + (long long)c * op.K + k4)) : make_float4(0.f, 0.f, 0.f, 0.f);
+                const float4 w = __ldg(reinterpret_cast<const float4*>(wrow + k4));
 #pragma unroll
                 for (int r = 0; r < R; ++r) {
                     const float4 a = *reinterpret_cast<const float4*>(&S.As[r * KC + k4]);
-#pragma unroll
-                    for (int c = 0; c < CPW; ++c) {
-                        acc[c][r] = fmaf(a.x, w[c].x, acc[c][r]); acc[c][r] = fmaf(a.y, w[c].y, acc[c][r]);
-                        acc[c][r] = fmaf(a.z, w[c].z, acc[c][r]); acc[c][r] = fmaf(a.w, w[c].w, acc[c][r]);
-                    }
+                    acc[r] = fmaf(a.x, w.x, acc[r]); acc[r] = fmaf(a.y, w.y, acc[r]);
+                    acc[r] = fmaf(a.z, w.z, acc[r]); acc[r] = fmaf(a.w, w.w, acc[r]);
                 }
             }
         }
         __syncthreads();
     }
     // ---- reduce over the lanes; lane r finishes row r ----
-#pragma unroll
-    for (int cc = 0; cc < CPW; ++cc) {
-    const int n = n0 + cc;
     float mine = 0.f;
 #pragma unroll
     for (int r = 0; r < R; ++r) {
-        const float v = warp_sum(acc[cc][r]);
+        const float v = warp_sum(acc[r]);
         if (lane == r) mine = v;
     }
     if (n < op.N && lane < R && S.slot[lane] >= 0) {
         const int b = S.b[lane], t = S.t[lane], slot = S.slot[lane];
         float y = mine + (op.bias ? op.bias[n % op.bias_mod] : 0.f);
-        if (op.epi == EPI_UPSAMPLE) {
-            // grouped transposed convolution, kernel 4, stride 2 (conv.py:271-282): outputs 2 t + j take tap j of this frame
-            // and, with `carry`, tap 2 + j of the previous one; decode_step upsamples every frame alone (carry = 0)
-            const float4 wu = *reinterpret_cast<const float4*>(op.wup + 4 * n);
-            float o0 = y * wu.x, o1 = y * wu.y;
-            if (op.carry) {
-                float* pp = op.up_prev + (long long)slot * op.N + n;
-                const float pv = *pp;
-                o0 = fmaf(pv, wu.z, o0); o1 = fmaf(pv, wu.w, o1);
-                *pp = y;
-            }
-            float* o = op.out + (long long)slot * op.out_stride + op.out_off0 + n;
-            o[0] = o0; o[op.N] = o1;
-        } else {
-            const long long e = (long long)op.out_off0 + (long long)t * op.N + n;
-            float* o = op.out + (long long)(op.out_by_row ? b : slot) * op.out_stride + e;
-            if (op.epi == EPI_GELU) y = gelu_erf(y);
-            else if (op.epi == EPI_SCALE_RES) y = op.res[(long long)slot * op.res_stride + op.res_off0 + (long long)t * op.N + n] + y * op.scale[n];
-            else if (op.epi == EPI_RES) y = op.res[(long long)slot * op.res_stride + op.res_off0 + (long long)t * op.N + n] + y;
-            *o = y;
-        }
+        store_row(op, b, slot, t, n, y);
     }
-    }
-    __syncthreads();   // S is reused by the next work item
 }
 
-template <int R, int CPW>
+template <int R>
 __global__ void __launch_bounds__(kThreads) rows_kernel(const RowOp op) {
     __shared__ __align__(16) RowsSmem S;
-    rows_body<R, true, CPW>(op, blockIdx.x, blockIdx.y, S);
+    rows_body<R>(op, blockIdx.x, blockIdx.y, S);
 }
 
-// The two-row Linears of up to 8 streams (the 32 transformer operations of a step): rows_kernel<R, 1>'s arithmetic -- the same
+// The two-row Linears of up to 8 streams (the 32 transformer operations of a step): rows_kernel<R>'s arithmetic -- the same
 // lane-interleaved sums, shuffle trees and LayerNorm loops, hence the same bits -- without its generality: a stream's two
 // input rows are one contiguous run, no im2col, prologue and epilogue fixed at compile time.  An operation at streaming batch
-// sizes is bound by the dependent instruction stream of its 8 warps (ncu: ~850 instructions per warp for rows_kernel<2, 1>),
+// sizes is bound by the dependent instruction stream of its 8 warps (ncu: ~850 instructions per warp for rows_kernel<2>),
 // not by bytes: fewer instructions per warp is what shortens it (one stream: 492 -> 462 us per step).
 template <int R, int PRO, int EPI>
 __global__ void __launch_bounds__(kThreads) lin_kernel(const RowOp op) {
     constexpr int KC = kStageFloats / R;                                // floats between staged rows (K <= KC, host)
     __shared__ __align__(16) float As[kStageFloats];
     __shared__ float s_mean[R], s_rstd[R];
-    __shared__ int s_slot[R / 2];
+    __shared__ int s_slot[R / 2];                                       // of every frame of every stream; its two rows are one run
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int K = op.K, n = blockIdx.x * kWarps + warp;                 // N is a multiple of 8 (host)
-    const int rows = 2 * op.batch;
+    const int pairs = op.batch * op.frames, rows = 2 * pairs;
     const float* wrow = op.W + (long long)n * K;
     float4 wpre[4];
 #pragma unroll
@@ -272,7 +288,7 @@ __global__ void __launch_bounds__(kThreads) lin_kernel(const RowOp op) {
         const char* wr = reinterpret_cast<const char*>(wrow);
         for (int l = lane; l < (K >> 5); l += 32) prefetch_l2(wr + ((long long)l << 7));
     }
-    if (tid < R / 2) s_slot[tid] = tid < op.batch ? (op.slots ? op.slots[tid] : tid) : -1;
+    if (tid < R / 2) s_slot[tid] = tid < pairs ? (op.slots ? op.slots[tid / op.frames] : tid / op.frames) : -1;
     __syncthreads();
     pdl_wait();
     pdl_go();
@@ -280,7 +296,7 @@ __global__ void __launch_bounds__(kThreads) lin_kernel(const RowOp op) {
 #pragma unroll
     for (int b = 0; b < R / 2; ++b) {                                   // a stream's two rows: 2 K contiguous floats
         const int slot = s_slot[b];
-        const float4* a4 = reinterpret_cast<const float4*>(op.in + (long long)(slot < 0 ? 0 : slot) * op.in_stride + (long long)op.in_hs * K);
+        const float4* a4 = reinterpret_cast<const float4*>(op.in + (long long)(slot < 0 ? 0 : slot) * op.in_stride + (long long)(op.in_hs + (slot < 0 ? 0 : 2 * (b % op.frames))) * K);
         for (int i = tid; i < 2 * q4; i += kThreads) {
             const int t = i >= q4 ? 1 : 0;
             *reinterpret_cast<float4*>(&As[(2 * b + t) * KC + ((i - t * q4) << 2)]) = slot < 0 ? make_float4(0.f, 0.f, 0.f, 0.f) : a4[i];
@@ -333,7 +349,7 @@ __global__ void __launch_bounds__(kThreads) lin_kernel(const RowOp op) {
         if (lane == r) mine = v;
     }
     if (lane < rows) {
-        const int slot = s_slot[lane >> 1], t = lane & 1;
+        const int slot = s_slot[lane >> 1], t = 2 * ((lane >> 1) % op.frames) + (lane & 1);
         float y = mine;
         const long long e = (long long)slot * op.out_stride + op.out_off0 + (long long)t * op.N + n;
         if (EPI == EPI_GELU) y = gelu_erf(y);
@@ -342,133 +358,115 @@ __global__ void __launch_bounds__(kThreads) lin_kernel(const RowOp op) {
     }
 }
 
-// The same product for MANY rows (12+ streams x the 16 .. 1920 rows of a SEANet stage): a 64 x 64 output tile per CTA, K in
-// steps of 16 through shared memory, 4 x 4 outputs per thread -- 16 FMAs per pair of 16-byte shared-memory loads instead of
-// the 4 of rows_kernel, whose one-weight-row-per-warp shape is built for a handful of rows.  Every output is one sequential
-// FMA chain over k = 0 .. K-1: deterministic and independent of what shares the launch, but a different order than
-// rows_kernel's lane-interleaved sums -- which kernel runs is decided by the BATCH SIZE alone (12+ streams), so a stream's bits
-// are the same in any batch of the same class (< 12 streams, 12+).  Prologues none | ELU | LayerNorm (row statistics in a pre-pass), epilogues bias |
-// residual | layer scale + residual | GELU: every operation of a step except the upsampler and the one-channel last convolution
-// (rowdot_kernel below).
-constexpr int kTM = 64, kTN = 64, kTK = 16, kTU = kTK / 16;   // kTU 16-byte pieces of A and of W per thread and K step
-// (K steps of 32: the many-row stages 15 .. 30 % slower -- fewer resident CTAs -- measured at 64 streams.)
-__global__ void __launch_bounds__(kThreads, 2) tile_kernel(const RowOp op) {
-    __shared__ __align__(16) float As[kTK][kTM + 4];
-    __shared__ __align__(16) float Ws[kTK][kTN + 4];
-    __shared__ int s_slot[kTM], s_t[kTM], s_b[kTM];
-    const int tid = threadIdx.x;
-    const int rows = op.batch * op.T;
-    const int row0 = blockIdx.y * kTM, n0 = blockIdx.x * kTN;
-    if (tid < kTM) {
-        const int row = row0 + tid;
+// The same product for MANY rows on packed-FMA tiles (f32_tile.cuh): every operation of a step from 12 streams on, and the SEANet stages
+// of 16 .. 1920 rows per stream for any number of streams, except the one-channel last convolution (rowdot_kernel below).  cp.async
+// gathers the rows (a causal convolution's im2col row is one contiguous run, a transposed convolution's two runs); ELUs were applied
+// where the rows were written, LayerNorm by norm_kernel in front.  K is shared by a cluster of CTAs where an operation has few tiles.
+// What an output is added up from -- which k a rank takes, its two chains, the order of ranks -- follows from the operation and the class
+// of the batch (fewer than 12 streams | 12+) alone, not from the tile's shape, so a stream's bits are the same in any batch of a class.
+// Bound by the FMAs and, with them in balance, shared-memory loads (f32_tile.cuh): 48 streams, 4 frames at once, 3.2 ms for 83 GFLOP (26
+// TFLOP/s; 64 x 64 plain-FMA tiles of 4 x 4 outputs and a warp per weight row before: 1.75 ms per single frame).  128 x 128 tiles of
+// 256 threads, ELU and LayerNorm applied by every block that reads the rows: 5.9 ms.
+template <int BM, int BN, int TM, int TN>
+__global__ void __launch_bounds__(f32t::Tile<BM, BN, TM, TN>::NT) tile_kernel(const RowOp op) {
+    using T = f32t::Tile<BM, BN, TM, TN>;
+    extern __shared__ __align__(16) float tile_sm[];
+    __shared__ int s_slot[BM], s_t[BM], s_b[BM];
+    const int tid = threadIdx.x, rows = op.batch * op.T;
+    const int row0 = blockIdx.y * BM, n0 = (int)(blockIdx.x / f32t::cluster_size()) * BN;
+    for (int i = tid; i < BM; i += T::NT) {   // (the slot table is constant during a step: read before the dependency wait)
+        const int row = row0 + i;
         int b = 0, t = 0, slot = -1;
         if (row < rows) { b = row / op.T; t = row - b * op.T; slot = op.slots ? op.slots[b] : b; }
-        s_slot[tid] = slot; s_t[tid] = t; s_b[tid] = b;
+        s_slot[i] = slot; s_t[i] = t; s_b[i] = b;
     }
     __syncthreads();
+    const int turn = op.tapstep < 0 ? op.in_c : op.K;      // transposed convolution: from here on the previous row's channels
+    int k_lo, k_hi;
+    T::range(op.K, k_lo, k_hi);
+    float out[TM][TN];
+    T::template product<false>(tile_sm, k_lo, k_hi,
+                               [&](int r) -> const float* {
+                                   return s_slot[r] < 0 ? nullptr : op.in + (long long)s_slot[r] * op.in_stride + (long long)(op.in_hs + s_t[r] + op.tap0) * op.in_c;
+                               },
+                               [&](int k) -> long long { return k >= turn ? k - 2 * op.in_c : k; },
+                               [&](int r) { return n0 + r < op.N ? op.W + (long long)(n0 + r) * op.K : nullptr; }, [](float4 v, int, int) { return v; },
+                               [] { pdl_wait(); pdl_go(); }, out);
+    T::finish(tile_sm, out, [&](int r, int c, float4 y) {
+        const int n = n0 + c;
+        if (s_slot[r] >= 0 && n < op.N) store_row4(op, s_b[r], s_slot[r], s_t[r], n, y);      // (N is a multiple of 4)
+    });
+}
+
+// LayerNorm of the rows a product on the tiles reads: one warp per row, the row in registers between its two passes.  (Every block of the
+// product taking the statistics of its 64 rows itself cost 90 us of a 105 us product.)
+constexpr int kNormRegs = 16;                              // floats per lane: rows of up to 512 (host)
+__global__ void __launch_bounds__(128) norm_kernel(const RowOp op) {
     pdl_wait();
     pdl_go();
-    const int lm = tid >> 2, lk = (tid & 3) << 2;      // this thread's row (of A and of W) and k offset of the 16-byte pieces it loads
-    const int a_slot = s_slot[lm];
-    const float* a_base = op.in + (long long)(a_slot < 0 ? 0 : a_slot) * op.in_stride + (long long)(op.in_hs + s_t[lm] + op.tap0) * op.in_c;
-    const bool w_ok = n0 + lm < op.N;
-    const float* w_base = op.W + (long long)(n0 + lm) * op.K;
-    auto load_a = [&](int k) -> float4 {
-        float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (a_slot >= 0) {
-            const int j = k / op.in_c, c = k - j * op.in_c;
-            v = *reinterpret_cast<const float4*>(a_base + (long long)j * op.tapstep * op.in_c + c);
-            if (op.pro == PRO_ELU) { v.x = elu1(v.x); v.y = elu1(v.y); v.z = elu1(v.z); v.w = elu1(v.w); }
-        }
-        return v;
-    };
-    auto load_w = [&](int k) -> float4 {
-        return w_ok ? __ldg(reinterpret_cast<const float4*>(w_base + k)) : make_float4(0.f, 0.f, 0.f, 0.f);
-    };
-    const int ty = tid >> 4, tx = tid & 15;
-    float acc[4][4];
+    const int row = blockIdx.x * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+    if (row >= op.batch * op.T) return;
+    const int b = row / op.T, t = row - b * op.T, slot = op.slots ? op.slots[b] : b;
+    const float* a = op.in + (long long)slot * op.in_stride + (long long)(op.in_hs + t) * op.K;
+    float v[kNormRegs], s = 0.f, d2 = 0.f;
 #pragma unroll
-    for (int i = 0; i < 4; ++i)
+    for (int i = 0; i < kNormRegs; ++i) { v[i] = lane + 32 * i < op.K ? a[lane + 32 * i] : 0.f; s += v[i]; }
+    const float mean = warp_sum(s) / (float)op.K;
 #pragma unroll
-        for (int j = 0; j < 4; ++j) acc[i][j] = 0.f;
-    float4 ra[kTU], rw[kTU];
+    for (int i = 0; i < kNormRegs; ++i) { const float d = lane + 32 * i < op.K ? v[i] - mean : 0.f; d2 = fmaf(d, d, d2); }
+    const float rstd = 1.0f / sqrtf(warp_sum(d2) / (float)op.K + op.eps);
+    float* o = op.out + (long long)slot * op.out_stride + op.out_off0 + (long long)t * op.K;
 #pragma unroll
-    for (int u = 0; u < kTU; ++u) { ra[u] = load_a(lk + 16 * u); rw[u] = load_w(lk + 16 * u); }
-    for (int k0 = 0; k0 < op.K; k0 += kTK) {
-#pragma unroll
-        for (int u = 0; u < kTU; ++u) {
-            const int kk = lk + 16 * u;
-            As[kk + 0][lm] = ra[u].x; As[kk + 1][lm] = ra[u].y; As[kk + 2][lm] = ra[u].z; As[kk + 3][lm] = ra[u].w;
-            Ws[kk + 0][lm] = rw[u].x; Ws[kk + 1][lm] = rw[u].y; Ws[kk + 2][lm] = rw[u].z; Ws[kk + 3][lm] = rw[u].w;
-        }
-        __syncthreads();
-        if (k0 + kTK < op.K) {   // next step's pieces in flight during the FMAs
-#pragma unroll
-            for (int u = 0; u < kTU; ++u) { ra[u] = load_a(k0 + kTK + lk + 16 * u); rw[u] = load_w(k0 + kTK + lk + 16 * u); }
-        }
-#pragma unroll
-        for (int k = 0; k < kTK; ++k) {
-            const float4 a = *reinterpret_cast<const float4*>(&As[k][ty * 4]);
-            const float4 w = *reinterpret_cast<const float4*>(&Ws[k][tx * 4]);
-            acc[0][0] = fmaf(a.x, w.x, acc[0][0]); acc[0][1] = fmaf(a.x, w.y, acc[0][1]); acc[0][2] = fmaf(a.x, w.z, acc[0][2]); acc[0][3] = fmaf(a.x, w.w, acc[0][3]);
-            acc[1][0] = fmaf(a.y, w.x, acc[1][0]); acc[1][1] = fmaf(a.y, w.y, acc[1][1]); acc[1][2] = fmaf(a.y, w.z, acc[1][2]); acc[1][3] = fmaf(a.y, w.w, acc[1][3]);
-            acc[2][0] = fmaf(a.z, w.x, acc[2][0]); acc[2][1] = fmaf(a.z, w.y, acc[2][1]); acc[2][2] = fmaf(a.z, w.z, acc[2][2]); acc[2][3] = fmaf(a.z, w.w, acc[2][3]);
-            acc[3][0] = fmaf(a.w, w.x, acc[3][0]); acc[3][1] = fmaf(a.w, w.y, acc[3][1]); acc[3][2] = fmaf(a.w, w.z, acc[3][2]); acc[3][3] = fmaf(a.w, w.w, acc[3][3]);
-        }
-        __syncthreads();
-    }
-    const int n = n0 + tx * 4;
-    if (n >= op.N) return;                      // (N is a multiple of 4: the four columns of a thread are all in or all out)
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        const int m = ty * 4 + i;
-        const int slot = s_slot[m];
-        if (slot < 0) continue;
-        const long long e = (long long)op.out_off0 + (long long)s_t[m] * op.N + n;
-        float4 y = make_float4(acc[i][0], acc[i][1], acc[i][2], acc[i][3]);
-        if (op.bias) {
-            y.x += op.bias[n % op.bias_mod]; y.y += op.bias[(n + 1) % op.bias_mod];
-            y.z += op.bias[(n + 2) % op.bias_mod]; y.w += op.bias[(n + 3) % op.bias_mod];
-        }
-        if (op.epi == EPI_RES) {
-            const float4 r = *reinterpret_cast<const float4*>(op.res + (long long)slot * op.res_stride + op.res_off0 + (long long)s_t[m] * op.N + n);
-            y.x = r.x + y.x; y.y = r.y + y.y; y.z = r.z + y.z; y.w = r.w + y.w;
-        }
-        *reinterpret_cast<float4*>(op.out + (long long)(op.out_by_row ? s_b[m] : slot) * op.out_stride + e) = y;
+    for (int i = 0; i < kNormRegs; ++i) {
+        const int k = lane + 32 * i;
+        if (k < op.K) o[k] = (v[i] - mean) * rstd * op.ln_w[k] + op.ln_b[k];
     }
 }
 
-// The last convolution (one output channel) for many rows: one thread per output sample, the weight vector in shared memory.
+// The last convolution (one output channel): a block brings the inputs of kDotRows neighbouring samples of one stream into shared memory
+// and four lanes share a sample's products.  (A thread per sample straight from global memory took 34 us for 48 streams: neighbouring
+// threads read runs 256 bytes apart, every input three times.  Here 17 us.)
+constexpr int kDotRows = 64;
+// floats between the staged rows: 4 of 8 16-byte bank groups apart, so that eight lanes -- two samples' four pieces -- never meet
+__host__ __device__ constexpr int dot_ld(int in_c) { return in_c + ((in_c / 4) % 8 <= 4 ? 4 - (in_c / 4) % 8 : 12 - (in_c / 4) % 8) * 4; }
 __global__ void __launch_bounds__(kThreads) rowdot_kernel(const RowOp op) {
-    __shared__ __align__(16) float w[1024];
-    const int tid = threadIdx.x;
+    extern __shared__ __align__(16) float dot_sm[];
+    const int tid = threadIdx.x, taps = op.K / op.in_c, t0 = blockIdx.x * kDotRows, n = min(kDotRows, op.T - t0), ld = dot_ld(op.in_c);
+    float *w = dot_sm, *a = dot_sm + op.K;
     for (int k = tid; k < op.K; k += kThreads) w[k] = op.W[k];
-    __syncthreads();
+    const int b = blockIdx.y, slot = op.slots ? op.slots[b] : b, c4 = op.in_c / 4;
     pdl_wait();
     pdl_go();
-    const int row = blockIdx.x * kThreads + tid;
-    if (row >= op.batch * op.T) return;
-    const int b = row / op.T, t = row - b * op.T;
-    const int slot = op.slots ? op.slots[b] : b;
-    const float* a = op.in + (long long)slot * op.in_stride + (long long)(op.in_hs + t + op.tap0) * op.in_c;   // contiguous im2col run
-    float acc = 0.f;
-    for (int k = 0; k < op.K; k += 4) {
-        float4 v = *reinterpret_cast<const float4*>(a + k);
-        if (op.pro == PRO_ELU) { v.x = elu1(v.x); v.y = elu1(v.y); v.z = elu1(v.z); v.w = elu1(v.w); }
-        const float4 ww = *reinterpret_cast<const float4*>(&w[k]);
-        acc = fmaf(v.x, ww.x, acc); acc = fmaf(v.y, ww.y, acc); acc = fmaf(v.z, ww.z, acc); acc = fmaf(v.w, ww.w, acc);
+    const float* src = op.in + (long long)slot * op.in_stride + (long long)(op.in_hs + t0 + op.tap0) * op.in_c;
+    for (int i = tid; i < (n + taps - 1) * c4; i += kThreads) {
+        const int r = i / c4, c = (i - r * c4) * 4;
+        *reinterpret_cast<float4*>(a + r * ld + c) = *reinterpret_cast<const float4*>(src + (long long)r * op.in_c + c);
     }
-    op.out[(long long)(op.out_by_row ? b : slot) * op.out_stride + op.out_off0 + t] = acc + (op.bias ? op.bias[0] : 0.f);
+    __syncthreads();
+    const int t = tid >> 2, q = tid & 3;
+    float acc = 0.f;
+    if (t < n)
+        for (int j = 0; j < taps; ++j)
+            for (int c = q * 4; c < op.in_c; c += 16) {
+                const float4 v = *reinterpret_cast<const float4*>(a + (t + j) * ld + c), ww = *reinterpret_cast<const float4*>(w + j * op.in_c + c);
+                acc = fmaf(v.x, ww.x, acc); acc = fmaf(v.y, ww.y, acc); acc = fmaf(v.z, ww.z, acc); acc = fmaf(v.w, ww.w, acc);
+            }
+    acc += __shfl_xor_sync(0xffffffffu, acc, 1);
+    acc += __shfl_xor_sync(0xffffffffu, acc, 2);
+    if (q == 0 && t < n) op.out[(long long)(op.out_by_row ? b : slot) * op.out_stride + op.out_off0 + t0 + t] = acc + (op.bias ? op.bias[0] : 0.f);
 }
+static_assert(kThreads == 4 * kDotRows, "four lanes per sample");
 
 // RVQ decode (rvq.py:118-130, 171-186): the semantic codebook's row | the sum of the acoustic codebooks' rows, in order.
 struct EmbedArgs {
     const float* books;   // [n_q][codebook_size][cdim], rows already divided by max(cluster_usage, eps)
     const int32_t* codes; const int32_t* slots; float* q; long long q_stride;
-    int n_q, cb_size, cdim, batch;
+    int n_q, cb_size, cdim, batch, frames;
 };
+// b: frame b % frames of batch row b / frames
 __device__ __forceinline__ void embed_body(const EmbedArgs& a, int b) {
-    const int slot = a.slots ? a.slots[b] : b;
+    const int row = b / a.frames, slot = a.slots ? a.slots[row] : row;
+    float* q = a.q + (long long)slot * a.q_stride + (b - row * a.frames) * 2 * a.cdim;
     for (int k = threadIdx.x; k < 2 * a.cdim; k += blockDim.x) {
         float v;
         if (k < a.cdim) {
@@ -482,7 +480,7 @@ __device__ __forceinline__ void embed_body(const EmbedArgs& a, int b) {
                 v = i == 1 ? e : v + e;
             }
         }
-        a.q[(long long)slot * a.q_stride + k] = v;
+        q[k] = v;
     }
 }
 __global__ void embed_kernel(const EmbedArgs a) {
@@ -505,13 +503,38 @@ struct AttnArgs {
     const float* rope; const int32_t* pos; const int32_t* slots; int32_t* err;
     float* part; unsigned int* arrive;           // [slot][head][split][2][hd + 2], [slot][head]
     int layer, dim, hd, max_pos, window, batch, heads, max_splits;
+    int frames, max_frames;                      // frames of the call; of more than one the keys and values are in the cache already
 };
-__device__ __forceinline__ void attn_body(const AttnArgs& a, int b, int h, int sp, float* sm) {
+// Keys (rotated) and values of a call of several frames -> the cache: a block per (stream, frame, head), the attention of all frames then
+// runs side by side.
+__global__ void __launch_bounds__(64) append_kernel(const AttnArgs a) {
+    pdl_wait();
+    pdl_go();
+    const int b = blockIdx.x / a.frames, f = blockIdx.x - b * a.frames, h = blockIdx.y;
+    const int slot = a.slots ? a.slots[b] : b, hd = a.hd, half = hd >> 1, p0 = 2 * (a.pos[slot] + f);
+    if (p0 + 2 > a.max_pos) { if (threadIdx.x == 0) *a.err = 1; return; }
+    float* kc = a.kv + (long long)slot * a.kv_slot_stride + (long long)a.layer * a.kv_layer_stride;
+    float* vc = kc + (long long)a.max_pos * a.dim;
+    for (int i = threadIdx.x; i < 2 * half; i += blockDim.x) {
+        const int t = i / half, j = i - t * half;
+        const float* row = a.qkv + (long long)slot * a.qkv_stride + (long long)(2 * f + t) * 3 * a.dim + h * hd;
+        const float cs = a.rope[(long long)(p0 + t) * hd + j], sn = a.rope[(long long)(p0 + t) * hd + half + j];
+        const float k1 = row[a.dim + j], k2 = row[a.dim + j + half];
+        const long long at = (long long)(p0 + t) * a.dim + h * hd;
+        kc[at + j] = k1 * cs - k2 * sn;
+        kc[at + j + half] = k2 * cs + k1 * sn;
+        vc[at + j] = row[2 * a.dim + j];
+        vc[at + j + half] = row[2 * a.dim + j + half];
+    }
+}
+
+// x: frame x % frames of batch row x / frames
+__device__ __forceinline__ void attn_body(const AttnArgs& a, int x, int h, int sp, float* sm) {
     __shared__ int s_last;
     const int tid = threadIdx.x;
-    const int slot = a.slots ? a.slots[b] : b;
+    const int b = x / a.frames, f = x - b * a.frames, slot = a.slots ? a.slots[b] : b;
     const int hd = a.hd, half = hd >> 1;
-    const int p0 = 2 * a.pos[slot];
+    const int p0 = 2 * (a.pos[slot] + f);
     if (p0 + 2 > a.max_pos) { if (tid == 0 && sp == 0) *a.err = 1; return; }   // (uniform over the CTA)
     const int L = p0 + 2;
     // visible positions: query t sees lo_t .. p0 + t
@@ -526,9 +549,9 @@ __device__ __forceinline__ void attn_body(const AttnArgs& a, int b, int h, int s
     float* S = red + 2 * kThreads;   // [2][kAttnChunk]
     float* kc = a.kv + (long long)slot * a.kv_slot_stride + (long long)a.layer * a.kv_layer_stride;
     float* vc = kc + (long long)a.max_pos * a.dim;
-    const float* src = a.qkv + (long long)slot * a.qkv_stride;
+    const float* src = a.qkv + (long long)slot * a.qkv_stride + (long long)(2 * f) * 3 * a.dim;
     const float scale = rsqrtf((float)hd);
-    const bool newest = sp == s_end - 1;          // the split that holds the step's own two positions appends them
+    const bool newest = a.frames == 1 && sp == s_end - 1;          // the split that holds the step's own two positions appends them
     for (int i = tid; i < 2 * half; i += kThreads) {   // (position t, pair i)
         const int t = i / half, j = i - t * half;
         const float* row = src + (long long)t * 3 * a.dim + h * hd;
@@ -596,8 +619,9 @@ __device__ __forceinline__ void attn_body(const AttnArgs& a, int b, int h, int s
     }
     red[tid] = o0; red[kThreads + tid] = o1;
     __syncthreads();
-    float* dst = a.att + (long long)slot * a.att_stride + h * hd;
-    float* mypart = a.part + (((long long)slot * a.heads + h) * a.max_splits) * (2 * (hd + 2));
+    float* dst = a.att + (long long)slot * a.att_stride + (long long)(2 * f) * a.dim + h * hd;
+    const long long unit = ((long long)slot * a.max_frames + f) * a.heads + h;
+    float* mypart = a.part + unit * a.max_splits * (2 * (hd + 2));
     if (tid < hd) {
         float s0 = 0.f, s1 = 0.f;
         for (int gg = 0; gg < G; ++gg) { s0 += red[gg * hd + tid]; s1 += red[kThreads + gg * hd + tid]; }
@@ -614,9 +638,9 @@ __device__ __forceinline__ void attn_body(const AttnArgs& a, int b, int h, int s
         __threadfence();
         __syncthreads();
         if (tid == 0) {
-            const unsigned int old = atomicAdd(a.arrive + (long long)slot * a.heads + h, 1u);
+            const unsigned int old = atomicAdd(a.arrive + unit, 1u);
             s_last = old == (unsigned int)(n_part - 1);
-            if (s_last) a.arrive[(long long)slot * a.heads + h] = 0u;
+            if (s_last) a.arrive[unit] = 0u;
         }
         __syncthreads();
         if (s_last) {
@@ -651,7 +675,7 @@ struct BufDesc { int off, hs, T, C; };
 struct ShiftArgs {
     float* arena; long long stride; const int32_t* slots; int32_t* pos; float* up_prev; int dim;
     int n_bufs; int reset;   // reset = 1: zero the history rows, the upsampler's carry and the position instead
-    int batch, pad;
+    int batch, frames;
     BufDesc bufs[kMaxBufs];
 };
 __device__ __forceinline__ void shift_body(const ShiftArgs& a, int b, int i, float* tmp /* 4096 floats */) {
@@ -661,14 +685,14 @@ __device__ __forceinline__ void shift_body(const ShiftArgs& a, int b, int i, flo
         if (a.reset) {
             for (int k = tid; k < a.dim; k += kThreads) a.up_prev[(long long)slot * a.dim + k] = 0.f;
             if (tid == 0) a.pos[slot] = 0;
-        } else if (tid == 0) a.pos[slot] += 1;
+        } else if (tid == 0) a.pos[slot] += a.frames;
         return;
     }
     const BufDesc d = a.bufs[i];
     float* base = a.arena + (long long)slot * a.stride + d.off;
     const int n = d.hs * d.C;
     if (a.reset) { for (int k = tid; k < n; k += kThreads) base[k] = 0.f; return; }
-    const float* src = base + (long long)d.T * d.C;   // rows T .. T + hs
+    const float* src = base + (long long)a.frames * d.T * d.C;   // the call's last hs rows
     for (int k0 = 0; k0 < n; k0 += 4096) {   // (source and destination overlap when T < hs: staged through shared memory)
         const int m = min(4096, n - k0);
         for (int k = tid; k < m; k += kThreads) tmp[k] = src[k0 + k];
@@ -690,7 +714,7 @@ __global__ void __launch_bounds__(kThreads) shift_kernel(const ShiftArgs a) {
 //  barrier.  Bit-identical, but 760 us per step against 500 us for the graph at one stream, 1.79 vs 1.37 ms at 8, and worse
 //  on 148 or 74 CTAs (1 102 / 1 509 us): an operation is a chain of dependent instructions and L2 round trips inside a
 //  CTA, which a barrier does not shorten, while the graph's kernel boundaries cost less than a 296-CTA barrier.)
-enum { OP_ROWS = 0, OP_ATTN = 1, OP_EMBED = 2, OP_SHIFT = 3 };
+enum { OP_ROWS = 0, OP_ATTN = 1, OP_EMBED = 2, OP_SHIFT = 3, OP_APPEND = 4 };
 struct OpRec {
     int kind, R;
     union { RowOp row; AttnArgs attn; EmbedArgs emb; ShiftArgs shift; };
@@ -740,8 +764,8 @@ struct SmolMimi {
     int ch0 = 0;                       // channels after conv_in
     // per-slot arena
     std::vector<MimiBuf> bufs;
-    int bX0 = 0, bQ = 0, bQKV = 0, bATT = 0, bFF = 0, bA0 = 0;
-    int bCT[SMOL_MIMI_MAX_RATIOS], bH[SMOL_MIMI_MAX_RATIOS], bR[SMOL_MIMI_MAX_RATIOS];
+    int bX0 = 0, bLN = 0, bQ = 0, bQKV = 0, bATT = 0, bFF = 0, bA0 = 0;
+    int bCT[SMOL_MIMI_MAX_RATIOS], bCE[SMOL_MIMI_MAX_RATIOS], bH[SMOL_MIMI_MAX_RATIOS], bR[SMOL_MIMI_MAX_RATIOS];
     size_t arena_floats = 0;
     // workspace layout (bytes)
     size_t o_books = 0, o_wcat = 0, o_up = 0, o_rope = 0, o_small = 0, o_conv_in = 0, o_conv_out = 0;
@@ -753,10 +777,11 @@ struct SmolMimi {
     int launches = 0;
     size_t attn_smem = 0, o_part = 0, o_arrive = 0;
     int max_splits = 1;
+    int max_frames = 1;                // frames one call may bring (rows of the arenas)
     // cached graph of one step
     cudaStream_t cap_stream = nullptr;
     // captured steps, keyed by (batch, buffers): a serving loop alternates between a few batch sizes
-    struct Step { const void* codes; const void* slots; const void* pcm; int batch; std::vector<OpRec> prog; cudaGraphExec_t graph; uint64_t used; };
+    struct Step { const void* codes; const void* slots; const void* pcm; int batch, frames; std::vector<OpRec> prog; cudaGraphExec_t graph; uint64_t used; };
     std::vector<Step> steps;
     uint64_t tick = 0;
     void drop_steps() { for (Step& s : steps) if (s.graph) cudaGraphExecDestroy(s.graph); steps.clear(); }
@@ -769,18 +794,20 @@ static int mimi_plan(SmolMimi* m) {
     const SmolMimiConfig& c = m->cfg;
     m->bufs.clear();
     size_t off = 0;
-    auto add = [&](int hs, int T, int C) { m->bufs.push_back({off, hs, T, C}); off += (size_t)(hs + T) * C; off = (off + 3) / 4 * 4; return (int)m->bufs.size() - 1; };
+    auto add = [&](int hs, int T, int C) { m->bufs.push_back({off, hs, T, C}); off += ((size_t)hs + (size_t)T * m->max_frames) * C; off = (off + 3) / 4 * 4; return (int)m->bufs.size() - 1; };
     m->ch0 = c.n_filters << c.n_ratios;
     m->bX0 = add(c.kernel - 1, 2, c.dim);
     m->bQ = add(0, 1, 2 * c.codebook_dim);
     m->bQKV = add(0, 2, 3 * c.dim);
     m->bATT = add(0, 2, c.dim);
+    m->bLN = add(0, 2, c.dim);
     m->bFF = add(0, 2, c.ffn);
     m->bA0 = add(1, 2, m->ch0);
     int T = 2, ch = m->ch0;
     for (int i = 0; i < c.n_ratios; ++i) {
         T *= c.ratios[i]; ch /= 2;
-        m->bCT[i] = add(c.res_kernel - 1, T, ch);
+        m->bCT[i] = add(0, T, ch);
+        m->bCE[i] = add(c.res_kernel - 1, T, ch);
         m->bH[i] = add(0, T, ch / 2);
         m->bR[i] = add(i + 1 < c.n_ratios ? 1 : c.last_kernel - 1, T, ch);
     }
@@ -817,8 +844,8 @@ static int mimi_plan(SmolMimi* m) {
     m->o_upprev = take((size_t)c.max_streams * c.dim);
     m->o_err = take(4);
     m->max_splits = (c.max_positions + kAttnChunk - 1) / kAttnChunk;
-    m->o_part = take((size_t)c.max_streams * c.n_heads * m->max_splits * 2 * (c.head_dim + 2));
-    m->o_arrive = take((size_t)c.max_streams * c.n_heads);
+    m->o_part = take((size_t)c.max_streams * m->max_frames * c.n_heads * m->max_splits * 2 * (c.head_dim + 2));
+    m->o_arrive = take((size_t)c.max_streams * m->max_frames * c.n_heads);
     m->total = o;
     m->attn_smem = (size_t)(2 * c.head_dim + 2 * kThreads + 2 * kAttnChunk) * 4;
     m->max_splits = (c.max_positions + kAttnChunk - 1) / kAttnChunk;
@@ -852,6 +879,13 @@ extern "C" void smol_mimi_destroy(SmolMimi* m) {
     if (m->cap_stream) cudaStreamDestroy(m->cap_stream);
     delete m;
 }
+extern "C" int smol_mimi_set_max_frames(SmolMimi* m, int32_t frames) {
+    if (!m || frames < 1 || frames > 8) return smol::capi_fail(SMOL_ERR_INVALID, "smol_mimi_set_max_frames: frames must be 1 .. 8");
+    if (m->bound) return smol::capi_fail(SMOL_ERR_INVALID, "smol_mimi_set_max_frames: call it before smol_mimi_workspace_bytes() and smol_mimi_bind()");
+    m->max_frames = m->cfg.upsample_carry ? 1 : frames;      // the carried upsampler goes frame by frame
+    mimi_plan(m);
+    return SMOL_OK;
+}
 extern "C" int32_t smol_mimi_samples_per_frame(const SmolMimi* m) { return m ? m->spf : 0; }
 extern "C" size_t smol_mimi_workspace_bytes(const SmolMimi* m) { return m ? m->total : 0; }
 extern "C" int32_t smol_mimi_launches_per_step(const SmolMimi* m) { return m ? m->launches : 0; }
@@ -865,7 +899,7 @@ static ShiftArgs shift_args(SmolMimi* m, const int32_t* slots, int reset) {
     ShiftArgs a{};
     a.arena = wsf(m, m->o_arena); a.stride = (long long)m->arena_floats; a.slots = slots;
     a.pos = reinterpret_cast<int32_t*>(m->ws + m->o_pos); a.up_prev = wsf(m, m->o_upprev); a.dim = m->cfg.dim;
-    a.n_bufs = 0; a.reset = reset;
+    a.n_bufs = 0; a.reset = reset; a.frames = 1;
     for (const MimiBuf& b : m->bufs) if (b.hs > 0) a.bufs[a.n_bufs++] = BufDesc{(int)b.off, b.hs, b.T, b.C};
     return a;
 }
@@ -939,7 +973,7 @@ extern "C" int smol_mimi_bind(SmolMimi* m, const SmolMimiWeights* w, void* d_wor
     MCU(d2d(bo, w->conv_out.bias, 1));
     MCU(cudaGetLastError());
     MCU(cudaMemsetAsync(m->ws + m->o_err, 0, 16, st));
-    MCU(cudaMemsetAsync(m->ws + m->o_arrive, 0, (size_t)c.max_streams * c.n_heads * 4, st));
+    MCU(cudaMemsetAsync(m->ws + m->o_arrive, 0, (size_t)c.max_streams * m->max_frames * c.n_heads * 4, st));
     if (m->attn_smem > 48 * 1024) MCU(cudaFuncSetAttribute(attn_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)m->attn_smem));
     m->bound = true;
     return smol_mimi_reset(m, nullptr, c.max_streams, stream);
@@ -963,23 +997,59 @@ static cudaError_t launch_pdl(void (*kern)(const Args), dim3 grid, dim3 block, s
 
 static int rows_R(int rows) { return rows <= 2 ? 2 : rows <= 4 ? 4 : rows <= 8 ? 8 : 16; }
 
-// 12+ streams: the many-row stages go through the tile kernel (decided by the batch size alone, see tile_kernel)
-constexpr int kTileMinBatch = 12;   // measured: 8 streams 1.13 ms per step on rows_kernel vs 1.23 on the tiles; 12 streams 1.35 vs 1.30
+constexpr int kTileMinBatch = 12;   // the class of 12+ streams
+static int rows_per_frame(const RowOp& op) { return op.T / op.frames; }
+// Operations on the packed-FMA tiles: see tile_kernel.  (Fewer than 12 streams: an operation of two rows per frame streams its weights
+// through rows_kernel / lin_kernel, which read them once for up to 16 rows.)
 static bool use_tile(const RowOp& op) {
-    static const int min_batch = [] { const char* e = getenv("SMOL_MIMI_TILE_MIN_BATCH"); return e ? atoi(e) : kTileMinBatch; }();
-    return op.batch >= min_batch && op.T >= 16 && op.N >= 16 && op.N % 4 == 0 && op.K % kTK == 0 &&
-           (op.pro == PRO_NONE || op.pro == PRO_ELU) && (op.epi == EPI_BIAS || op.epi == EPI_RES);
+    return (op.batch >= kTileMinBatch || rows_per_frame(op) >= 16) && op.N >= 16 && op.N % 4 == 0 && op.bias_mod % (op.bias ? 4 : 1) == 0 && op.K % 4 == 0 && op.in_c % 4 == 0 &&
+           (op.tapstep > 0 || op.K == 2 * op.in_c) && (op.pro == PRO_NONE || (op.norm_at && op.K <= 32 * kNormRegs));
 }
+template <int BM, int BN, int TM, int TN>
+static cudaError_t launch_tile(const RowOp& op, int split, cudaStream_t st) {
+    using T = smol::f32t::Tile<BM, BN, TM, TN>;
+    if (T::kSmemBytes > 48 * 1024)
+        if (const cudaError_t e = cudaFuncSetAttribute(tile_kernel<BM, BN, TM, TN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)T::kSmemBytes)) return e;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3((op.N + BN - 1) / BN * split, (op.batch * op.T + BM - 1) / BM);
+    cfg.blockDim = dim3(T::NT);
+    cfg.dynamicSmemBytes = T::kSmemBytes;
+    cfg.stream = st;
+    cudaLaunchAttribute at[2];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = split; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
+    at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = g_pdl ? 2 : 1;
+    return cudaLaunchKernelEx(&cfg, tile_kernel<BM, BN, TM, TN>, op);
+}
+static cudaError_t launch_tiles(const RowOp& op, cudaStream_t st) {
+    const int rows = op.batch * op.T;
+    // CTAs per tile: from the operation and the fewest rows of its class, so that a stream's sums do not depend on the batch
+    const int least = rows_per_frame(op) * (op.batch >= kTileMinBatch ? kTileMinBatch : 1);
+    const long long least_tiles = (long long)((least + 31) / 32) * ((op.N + 63) / 64);
+    int split = 1;
+    while (split < 8 && least_tiles * split < 148 && op.K / (2 * split) >= 128) split *= 2;
+    // the tile: the largest that still gives every SM two CTAs (four of a 64 x 64 tile's two warps run side by side on an SM)
+    auto ctas = [&](int bm, int bn) { return (long long)((rows + bm - 1) / bm) * ((op.N + bn - 1) / bn) * split; };
+    if (op.N > 32 && rows >= 64 && ctas(64, 64) >= 2 * 148) return launch_tile<64, 64, 8, 8>(op, split, st);
+    if (op.N <= 32 && rows >= 64 && ctas(64, 32) >= 2 * 148) return launch_tile<64, 32, 8, 4>(op, split, st);
+    if (rows > 16 && op.N > 32 && ctas(32, 64) >= 2 * 148) return launch_tile<32, 64, 8, 8>(op, split, st);
+    if (rows > 16) return launch_tile<32, 32, 4, 4>(op, split, st);
+    return launch_tile<16, 32, 4, 4>(op, split, st);
+}
+static size_t rowdot_smem(const RowOp& op) { return ((size_t)op.K + (size_t)(kDotRows + op.K / op.in_c - 1) * dot_ld(op.in_c)) * 4; }
 static bool use_rowdot(const RowOp& op) {
-    static const int min_batch = [] { const char* e = getenv("SMOL_MIMI_TILE_MIN_BATCH"); return e ? atoi(e) : kTileMinBatch; }();
-    return op.batch >= min_batch && op.N == 1 && op.K <= 1024 && op.K % 4 == 0 && op.tapstep > 0 && op.epi == EPI_BIAS && op.pro != PRO_LN;
+    return (op.batch >= kTileMinBatch || rows_per_frame(op) >= 16) && op.N == 1 && op.in_c % 4 == 0 && op.K % op.in_c == 0 && op.tapstep > 0 &&
+           op.epi == EPI_BIAS && op.pro != PRO_LN && !op.elu && !op.raw && rowdot_smem(op) <= 48 * 1024;
 }
 
-// the two-row Linears of up to 8 streams: the lean form of rows_kernel<R, 1> (same bits)
+// the two-row Linears of up to 8 streams: the lean form of rows_kernel<R> (same bits)
 static bool use_lin(const RowOp& op) {
     static const bool off = [] { const char* e = getenv("SMOL_MIMI_LIN2"); return e && e[0] == '0'; }();
     const int R = rows_R(op.batch * op.T);
-    return !off && op.batch <= 8 && op.T == 2 && op.K == op.in_c && op.tapstep > 0 && op.tap0 == 0 && op.N % kWarps == 0 && op.K >= 512 &&
+    return !off && op.batch * op.frames <= 8 && rows_per_frame(op) == 2 && !op.elu && !op.raw && op.K == op.in_c && op.tapstep > 0 && op.tap0 == 0 && op.N % kWarps == 0 && op.K >= 512 &&
            op.K <= kStageFloats / R && op.K % 128 == 0 && op.bias == nullptr && op.out_by_row == 0 &&
            ((op.pro == PRO_LN && (op.epi == EPI_BIAS || op.epi == EPI_GELU)) || (op.pro == PRO_NONE && op.epi == EPI_SCALE_RES));
 }
@@ -1001,41 +1071,38 @@ static cudaError_t launch_rows(const RowOp& op, cudaStream_t st) {
         }
     }
     if (use_tile(op)) {
-        const dim3 grid((op.N + kTN - 1) / kTN, (op.batch * op.T + kTM - 1) / kTM);
-        return launch_pdl(tile_kernel, grid, dim3(kThreads), 0, st, op);
+        if (op.pro != PRO_LN) return launch_tiles(op, st);
+        RowOp norm = op, product = op;
+        norm.out = op.norm_at; norm.out_stride = op.in_stride; norm.out_off0 = 0;
+        const cudaError_t e = launch_pdl(norm_kernel, dim3((op.batch * op.T + 3) / 4), dim3(128), 0, st, norm);
+        if (e != cudaSuccess) return e;
+        product.in = op.norm_at; product.in_hs = 0; product.pro = PRO_NONE;
+        return launch_tiles(product, st);
     }
-    if (use_rowdot(op)) return launch_pdl(rowdot_kernel, dim3((op.batch * op.T + kThreads - 1) / kThreads), dim3(kThreads), 0, st, op);
+    if (use_rowdot(op)) return launch_pdl(rowdot_kernel, dim3((op.T + kDotRows - 1) / kDotRows, op.batch), dim3(kThreads), rowdot_smem(op), st, op);
     const int rows = op.batch * op.T;
     const int R = rows_R(rows);
-    // 64+ rows (the SEANet stages below 12 streams, the two-row operations from 32 streams on): four weight rows per warp -- the
-    // same bits, fewer and fatter CTAs.  Measured per step: 4 streams 825 -> 748 us, 32 streams 1.99 -> 1.73 ms, 64 streams
-    // 3.22 -> 2.41 ms; operations of 16 rows (8 streams' Linears) lose 12 % with it, hence the bar.
-    static const int cpw_n = [] { const char* e = getenv("SMOL_MIMI_CPW_MIN_N"); return e ? atoi(e) : 64; }();
-    if (R == 16 && rows >= 64 && op.N >= cpw_n) {
-        const dim3 grid4((op.N + 4 * kWarps - 1) / (4 * kWarps), (rows + R - 1) / R);
-        return launch_pdl(rows_kernel<16, 4>, grid4, dim3(kThreads), 0, st, op);
-    }
     const dim3 grid((op.N + kWarps - 1) / kWarps, (rows + R - 1) / R);
     switch (R) {
-        case 2: return launch_pdl(rows_kernel<2, 1>, grid, dim3(kThreads), 0, st, op);
-        case 4: return launch_pdl(rows_kernel<4, 1>, grid, dim3(kThreads), 0, st, op);
-        case 8: return launch_pdl(rows_kernel<8, 1>, grid, dim3(kThreads), 0, st, op);
-        default: return launch_pdl(rows_kernel<16, 1>, grid, dim3(kThreads), 0, st, op);
+        case 2: return launch_pdl(rows_kernel<2>, grid, dim3(kThreads), 0, st, op);
+        case 4: return launch_pdl(rows_kernel<4>, grid, dim3(kThreads), 0, st, op);
+        case 8: return launch_pdl(rows_kernel<8>, grid, dim3(kThreads), 0, st, op);
+        default: return launch_pdl(rows_kernel<16>, grid, dim3(kThreads), 0, st, op);
     }
 }
 
 // The step as a program: every operation in order (executed by one launch each, or by the persistent kernel).
-static void mimi_program(SmolMimi* m, const int32_t* d_codes, const int32_t* d_slots, int batch, float* d_pcm, std::vector<OpRec>& prog) {
+static void mimi_program(SmolMimi* m, const int32_t* d_codes, const int32_t* d_slots, int batch, int frames, float* d_pcm, std::vector<OpRec>& prog) {
     const SmolMimiConfig& c = m->cfg;
     float* arena = wsf(m, m->o_arena);
     const long long AS = (long long)m->arena_floats;
     prog.clear();
     auto buf = [&](int i) -> const MimiBuf& { return m->bufs[i]; };
-    auto base_op = [&]() { RowOp op{}; op.slots = d_slots; op.batch = batch; op.in_stride = AS; op.out_stride = AS; op.res_stride = AS; op.bias_mod = 1; op.tapstep = 1; return op; };
+    auto base_op = [&]() { RowOp op{}; op.slots = d_slots; op.batch = batch; op.frames = frames; op.in_stride = AS; op.out_stride = AS; op.res_stride = AS; op.bias_mod = 1; op.tapstep = 1; return op; };
     // input of an op: buffer bi, `taps` rows ending at the current one (conv) or {current, previous} (transposed conv)
     auto set_in = [&](RowOp& op, int bi, int taps, bool transposed) {
         const MimiBuf& b = buf(bi);
-        op.in = arena + b.off; op.in_hs = b.hs; op.in_c = b.C; op.T = b.T; op.K = taps * b.C;
+        op.in = arena + b.off; op.in_hs = b.hs; op.in_c = b.C; op.T = b.T * frames; op.K = taps * b.C;
         op.tap0 = transposed ? 0 : -(taps - 1); op.tapstep = transposed ? -1 : 1;
     };
     auto set_out = [&](RowOp& op, int bi) { const MimiBuf& b = buf(bi); op.out = arena + b.off; op.out_off0 = b.hs * b.C; };
@@ -1044,7 +1111,7 @@ static void mimi_program(SmolMimi* m, const int32_t* d_codes, const int32_t* d_s
 
     {   // RVQ rows -> Q; projection + upsample -> the residual stream (current rows of X0)
         OpRec r{}; r.kind = OP_EMBED;
-        r.emb = EmbedArgs{wsf(m, m->o_books), d_codes, d_slots, arena + buf(m->bQ).off, AS, c.n_q, c.codebook_size, c.codebook_dim, batch};
+        r.emb = EmbedArgs{wsf(m, m->o_books), d_codes, d_slots, arena + buf(m->bQ).off, AS, c.n_q, c.codebook_size, c.codebook_dim, batch, frames};
         prog.push_back(r);
         RowOp op = base_op();
         set_in(op, m->bQ, 1, false);
@@ -1058,7 +1125,7 @@ static void mimi_program(SmolMimi* m, const int32_t* d_codes, const int32_t* d_s
         {   // LayerNorm -> q | k | v
             RowOp op = base_op();
             set_in(op, m->bX0, 1, false);
-            op.pro = PRO_LN; op.ln_w = vec; op.ln_b = vec + c.dim; op.eps = c.norm_eps;
+            op.pro = PRO_LN; op.ln_w = vec; op.ln_b = vec + c.dim; op.eps = c.norm_eps; op.norm_at = arena + buf(m->bLN).off;
             op.W = wsf(m, m->o_qkv[l]); op.N = 3 * c.dim; op.epi = EPI_BIAS;
             set_out(op, m->bQKV);
             push_rows(op);
@@ -1072,6 +1139,8 @@ static void mimi_program(SmolMimi* m, const int32_t* d_codes, const int32_t* d_s
             a.err = reinterpret_cast<int32_t*>(m->ws + m->o_err);
             a.part = wsf(m, m->o_part); a.arrive = reinterpret_cast<unsigned int*>(m->ws + m->o_arrive); a.max_splits = m->max_splits;
             a.layer = l; a.dim = c.dim; a.hd = c.head_dim; a.max_pos = c.max_positions; a.window = c.window; a.batch = batch; a.heads = c.n_heads;
+            a.frames = frames; a.max_frames = m->max_frames;
+            if (frames > 1) { r.kind = OP_APPEND; prog.push_back(r); r.kind = OP_ATTN; }
             prog.push_back(r);
         }
         {   // o_proj, layer scale, residual (in place on the stream)
@@ -1084,7 +1153,7 @@ static void mimi_program(SmolMimi* m, const int32_t* d_codes, const int32_t* d_s
         {   // LayerNorm -> fc1 -> GELU
             RowOp op = base_op();
             set_in(op, m->bX0, 1, false);
-            op.pro = PRO_LN; op.ln_w = vec + 2 * c.dim; op.ln_b = vec + 3 * c.dim; op.eps = c.norm_eps;
+            op.pro = PRO_LN; op.ln_w = vec + 2 * c.dim; op.ln_b = vec + 3 * c.dim; op.eps = c.norm_eps; op.norm_at = arena + buf(m->bLN).off;
             op.W = wsf(m, m->o_fc1[l]); op.N = c.ffn; op.epi = EPI_GELU;
             set_out(op, m->bFF);
             push_rows(op);
@@ -1102,7 +1171,7 @@ static void mimi_program(SmolMimi* m, const int32_t* d_codes, const int32_t* d_s
     {
         RowOp op = base_op();
         set_in(op, m->bX0, c.kernel, false);
-        op.W = wsf(m, m->o_conv_in); op.N = m->ch0; op.bias = bias; op.bias_mod = m->ch0; op.epi = EPI_BIAS;
+        op.W = wsf(m, m->o_conv_in); op.N = m->ch0; op.bias = bias; op.bias_mod = m->ch0; op.epi = EPI_BIAS; op.elu = 1;
         set_out(op, m->bA0);
         push_rows(op);
         bias += m->ch0;
@@ -1111,41 +1180,43 @@ static void mimi_program(SmolMimi* m, const int32_t* d_codes, const int32_t* d_s
     for (int i = 0; i < c.n_ratios; ++i) {
         const int r = c.ratios[i];
         ch /= 2;
-        {   // ELU -> transposed convolution (kernel 2 r, stride r): row t -> r output rows, contiguous
+        // Every buffer behind the first convolution holds rows as their readers want them, after the ELU; a block's residual is kept beside.
+        {   // transposed convolution (kernel 2 r, stride r): row t -> r output rows, contiguous
             RowOp op = base_op();
             set_in(op, prev, 2, true);
-            op.pro = PRO_ELU; op.W = wsf(m, m->o_ct[i]); op.N = r * ch; op.bias = bias; op.bias_mod = ch; op.epi = EPI_BIAS;
-            set_out(op, m->bCT[i]);
+            op.W = wsf(m, m->o_ct[i]); op.N = r * ch; op.bias = bias; op.bias_mod = ch; op.epi = EPI_BIAS;
+            set_out(op, m->bCE[i]);
+            op.elu = 1; op.raw = arena + buf(m->bCT[i]).off; op.raw_stride = AS; op.raw_off0 = 0;
             push_rows(op);
             bias += ch;
         }
-        {   // residual block: ELU -> conv k3 -> ELU -> conv k1, + skip
+        {   // residual block: conv k3 -> ELU -> conv k1, + skip, ELU
             RowOp op = base_op();
-            set_in(op, m->bCT[i], c.res_kernel, false);
-            op.pro = PRO_ELU; op.W = wsf(m, m->o_r1[i]); op.N = ch / 2; op.bias = bias; op.bias_mod = ch / 2; op.epi = EPI_BIAS;
+            set_in(op, m->bCE[i], c.res_kernel, false);
+            op.elu = 1; op.W = wsf(m, m->o_r1[i]); op.N = ch / 2; op.bias = bias; op.bias_mod = ch / 2; op.epi = EPI_BIAS;
             set_out(op, m->bH[i]);
             push_rows(op);
             bias += ch / 2;
             RowOp o2 = base_op();
             set_in(o2, m->bH[i], 1, false);
-            o2.pro = PRO_ELU; o2.W = wsf(m, m->o_r2[i]); o2.N = ch; o2.bias = bias; o2.bias_mod = ch; o2.epi = EPI_RES;
+            o2.elu = 1; o2.W = wsf(m, m->o_r2[i]); o2.N = ch; o2.bias = bias; o2.bias_mod = ch; o2.epi = EPI_RES;
             set_out(o2, m->bR[i]); set_res(o2, m->bCT[i]);
             push_rows(o2);
             bias += ch;
         }
         prev = m->bR[i];
     }
-    {   // ELU -> conv k3 -> PCM (the caller's buffer, row b)
+    {   // conv k3 -> PCM (the caller's buffer, row b)
         RowOp op = base_op();
         set_in(op, prev, c.last_kernel, false);
-        op.pro = PRO_ELU; op.W = wsf(m, m->o_conv_out); op.N = 1; op.bias = bias; op.bias_mod = 1; op.epi = EPI_BIAS;
-        op.out = d_pcm; op.out_stride = m->spf; op.out_off0 = 0; op.out_by_row = 1;
+        op.W = wsf(m, m->o_conv_out); op.N = 1; op.bias = bias; op.bias_mod = 1; op.epi = EPI_BIAS;
+        op.out = d_pcm; op.out_stride = (long long)m->spf * frames; op.out_off0 = 0; op.out_by_row = 1;
         push_rows(op);
     }
     {
         OpRec r{}; r.kind = OP_SHIFT;
         r.shift = shift_args(m, d_slots, 0);
-        r.shift.batch = batch;
+        r.shift.batch = batch; r.shift.frames = frames;
         prog.push_back(r);
     }
 }
@@ -1155,19 +1226,34 @@ static int mimi_enqueue(SmolMimi* m, const std::vector<OpRec>& prog, cudaStream_
     for (const OpRec& r : prog) {
         switch (r.kind) {
             case OP_ROWS: MCU(launch_rows(r.row, st)); break;
-            case OP_ATTN: MCU(launch_pdl(attn_kernel, dim3(r.attn.batch, r.attn.heads, r.attn.max_splits), dim3(kThreads), m->attn_smem, st, r.attn)); break;
-            case OP_EMBED: MCU(launch_pdl(embed_kernel, dim3(r.emb.batch), dim3(256), 0, st, r.emb)); break;
+            case OP_ATTN: MCU(launch_pdl(attn_kernel, dim3(r.attn.batch * r.attn.frames, r.attn.heads, r.attn.max_splits), dim3(kThreads), m->attn_smem, st, r.attn)); break;
+            case OP_APPEND: MCU(launch_pdl(append_kernel, dim3(r.attn.batch * r.attn.frames, r.attn.heads), dim3(64), 0, st, r.attn)); break;
+            case OP_EMBED: MCU(launch_pdl(embed_kernel, dim3(r.emb.batch * r.emb.frames), dim3(256), 0, st, r.emb)); break;
             default: MCU(launch_pdl(shift_kernel, dim3(r.shift.batch, r.shift.n_bufs + 1), dim3(kThreads), 0, st, r.shift)); break;
         }
     }
-    m->launches = (int)prog.size();
+    int launches = (int)prog.size();
+    for (const OpRec& r : prog) launches += r.kind == OP_ROWS && r.row.pro == PRO_LN && use_tile(r.row);
+    m->launches = launches;
     return SMOL_OK;
 }
 
+extern "C" int32_t smol_mimi_max_frames(const SmolMimi* m, int32_t batch) {
+    if (!m || batch < 1) return 0;
+    // fewer than 12 streams: as many rows as the row kernels take at once (16), so that a frame's arithmetic is decode_step's
+    const int most = batch >= kTileMinBatch ? 4 : batch <= 8 ? 8 / batch : 1;
+    return most < m->max_frames ? most : m->max_frames;
+}
+
 extern "C" int smol_mimi_decode_step(SmolMimi* m, const int32_t* d_codes, const int32_t* d_slots, int32_t batch, float* d_pcm, void* stream) {
+    return smol_mimi_decode_frames(m, d_codes, d_slots, batch, 1, d_pcm, stream);
+}
+
+extern "C" int smol_mimi_decode_frames(SmolMimi* m, const int32_t* d_codes, const int32_t* d_slots, int32_t batch, int32_t frames, float* d_pcm, void* stream) {
     if (!m || !d_codes || !d_pcm) return smol::capi_fail(SMOL_ERR_INVALID, "smol_mimi_decode_step: null argument");
     if (!m->bound) return smol::capi_fail(SMOL_ERR_UNBOUND, "smol_mimi_decode_step: weights / workspace not bound");
     if (batch < 1 || batch > m->cfg.max_streams) return smol::capi_fail(SMOL_ERR_CAPACITY, "smol_mimi_decode_step: batch outside 1 .. max_streams");
+    if (frames < 1 || frames > smol_mimi_max_frames(m, batch)) return smol::capi_fail(SMOL_ERR_CAPACITY, "smol_mimi_decode_frames: frames outside 1 .. smol_mimi_max_frames()");
     cudaStream_t st = (cudaStream_t)stream;
     const int mode = m->cfg.use_graph;   // 0: one launch per operation; 1: those launches replayed as a CUDA graph
     // programmatic dependent launch: every kernel fetches its first weights and prefetches its rows into L2 before the
@@ -1178,7 +1264,7 @@ extern "C" int smol_mimi_decode_step(SmolMimi* m, const int32_t* d_codes, const 
     g_pdl = pe ? pe[0] != '0' : (mode == 0 || batch < kTileMinBatch);
     SmolMimi::Step* step = nullptr;
     for (SmolMimi::Step& c : m->steps)
-        if (c.codes == d_codes && c.slots == d_slots && c.pcm == d_pcm && c.batch == batch) { step = &c; break; }
+        if (c.codes == d_codes && c.slots == d_slots && c.pcm == d_pcm && c.batch == batch && c.frames == frames) { step = &c; break; }
     if (!step) {
         if (m->steps.size() >= kMaxSteps) {   // evict the least recently used
             size_t lru = 0;
@@ -1186,9 +1272,9 @@ extern "C" int smol_mimi_decode_step(SmolMimi* m, const int32_t* d_codes, const 
             if (m->steps[lru].graph) cudaGraphExecDestroy(m->steps[lru].graph);
             m->steps.erase(m->steps.begin() + lru);
         }
-        m->steps.push_back(SmolMimi::Step{d_codes, d_slots, d_pcm, batch, {}, nullptr, 0});
+        m->steps.push_back(SmolMimi::Step{d_codes, d_slots, d_pcm, batch, frames, {}, nullptr, 0});
         step = &m->steps.back();
-        mimi_program(m, d_codes, d_slots, batch, d_pcm, step->prog);
+        mimi_program(m, d_codes, d_slots, batch, frames, d_pcm, step->prog);
     }
     step->used = ++m->tick;
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;

@@ -128,6 +128,8 @@ class MimiModel:
         h = C.c_void_p()
         _capi.check(self._lib.smol_mimi_create(C.byref(cfg), C.byref(h)))
         self._h = h
+        # room for decode() to take several frames of a stream at once: 3 MB per stream and frame
+        _capi.check(self._lib.smol_mimi_set_max_frames(h, 8 if max_streams <= 16 else 4))
         self.samples_per_frame = int(self._lib.smol_mimi_samples_per_frame(h))
         assert self.samples_per_frame == 2 * math.prod(c.seanet.ratios)
         self._ws: Optional[torch.Tensor] = None
@@ -221,11 +223,15 @@ class MimiModel:
     # ---- streams ------------------------------------------------------------------------------------------------------
     def make_cache(self) -> MimiCache:
         """A fresh stream (make_prompt_cache(codec.decoder_transformer), __init__.py:86, plus MimiDecoder.reset)."""
-        if not self._free:
+        return self._open(1)[0]
+
+    def _open(self, n: int) -> List[MimiCache]:
+        """n fresh streams, their slots reset together."""
+        if len(self._free) < n:
             raise RuntimeError(f"MimiModel: all {self.max_streams} stream slots are in use (release_cache() one)")
-        slot = self._free.pop()
-        self._reset([slot])
-        return MimiCache(slot)
+        slots = [self._free.pop() for _ in range(n)]
+        self._reset(slots)
+        return [MimiCache(s) for s in slots]
 
     def release_cache(self, cache: MimiCache) -> None:
         self._free.append(cache.slot)
@@ -241,12 +247,32 @@ class MimiModel:
         for s in slots:
             self._frames[s] = 0
 
-    def _buffers(self, batch: int):
-        if batch not in self._io:
-            self._io[batch] = (torch.zeros(batch, self.num_codebooks, dtype=torch.int32, device=self.device),
-                               torch.zeros(batch, dtype=torch.int32, device=self.device),
-                               torch.zeros(batch, self.samples_per_frame, dtype=torch.float32, device=self.device))
-        return self._io[batch]
+    def _buffers(self, batch: int, frames: int = 1):
+        key = (batch, frames)
+        if key not in self._io:
+            self._io[key] = (torch.zeros(batch, frames, self.num_codebooks, dtype=torch.int32, device=self.device),
+                             torch.zeros(batch, dtype=torch.int32, device=self.device),
+                             torch.zeros(batch, frames * self.samples_per_frame, dtype=torch.float32, device=self.device))
+        return self._io[key]
+
+    def _run(self, codes: torch.Tensor, caches: Sequence[MimiCache]) -> torch.Tensor:
+        """codes [B, frames, n_q] -> PCM [B, frames * samples_per_frame] (a view of an internal buffer)."""
+        B, frames = codes.shape[:2]
+        for c in caches:
+            if self._frames[c.slot] + frames > self.max_frames:
+                raise RuntimeError(f"MimiModel: stream in slot {c.slot} is at max_frames = {self.max_frames}")
+        d_codes, d_slots, d_pcm = self._buffers(B, frames)
+        d_codes.copy_(codes.to(torch.int32), non_blocking=True)
+        slots = tuple(c.slot for c in caches)
+        if self._io_slots.get((B, frames)) != slots:      # a batch's slot table changes only when streams come and go
+            d_slots.copy_(torch.tensor(slots, dtype=torch.int32), non_blocking=True)
+            self._io_slots[(B, frames)] = slots
+        _capi.check(self._lib.smol_mimi_decode_frames(self._h, C.c_void_p(d_codes.data_ptr()), C.c_void_p(d_slots.data_ptr()), B, frames,
+                                                      C.c_void_p(d_pcm.data_ptr()), C.c_void_p(self._stream())))
+        for c in caches:
+            self._frames[c.slot] += frames
+            c.frames = self._frames[c.slot]
+        return d_pcm
 
     def decode_step(self, codes: torch.Tensor, cache: Union[MimiCache, Sequence[MimiCache]]) -> torch.Tensor:
         """codes [B, n_q, 1] (or [B, n_q]) -> PCM [B, 1, samples_per_frame]; row b continues the stream of cache[b]
@@ -262,33 +288,29 @@ class MimiModel:
             raise ValueError(f"decode_step: codes {tuple(codes.shape)} vs {len(caches)} caches x {self.num_codebooks} codebooks")
         if len({c.slot for c in caches}) != B:
             raise ValueError("decode_step: two rows of the batch name the same stream")
-        for c in caches:
-            if self._frames[c.slot] >= self.max_frames:
-                raise RuntimeError(f"MimiModel: stream in slot {c.slot} is at max_frames = {self.max_frames}")
-        d_codes, d_slots, d_pcm = self._buffers(B)
-        d_codes.copy_(codes.to(torch.int32), non_blocking=True)
-        slots = tuple(c.slot for c in caches)
-        if self._io_slots.get(B) != slots:      # the slot table of this batch size changes only when streams come and go
-            d_slots.copy_(torch.tensor(slots, dtype=torch.int32), non_blocking=True)
-            self._io_slots[B] = slots
-        _capi.check(self._lib.smol_mimi_decode_step(self._h, C.c_void_p(d_codes.data_ptr()), C.c_void_p(d_slots.data_ptr()), B,
-                                                    C.c_void_p(d_pcm.data_ptr()), C.c_void_p(self._stream())))
-        for c in caches:
-            self._frames[c.slot] += 1
-            c.frames = self._frames[c.slot]
-        return d_pcm.view(B, 1, self.samples_per_frame)
+        return self._run(codes[:, None], caches).view(B, 1, self.samples_per_frame)
 
     def decode(self, audio_codes: torch.Tensor, cache: Optional[Sequence[MimiCache]] = None) -> torch.Tensor:
-        """codes [B, n_q, T] -> PCM [B, 1, T * samples_per_frame] as a run of streaming steps over fresh (or the given) streams.
+        """codes [B, n_q, T] -> PCM [B, 1, T * samples_per_frame] as a run of streaming steps over fresh (or the given) streams, several
+        frames per step where they give the same bits.
         With ``upsample_carry=True`` this equals the reference's whole-sequence ``decode`` (codec/mimi.py:88-100); with the
         default it is what a run of the reference's ``decode_step`` calls produces."""
         B, _, T = audio_codes.shape
         own = cache is None
-        caches = [self.make_cache() for _ in range(B)] if own else list(cache)
-        out = torch.empty(B, 1, T * self.samples_per_frame, dtype=torch.float32, device=self.device)
-        codes = audio_codes.to(self.device)
-        for t in range(T):
-            out[:, :, t * self.samples_per_frame:(t + 1) * self.samples_per_frame] = self.decode_step(codes[:, :, t], caches)
+        caches = self._open(B) if own else list(cache)
+        if len(caches) != B or audio_codes.shape[1] != self.num_codebooks:
+            raise ValueError(f"decode: codes {tuple(audio_codes.shape)} vs {len(caches)} caches x {self.num_codebooks} codebooks")
+        if len({c.slot for c in caches}) != B:
+            raise ValueError("decode: two rows of the batch name the same stream")
+        n = self.samples_per_frame
+        out = torch.empty(B, 1, T * n, dtype=torch.float32, device=self.device)
+        codes = audio_codes.to(self.device).transpose(1, 2)
+        most = max(1, int(self._lib.smol_mimi_max_frames(self._h, B)))
+        t = 0
+        while t < T:
+            frames = min(most, T - t)
+            out[:, 0, t * n:(t + frames) * n] = self._run(codes[:, t:t + frames], caches)
+            t += frames
         if own:
             for c in caches:
                 self.release_cache(c)

@@ -94,3 +94,19 @@ def test_four_token_scan_of_prompts(dim):
                 assert rel_err(first[at:at + n], want[i][:n]) < TOL[torch.float32]
             assert rel_err(then[18 * i:18 * i + 18], want[i][n:]) < TOL[torch.float32]
             at += n
+
+
+@pytest.mark.parametrize("streams,frames", [(1, 11), (3, 5), (8, 3), (11, 2), (12, 9), (17, 6)])
+def test_codec_runs_of_frames_equal_single_steps(streams, frames):
+    """decode() takes up to 8 frames of few streams, 4 of many, at once: bit for bit what decode_step returns frame by frame."""
+    from smoltts_b200.mimi import MimiModel
+    from smoltts_b200.synth import make_mimi_state_dict
+
+    m = MimiModel(max_streams=streams, max_frames=16)
+    m.load_state_dict(make_mimi_state_dict(3))
+    codes = torch.randint(0, 2048, (streams, 8, frames), generator=torch.Generator().manual_seed(frames))
+    whole = m.decode(codes)
+    caches = [m.make_cache() for _ in range(streams)]
+    steps = torch.cat([m.decode_step(codes[:, :, t:t + 1], caches).clone() for t in range(frames)], -1)
+    assert torch.equal(whole, steps)
+    assert not m.overflowed()

@@ -46,6 +46,8 @@ __host__ __device__ constexpr int group_scan_buf_floats(int DK) { return group_s
 // (their only product is made by the kernel in front).  DELTA: keys with keys too, and the own products are there already.
 template <bool DELTA>
 __global__ void __launch_bounds__(128) scan_pairs_kernel(const GroupScanArgs A, float* __restrict__ pairs) {
+    dep_wait();
+    dep_go();
     const int g = blockIdx.z * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
     const int t0 = A.seq_start[blockIdx.y], n_all = A.seq_start[blockIdx.y + 1] - t0, r0 = blockIdx.x * kScanGroup;
     if (g >= A.G || n_all <= 1 || r0 >= n_all) return;
@@ -109,6 +111,8 @@ __device__ __forceinline__ void group_scan_stage(const GroupScanArgs& A, float* 
 
 template <int DK, bool DELTA>
 __global__ void __launch_bounds__(gla_block_cols(DK) * gla_lanes(DK)) group_scan_kernel(const GroupScanArgs A, float* state_pool, float* __restrict__ o_raw) {
+    dep_wait();
+    dep_go();
     constexpr int L = gla_lanes(DK), CB = gla_block_cols(DK), RV = DK / L / 4, CH = group_scan_chunk(DK), PL = CH * DK;
     constexpr int kBuf = group_scan_buf_floats(DK), GS = kScanGroup;
     static_assert(L >= GS && kBuf % 4 == 0, "a lane per token of a group stores its result; 16-byte buffers");
@@ -272,6 +276,8 @@ struct GatedDeltaArgs {
 constexpr int kGatedDeltaCols = 64;
 __global__ void __launch_bounds__(128) gated_delta_prep_kernel(const GatedDeltaArgs A, const float* __restrict__ slots, float* __restrict__ qkv,
                                                                float* __restrict__ head, float* __restrict__ pairs) {
+    dep_wait();
+    dep_go();
     const int t = blockIdx.x, warp = blockIdx.y * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
     const ConvIo& C = A.conv;
     const int s = A.tok_seq[t], r = t - C.seq_start[s], pos0 = C.seq_pos0[s], slot = C.seq_slot[s];
@@ -354,6 +360,8 @@ constexpr int kMlstmTile = 1024;
 // head: (decay, write weight) [T][H]; floor [T][H]
 __global__ void __launch_bounds__(kMlstmTile) mlstm_gate_kernel(const MlstmArgs A, float* __restrict__ slots, float* __restrict__ head, float* __restrict__ floor_,
                                                               float* __restrict__ pairs) {
+    dep_wait();
+    dep_go();
     __shared__ float wf[kMlstmTile / 32], wi[kMlstmTile / 32], ms[kMlstmTile + 1];
     const int s = blockIdx.x / A.H, h = blockIdx.x % A.H, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int t0 = A.seq_start[s], t1 = A.seq_start[s + 1], slot = A.seq_slot[s];

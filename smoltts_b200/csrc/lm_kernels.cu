@@ -62,6 +62,8 @@ __device__ __forceinline__ float block_sum(float v, float* red) {
 template <class T>
 __global__ void embed_norm_kernel(const int32_t* __restrict__ tokens, const T* __restrict__ embed, float scale, int D, int vocab,
                                   const float* __restrict__ wn, float eps, float* __restrict__ x, T* __restrict__ hn, const float woff) {
+    dep_wait();
+    dep_go();
     __shared__ float red[33];
     const int t = blockIdx.x;
     int tok = tokens[t];
@@ -82,6 +84,8 @@ __global__ void embed_norm_kernel(const int32_t* __restrict__ tokens, const T* _
 template <class T>
 __global__ void norm_rows_kernel(const float* __restrict__ x, const int32_t* __restrict__ rows, const float* __restrict__ w, float eps,
                                  int D, T* __restrict__ out, const float woff) {
+    dep_wait();
+    dep_go();
     __shared__ float red[33];
     const int r = blockIdx.x;
     const float* xr = x + (size_t)(rows ? rows[r] : r) * D;
@@ -113,6 +117,8 @@ template <class T>
 __global__ void add_norm_kernel(float* __restrict__ x, const float* __restrict__ y, const float* __restrict__ wb,
                                 const float* __restrict__ ls, const float* __restrict__ wn, float eps, int D, T* __restrict__ hn,
                                 const float woff, const float* __restrict__ yb, const RoutedSum rs, const T* hin) {
+    dep_wait();
+    dep_go();
     extern __shared__ float row[];
     __shared__ float red[33];
     const size_t o = (size_t)blockIdx.x * D;
@@ -214,6 +220,8 @@ template <> __device__ __forceinline__ void store4<bf16>(bf16* p, float a, float
 // are taken in one pass and reduced together; rows whose length is a multiple of 4 move as 16-byte pieces.
 template <class T>
 __global__ void polynorm_kernel(const float* __restrict__ z, const float* __restrict__ coef, float eps, int F, T* __restrict__ out) {
+    dep_wait();
+    dep_go();
     __shared__ float red[3][33];
     const size_t o = (size_t)blockIdx.x * F;
     const bool vec = F % 4 == 0;
@@ -278,6 +286,7 @@ static GemmIo plain_io(int K, int N) {
 template <int BM, int BN, int TM, int TN>
 __global__ void __launch_bounds__(f32t::Tile<BM, BN, TM, TN>::NT) gemm_f32_tile_kernel(const float* __restrict__ a, const float* __restrict__ w,
                                                                                        float* __restrict__ y, int M, int N, int K, const GemmIo io) {
+    dep_wait();      // (and no early dep_go: the next kernel's blocks would take room from the CTAs that are still to come)
     using T = f32t::Tile<BM, BN, TM, TN>;
     extern __shared__ __align__(16) float f32_sm[];
     __shared__ long long arow[BM];
@@ -320,6 +329,8 @@ __global__ void __launch_bounds__(f32t::Tile<BM, BN, TM, TN>::NT) gemm_f32_tile_
 template <int BM, int BN, int BK, int TM, int TN>
 __global__ void __launch_bounds__((BM / TM) * (BN / TN)) gemm_f32_kernel(const float* __restrict__ a, const float* __restrict__ w,
                                                                         float* __restrict__ y, int M, int N, int K, const GemmIo io) {
+    dep_wait();
+    dep_go();
     constexpr int NT = (BM / TM) * (BN / TN);
     __shared__ float As[BK][BM + 1];
     __shared__ float Ws[BK][BN + 1];
@@ -432,6 +443,8 @@ __device__ __forceinline__ void gemm_stash(bf16* dst, const uint4 (&reg)[ROWS * 
 template <int WR, int WC, int MT, int NT>
 __global__ void __launch_bounds__(128) gemm_bf16_kernel(const bf16* __restrict__ a, const bf16* __restrict__ w, float* __restrict__ y,
                                                         int M, int N, int K, const GemmIo io, const bool vec) {
+    dep_wait();
+    dep_go();
     static_assert(WR * WC == 4, "four warps");
     constexpr int BM = WR * MT * 16, BN = WC * NT * 8;
     static_assert(BM % 32 == 0 && BN % 32 == 0, "tile rows are fetched 32 at a time");
@@ -556,14 +569,20 @@ __global__ void __launch_bounds__(WARPS * 32) gemm_few_kernel(const bf16* __rest
 #pragma unroll
         for (int e = 0; e < 4; ++e) acc[i][e] = 0.0f;
     const uint4 zero = make_uint4(0, 0, 0, 0);
-    for (int k0 = warp * 32; k0 < K; k0 += WARPS * 32 * U) {
-        uint4 p[U][WT], x[U][AT];
+    uint4 p[U][WT];
+    auto load_weights = [&](int k0) {
 #pragma unroll
         for (int u = 0; u < U; ++u) {
             const int k = k0 + u * WARPS * 32;
 #pragma unroll
             for (int i = 0; i < WT; ++i) p[u][i] = k + tq * 8 < K ? ldg_stream(wr[i] + k) : zero;
         }
+    };
+    load_weights(warp * 32);             // no kernel writes weights: the first ones are on their way before the wait
+    dep_wait();
+    dep_go();
+    for (int k0 = warp * 32; k0 < K; k0 += WARPS * 32 * U) {
+        uint4 x[U][AT];
 #pragma unroll
         for (int u = 0; u < U; ++u) {
             const int k = k0 + u * WARPS * 32 + tq * 8;
@@ -585,6 +604,7 @@ __global__ void __launch_bounds__(WARPS * 32) gemm_few_kernel(const bf16* __rest
                     mma_bf16_16816(acc[i], x[u][2 * i].z, x[u][2 * i + 1].z, x[u][2 * i].w, x[u][2 * i + 1].w, p[u][0].z, p[u][0].w);
                 }
             }
+        load_weights(k0 + WARPS * 32 * U);
     }
     // part[warp][m * NR + n]: neighbouring outputs of a row side by side.  acc[.][e]: tile row g + (e / 2) * 8, tile column 2 tq + e % 2
 #pragma unroll
@@ -685,6 +705,8 @@ __device__ __forceinline__ float attn_score(const AttnArgs& A, float dot, int di
 // q_norm / k_norm == nullptr: no norm.
 template <class T>
 __global__ void attn_prep_kernel(const AttnArgs A, T* __restrict__ qbuf, T* __restrict__ pool) {
+    dep_wait();
+    dep_go();
     const int lane = threadIdx.x & 31;
     const int unit = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     const int HQ = A.H * A.maps, GK = A.G * A.maps, slots = HQ + (A.own_kv ? GK + A.G : 0);
@@ -738,6 +760,8 @@ constexpr int kMaxRotPairs = 256;
 
 template <class T, bool ROT>
 __global__ void __launch_bounds__(256) attn_prep_whole_kernel(const AttnArgs A, T* __restrict__ qbuf, T* __restrict__ pool) {
+    dep_wait();
+    dep_go();
     __shared__ float red[2][33];
     __shared__ float turn[2][ROT ? kMaxRotPairs : 1];
     const int t = blockIdx.x, nq = A.H * A.d, nk = A.G * A.d, nv = A.G * A.dv;
@@ -874,6 +898,8 @@ __device__ __forceinline__ void attn_finish(const AttnArgs& A, size_t t, int h, 
 template <class T, int MAXV, int MAPS>
 __global__ void __launch_bounds__(kAttnWarps * 32) attn_kernel(const AttnArgs A, const T* __restrict__ qbuf, const T* __restrict__ pool,
                                                                T* __restrict__ out) {
+    dep_wait();
+    dep_go();
     extern __shared__ float qs_all[];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int unit = blockIdx.x * kAttnWarps + warp;
@@ -991,6 +1017,8 @@ template <class T> __host__ __device__ constexpr int split_value_ld(int dv) { re
 
 template <class T, int MAXV, int KPL>
 __global__ void __launch_bounds__(256) attn_split_kernel(const AttnArgs A, const T* __restrict__ qbuf, const T* __restrict__ pool) {
+    dep_wait();
+    dep_go();
     // One block per (row, key/value head x group of up to 8 of its query rows, key range); one warp per query row (a query
     // head, or one of its maps: the block then stages every map's keys beside the values they share).
     // 32 * KPL keys and values at a time (KPL keys per lane) are staged in shared memory (rows padded by 16 bytes: conflict-free
@@ -1120,6 +1148,8 @@ __global__ void __launch_bounds__(256) attn_split_kernel(const AttnArgs A, const
 constexpr int kMergeWarps = 8;      // per map
 template <class T, int MAXV, int MAPS>
 __global__ void __launch_bounds__(kMergeWarps * MAPS * 32) attn_merge_kernel(const AttnArgs A, T* __restrict__ out) {
+    dep_wait();
+    dep_go();
     constexpr int PER = kMergeWarps, ALL = PER * MAPS;   // warps per map, of the block
     extern __shared__ float share[];                    // [ALL][dv], then [ALL] denominators
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -1275,6 +1305,8 @@ __device__ __forceinline__ void stage_rows(bf16* dst, int cols, RowPtr src) {
 template <int DK, int DV, bool VK, int MAPS>
 __global__ void __launch_bounds__(128 * MAPS) attn_flash_kernel(const AttnArgs A, const bf16* __restrict__ qbuf, const bf16* __restrict__ pool,
                                                          bf16* __restrict__ out) {
+    dep_wait();
+    dep_go();
     constexpr int LD = DK + 8, kTile = 64 * LD, LDV = VK ? LD : DV + 8, kTileV = 64 * LDV;
     static_assert(!VK || (DV <= DK && MAPS == 1), "values inside the key rows");
     constexpr int NTHR = 128 * MAPS;
@@ -1505,6 +1537,8 @@ struct DeltaArgs {
 // One token per block made 2048 tokens of 12 x 64 channels and rank 64 read 400 MB of it: 84 us; eight: 27 us.
 template <int TT>
 __global__ void __launch_bounds__(128) delta_prep_kernel(const DeltaArgs A, float* __restrict__ decay, float* __restrict__ ukey, float* __restrict__ aukey) {
+    dep_wait();
+    dep_go();
     extern __shared__ float th[];   // tanh(inner) [rank][TT], then 1/|k| [TT][H]
     const int t0 = blockIdx.x * TT, nt = min(TT, A.n_tokens - t0), HD = A.H * A.d;      // blockIdx.y: a slice of blockDim.x channels
     float* inv = th + A.rank * TT;
@@ -1629,6 +1663,8 @@ __global__ void __launch_bounds__(delta_block_cols(DK) * delta_lanes(DK)) delta_
                                                                                            const float* __restrict__ ukey,
                                                                                            const float* __restrict__ aukey,
                                                                                            float* __restrict__ state_pool, float* __restrict__ o_raw) {
+    dep_wait();
+    dep_go();
     constexpr int L = delta_lanes(DK), CB = delta_block_cols(DK), NS = DK / CB, RV = DK / L / 4, PL = kDeltaChunk * DK;
     constexpr int kBuf = delta_buf_floats(DK);
     static_assert(DK % (4 * L) == 0, "every lane owns whole 16-byte pieces");
@@ -1739,6 +1775,8 @@ __global__ void __launch_bounds__(delta_block_cols(DK) * delta_lanes(DK)) delta_
 // gate, written in T.  One warp per (token, head).
 template <class T>
 __global__ void delta_out_kernel(const DeltaArgs A, const float* __restrict__ o_raw, T* __restrict__ out) {
+    dep_wait();
+    dep_go();
     const int lane = threadIdx.x & 31;
     const int unit = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     if (unit >= A.n_tokens * A.H) return;
@@ -1759,6 +1797,8 @@ __global__ void __launch_bounds__(kThreads) lm_sample_kernel(const float* __rest
                                                              float top_p, float min_p, unsigned long long seed,
                                                              const int32_t* __restrict__ seq_id, const int32_t* __restrict__ step,
                                                              int32_t* __restrict__ out) {
+    dep_wait();
+    dep_go();
     extern __shared__ __align__(16) float lg[];
     __shared__ SampleScratch sc;
     for (int b = blockIdx.x; b < rows; b += gridDim.x) {
@@ -2383,6 +2423,41 @@ extern "C" int smol_lm_bind(SmolLm* m, const SmolLmGlobals* g, void* d_workspace
     return SMOL_OK;
 }
 
+// The kernels of a step are launched with programmatic stream serialization and begin with dep_wait(): a kernel's blocks are set up while
+// the kernel before it drains, instead of after.  What bounds a decoding step is its chain of some hundred dependent kernels of two to ten
+// microseconds: 10 layers of width 768, one token against 2048 cached ones, 4 steps 1780 us -> 1560; 5 sequences of 700 through 4 layers of
+// width 1536, 1024 -> 940.  A launch right after a wait for another stream's event goes out plainly.
+static thread_local bool t_plain_next = false;
+static cudaError_t wait_event(cudaStream_t st, cudaEvent_t e) {
+    t_plain_next = true;
+    return cudaStreamWaitEvent(st, e, 0);
+}
+template <class... P, class... X>
+static cudaError_t pdl_launch(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, X&&... args) {
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = t_plain_next ? 0 : 1;
+    t_plain_next = false;
+    return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(std::forward<X>(args))...);
+}
+
+// Kernels whose few long blocks need the SMs to themselves: set up early, they crowd onto those SMs that the kernel before leaves first,
+// two or three to one, and the rest stay idle.  Scans, attention and fp32 products of prompts are launched this way; with all of them early,
+// 2048 tokens through two layers of width 768 took 786 us instead of 665 (706 with every launch plain), 300 in fp32 917 instead of 830.
+// The tcgen05 products keep the SM to themselves by their shared memory and gain by the early start (1164 us instead of 1138).
+template <class... P, class... X>
+static cudaError_t plain_launch(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, X&&... args) {
+    t_plain_next = true;
+    return pdl_launch(kernel, grid, block, smem, st, std::forward<X>(args)...);
+}
+
 // y fp32 [M, N] = a [M, K] . w [N, K]^T
 template <class T>
 static cudaError_t linear(SmolLm* m, const T* a, const T* w, float* y, int M, int N, int K, cudaStream_t st);
@@ -2413,6 +2488,7 @@ static cudaError_t launch_f32_tile(const float* a, const float* w, float* y, int
     at[0].val.clusterDim.x = S; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
     cfg.attrs = at;
     cfg.numAttrs = 1;
+    t_plain_next = false;      // launched plainly, as plain_launch does
     return cudaLaunchKernelEx(&cfg, gemm_f32_tile_kernel<BM, BN, TM, TN>, a, w, y, M, N, K, io);
 }
 
@@ -2428,13 +2504,13 @@ cudaError_t linear_ex<float>(SmolLm* m, const float* a, const float* w, float* y
     }
     if (io.tile_group) {
         dim3 grid((N + 63) / 64, tiles, 1);
-        gemm_f32_kernel<32, 64, 16, 2, 4><<<grid, 256, 0, st>>>(a, w, y, M, N, K, io);
+        pdl_launch(gemm_f32_kernel<32, 64, 16, 2, 4>, grid, 256, 0, st, a, w, y, M, N, K, io);
     } else if (M <= 16) {
         dim3 grid((N + 63) / 64, (M + 15) / 16, batch);
-        gemm_f32_kernel<16, 64, 16, 1, 4><<<grid, 256, 0, st>>>(a, w, y, M, N, K, io);
+        pdl_launch(gemm_f32_kernel<16, 64, 16, 1, 4>, grid, 256, 0, st, a, w, y, M, N, K, io);
     } else {
         dim3 grid((N + 63) / 64, (M + 63) / 64, batch);
-        gemm_f32_kernel<64, 64, 16, 4, 4><<<grid, 256, 0, st>>>(a, w, y, M, N, K, io);
+        pdl_launch(gemm_f32_kernel<64, 64, 16, 4, 4>, grid, 256, 0, st, a, w, y, M, N, K, io);
     }
     return cudaGetLastError();
 }
@@ -2456,16 +2532,16 @@ cudaError_t linear_ex<bf16>(SmolLm* m, const bf16* a, const bf16* w, float* y, i
     const bool vec = io_vec(a, w, K, io);
     if (io.tile_group) {
         dim3 grid((N + 31) / 32, tiles, 1);
-        gemm_bf16_kernel<1, 4, 2, 1><<<grid, 128, 0, st>>>(a, w, y, M, N, K, io, vec);       // 32 x 32
+        pdl_launch(gemm_bf16_kernel<1, 4, 2, 1>, grid, 128, 0, st, a, w, y, M, N, K, io, vec);       // 32 x 32
     } else if (M <= 32) {
         dim3 grid((N + 31) / 32, (M + 31) / 32, batch);
-        gemm_bf16_kernel<1, 4, 2, 1><<<grid, 128, 0, st>>>(a, w, y, M, N, K, io, vec);       // 32 x 32
+        pdl_launch(gemm_bf16_kernel<1, 4, 2, 1>, grid, 128, 0, st, a, w, y, M, N, K, io, vec);       // 32 x 32
     } else if (M <= 256 || ((N + 63) / 64) * ((M + 127) / 128) * batch < 2 * 148) {      // 128-row tiles only when they still fill the GPU twice
         dim3 grid((N + 63) / 64, (M + 63) / 64, batch);
-        gemm_bf16_kernel<2, 2, 2, 4><<<grid, 128, 0, st>>>(a, w, y, M, N, K, io, vec);       // 64 x 64
+        pdl_launch(gemm_bf16_kernel<2, 2, 2, 4>, grid, 128, 0, st, a, w, y, M, N, K, io, vec);       // 64 x 64
     } else {
         dim3 grid((N + 63) / 64, (M + 127) / 128, batch);
-        gemm_bf16_kernel<2, 2, 4, 4><<<grid, 128, 0, st>>>(a, w, y, M, N, K, io, vec);       // 128 x 64
+        pdl_launch(gemm_bf16_kernel<2, 2, 4, 4>, grid, 128, 0, st, a, w, y, M, N, K, io, vec);       // 128 x 64
     }
     m->launches++;
     return cudaGetLastError();
@@ -2494,7 +2570,7 @@ static bool launch_gemm_tc_sized(const bf16* a, const bf16* w, float* y, int M, 
         return false;
     const long long tiles = (long long)row_tiles * ((N + BN - 1) / BN);
     const int grid = io.tile_group ? n_sms : (int)std::min<long long>(tiles, n_sms);
-    gemm_tc_kernel<BN><<<grid, kTcThreads, gemm_tc_smem<BN>(), st>>>(ta, tw, y, M, N, K, io);
+    pdl_launch(gemm_tc_kernel<BN>, grid, kTcThreads, gemm_tc_smem<BN>(), st, ta, tw, y, M, N, K, io);
     return true;
 }
 // false: the driver refused a tensor map (the caller takes another form)
@@ -2520,8 +2596,8 @@ cudaError_t linear<bf16>(SmolLm* m, const bf16* a, const bf16* w, float* y, int 
         // the block's shape by N and K alone: a row's result must not depend on what else the step holds beyond its number of rows
 #define SMOL_FEW(NR, MT)                                                                                          \
         do {                                                                                                      \
-            if (K >= kFewLongK) gemm_few_kernel<NR, MT, 16><<<(N + NR - 1) / NR, 512, 0, st>>>(a, w, y, M, N, K); \
-            else gemm_few_kernel<NR, MT, 8><<<(N + NR - 1) / NR, 256, 0, st>>>(a, w, y, M, N, K);                 \
+            if (K >= kFewLongK) pdl_launch(gemm_few_kernel<NR, MT, 16>, (N + NR - 1) / NR, 512, 0, st, a, w, y, M, N, K); \
+            else pdl_launch(gemm_few_kernel<NR, MT, 8>, (N + NR - 1) / NR, 256, 0, st, a, w, y, M, N, K);                 \
         } while (0)
         if (N < kFewWideN) {
             if (M <= 16) SMOL_FEW(8, 1);
@@ -2552,7 +2628,7 @@ template <int DK>
 static cudaError_t launch_scan(const DeltaArgs& A, int n_seqs, const float* dec, const float* u, const float* au, float* pool, float* o_raw,
                                cudaStream_t st) {
     constexpr int threads = delta_block_cols(DK) * delta_lanes(DK), groups = DK / delta_block_cols(DK);
-    delta_scan_kernel<DK><<<n_seqs * A.H * groups, threads, 2 * delta_buf_floats(DK) * sizeof(float), st>>>(A, dec, u, au, pool, o_raw);
+    pdl_launch(delta_scan_kernel<DK>, n_seqs * A.H * groups, threads, 2 * delta_buf_floats(DK) * sizeof(float), st, A, dec, u, au, pool, o_raw);
     return cudaGetLastError();
 }
 
@@ -2563,10 +2639,10 @@ static cudaError_t launch_quad_sized(SmolLm* m, QuadSource Q, QuadArgs A, int n_
     constexpr int FORM = quad_form(KIND);
     float* rec = reinterpret_cast<float*>(m->ws + m->o_rec);
     Q.cap = A.cap = m->cfg.max_step_tokens / kQuad + m->cfg.max_step_seqs + 1;
-    quad_prep_kernel<KIND, DK><<<dim3((max_n + kQuad - 1) / kQuad, n_seqs, (Q.H + 3) / 4), 128, 0, st>>>(Q, rec);
+    pdl_launch(quad_prep_kernel<KIND, DK>, dim3((max_n + kQuad - 1) / kQuad, n_seqs, (Q.H + 3) / 4), 128, 0, st, Q, rec);
     A.rec = rec;
     const int parts = (A.dv + kQuadCols - 1) / kQuadCols;
-    quad_scan_kernel<DK, FORM><<<n_seqs * A.H * parts, kQuadThreads, std::max(quad_smem(FORM, DK), min_smem), st>>>(A, m->slots, o_raw);
+    plain_launch(quad_scan_kernel<DK, FORM>, n_seqs * A.H * parts, kQuadThreads, std::max(quad_smem(FORM, DK), min_smem), st, A, m->slots, o_raw);
     m->launches += 1;
     return cudaGetLastError();
 }
@@ -2585,8 +2661,8 @@ static cudaError_t launch_gla_scan(const GlaArgs& A, int n_seqs, const float* de
     constexpr int CB = gla_block_cols(DK), threads = CB * gla_lanes(DK);
     const int groups = (A.dv + CB - 1) / CB;
     const size_t smem = std::max(2 * gla_buf_floats(DK) * sizeof(float), min_smem);
-    if (A.head_decay) gla_scan_kernel<DK, true><<<n_seqs * A.H * groups, threads, smem, st>>>(A, dec, pool, o_raw);
-    else gla_scan_kernel<DK, false><<<n_seqs * A.H * groups, threads, smem, st>>>(A, dec, pool, o_raw);
+    if (A.head_decay) pdl_launch(gla_scan_kernel<DK, true>, n_seqs * A.H * groups, threads, smem, st, A, dec, pool, o_raw);
+    else pdl_launch(gla_scan_kernel<DK, false>, n_seqs * A.H * groups, threads, smem, st, A, dec, pool, o_raw);
     return cudaGetLastError();
 }
 // the scan over key sizes up to 256: the smallest built size that holds A.d
@@ -2609,7 +2685,7 @@ template <int DK, bool DELTA>
 static cudaError_t launch_group_scan(const GroupScanArgs& A, int n_seqs, float* pool, float* o_raw, cudaStream_t st, size_t min_smem) {
     constexpr int CB = gla_block_cols(DK), threads = CB * gla_lanes(DK);
     const int parts = (A.dv + (A.unit_out ? 1 : 0) + CB - 1) / CB;
-    group_scan_kernel<DK, DELTA><<<n_seqs * A.H * parts, threads, std::max(2 * group_scan_buf_floats(DK) * sizeof(float), min_smem), st>>>(A, pool, o_raw);
+    plain_launch(group_scan_kernel<DK, DELTA>, n_seqs * A.H * parts, threads, std::max(2 * group_scan_buf_floats(DK) * sizeof(float), min_smem), st, A, pool, o_raw);
     return cudaGetLastError();
 }
 // The four-token scan: the group's products (not needed where every sequence brings one token), then the recurrence itself.
@@ -2617,7 +2693,7 @@ template <bool DELTA>
 static cudaError_t launch_group_scan_any(SmolLm* m, const GroupScanArgs& A, float* pairs, int n_seqs, int max_n, float* pool, float* o_raw, cudaStream_t st,
                                          size_t min_smem = 0) {
     if (max_n > 1) {
-        scan_pairs_kernel<DELTA><<<dim3((max_n + kScanGroup - 1) / kScanGroup, n_seqs, (A.G + 3) / 4), 128, 0, st>>>(A, pairs);
+        pdl_launch(scan_pairs_kernel<DELTA>, dim3((max_n + kScanGroup - 1) / kScanGroup, n_seqs, (A.G + 3) / 4), 128, 0, st, A, pairs);
         m->launches++;
     }
     m->launches++;
@@ -2650,7 +2726,7 @@ static void launch_attention(SmolLm* m, const SmolLmStep* s, AttnArgs& A, bool f
             const bf16* qb = reinterpret_cast<const bf16*>(qbuf);
             const bf16* pl = reinterpret_cast<const bf16*>(pool);
             bf16* mx = reinterpret_cast<bf16*>(mix);
-#define SMOL_FLASH(DK, DV, VK) attn_flash_kernel<DK, DV, VK, MAPS><<<grid, 128 * MAPS, flash_smem_bytes(DK, DV, VK, MAPS), st>>>(A, qb, pl, mx)
+#define SMOL_FLASH(DK, DV, VK) plain_launch(attn_flash_kernel<DK, DV, VK, MAPS>, grid, 128 * MAPS, flash_smem_bytes(DK, DV, VK, MAPS), st, A, qb, pl, mx)
             bool done = false;
             if constexpr (MAPS == 1) {
                 done = A.v_in_k != 0;
@@ -2669,7 +2745,7 @@ static void launch_attention(SmolLm* m, const SmolLmStep* s, AttnArgs& A, bool f
         } else {
             // every row, also those of short sequences
             const int au = Tn * A.H;
-            attn_kernel<T, MAXV, MAPS><<<(au + kAttnWarps - 1) / kAttnWarps, kAttnWarps * 32, kAttnWarps * A.d * sizeof(float), st>>>(A, qbuf, pool, mix);
+            plain_launch(attn_kernel<T, MAXV, MAPS>, (au + kAttnWarps - 1) / kAttnWarps, kAttnWarps * 32, kAttnWarps * A.d * sizeof(float), st, A, qbuf, pool, mix);
         }
         m->launches += 1;
     }
@@ -2683,10 +2759,10 @@ static void launch_attention(SmolLm* m, const SmolLmStep* s, AttnArgs& A, bool f
         bool wide = false;
         if constexpr (MAXV == 8) {
             wide = smem_of(64) <= (size_t)kAttnSplitWideSmem;
-            if (wide) attn_split_kernel<T, MAXV, 2><<<grid, nwarp * 32, smem_of(64), st>>>(A, qbuf, pool);
+            if (wide) pdl_launch(attn_split_kernel<T, MAXV, 2>, grid, nwarp * 32, smem_of(64), st, A, qbuf, pool);
         }
-        if (!wide) attn_split_kernel<T, MAXV, 1><<<grid, nwarp * 32, smem_of(32), st>>>(A, qbuf, pool);
-        attn_merge_kernel<T, MAXV, MAPS><<<A.short_rows * A.H, kMergeWarps * MAPS * 32, kMergeWarps * MAPS * (A.dv + 1) * sizeof(float), st>>>(A, mix);
+        if (!wide) pdl_launch(attn_split_kernel<T, MAXV, 1>, grid, nwarp * 32, smem_of(32), st, A, qbuf, pool);
+        pdl_launch(attn_merge_kernel<T, MAXV, MAPS>, A.short_rows * A.H, kMergeWarps * MAPS * 32, kMergeWarps * MAPS * (A.dv + 1) * sizeof(float), st, A, mix);
         m->launches += 2;
     }
 }
@@ -2701,11 +2777,11 @@ template <int DK, int HPW>
 static bool launch_sigmoid_flash_sized(const SigmoidArgs& S, dim3 grid, int threads, const bf16* qbuf, const bf16* pool, bf16* out, cudaStream_t st) {
     const AttnArgs& A = S.a;
     if (sigmoid_flash_smem(A.H, A.G, DK, 64) <= (size_t)kSigmoidSmemMax) {
-        sigmoid_flash_kernel<DK, HPW, 64><<<grid, threads, sigmoid_flash_smem(A.H, A.G, DK, 64), st>>>(S, qbuf, pool, out);
+        pdl_launch(sigmoid_flash_kernel<DK, HPW, 64>, grid, threads, sigmoid_flash_smem(A.H, A.G, DK, 64), st, S, qbuf, pool, out);
         return true;
     }
     if (sigmoid_flash_smem(A.H, A.G, DK, 32) <= (size_t)kSigmoidSmemMax) {
-        sigmoid_flash_kernel<DK, HPW, 32><<<grid, threads, sigmoid_flash_smem(A.H, A.G, DK, 32), st>>>(S, qbuf, pool, out);
+        pdl_launch(sigmoid_flash_kernel<DK, HPW, 32>, grid, threads, sigmoid_flash_smem(A.H, A.G, DK, 32), st, S, qbuf, pool, out);
         return true;
     }
     return false;
@@ -2742,7 +2818,7 @@ static bool launch_sigmoid_flash(SmolLm* m, const SmolLmStep* s, SigmoidArgs& S,
         else done = false;
     }
     if (done && S.n_ranges > 1) {
-        sigmoid_merge_kernel<<<A.n_tokens, 128, 0, st>>>(S, out);
+        pdl_launch(sigmoid_merge_kernel, A.n_tokens, 128, 0, st, S, out);
         m->launches += 1;
     }
     if (done) m->launches += 1;
@@ -2755,8 +2831,8 @@ static void launch_residual_norm(const ResidualArgs& A, int rows, int threads, T
     for (const void* p : {(const void*)A.x, (const void*)A.y, (const void*)A.y2, (const void*)A.y_w, (const void*)A.y2_w, (const void*)A.rs.yp, (const void*)A.trace,
                           (const void*)A.x0, (const void*)A.cat, (const void*)A.y_b, (const void*)A.next.w, (const void*)A.next.shift, (const void*)hn})
         at |= reinterpret_cast<uintptr_t>(p);
-    if (A.D % 4 == 0 && at % 16 == 0) residual_norm_kernel<T, true><<<rows, threads, A.D * sizeof(float), st>>>(A, hn);
-    else residual_norm_kernel<T, false><<<rows, threads, A.D * sizeof(float), st>>>(A, hn);
+    if (A.D % 4 == 0 && at % 16 == 0) pdl_launch(residual_norm_kernel<T, true>, rows, threads, A.D * sizeof(float), st, A, hn);
+    else pdl_launch(residual_norm_kernel<T, false>, rows, threads, A.D * sizeof(float), st, A, hn);
 }
 
 template <class T>
@@ -2797,16 +2873,16 @@ static int step_impl(SmolLm* m, const SmolLmStep* s, cudaStream_t st) {
     auto cast_grid = [](size_t n) { return (int)std::min<size_t>((n + 255) / 256, 148 * 8); };
 
     if (postnorm) {
-        embed_gain_norm_kernel<T><<<Tn, nthr, 0, st>>>(s->tokens, static_cast<const T*>(m->g.embed), D, c.vocab, m->g.embed_norm, c.norm_eps, x, hist, hn);
+        pdl_launch(embed_gain_norm_kernel<T>, Tn, nthr, 0, st, s->tokens, static_cast<const T*>(m->g.embed), D, c.vocab, m->g.embed_norm, c.norm_eps, x, hist, hn);
     } else if (outnorm) {
-        embed_prenorm_kernel<T><<<Tn, nthr, 0, st>>>(s->tokens, static_cast<const T*>(m->g.embed), c.embed_scale, D, c.vocab, copy_row, x, nullptr, hn, nullptr);
+        pdl_launch(embed_prenorm_kernel<T>, Tn, nthr, 0, st, s->tokens, static_cast<const T*>(m->g.embed), c.embed_scale, D, c.vocab, copy_row, x, nullptr, hn, nullptr);
     } else if (prenorm || parallel) {
         const SmolLmLayer& L0 = m->layers[m->runs[0].layer];
         const bool merge = m->runs[0].flags & SMOL_LM_RUN_MERGE_EMBED;
-        embed_prenorm_kernel<T><<<Tn, nthr, 0, st>>>(s->tokens, static_cast<const T*>(m->g.embed), c.embed_scale, D, c.vocab,
+        pdl_launch(embed_prenorm_kernel<T>, Tn, nthr, 0, st, s->tokens, static_cast<const T*>(m->g.embed), c.embed_scale, D, c.vocab,
                                                      merge ? no_norm : norm_of(L0.norm1, L0.norm1_shift, L0.norm1_alpha), x, x0, hn, cat);
     } else {
-        embed_norm_kernel<T><<<Tn, nthr, 0, st>>>(s->tokens, static_cast<const T*>(m->g.embed), c.embed_scale, D, c.vocab,
+        pdl_launch(embed_norm_kernel<T>, Tn, nthr, 0, st, s->tokens, static_cast<const T*>(m->g.embed), c.embed_scale, D, c.vocab,
                                                   m->layers[m->runs[0].layer].norm1, c.norm_eps, x, hn, woff);
     }
     m->launches++;
@@ -2817,7 +2893,7 @@ static int step_impl(SmolLm* m, const SmolLmStep* s, cudaStream_t st) {
         if (R.flags & SMOL_LM_RUN_MERGE_EMBED) {
             // the stream starts anew from the merged rows, which the previous run's last kernel (or the embedding) has left in cat
             CU(linear<T>(m, cat, static_cast<const T*>(m->g.w_merge), x, Tn, D, 2 * D, st));
-            prenorm_rows_kernel<T><<<Tn, nthr, 0, st>>>(x, nullptr, norm_of(L.norm1, L.norm1_shift, L.norm1_alpha), D, hn);
+            pdl_launch(prenorm_rows_kernel<T>, Tn, nthr, 0, st, x, nullptr, norm_of(L.norm1, L.norm1_shift, L.norm1_alpha), D, hn);
             m->launches++;
         }
         CU(linear<T>(m, hn, static_cast<const T*>(L.w_in), proj, Tn, n_in, D, st));
@@ -2849,11 +2925,11 @@ static int step_impl(SmolLm* m, const SmolLmStep* s, cudaStream_t st) {
                 const int threads = Tn > 64 ? 128 : 256;      // few tokens: more loads in flight per token
                 A.rot_pairs = M.rot_dims / 2; A.rot_half = M.rot_half; A.rot_mult = M.rot_mult != 0.0f ? M.rot_mult : 1.0f;
                 A.freq = reinterpret_cast<const float*>(m->ws + m->o_freq) + Ri.freq_off;
-                if (A.rot_pairs > 0) attn_prep_whole_kernel<T, true><<<Tn, threads, 0, ms>>>(A, qbuf, pool);
-                else attn_prep_whole_kernel<T, false><<<Tn, threads, 0, ms>>>(A, qbuf, pool);
+                if (A.rot_pairs > 0) pdl_launch(attn_prep_whole_kernel<T, true>, Tn, threads, 0, ms, A, qbuf, pool);
+                else pdl_launch(attn_prep_whole_kernel<T, false>, Tn, threads, 0, ms, A, qbuf, pool);
             } else {
                 const int units = Tn * (M.heads * A.maps + (A.own_kv ? M.kv_heads * (A.maps + 1) : 0));
-                attn_prep_kernel<T><<<(units + 3) / 4, 128, 0, ms>>>(A, qbuf, pool);
+                pdl_launch(attn_prep_kernel<T>, (units + 3) / 4, 128, 0, ms, A, qbuf, pool);
             }
             m->launches += 1;
             const bool flash = sizeof(T) == 2 && std::max(M.dim, M.vdim) <= 128;
@@ -2876,7 +2952,7 @@ static int step_impl(SmolLm* m, const SmolLmStep* s, cudaStream_t st) {
             P.slot_floats = m->slot_floats; P.conv_off = Ri.conv_off; P.n_slots = m->n_slots; P.err = err;
             P.out_ld = out_ld_now; P.out_scale = M.mix_scale;
             const dim3 cgrid(Tn, (ch + 127) / 128);
-            ssd_conv_kernel<<<cgrid, 128, 0, ms>>>(P, m->slots, conv, head);
+            pdl_launch(ssd_conv_kernel, cgrid, 128, 0, ms, P, m->slots, conv, head);
             GlaArgs A;
             A.proj = pj; A.n_in = n_in; A.H = M.heads; A.d = M.n_state; A.dv = M.vdim; A.rank = 0; A.n_tokens = Tn;
             A.q_scale = 1.0f; A.tau = 1.0f; A.eps = c.norm_eps;
@@ -2889,7 +2965,7 @@ static int step_impl(SmolLm* m, const SmolLmStep* s, cudaStream_t st) {
             A.head_decay = head; A.head_step = head + (size_t)Tn * M.heads; A.head_ld = M.heads;
             A.out_ld = out_ld_now; A.out_scale = 1.0f;
             CU(launch_gla_scan_any(m, A, s->n_seqs, max_n, nullptr, m->slots, oraw, ms));
-            ssd_out_kernel<T><<<dim3(Tn, M.norm_parts), 256, 0, ms>>>(P, oraw, conv, mix_at, m->slots);
+            pdl_launch(ssd_out_kernel<T>, dim3(Tn, M.norm_parts), 256, 0, ms, P, oraw, conv, mix_at, m->slots);
             m->launches += 3;
             return SMOL_OK;
         };
@@ -2915,7 +2991,7 @@ static int step_impl(SmolLm* m, const SmolLmStep* s, cudaStream_t st) {
             S.range_len = 1 << 30; S.n_ranges = 1; S.partial = nullptr;
             S.freq = reinterpret_cast<const float*>(m->ws + m->o_freq) + Ri.freq_off;
             const int units = Tn * (M.heads + M.kv_heads);
-            sigmoid_prep_kernel<T><<<(units + 3) / 4, 128, 0, ms>>>(S, qbuf, pool);
+            pdl_launch(sigmoid_prep_kernel<T>, (units + 3) / 4, 128, 0, ms, S, qbuf, pool);
             m->launches += 1;
             const int min_n = s->min_seq_tokens > 0 ? s->min_seq_tokens : 1;
             // sequences that bring more than a few tokens take the tiled tensor-core form (bf16), the others a warp per head
@@ -2932,9 +3008,9 @@ static int step_impl(SmolLm* m, const SmolLmStep* s, cudaStream_t st) {
                 A.n_splits = std::min(m->max_splits, (max_pos / m->split_len + 4) / 4 * 4);
                 if (M.chunk > 0) A.n_splits = std::min(A.n_splits, ((M.chunk - 1) / m->split_len + 2 + 3) / 4 * 4);      // ranges a chunk can touch
                 const dim3 grid(A.short_rows, A.n_splits);
-                if (M.vdim <= 256) sigmoid_split_kernel<T, 8><<<grid, M.heads * 32, split_smem, ms>>>(S, qbuf, pool);
-                else sigmoid_split_kernel<T, 16><<<grid, M.heads * 32, split_smem, ms>>>(S, qbuf, pool);
-                sigmoid_short_merge_kernel<T><<<A.short_rows, 128, 0, ms>>>(S, mix_at);
+                if (M.vdim <= 256) pdl_launch(sigmoid_split_kernel<T, 8>, grid, M.heads * 32, split_smem, ms, S, qbuf, pool);
+                else pdl_launch(sigmoid_split_kernel<T, 16>, grid, M.heads * 32, split_smem, ms, S, qbuf, pool);
+                pdl_launch(sigmoid_short_merge_kernel<T>, A.short_rows, 128, 0, ms, S, mix_at);
                 m->launches += 2;
             }
             const bool long_left = max_n > kShortSeq && !tiled, short_left = min_n <= kShortSeq && !split;
@@ -2942,8 +3018,8 @@ static int step_impl(SmolLm* m, const SmolLmStep* s, cudaStream_t st) {
                 // the warp-per-head form: every row, or only the rows the other two forms left
                 S.only = (long_left && short_left) ? 0 : long_left ? 1 : 2;
                 const size_t smem = ((size_t)M.heads * (M.dim + 32) + (size_t)M.heads * M.heads) * sizeof(float);
-                if (M.vdim <= 256) sigmoid_attn_kernel<T, 8><<<Tn, M.heads * 32, smem, ms>>>(S, qbuf, pool, mix_at);
-                else sigmoid_attn_kernel<T, 16><<<Tn, M.heads * 32, smem, ms>>>(S, qbuf, pool, mix_at);
+                if (M.vdim <= 256) pdl_launch(sigmoid_attn_kernel<T, 8>, Tn, M.heads * 32, smem, ms, S, qbuf, pool, mix_at);
+                else pdl_launch(sigmoid_attn_kernel<T, 16>, Tn, M.heads * 32, smem, ms, S, qbuf, pool, mix_at);
                 m->launches += 1;
             }
             return SMOL_OK;
@@ -2964,14 +3040,14 @@ static int step_impl(SmolLm* m, const SmolLmStep* s, cudaStream_t st) {
         auto lightning = [&](const SmolLmLayer& M, const RunInfo& Ri, const float* pj, T* mix_at, int ld) -> int {
             const int hd = M.heads * M.dim, hv = M.heads * M.vdim, na = 2 * hd + hv;
             LinPrepArgs P{pj, n_in, M.heads, M.dim, M.vdim, Tn, M.head_decay, nullptr, nullptr};
-            lightning_prep_kernel<<<dim3(Tn, (na + 1023) / 1024), 256, 0, ms>>>(P, conv, head);
+            pdl_launch(lightning_prep_kernel, dim3(Tn, (na + 1023) / 1024), 256, 0, ms, P, conv, head);
             GlaArgs A = scan_args(M, Ri, pj);
             A.q_src = conv; A.k_src = conv + hd; A.v_src = conv + 2 * hd;
             A.q_ld = A.k_ld = A.v_ld = na;
             A.head_decay = head; A.head_step = head + (size_t)Tn * M.heads;
             CU(launch_gla_scan_any(m, A, s->n_seqs, max_n, nullptr, m->slots, oraw, ms));
             LinOutArgs O{pj, n_in, hv, hv, hv, 1, ld, (size_t)2 * hd + hv, c.norm_eps, 1.0f, M.out_norm};
-            lin_attn_out_kernel<T><<<dim3(Tn, 1), 256, 0, ms>>>(O, oraw, mix_at);
+            pdl_launch(lin_attn_out_kernel<T>, dim3(Tn, 1), 256, 0, ms, O, oraw, mix_at);
             m->launches += 3;
             return SMOL_OK;
         };
@@ -2979,14 +3055,14 @@ static int step_impl(SmolLm* m, const SmolLmStep* s, cudaStream_t st) {
         auto retention = [&](const SmolLmLayer& M, const RunInfo& Ri, const float* pj, T* mix_at, int ld) -> int {
             const int hd = M.heads * M.dim, pairs = M.rot_dims / 2, per = M.heads * (M.dim - pairs);
             RetentionArgs P{pj, n_in, M.heads, M.dim, pairs, M.rot_half, M.score_scale, reinterpret_cast<const float*>(m->ws + m->o_freq) + Ri.freq_off, s->tok_pos};
-            retention_prep_kernel<<<dim3(Tn, (per + 511) / 512), 128, 0, ms>>>(P, conv);
+            pdl_launch(retention_prep_kernel, dim3(Tn, (per + 511) / 512), 128, 0, ms, P, conv);
             GlaArgs A = scan_args(M, Ri, pj);
             A.q_src = conv; A.k_src = conv + hd; A.v_src = pj + 2 * hd;
             A.q_ld = A.k_ld = 2 * hd; A.v_ld = n_in;
             A.head_decay = M.head_decay; A.head_ld = 0;
             CU(launch_gla_scan_any(m, A, s->n_seqs, max_n, nullptr, m->slots, oraw, ms, parallel && Tn > kGraphMaxTokens ? kScanSpread : 0));
             A.out_ld = ld; A.out_scale = M.mix_scale;
-            gla_out_kernel<T><<<(Tn * M.heads + 3) / 4, 128, 0, ms>>>(A, oraw, mix_at);
+            pdl_launch(gla_out_kernel<T>, (Tn * M.heads + 3) / 4, 128, 0, ms, A, oraw, mix_at);
             m->launches += 3;
             return SMOL_OK;
         };
@@ -3011,7 +3087,7 @@ static int step_impl(SmolLm* m, const SmolLmStep* s, cudaStream_t st) {
             P.tok_seq = s->tok_seq; P.err = err;
             P.conv = ConvIo{pj, nullptr, n_in, ch, M.conv_taps, M.conv_w, nullptr, s->seq_start, s->seq_pos0, s->seq_slot, m->slot_floats, Ri.conv_off, m->n_slots};
             const int warps = M.kv_heads + (hv + kGatedDeltaCols - 1) / kGatedDeltaCols;
-            gated_delta_prep_kernel<<<dim3(Tn, (warps + 3) / 4), 128, 0, ms>>>(P, m->slots, conv, head, pairs);
+            pdl_launch(gated_delta_prep_kernel, dim3(Tn, (warps + 3) / 4), 128, 0, ms, P, m->slots, conv, head, pairs);
             GroupScanArgs S = group_args(M, Ri, M.kv_heads);
             S.q_src = conv; S.k_src = conv + gd; S.v_src = conv + 2 * gd;
             S.q_ld = S.k_ld = S.v_ld = ch;
@@ -3019,7 +3095,7 @@ static int step_impl(SmolLm* m, const SmolLmStep* s, cudaStream_t st) {
             CU(launch_group_scan_any<true>(m, S, pairs, s->n_seqs, max_n, m->slots, oraw, ms));
             GlaArgs A = scan_args(M, Ri, pj);
             A.out_norm = M.out_norm; A.gate_off = ch; A.out_ld = ld; A.out_scale = M.mix_scale;
-            gla_out_kernel<T><<<(Tn * M.heads + 3) / 4, 128, 0, ms>>>(A, oraw, mix_at);
+            pdl_launch(gla_out_kernel<T>, (Tn * M.heads + 3) / 4, 128, 0, ms, A, oraw, mix_at);
             m->launches += 2;
             return SMOL_OK;
         };
@@ -3034,7 +3110,7 @@ static int step_impl(SmolLm* m, const SmolLmStep* s, cudaStream_t st) {
             P.i_bias = M.rate_bias; P.f_bias = M.decay_bias;
             P.seq_start = s->seq_start; P.seq_pos0 = s->seq_pos0; P.seq_slot = s->seq_slot;
             P.slot_floats = m->slot_floats; P.m_off = Ri.m_off; P.n_slots = m->n_slots; P.err = err;
-            mlstm_gate_kernel<<<s->n_seqs * M.heads, std::min(kMlstmTile, (max_n + 31) / 32 * 32), 0, ms>>>(P, m->slots, head, floor_at, pairs);
+            pdl_launch(mlstm_gate_kernel, s->n_seqs * M.heads, std::min(kMlstmTile, (max_n + 31) / 32 * 32), 0, ms, P, m->slots, head, floor_at, pairs);
             GroupScanArgs S = group_args(M, Ri, M.heads);
             S.q_src = pj; S.k_src = pj + hd; S.v_src = pj + 2 * hd;
             S.q_ld = S.k_ld = S.v_ld = n_in;
@@ -3044,7 +3120,7 @@ static int step_impl(SmolLm* m, const SmolLmStep* s, cudaStream_t st) {
             GlaArgs A = scan_args(M, Ri, pj);
             A.den = den; A.den_floor = floor_at; A.den_eps = M.den_eps;
             A.out_norm = M.out_norm; A.norm_own = 1; A.gate_sigmoid = 1; A.out_ld = ld; A.out_scale = M.mix_scale;
-            gla_out_kernel<T><<<(Tn * M.heads + 3) / 4, 128, 0, ms>>>(A, oraw, mix_at);
+            pdl_launch(gla_out_kernel<T>, (Tn * M.heads + 3) / 4, 128, 0, ms, A, oraw, mix_at);
             m->launches += 2;
             return SMOL_OK;
         };
@@ -3068,12 +3144,12 @@ static int step_impl(SmolLm* m, const SmolLmStep* s, cudaStream_t st) {
         auto feed_forward = [&](cudaStream_t st) -> int {
             if (L.mlp == SMOL_LM_MLP_POLYNORM) {
                 CU(linear<T>(m, hn, static_cast<const T*>(L.w_up), z, Tn, L.ff, D, st));
-                polynorm_kernel<T><<<Tn, 256, 0, st>>>(z, L.act, c.norm_eps, L.ff, act);
+                pdl_launch(polynorm_kernel<T>, Tn, 256, 0, st, z, L.act, c.norm_eps, L.ff, act);
                 CU(linear<T>(m, act, static_cast<const T*>(L.w_down), y, Tn, D, L.ff, st));
                 m->launches += 1;
             } else if (L.mlp == SMOL_LM_MLP_GATED) {
                 CU(linear<T>(m, hn, static_cast<const T*>(L.w_up), z, Tn, 2 * L.ff, D, st));
-                gated_act_kernel<T><<<cast_grid((size_t)Tn * L.ff / 4), 256, 0, st>>>(z, L.ff, actp_of(L), (size_t)Tn, act);
+                pdl_launch(gated_act_kernel<T>, cast_grid((size_t)Tn * L.ff / 4), 256, 0, st, z, L.ff, actp_of(L), (size_t)Tn, act);
                 CU(linear<T>(m, act, static_cast<const T*>(L.w_down), y, Tn, D, L.ff, st));
                 m->launches += 1;
             } else if (L.mlp == SMOL_LM_MLP_EXPERTS) {
@@ -3110,8 +3186,8 @@ static int step_impl(SmolLm* m, const SmolLmStep* s, cudaStream_t st) {
                     Rt.unit_out = mix + mix_cols_of(L); Rt.unit_ff = L.shared_ff; Rt.unit_ld = mix_ld;
                 }
                 const dim3 rgrid(Tn, parallel ? 1 : (Rt.E + 3) / 4);
-                if (postnorm) moe_route_kernel<float><<<rgrid, 128, 0, st>>>(Rt, x, r_logits, r_done, sel_id, sel_w);
-                else moe_route_kernel<T><<<rgrid, 128, 0, st>>>(Rt, hn, r_logits, r_done, sel_id, sel_w);
+                if (postnorm) pdl_launch(moe_route_kernel<float>, rgrid, 128, 0, st, Rt, x, r_logits, r_done, sel_id, sel_w);
+                else pdl_launch(moe_route_kernel<T>, rgrid, 128, 0, st, Rt, hn, r_logits, r_done, sel_id, sel_w);
                 m->launches += 1;
                 if (L.n_experts > 0) {
                     // three forms of the two grouped products, by how many rows an expert gets: a warp per output column for
@@ -3121,7 +3197,7 @@ static int step_impl(SmolLm* m, const SmolLmStep* s, cudaStream_t st) {
                                      NF >= kTcMinCols && D >= kTcMinCols && D >= smol::umma::kBK && L.ff >= smol::umma::kBK;
                     const int tile_rows = big ? smol::umma::kM : kGroupTile;
                     if (!direct) {
-                        moe_index_kernel<<<1, 256, 0, st>>>(sel_id, pairs, L.n_experts, tile_rows, seg, perm, slot_of, tile_g, tile_r, n_tiles);
+                        pdl_launch(moe_index_kernel, 1, 256, 0, st, sel_id, pairs, L.n_experts, tile_rows, seg, perm, slot_of, tile_g, tile_r, n_tiles);
                         m->launches++;
                     }
                     const int tiles = pairs / kGroupTile + L.n_experts;
@@ -3136,22 +3212,22 @@ static int step_impl(SmolLm* m, const SmolLmStep* s, cudaStream_t st) {
                     // its weight, and the products read that copy
                     T* ap = reinterpret_cast<T*>(m->ws + m->o_ap);
                     if (L.route_input) {
-                        moe_gather_scaled_kernel<T><<<pairs, 128, 0, st>>>(hn, perm, L.top_k, sel_w, seg + L.n_experts, D, ap);
+                        pdl_launch(moe_gather_scaled_kernel<T>, pairs, 128, 0, st, hn, perm, L.top_k, sel_w, seg + L.n_experts, D, ap);
                         m->launches++;
                     }
                     if (few) {
-                        moe_gemv_kernel<false><<<dim3((NF + 7) / 8, pairs), 256, 0, st>>>(L.route_input ? ap : hn, perm, L.route_input ? 0 : L.top_k, sel_id,
+                        pdl_launch(moe_gemv_kernel<false>, dim3((NF + 7) / 8, pairs), 256, 0, st, L.route_input ? ap : hn, perm, L.route_input ? 0 : L.top_k, sel_id,
                                                                                          seg + L.n_experts, reinterpret_cast<const bf16*>(L.w_experts_in), io.sw,
                                                                                          zp, NF, D, expert_actp(L));
                         // the second product applies the activation as it reads the first one's result
-                        moe_gemv_kernel<true><<<dim3((D + 7) / 8, pairs), 256, L.ff * sizeof(bf16), st>>>(zp, perm, 0, sel_id, seg + L.n_experts,
+                        pdl_launch(moe_gemv_kernel<true>, dim3((D + 7) / 8, pairs), 256, L.ff * sizeof(bf16), st, zp, perm, 0, sel_id, seg + L.n_experts,
                                                                                         reinterpret_cast<const bf16*>(L.w_experts_out), io2.sw, yp, D, L.ff, expert_actp(L));
                         m->launches += 1;
                     } else {
                         bool done = false;
                         if (big) {
                             if (!L.route_input) {
-                                moe_gather_kernel<<<pairs, 128, 0, st>>>(reinterpret_cast<const bf16*>(hn), perm, L.top_k, seg + L.n_experts, D,
+                                pdl_launch(moe_gather_kernel, pairs, 128, 0, st, reinterpret_cast<const bf16*>(hn), perm, L.top_k, seg + L.n_experts, D,
                                                                          reinterpret_cast<bf16*>(ap));
                                 m->launches++;
                             }
@@ -3162,7 +3238,7 @@ static int step_impl(SmolLm* m, const SmolLmStep* s, cudaStream_t st) {
                             if (!L.route_input) { io.gather = perm; io.gather_div = L.top_k; }
                             CU(linear_ex<T>(m, L.route_input ? ap : hn, static_cast<const T*>(L.w_experts_in), zp, pairs, NF, D, io, 1, tiles, st));
                         }
-                        gated_act_kernel<T><<<cast_grid(act_n / 4), 256, 0, st>>>(zp, L.ff, expert_actp(L), (size_t)pairs, actp);
+                        pdl_launch(gated_act_kernel<T>, cast_grid(act_n / 4), 256, 0, st, zp, L.ff, expert_actp(L), (size_t)pairs, actp);
                         if (!(big && linear_grouped_tc(m, reinterpret_cast<const bf16*>(actp), reinterpret_cast<const bf16*>(L.w_experts_out), yp, pairs,
                                                        L.n_experts, D, L.ff, io2, st)))
                             CU(linear_ex<T>(m, actp, static_cast<const T*>(L.w_experts_out), yp, pairs, D, L.ff, io2, 1, tiles, st));
@@ -3175,7 +3251,7 @@ static int step_impl(SmolLm* m, const SmolLmStep* s, cudaStream_t st) {
                     // the expert every token uses: its result lands in y and joins the routed sum in the kernel that follows
                     const int SF = L.ff_plain ? L.shared_ff : 2 * L.shared_ff;
                     CU(linear<T>(m, hn, static_cast<const T*>(L.w_shared_in), z, Tn, SF, D, st));
-                    gated_act_kernel<T><<<cast_grid((size_t)Tn * L.shared_ff / 4), 256, 0, st>>>(z, L.shared_ff, expert_actp(L), (size_t)Tn, act);
+                    pdl_launch(gated_act_kernel<T>, cast_grid((size_t)Tn * L.shared_ff / 4), 256, 0, st, z, L.shared_ff, expert_actp(L), (size_t)Tn, act);
                     CU(linear<T>(m, act, static_cast<const T*>(L.w_shared_out), y, Tn, D, L.shared_ff, st));
                     m->launches += 1;
                 }
@@ -3189,7 +3265,7 @@ static int step_impl(SmolLm* m, const SmolLmStep* s, cudaStream_t st) {
         if (parallel && L.mlp != SMOL_LM_MLP_NONE) {
             if (beside) {
                 CU(cudaEventRecord(m->ff_start, st));
-                CU(cudaStreamWaitEvent(m->ff_stream, m->ff_start, 0));
+                CU(wait_event(m->ff_stream, m->ff_start));
             }
             const int rc = feed_forward(beside ? m->ff_stream : st);
             if (rc != SMOL_OK) return rc;
@@ -3207,7 +3283,7 @@ static int step_impl(SmolLm* m, const SmolLmStep* s, cudaStream_t st) {
             };
             if (fork) {
                 CU(cudaEventRecord(m->ff_start, st));
-                CU(cudaStreamWaitEvent(m->ff_stream, m->ff_start, 0));
+                CU(wait_event(m->ff_stream, m->ff_start));
                 ms = m->ff_stream;
                 rc = run_side();
                 CU(cudaEventRecord(m->ff_done, m->ff_stream));
@@ -3215,20 +3291,20 @@ static int step_impl(SmolLm* m, const SmolLmStep* s, cudaStream_t st) {
             }
             if (rc == SMOL_OK) rc = run_mixer(L, R, proj, L.in_bias, mix, own_proj ? mix_cols_of(L) : mix_ld);
             if (rc == SMOL_OK && L.side && !fork) rc = run_side();
-            if (rc == SMOL_OK && fork) CU(cudaStreamWaitEvent(st, m->ff_done, 0));
+            if (rc == SMOL_OK && fork) CU(wait_event(st, m->ff_done));
             if (rc != SMOL_OK) return rc;
             mix_cols = own_proj ? mix_cols_of(L) : mix_ld;
         } else if (L.mixer == SMOL_LM_MIX_HGRN2) {
             // q = silu(.), decay = the bounded forget gate, key = 1 - decay; norm per head, no gate
             const int hd = L.heads * L.dim, hv = L.heads * L.vdim;
             LinPrepArgs P{proj, n_in, L.heads, L.dim, L.vdim, Tn, nullptr, L.rate_bias, L.forget_lower};
-            hgrn2_prep_kernel<<<dim3(Tn, (hd + 1023) / 1024), 256, 0, st>>>(P, uk, auk, dec);
+            pdl_launch(hgrn2_prep_kernel, dim3(Tn, (hd + 1023) / 1024), 256, 0, st, P, uk, auk, dec);
             GlaArgs A = scan_args(L, R, proj);
             A.q_src = uk; A.k_src = auk; A.v_src = proj + 2 * hd;
             A.q_ld = A.k_ld = hd; A.v_ld = n_in;
             CU(launch_gla_scan_any(m, A, s->n_seqs, max_n, dec, m->slots, oraw, st));
             LinOutArgs O{proj, n_in, hv, L.vdim, L.vdim, 0, hv, 0, c.norm_eps, 1.0f, L.out_norm};
-            lin_attn_out_kernel<T><<<dim3(Tn, L.heads), 128, 0, st>>>(O, oraw, mix);
+            pdl_launch(lin_attn_out_kernel<T>, dim3(Tn, L.heads), 128, 0, st, O, oraw, mix);
             m->launches += 3;
             mix_cols = hv;
         } else if (L.mixer == SMOL_LM_MIX_LATENT_ATTENTION) {
@@ -3251,7 +3327,7 @@ static int step_impl(SmolLm* m, const SmolLmStep* s, cudaStream_t st) {
                 P.tok_seq = s->tok_seq; P.tok_pos = s->tok_pos; P.block_table = s->block_table;
                 P.max_pages = s->max_pages; P.page_size = c.page_size; P.n_pages = m->n_pages; P.n_tokens = Tn;
                 P.page_elems = m->page_elems; P.k_off = R.k_off; P.err = err;
-                latent_prep_kernel<T><<<Tn, 128, 0, st>>>(P, cq, pool);
+                pdl_launch(latent_prep_kernel<T>, Tn, 128, 0, st, P, cq, pool);
                 CU(linear<T>(m, cq, static_cast<const T*>(L.w_q_up), qf, Tn, L.heads * qw, L.q_rank, st));
                 // per head: the unrotated query [Tn, dim] times the transposed key expansion [kv_rank, dim]^T, written where
                 // the attention reads its queries (bf16 engine: read from the fp32 q, written in bf16)
@@ -3261,7 +3337,7 @@ static int step_impl(SmolLm* m, const SmolLmStep* s, cudaStream_t st) {
                 io.a_f32 = io.y_bf16 = kIsF32 ? 0 : 1;
                 CU(linear_ex<T>(m, reinterpret_cast<const T*>(qf), static_cast<const T*>(L.w_k_up_t), reinterpret_cast<float*>(qbuf), Tn, L.kv_rank,
                                 L.dim, io, L.heads, 0, st));
-                latent_query_kernel<T><<<(Tn * L.heads + 3) / 4, 128, 0, st>>>(P, qf, qbuf);
+                pdl_launch(latent_query_kernel<T>, (Tn * L.heads + 3) / 4, 128, 0, st, P, qf, qbuf);
                 m->launches += 2;
                 A.G = 1; A.d = dk; A.dv = L.kv_rank;
                 A.k_ld = dk; A.v_ld = dk; A.v_in_k = 1;
@@ -3290,10 +3366,10 @@ static int step_impl(SmolLm* m, const SmolLmStep* s, cudaStream_t st) {
             gla_sources_from_proj(A);
             const int slices = (L.heads * L.dim + 127) / 128;
             if (Tn >= kDecayMinTokens && kDecayTokens * L.rank * sizeof(float) <= 48 * 1024)
-                gla_prep_kernel<kDecayTokens><<<dim3((Tn + kDecayTokens - 1) / kDecayTokens, slices), 128, kDecayTokens * L.rank * sizeof(float), st>>>(A, dec);
-            else gla_prep_kernel<1><<<dim3(Tn, slices), 128, L.rank * sizeof(float), st>>>(A, dec);
+                pdl_launch(gla_prep_kernel<kDecayTokens>, dim3((Tn + kDecayTokens - 1) / kDecayTokens, slices), 128, kDecayTokens * L.rank * sizeof(float), st, A, dec);
+            else pdl_launch(gla_prep_kernel<1>, dim3(Tn, slices), 128, L.rank * sizeof(float), st, A, dec);
             CU(launch_gla_scan_any(m, A, s->n_seqs, max_n, dec, m->slots, oraw, st));
-            gla_out_kernel<T><<<(Tn * L.heads + 3) / 4, 128, 0, st>>>(A, oraw, mix);
+            pdl_launch(gla_out_kernel<T>, (Tn * L.heads + 3) / 4, 128, 0, st, A, oraw, mix);
             m->launches += 3;
             mix_cols = L.heads * L.vdim;
         } else {
@@ -3308,8 +3384,8 @@ static int step_impl(SmolLm* m, const SmolLmStep* s, cudaStream_t st) {
             const size_t prep_smem = (size_t)(L.rank + L.heads) * sizeof(float);
             const int slices = (L.heads * L.dim + 127) / 128;
             if (Tn >= kDecayMinTokens && kDecayTokens * prep_smem <= 48 * 1024)
-                delta_prep_kernel<kDecayTokens><<<dim3((Tn + kDecayTokens - 1) / kDecayTokens, slices), 128, kDecayTokens * prep_smem, st>>>(A, dec, u_to, au_to);
-            else delta_prep_kernel<1><<<dim3(Tn, slices), 128, prep_smem, st>>>(A, dec, u_to, au_to);
+                pdl_launch(delta_prep_kernel<kDecayTokens>, dim3((Tn + kDecayTokens - 1) / kDecayTokens, slices), 128, kDecayTokens * prep_smem, st, A, dec, u_to, au_to);
+            else pdl_launch(delta_prep_kernel<1>, dim3(Tn, slices), 128, prep_smem, st, A, dec, u_to, au_to);
             cudaError_t e;
             if (quad) {
                 const int HD = L.heads * L.dim;
@@ -3322,11 +3398,11 @@ static int step_impl(SmolLm* m, const SmolLmStep* s, cudaStream_t st) {
             else if (L.dim <= 128) e = launch_scan<128>(A, s->n_seqs, dec, uk, auk, m->slots, oraw, st);
             else e = launch_scan<256>(A, s->n_seqs, dec, uk, auk, m->slots, oraw, st);
             CU(e);
-            delta_out_kernel<T><<<(Tn * L.heads + 3) / 4, 128, 0, st>>>(A, oraw, mix);
+            pdl_launch(delta_out_kernel<T>, (Tn * L.heads + 3) / 4, 128, 0, st, A, oraw, mix);
             m->launches += 3;
             mix_cols = L.heads * L.dim;
         }
-        if (beside) CU(cudaStreamWaitEvent(st, m->ff_done, 0));      // also: w_out covers the shared expert's unit
+        if (beside) CU(wait_event(st, m->ff_done));      // also: w_out covers the shared expert's unit
         CU(linear<T>(m, mix_in, static_cast<const T*>(L.w_out), y, Tn, D, mix_cols, st));
         if (own_proj) CU(linear<T>(m, mix2, static_cast<const T*>(L.side->w_out), y2, Tn, D, mix_cols_of(*L.side), st));
         const bool last = n + 1 == m->runs.size();
@@ -3398,38 +3474,38 @@ static int step_impl(SmolLm* m, const SmolLmStep* s, cudaStream_t st) {
             // x <- g1 * rms_divide(alpha x + mixer); x <- g2 * rms_divide(alpha x + ff); the layer's result joins the history
             // and the stream becomes the weighted sum of the history
             const bool has_ff = L.mlp != SMOL_LM_MLP_NONE;
-            post_norm_kernel<T><<<Tn, nthr, 2 * D * sizeof(float), st>>>(x, y, c.residual_alpha, L.norm1, c.norm_eps, D, has_ff ? nullptr : hist,
+            pdl_launch(post_norm_kernel<T>, Tn, nthr, 2 * D * sizeof(float), st, x, y, c.residual_alpha, L.norm1, c.norm_eps, D, has_ff ? nullptr : hist,
                                                                       hist_stride, (int)n + 2, L.depth_mix, nullptr, hn, no_sum);
             m->launches += 1;
             if (has_ff) {
                 const int rc = feed_forward(st);
                 if (rc != SMOL_OK) return rc;
-                post_norm_kernel<T><<<Tn, nthr, 2 * D * sizeof(float), st>>>(x, y, c.residual_alpha, L.norm2, c.norm_eps, D, hist, hist_stride,
+                pdl_launch(post_norm_kernel<T>, Tn, nthr, 2 * D * sizeof(float), st, x, y, c.residual_alpha, L.norm2, c.norm_eps, D, hist, hist_stride,
                                                                           (int)n + 2, L.depth_mix, nullptr, hn, routed);
                 m->launches += 1;
             }
         } else if (L.mlp != SMOL_LM_MLP_NONE) {
-            add_norm_kernel<T><<<Tn, nthr, D * sizeof(float), st>>>(x, y, L.norm1b, L.ls1, L.norm2, c.norm_eps, D, hn, woff, L.out_bias, no_sum, hn);
+            pdl_launch(add_norm_kernel<T>, Tn, nthr, D * sizeof(float), st, x, y, L.norm1b, L.ls1, L.norm2, c.norm_eps, D, hn, woff, L.out_bias, no_sum, hn);
             const int rc = feed_forward(st);
             if (rc != SMOL_OK) return rc;
-            add_norm_kernel<T><<<Tn, nthr, D * sizeof(float), st>>>(x, y, L.norm2b, L.ls2, next_norm1, c.norm_eps, D, hn, woff, nullptr, routed, hn);
+            pdl_launch(add_norm_kernel<T>, Tn, nthr, D * sizeof(float), st, x, y, L.norm2b, L.ls2, next_norm1, c.norm_eps, D, hn, woff, nullptr, routed, hn);
             m->launches += 2;
         } else {
-            add_norm_kernel<T><<<Tn, nthr, D * sizeof(float), st>>>(x, y, L.norm1b, L.ls1, next_norm1, c.norm_eps, D, hn, woff, L.out_bias, no_sum, hn);
+            pdl_launch(add_norm_kernel<T>, Tn, nthr, D * sizeof(float), st, x, y, L.norm1b, L.ls1, next_norm1, c.norm_eps, D, hn, woff, L.out_bias, no_sum, hn);
             m->launches += 1;
         }
         if (s->trace && !prenorm && !parallel && !outnorm) CU(cudaMemcpyAsync(s->trace + n * (size_t)Tn * D, x, (size_t)Tn * D * 4, cudaMemcpyDeviceToDevice, st));
     }
     if (s->n_want > 0) {
-        if (postnorm) post_norm_kernel<T><<<s->n_want, nthr, 2 * D * sizeof(float), st>>>(x, nullptr, c.logit_scale, m->g.final_norm, c.norm_eps, D, nullptr, 0, 0,
+        if (postnorm) pdl_launch(post_norm_kernel<T>, s->n_want, nthr, 2 * D * sizeof(float), st, x, nullptr, c.logit_scale, m->g.final_norm, c.norm_eps, D, nullptr, 0, 0,
                                                                                       nullptr, s->want_rows, hw, RoutedSum{nullptr, nullptr, nullptr, 0});
-        else if (prenorm || parallel || outnorm) prenorm_rows_kernel<T><<<s->n_want, nthr, 0, st>>>(x, s->want_rows, norm_of(m->g.final_norm, m->g.final_norm_shift, m->g.final_norm_alpha), D, hw);
-        else norm_rows_kernel<T><<<s->n_want, nthr, 0, st>>>(x, s->want_rows, m->g.final_norm, c.norm_eps, D, hw, woff);
+        else if (prenorm || parallel || outnorm) pdl_launch(prenorm_rows_kernel<T>, s->n_want, nthr, 0, st, x, s->want_rows, norm_of(m->g.final_norm, m->g.final_norm_shift, m->g.final_norm_alpha), D, hw);
+        else pdl_launch(norm_rows_kernel<T>, s->n_want, nthr, 0, st, x, s->want_rows, m->g.final_norm, c.norm_eps, D, hw, woff);
         m->launches++;
         CU(linear<T>(m, hw, static_cast<const T*>(m->g.head), s->logits, s->n_want, c.vocab, D, st));
         const float lscale = postnorm ? 1.0f : c.logit_scale;      // the post-norm block scales inside the final norm
         if (lscale != 1.0f || c.logit_softcap > 0.0f) {
-            logit_finish_kernel<<<cast_grid((size_t)s->n_want * c.vocab), 256, 0, st>>>(s->logits, lscale, c.logit_softcap, (size_t)s->n_want * c.vocab);
+            pdl_launch(logit_finish_kernel, cast_grid((size_t)s->n_want * c.vocab), 256, 0, st, s->logits, lscale, c.logit_softcap, (size_t)s->n_want * c.vocab);
             m->launches++;
         }
     }
@@ -3501,10 +3577,10 @@ extern "C" int smol_lm_sample(SmolLm* m, const float* d_logits, int32_t rows, in
     const int grid = rows < 1024 ? rows : 1024;
     if (n <= smol::kThreads * 8) {
         CU(cudaFuncSetAttribute(lm_sample_kernel<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024));
-        lm_sample_kernel<8><<<grid, smol::kThreads, smem, st>>>(d_logits, n, rows, temp, top_k, top_p, min_p, seed, d_seq_id, d_step, d_out);
+        pdl_launch(lm_sample_kernel<8>, grid, smol::kThreads, smem, st, d_logits, n, rows, temp, top_k, top_p, min_p, seed, d_seq_id, d_step, d_out);
     } else {
         CU(cudaFuncSetAttribute(lm_sample_kernel<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024));
-        lm_sample_kernel<64><<<grid, smol::kThreads, smem, st>>>(d_logits, n, rows, temp, top_k, top_p, min_p, seed, d_seq_id, d_step, d_out);
+        pdl_launch(lm_sample_kernel<64>, grid, smol::kThreads, smem, st, d_logits, n, rows, temp, top_k, top_p, min_p, seed, d_seq_id, d_step, d_out);
     }
     CU(cudaGetLastError());
     m->launches++;

@@ -53,6 +53,8 @@ template <class T>
 __global__ void embed_gain_norm_kernel(const int32_t* __restrict__ tokens, const T* __restrict__ embed, int D, int vocab,
                                        const float* __restrict__ gain, float eps, float* __restrict__ x, float* __restrict__ hist0,
                                        T* __restrict__ hn) {
+    dep_wait();
+    dep_go();
     __shared__ float red[33];
     const int t = blockIdx.x;
     int tok = tokens[t];
@@ -84,6 +86,8 @@ template <class T>
 __global__ void post_norm_kernel(float* __restrict__ x, const float* __restrict__ y, float alpha, const float* __restrict__ gain, float eps,
                                  int D, float* __restrict__ hist, size_t hist_stride, int n_hist, const float* __restrict__ mix,
                                  const int32_t* __restrict__ rows, T* __restrict__ hn, const RoutedSum rs) {
+    dep_wait();
+    dep_go();
     extern __shared__ float row[];          // the row before the division [D], then the earlier history's weighted sum [D]
     __shared__ float red[33];
     const size_t o = (size_t)(rows ? rows[blockIdx.x] : blockIdx.x) * D, oo = (size_t)blockIdx.x * D;
@@ -243,6 +247,8 @@ __device__ __forceinline__ void rotate_pair(float a, float b, int pos, float fre
 // One block per token: the normed query latent -> cq (T), the normed key/value latent and the rotated key part -> the pool.
 template <class T>
 __global__ void latent_prep_kernel(const LatentArgs A, T* __restrict__ cq, T* __restrict__ pool) {
+    dep_wait();
+    dep_go();
     __shared__ float red[2][33];
     const int t = blockIdx.x;
     const float* row = A.proj + (size_t)t * A.n_in;
@@ -285,6 +291,8 @@ __global__ void latent_prep_kernel(const LatentArgs A, T* __restrict__ cq, T* __
 // One warp per (token, head).
 template <class T>
 __global__ void latent_query_kernel(const LatentArgs A, const float* __restrict__ q, T* __restrict__ qbuf) {
+    dep_wait();
+    dep_go();
     const int lane = threadIdx.x & 31;
     const int unit = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     if (unit >= A.n_tokens * A.H) return;
@@ -343,6 +351,8 @@ __host__ __device__ inline void gla_sources_from_proj(GlaArgs& A) {
 // decay[t][c] for the H*d key channels; a block takes TT tokens and blockDim.x channels (as delta_prep_kernel, for its reason)
 template <int TT>
 __global__ void __launch_bounds__(128) gla_prep_kernel(const GlaArgs A, float* __restrict__ decay) {
+    dep_wait();
+    dep_go();
     extern __shared__ float inner[];      // [rank][TT]
     const int t0 = blockIdx.x * TT, nt = min(TT, A.n_tokens - t0), HD = A.H * A.d;
     const size_t at = 2 * HD + 2 * A.H * A.dv;
@@ -412,6 +422,8 @@ template <int DK, bool SCALAR>
 __global__ void __launch_bounds__(gla_block_cols(DK) * gla_lanes(DK)) gla_scan_kernel(const GlaArgs A, const float* __restrict__ decay,
                                                                                          float* __restrict__ state_pool,
                                                                                          float* __restrict__ o_raw) {
+    dep_wait();
+    dep_go();
     constexpr int L = gla_lanes(DK), CB = gla_block_cols(DK), RV = DK / L / 4, PL = kDeltaChunk * DK;
     constexpr int kBuf = gla_buf_floats(DK);
     static_assert(DK % (4 * L) == 0, "every lane owns whole 16-byte pieces");
@@ -521,6 +533,8 @@ __global__ void __launch_bounds__(gla_block_cols(DK) * gla_lanes(DK)) gla_scan_k
 // T.  One warp per (token, head).
 template <class T>
 __global__ void gla_out_kernel(const GlaArgs A, const float* __restrict__ o_raw, T* __restrict__ out) {
+    dep_wait();
+    dep_go();
     const int lane = threadIdx.x & 31;
     const int unit = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     if (unit >= A.n_tokens * A.H) return;
@@ -643,6 +657,8 @@ __device__ __forceinline__ ConvIo conv_of(const SsdArgs& A) {
 // Blocks (token, slice of channels): the convolved channels.  The block of a token's first slice also
 // leaves the heads' step dt = softplus(dt + bias) and decay exp(-exp(a_log) * dt) in `head` ([T][H] decay, then [T][H] step).
 __global__ void ssd_conv_kernel(const SsdArgs A, const float* __restrict__ slots, float* __restrict__ conv, float* __restrict__ head) {
+    dep_wait();
+    dep_go();
     const int t = blockIdx.x, inner = A.H * A.dv, ch = inner + 2 * A.G * A.N;
     const int s = A.tok_seq[t], t0 = A.seq_start[s], pos0 = A.seq_pos0[s];
     const int r = t - t0;                      // the token's place in this step's portion
@@ -668,6 +684,8 @@ __global__ void ssd_conv_kernel(const SsdArgs A, const float* __restrict__ slots
 template <class T>
 __global__ void ssd_out_kernel(const SsdArgs A, const float* __restrict__ o_raw, const float* __restrict__ conv, T* __restrict__ out,
                                float* __restrict__ slots) {
+    dep_wait();
+    dep_go();
     __shared__ float red[33];
     const int t = blockIdx.x, inner = A.H * A.dv, ch = inner + 2 * A.G * A.N, len = inner / A.parts;
     const int c0 = blockIdx.y * len;
@@ -721,6 +739,8 @@ __global__ void ssd_out_kernel(const SsdArgs A, const float* __restrict__ o_raw,
 // Gated feed-forward: z rows hold gate [F] | up [F]; out = the gated unit's value (act(gate) * up, or the clamped form) in T.
 template <class T>
 __global__ void gated_act_kernel(const float* __restrict__ z, int F, const ActParams kind, size_t rows, T* __restrict__ out) {
+    dep_wait();
+    dep_go();
     const size_t ld = kind.plain ? F : 2 * F, uo = kind.plain ? 0 : F;      // plain: the "up" operand is the value itself, unused
     if (F % 4 == 0) {                      // 16-byte pieces
         const size_t n = rows * (F / 4);
@@ -777,6 +797,8 @@ constexpr int kMaxTop = 32;
 template <class TI>
 __global__ void __launch_bounds__(128) moe_route_kernel(const RouteArgs A, const TI* __restrict__ x, float* __restrict__ logits,
                                                         int32_t* __restrict__ done, int32_t* __restrict__ sel_id, float* __restrict__ sel_w) {
+    dep_wait();
+    dep_go();
     __shared__ float s[kMaxRouted], choice[kMaxRouted], gscore[kMaxRouted];
     __shared__ float red[33];
     __shared__ float top_s[kMaxTop];
@@ -916,6 +938,8 @@ __global__ void __launch_bounds__(256) moe_index_kernel(const int32_t* __restric
                                                         int32_t* __restrict__ seg, int32_t* __restrict__ perm, int32_t* __restrict__ slot_of,
                                                         int32_t* __restrict__ tile_group, int32_t* __restrict__ tile_row0,
                                                         int32_t* __restrict__ n_tiles) {
+    dep_wait();
+    dep_go();
     __shared__ int count[kMaxRouted + 1], cursor[kMaxRouted];
     for (int e = threadIdx.x; e <= E_real; e += blockDim.x) count[e] = 0;
     __syncthreads();
@@ -956,6 +980,8 @@ __global__ void __launch_bounds__(256) moe_index_kernel(const int32_t* __restric
 // the input row of pair perm[r].  One block per row; rows beyond the sorted pairs (*n_sorted) are left alone.
 __global__ void moe_gather_kernel(const bf16* __restrict__ h, const int32_t* __restrict__ perm, int div, const int32_t* __restrict__ n_sorted,
                                   int D, bf16* __restrict__ out) {
+    dep_wait();
+    dep_go();
     const int r = blockIdx.x;
     if (r >= *n_sorted) return;
     const bf16* src = h + (size_t)(perm[r] / div) * D;
@@ -972,6 +998,8 @@ __global__ void moe_gather_kernel(const bf16* __restrict__ h, const int32_t* __r
 template <class T>
 __global__ void moe_gather_scaled_kernel(const T* __restrict__ h, const int32_t* __restrict__ perm, int div, const float* __restrict__ sel_w,
                                          const int32_t* __restrict__ n_sorted, int D, T* __restrict__ out) {
+    dep_wait();
+    dep_go();
     const int r = blockIdx.x;
     if (r >= *n_sorted) return;
     const int pair = perm[r];
@@ -992,6 +1020,8 @@ __global__ void __launch_bounds__(256) moe_gemv_kernel(const void* __restrict__ 
                                                        const int32_t* __restrict__ sel_id, const int32_t* __restrict__ n_sorted,
                                                        const bf16* __restrict__ w, long long w_stride, float* __restrict__ y, int N, int K,
                                                        const ActParams act) {
+    dep_wait();
+    dep_go();
     extern __shared__ __align__(16) unsigned char unit_smem[];      // ACT: the row's unit values [K]
     const int r = blockIdx.y;
     if (r >= *n_sorted) return;

@@ -77,6 +77,8 @@ __device__ __forceinline__ float scatter_sum(float (&v)[N], int lane) {
 // One warp per (group, sequence, head).
 template <int KIND, int DK>
 __global__ void __launch_bounds__(128) quad_prep_kernel(const QuadSource A, float* __restrict__ rec) {
+    dep_wait();
+    dep_go();
     constexpr int FORM = quad_form(KIND), NV = quad_vecs(FORM), NP = quad_products(FORM), NS = FORM == kFormGeneral ? 32 : 16;
     const int h = blockIdx.z * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31, seq = blockIdx.y;
     const int t0 = A.seq_start[seq], n_all = A.seq_start[seq + 1] - t0, r0 = blockIdx.x * kQuad;
@@ -224,6 +226,8 @@ __device__ __forceinline__ void copy_float(float* dst, const float* src, bool in
 
 template <int DK, int FORM>
 __global__ void __launch_bounds__(kQuadThreads, 1) quad_scan_kernel(const QuadArgs A, float* state_pool, float* __restrict__ o_raw) {
+    dep_wait();
+    dep_go();
     using f32t::fma2;
     constexpr int L = kQuadLanes, CB = kQuadCols, RV = DK / L / 4, NB = kQuadRing, NG = quad_chunk(DK), RF = quad_record(FORM, DK), NV = quad_vecs(FORM);
     constexpr int kAt = FORM == kFormGeneral ? 12 : 4;      // the k vectors

@@ -117,6 +117,8 @@ __device__ __forceinline__ void layer_norm_row(const NormSpec& nm, int D, T* __r
 template <class T>
 __global__ void embed_prenorm_kernel(const int32_t* __restrict__ tokens, const T* __restrict__ embed, float scale, int D, int vocab,
                                      const NormSpec nm, float* __restrict__ x, float* __restrict__ x0, T* __restrict__ hn, T* __restrict__ cat) {
+    dep_wait();
+    dep_go();
     __shared__ float red[3][33];
     const int t = blockIdx.x;
     int tok = tokens[t];
@@ -147,6 +149,8 @@ __global__ void embed_prenorm_kernel(const int32_t* __restrict__ tokens, const T
 // The norm of selected rows -> T (the final norm of the rows whose logits are wanted).
 template <class T>
 __global__ void prenorm_rows_kernel(const float* __restrict__ x, const int32_t* __restrict__ rows, const NormSpec nm, int D, T* __restrict__ out) {
+    dep_wait();
+    dep_go();
     __shared__ float red[3][33];
     const float* xr = x + (size_t)(rows ? rows[blockIdx.x] : blockIdx.x) * D;
     const size_t o = (size_t)blockIdx.x * D;
@@ -191,6 +195,8 @@ struct ResidualArgs {
 
 template <class T, bool VEC>
 __global__ void residual_norm_kernel(const ResidualArgs A, T* __restrict__ hn) {
+    dep_wait();
+    dep_go();
     extern __shared__ float row[];
     __shared__ float red3[3][33];
     const int D = A.D;
@@ -365,6 +371,8 @@ __device__ __forceinline__ int sigmoid_first_key(const SigmoidArgs& S, int pos) 
 // cached key.  A lane owns whole pairs, so a pair is rotated where it was loaded.
 template <class T>
 __global__ void sigmoid_prep_kernel(const SigmoidArgs S, T* __restrict__ qbuf, T* __restrict__ pool) {
+    dep_wait();
+    dep_go();
     const AttnArgs& A = S.a;
     const int lane = threadIdx.x & 31;
     const int unit = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
@@ -427,6 +435,8 @@ constexpr int kSigmoidRanges = 6;             // most key ranges a row tile of t
 template <class T, int MAXV>
 __global__ void __launch_bounds__(kSigmoidMaxHeads * 32) sigmoid_attn_kernel(const SigmoidArgs S, const T* __restrict__ qbuf,
                                                                             const T* __restrict__ pool, T* __restrict__ out) {
+    dep_wait();
+    dep_go();
     extern __shared__ float sig_smem[];      // queries [H][d], weights [H][32], mixing matrix [H][H]
     const AttnArgs& A = S.a;
     const int h = threadIdx.x >> 5, lane = threadIdx.x & 31, H = A.H;
@@ -495,6 +505,8 @@ __host__ __device__ inline size_t sigmoid_split_smem(int H, int G, int d, int dv
 
 template <class T, int MAXV>
 __global__ void __launch_bounds__(kSigmoidMaxHeads * 32) sigmoid_split_kernel(const SigmoidArgs S, const T* __restrict__ qbuf, const T* __restrict__ pool) {
+    dep_wait();
+    dep_go();
     extern __shared__ __align__(16) unsigned char ss_raw[];
     constexpr int kPad = 16 / (int)sizeof(T);
     const AttnArgs& A = S.a;
@@ -564,6 +576,8 @@ __global__ void __launch_bounds__(kSigmoidMaxHeads * 32) sigmoid_split_kernel(co
 // One block per row of a short sequence: adds the ranges' partial sums in range order, applies the head's gate, writes T.
 template <class T>
 __global__ void sigmoid_short_merge_kernel(const SigmoidArgs S, T* __restrict__ out) {
+    dep_wait();
+    dep_go();
     const AttnArgs& A = S.a;
     const int s = blockIdx.x / kShortSeq, r = blockIdx.x % kShortSeq;
     const int t0 = A.seq_start[s], n = A.seq_start[s + 1] - t0;
@@ -593,6 +607,8 @@ __global__ void sigmoid_short_merge_kernel(const SigmoidArgs S, T* __restrict__ 
 template <int DK, int HPW, int KT>
 __global__ void __launch_bounds__(512) sigmoid_flash_kernel(const SigmoidArgs S, const bf16* __restrict__ qbuf,
                                                                           const bf16* __restrict__ pool, bf16* __restrict__ out) {
+    dep_wait();
+    dep_go();
     constexpr int LD = DK + 8, LDW = KT + 8;
     extern __shared__ __align__(16) unsigned char sf_smem[];
     const AttnArgs& A = S.a;
@@ -749,6 +765,8 @@ __global__ void __launch_bounds__(512) sigmoid_flash_kernel(const SigmoidArgs S,
 
 // Adds a row's partial sums over its key ranges in range order, applies the head's gate and writes bf16.  One block per token.
 __global__ void sigmoid_merge_kernel(const SigmoidArgs S, bf16* __restrict__ out) {
+    dep_wait();
+    dep_go();
     const AttnArgs& A = S.a;
     const int t = blockIdx.x, s = A.tok_seq[t];
     const int t0 = A.seq_start[s], n = A.seq_start[s + 1] - t0;
@@ -777,6 +795,8 @@ struct LinPrepArgs {
 };
 
 __global__ void lightning_prep_kernel(const LinPrepArgs A, float* __restrict__ act, float* __restrict__ head) {
+    dep_wait();
+    dep_go();
     const int t = blockIdx.x, n = 2 * A.H * A.d + A.H * A.dv;
     const float* row = A.proj + (size_t)t * A.n_in;
     for (int c = blockIdx.y * blockDim.x + threadIdx.x; c < n; c += gridDim.y * blockDim.x) act[(size_t)t * n + c] = silu_(row[c]);
@@ -787,6 +807,8 @@ __global__ void lightning_prep_kernel(const LinPrepArgs A, float* __restrict__ a
 }
 
 __global__ void hgrn2_prep_kernel(const LinPrepArgs A, float* __restrict__ qv, float* __restrict__ key, float* __restrict__ decay) {
+    dep_wait();
+    dep_go();
     const int t = blockIdx.x, HD = A.H * A.d;
     const float* row = A.proj + (size_t)t * A.n_in;
     for (int c = blockIdx.y * blockDim.x + threadIdx.x; c < HD; c += gridDim.y * blockDim.x) {
@@ -810,6 +832,8 @@ struct RetentionArgs {
 };
 
 __global__ void retention_prep_kernel(const RetentionArgs A, float* __restrict__ qk) {
+    dep_wait();
+    dep_go();
     const int t = blockIdx.x, HD = A.H * A.d, per = A.d - A.pairs;
     const int pos = A.tok_pos[t];
     const float *q = A.proj + (size_t)t * A.n_in, *k = q + HD;
@@ -835,6 +859,8 @@ __global__ void retention_prep_kernel(const RetentionArgs A, float* __restrict__
 
 // The logits' last step: times scale, then bent to cap * tanh(v / cap) (cap 0: not bent).
 __global__ void logit_finish_kernel(float* __restrict__ v, float scale, float cap, size_t n) {
+    dep_wait();
+    dep_go();
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
         const float z = v[i] * scale;
         v[i] = cap > 0.0f ? cap * tanhf(z / cap) : z;
@@ -854,6 +880,8 @@ struct LinOutArgs {
 
 template <class T>
 __global__ void lin_attn_out_kernel(const LinOutArgs A, const float* __restrict__ o_raw, T* __restrict__ out) {
+    dep_wait();
+    dep_go();
     __shared__ float red[33];
     const int t = blockIdx.x, c0 = blockIdx.y * A.len;
     const float* o = o_raw + (size_t)t * A.cols;

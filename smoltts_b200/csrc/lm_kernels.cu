@@ -1814,6 +1814,7 @@ __global__ void __launch_bounds__(kThreads) lm_sample_kernel(const float* __rest
 }  // namespace lm
 }  // namespace smol
 
+#include "lm_flash_tc.cuh"
 #include "lm_mechanisms.cuh"
 #include "lm_sigmoid_linear.cuh"
 #include "lm_delta_mlstm.cuh"
@@ -2361,6 +2362,17 @@ static cudaError_t set_kernel_attributes() {
     SMOL_FLASH_ATTR(64, 128, false, 2);
     SMOL_FLASH_ATTR(128, 128, false, 2);
 #undef SMOL_FLASH_ATTR
+#define SMOL_FLASH_TC_ATTR(DK, DV, VK, MAPS) \
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(attn_flash_tc_kernel<DK, DV, VK, MAPS>, cudaFuncAttributeMaxDynamicSharedMemorySize, ft_smem(DK, DV, VK, MAPS))
+    SMOL_FLASH_TC_ATTR(64, 64, false, 1);
+    SMOL_FLASH_TC_ATTR(64, 128, false, 1);
+    SMOL_FLASH_TC_ATTR(128, 128, false, 1);
+    SMOL_FLASH_TC_ATTR(64, 64, true, 1);
+    SMOL_FLASH_TC_ATTR(128, 128, true, 1);
+    SMOL_FLASH_TC_ATTR(192, 128, true, 1);
+    SMOL_FLASH_TC_ATTR(64, 64, false, 2);
+    SMOL_FLASH_TC_ATTR(64, 128, false, 2);
+#undef SMOL_FLASH_TC_ATTR
     return e;
 }
 
@@ -2704,6 +2716,33 @@ static cudaError_t launch_group_scan_any(SmolLm* m, const GroupScanArgs& A, floa
     return launch_group_scan<256, DELTA>(A, n_seqs, pool, o_raw, st, min_smem);
 }
 
+// attn_flash_tc_kernel where a sequence brings more than kFtMinRows tokens and every row it copies is made of whole 16-byte pieces.
+// False: not launched (few tokens, unaligned rows, sizes it is not built for).
+template <int MAPS>
+static bool launch_flash_tc(const AttnArgs& A, int n_seqs, int max_n, const bf16* qbuf, const bf16* pool, bf16* out, cudaStream_t st) {
+    const size_t rows = A.d | A.dv | A.out_ld | A.page_elems | A.k_off | A.k_ld | (A.v_in_k ? 0 : A.v_off | A.v_ld);
+    if (max_n <= kFtMinRows || rows % 8 != 0 || (reinterpret_cast<uintptr_t>(qbuf) | reinterpret_cast<uintptr_t>(pool) | reinterpret_cast<uintptr_t>(out)) % 16 != 0) return false;
+    if (A.dv > 128 || A.d > (MAPS == 2 ? 64 : A.v_in_k ? 192 : 128)) return false;
+    const dim3 grid(A.H, n_seqs, (max_n + kFtRows - 1) / kFtRows);
+#define SMOL_FLASH_TC(DK, DV, VK) plain_launch(attn_flash_tc_kernel<DK, DV, VK, MAPS>, grid, kFtThreads, ft_smem(DK, DV, VK, MAPS), st, A, qbuf, pool, out)
+    if constexpr (MAPS == 1) {
+        if (A.v_in_k) {
+            if (A.d <= 64) SMOL_FLASH_TC(64, 64, true);
+            else if (A.d <= 128) SMOL_FLASH_TC(128, 128, true);
+            else SMOL_FLASH_TC(192, 128, true);
+            return true;
+        }
+        if (A.d > 64) {
+            SMOL_FLASH_TC(128, 128, false);
+            return true;
+        }
+    }
+    if (A.dv <= 64) SMOL_FLASH_TC(64, 64, false);
+    else SMOL_FLASH_TC(64, 128, false);
+#undef SMOL_FLASH_TC
+    return true;
+}
+
 // The attention kernels over the rows of a step: prompt portions on the tensor-core form (bf16, `flash`) or the
 // warp-per-row form, sequences of few tokens on the split-range form.  `A` is complete except for the fields set here.
 template <class T, int MAXV, int MAPS>
@@ -2727,14 +2766,14 @@ static void launch_attention(SmolLm* m, const SmolLmStep* s, AttnArgs& A, bool f
             const bf16* pl = reinterpret_cast<const bf16*>(pool);
             bf16* mx = reinterpret_cast<bf16*>(mix);
 #define SMOL_FLASH(DK, DV, VK) plain_launch(attn_flash_kernel<DK, DV, VK, MAPS>, grid, 128 * MAPS, flash_smem_bytes(DK, DV, VK, MAPS), st, A, qb, pl, mx)
-            bool done = false;
+            bool done = launch_flash_tc<MAPS>(A, s->n_seqs, max_n, qb, pl, mx, st);
             if constexpr (MAPS == 1) {
-                done = A.v_in_k != 0;
-                if (!A.v_in_k) {
+                if (done || !A.v_in_k) {
                 } else if (A.d <= 64) SMOL_FLASH(64, 64, true);
                 else if (A.d <= 128) SMOL_FLASH(128, 128, true);
                 else if (A.dv <= 128) SMOL_FLASH(192, 128, true);
                 else SMOL_FLASH(192, 192, true);
+                done = done || A.v_in_k;
             }
             if (done) {
             } else if (hp <= 32) SMOL_FLASH(32, 32, false);

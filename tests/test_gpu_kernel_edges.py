@@ -110,3 +110,50 @@ def test_codec_runs_of_frames_equal_single_steps(streams, frames):
     steps = torch.cat([m.decode_step(codes[:, :, t:t + 1], caches).clone() for t in range(frames)], -1)
     assert torch.equal(whole, steps)
     assert not m.overflowed()
+
+
+ATTENTION_FORMS = {"sink-64-64": ("pamasun", lambda u: u.attn(heads=4, kv_heads=2, dim=64, vdim=64, ff=0)),
+                   "sink-40-72": ("pamasun", lambda u: u.attn(heads=2, kv_heads=1, dim=40, vdim=72, ff=0)),
+                   "sink-104-8": ("pamasun", lambda u: u.attn(heads=3, kv_heads=3, dim=104, vdim=8, ff=0)),
+                   "latent-48": ("maferax", lambda u: u.latent(heads=3, dim=16, rot_dim=8, vdim=16, q_rank=24, kv_rank=40)),
+                   "latent-160": ("maferax", lambda u: u.latent(heads=2, dim=32, rot_dim=32, vdim=32, q_rank=24, kv_rank=128)),
+                   "maps-64-128": ("virusun", lambda u: u.att(heads=2, kv_heads=1, dim=64, vdim=128)),
+                   "maps-24-40": ("virusun", lambda u: u.att(heads=4, kv_heads=2, dim=24, vdim=40)),
+                   "rotated-32-16": ("virusun", lambda u: u.par(u.left(heads=4, kv_heads=2, dim=32, vdim=16))),
+                   "window-48-16": ("sunutar", lambda u: u.layer(u.left(dim=48, vdim=16, window=100))),
+                   "capped-24-24": ("bizulix", lambda u: u.att(dim=24, vdim=24))}
+
+
+@pytest.mark.parametrize("form", ATTENTION_FORMS)
+def test_prompt_attention_of_128_row_tiles(form):
+    """bf16 prompts that end at and around the tiles' 128 rows and the steps' 64 keys, beside a sequence of three tokens, continued by a
+    second portion: as close to the oracle as the same prompts in portions of at most 64 tokens, which the other kernel takes.  The two
+    differ in the order of fp32 sums, so at most by one bf16 rounding (2^-8) of what each writes."""
+    import importlib
+
+    name, layer = ATTENTION_FORMS[form]
+    u = importlib.import_module(f"{name}_util")
+    cfg = u.config([layer(u)], vocab=61, width=48)
+    model, orc, _ = u.engine_and_oracle(cfg, seed=6, dtype=torch.bfloat16, max_tokens=2048, max_seqs=5, page_size=16, max_step_tokens=640)
+    lens, more = (193, 128, 129, 65, 3), 66
+    toks = [tokens(n + more, 61, n) for n in lens]
+    want = [orc.forward(t) for t in toks]
+
+    def rows(portions):
+        seqs, out = [model.open_sequence() for _ in lens], [[] for _ in lens]
+        for step in portions:
+            got = model.forward([(s, t[a:b], list(range(b - a))) for s, t, (a, b) in zip(seqs, toks, step) if b > a]).clone()
+            at = 0
+            for o, (a, b) in zip(out, step):
+                o.append(got[at:at + b - a])
+                at += b - a
+        for s in seqs:
+            model.close_sequence(s)
+        return [torch.cat(o) for o in out]
+
+    whole = rows([[(0, n) for n in lens], [(n, n + more) for n in lens]])
+    pieces = rows([[(min(a, n + more), min(a + 64, n + more)) for n in lens] for a in range(0, max(lens) + more, 64)])
+    for w, p, o in zip(whole, pieces, want):
+        assert rel_err(w, o) < TOL[torch.bfloat16]
+        assert rel_err(w, o) < 1.5 * rel_err(p, o) + 2.0 ** -8
+    model.check_device_errors()

@@ -1,9 +1,8 @@
 // Softmax attention of prompt portions on the 5th-generation tensor cores, bf16 (sm_100a).  Included by lm_kernels.cu.
 //
 // One block per (128 rows of a sequence in this step, sequence, query head).  Keys and values come 64 positions at a time from the paged
-// pool.  The roles run side by side: three loader warps keep a ring of three stages filled (one each, so that three stages' loads are in
-// flight; 128-byte-swizzled rows of 64 columns, which serve the product with the queries k-contiguous and the one with the weights
-// n-contiguous, so nothing is transposed), one thread issues the tcgen05 products, eight warps take the scores out of tensor memory -- two threads per row, half the columns each -- and keep the running softmax.  The scores of the next 64
+// pool.  The roles run side by side: loader warps keep a ring of three or four stages filled (one each, so that as many loads are in flight; 128-byte-swizzled rows of 64 columns, which serve the product with the queries k-contiguous and the one with the weights
+// n-contiguous, so nothing is transposed), one thread issues the tcgen05 products, sixteen warps take the scores out of tensor memory -- four threads per row, 16 columns each -- and keep the running softmax.  The scores of the next 64
 // positions are multiplied while the current ones are worked on, the product with the values while the next ones are.  That product is
 // read back from tensor memory and joins the fp32 running sums, which stay in registers.
 //
@@ -11,27 +10,31 @@
 // remainder (two MMAs), the sink is the initial state of the running softmax, and a row takes nothing from 64 positions it does not see.
 // Differential attention (MAPS 2) walks the keys once per map; the first map's result waits in shared memory, each thread's own part.
 //
-// What bounds it: the softmax's own instructions, 64 x 128 scores a step with one exponential (and, with a distance penalty, one
-// logarithm) each.  2048 tokens, 12 heads of 64 with a distance penalty: 84 us, attn_flash_kernel
-// 165; 1801 tokens, 12 heads of 128: 98 against 219; 1024 tokens, 12 heads over a latent of 160: 48 against 101; 3 x 1000 tokens, 6 heads
-// of two maps: 99 against 116.
+// What bounds it: the instructions of a step, the loaders' as much as the softmax's 64 x 128 scores with one exponential (and, with a distance
+// penalty, one logarithm) each -- hence four threads per row, whose latencies cover one another, and a warp per stage.  Two threads per row
+// and three stages: 84 / 98 / 48 / 99 us instead of the following.
+// 2048 tokens, 12 heads of 64 with a distance penalty: 64 us, attn_flash_kernel 165; 1801 tokens, 12 heads of 128: 82 against 219; 1024
+// tokens, 12 heads over a latent of 160: 42 against 101; 3 x 1000 tokens, 6 heads of two maps: 97 against 116.
 #pragma once
 
 namespace smol {
 namespace lm {
 
 constexpr int kFtRows = 128, kFtKeys = 64;
-constexpr int kFtMinRows = 64;          // sequences of at most this many tokens: attn_flash_kernel
-constexpr int kFtSoftWarps = 8, kFtStages = 3, kFtThreads = (kFtSoftWarps + 1 + kFtStages) * 32;
+constexpr int kFtParts = 4, kFtCols = kFtKeys / kFtParts;                   // threads per row, score columns of each
+constexpr int kFtSoftWarps = 4 * kFtParts, kFtMaxStages = 4;
 constexpr int kFtPBytes = kFtRows * kFtKeys * 2;                              // heads or remainders of a step's weights
 // VK: the values are the first columns of the key rows
 __host__ __device__ constexpr int ft_stage_bytes(int DK, int DV, bool VK) { return kFtKeys * 2 * (DK + (VK ? 0 : DV)); }
+// three stages where a fourth does not fit
+__host__ __device__ constexpr int ft_stages(int DV, int MAPS) { return MAPS == 2 && DV == 128 ? 3 : kFtMaxStages; }
+__host__ __device__ constexpr int ft_threads(int DV, int MAPS) { return (kFtSoftWarps + 1 + ft_stages(DV, MAPS)) * 32; }
 __host__ __device__ constexpr int ft_smem(int DK, int DV, bool VK, int MAPS) {
-    return 1024 + MAPS * kFtRows * DK * 2 + kFtStages * ft_stage_bytes(DK, DV, VK) + 2 * kFtPBytes + (MAPS - 1) * kFtRows * DV * 4;
+    return 1024 + MAPS * kFtRows * DK * 2 + ft_stages(DV, MAPS) * ft_stage_bytes(DK, DV, VK) + 2 * kFtPBytes + (MAPS - 1) * kFtRows * DV * 4;
 }
 
 struct FlashTcBars {
-    uint64_t full[kFtStages], empty[kFtStages];          // stages of keys and values
+    uint64_t full[kFtMaxStages], empty[kFtMaxStages];          // stages of keys and values
     uint64_t s_full[2], s_empty[2];      // scores in tensor memory
     uint64_t p_full, o_full;             // weights in shared memory (their product's last result has been read); weights x values in tensor memory
     uint32_t tmem;
@@ -49,32 +52,60 @@ __device__ __forceinline__ uint32_t instr_desc_bn(int n) { return umma::instr_de
 __device__ __forceinline__ uint64_t smem_desc_bn(uint32_t addr) {
     return (uint64_t)((addr & 0x3FFFFu) >> 4) | ((uint64_t)(kFtKeys * 128 >> 4) << 16) | ((uint64_t)(1024 >> 4) << 32) | (1ull << 46) | (2ull << 61);
 }
-// The scores of a thread's row and 32 keys from j0 on, dist = position - j0; `seen`: every key is, else masked by distance.
-template <bool CAP, bool PENALTY, bool SLOPE>
-__device__ __forceinline__ void ft_scores(const AttnArgs& A, float (&S)[32], int dist, bool seen, int win, float r1, float r2, float slope) {
-    const float d0 = (float)dist;
+__device__ __forceinline__ float log2_fast(float x) {      // hardware instruction, x >= 1
+    float y;
+    asm("lg2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return y;
+}
+__device__ __forceinline__ float max_of(const float (&S)[kFtCols]) {
+    float part[4] = {S[0], S[1], S[2], S[3]};
 #pragma unroll
-    for (int e = 0; e < 32; ++e) {
-        float v = S[e] * A.scale;
-        if (CAP && A.softcap > 0.0f) v = A.softcap * (1.0f - __fdividef(2.0f, __expf(v * A.two_over_cap) + 1.0f));
-        if (PENALTY) v -= r1 * __logf(fmaf(r2, d0 - (float)e, 1.0f));
-        if (SLOPE) v -= slope * (d0 - (float)e);
-        S[e] = seen || (dist - e >= 0 && dist - e < win) ? v : -INFINITY;
+    for (int e = 4; e < kFtCols; ++e) part[e % 4] = fmaxf(part[e % 4], S[e]);
+    return fmaxf(fmaxf(part[0], part[1]), fmaxf(part[2], part[3]));
+}
+// The scores of a thread's columns in units of log2 (multiplied by log2 e), dist = the row's position - the first column's; MASK: columns the
+// row does not see are -inf.  The distance penalty r1 ln(1 + r2 d) is r1 log2(1 + r2 d) in these units.
+template <bool GENERAL, bool PENALTY, bool MASK>
+__device__ __forceinline__ void ft_scores(const AttnArgs& A, float (&S)[kFtCols], int dist, int win, float r1, float r2, float slope) {
+    constexpr float kLog2e = 1.4426950408889634f;
+    const float d0 = (float)dist, x0 = fmaf(r2, d0, 1.0f), scale = A.scale * kLog2e;
+#pragma unroll
+    for (int e = 0; e < kFtCols; ++e) {
+        float v;
+        if (GENERAL) {
+            v = S[e] * A.scale;
+            if (A.softcap > 0.0f) v = A.softcap * (1.0f - __fdividef(2.0f, __expf(v * A.two_over_cap) + 1.0f));
+            v = (v - slope * (d0 - (float)e)) * kLog2e;
+            if (PENALTY) v = fmaf(-r1, log2_fast(fmaf(-(float)e, r2, x0)), v);
+        } else if (PENALTY) {
+            v = fmaf(S[e], scale, -r1 * log2_fast(fmaf(-(float)e, r2, x0)));
+        } else {
+            v = S[e] * scale;
+        }
+        S[e] = !MASK || (dist - e >= 0 && dist - e < win) ? v : -INFINITY;
     }
+}
+template <bool MASK>
+__device__ __forceinline__ void ft_scores_any(const AttnArgs& A, float (&S)[kFtCols], int dist, int win, float r1, float r2, float slope) {
+    if (A.softcap > 0.0f || A.slope) {
+        if (A.r1) ft_scores<true, true, MASK>(A, S, dist, win, r1, r2, slope);
+        else ft_scores<true, false, MASK>(A, S, dist, win, r1, r2, slope);
+    } else if (A.r1) ft_scores<false, true, MASK>(A, S, dist, win, r1, r2, slope);
+    else ft_scores<false, false, MASK>(A, S, dist, win, r1, r2, slope);
 }
 
 // DK / DV: key and value sizes padded to multiples of 64 (zeros).  d, dv and every row stride and offset are multiples of 8 elements.
 template <int DK, int DV, bool VK, int MAPS>
-__global__ void __launch_bounds__(kFtThreads, 1) attn_flash_tc_kernel(const AttnArgs A, const bf16* __restrict__ qbuf, const bf16* __restrict__ pool,
+__global__ void __launch_bounds__(ft_threads(DV, MAPS), 1) attn_flash_tc_kernel(const AttnArgs A, const bf16* __restrict__ qbuf, const bf16* __restrict__ pool,
                                                                       bf16* __restrict__ out) {
-    constexpr int NB = kFtStages, SB = ft_stage_bytes(DK, DV, VK), OC = DV / 2;
+    constexpr int NB = ft_stages(DV, MAPS), SB = ft_stage_bytes(DK, DV, VK), OC = DV / kFtParts;
     static_assert(DK % 64 == 0 && DV % 64 == 0 && DV <= 128 && (!VK || (DV <= DK && MAPS == 1)), "tile sizes");
     extern __shared__ unsigned char ft_smem_raw[];
     __shared__ FlashTcBars bars;
-    __shared__ float s_max[2][2][kFtRows], s_sum[2][2][kFtRows];
+    __shared__ float s_max[2][kFtParts][kFtRows], s_sum[2][kFtParts][kFtRows];
     unsigned char* base = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(ft_smem_raw) + 1023) & ~(uintptr_t)1023);
     unsigned char *Qs = base, *KV = Qs + MAPS * kFtRows * DK * 2, *Ps = KV + NB * SB;          // Ps: heads, then remainders
-    float* first_map = reinterpret_cast<float*>(Ps + 2 * kFtPBytes);                           // MAPS 2: [OC][256]
+    float* first_map = reinterpret_cast<float*>(Ps + 2 * kFtPBytes);                           // MAPS 2: [OC][threads of the softmax]
     dep_wait();
     dep_go();
     const int s = blockIdx.y, t0 = A.seq_start[s], n = A.seq_start[s + 1] - t0;
@@ -93,7 +124,7 @@ __global__ void __launch_bounds__(kFtThreads, 1) attn_flash_tc_kernel(const Attn
     }
     if (warp == kFtSoftWarps) umma::tmem_alloc(&bars.tmem);
     // queries of the tile: rows beyond the sequence and columns beyond d are zeros
-    for (int i = threadIdx.x; i < MAPS * kFtRows * (DK / 8); i += kFtThreads) {
+    for (int i = threadIdx.x; i < MAPS * kFtRows * (DK / 8); i += ft_threads(DV, MAPS)) {
         const int mp = i / (kFtRows * (DK / 8)), r = i / (DK / 8) % kFtRows, c = i % (DK / 8);
         const bool in = row0 + r < n && c * 8 < A.d;
         cp_async16_or_zero(Qs + mp * (kFtRows * DK * 2) + (c / 8) * (kFtRows * 128) + sw128_at(r, c % 8),
@@ -183,49 +214,49 @@ __global__ void __launch_bounds__(kFtThreads, 1) attn_flash_tc_kernel(const Attn
             values(steps - 1);
         }
     } else {
-        // ---- softmax: warps w and w + 4 share rows 32 (w % 4) .. + 31; columns 32 (w / 4) .. + 31 of the scores, half of the values' ----
-        const int quad = warp & 3, half = warp >> 2, row = quad * 32 + lane, i_pos = pos0 + row0 + row, first_pos = i_pos - lane;
+        // ---- softmax: warps q, q + 4, q + 8, q + 12 share rows 32 q .. + 31; part p has columns 16 p .. + 15 of the scores, a quarter of the values' ----
+        const int quad = warp & 3, part = warp >> 2, row = quad * 32 + lane, i_pos = pos0 + row0 + row, first_pos = i_pos - lane;
         const uint32_t lanes = (uint32_t)(quad * 32) << 16;
-        const float r1 = A.r1 ? A.r1[h] : 0.0f, r2 = A.r1 ? A.r2[h] : 0.0f, sink = A.sink ? A.sink[h] : -INFINITY, slope = A.slope ? A.slope[h] : 0.0f;
+        constexpr float kLog2e = 1.4426950408889634f;
+        const float r1 = A.r1 ? A.r1[h] : 0.0f, r2 = A.r1 ? A.r2[h] : 0.0f, sink = A.sink ? A.sink[h] * kLog2e : -INFINITY, slope = A.slope ? A.slope[h] : 0.0f;
         const int win = A.window > 0 ? A.window : 0x3fffffff;
         // the score is the scaled product alone
         const bool plain = !A.r1 && !A.slope && A.softcap == 0.0f && A.window == 0 && A.scale > 0.0f;
-        constexpr float kLog2e = 1.4426950408889634f;
-        float m = sink, l = (half == 0 && A.sink) ? 1.0f : 0.0f;
+        float m = sink, l = (part == 0 && A.sink) ? 1.0f : 0.0f;      // m in units of log2
         float o[OC];
 #pragma unroll
         for (int c = 0; c < OC; ++c) o[c] = 0.0f;
+        auto row_barrier = [&] { asm volatile("bar.sync %0, %1;" ::"r"(quad + 1), "n"(kFtParts * 32) : "memory"); };
+        auto over_parts = [&](const float (&x)[kFtParts][kFtRows]) { return (x[0][row] + x[1][row]) + (x[2][row] + x[3][row]); };
         // o += weights x values of step i, whose keys begin at j0
         auto take_product = [&](int i, int j0) {
             umma::bar_wait(&bars.o_full, i & 1);
             __syncwarp();
             umma::fence_after_sync();
             const bool sees = j0 <= i_pos && j0 + kFtKeys - 1 > i_pos - win;
+            uint32_t v[OC / 8][8];
 #pragma unroll
-            for (int c = 0; c < OC; c += 16) {
-                uint32_t v[2][8];
-                umma::tmem_ld8_issue(tm_o + half * OC + c + lanes, v[0]);
-                umma::tmem_ld8_issue(tm_o + half * OC + c + 8 + lanes, v[1]);
-                umma::tmem_ld_wait();
+            for (int x = 0; x < OC / 8; ++x) umma::tmem_ld8_issue(tm_o + part * OC + 8 * x + lanes, v[x]);
+            umma::tmem_ld_wait();
 #pragma unroll
-                for (int e = 0; e < 16; ++e) o[c + e] += sees ? __uint_as_float(v[e / 8][e % 8]) : 0.0f;
-            }
+            for (int e = 0; e < OC; ++e) o[e] += sees ? __uint_as_float(v[e / 8][e % 8]) : 0.0f;
             umma::fence_before_sync();
         };
         float inv = 0.0f;
         for (int i = 0; i < steps; ++i) {
-            const int b = i & 1, map = MAPS == 2 && i >= tiles, jt = j_start + (i - map * tiles) * kFtKeys, j0 = jt + half * 32;
+            const int b = i & 1, map = MAPS == 2 && i >= tiles, jt = j_start + (i - map * tiles) * kFtKeys, j0 = jt + part * kFtCols;
             const bool fresh = i == 0 || (MAPS == 2 && i == tiles);
             umma::bar_wait(&bars.s_full[b], (i >> 1) & 1);
             __syncwarp();
             umma::fence_after_sync();
-            float S[32];
+            float S[kFtCols];
             {
-                uint32_t v[32];
-                tmem_ld32_issue(tmem + b * kFtKeys + half * 32 + lanes, v);
+                uint32_t v[kFtCols / 8][8];
+#pragma unroll
+                for (int x = 0; x < kFtCols / 8; ++x) umma::tmem_ld8_issue(tmem + b * kFtKeys + part * kFtCols + 8 * x + lanes, v[x]);
                 umma::tmem_ld_wait();
 #pragma unroll
-                for (int e = 0; e < 32; ++e) S[e] = __uint_as_float(v[e]);
+                for (int e = 0; e < kFtCols; ++e) S[e] = __uint_as_float(v[e / 8][e % 8]);
             }
             umma::fence_before_sync();
             __syncwarp();
@@ -233,43 +264,35 @@ __global__ void __launch_bounds__(kFtThreads, 1) attn_flash_tc_kernel(const Attn
             if (MAPS == 2 && i == tiles) {
                 // the first map is complete
                 take_product(i - 1, j_start + (tiles - 1) * kFtKeys);
-                s_sum[0][half][row] = l;
-                asm volatile("bar.sync %0, 64;" ::"r"(quad + 1) : "memory");
-                inv = 1.0f / (s_sum[0][0][row] + s_sum[0][1][row]);
+                s_sum[0][part][row] = l;
+                row_barrier();
+                inv = 1.0f / over_parts(s_sum[0]);
 #pragma unroll
                 for (int c = 0; c < OC; ++c) { first_map[c * (kFtSoftWarps * 32) + threadIdx.x] = o[c] * inv; o[c] = 0.0f; }
                 m = sink;
-                l = (half == 0 && A.sink) ? 1.0f : 0.0f;
+                l = (part == 0 && A.sink) ? 1.0f : 0.0f;
             }
-            const bool direct = plain && j0 + 31 <= first_pos;
-            float mx = -INFINITY;
-            if (!direct) {
-                const bool seen = j0 + 31 <= first_pos && A.window == 0;       // every row of the warp sees every key
-                if (A.softcap > 0.0f || A.slope) {
-                    if (A.r1) ft_scores<true, true, true>(A, S, i_pos - j0, seen, win, r1, r2, slope);
-                    else ft_scores<true, false, true>(A, S, i_pos - j0, seen, win, r1, r2, slope);
-                } else if (A.r1) ft_scores<false, true, false>(A, S, i_pos - j0, seen, win, r1, r2, slope);
-                else ft_scores<false, false, false>(A, S, i_pos - j0, seen, win, r1, r2, slope);
-            }
-#pragma unroll
-            for (int e = 0; e < 32; ++e) mx = fmaxf(mx, S[e]);
-            if (direct) mx *= A.scale;
-            s_max[b][half][row] = mx;
-            asm volatile("bar.sync %0, 64;" ::"r"(quad + 1) : "memory");
-            mx = fmaxf(mx, s_max[b][half ^ 1][row]);
+            const bool seen = j0 + kFtCols - 1 <= first_pos && A.window == 0, direct = plain && seen;       // every row of the warp sees every column
+            if (!seen) ft_scores_any<true>(A, S, i_pos - j0, win, r1, r2, slope);
+            else if (!direct) ft_scores_any<false>(A, S, i_pos - j0, win, r1, r2, slope);
+            const float mul = direct ? A.scale * kLog2e : 1.0f;
+            s_max[b][part][row] = max_of(S) * mul;
+            row_barrier();
+            const float mx = fmaxf(fmaxf(s_max[b][0][row], s_max[b][1][row]), fmaxf(s_max[b][2][row], s_max[b][3][row]));
             // without a sink a row of the tile's padding (or outside a window) may have seen no key yet: keep its maximum finite
-            const float mn = fmaxf(fmaxf(m, mx), -1e30f), corr = exp2_fast((m - mn) * kLog2e);
+            const float mn = fmaxf(fmaxf(m, mx), -1e30f), corr = exp2_fast(m - mn);
             m = mn;
-            const float mul = direct ? A.scale * kLog2e : kLog2e, off = -mn * kLog2e;
             l *= corr;
-            uint32_t hi[16], lo[16];
+            uint32_t hi[kFtCols / 2], lo[kFtCols / 2];
+            float sums[2] = {0.0f, 0.0f};
 #pragma unroll
-            for (int e = 0; e < 16; ++e) {
-                const float w0 = exp2_fast(fmaf(S[2 * e], mul, off)), w1 = exp2_fast(fmaf(S[2 * e + 1], mul, off));
-                l += w0 + w1;
+            for (int e = 0; e < kFtCols / 2; ++e) {
+                const float w0 = exp2_fast(fmaf(S[2 * e], mul, -mn)), w1 = exp2_fast(fmaf(S[2 * e + 1], mul, -mn));
+                sums[e % 2] += w0 + w1;
                 hi[e] = pack_bf16(w0, w1);
                 lo[e] = pack_bf16(w0 - bf_lo(hi[e]), w1 - bf_hi(hi[e]));
             }
+            l += sums[0] + sums[1];
             if (!fresh) {
                 take_product(i - 1, jt - kFtKeys);
 #pragma unroll
@@ -277,8 +300,8 @@ __global__ void __launch_bounds__(kFtThreads, 1) attn_flash_tc_kernel(const Attn
             }
             // (the product of the step before is complete: its weights are no longer read)
 #pragma unroll
-            for (int c = 0; c < 4; ++c) {
-                unsigned char* to = Ps + sw128_at(row, half * 4 + c);
+            for (int c = 0; c < kFtCols / 8; ++c) {
+                unsigned char* to = Ps + sw128_at(row, part * (kFtCols / 8) + c);
                 *reinterpret_cast<uint4*>(to) = make_uint4(hi[4 * c], hi[4 * c + 1], hi[4 * c + 2], hi[4 * c + 3]);
                 *reinterpret_cast<uint4*>(to + kFtPBytes) = make_uint4(lo[4 * c], lo[4 * c + 1], lo[4 * c + 2], lo[4 * c + 3]);
             }
@@ -287,9 +310,9 @@ __global__ void __launch_bounds__(kFtThreads, 1) attn_flash_tc_kernel(const Attn
             if (lane == 0) bar_arrive(&bars.p_full);
         }
         take_product(steps - 1, j_start + (tiles - 1) * kFtKeys);
-        s_sum[1][half][row] = l;
-        asm volatile("bar.sync %0, 64;" ::"r"(quad + 1) : "memory");
-        inv = 1.0f / (s_sum[1][0][row] + s_sum[1][1][row]);
+        s_sum[1][part][row] = l;
+        row_barrier();
+        inv = 1.0f / over_parts(s_sum[1]);
         float scale = inv;
         if (MAPS == 2) {
             float ss = 0.0f;
@@ -298,15 +321,15 @@ __global__ void __launch_bounds__(kFtThreads, 1) attn_flash_tc_kernel(const Attn
                 o[c] = fmaf(-A.diff_lambda, o[c] * inv, first_map[c * (kFtSoftWarps * 32) + threadIdx.x]);
                 ss = fmaf(o[c], o[c], ss);                                      // columns beyond dv hold zeros
             }
-            s_max[0][half][row] = ss;
-            asm volatile("bar.sync %0, 64;" ::"r"(quad + 1) : "memory");
-            scale = A.diff_scale / sqrtf((s_max[0][0][row] + s_max[0][1][row]) / (float)A.dv + A.eps);
+            s_max[0][part][row] = ss;
+            row_barrier();
+            scale = A.diff_scale / sqrtf(over_parts(s_max[0]) / (float)A.dv + A.eps);
         }
         if (row0 + row < n) {
             const size_t t = t0 + row0 + row;
 #pragma unroll
             for (int c = 0; c < OC; c += 8) {
-                const int col = half * OC + c;
+                const int col = part * OC + c;
                 if (col < A.dv) {
                     float v[8];
 #pragma unroll

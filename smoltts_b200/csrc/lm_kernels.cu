@@ -2716,15 +2716,18 @@ static cudaError_t launch_group_scan_any(SmolLm* m, const GroupScanArgs& A, floa
     return launch_group_scan<256, DELTA>(A, n_seqs, pool, o_raw, st, min_smem);
 }
 
-// attn_flash_tc_kernel where a sequence brings more than kFtMinRows tokens and every row it copies is made of whole 16-byte pieces.
-// False: not launched (few tokens, unaligned rows, sizes it is not built for).
+// attn_flash_tc_kernel where every row it copies is made of whole 16-byte pieces.  False: not launched (unaligned rows, sizes it is not built
+// for).  Against attn_flash_kernel it is the faster one from 16 tokens on (16 tokens, 12 heads of 64, after 0 / 1500 others: 11 / 46 us, 16 / 113).
+// Two maps it takes one after the other, attn_flash_kernel side by side: there it is left out as long as the 64-row blocks of that kernel have
+// an SM each (512 tokens, 6 heads: 63 us against 56; 3 x 1000 tokens: 97 against 116).
 template <int MAPS>
 static bool launch_flash_tc(const AttnArgs& A, int n_seqs, int max_n, const bf16* qbuf, const bf16* pool, bf16* out, cudaStream_t st) {
     const size_t rows = A.d | A.dv | A.out_ld | A.page_elems | A.k_off | A.k_ld | (A.v_in_k ? 0 : A.v_off | A.v_ld);
-    if (max_n <= kFtMinRows || rows % 8 != 0 || (reinterpret_cast<uintptr_t>(qbuf) | reinterpret_cast<uintptr_t>(pool) | reinterpret_cast<uintptr_t>(out)) % 16 != 0) return false;
+    if (rows % 8 != 0 || (reinterpret_cast<uintptr_t>(qbuf) | reinterpret_cast<uintptr_t>(pool) | reinterpret_cast<uintptr_t>(out)) % 16 != 0) return false;
     if (A.dv > 128 || A.d > (MAPS == 2 ? 64 : A.v_in_k ? 192 : 128)) return false;
+    if (MAPS == 2 && (long long)A.H * n_seqs * ((max_n + 63) / 64) <= 148) return false;
     const dim3 grid(A.H, n_seqs, (max_n + kFtRows - 1) / kFtRows);
-#define SMOL_FLASH_TC(DK, DV, VK) plain_launch(attn_flash_tc_kernel<DK, DV, VK, MAPS>, grid, kFtThreads, ft_smem(DK, DV, VK, MAPS), st, A, qbuf, pool, out)
+#define SMOL_FLASH_TC(DK, DV, VK) plain_launch(attn_flash_tc_kernel<DK, DV, VK, MAPS>, grid, ft_threads(DV, MAPS), ft_smem(DK, DV, VK, MAPS), st, A, qbuf, pool, out)
     if constexpr (MAPS == 1) {
         if (A.v_in_k) {
             if (A.d <= 64) SMOL_FLASH_TC(64, 64, true);

@@ -11,11 +11,14 @@
 // Differential attention (MAPS 2) walks the keys once per map; the first map's result waits in shared memory, each thread's own part.
 //
 // What bounds it: the instructions of a step, the loaders' as much as the softmax's 64 x 128 scores with one exponential (and, with a distance
-// penalty, one logarithm) each -- hence four threads per row, whose latencies cover one another, and a warp per stage.  Two threads per row
-// and three stages: 84 / 98 / 48 / 99 us instead of the following.
-// 2048 tokens, 12 heads of 64 with a distance penalty: 64 us, attn_flash_kernel 165; 1801 tokens, 12 heads of 128: 82 against 219; 1024
-// tokens, 12 heads over a latent of 160: 42 against 101; 3 x 1000 tokens, 6 heads of two maps: 97 against 116.
+// penalty, one logarithm) each -- hence four threads per row, whose latencies cover one another, a warp per stage, and addresses that advance
+// by constants.  Two threads per row and three stages: 84 / 98 / 48 / 99 us instead of the following; a look at the page, the limit and the
+// swizzle for every row copied: 64 / 82 / 42 / 97.
+// 2048 tokens, 12 heads of 64 with a distance penalty: 57 us, attn_flash_kernel 165; 1801 tokens, 12 heads of 128: 74 against 219; 1024
+// tokens, 12 heads over a latent of 160: 40 against 101; 3 x 1000 tokens, 6 heads of two maps: 72 against 116.
 #pragma once
+
+#include <type_traits>
 
 namespace smol {
 namespace lm {
@@ -157,7 +160,28 @@ __global__ void __launch_bounds__(ft_threads(DV, MAPS), 1) attn_flash_tc_kernel(
             if (i >= NB) umma::bar_wait(&bars.empty[st], (i / NB - 1) & 1);
             __syncwarp();
             // 64 rows of a head into blocks of 64 columns, eight lanes per row, four rows at a time; zeros beyond `width` and last_pos
-            auto copy = [&](unsigned char* to, int blocks, size_t off, int head, int ld, int width) {
+            auto copy = [&](unsigned char* to, auto blocks_of, size_t off, int head, int ld, int width) {
+                constexpr int blocks = decltype(blocks_of)::value;
+                if (one_page && j0 + kFtKeys - 1 <= last_pos) {
+                    // whole rows of one page: addresses advance by constants (rows y 4 .. + 3: the swizzle alternates with y)
+                    const bf16* p = page[0] + off + ((size_t)head * A.page_size + in_page[0] + (lane >> 3)) * ld;
+                    const uint32_t d = umma::s2u(to) + (lane >> 3) * 128;
+                    const uint32_t d01[2] = {d + (((lane & 7) ^ (lane >> 3)) << 4), d + (((lane & 7) ^ (4 + (lane >> 3))) << 4)};
+                    uint32_t bytes[blocks];
+                    int col[blocks];
+#pragma unroll
+                    for (int cb = 0; cb < blocks; ++cb) {
+                        const int c = cb * 64 + (lane & 7) * 8;
+                        bytes[cb] = c < width ? 16 : 0;
+                        col[cb] = c < width ? c : 0;
+                    }
+#pragma unroll
+                    for (int y = 0; y < 16; ++y, p += 4 * (size_t)ld)
+#pragma unroll
+                        for (int cb = 0; cb < blocks; ++cb)
+                            asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d01[y & 1] + y * 512 + cb * (kFtKeys * 128)), "l"(p + col[cb]), "r"(bytes[cb]) : "memory");
+                    return;
+                }
 #pragma unroll
                 for (int x = 0; x < 2; ++x) {
                     const bf16* at = page[x] + off + ((size_t)head * A.page_size + in_page[x]) * ld;
@@ -174,8 +198,8 @@ __global__ void __launch_bounds__(ft_threads(DV, MAPS), 1) attn_flash_tc_kernel(
                     }
                 }
             };
-            copy(Kt, DK / 64, A.k_off, g * MAPS + map, A.k_ld, A.d);
-            if (!VK) copy(Kt + kFtKeys * DK * 2, DV / 64, A.v_off, g, A.v_ld, A.dv);
+            copy(Kt, std::integral_constant<int, DK / 64>{}, A.k_off, g * MAPS + map, A.k_ld, A.d);
+            if (!VK) copy(Kt + kFtKeys * DK * 2, std::integral_constant<int, DV / 64>{}, A.v_off, g, A.v_ld, A.dv);
             cp_async_commit_group();
             cp_async_wait_group<0>();
             umma::fence_async_smem();

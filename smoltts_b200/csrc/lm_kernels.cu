@@ -1241,7 +1241,8 @@ __global__ void __launch_bounds__(kMergeWarps * MAPS * 32) attn_merge_kernel(con
 }
 
 // ---------------------------------------------------------------------------------------------------------------------
-// Attention for prompt portions, bf16, on the tensor cores (mma.sync m16n8k16, fp32 accumulation).  One block per
+// Attention for prompt portions, bf16, on mma.sync m16n8k16 (fp32 accumulation): the forms that attn_flash_tc_kernel does not serve (see
+// launch_flash_tc).  One block per
 // (64-row tile of a sequence's rows in this step, sequence, query head); each of the four warps owns 16 rows.  Keys and
 // values are staged 64 positions at a time from the paged pool into shared memory (head sizes padded with zeros to DP).
 // Scores, the distance penalty, the running maximum and the softmax weights are fp32; for the weights x values product a
@@ -2719,7 +2720,7 @@ static cudaError_t launch_group_scan_any(SmolLm* m, const GroupScanArgs& A, floa
 // attn_flash_tc_kernel where every row it copies is made of whole 16-byte pieces.  False: not launched (unaligned rows, sizes it is not built
 // for).  Against attn_flash_kernel it is the faster one from 16 tokens on (16 tokens, 12 heads of 64, after 0 / 1500 others: 11 / 46 us, 16 / 113).
 // Two maps it takes one after the other, attn_flash_kernel side by side: there it is left out as long as the 64-row blocks of that kernel have
-// an SM each (512 tokens, 6 heads: 63 us against 56; 3 x 1000 tokens: 97 against 116).
+// an SM each (512 tokens, 6 heads: 63 us against 56, measured when 3 x 1000 tokens took 97; those take 72 now against 116).
 template <int MAPS>
 static bool launch_flash_tc(const AttnArgs& A, int n_seqs, int max_n, const bf16* qbuf, const bf16* pool, bf16* out, cudaStream_t st) {
     const size_t rows = A.d | A.dv | A.out_ld | A.page_elems | A.k_off | A.k_ld | (A.v_in_k ? 0 : A.v_off | A.v_ld);

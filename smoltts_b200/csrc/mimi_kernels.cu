@@ -7,7 +7,7 @@
 // same bits alone or in any batch.
 //
 // At streaming batch sizes every stage is a handful of rows (2 .. 1920 per stream) against a weight matrix that is read
-// once: weight-streaming "row" products.  ONE kernel shape carries them all (rows_kernel): a CTA stages up to 16 input
+// once: weight-streaming "row" products (rows_kernel): a CTA stages up to 16 input
 // rows in shared memory -- gathered straight from the producer's buffer, im2col of a causal convolution = a contiguous run
 // of (kernel x channels) floats that begins in the carried history rows; LayerNorm applied while staging -- and every
 // warp streams one weight row with 16-byte loads against all staged rows, finishing with a shuffle reduction and a fused
@@ -17,7 +17,7 @@
 // tiles on packed FMAs (tile_kernel), the one-channel last convolution from shared memory (rowdot_kernel).  Attention: one CTA per (stream, head, split
 // of 512 cached positions), partial softmaxes combined in split order.  Everything a stream carries (convolution history
 // rows, the upsampler's previous embedding, KV cache, position) lives in per-slot arenas of the caller's workspace; a step is
-// a program of 57 operations, one launch each, replayed as one CUDA graph.
+// a program of 57 operations (and the LayerNorms where the Linears run on tiles), one launch each, replayed as one CUDA graph.
 //
 // Reference map (C = mlx_inference/src/smoltts_mlx/codec/): RVQ decode C/rvq.py:118-130,171-186; upsample C/conv.py:225-282;
 // transformer C/transformer.py:36-150; Conv1d.step C/conv.py:133-160; ConvTranspose1d.step C/conv.py:207-221; residual

@@ -68,7 +68,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) gemm_tc_kernel(const __grid_con
     __syncthreads();
     umma::fence_after_sync();
     const uint32_t tmem = bars.tmem;
-    if (warp != 2 || io.tile_group) dep_wait();      // a plain product's weights need not wait for the kernel before
+    if (warp != 2 || io.tile_group) dep_wait();      // a plain product's weights need not wait for the kernel before (smol_lm_linear, whose w that may have made, launches plainly)
     dep_go();
     const int m_tiles = io.tile_group ? *io.n_tiles : (M + umma::kM - 1) / umma::kM, n_tiles = (N + BN - 1) / BN;
     const int tiles = m_tiles * n_tiles, nk = (K + umma::kBK - 1) / umma::kBK;

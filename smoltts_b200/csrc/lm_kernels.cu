@@ -578,7 +578,7 @@ __global__ void __launch_bounds__(WARPS * 32) gemm_few_kernel(const bf16* __rest
             for (int i = 0; i < WT; ++i) p[u][i] = k + tq * 8 < K ? ldg_stream(wr[i] + k) : zero;
         }
     };
-    load_weights(warp * 32);             // no kernel writes weights: the first ones are on their way before the wait
+    load_weights(warp * 32);             // no kernel of a step writes weights: the first ones are on their way before the wait (smol_lm_linear launches plainly)
     dep_wait();
     dep_go();
     for (int k0 = warp * 32; k0 < K; k0 += WARPS * 32 * U) {
@@ -3606,6 +3606,8 @@ extern "C" int smol_lm_step(SmolLm* m, const SmolLmStep* s, void* stream) {
 extern "C" int smol_lm_linear(SmolLm* m, const void* d_a, const void* d_w, float* d_y, int32_t M, int32_t N, int32_t K, void* stream) {
     if (!m || !d_a || !d_w || !d_y || M < 1 || N < 1 || K < 1) return fail(SMOL_ERR_INVALID, "smol_lm_linear: bad argument");
     cudaStream_t st = static_cast<cudaStream_t>(stream);
+    // w is the caller's: the kernel in front may have made it, and the products read w before they wait for that kernel
+    t_plain_next = true;
     if (m->cfg.dtype == SMOL_LM_F32) CU(linear<float>(m, static_cast<const float*>(d_a), static_cast<const float*>(d_w), d_y, M, N, K, st));
     else CU(linear<bf16>(m, static_cast<const bf16*>(d_a), static_cast<const bf16*>(d_w), d_y, M, N, K, st));
     return SMOL_OK;

@@ -230,7 +230,8 @@ class MimiModel:
         if len(self._free) < n:
             raise RuntimeError(f"MimiModel: all {self.max_streams} stream slots are in use (release_cache() one)")
         slots = [self._free.pop() for _ in range(n)]
-        self._reset(slots)
+        if slots:
+            self._reset(slots)
         return [MimiCache(s) for s in slots]
 
     def release_cache(self, cache: MimiCache) -> None:
@@ -295,25 +296,28 @@ class MimiModel:
         frames per step where they give the same bits.
         With ``upsample_carry=True`` this equals the reference's whole-sequence ``decode`` (codec/mimi.py:88-100); with the
         default it is what a run of the reference's ``decode_step`` calls produces."""
-        B, _, T = audio_codes.shape
-        own = cache is None
-        caches = self._open(B) if own else list(cache)
-        if len(caches) != B or audio_codes.shape[1] != self.num_codebooks:
-            raise ValueError(f"decode: codes {tuple(audio_codes.shape)} vs {len(caches)} caches x {self.num_codebooks} codebooks")
-        if len({c.slot for c in caches}) != B:
+        B, n_q, T = audio_codes.shape
+        own, n = cache is None, self.samples_per_frame
+        caches = [] if own else list(cache)
+        if T and n_q != self.num_codebooks or not own and len(caches) != B:
+            raise ValueError(f"decode: codes {tuple(audio_codes.shape)} vs {B if own else len(caches)} caches x {self.num_codebooks} codebooks")
+        if not own and len({c.slot for c in caches}) != B:
             raise ValueError("decode: two rows of the batch name the same stream")
-        n = self.samples_per_frame
-        out = torch.empty(B, 1, T * n, dtype=torch.float32, device=self.device)
-        codes = audio_codes.to(self.device).transpose(1, 2)
-        most = max(1, int(self._lib.smol_mimi_max_frames(self._h, B)))
-        t = 0
-        while t < T:
-            frames = min(most, T - t)
-            out[:, 0, t * n:(t + frames) * n] = self._run(codes[:, t:t + frames], caches)
-            t += frames
+        if own and T > self.max_frames:
+            raise RuntimeError(f"MimiModel: {T} frames against max_frames = {self.max_frames}")
         if own:
-            for c in caches:
-                self.release_cache(c)
+            caches = self._open(B)
+        try:
+            out = torch.empty(B, 1, T * n, dtype=torch.float32, device=self.device)
+            codes = audio_codes.to(self.device).transpose(1, 2)
+            most = max(1, int(self._lib.smol_mimi_max_frames(self._h, B)))
+            for t in range(0, T, most):
+                frames = min(most, T - t)
+                out[:, 0, t * n:(t + frames) * n] = self._run(codes[:, t:t + frames], caches)
+        finally:
+            if own:
+                for c in caches:
+                    self.release_cache(c)
         return out
 
     def flops_per_frame(self) -> int:

@@ -69,6 +69,19 @@ def test_steps_match_transformers_goldens_under_both_upsampling_rules():
     _close("decode() helper", carry.decode(codes), g["full"])
 
 
+def test_refused_decodes_leave_every_slot_free():
+    m = _model(max_streams=2, max_frames=4)
+    for codes in (torch.zeros(2, 7, 3, dtype=torch.int64), torch.zeros(2, 8, 5, dtype=torch.int64)):
+        for _ in range(2):
+            with pytest.raises((ValueError, RuntimeError)):
+                m.decode(codes)
+    with pytest.raises(ValueError):
+        m.decode(torch.zeros(2, 8, 3, dtype=torch.int64), [m_cache := m.make_cache()])
+    m.release_cache(m_cache)
+    assert m.decode(torch.zeros(2, 8, 4, dtype=torch.int64)).shape == (2, 1, 4 * 1920)
+    assert m.decode(torch.zeros(2, 8, 0, dtype=torch.int64)).shape == (2, 1, 0)
+
+
 def test_transformer_output_matches_goldens():
     g = np.load(f"{GOLDEN_DIR}/mimi.npz")
     codes = torch.from_numpy(g["codes"]).long()

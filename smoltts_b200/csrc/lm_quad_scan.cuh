@@ -344,10 +344,12 @@ __global__ void __launch_bounds__(kQuadThreads, 1) quad_scan_kernel(const QuadAr
             val[0] = keep + __shfl_xor_sync(0xffffffffu, send, 1);
         }
         float o = val[0];
+        // of the tokens after mt the output takes nothing, also where they are not finite (their products in the record are zeros)
+        const float v1 = mt >= 1 ? v[1] : 0.0f, v2 = mt >= 2 ? v[2] : 0.0f, v3 = mt >= 3 ? v[3] : 0.0f;
         if (FORM == kFormAdd) {
             o += __shfl_xor_sync(0xffffffffu, o, 4);
             const float4 kr = pr[mt];
-            o = fmaf(kr.x, v[0], o); o = fmaf(kr.y, v[1], o); o = fmaf(kr.z, v[2], o); o = fmaf(kr.w, v[3], o);
+            o = fmaf(kr.x, v[0], o); o = fmaf(kr.y, v1, o); o = fmaf(kr.z, v2, o); o = fmaf(kr.w, v3, o);
         } else {
             float b[4];
 #pragma unroll
@@ -359,8 +361,8 @@ __global__ void __launch_bounds__(kQuadThreads, 1) quad_scan_kernel(const QuadAr
             const float s2 = fmaf(a2.y, s1, fmaf(a2.x, s0, fmaf(k2.y, v[1], fmaf(k2.x, v[0], b[2]))));
             const float s3 = fmaf(a3.z, s2, fmaf(a3.y, s1, fmaf(a3.x, s0, fmaf(k3.z, v[2], fmaf(k3.y, v[1], fmaf(k3.x, v[0], b[3]))))));
             const float4 ar = pr[mt * PW + 2], kr = pr[mt * PW + 3];
-            o = fmaf(kr.x, v[0], o); o = fmaf(kr.y, v[1], o); o = fmaf(kr.z, v[2], o); o = fmaf(kr.w, v[3], o);
-            o = fmaf(ar.x, s0, o); o = fmaf(ar.y, s1, o); o = fmaf(ar.z, s2, o); o = fmaf(ar.w, s3, o);
+            o = fmaf(kr.x, v[0], o); o = fmaf(kr.y, v1, o); o = fmaf(kr.z, v2, o); o = fmaf(kr.w, v3, o);
+            o = fmaf(ar.x, s0, o); o = fmaf(ar.y, mt >= 1 ? s1 : 0.0f, o); o = fmaf(ar.z, mt >= 2 ? s2 : 0.0f, o); o = fmaf(ar.w, mt >= 3 ? s3 : 0.0f, o);
             const unsigned long long z[4] = {both(s0), both(s1), both(s2), both(s3)};
 #pragma unroll
             for (int e = 0; e < RV; ++e)

@@ -116,6 +116,34 @@ def test_four_token_scan_of_prompts(dim):
             at += n
 
 
+def test_tokens_take_nothing_from_later_ones_in_the_four_token_scan():
+    """A token that is not finite leaves the logits of every earlier one as they are, whatever its place among the scan's four."""
+    import maferax_util as mu
+
+    bad = 60
+    cases = [(config([delta(heads=3, dim=16, ff=0, rank=5)], vocab=61, width=48), engine_and_oracle),
+             (mu.config([mu.gla(heads=2, dim=16, vdim=11)], vocab=61, width=48), mu.engine_and_oracle)]
+
+    def spoil(w):
+        w["embed"][bad] = float("nan")
+
+    for cfg, make in cases:
+        model, _, _ = make(cfg, seed=5, edit=spoil, max_step_tokens=256)
+        toks = [t % bad for t in tokens(27, 61, 1)]
+
+        def logits(row):
+            seq = model.open_sequence()
+            out = model.forward([(seq, row, list(range(len(row))))]).clone()
+            model.close_sequence(seq)
+            return out
+
+        want = logits(toks)
+        for at in range(19, 26):
+            got = logits(toks[:at] + [bad] + toks[at + 1:])
+            assert torch.equal(got[:at], want[:at])
+            assert not bool(got[at:].isfinite().any())
+
+
 @pytest.mark.parametrize("streams,frames", [(1, 11), (3, 5), (8, 3), (11, 2), (12, 9), (17, 6)])
 def test_codec_runs_of_frames_equal_single_steps(streams, frames):
     """decode() takes up to 8 frames of few streams, 4 of many, at once: bit for bit what decode_step returns frame by frame."""

@@ -2485,12 +2485,12 @@ template <int BM, int BN, int TM, int TN>
 static cudaError_t launch_f32_tile(const float* a, const float* w, float* y, int M, int N, int K, const GemmIo& io, int batch, int row_tiles, cudaStream_t st) {
     using T = smol::f32t::Tile<BM, BN, TM, TN>;
     const int cols = (N + BN - 1) / BN;
-    // CTAs per tile: as many as bring the grid to about six per SM (four of a 64 x 64 tile's run side by side; fewer leave its FMAs waiting
-    // for loads and some SMs with a third more work than others), each with at least 128 k
+    // CTAs per tile: as many as bring the grid of a single row of tiles to about four per SM, each with at least 128 k.  From N, K and the
+    // batch alone: a row's sums must not depend on how many rows the step holds.  (With S from the rows as well 1024 rows of 4608 x 768 took 179 us, 201 now,
+    // and 343 without a split; 300 rows 74 either way.)
     int S = 1;
-    while (S < 8 && (long long)cols * row_tiles * batch * S < 4 * 148 && K / (2 * S) >= 128) S *= 2;
-    if (T::kSmemBytes > 48 * 1024)
-        if (const cudaError_t e = cudaFuncSetAttribute(gemm_f32_tile_kernel<BM, BN, TM, TN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)T::kSmemBytes)) return e;
+    while (S < 8 && (long long)cols * batch * S < 4 * 148 && K / (2 * S) >= 128) S *= 2;
+    static_assert(T::kSmemBytes <= 48 * 1024, "no attribute needed");
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3(cols * S, row_tiles, batch);
     cfg.blockDim = dim3(T::NT);

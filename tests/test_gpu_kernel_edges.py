@@ -67,12 +67,23 @@ F32_TILES = ((1, 1, 4), (16, 65, 36), (17, 64, 128), (64, 63, 132), (65, 130, 26
 
 @pytest.mark.parametrize("M,N,K", F32_TILES)
 def test_float32_products(M, N, K):
-    """16-, 64- and 128-row tiles, steps of 16 k with a ragged last one, K shared by 1 to 8 thread blocks."""
+    """16- and 64-row tiles, steps of 16 k with a ragged last one, K shared by 1 to 8 thread blocks."""
     model, _, _ = engine_and_oracle(config([attn(ff=0)]), seed=9)
     g = torch.Generator(device="cuda").manual_seed(M * 31 + K)
     a, w = (torch.randn(r, K, device="cuda", generator=g) for r in (M, N))
     err = (model.linear(a, w).double() - a.double() @ w.double().T).abs()
     assert bool((err <= product_bound(a, w)).all())
+
+
+@pytest.mark.parametrize("N,K", [(768, 768), (4608, 768), (96, 4608), (2400, 1028), (70, 70)])
+def test_float32_rows_do_not_depend_on_their_number(N, K):
+    """A float32 row's product has the same bits whatever the number of rows beside it."""
+    model, _, _ = engine_and_oracle(config([attn(ff=0)]), seed=9)
+    g = torch.Generator(device="cuda").manual_seed(N + K)
+    a, w = (torch.randn(r, K, device="cuda", generator=g) for r in (1300, N))
+    whole = model.linear(a, w)
+    for M in (1, 16, 17, 64, 65, 300, 700):
+        assert torch.equal(model.linear(a[:M], w), whole[:M]), M
 
 
 @pytest.mark.parametrize("n", [127, 128, 129, 135, 136])

@@ -68,16 +68,16 @@ struct Tile {
     __device__ static __forceinline__ int column_at(int p) { return column(p % THN, p / THN); }
 
     // k in [k_lo, k_hi) (multiples of 4).  a_row(r) / w_row(r): a row's address, nullptr for zeros; a_at(k): where in its row k lies.
-    // shape(v, r, k): what becomes of 4 floats of A before they are multiplied (SHAPE; called once per piece by the thread that copied it).
     // before(): called after the first copies of W are on their way and before anything of A is read.
-    template <bool SHAPE, class ARow, class AAt, class WRow, class Shape, class Before>
-    __device__ static __forceinline__ void product(float* sm, int k_lo, int k_hi, ARow a_row, AAt a_at, WRow w_row, Shape shape, Before before, float (&out)[TM][TN]) {
+    // RUN > 0: the two chains of an output are added up and begin anew every RUN steps.
+    template <int RUN, class ARow, class AAt, class WRow, class Before>
+    __device__ static __forceinline__ void product(float* sm, int k_lo, int k_hi, ARow a_row, AAt a_at, WRow w_row, Before before, float (&out)[TM][TN]) {
         const int tid = threadIdx.x, row_y = ty(), row_x = tx(), kp = (tid & 3) * 4;      // kp: this thread's place in a step
         unsigned long long acc[TM][TN];
 #pragma unroll
         for (int i = 0; i < TM; ++i)
 #pragma unroll
-            for (int j = 0; j < TN; ++j) acc[i][j] = 0ull;
+            for (int j = 0; j < TN; ++j) { acc[i][j] = 0ull; out[i][j] = 0.0f; }
         const int steps = (k_hi - k_lo + kBK - 1) / kBK;
         const float *ap[PA], *wp[PW], *any = w_row(0);      // (column 0 is always there)
 #pragma unroll
@@ -118,18 +118,8 @@ struct Tile {
             commit();
         }
         for (int s = 0; s < steps; ++s) {
-            float* As = sm + (s % kStages) * kStageFloats;
-            const float* Ws = As + BM * kLD;
+            const float *As = sm + (s % kStages) * kStageFloats, *Ws = As + BM * kLD;
             wait<kStages - 2>();
-            if (SHAPE) {
-#pragma unroll
-                for (int x = 0; x < PA; ++x) {
-                    const int r = (tid + x * NT) >> 2, k = k_lo + s * kBK + kp;
-                    if (BM * 4 % NT != 0 && r >= BM) break;
-                    float4* p = reinterpret_cast<float4*>(As + r * kLD + kp);
-                    if (k < k_hi) *p = shape(*p, r, k);
-                }
-            }
             __syncthreads();
             if (s + kStages - 1 < steps) { copy_w(s + kStages - 1); copy_a(s + kStages - 1); }
             commit();
@@ -149,12 +139,18 @@ struct Tile {
 #pragma unroll
                     for (int j = 0; j < TN; ++j) acc[i][j] = fma2(a[i].y, w[j].y, acc[i][j]);
             }
+            if (RUN > 0 && s % RUN == RUN - 1) {
+#pragma unroll
+                for (int i = 0; i < TM; ++i)
+#pragma unroll
+                    for (int j = 0; j < TN; ++j) { out[i][j] += pair_sum(acc[i][j]); acc[i][j] = 0ull; }
+            }
         }
         wait<0>();
 #pragma unroll
         for (int i = 0; i < TM; ++i)
 #pragma unroll
-            for (int j = 0; j < TN; ++j) out[i][j] = pair_sum(acc[i][j]);
+            for (int j = 0; j < TN; ++j) out[i][j] += pair_sum(acc[i][j]);
     }
 
     // Hands the outputs of the tile to done(row, column, four values) -- four columns from a multiple of 4 on: straight from the

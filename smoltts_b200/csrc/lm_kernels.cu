@@ -310,9 +310,8 @@ __global__ void __launch_bounds__(f32t::Tile<BM, BN, TM, TN>::NT) gemm_f32_tile_
     int k_lo, k_hi;
     T::range(K, k_lo, k_hi);
     float out[TM][TN];
-    T::template product<false>(f32_sm, k_lo, k_hi, [&](int r) { return arow[r] >= 0 ? a + arow[r] : nullptr; }, [](int k) -> long long { return k; },
-                               [&](int r) { return n0 + r < N ? w + (size_t)(n0 + r) * K : nullptr; },
-                               [](float4 v, int, int) { return v; }, [] {}, out);
+    T::template product<0>(f32_sm, k_lo, k_hi, [&](int r) { return arow[r] >= 0 ? a + arow[r] : nullptr; }, [](int k) -> long long { return k; },
+                           [&](int r) { return n0 + r < N ? w + (size_t)(n0 + r) * K : nullptr; }, [] {}, out);
     const bool whole = io.ldy % 4 == 0 && reinterpret_cast<uintptr_t>(y) % 16 == 0;
     T::finish(f32_sm, out, [&](int r, int c, float4 v) {
         if (m0 + r >= M) return;

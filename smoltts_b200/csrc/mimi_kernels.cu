@@ -364,10 +364,10 @@ __global__ void __launch_bounds__(kThreads) lin_kernel(const RowOp op) {
 // where the rows were written, LayerNorm by norm_kernel in front.  K is shared by a cluster of CTAs where an operation has few tiles.
 // What an output is added up from -- which k a rank takes, its two chains, the order of ranks -- follows from the operation and the class
 // of the batch (fewer than 12 streams | 12+) alone, not from the tile's shape, so a stream's bits are the same in any batch of a class.
-// Bound by the FMAs and, with them in balance, shared-memory loads (f32_tile.cuh): 48 streams, 4 frames at once, 3.2 ms for 83 GFLOP (26
+// Bound by the FMAs and, with them in balance, shared-memory loads (f32_tile.cuh): 48 streams, 4 frames at once, 3.59 ms for 83 GFLOP (23
 // TFLOP/s; 64 x 64 plain-FMA tiles of 4 x 4 outputs and a warp per weight row before: 1.75 ms per single frame).  128 x 128 tiles of
 // 256 threads, ELU and LayerNorm applied by every block that reads the rows: 5.9 ms.
-template <int BM, int BN, int TM, int TN>
+template <int BM, int BN, int TM, int TN, int RUN>
 __global__ void __launch_bounds__(f32t::Tile<BM, BN, TM, TN>::NT) tile_kernel(const RowOp op) {
     using T = f32t::Tile<BM, BN, TM, TN>;
     extern __shared__ __align__(16) float tile_sm[];
@@ -385,13 +385,12 @@ __global__ void __launch_bounds__(f32t::Tile<BM, BN, TM, TN>::NT) tile_kernel(co
     int k_lo, k_hi;
     T::range(op.K, k_lo, k_hi);
     float out[TM][TN];
-    T::template product<false>(tile_sm, k_lo, k_hi,
-                               [&](int r) -> const float* {
-                                   return s_slot[r] < 0 ? nullptr : op.in + (long long)s_slot[r] * op.in_stride + (long long)(op.in_hs + s_t[r] + op.tap0) * op.in_c;
-                               },
-                               [&](int k) -> long long { return k >= turn ? k - 2 * op.in_c : k; },
-                               [&](int r) { return n0 + r < op.N ? op.W + (long long)(n0 + r) * op.K : nullptr; }, [](float4 v, int, int) { return v; },
-                               [] { pdl_wait(); pdl_go(); }, out);
+    T::template product<RUN>(tile_sm, k_lo, k_hi,
+                             [&](int r) -> const float* {
+                                 return s_slot[r] < 0 ? nullptr : op.in + (long long)s_slot[r] * op.in_stride + (long long)(op.in_hs + s_t[r] + op.tap0) * op.in_c;
+                             },
+                             [&](int k) -> long long { return k >= turn ? k - 2 * op.in_c : k; },
+                             [&](int r) { return n0 + r < op.N ? op.W + (long long)(n0 + r) * op.K : nullptr; }, [] { pdl_wait(); pdl_go(); }, out);
     T::finish(tile_sm, out, [&](int r, int c, float4 y) {
         const int n = n0 + c;
         if (s_slot[r] >= 0 && n < op.N) store_row4(op, s_b[r], s_slot[r], s_t[r], n, y);      // (N is a multiple of 4)
@@ -444,13 +443,17 @@ __global__ void __launch_bounds__(kThreads) rowdot_kernel(const RowOp op) {
     }
     __syncthreads();
     const int t = tid >> 2, q = tid & 3;
-    float acc = 0.f;
+    float part[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
     if (t < n)
         for (int j = 0; j < taps; ++j)
-            for (int c = q * 4; c < op.in_c; c += 16) {
+            for (int c = q * 4; c < op.in_c; c += 32) {
                 const float4 v = *reinterpret_cast<const float4*>(a + (t + j) * ld + c), ww = *reinterpret_cast<const float4*>(w + j * op.in_c + c);
-                acc = fmaf(v.x, ww.x, acc); acc = fmaf(v.y, ww.y, acc); acc = fmaf(v.z, ww.z, acc); acc = fmaf(v.w, ww.w, acc);
+                part[0] = fmaf(v.x, ww.x, part[0]); part[1] = fmaf(v.y, ww.y, part[1]); part[2] = fmaf(v.z, ww.z, part[2]); part[3] = fmaf(v.w, ww.w, part[3]);
+                if (c + 16 >= op.in_c) break;
+                const float4 v2 = *reinterpret_cast<const float4*>(a + (t + j) * ld + c + 16), w2 = *reinterpret_cast<const float4*>(w + j * op.in_c + c + 16);
+                part[4] = fmaf(v2.x, w2.x, part[4]); part[5] = fmaf(v2.y, w2.y, part[5]); part[6] = fmaf(v2.z, w2.z, part[6]); part[7] = fmaf(v2.w, w2.w, part[7]);
             }
+    float acc = ((part[0] + part[4]) + (part[1] + part[5])) + ((part[2] + part[6]) + (part[3] + part[7]));
     acc += __shfl_xor_sync(0xffffffffu, acc, 1);
     acc += __shfl_xor_sync(0xffffffffu, acc, 2);
     if (q == 0 && t < n) op.out[(long long)(op.out_by_row ? b : slot) * op.out_stride + op.out_off0 + t0 + t] = acc + (op.bias ? op.bias[0] : 0.f);
@@ -1001,15 +1004,17 @@ constexpr int kTileMinBatch = 12;   // the class of 12+ streams
 static int rows_per_frame(const RowOp& op) { return op.T / op.frames; }
 // Operations on the packed-FMA tiles: see tile_kernel.  (Fewer than 12 streams: an operation of two rows per frame streams its weights
 // through rows_kernel / lin_kernel, which read them once for up to 16 rows.)
+// Fewer streams: partial sums of 16 k (f32_tile.cuh).  Error of the samples against 64 bits, mean over five sets of weights: 4.2e-7 (4.3e-7 of
+// rows_kernel's 32 chains); without partial sums 5.5e-7, of 64 k 4.6e-7, of 32 k 4.3e-7.  8 steps of one stream take 2.41 to 2.45 ms with any.
+constexpr int kFewStreamRun = 1;
 static bool use_tile(const RowOp& op) {
     return (op.batch >= kTileMinBatch || rows_per_frame(op) >= 16) && op.N >= 16 && op.N % 4 == 0 && op.bias_mod % (op.bias ? 4 : 1) == 0 && op.K % 4 == 0 && op.in_c % 4 == 0 &&
            (op.tapstep > 0 || op.K == 2 * op.in_c) && (op.pro == PRO_NONE || (op.norm_at && op.K <= 32 * kNormRegs));
 }
-template <int BM, int BN, int TM, int TN>
-static cudaError_t launch_tile(const RowOp& op, int split, cudaStream_t st) {
+template <int BM, int BN, int TM, int TN, int RUN>
+static cudaError_t launch_tile_run(const RowOp& op, int split, cudaStream_t st) {
     using T = smol::f32t::Tile<BM, BN, TM, TN>;
-    if (T::kSmemBytes > 48 * 1024)
-        if (const cudaError_t e = cudaFuncSetAttribute(tile_kernel<BM, BN, TM, TN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)T::kSmemBytes)) return e;
+    static_assert(T::kSmemBytes <= 48 * 1024, "no attribute needed");
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3((op.N + BN - 1) / BN * split, (op.batch * op.T + BM - 1) / BM);
     cfg.blockDim = dim3(T::NT);
@@ -1022,7 +1027,11 @@ static cudaError_t launch_tile(const RowOp& op, int split, cudaStream_t st) {
     at[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = at;
     cfg.numAttrs = g_pdl ? 2 : 1;
-    return cudaLaunchKernelEx(&cfg, tile_kernel<BM, BN, TM, TN>, op);
+    return cudaLaunchKernelEx(&cfg, tile_kernel<BM, BN, TM, TN, RUN>, op);
+}
+template <int BM, int BN, int TM, int TN>
+static cudaError_t launch_tile(const RowOp& op, int split, cudaStream_t st) {
+    return op.batch >= kTileMinBatch ? launch_tile_run<BM, BN, TM, TN, 0>(op, split, st) : launch_tile_run<BM, BN, TM, TN, kFewStreamRun>(op, split, st);
 }
 static cudaError_t launch_tiles(const RowOp& op, cudaStream_t st) {
     const int rows = op.batch * op.T;

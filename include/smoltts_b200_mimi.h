@@ -106,9 +106,10 @@ int smol_mimi_decode_frames(SmolMimi* m, const int32_t* d_codes, const int32_t* 
                             void* stream);
 
 /* Test / profiling hooks: intermediate buffers by name ("emb": upsampled embeddings, "xf": transformer output; slot-major),
- * kernel launches per step, device-side error word (nonzero: a stream ran past max_positions). */
+ * kernel launches per step, graphs captured so far, device-side error word (nonzero: a stream ran past max_positions). */
 void* smol_mimi_debug_buffer(SmolMimi* m, const char* name, int64_t* slot_stride_floats);
 int32_t smol_mimi_launches_per_step(const SmolMimi* m);
+int64_t smol_mimi_captures(const SmolMimi* m);
 int32_t* smol_mimi_error_word(SmolMimi* m);
 
 #ifdef __cplusplus

@@ -131,6 +131,7 @@ PROTOTYPES = {
     "smol_mimi_decode_frames": (C.c_int, [C.c_void_p, C.c_void_p, C.c_void_p, C.c_int32, C.c_int32, C.c_void_p, C.c_void_p]),
     "smol_mimi_debug_buffer": (C.c_void_p, [C.c_void_p, C.c_char_p, C.POINTER(C.c_int64)]),
     "smol_mimi_launches_per_step": (C.c_int32, [C.c_void_p]),
+    "smol_mimi_captures": (C.c_int64, [C.c_void_p]),
     "smol_mimi_error_word": (C.c_void_p, [C.c_void_p]),
 }
 

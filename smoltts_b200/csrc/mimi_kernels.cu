@@ -787,9 +787,11 @@ struct SmolMimi {
     struct Step { const void* codes; const void* slots; const void* pcm; int batch, frames; std::vector<OpRec> prog; cudaGraphExec_t graph; uint64_t used; };
     std::vector<Step> steps;
     uint64_t tick = 0;
+    int64_t captures = 0;
     void drop_steps() { for (Step& s : steps) if (s.graph) cudaGraphExecDestroy(s.graph); steps.clear(); }
 };
-constexpr size_t kMaxSteps = 16;
+constexpr size_t kMaxSteps = 16;        // of one frame: as many batch sizes
+constexpr size_t kMaxRunSteps = 64;     // of several: a batch of 12 and more streams has up to three, a few streams up to seven
 
 static size_t al(size_t v) { return (v + 255) / 256 * 256; }
 
@@ -892,6 +894,7 @@ extern "C" int smol_mimi_set_max_frames(SmolMimi* m, int32_t frames) {
 extern "C" int32_t smol_mimi_samples_per_frame(const SmolMimi* m) { return m ? m->spf : 0; }
 extern "C" size_t smol_mimi_workspace_bytes(const SmolMimi* m) { return m ? m->total : 0; }
 extern "C" int32_t smol_mimi_launches_per_step(const SmolMimi* m) { return m ? m->launches : 0; }
+extern "C" int64_t smol_mimi_captures(const SmolMimi* m) { return m ? m->captures : 0; }
 extern "C" int32_t* smol_mimi_error_word(SmolMimi* m) { return (m && m->bound) ? reinterpret_cast<int32_t*>(m->ws + m->o_err) : nullptr; }
 
 #define MCU(call) do { cudaError_t e__ = (call); if (e__ != cudaSuccess) return smol::capi_cuda_fail(e__, #call); } while (0)
@@ -1001,12 +1004,12 @@ static cudaError_t launch_pdl(void (*kern)(const Args), dim3 grid, dim3 block, s
 static int rows_R(int rows) { return rows <= 2 ? 2 : rows <= 4 ? 4 : rows <= 8 ? 8 : 16; }
 
 constexpr int kTileMinBatch = 12;   // the class of 12+ streams
-static int rows_per_frame(const RowOp& op) { return op.T / op.frames; }
-// Operations on the packed-FMA tiles: see tile_kernel.  (Fewer than 12 streams: an operation of two rows per frame streams its weights
-// through rows_kernel / lin_kernel, which read them once for up to 16 rows.)
 // Fewer streams: partial sums of 16 k (f32_tile.cuh).  Error of the samples against 64 bits, mean over five sets of weights: 4.2e-7 (4.3e-7 of
 // rows_kernel's 32 chains); without partial sums 5.5e-7, of 64 k 4.6e-7, of 32 k 4.3e-7.  8 steps of one stream take 2.41 to 2.45 ms with any.
 constexpr int kFewStreamRun = 1;
+static int rows_per_frame(const RowOp& op) { return op.T / op.frames; }
+// Operations on the packed-FMA tiles: see tile_kernel.  (Fewer than 12 streams: an operation of two rows per frame streams its weights
+// through rows_kernel / lin_kernel, which read them once for up to 16 rows.)
 static bool use_tile(const RowOp& op) {
     return (op.batch >= kTileMinBatch || rows_per_frame(op) >= 16) && op.N >= 16 && op.N % 4 == 0 && op.bias_mod % (op.bias ? 4 : 1) == 0 && op.K % 4 == 0 && op.in_c % 4 == 0 &&
            (op.tapstep > 0 || op.K == 2 * op.in_c) && (op.pro == PRO_NONE || (op.norm_at && op.K <= 32 * kNormRegs));
@@ -1275,9 +1278,14 @@ extern "C" int smol_mimi_decode_frames(SmolMimi* m, const int32_t* d_codes, cons
     for (SmolMimi::Step& c : m->steps)
         if (c.codes == d_codes && c.slots == d_slots && c.pcm == d_pcm && c.batch == batch && c.frames == frames) { step = &c; break; }
     if (!step) {
-        if (m->steps.size() >= kMaxSteps) {   // evict the least recently used
-            size_t lru = 0;
-            for (size_t i = 1; i < m->steps.size(); ++i) if (m->steps[i].used < m->steps[lru].used) lru = i;
+        // evict the least recently used of its kind: runs of frames push no single step out
+        size_t lru = m->steps.size(), kin = 0;
+        for (size_t i = 0; i < m->steps.size(); ++i) {
+            if ((m->steps[i].frames > 1) != (frames > 1)) continue;
+            ++kin;
+            if (lru == m->steps.size() || m->steps[i].used < m->steps[lru].used) lru = i;
+        }
+        if (kin >= (frames > 1 ? kMaxRunSteps : kMaxSteps)) {
             if (m->steps[lru].graph) cudaGraphExecDestroy(m->steps[lru].graph);
             m->steps.erase(m->steps.begin() + lru);
         }
@@ -1300,6 +1308,7 @@ extern "C" int smol_mimi_decode_frames(SmolMimi* m, const int32_t* d_codes, cons
         const cudaError_t ei = cudaGraphInstantiate(&step->graph, g, 0);
         cudaGraphDestroy(g);
         MCU(ei);
+        ++m->captures;
     }
     MCU(cudaGraphLaunch(step->graph, st));
     return SMOL_OK;

@@ -135,8 +135,9 @@ class MimiModel:
         self._ws: Optional[torch.Tensor] = None
         self._free = list(range(max_streams - 1, -1, -1))
         self._frames = [0] * max_streams
-        self._io: Dict[int, tuple] = {}   # batch -> (codes, slots, pcm) device buffers with stable addresses (graph replay)
-        self._io_slots: Dict[int, tuple] = {}
+        # (batch, whether of several frames) -> (codes, slots, pcm) device buffers with stable addresses (graph replay)
+        self._io: Dict[tuple, tuple] = {}
+        self._io_slots: Dict[tuple, tuple] = {}
 
     def __del__(self):
         try:
@@ -249,12 +250,16 @@ class MimiModel:
             self._frames[s] = 0
 
     def _buffers(self, batch: int, frames: int = 1):
-        key = (batch, frames)
+        """Buffers of a call: its own of one frame, the front of the batch's largest run's of several."""
+        key = (batch, frames > 1)
         if key not in self._io:
-            self._io[key] = (torch.zeros(batch, frames, self.num_codebooks, dtype=torch.int32, device=self.device),
+            most = int(self._lib.smol_mimi_max_frames(self._h, batch)) if frames > 1 else 1
+            self._io[key] = (torch.zeros(batch * most * self.num_codebooks, dtype=torch.int32, device=self.device),
                              torch.zeros(batch, dtype=torch.int32, device=self.device),
-                             torch.zeros(batch, frames * self.samples_per_frame, dtype=torch.float32, device=self.device))
-        return self._io[key]
+                             torch.zeros(batch * most * self.samples_per_frame, dtype=torch.float32, device=self.device))
+        codes, slots, pcm = self._io[key]
+        return (codes[:batch * frames * self.num_codebooks].view(batch, frames, self.num_codebooks), slots,
+                pcm[:batch * frames * self.samples_per_frame].view(batch, frames * self.samples_per_frame))
 
     def _run(self, codes: torch.Tensor, caches: Sequence[MimiCache]) -> torch.Tensor:
         """codes [B, frames, n_q] -> PCM [B, frames * samples_per_frame] (a view of an internal buffer)."""
@@ -265,9 +270,10 @@ class MimiModel:
         d_codes, d_slots, d_pcm = self._buffers(B, frames)
         d_codes.copy_(codes.to(torch.int32), non_blocking=True)
         slots = tuple(c.slot for c in caches)
-        if self._io_slots.get((B, frames)) != slots:      # a batch's slot table changes only when streams come and go
+        key = (B, frames > 1)
+        if self._io_slots.get(key) != slots:      # a batch's slot table changes only when streams come and go
             d_slots.copy_(torch.tensor(slots, dtype=torch.int32), non_blocking=True)
-            self._io_slots[(B, frames)] = slots
+            self._io_slots[key] = slots
         _capi.check(self._lib.smol_mimi_decode_frames(self._h, C.c_void_p(d_codes.data_ptr()), C.c_void_p(d_slots.data_ptr()), B, frames,
                                                       C.c_void_p(d_pcm.data_ptr()), C.c_void_p(self._stream())))
         for c in caches:

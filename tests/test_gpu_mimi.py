@@ -82,6 +82,44 @@ def test_refused_decodes_leave_every_slot_free():
     assert m.decode(torch.zeros(2, 8, 0, dtype=torch.int64)).shape == (2, 1, 0)
 
 
+def test_runs_of_frames_push_no_single_step_out():
+    """A streaming loop over sixteen batch sizes keeps its captured steps beside whole utterances of any length, and a batch has one set of
+    buffers for single steps and one for runs."""
+    m = _model(max_streams=16, max_frames=24)
+    codes = torch.randint(0, 2048, (16, 8, 23), generator=torch.Generator().manual_seed(1))
+
+    def stream():
+        return [_run(m, codes[:b, :, :1]) for b in range(1, 17)]
+
+    first = stream()
+    for b, frames in [(1, 23), (1, 14), (2, 23), (3, 5), (4, 7), (12, 23), (13, 22), (16, 21)]:
+        m.decode(codes[:b, :, :frames])
+    captured = m._lib.smol_mimi_captures(m._h)
+    assert all(torch.equal(a, b) for a, b in zip(first, stream()))
+    assert m._lib.smol_mimi_captures(m._h) == captured
+    assert len(m._io) == 16 + 7
+
+
+def test_few_streams_are_summed_in_short_runs():
+    """Against the oracle in float64 one stream is closer than the same stream among twelve, whose sums run over a thread block's whole share of K:
+    the error of a sum grows with the root of its chain, which is 8 to 64 times shorter; layers that both classes share leave 0.63 of it."""
+    from oracle.mimi_oracle import MimiOracle, StreamState
+
+    m = _model(max_streams=12, max_frames=64)
+    o = MimiOracle(_sd())
+    o.sd = {k: v.double() for k, v in o.sd.items()}
+    few, many = 0.0, 0.0
+    for seed in range(3):
+        codes = torch.randint(0, 2048, (1, 8, 4), generator=torch.Generator().manual_seed(seed))
+        st = StreamState()
+        want = torch.cat([o.decode_step(codes[:, :, t:t + 1], st) for t in range(4)], -1)
+        error = lambda got: float((got.double().cpu() - want).norm() / want.norm())  # noqa: E731
+        few += error(m.decode(codes))
+        many += error(m.decode(codes.expand(12, -1, -1))[:1])
+    print(f"error against 64 bits: one stream {few / 3:.3g}, among twelve {many / 3:.3g}")
+    assert few < 0.63 * many
+
+
 def test_transformer_output_matches_goldens():
     g = np.load(f"{GOLDEN_DIR}/mimi.npz")
     codes = torch.from_numpy(g["codes"]).long()

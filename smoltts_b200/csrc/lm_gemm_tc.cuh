@@ -2,8 +2,14 @@
 //
 // y[M, N] = a[M, K] . w[N, K]^T in tiles of 128 rows x BN columns, one persistent CTA per SM walking them; row tiles that share a weight
 // tile run on neighbouring CTAs.  The roles of a CTA overlap instead of taking turns: two threads keep TMA loads of 64-element K stages
-// going through a ring, one thread issues tcgen05.mma into one of two accumulators in tensor memory, and four warps drain the other
-// accumulator while the next tile is multiplied.
+// going through a ring, a warp issues tcgen05.mma into one of two accumulators in tensor memory, and eight warps drain the other
+// accumulator meanwhile.
+//
+// An accumulator drops what lies below its last place with every MMA, so K is summed in four parts, each in an accumulator begun anew, which
+// the draining warps add in fp32 registers: error against 64 bits 1.8e-7 at K = 768, 1.1e-6 at 4608 (one accumulator over all of K: 7.3e-7 and
+// 5.0e-6; values in [0, 1): 2.4e-7 and 2.2e-6 against 1.3e-6 and 1.5e-5).  It costs no time as the MMAs are issued now: the whole warp walks, one
+// elected lane issues, and the operands stay in uniform registers (2048 x 768 x 4608 27 us, 1801 x 1536 x 6144 36; one accumulator and a
+// single thread walking 29 and 39, four parts and a single thread 47 and 63).
 //
 // What bounds it: a stage brings (128 + BN) x 128 bytes through the SM's 64 bytes per clock from L2 and takes 2 BN clocks of the tensor
 // pipe, so up to BN = 128 the loads take twice as long as the MMAs and at 256 half again; wide tiles win as long as they still fill the
@@ -17,14 +23,16 @@
 namespace smol {
 namespace lm {
 
-constexpr int kTcThreads = 256;          // warps 0 and 2: loads of activations and weights, 1: MMAs, 4 to 7: epilogue
+constexpr int kTcEpilogueWarps = 8;
+constexpr int kTcThreads = 128 + kTcEpilogueWarps * 32;      // warps 0 and 2: loads of activations and weights, 1: MMAs, 4 to 11: epilogue
+constexpr int kTcParts = 4;              // partial sums of a tile: a quarter of K each
 constexpr int kTcMinRows = 257;          // below this the mma.sync tiles fill the GPU better than 128-row tiles
 constexpr int kTcMinCols = 96;
-constexpr int kTcStageLd = 36;           // floats between the staged rows of a 32 x 32 piece: conflict-free for 16-byte accesses
+constexpr int kTcStageLd = 36;           // floats between the staged rows of a 16 x 32 piece: conflict-free for 16-byte accesses
 
 template <int BN> constexpr int gemm_tc_stages() { return BN >= 256 ? 4 : BN >= 192 ? 5 : 6; }
 template <int BN> constexpr int gemm_tc_stage_bytes() { return (umma::kM + BN) * umma::kBK * 2; }
-template <int BN> constexpr int gemm_tc_smem() { return gemm_tc_stages<BN>() * gemm_tc_stage_bytes<BN>() + 4 * 32 * kTcStageLd * 4 + 1024; }
+template <int BN> constexpr int gemm_tc_smem() { return gemm_tc_stages<BN>() * gemm_tc_stage_bytes<BN>() + kTcEpilogueWarps * 16 * kTcStageLd * 4 + 1024; }
 
 struct GemmTcBars {
     uint64_t full[8], empty[8];      // ring stages: bytes landed / consumed by the MMAs
@@ -35,15 +43,25 @@ struct GemmTcBars {
 __device__ __forceinline__ void bar_arrive(uint64_t* bar) {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(umma::s2u(bar)) : "memory");
 }
-__device__ __forceinline__ void tmem_ld32_issue(uint32_t taddr, uint32_t (&r)[32]) {
+__device__ __forceinline__ void tmem_ld16_issue(uint32_t taddr, uint32_t (&r)[16]) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]),
+                   "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+                 : "r"(taddr) : "memory");
+}
+
+// One MMA / one commit by the warp's elected lane, every lane calling: the operands stay in uniform registers.  `more` 0: the accumulator begins anew.
+__device__ __forceinline__ void mma_bf16_one(uint32_t d, uint64_t a, uint64_t b, uint32_t idesc, uint32_t more) {
     asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
-        "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
-        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]),
-          "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]), "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]),
-          "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]),
-          "=r"(r[31])
-        : "r"(taddr) : "memory");
+        "{\n\t.reg .pred p, e;\n\tsetp.ne.u32 p, %4, 0;\n\telect.sync _|e, 0xffffffff;\n\t"
+        "@e tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+        ::"r"(d), "l"(a), "l"(b), "r"(idesc), "r"(more) : "memory");
+}
+__device__ __forceinline__ void commit_one(uint64_t* bar) {
+    asm volatile(
+        "{\n\t.reg .pred e;\n\telect.sync _|e, 0xffffffff;\n\t"
+        "@e tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}"
+        ::"r"(umma::s2u(bar)) : "memory");
 }
 
 // Grouped rows (io.tile_group != nullptr): the row tiles come from the device-built table (128 rows each, group g's rows end
@@ -52,7 +70,7 @@ __device__ __forceinline__ void tmem_ld32_issue(uint32_t taddr, uint32_t (&r)[32
 template <int BN>
 __global__ void __launch_bounds__(kTcThreads, 1) gemm_tc_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CUtensorMap tm_w,
                                                                 float* __restrict__ y, const int M, const int N, const int K, const GemmIo io) {
-    constexpr int ST = gemm_tc_stages<BN>(), SB = gemm_tc_stage_bytes<BN>(), kA = umma::kM * umma::kBK * 2;
+    constexpr int ST = gemm_tc_stages<BN>(), SB = gemm_tc_stage_bytes<BN>(), kA = umma::kM * umma::kBK * 2, kSteps = umma::kBK / 16;
     static_assert(BN % 32 == 0 && BN <= 256 && ST <= 8, "tile width");
     extern __shared__ unsigned char tc_smem[];
     __shared__ GemmTcBars bars;
@@ -60,7 +78,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) gemm_tc_kernel(const __grid_con
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     if (threadIdx.x == 0) {
         for (int s = 0; s < ST; ++s) { umma::bar_init(&bars.full[s], 2); umma::bar_init(&bars.empty[s], 1); }
-        for (int i = 0; i < 2; ++i) { umma::bar_init(&bars.acc_full[i], 1); umma::bar_init(&bars.acc_empty[i], 4); }
+        for (int i = 0; i < 2; ++i) { umma::bar_init(&bars.acc_full[i], 1); umma::bar_init(&bars.acc_empty[i], kTcEpilogueWarps); }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == 1) umma::tmem_alloc(&bars.tmem);
@@ -103,69 +121,106 @@ __global__ void __launch_bounds__(kTcThreads, 1) gemm_tc_kernel(const __grid_con
                 }
             }
         }
-    } else if (warp == 1 && lane == 0) {
-        // ---- MMAs ----
+    } else if (warp == 1) {
+        // ---- MMAs: nk of the tile's 4 nk into one accumulator, the next nk into the other (the whole warp walks, one lane issues) ----
         const uint32_t idesc = umma::instr_desc(BN);
-        uint32_t c = 0, t = 0;
-        for (int u = blockIdx.x; u < tiles; u += gridDim.x, ++t) {
-            const uint32_t b = t & 1u, d = tmem + b * BN;
-            if (t >= 2) umma::bar_wait(&bars.acc_empty[b], (t / 2 - 1u) & 1u);
-            umma::fence_after_sync();
+        uint32_t c = 0, p = 0;      // stages, parts so far
+        for (int u = blockIdx.x; u < tiles; u += gridDim.x) {
+            int n = 0;              // MMAs of the part so far
             for (int kc = 0; kc < nk; ++kc, ++c) {
                 const uint32_t s = c % ST;
                 umma::bar_wait(&bars.full[s], (c / ST) & 1u);
+                if (n == 0 && p >= 2) umma::bar_wait(&bars.acc_empty[p & 1u], (p / 2 - 1u) & 1u);
                 umma::fence_after_sync();
-                const uint32_t at = umma::s2u(ring + (size_t)s * SB);
+                const uint64_t da = umma::smem_desc_sw128(umma::s2u(ring + (size_t)s * SB)), dw = umma::smem_desc_sw128(umma::s2u(ring + (size_t)s * SB) + kA);
+                if (n + kSteps <= nk) {
 #pragma unroll
-                for (int q = 0; q < umma::kBK / 16; ++q)
-                    umma::mma_bf16(d, umma::smem_desc_sw128(at + q * 32), umma::smem_desc_sw128(at + kA + q * 32), idesc, (kc > 0 || q > 0) ? 1u : 0u);
-                umma::commit(&bars.empty[s]);
+                    for (int q = 0; q < kSteps; ++q) mma_bf16_one(tmem + (p & 1u) * BN, da + q * 2, dw + q * 2, idesc, (uint32_t)(n + q));
+                    n += kSteps;
+                } else {
+#pragma unroll 1
+                    for (int q = 0; q < kSteps; ++q) {
+                        if (n == nk) {
+                            commit_one(&bars.acc_full[p++ & 1u]);
+                            n = 0;
+                            if (p >= 2) umma::bar_wait(&bars.acc_empty[p & 1u], (p / 2 - 1u) & 1u);
+                            umma::fence_after_sync();
+                        }
+                        mma_bf16_one(tmem + (p & 1u) * BN, da + q * 2, dw + q * 2, idesc, (uint32_t)n);
+                        ++n;
+                    }
+                }
+                commit_one(&bars.empty[s]);
+                if (n == nk) {                                   // after `empty`: nothing of the block's is in flight once its last part is read
+                    commit_one(&bars.acc_full[p++ & 1u]);
+                    n = 0;
+                }
             }
-            umma::commit(&bars.acc_full[b]);
         }
     } else if (warp >= 4) {
-        // ---- epilogue: warp w drains the accumulator rows 32 (w - 4) .. + 31, 32 columns at a time ----
-        float* stage = reinterpret_cast<float*>(ring + (size_t)ST * SB) + (warp - 4) * 32 * kTcStageLd;
+        // ---- epilogue: rows 32 (w % 4) .. + 31, half of the columns ----
+        constexpr int HC = (BN / 2 + 31) / 32 * 32;      // columns of the first half
+        const int quad = warp & 3, half = (warp - 4) >> 2, cols = half ? BN - HC : HC;
+        float* stage = reinterpret_cast<float*>(ring + (size_t)ST * SB) + (warp - 4) * 16 * kTcStageLd;
         const bool vec = N % 4 == 0 && reinterpret_cast<uintptr_t>(y) % 16 == 0;
-        uint32_t t = 0;
-        for (int u = blockIdx.x; u < tiles; u += gridDim.x, ++t) {
+        uint32_t p = 0;
+        for (int u = blockIdx.x; u < tiles; u += gridDim.x) {
             int m0, m_end, w_row;
             place(u, m0, m_end, w_row);
-            const int n0 = (u / m_tiles) * BN, r0 = m0 + (warp - 4) * 32;
-            const uint32_t b = t & 1u;
-            umma::bar_wait(&bars.acc_full[b], (t / 2) & 1u);
-            umma::fence_after_sync();
-            const uint32_t d = tmem + b * BN + ((uint32_t)((warp - 4) * 32) << 16);
-#pragma unroll 1
-            for (int c0 = 0; c0 < BN && n0 + c0 < N; c0 += 32) {
-                uint32_t v[32];
-                tmem_ld32_issue(d + c0, v);
-                umma::tmem_ld_wait();
-                if (r0 >= m_end) continue;
-                __syncwarp();
+            const int n0 = (u / m_tiles) * BN + half * HC, r0 = m0 + quad * 32, here = min(cols, N - n0);
+            float sum[HC];
 #pragma unroll
-                for (int i = 0; i < 8; ++i) *reinterpret_cast<uint4*>(stage + lane * kTcStageLd + i * 4) = make_uint4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
+            for (int i = 0; i < HC; ++i) sum[i] = 0.0f;
+#pragma unroll 1
+            for (int x = 0; x < kTcParts; ++x, ++p) {
+                const uint32_t b = p & 1u, d = tmem + b * BN + half * HC + ((uint32_t)(quad * 32) << 16);
+                umma::bar_wait(&bars.acc_full[b], (p / 2) & 1u);
                 __syncwarp();
+                umma::fence_after_sync();
+#pragma unroll
+                for (int c0 = 0; c0 < HC; c0 += 16) {
+                    if (c0 >= here) break;
+                    uint32_t v[16];
+                    tmem_ld16_issue(d + c0, v);
+                    umma::tmem_ld_wait();
+#pragma unroll
+                    for (int e = 0; e < 16; ++e) sum[c0 + e] += __uint_as_float(v[e]);
+                }
+                umma::fence_before_sync();
+                __syncwarp();
+                if (lane == 0) bar_arrive(&bars.acc_empty[b]);
+            }
+            if (r0 >= m_end) continue;
+#pragma unroll
+            for (int c0 = 0; c0 < HC; c0 += 32) {
+                if (c0 >= here) break;
                 const int col = n0 + c0 + (lane & 7) * 4;
 #pragma unroll
-                for (int i = 0; i < 8; ++i) {
-                    const int r = i * 4 + (lane >> 3), m = r0 + r;
-                    const float4 o = *reinterpret_cast<const float4*>(stage + r * kTcStageLd + (lane & 7) * 4);
-                    if (m >= m_end) continue;
-                    float* p = y + (size_t)m * N + col;
-                    if (vec) {
-                        if (col < N) *reinterpret_cast<float4*>(p) = o;
-                    } else {
-                        if (col < N) p[0] = o.x;
-                        if (col + 1 < N) p[1] = o.y;
-                        if (col + 2 < N) p[2] = o.z;
-                        if (col + 3 < N) p[3] = o.w;
+                for (int h = 0; h < 2; ++h) {            // 16 rows at a time
+                    __syncwarp();
+                    if (lane >> 4 == h) {
+#pragma unroll
+                        for (int i = 0; i < 8; ++i)
+                            *reinterpret_cast<float4*>(stage + (lane & 15) * kTcStageLd + i * 4) = make_float4(sum[c0 + 4 * i], sum[c0 + 4 * i + 1], sum[c0 + 4 * i + 2], sum[c0 + 4 * i + 3]);
+                    }
+                    __syncwarp();
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) {
+                        const int r = i * 4 + (lane >> 3), m = r0 + h * 16 + r;
+                        const float4 o = *reinterpret_cast<const float4*>(stage + r * kTcStageLd + (lane & 7) * 4);
+                        if (m >= m_end) continue;
+                        float* to = y + (size_t)m * N + col;
+                        if (vec) {
+                            if (col < N) *reinterpret_cast<float4*>(to) = o;
+                        } else {
+                            if (col < N) to[0] = o.x;
+                            if (col + 1 < N) to[1] = o.y;
+                            if (col + 2 < N) to[2] = o.z;
+                            if (col + 3 < N) to[3] = o.w;
+                        }
                     }
                 }
             }
-            umma::fence_before_sync();
-            __syncwarp();
-            if (lane == 0) bar_arrive(&bars.acc_empty[b]);
         }
     }
     __syncwarp();

@@ -42,6 +42,19 @@ def test_products_of_many_rows(M, N, K):
     assert bool((err <= product_bound(a, w)).all())
 
 
+@pytest.mark.parametrize("M,N,K", [(3, 768, 4608), (5, 2400, 4096), (20, 768, 4608), (300, 768, 768), (300, 768, 4608), (1024, 4608, 1024), (600, 2049, 1000)])
+def test_products_of_positive_values_lose_no_more_than_their_chains(M, N, K):
+    """An MMA drops up to the last place (2^-23) of the sum it adds to, always downwards where all products are positive.  Few rows: every MMA
+    starts from zero, so 2^-23 of the result.  Many rows: four chains of K / 64 MMAs whose sum grows evenly, so half of K / 64 places, and one for
+    the four parts."""
+    model, _, _ = engine_and_oracle(config([attn(ff=0)]), seed=9, dtype=torch.bfloat16)
+    g = torch.Generator(device="cuda").manual_seed(M * 31 + K)
+    a, w = (torch.rand(r, K, device="cuda", generator=g).bfloat16() for r in (M, N))
+    want = a.double() @ w.double().T
+    places = 1.0 if M <= 32 else 0.5 * -(-K // 64) + 1.0
+    assert float(((model.linear(a, w).double() - want) / want).pow(2).mean().sqrt()) < places * 2.0 ** -23
+
+
 @pytest.mark.parametrize("dtype,M", [(torch.bfloat16, 3), (torch.bfloat16, 40), (torch.bfloat16, 300), (torch.float32, 3), (torch.float32, 300)])
 def test_a_product_waits_for_the_kernel_that_makes_its_weights(dtype, M):
     """linear()'s weights may come from the kernel just in front, and the products read weights before they wait for that kernel: every

@@ -2651,8 +2651,11 @@ static cudaError_t launch_scan(const DeltaArgs& A, int n_seqs, const float* dec,
     return cudaGetLastError();
 }
 
-// The four-token scan over a step in which some sequence brings at least kQuadMinTokens tokens (fewer: its two launches cost more than
-// the chain they shorten).
+// The four-token scan over a step in which some sequence brings at least kQuadMinTokens tokens, kQuadMeanTokens in the mean (fewer: its two
+// launches and the records of single tokens cost more than the chain they shorten).  One layer of 12 x 64 x 64 as a whole, generalized delta rule,
+// 16 / 24 / 40 / 300 / 1200 tokens: 61 / 68 / 166 / 142 / 275 us against 56 / 65 / 165 / 166 / 370; the two scans alone, 17 tokens
+// beside 15 / 63 single ones: 28 / 67 us against 11 / 20.
+static bool quad_pays(int n_seqs, int n_tokens, int max_n) { return max_n >= kQuadMinTokens && n_tokens >= kQuadMeanTokens * n_seqs; }
 template <int KIND, int DK>
 static cudaError_t launch_quad_sized(SmolLm* m, QuadSource Q, QuadArgs A, int n_seqs, int max_n, float* o_raw, cudaStream_t st, size_t min_smem) {
     constexpr int FORM = quad_form(KIND);
@@ -2685,9 +2688,9 @@ static cudaError_t launch_gla_scan(const GlaArgs& A, int n_seqs, const float* de
     return cudaGetLastError();
 }
 // the scan over key sizes up to 256: the smallest built size that holds A.d
-static cudaError_t launch_gla_scan_any(SmolLm* m, const GlaArgs& A, int n_seqs, int max_n, const float* dec, float* pool, float* o_raw, cudaStream_t st,
+static cudaError_t launch_gla_scan_any(SmolLm* m, const GlaArgs& A, int n_seqs, int n_tokens, int max_n, const float* dec, float* pool, float* o_raw, cudaStream_t st,
                                         size_t min_smem = 0) {
-    if (max_n >= kQuadMinTokens) {
+    if (quad_pays(n_seqs, n_tokens, max_n)) {
         QuadSource Q{A.H, A.qk_share, A.d, A.q_src, A.k_src, A.q_ld, A.k_ld, dec, A.head_decay, A.head_step, A.head_ld, 1, nullptr, nullptr, 0.0f, A.seq_start, 0};
         QuadArgs S{A.H, A.d, A.dv, nullptr, 0, A.v_src, A.v_ld, A.q_scale, A.seq_start, A.seq_pos0, A.seq_slot, A.slot_floats, A.state_off, A.n_slots, A.err};
         if (A.head_decay) return launch_quad<kQuadHeadDecay>(m, Q, S, n_seqs, max_n, o_raw, st, min_smem);
@@ -3013,7 +3016,7 @@ static int step_impl(SmolLm* m, const SmolLmStep* s, cudaStream_t st) {
             A.qk_share = M.heads / M.bc_groups;
             A.head_decay = head; A.head_step = head + (size_t)Tn * M.heads; A.head_ld = M.heads;
             A.out_ld = out_ld_now; A.out_scale = 1.0f;
-            CU(launch_gla_scan_any(m, A, s->n_seqs, max_n, nullptr, m->slots, oraw, ms));
+            CU(launch_gla_scan_any(m, A, s->n_seqs, Tn, max_n, nullptr, m->slots, oraw, ms));
             pdl_launch(ssd_out_kernel<T>, dim3(Tn, M.norm_parts), 256, 0, ms, P, oraw, conv, mix_at, m->slots);
             m->launches += 3;
             return SMOL_OK;
@@ -3094,7 +3097,7 @@ static int step_impl(SmolLm* m, const SmolLmStep* s, cudaStream_t st) {
             A.q_src = conv; A.k_src = conv + hd; A.v_src = conv + 2 * hd;
             A.q_ld = A.k_ld = A.v_ld = na;
             A.head_decay = head; A.head_step = head + (size_t)Tn * M.heads;
-            CU(launch_gla_scan_any(m, A, s->n_seqs, max_n, nullptr, m->slots, oraw, ms));
+            CU(launch_gla_scan_any(m, A, s->n_seqs, Tn, max_n, nullptr, m->slots, oraw, ms));
             LinOutArgs O{pj, n_in, hv, hv, hv, 1, ld, (size_t)2 * hd + hv, c.norm_eps, 1.0f, M.out_norm};
             pdl_launch(lin_attn_out_kernel<T>, dim3(Tn, 1), 256, 0, ms, O, oraw, mix_at);
             m->launches += 3;
@@ -3109,7 +3112,7 @@ static int step_impl(SmolLm* m, const SmolLmStep* s, cudaStream_t st) {
             A.q_src = conv; A.k_src = conv + hd; A.v_src = pj + 2 * hd;
             A.q_ld = A.k_ld = 2 * hd; A.v_ld = n_in;
             A.head_decay = M.head_decay; A.head_ld = 0;
-            CU(launch_gla_scan_any(m, A, s->n_seqs, max_n, nullptr, m->slots, oraw, ms, parallel && Tn > kGraphMaxTokens ? kScanSpread : 0));
+            CU(launch_gla_scan_any(m, A, s->n_seqs, Tn, max_n, nullptr, m->slots, oraw, ms, parallel && Tn > kGraphMaxTokens ? kScanSpread : 0));
             A.out_ld = ld; A.out_scale = M.mix_scale;
             pdl_launch(gla_out_kernel<T>, (Tn * M.heads + 3) / 4, 128, 0, ms, A, oraw, mix_at);
             m->launches += 3;
@@ -3351,7 +3354,7 @@ static int step_impl(SmolLm* m, const SmolLmStep* s, cudaStream_t st) {
             GlaArgs A = scan_args(L, R, proj);
             A.q_src = uk; A.k_src = auk; A.v_src = proj + 2 * hd;
             A.q_ld = A.k_ld = hd; A.v_ld = n_in;
-            CU(launch_gla_scan_any(m, A, s->n_seqs, max_n, dec, m->slots, oraw, st));
+            CU(launch_gla_scan_any(m, A, s->n_seqs, Tn, max_n, dec, m->slots, oraw, st));
             LinOutArgs O{proj, n_in, hv, L.vdim, L.vdim, 0, hv, 0, c.norm_eps, 1.0f, L.out_norm};
             pdl_launch(lin_attn_out_kernel<T>, dim3(Tn, L.heads), 128, 0, st, O, oraw, mix);
             m->launches += 3;
@@ -3417,7 +3420,7 @@ static int step_impl(SmolLm* m, const SmolLmStep* s, cudaStream_t st) {
             if (Tn >= kDecayMinTokens && kDecayTokens * L.rank * sizeof(float) <= 48 * 1024)
                 pdl_launch(gla_prep_kernel<kDecayTokens>, dim3((Tn + kDecayTokens - 1) / kDecayTokens, slices), 128, kDecayTokens * L.rank * sizeof(float), st, A, dec);
             else pdl_launch(gla_prep_kernel<1>, dim3(Tn, slices), 128, L.rank * sizeof(float), st, A, dec);
-            CU(launch_gla_scan_any(m, A, s->n_seqs, max_n, dec, m->slots, oraw, st));
+            CU(launch_gla_scan_any(m, A, s->n_seqs, Tn, max_n, dec, m->slots, oraw, st));
             pdl_launch(gla_out_kernel<T>, (Tn * L.heads + 3) / 4, 128, 0, st, A, oraw, mix);
             m->launches += 3;
             mix_cols = L.heads * L.vdim;
@@ -3428,7 +3431,7 @@ static int step_impl(SmolLm* m, const SmolLmStep* s, cudaStream_t st) {
             A.rate_bias = L.rate_bias; A.decay_w2 = L.decay_w2; A.decay_bias = L.decay_bias; A.out_norm = L.out_norm;
             A.seq_start = s->seq_start; A.seq_pos0 = s->seq_pos0; A.seq_slot = s->seq_slot;
             A.slot_floats = m->slot_floats; A.state_off = R.state_off; A.n_slots = m->n_slots; A.err = err;
-            const bool quad = max_n >= kQuadMinTokens;
+            const bool quad = quad_pays(s->n_seqs, Tn, max_n);
             float *u_to = quad ? nullptr : uk, *au_to = quad ? nullptr : auk;
             const size_t prep_smem = (size_t)(L.rank + L.heads) * sizeof(float);
             const int slices = (L.heads * L.dim + 127) / 128;

@@ -26,7 +26,8 @@ namespace smol {
 namespace lm {
 
 constexpr int kQuad = 4;                 // tokens of a group
-constexpr int kQuadMinTokens = 16;       // fewer tokens in every sequence: the scans without a record
+constexpr int kQuadMinTokens = 32;       // fewer tokens in every sequence: the scans without a record
+constexpr int kQuadMeanTokens = 16;      // fewer tokens per sequence in the mean: likewise
 constexpr int kQuadLanes = 8, kQuadCols = 8, kQuadThreads = kQuadLanes * kQuadCols + 32;
 constexpr int kQuadRing = 4;             // copies of the ring
 __host__ __device__ constexpr int quad_chunk(int DK) { return DK <= 64 ? 4 : DK <= 128 ? 2 : 1; }      // groups per copy

@@ -114,7 +114,7 @@ def test_decay_preparation_over_groups_of_tokens(n):
 @pytest.mark.parametrize("dim", [5, 32, 33, 64, 96, 200])
 def test_four_token_scan_of_prompts(dim):
     """Every form of the recurrence, padded key channels, groups and chunks that end anywhere: sequences of 16 to 67 tokens beside a
-    single token, continued by a second portion, against the oracles."""
+    single token, continued by a second portion of 34 each, against the oracles."""
     import maferax_util as mu
     import virusun_util as vu
 
@@ -125,18 +125,18 @@ def test_four_token_scan_of_prompts(dim):
              (vu.config([vu.par(b=vu.right(heads=2, dim=dim, vdim=8))], vocab=61, width=48), vu.engine_and_oracle)]
     for cfg, make in cases:
         model, orc, _ = make(cfg, seed=4, max_tokens=2048, max_seqs=4, page_size=16, max_step_tokens=256)
-        toks = [tokens(n + 18, 61, n) for n in lens]
+        toks = [tokens(n + 34, 61, n) for n in lens]
         want = [orc.forward(t) for t in toks]
         seqs = [model.open_sequence() for _ in lens]
         first = model.forward([(s, t[:n], list(range(n))) for s, t, n in zip(seqs, toks, lens)]).clone()
-        then = model.forward([(s, t[n:], list(range(18))) for s, t, n in zip(seqs, toks, lens)]).clone()
+        then = model.forward([(s, t[n:], list(range(34))) for s, t, n in zip(seqs, toks, lens)]).clone()
         for s in seqs:
             model.close_sequence(s)
         at = 0
         for i, n in enumerate(lens):
             if n > 1:
                 assert rel_err(first[at:at + n], want[i][:n]) < TOL[torch.float32]
-            assert rel_err(then[18 * i:18 * i + 18], want[i][n:]) < TOL[torch.float32]
+            assert rel_err(then[34 * i:34 * i + 34], want[i][n:]) < TOL[torch.float32]
             at += n
 
 
@@ -153,7 +153,7 @@ def test_tokens_take_nothing_from_later_ones_in_the_four_token_scan():
 
     for cfg, make in cases:
         model, _, _ = make(cfg, seed=5, edit=spoil, max_step_tokens=256)
-        toks = [t % bad for t in tokens(27, 61, 1)]
+        toks = [t % bad for t in tokens(43, 61, 1)]
 
         def logits(row):
             seq = model.open_sequence()
@@ -162,7 +162,7 @@ def test_tokens_take_nothing_from_later_ones_in_the_four_token_scan():
             return out
 
         want = logits(toks)
-        for at in range(19, 26):
+        for at in range(35, 42):
             got = logits(toks[:at] + [bad] + toks[at + 1:])
             assert torch.equal(got[:at], want[:at])
             assert not bool(got[at:].isfinite().any())

@@ -110,7 +110,6 @@ __global__ void __launch_bounds__(ft_threads(DV, MAPS), 1) attn_flash_tc_kernel(
     unsigned char *Qs = base, *KV = Qs + MAPS * kFtRows * DK * 2, *Ps = KV + NB * SB;          // Ps: heads, then remainders
     float* first_map = reinterpret_cast<float*>(Ps + 2 * kFtPBytes);                           // MAPS 2: [OC][threads of the softmax]
     dep_wait();
-    dep_go();
     const int s = blockIdx.y, t0 = A.seq_start[s], n = A.seq_start[s + 1] - t0;
     const int tile = gridDim.z - 1 - blockIdx.z;                                               // the tiles with the most keys start first
     if (n <= kShortSeq || tile * kFtRows >= n) return;
@@ -138,6 +137,7 @@ __global__ void __launch_bounds__(ft_threads(DV, MAPS), 1) attn_flash_tc_kernel(
     umma::fence_async_smem();
     umma::fence_before_sync();
     __syncthreads();
+    dep_go();      // behind the allocation: a kernel set up early that wants tensor memory too must not get it first
     umma::fence_after_sync();
     const uint32_t tmem = bars.tmem, tm_o = tmem + 2 * kFtKeys;                                 // scores at columns 0 and 64, products from 128 on
     if (warp > kFtSoftWarps) {

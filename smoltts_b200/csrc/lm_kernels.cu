@@ -2555,7 +2555,7 @@ cudaError_t linear_ex<bf16>(SmolLm* m, const bf16* a, const bf16* w, float* y, i
     } else if (M <= 32) {
         dim3 grid((N + 31) / 32, (M + 31) / 32, batch);
         pdl_launch(gemm_bf16_kernel<1, 4, 2, 1>, grid, 128, 0, st, a, w, y, M, N, K, io, vec);       // 32 x 32
-    } else if (M <= 256 || ((N + 63) / 64) * ((M + 127) / 128) * batch < 2 * 148) {      // 128-row tiles only when they still fill the GPU twice
+    } else if (M <= 256 || ((N + 63) / 64) * ((M + 127) / 128) * batch < 2 * m->n_sms) {      // 128-row tiles only when they still fill the GPU twice
         dim3 grid((N + 63) / 64, (M + 63) / 64, batch);
         pdl_launch(gemm_bf16_kernel<2, 2, 2, 4>, grid, 128, 0, st, a, w, y, M, N, K, io, vec);       // 64 x 64
     } else {
@@ -2727,15 +2727,23 @@ static cudaError_t launch_group_scan_any(SmolLm* m, const GroupScanArgs& A, floa
 }
 
 // attn_flash_tc_kernel where every row it copies is made of whole 16-byte pieces.  False: not launched (unaligned rows, sizes it is not built
-// for).  Against attn_flash_kernel it is the faster one from 16 tokens on (16 tokens, 12 heads of 64, after 0 / 1500 others: 11 / 46 us, 16 / 113).
-// Two maps it takes one after the other, attn_flash_kernel side by side: there it is left out as long as the 64-row blocks of that kernel have
-// an SM each (512 tokens, 6 heads: 63 us against 56, measured when 3 x 1000 tokens took 97; those take 72 now against 116).
+// for, or attn_flash_kernel is the faster one).  A block takes an SM to itself, pads to 128 rows and spends 10 us or so before and after its keys,
+// so it loses where there are more blocks than SMs and little to do in each: 12 heads of 64, 16 x 12 tokens 22 us against 17, 32 x 64 31
+// against 21, 64 x 20 behind 100 others 70 against 47; but 16 x 16 behind 512 43 against 56, 8 x 300 33 against 42, one sequence of 9 11
+// against 16.  A narrow latent (40 + 8), whose rows are keys and values in one: 16 x 16 behind 512 37 against 29.  Wider rows (128): 16 x 12
+// 31 against 30, 32 x 64 56 against 65.  Heads of 16, one sequence of 9: 11 against 8.  Two maps: faster everywhere (12 heads of 64 / 128, 9 / 100 / 512 / 1536
+// tokens 18 / 31 / 51 / 96 us against 27 / 33 / 55 / 144).  `keys`: positions in whole groups of ranges, as the captured steps know them.
 template <int MAPS>
-static bool launch_flash_tc(const AttnArgs& A, int n_seqs, int max_n, const bf16* qbuf, const bf16* pool, bf16* out, cudaStream_t st) {
+static bool launch_flash_tc(const AttnArgs& A, int n_seqs, int max_n, int keys, int n_sms, const bf16* qbuf, const bf16* pool, bf16* out, cudaStream_t st) {
+    constexpr int kFewKeys = 256;
     const size_t rows = A.d | A.dv | A.out_ld | A.page_elems | A.k_off | A.k_ld | (A.v_in_k ? 0 : A.v_off | A.v_ld);
     if (rows % 8 != 0 || (reinterpret_cast<uintptr_t>(qbuf) | reinterpret_cast<uintptr_t>(pool) | reinterpret_cast<uintptr_t>(out)) % 16 != 0) return false;
     if (A.dv > 128 || A.d > (MAPS == 2 ? 64 : A.v_in_k ? 192 : 128)) return false;
-    if (MAPS == 2 && (long long)A.H * n_seqs * ((max_n + 63) / 64) <= 148) return false;
+    if (MAPS == 1) {
+        const bool narrow = A.d <= 64 && A.dv <= 64, crowded = (long long)A.H * n_seqs > n_sms;
+        if (crowded && max_n <= (narrow ? 64 : 16) && (keys <= kFewKeys || (narrow && A.v_in_k))) return false;
+        if (!A.v_in_k && A.d <= 32 && A.dv <= 32 && max_n <= 16 && keys <= kFewKeys) return false;
+    }
     const dim3 grid(A.H, n_seqs, (max_n + kFtRows - 1) / kFtRows);
 #define SMOL_FLASH_TC(DK, DV, VK) plain_launch(attn_flash_tc_kernel<DK, DV, VK, MAPS>, grid, ft_threads(DV, MAPS), ft_smem(DK, DV, VK, MAPS), st, A, qbuf, pool, out)
     if constexpr (MAPS == 1) {
@@ -2773,13 +2781,14 @@ static void launch_attention(SmolLm* m, const SmolLmStep* s, AttnArgs& A, bool f
     if (A.window > 0) A.n_splits = std::min(A.n_splits, ((A.window - 1) / m->split_len + 2 + 3) / 4 * 4);      // ranges a window can touch
     if (max_n > kShortSeq) {
         if (flash) {
+    const int keys = A.n_splits * m->split_len;
             dim3 grid(A.H, s->n_seqs, (max_n + 63) / 64);
             const int hp = std::max(A.d, A.dv);
             const bf16* qb = reinterpret_cast<const bf16*>(qbuf);
             const bf16* pl = reinterpret_cast<const bf16*>(pool);
             bf16* mx = reinterpret_cast<bf16*>(mix);
 #define SMOL_FLASH(DK, DV, VK) plain_launch(attn_flash_kernel<DK, DV, VK, MAPS>, grid, 128 * MAPS, flash_smem_bytes(DK, DV, VK, MAPS), st, A, qb, pl, mx)
-            bool done = launch_flash_tc<MAPS>(A, s->n_seqs, max_n, qb, pl, mx, st);
+            bool done = launch_flash_tc<MAPS>(A, s->n_seqs, max_n, keys, m->n_sms, qb, pl, mx, st);
             if constexpr (MAPS == 1) {
                 if (done || !A.v_in_k) {
                 } else if (A.d <= 64) SMOL_FLASH(64, 64, true);

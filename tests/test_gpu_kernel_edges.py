@@ -188,25 +188,29 @@ ATTENTION_FORMS = {"sink-64-64": ("pamasun", lambda u: u.attn(heads=4, kv_heads=
                    "sink-40-72": ("pamasun", lambda u: u.attn(heads=2, kv_heads=1, dim=40, vdim=72, ff=0)),
                    "sink-104-8": ("pamasun", lambda u: u.attn(heads=3, kv_heads=3, dim=104, vdim=8, ff=0)),
                    "latent-48": ("maferax", lambda u: u.latent(heads=3, dim=16, rot_dim=8, vdim=16, q_rank=24, kv_rank=40)),
+                   "latent-96": ("maferax", lambda u: u.latent(heads=3, dim=16, rot_dim=16, vdim=16, q_rank=24, kv_rank=80)),
                    "latent-160": ("maferax", lambda u: u.latent(heads=2, dim=32, rot_dim=32, vdim=32, q_rank=24, kv_rank=128)),
                    "maps-64-128": ("virusun", lambda u: u.att(heads=2, kv_heads=1, dim=64, vdim=128)),
                    "maps-24-40": ("virusun", lambda u: u.att(heads=4, kv_heads=2, dim=24, vdim=40)),
+                   "many-maps-64-128": ("virusun", lambda u: u.att(heads=10, kv_heads=2, dim=64, vdim=128)),
+                   "many-maps-24-40": ("virusun", lambda u: u.att(heads=10, kv_heads=5, dim=24, vdim=40)),
                    "rotated-32-16": ("virusun", lambda u: u.par(u.left(heads=4, kv_heads=2, dim=32, vdim=16))),
                    "window-48-16": ("sunutar", lambda u: u.layer(u.left(dim=48, vdim=16, window=100))),
                    "capped-24-24": ("bizulix", lambda u: u.att(dim=24, vdim=24))}
 
 
+@pytest.mark.parametrize("page_size", [16, 64])
 @pytest.mark.parametrize("form", ATTENTION_FORMS)
-def test_prompt_attention_of_128_row_tiles(form):
+def test_prompt_attention_of_128_row_tiles(form, page_size):
     """bf16 prompts that end at and around the tiles' 128 rows and the steps' 64 keys, beside a sequence of three tokens, continued by a
-    second portion: as close to the oracle as the same prompts in portions of at most 64 tokens, which the other kernel takes.  The two
+    second portion: as close to the oracle as the same prompts in portions of at most 8 tokens, which the few-token kernel takes.  The two
     differ in the order of fp32 sums, so at most by one bf16 rounding (2^-8) of what each writes."""
     import importlib
 
     name, layer = ATTENTION_FORMS[form]
     u = importlib.import_module(f"{name}_util")
     cfg = u.config([layer(u)], vocab=61, width=48)
-    model, orc, _ = u.engine_and_oracle(cfg, seed=6, dtype=torch.bfloat16, max_tokens=2048, max_seqs=5, page_size=16, max_step_tokens=640)
+    model, orc, _ = u.engine_and_oracle(cfg, seed=6, dtype=torch.bfloat16, max_tokens=2048, max_seqs=5, page_size=page_size, max_step_tokens=640)
     lens, more = (193, 128, 129, 65, 3), 66
     toks = [tokens(n + more, 61, n) for n in lens]
     want = [orc.forward(t) for t in toks]
@@ -224,8 +228,34 @@ def test_prompt_attention_of_128_row_tiles(form):
         return [torch.cat(o) for o in out]
 
     whole = rows([[(0, n) for n in lens], [(n, n + more) for n in lens]])
-    pieces = rows([[(min(a, n + more), min(a + 64, n + more)) for n in lens] for a in range(0, max(lens) + more, 64)])
+    pieces = rows([[(min(a, n + more), min(a + 8, n + more)) for n in lens] for a in range(0, max(lens) + more, 8)])
     for w, p, o in zip(whole, pieces, want):
         assert rel_err(w, o) < TOL[torch.bfloat16]
         assert rel_err(w, o) < 1.5 * rel_err(p, o) + 2.0 ** -8
     model.check_device_errors()
+
+
+@pytest.mark.parametrize("form", ["narrow", "wide", "latent"])
+def test_many_short_prompts_beside_each_other(form):
+    """More (sequence, head) pairs than SMs with a few tokens each are taken by the 64-row kernel, each of them alone by the 128-row one: both as
+    close to the oracle as one bf16 rounding (2^-8) of what they write."""
+    import maferax_util as mu
+
+    cfg, u = {"narrow": (config([attn(heads=12, kv_heads=4, dim=64, vdim=64, ff=0)], vocab=61, width=48), None),
+              "wide": (config([attn(heads=12, kv_heads=4, dim=72, vdim=128, ff=0)], vocab=61, width=48), None),
+              "latent": (mu.config([mu.latent(heads=12, dim=16, rot_dim=8, vdim=16, q_rank=24, kv_rank=40)], vocab=61, width=48), mu)}[form]
+    lens = [9 + i % 8 for i in range(14)]
+    model, orc, _ = (u.engine_and_oracle if u else engine_and_oracle)(cfg, seed=8, dtype=torch.bfloat16, max_tokens=2048, max_seqs=16, page_size=64, max_step_tokens=256)
+    toks = [tokens(n, 61, n + i) for i, n in enumerate(lens)]
+
+    def run(group):
+        seqs = [model.open_sequence() for _ in group]
+        got = model.forward([(s, t, list(range(len(t)))) for s, t in zip(seqs, group)]).clone()
+        for s in seqs:
+            model.close_sequence(s)
+        return got.split([len(t) for t in group])
+
+    for t, together, alone in zip(toks, run(toks), [run([t])[0] for t in toks]):
+        want = orc.forward(t)
+        assert rel_err(together, want) < TOL[torch.bfloat16]
+        assert rel_err(together, want) < 1.5 * rel_err(alone, want) + 2.0 ** -8

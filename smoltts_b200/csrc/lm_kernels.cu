@@ -2444,7 +2444,7 @@ extern "C" int smol_lm_bind(SmolLm* m, const SmolLmGlobals* g, void* d_workspace
 
 // The kernels of a step are launched with programmatic stream serialization and begin with dep_wait(): a kernel's blocks are set up while
 // the kernel before it drains, instead of after.  What bounds a decoding step is its chain of some hundred dependent kernels of two to ten
-// microseconds: 10 layers of width 768, one token against 2048 cached ones, 4 steps 1780 us -> 1560; 5 sequences of 700 through 4 layers of
+// microseconds: 10 layers of width 768, one token against 2048 cached ones, 4 steps 1780 us -> 1615; 5 sequences of 700 through 4 layers of
 // width 1536, 1024 -> 940.  A launch right after a wait for another stream's event goes out plainly.
 static thread_local bool t_plain_next = false;
 static cudaError_t wait_event(cudaStream_t st, cudaEvent_t e) {
@@ -2470,7 +2470,7 @@ static cudaError_t pdl_launch(void (*kernel)(P...), dim3 grid, dim3 block, size_
 // Kernels whose few long blocks need the SMs to themselves: set up early, they crowd onto those SMs that the kernel before leaves first,
 // two or three to one, and the rest stay idle.  Scans, attention and fp32 products of prompts are launched this way; with all of them early,
 // 2048 tokens through two layers of width 768 took 786 us instead of 665 (706 with every launch plain), 300 in fp32 917 instead of 830.
-// The tcgen05 products keep the SM to themselves by their shared memory and gain by the early start (1164 us instead of 1138).
+// The tcgen05 products keep the SM to themselves by their shared memory and gain by the early start (1138 us instead of 1164).
 template <class... P, class... X>
 static cudaError_t plain_launch(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, X&&... args) {
     t_plain_next = true;
@@ -2778,10 +2778,10 @@ static void launch_attention(SmolLm* m, const SmolLmStep* s, AttnArgs& A, bool f
     const int max_n = s->max_seq_tokens > 0 ? s->max_seq_tokens : Tn;
     const int max_pos = s->max_pos > 0 ? std::min(s->max_pos, c.max_context - 1) : c.max_context - 1;
     A.n_splits = std::min(m->max_splits, (max_pos / m->split_len + 4) / 4 * 4);
+    const int keys = A.n_splits * m->split_len;
     if (A.window > 0) A.n_splits = std::min(A.n_splits, ((A.window - 1) / m->split_len + 2 + 3) / 4 * 4);      // ranges a window can touch
     if (max_n > kShortSeq) {
         if (flash) {
-    const int keys = A.n_splits * m->split_len;
             dim3 grid(A.H, s->n_seqs, (max_n + 63) / 64);
             const int hp = std::max(A.d, A.dv);
             const bf16* qb = reinterpret_cast<const bf16*>(qbuf);

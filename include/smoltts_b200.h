@@ -134,6 +134,10 @@ int smol_kv_bind(SmolModel* m, void* d_kv_pool, int32_t n_pages);
  * d_prompt [B, R, s_max] int32, d_prompt_len [B]. */
 int smol_prefill(SmolModel* m, const SmolBatch* b, int32_t batch, const int32_t* d_prompt,
                  const int32_t* d_prompt_len, int32_t s_max, void* stream);
+/* The prompt of ONE sequence and the logits of its last position (batch slot 0): d_prompt [R, n] ids; all n columns are
+ * cached (n positions on top of what the sequence holds), the last one also stays in SmolBatch.tokens.  Writes
+ * "token_logits" row 0 and "x" row 0.  n must reach option "tc_min_batch" (SMOL_ERR_UNSUPPORTED otherwise). */
+int smol_prompt_logits(SmolModel* m, const SmolBatch* b, const int32_t* d_prompt, int32_t n, void* stream);
 
 /* forward_generate with S == 1 (M:173-192): embed(tokens) -> slow layers (KV append at
  * seq_len) -> norm -> LM head.  Writes fp32 token logits [B, V] (bf16-rounded values) and
@@ -193,9 +197,9 @@ int smol_set_frame_clock(SmolModel* m, uint64_t* d_frame_ns, int32_t capacity);
  * captured in a CUDA graph;  "n_ctas" = grid size (default: one CTA per SM);  "ll_flags" = A/B switches of the
  * data-flow kernel used by tools/ll_ncu.py (0 = the shipped configuration);
  * "tc_min_batch" (default 9: the measured crossover) = rows (sequences of a decode call, sequences x prompt positions of a prefill iteration)
- * from which the tcgen05 variant runs, 0 = never;  "prefill_tile" = cap on the prompt positions per prefill iteration
- * (0 = as many as fit: 128 rows on the tensor-core variant, 8 on the CUDA-core variants).
- * smol_get_option also answers "n_sms", "smem_bytes", "ll_ready", "tc_ready" (1 once the tcgen05 variant has been set up). */
+ * from which the tensor-core variant runs, 0 = never;  "prefill_tile" = cap on the prompt positions per prefill iteration
+ * (0 = as many as fit: 1024 rows on the tensor-core variant, 8 on the CUDA-core variants).
+ * smol_get_option also answers "n_sms", "smem_bytes", "ll_ready", "tc_ready" (1 once the tensor-core variant has been set up). */
 int smol_set_option(SmolModel* m, const char* name, int64_t value);
 int64_t smol_get_option(const SmolModel* m, const char* name);
 

@@ -98,6 +98,7 @@ PROTOTYPES = {
     "smol_bind_workspace": (C.c_int, [C.c_void_p, C.c_void_p, C.c_size_t]),
     "smol_kv_page_bytes": (C.c_size_t, [C.c_void_p]),
     "smol_kv_bind": (C.c_int, [C.c_void_p, C.c_void_p, C.c_int32]),
+    "smol_prompt_logits": (C.c_int, [C.c_void_p, C.POINTER(SmolBatch), C.c_void_p, C.c_int32, C.c_void_p]),
     "smol_prefill": (C.c_int, [C.c_void_p, C.POINTER(SmolBatch), C.c_int32, C.c_void_p, C.c_void_p, C.c_int32, C.c_void_p]),
     "smol_slow_step": (C.c_int, [C.c_void_p, C.POINTER(SmolBatch), C.c_int32, C.c_int32, C.c_void_p]),
     "smol_fast_step": (C.c_int, [C.c_void_p, C.POINTER(SmolBatch), C.c_int32, C.c_int32, C.c_int32, C.c_void_p]),

@@ -16,7 +16,10 @@
 
 namespace smol {
 size_t decode_xs_bytes(const DevModel& M, int bt);
-size_t decode_stage_bytes(const DevModel& M, int n_ctas);
+size_t decode_stage_bytes(const DevModel& M, int n_ctas, int bt);
+void rows_plan(const DevModel& M, int rows, int n_ctas, RowsPlan (*plan)[6]);
+cudaError_t prompt_configure(int* per_sm);
+cudaError_t prompt_launch(const DevModel& M, const CallArgs& A, int n_ctas, cudaStream_t stream);
 int decode_batch_tile(int batch);
 cudaError_t decode_configure(int bt, size_t smem);
 cudaError_t decode_max_ctas(int bt, size_t smem, int* per_sm);
@@ -33,6 +36,7 @@ bool ll2_plan(const DevModel& M, int holdoff, int flags, ll2::SmemPlan* sp, size
 cudaError_t ll2_configure(size_t smem);
 cudaError_t ll2_max_ctas(size_t smem, int* per_sm);
 cudaError_t ll2_launch(const DevModel& M, const CallArgs& A, const ll2::SmemPlan& sp, size_t smem, int n_ctas, cudaStream_t stream);
+cudaError_t rows_pack_launch(uint16_t* dst, const uint16_t* a, const uint16_t* b, int rows, int K, cudaStream_t stream);
 cudaError_t ll2_pack_launch(uint16_t* dst, const uint16_t* a, const uint16_t* b, int rows, int K, cudaStream_t stream);
 }  // namespace smol
 
@@ -67,15 +71,18 @@ struct SmolModel {
                                // barrier kernel / its tcgen05 variant (measured at bs=8: 1.5 ms per frame step against 2.3 ms)
     smol::ll2::SmemPlan ll2_sp;
     size_t ll2_smem = 0;
+    bool tmaps_ready = false;  // tensor maps of the prompt kernel (rebuilt after a weight / workspace bind)
+    bool prompt_ready = false; // its function attributes
     bool packed_ready = false; // tensor-core GEMV layout of the bound weights (rebuilt after a weight / workspace bind)
     int64_t launches = 0;
+    alignas(64) unsigned char kv_map[128] = {0};   // tensor map of the bound KV pool (tensor-core variant)
+    bool kv_map_ready = false;
     // mode 1: cached CUDA graph of one frame
     cudaGraphExec_t frame_graph = nullptr;
     cudaStream_t capture_stream = nullptr;  // the caller's stream may be the legacy default stream, which cannot capture
     GraphKey frame_key;
     bool frame_key_valid = false;
     int64_t frame_graph_launches = 0;
-    bool tmaps_ready = false;  // tensor maps of the tcgen05 variant (rebuilt after a weight / workspace bind)
 };
 
 static thread_local std::string g_err;
@@ -105,7 +112,7 @@ static int imax(int a, int b) { return a > b ? a : b; }
 
 struct WsLayout {
     size_t x, h, xf, q, attn, act, xn, silu_lut, tmaps, kpart, fkv, token_logits, depth_logits, frame_tokens, partial, split_count, barrier;
-    size_t ll, ll_epoch, ll2_score, ll2_tok, ll2_cand, packed, total;
+    size_t ll, ll_epoch, ll2_score, ll2_tok, ll2_cand, packed, packed_rows, total;
 };
 
 static int ll_batch_of(const SmolConfig& c) { (void)c; return smol::kLL2MaxTeams; }  // word regions for up to 8 teams
@@ -129,11 +136,11 @@ static size_t ll_regions(const SmolConfig& c, int depth, int bl, uint32_t* off, 
 
 static int ll2_score_len(const SmolConfig& c) { return (c.max_seq_len + 511) / 512 * 512; }
 // every GEMV matrix once more, in the tensor-core GEMV layout of the second-generation data-flow kernel
-static size_t packed_bytes(const SmolConfig& c, int depth) {
+static size_t packed_bytes(const SmolConfig& c, int depth) {   // (whole 16-row tiles: a ragged last one is padded)
     auto layer = [](size_t qkv_rows, size_t D, size_t F) { return (qkv_rows * D + D * D + 3 * D * F) * 2; };
     const size_t slow = layer((size_t)(c.n_head + 2 * c.n_local_heads) * 64, c.dim, c.intermediate_size);
     const size_t fast = layer((size_t)(c.fast_n_head + 2 * c.fast_n_local_heads) * 64, c.fast_dim, c.fast_intermediate_size);
-    const size_t heads = ((size_t)c.vocab_size * c.dim + (size_t)c.codebook_size * (c.depthwise_output ? depth : 1) * c.fast_dim) * 2;
+    const size_t heads = (align_up(c.vocab_size, 16) * c.dim + align_up(c.codebook_size, 16) * (c.depthwise_output ? depth : 1) * c.fast_dim) * 2;
     return c.n_layer * align_up(slow, 256) + c.n_fast_layer * align_up(fast, 256) + align_up(heads, 256) + 4096;
 }
 
@@ -161,10 +168,10 @@ static WsLayout ws_layout(const SmolConfig& c, int depth) {
     L.q = take(B * imax(c.n_head, c.fast_n_head) * 64 * 2);
     L.attn = take(B * dmax * 2);
     L.act = take(B * imax(c.intermediate_size, c.fast_intermediate_size) * 2);
-    L.xn = take(B * dmax * 2);
+    L.xn = take(B * c.dim * 2);
     L.silu_lut = take(65536 * 2);
     L.tmaps = take((size_t)smol::kTmTotal * smol::kTensorMapBytes);
-    L.kpart = take((size_t)smol::kTcKSplit * B * dmax * 4);
+    L.kpart = take((size_t)smol::kTcKSplit * B * c.dim * 4);
     L.fkv = take(B * c.n_fast_layer * 2 * depth * c.fast_n_local_heads * 64 * 2);
     L.token_logits = take(B * c.vocab_size * 4);
     L.depth_logits = take(B * depth * c.codebook_size * 4);
@@ -179,12 +186,16 @@ static WsLayout ws_layout(const SmolConfig& c, int depth) {
     L.ll2_tok = take((size_t)bl * (1 + depth) * smol::kLLMaxCtas * 8);
     L.ll2_cand = take((size_t)bl * (1 + depth) * smol::kLLRep * smol::kLLMaxCtas * 8);
     L.packed = take(packed_bytes(c, depth));
+    L.packed_rows = take(packed_bytes(c, depth));
     L.total = off;
     return L;
 }
 
 static int depth_of(const SmolConfig& c) { return c.num_codebooks - (c.duplicate_code_0 ? 0 : 1); }
 
+static bool tc_eligible(const SmolConfig& c) {   // whole 32-element blocks of K for every slice
+    return (c.dim % 64) == 0 && (c.fast_dim % 64) == 0 && (c.intermediate_size % 64) == 0 && (c.fast_intermediate_size % 64) == 0;
+}
 static int ensure_tmaps(SmolModel* m);
 static int ensure_packed(SmolModel* m);
 
@@ -280,10 +291,10 @@ int smol_bind_weights(SmolModel* m, const SmolWeights* w) {
     for (int l = 0; l < c.n_fast_layer; ++l)
         if (!bind_layer(w->fast_layers[l], d.fast_layers[l], "fast_layers[*]")) return SMOL_ERR_INVALID;
     m->weights_bound = true;
-    m->tmaps_ready = false;
     m->frame_key_valid = false;
     m->packed_ready = false;
-    // tensor maps and the packed GEMV layout are built here, at setup time: compute calls stay asynchronous and capturable
+    m->tmaps_ready = false;
+    // tensor maps and the packed layout are built here, at setup time: compute calls stay asynchronous and capturable
     if (m->ws_bound) {
         const int rc = ensure_tmaps(m);
         return rc ? rc : ensure_packed(m);
@@ -307,10 +318,10 @@ int smol_bind_workspace(SmolModel* m, void* d_workspace, size_t bytes) {
     d.q = (uint16_t*)(base + L.q); d.attn = (uint16_t*)(base + L.attn); d.act = (uint16_t*)(base + L.act);
     d.fkv = (uint16_t*)(base + L.fkv);
     d.xn = (uint16_t*)(base + L.xn); d.tmaps = (const unsigned char*)(base + L.tmaps);
-    d.silu_lut = (const uint16_t*)(base + L.silu_lut);
-    CU(smol::silu_lut_launch((uint16_t*)(base + L.silu_lut), nullptr));  // setup-time (synchronous with the memsets below)
     d.kpart = (float*)(base + L.kpart); d.ws_rows = ws_rows(m->cfg);
     m->tmaps_ready = false;
+    d.silu_lut = (const uint16_t*)(base + L.silu_lut);
+    CU(smol::silu_lut_launch((uint16_t*)(base + L.silu_lut), nullptr));  // setup-time (synchronous with the memsets below)
     d.token_logits = (float*)(base + L.token_logits); d.depth_logits = (float*)(base + L.depth_logits);
     d.frame_tokens = (int32_t*)(base + L.frame_tokens);
     d.partial = (float*)(base + L.partial); d.split_count = (uint32_t*)(base + L.split_count);
@@ -342,6 +353,7 @@ int smol_kv_bind(SmolModel* m, void* d_kv_pool, int32_t n_pages) {
     if (((uintptr_t)d_kv_pool) & 15) return fail(SMOL_ERR_INVALID, "smol_kv_bind: pool must be 16-byte aligned");
     m->dm.kv_pool = reinterpret_cast<uint16_t*>(d_kv_pool);
     m->dm.n_pages = n_pages;
+    m->kv_map_ready = false;
     m->kv_bound = true;
     m->frame_key_valid = false;
     return SMOL_OK;
@@ -367,54 +379,40 @@ static int ensure_configured(SmolModel* m) {
     return SMOL_OK;
 }
 
-// TMA tensor maps of the tcgen05 variant: encoded on the host and copied into the workspace once per bind (setup-time,
-// synchronous; compute calls never come here again).
-static bool tc_eligible(const SmolConfig& c) {  // the tiles stream K in 64-element stages
-    return (c.dim % 64) == 0 && (c.fast_dim % 64) == 0 && (c.intermediate_size % 64) == 0 && (c.fast_intermediate_size % 64) == 0;
-}
 
+// TMA tensor maps of the prompt kernel: encoded on the host and copied into the workspace once per bind (setup-time,
+// synchronous; compute calls never come here again).
 static int ensure_tmaps(SmolModel* m) {
     if (m->tmaps_ready) return SMOL_OK;
     const SmolConfig& c = m->cfg;
     if (!tc_eligible(c)) { m->tmaps_ready = true; return SMOL_OK; }  // such a model stays on the CUDA-core variants
     const DevModel& d = m->dm;
-    const int n_slots = smol::kTmTotal;
-    std::vector<CUtensorMap> maps((size_t)n_slots);
+    std::vector<CUtensorMap> maps((size_t)smol::kTmTotal);
     std::memset(maps.data(), 0, maps.size() * sizeof(CUtensorMap));
     static_assert(sizeof(CUtensorMap) == smol::kTensorMapBytes, "tensor map size");
     const uint64_t rows = (uint64_t)ws_rows(c);
-    const int dmax = imax(c.dim, c.fast_dim), fmax = imax(c.intermediate_size, c.fast_intermediate_size);
     bool ok = true;
-    auto act = [&](int slot, const void* p, int K, int pitch) {
+    auto act = [&](int slot, const void* p, int K) {
         for (int i = 0; i < 3; ++i)  // 128-, 64- and 32-row boxes
-            ok = ok && smol::make_tensor_map_2d(&maps[slot + i * smol::TM_ACT_MAPS], p, rows, K, pitch, 128u >> i);
+            ok = ok && smol::make_tensor_map_2d(&maps[slot + i * smol::TM_ACT_MAPS], p, rows, K, K, 128u >> i);
     };
     auto wgt = [&](int index, const void* p, uint64_t n, int K) {
         for (int box = 16; box <= 16 * smol::kTmWeightBoxes; box += 16)
             ok = ok && smol::make_tensor_map_2d(&maps[smol::tm_weight_slot(index, box)], p, n, K, K, (uint32_t)box);
     };
-    act(smol::TM_XN_S, d.xn, c.dim, dmax);
-    act(smol::TM_XN_F, d.xn, c.fast_dim, dmax);
-    act(smol::TM_ATTN_S, d.attn, c.dim, dmax);
-    act(smol::TM_ATTN_F, d.attn, c.fast_dim, dmax);
-    act(smol::TM_ACT_S, d.act, c.intermediate_size, fmax);
-    act(smol::TM_ACT_F, d.act, c.fast_intermediate_size, fmax);
-    wgt(0, d.head, c.vocab_size, c.dim);
-    wgt(1, d.fast_output, (uint64_t)c.codebook_size * (c.depthwise_output ? d.depth : 1), c.fast_dim);
-    for (int f = 0; f < 2; ++f) {
-        const int nl = f ? c.n_fast_layer : c.n_layer, D = f ? c.fast_dim : c.dim, F = f ? c.fast_intermediate_size : c.intermediate_size;
-        const int qkv = ((f ? c.fast_n_head : c.n_head) + 2 * (f ? c.fast_n_local_heads : c.n_local_heads)) * 64;
-        for (int l = 0; l < nl; ++l) {
-            const smol::DevLayer& L = f ? d.fast_layers[l] : d.layers[l];
-            wgt(smol::tm_weight_index(c.n_layer, f, l, 0), L.wqkv, qkv, D);
-            wgt(smol::tm_weight_index(c.n_layer, f, l, 1), L.wo, D, D);
-            wgt(smol::tm_weight_index(c.n_layer, f, l, 2), L.w1, F, D);
-            wgt(smol::tm_weight_index(c.n_layer, f, l, 3), L.w3, F, D);
-            wgt(smol::tm_weight_index(c.n_layer, f, l, 4), L.w2, D, F);
-        }
+    act(smol::TM_XN, d.xn, c.dim);
+    act(smol::TM_ATTN, d.attn, c.dim);
+    act(smol::TM_ACT, d.act, c.intermediate_size);
+    for (int l = 0; l < c.n_layer; ++l) {
+        const smol::DevLayer& L = d.layers[l];
+        wgt(smol::tm_weight_index(l, 0), L.wqkv, (uint64_t)(c.n_head + 2 * c.n_local_heads) * 64, c.dim);
+        wgt(smol::tm_weight_index(l, 1), L.wo, c.dim, c.dim);
+        wgt(smol::tm_weight_index(l, 2), L.w1, c.intermediate_size, c.dim);
+        wgt(smol::tm_weight_index(l, 3), L.w3, c.intermediate_size, c.dim);
+        wgt(smol::tm_weight_index(l, 4), L.w2, c.dim, c.intermediate_size);
     }
-    if (!ok) return fail(SMOL_ERR_CUDA, "cuTensorMapEncodeTiled failed for the tensor-core variant's operands");
-    CU(cudaMemcpy(const_cast<unsigned char*>(d.tmaps), maps.data(), (size_t)n_slots * smol::kTensorMapBytes, cudaMemcpyHostToDevice));
+    if (!ok) return fail(SMOL_ERR_CUDA, "cuTensorMapEncodeTiled failed for the prompt kernel's operands");
+    CU(cudaMemcpy(const_cast<unsigned char*>(d.tmaps), maps.data(), (size_t)smol::kTmTotal * smol::kTensorMapBytes, cudaMemcpyHostToDevice));
     m->tmaps_ready = true;
     return SMOL_OK;
 }
@@ -422,39 +420,45 @@ static int ensure_tmaps(SmolModel* m) {
 // The bound weights once more in the tensor-core GEMV layout ([16-row tile][K / 32][MMA step][lane][16 B]: ll2_kernel.cu),
 // written into the workspace by a device kernel at bind time (setup-time; the borrowed checkpoint tensors stay as they are
 // for the other kernels).
+// ... and once more as plain MMA fragments for the batched decode (rows_phases.cuh).
 static int ensure_packed(SmolModel* m) {
     if (m->packed_ready) return SMOL_OK;
     const SmolConfig& c = m->cfg;
     DevModel& d = m->dm;
-    if (c.dim % 32 || c.fast_dim % 32 || c.intermediate_size % 32 || c.fast_intermediate_size % 32 || c.vocab_size % 16 || c.codebook_size % 16) {
-        m->packed_ready = true;   // such a model stays on the other kernels (ll2_plan refuses it)
-        m->ll2_state = -1;
-        return SMOL_OK;
-    }
     char* ws = reinterpret_cast<char*>(d.x) - ws_layout(c, d.depth).x;
-    char* p = ws + ws_layout(c, d.depth).packed;
+    char* p = nullptr;
+    cudaError_t (*pack)(uint16_t*, const uint16_t*, const uint16_t*, int, int, cudaStream_t) = nullptr;
+    bool ok = true;
     auto put = [&](const uint16_t* a, const uint16_t* b, int rows, int K) -> const uint16_t* {
         uint16_t* dst = reinterpret_cast<uint16_t*>(p);
-        p += align_up((size_t)rows * (b ? 2 : 1) * K * 2, 256);
-        return smol::ll2_pack_launch(dst, a, b, rows, K, nullptr) == cudaSuccess ? dst : nullptr;
+        p += align_up(align_up((size_t)rows, 16) * (b ? 2 : 1) * K * 2, 256);
+        ok = ok && pack(dst, a, b, rows, K, nullptr) == cudaSuccess;
+        return dst;
     };
-    bool ok = true;
-    for (int f = 0; f < 2; ++f) {
-        const int nl = f ? c.n_fast_layer : c.n_layer, D = f ? c.fast_dim : c.dim, F = f ? c.fast_intermediate_size : c.intermediate_size;
-        const int qkv = ((f ? c.fast_n_head : c.n_head) + 2 * (f ? c.fast_n_local_heads : c.n_local_heads)) * 64;
-        for (int l = 0; l < nl; ++l) {
-            smol::DevLayer& L = f ? d.fast_layers[l] : d.layers[l];
-            L.pk_wqkv = put(L.wqkv, nullptr, qkv, D);
-            L.pk_wo = put(L.wo, nullptr, D, D);
-            L.pk_w13 = put(L.w1, L.w3, F, D);
-            L.pk_w2 = put(L.w2, nullptr, D, F);
-            ok = ok && L.pk_wqkv && L.pk_wo && L.pk_w13 && L.pk_w2;
+    const bool ll = !(c.dim % 32 || c.fast_dim % 32 || c.intermediate_size % 32 || c.fast_intermediate_size % 32 || c.vocab_size % 16 || c.codebook_size % 16);
+    if (!ll) m->ll2_state = -1;   // such a model stays on the other kernels (ll2_plan refuses it)
+    for (int form = 0; form < 2; ++form) {
+        if (form == 0 ? !ll : !tc_eligible(c)) continue;
+        p = ws + (form == 0 ? ws_layout(c, d.depth).packed : ws_layout(c, d.depth).packed_rows);
+        pack = form == 0 ? smol::ll2_pack_launch : smol::rows_pack_launch;
+        for (int f = 0; f < 2; ++f) {
+            const int nl = f ? c.n_fast_layer : c.n_layer, D = f ? c.fast_dim : c.dim, F = f ? c.fast_intermediate_size : c.intermediate_size;
+            const int qkv = ((f ? c.fast_n_head : c.n_head) + 2 * (f ? c.fast_n_local_heads : c.n_local_heads)) * 64;
+            for (int l = 0; l < nl; ++l) {
+                smol::DevLayer& L = f ? d.fast_layers[l] : d.layers[l];
+                (form ? L.pr_wqkv : L.pk_wqkv) = put(L.wqkv, nullptr, qkv, D);
+                (form ? L.pr_wo : L.pk_wo) = put(L.wo, nullptr, D, D);
+                (form ? L.pr_w13 : L.pk_w13) = put(L.w1, L.w3, F, D);
+                (form ? L.pr_w2 : L.pk_w2) = put(L.w2, nullptr, D, F);
+            }
+        }
+        (form ? d.pr_head : d.pk_head) = put(d.head, nullptr, c.vocab_size, c.dim);
+        for (int i = 0; i < (c.depthwise_output ? d.depth : 1); ++i) {   // one matrix per depth position, whole tiles each
+            const uint16_t* q = put(d.fast_output + (size_t)i * c.codebook_size * c.fast_dim, nullptr, c.codebook_size, c.fast_dim);
+            if (i == 0) (form ? d.pr_fast_output : d.pk_fast_output) = q;
         }
     }
-    d.pk_head = put(d.head, nullptr, c.vocab_size, c.dim);
-    d.pk_fast_output = put(d.fast_output, nullptr, c.codebook_size * (c.depthwise_output ? d.depth : 1), c.fast_dim);
-    ok = ok && d.pk_head && d.pk_fast_output;
-    if (!ok) return fail(SMOL_ERR_CUDA, "packing the weights for the data-flow kernel failed");
+    if (!ok) return fail(SMOL_ERR_CUDA, "packing the weights for the tensor-core kernels failed");
     CU(cudaDeviceSynchronize());   // setup-time only
     m->packed_ready = true;
     m->frame_key_valid = false;
@@ -486,15 +490,26 @@ static int ll2_solo_ctas(const SmolModel* m) {
     return m->n_ctas;
 }
 
+static int ensure_kv_map(SmolModel* m) {
+    if (!m->kv_map_ready) {   // the batch attention reads the pool through a tensor map: one row per position and head
+        static_assert(sizeof(CUtensorMap) == sizeof(CallArgs::kv_map), "tensor map size");
+        if ((uint64_t)m->dm.n_pages * m->cfg.n_layer > 0x7fffffffull) return fail(SMOL_ERR_UNSUPPORTED, "KV pool of more than 2^31 pages times layers");
+        if (!smol::make_tensor_map_kv(reinterpret_cast<CUtensorMap*>(m->kv_map), m->dm.kv_pool, (uint64_t)m->dm.n_pages * m->cfg.n_layer,
+                                      (uint64_t)m->cfg.n_local_heads * m->cfg.page_size))
+            return fail(SMOL_ERR_CUDA, "cuTensorMapEncodeTiled failed for the KV pool");
+        m->kv_map_ready = true;
+    }
+    return SMOL_OK;
+}
 // Shared-memory budget and function attributes of the kernel variant for this batch tile.
 static int ensure_tile(SmolModel* m, int bt) {
     if (bt == 0) {
-        const int rc = ensure_tmaps(m);
+        const int rc = ensure_kv_map(m);
         if (rc) return rc;
     }
     if (m->tile_ready[bt]) return SMOL_OK;
     m->xs_bytes[bt] = smol::decode_xs_bytes(m->dm, bt);
-    m->smem[bt] = m->xs_bytes[bt] + (bt == 0 ? 0 : smol::decode_stage_bytes(m->dm, m->n_ctas));  // bt 0: tensor-core variant, ring only
+    m->smem[bt] = m->xs_bytes[bt] + smol::decode_stage_bytes(m->dm, m->n_ctas, bt);
     if (m->smem[bt] > 227 * 1024)
         return fail(SMOL_ERR_UNSUPPORTED, "activation tile + weight stage exceed 227 KB of shared memory");
     CU(smol::decode_configure(bt, m->smem[bt]));
@@ -541,6 +556,10 @@ static int enqueue(SmolModel* m, CallArgs A, cudaStream_t stream, bool whole_ite
     rc = ensure_tile(m, bt);
     if (rc) return rc;
     A.repeat = m->repeat;
+    if (bt == 0) {
+        smol::rows_plan(m->dm, A.batch, m->n_ctas, A.rows_plan);
+        std::memcpy(A.kv_map, m->kv_map, sizeof(A.kv_map));
+    }
     if (m->mode != 1) {
         A.cooperative = 1;
         CU(smol::decode_launch(m->dm, A, bt, m->n_ctas, m->smem[bt], (int)m->xs_bytes[bt], stream));
@@ -569,19 +588,13 @@ static int enqueue(SmolModel* m, CallArgs A, cudaStream_t stream, bool whole_ite
             const smol::Phase ph = smol::unpack_phase(m->dm.prog[p]);
             const bool weights = ph.kind != smol::PH_ATTN && ph.kind != smol::PH_SAMPLE;
             if (bt == 0 && weights) {
-                // the grid barriers between a phase's pre-step, tiles and post-step become launch boundaries
-                const bool post = smol::tc_has_poststep(ph);
+                // the grid barrier between a phase's pre-step and its tiles becomes a launch boundary
                 if (smol::tc_has_prestep(ph)) {
                     A.tc_part = 1;
                     CU(smol::decode_launch(m->dm, A, bt, m->n_ctas, m->smem[bt], (int)m->xs_bytes[bt], stream));
                     m->launches += 1;
                 }
                 A.tc_part = 2;
-                if (post) {
-                    CU(smol::decode_launch(m->dm, A, bt, m->n_ctas, m->smem[bt], (int)m->xs_bytes[bt], stream));
-                    m->launches += 1;
-                    A.tc_part = 3;
-                }
             }
             A.finalize = last ? finalize : 0;
             A.advance = (p == end - 1) ? advance : 0;
@@ -589,6 +602,24 @@ static int enqueue(SmolModel* m, CallArgs A, cudaStream_t stream, bool whole_ite
             m->launches += 1;
         }
     }
+    return SMOL_OK;
+}
+
+// A prompt on the tensor cores: one cooperative launch over all its tiles, in every mode.
+static int enqueue_prompt(SmolModel* m, CallArgs A, cudaStream_t stream) {
+    int rc = ensure_tmaps(m);
+    if (rc || (rc = ensure_kv_map(m))) return rc;
+    if (!m->prompt_ready) {
+        int per_sm = 0;
+        CU(smol::prompt_configure(&per_sm));
+        if (per_sm < 1) return fail(SMOL_ERR_UNSUPPORTED, "prompt kernel does not fit on an SM");
+        m->prompt_ready = true;
+    }
+    A.cooperative = 1;
+    A.tc_split = m->tc_attn_split;
+    std::memcpy(A.kv_map, m->kv_map, sizeof(A.kv_map));
+    CU(smol::prompt_launch(m->dm, A, m->n_ctas, stream));
+    m->launches += 1;
     return SMOL_OK;
 }
 
@@ -635,7 +666,30 @@ int smol_prefill(SmolModel* m, const SmolBatch* b, int32_t batch, const int32_t*
     A.prompt = d_prompt;
     A.prompt_len = d_prompt_len;
     A.s_max = s_max;
+    if (use_tc(m, A.batch)) return enqueue_prompt(m, A, (cudaStream_t)stream);
     return enqueue(m, A, (cudaStream_t)stream, T == 1);  // tiled prefill runs on the barrier kernel
+}
+
+int smol_prompt_logits(SmolModel* m, const SmolBatch* b, const int32_t* d_prompt, int32_t n, void* stream) {
+    if (!m) return fail(SMOL_ERR_INVALID, "null model");
+    int rc = ensure_configured(m);
+    if (rc) return rc;
+    if ((rc = check_batch(m, b, 1))) return rc;
+    if (!d_prompt || n < 1) return fail(SMOL_ERR_INVALID, "smol_prompt_logits: bad prompt");
+    if (!use_tc(m, n)) return fail(SMOL_ERR_UNSUPPORTED, "smol_prompt_logits: fewer positions than option \"tc_min_batch\", or a model outside the tensor-core variant");
+    CallArgs A = base_args(b, 1, nullptr);
+    A.mode = 1;
+    int T = n < kPrefillRows ? n : kPrefillRows;
+    if (m->prefill_tile > 0 && m->prefill_tile < T) T = m->prefill_tile;
+    if (!use_tc(m, T)) T = m->tc_min_batch;
+    A.tile_t = T;
+    A.batch = T;
+    A.prompt = d_prompt;
+    A.s_max = n;
+    A.whole_prompt = n;
+    A.n_iter = (n + T - 1) / T;
+    A.head_row = n - 1 - (A.n_iter - 1) * T;
+    return enqueue_prompt(m, A, (cudaStream_t)stream);
 }
 
 int smol_slow_step(SmolModel* m, const SmolBatch* b, int32_t batch, int32_t advance, void* stream) {

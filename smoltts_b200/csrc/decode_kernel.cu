@@ -124,9 +124,11 @@ __device__ __forceinline__ void bulk_g2s(void* dst, const void* src, uint32_t by
                  ::"r"(smem_u32(dst)), "l"(src), "r"(bytes), "r"(smem_u32(bar)) : "memory");
 }
 __device__ __forceinline__ void fence_proxy_async() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
-// Generic-proxy writes (st.global of activations) <-> async-proxy reads (TMA tensor loads of the same buffers by other
-// CTAs): fenced on both sides of the grid barrier in the tensor-core variant.
+
+// Generic-proxy writes (st.global of activations) <-> async-proxy reads (bulk copies of the same rows by other CTAs): fenced
+// on both sides of the grid barrier in the tensor-core variant.
 __device__ __forceinline__ void fence_proxy_async_all() { asm volatile("fence.proxy.async;" ::: "memory"); }
+__device__ __forceinline__ void fence_proxy_async_global() { asm volatile("fence.proxy.async.global;" ::: "memory"); }
 
 struct Ctx {
     int cta, n_ctas, warp, lane, tid;
@@ -350,8 +352,16 @@ __device__ __forceinline__ int row_off(const CallArgs& A, int bg) { return A.til
 __device__ __forceinline__ int prefill_t(const CallArgs& A, const Ctx& c, int bg) {
     return A.iter_base + c.iter * (A.tile_t > 1 ? A.tile_t : 1) + row_off(A, bg);
 }
+// Prompt positions of sequence b that a prefill caches: all but the last column, which stays pending, or -- where the call
+// wants the last position's logits -- all of them (their number comes with the launch).
+__device__ __forceinline__ int prompt_positions(const CallArgs& A, int b) {
+    return A.whole_prompt > 0 ? A.whole_prompt : ldcg_i32(A.prompt_len + b) - 1;
+}
+__device__ __forceinline__ int prompt_last(const CallArgs& A, int b) {   // last column of the prompt
+    return A.whole_prompt > 0 ? A.whole_prompt - 1 : ldcg_i32(A.prompt_len + b) - 1;
+}
 __device__ __forceinline__ bool seq_active(const DevModel& M, const CallArgs& A, const Ctx& c, int bg) {
-    if (A.mode == 1) return prefill_t(A, c, bg) < ldcg_i32(A.prompt_len + row_seq(A, bg)) - 1;
+    if (A.mode == 1) return prefill_t(A, c, bg) < prompt_positions(A, row_seq(A, bg));
     return A.b.finished == nullptr || __ldcg(A.b.finished + bg) == 0;
 }
 
@@ -360,8 +370,8 @@ __device__ __forceinline__ int input_token(const DevModel& M, const CallArgs& A,
     if (A.mode == 1) {
         int t = prefill_t(A, c, bg);
         const int b = row_seq(A, bg);
-        const int len = ldcg_i32(A.prompt_len + b);
-        if (t > len - 1) t = len - 1;
+        const int last = prompt_last(A, b);
+        if (t > last) t = last;
         return ldcg_i32(A.prompt + ((size_t)b * M.n_rows + r) * A.s_max + t);
     }
     return ldcg_i32(A.b.tokens + (size_t)bg * M.n_rows + r);
@@ -489,14 +499,14 @@ __device__ __forceinline__ void fast_attention_rows(const DevModel& M, const Ctx
 // heads of a kv head share every K/V read.  Each 8-lane group owns one cached position per step
 // and keeps its own online-softmax state; states are merged across groups, warps and (through a
 // last-arriver fix-up in global memory) splits, always in a fixed order.
-__device__ void phase_attn_g(const DevModel& M, const CallArgs& A, const Ctx& c, const Phase& ph, int s_max) {
+__device__ void phase_attn_g(const DevModel& M, const CallArgs& A, const Ctx& c, const Phase& ph, int s_max, int row0, int n_rows) {
     constexpr int GM = kMaxGroup;
     const int Hq = M.n_head, Hkv = M.n_kv, ps = M.page_size, G = Hq / Hkv;
     const int dch = c.lane & 7, psub = c.lane >> 3;
     float* red = c.xs;  // [kWarps][G][kPartialStride]
-    const int n_units = A.batch * Hkv * s_max;
+    const int n_units = n_rows * Hkv * s_max;
     for (int u = c.cta; u < n_units; u += c.n_ctas) {
-        const int s = u % s_max, kvh = (u / s_max) % Hkv, b = u / (s_max * Hkv);
+        const int s = u % s_max, kvh = (u / s_max) % Hkv, b = row0 + u / (s_max * Hkv);
         const int bs = row_seq(A, b);  // the sequence whose cache this row reads (prefill tiles: several rows per sequence)
         int Lb = ldcg_i32(A.b.seq_len + bs) + row_off(A, b) + 1;
         const int cap = A.b.max_pages * ps;
@@ -654,14 +664,13 @@ __device__ int attn_splits(const DevModel& M, int batch, int n_ctas) {
 }
 
 __device__ void phase_attn(const DevModel& M, const CallArgs& A, const Ctx& c, const Phase& ph) {
-    phase_attn_g(M, A, c, ph, attn_splits(M, A.batch, c.n_ctas));
+    phase_attn_g(M, A, c, ph, attn_splits(M, A.batch, c.n_ctas), 0, A.batch);
 }
 
 }  // namespace smol
-#include "tc_phases.cuh"
+#include "rows_phases.cuh"
+#include "prompt_phases.cuh"
 namespace smol {
-
-__shared__ __align__(8) umma::Bars g_tc_bars;
 
 // Every phase that streams weights: [gather / RMSNorm / fast attention] -> staged-weight GEMV ->
 // epilogue.  One function so that each building block is instantiated exactly once (code size is what
@@ -799,11 +808,7 @@ __device__ void phase_gemv(const DevModel& M, const CallArgs& A, const Ctx& c, c
 
 // Sampling of one id per sequence (G:88-99 slow, G:118-132 depth) and, after the last depth code,
 // frame assembly and the stop rule (G:143-166).
-// tc_feed (tensor-core variant, cooperative launch, a depth step follows in the launch): the CTA that chose row b's id also
-// writes the next depth step's input -- the slow hidden state after the slow id, the embedding of the code after a depth
-// code (G:136-140) -- to the fast residual stream and its RMSNorm to M.xn, exactly as that step's own pre-step would
-// (tc_row_step: same chunks per warp, same order of additions), which then is skipped.
-__device__ void phase_sample(const DevModel& M, const CallArgs& A, const Ctx& c, const Phase& ph, bool tc_feed = false) {
+__device__ void phase_sample(const DevModel& M, const CallArgs& A, const Ctx& c, const Phase& ph) {
     const bool fast = ph.fast != 0;
     const int N = fast ? M.codebook_size : M.vocab;
     const int r = fast ? 1 + ph.depth_pos : 0;
@@ -840,56 +845,23 @@ __device__ void phase_sample(const DevModel& M, const CallArgs& A, const Ctx& c,
                 }
             }
         }
-        if (tc_feed) {
-            const int D = M.fdim, nch = D >> 3, ch = c.tid;
-            const int next_pos = fast ? ph.depth_pos + 1 : 0;
-            const uint16_t* row = !fast ? M.x + (size_t)b * D
-                                        : M.fast_embeddings + (size_t)(tok + (M.depthwise_wte ? (M.dup0 ? next_pos - 1 : next_pos) * M.codebook_size : 0)) * D;
-            const uint16_t* norm_w = M.fast_layers[0].attention_norm;
-            float x[8];
-            float ss = 0.f;
-            uint4 wv = make_uint4(0u, 0u, 0u, 0u);
-            if (ch < nch) {
-                wv = __ldg(reinterpret_cast<const uint4*>(norm_w + ch * 8));
-                unpack8(ldcg_v4(row + ch * 8), x);
-#pragma unroll
-                for (int e = 0; e < 8; ++e) ss = fmaf(x[e], x[e], ss);
-            }
-            ss = warp_sum(ss);
-            if (c.lane == 0) g_part[c.warp] = ss;
-            __syncthreads();
-            if (ch < nch) {
-                float t = 0.f;
-                for (int i = 0; i < 3; ++i) t += g_part[i];
-                const float mean = __fdiv_rn(t, (float)D);
-                const float rs = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(mean, M.eps)));
-                uint4 raw;
-                raw.x = pack_bf16(x[0], x[1]); raw.y = pack_bf16(x[2], x[3]); raw.z = pack_bf16(x[4], x[5]); raw.w = pack_bf16(x[6], x[7]);
-                *reinterpret_cast<uint4*>(M.xf + (size_t)b * D + ch * 8) = raw;
-                float wf[8];
-                unpack8(wv, wf);
-                uint4 o;
-                o.x = pack_bf16(__fmul_rn(bf16_round(__fmul_rn(x[0], rs)), wf[0]), __fmul_rn(bf16_round(__fmul_rn(x[1], rs)), wf[1]));
-                o.y = pack_bf16(__fmul_rn(bf16_round(__fmul_rn(x[2], rs)), wf[2]), __fmul_rn(bf16_round(__fmul_rn(x[3], rs)), wf[3]));
-                o.z = pack_bf16(__fmul_rn(bf16_round(__fmul_rn(x[4], rs)), wf[4]), __fmul_rn(bf16_round(__fmul_rn(x[5], rs)), wf[5]));
-                o.w = pack_bf16(__fmul_rn(bf16_round(__fmul_rn(x[6], rs)), wf[6]), __fmul_rn(bf16_round(__fmul_rn(x[7], rs)), wf[7]));
-                *reinterpret_cast<uint4*>(M.xn + (size_t)b * D + ch * 8) = o;
-            }
-        }
         __syncthreads();
     }
 }
 
-// BT == 0: the tensor-core variant (tc_phases.cuh) -- 128-row tiles, batch attention, cooperative launches only.
+// BT == 0: the tensor-core variant (rows_phases.cuh) for 9 and more rows.
 template <int BT>
 __device__ __forceinline__ void run_phase(const DevModel& M, const CallArgs& A, const Ctx& c, const Phase& ph,
-                                          uint32_t& parity, umma::Pipe& pipe, uint32_t& target, bool first_in_launch,
-                                          bool next_in_launch) {
+                                          uint32_t& parity, RowsSync& sy, uint32_t packed_phase, const RowsStep* step) {
     if (BT == 0) {
-        if (ph.kind == PH_ATTN) phase_attn_batch(M, A, c, ph);
-        else if (ph.kind == PH_SAMPLE)
-            phase_sample(M, A, c, ph, A.cooperative && next_in_launch && !A.fast_from_xf && !(ph.fast && ph.depth_pos == M.depth - 1));
-        else phase_gemm_tc(M, A, c, ph, &g_tc_bars, pipe, target, first_in_launch, next_in_launch);
+        if (ph.kind == PH_ATTN) {
+            phase_attn_batch<false>(M, A, c, ph, sy, A.kv_map);
+        } else if (ph.kind == PH_SAMPLE) {
+            rows_sync_in(M, sy);
+            phase_sample(M, A, c, ph);
+        } else {
+            phase_rows(M, A, c, packed_phase, sy, step);
+        }
         return;
     }
     if (ph.kind == PH_ATTN) phase_attn(M, A, c, ph);
@@ -911,7 +883,7 @@ __device__ __forceinline__ bool next_weight_phase(const DevModel& M, const CallA
 template <int BT>
 __global__ void __launch_bounds__(kThreads, 1)
 smol_decode_kernel(const __grid_constant__ DevModel M, const __grid_constant__ CallArgs A, const int xs_bytes) {
-    extern __shared__ __align__(128) unsigned char smem_dyn[];
+    extern __shared__ __align__(1024) unsigned char smem_dyn[];
     Ctx c;
     c.cta = blockIdx.x; c.n_ctas = gridDim.x; c.tid = threadIdx.x;
     c.warp = threadIdx.x >> 5; c.lane = threadIdx.x & 31;
@@ -920,7 +892,10 @@ smol_decode_kernel(const __grid_constant__ DevModel M, const __grid_constant__ C
     c.iter = 0;
 
     if (c.tid == 0) {
-        for (int w = 0; w < kWarps; ++w) mbar_init(&g_mbar[w], 1u);
+        for (int w = 0; w < kWarps; ++w) {
+            mbar_init(&g_mbar[w], 1u);
+            if (BT == 0) { for (int i = 2 * w; i < 2 * w + 2; ++i) { mbar_init(&g_kvbar[i], 1u); g_kvpar[i] = 0u; } }
+        }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     __syncthreads();
@@ -928,37 +903,53 @@ smol_decode_kernel(const __grid_constant__ DevModel M, const __grid_constant__ C
     uint32_t target = 0;
     if (A.cooperative) target = ldcg_u32(M.barrier + 1);
     uint32_t parity = 0;
-    umma::Pipe pipe;
-    pipe.chunk = 0; pipe.tile = 0;
-    if (BT == 0) umma::setup(&g_tc_bars, pipe, (uint32_t)umma::kAcc, 2u);
     const int per_iter = (A.mode == 1) ? phases_per_prefill_step(M.n_layer)
                                        : phases_per_frame(M.n_layer, M.n_flayer, M.depth);
     const bool prof_cta = (M.prof != nullptr) && c.cta == 0;  // CTA-uniform
     const bool prof = prof_cta && c.tid == 0;
     unsigned long long t0 = 0, t1 = 0;
+    RowsSync sy;
+    sy.target = target; sy.par_w = 0; sy.par_x = 0; sy.pending = false; sy.phase = 0; sy.next = -1; sy.waits_for = 0;
+    RowsStep* steps = reinterpret_cast<RowsStep*>(smem_dyn);   // tensor-core variant: phase table | rows, partial sums | weights
+    if (BT == 0) {
+        c.xs = reinterpret_cast<float*>(smem_dyn + xs_bytes - kRowsP);
+        rows_tables(M, A, c, steps);
+    }
     int st_it = -1, st_p = -1;  // (iteration, phase) whose weights are staged / in flight
     for (int it = 0; it < A.n_iter; ++it) {
         c.iter = it;
         for (int p = A.phase_begin; p < A.phase_end; ++p) {
-            const Phase ph = unpack_phase(M.prog[p]);
-            const bool has_w = BT != 0 && ph.kind != PH_ATTN && ph.kind != PH_SAMPLE;  // weights staged a phase ahead (GEMV variants)
+            const uint32_t packed_phase = M.prog[p];
+            const Phase ph = unpack_phase(packed_phase);
+            const bool has_w = ph.kind != PH_ATTN && ph.kind != PH_SAMPLE;  // weights are staged a phase ahead
+            const RowsStep* step = steps + (p - A.phase_begin);
             if (prof) t0 = globaltimer_ns();
             if (has_w && !(st_it == it && st_p == p)) {  // cold start of a launch
-                stage_issue(c, phase_plan(M, ph));
+                if (BT == 0) {
+                    if (c.tid == kThreads - 32 && A.tc_part != 1) rows_issue(c.stage + g_rk[ph.fast][ph.kind].off, step->w, g_rk[ph.fast][ph.kind].bytes);
+                } else {
+                    stage_issue(c, phase_plan(M, ph));
+                }
                 st_it = it; st_p = p;
             }
-            run_phase<BT>(M, A, c, ph, parity, pipe, target, p == A.phase_begin, p + 1 < A.phase_end);
+            if (BT == 0 && has_w) {   // the tiles of the next weight phase are fetched from inside this one
+                int nit = it, np = p;
+                sy.phase = p;
+                sy.next = next_weight_phase(M, A, nit, np) ? np : -1;
+                if (sy.next >= 0) { st_it = nit; st_p = np; }
+            }
+            run_phase<BT>(M, A, c, ph, parity, sy, packed_phase, step);
             if (prof_cta) {
                 __syncthreads();
                 if (prof) t1 = globaltimer_ns();
             }
-            // (tensor-core variant, one phase per launch: a phase may take up to three launches; bookkeeping runs in the last)
-            const bool final_part = A.tc_part == 0 || A.tc_part == (tc_has_poststep(ph) ? 3 : 2);
+            // (tensor-core variant, one phase per launch: a phase may take two launches; bookkeeping runs in the last)
+            const bool final_part = A.tc_part != 1;
             if (c.cta == 0 && p == per_iter - 1 && A.mode == 1 && final_part) {
                 // prefill bookkeeping: every sequence advances by the positions of this tile that lie inside its prompt
                 const int T = A.tile_t > 1 ? A.tile_t : 1;
                 for (int b = c.tid; b < A.real_batch; b += kThreads) {
-                    int n_act = ldcg_i32(A.prompt_len + b) - 1 - (A.iter_base + c.iter * T);
+                    int n_act = prompt_positions(A, b) - (A.iter_base + c.iter * T);
                     n_act = n_act < 0 ? 0 : (n_act > T ? T : n_act);
                     if (n_act) A.b.seq_len[b] = ldcg_i32(A.b.seq_len + b) + n_act;
                 }
@@ -968,11 +959,13 @@ smol_decode_kernel(const __grid_constant__ DevModel M, const __grid_constant__ C
             }
             const bool last = (it == A.n_iter - 1) && (p == A.phase_end - 1);
             const bool sync = A.cooperative && !last;
-            if (sync) {
-                if (BT == 0) fence_proxy_async_all();
-                grid_arrive(M.barrier, target, (uint32_t)c.n_ctas);
+            if (BT == 0) {
+                if (prof) { M.prof[2 * p] += t1 - t0; sy.waits_for = p; }
+                if (sync) rows_arrive(M, c, sy);
+                continue;
             }
-            if (has_w) {
+            if (sync) grid_arrive(M.barrier, target, (uint32_t)c.n_ctas);
+            if (BT != 0 && has_w) {
                 // Every warp is past its last read of the stage buffer (phases end with a block barrier):
                 // stream the next weight phase in while the other CTAs arrive at the grid barrier.
                 int nit = it, np = p;
@@ -983,7 +976,6 @@ smol_decode_kernel(const __grid_constant__ DevModel M, const __grid_constant__ C
             }
             if (sync) {
                 grid_wait(M.barrier, target);
-                if (BT == 0 && (c.tid == umma::kTmaProducerA || c.tid == umma::kTmaProducerB)) fence_proxy_async_all();   // the threads that issue TMA loads
             }
             if (prof) {  // [2p] CTA 0's own time in the phase, [2p+1] its wait at the barrier that follows
                 const unsigned long long t2 = globaltimer_ns();
@@ -996,12 +988,10 @@ smol_decode_kernel(const __grid_constant__ DevModel M, const __grid_constant__ C
         // leave the last prompt column as the pending input of the first decode frame (G:66-73)
         for (int i = c.tid; i < A.real_batch * M.n_rows; i += kThreads) {
             const int b = i / M.n_rows, r = i - b * M.n_rows;
-            const int len = ldcg_i32(A.prompt_len + b);
-            A.b.tokens[i] = ldcg_i32(A.prompt + ((size_t)b * M.n_rows + r) * A.s_max + (len - 1));
+            A.b.tokens[i] = ldcg_i32(A.prompt + ((size_t)b * M.n_rows + r) * A.s_max + prompt_last(A, b));
         }
     }
-    if (A.cooperative && c.cta == 0 && c.tid == 0) M.barrier[1] = target;
-    if (BT == 0) umma::teardown(&g_tc_bars);
+    if (A.cooperative && c.cta == 0 && c.tid == 0) M.barrier[1] = BT == 0 ? sy.target : target;
 }
 
 // Stand-alone sampler on caller-provided logits [B][n] (smol_sample): one CTA per sequence.
@@ -1051,6 +1041,31 @@ cudaError_t silu_lut_launch(uint16_t* lut, cudaStream_t stream) {
     return cudaGetLastError();
 }
 
+// A matrix [rows][K] as mma.m16n8k16 A fragments: [16-row tile][K / 16][lane][16 bytes = a0..a3]; with b (the gated MLP) a tile is
+// 8 rows of a over the same 8 rows of b.  Rows past the matrix are zeros.
+__global__ void smol_rows_pack_kernel(uint16_t* dst, const uint16_t* a, const uint16_t* b, int rows, int K) {
+    const int steps = K / 16;
+    const size_t n = (size_t)(b ? rows / 8 : (rows + 15) / 16) * steps * 32;
+    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
+        const int lane = (int)(i & 31), g = lane >> 2, c = lane & 3;
+        const size_t rest = i >> 5, tile = rest / steps;
+        const int e = (int)(rest % steps) * 16 + 2 * c;
+        const size_t r0 = b ? tile * 8 + g : tile * 16 + g, r1 = b ? r0 : r0 + 8;
+        const uint16_t* hi = b ? b : a;
+        const bool in0 = r0 < (size_t)rows, in1 = r1 < (size_t)rows;
+        uint4 v;
+        v.x = in0 ? *reinterpret_cast<const uint32_t*>(a + r0 * K + e) : 0u;
+        v.y = in1 ? *reinterpret_cast<const uint32_t*>(hi + r1 * K + e) : 0u;
+        v.z = in0 ? *reinterpret_cast<const uint32_t*>(a + r0 * K + e + 8) : 0u;
+        v.w = in1 ? *reinterpret_cast<const uint32_t*>(hi + r1 * K + e + 8) : 0u;
+        *reinterpret_cast<uint4*>(dst + i * 8) = v;
+    }
+}
+cudaError_t rows_pack_launch(uint16_t* dst, const uint16_t* a, const uint16_t* b, int rows, int K, cudaStream_t stream) {
+    smol_rows_pack_kernel<<<1024, 256, 0, stream>>>(dst, a, b, rows, K);
+    return cudaGetLastError();
+}
+
 cudaError_t store_codes_launch(int32_t* frame_tokens, const int32_t* codes, int batch, int n_rows, int row,
                                cudaStream_t stream) {
     smol_store_codes_kernel<<<(batch + 127) / 128, 128, 0, stream>>>(frame_tokens, codes, batch, n_rows, row);
@@ -1061,7 +1076,8 @@ cudaError_t store_codes_launch(int32_t* frame_tokens, const int32_t* codes, int 
 // Activation region: the batch tile's rows in fp32 (also the attention merge scratch and the
 // sampler's logits row).  Sized for the batch the model was created for.
 size_t decode_xs_bytes(const DevModel& M, int bt) {
-    if (bt == 0) return (size_t)umma::kRingBytes + 2048 + kTcRows * 4;  // 1024-aligned ring + RoPE positions of the tile's rows
+    if (bt == 0)   // partial sums (the sampler's logits row, <= 16 KB, fits too) and the phase table
+        return (size_t)kRowsP + ((size_t)phases_per_frame(M.n_layer, M.n_flayer, M.depth) * sizeof(RowsStep) + 1023) / 1024 * 1024;
     int kmax = M.dim;
     if (M.inter > kmax) kmax = M.inter;
     if (M.fdim > kmax) kmax = M.fdim;
@@ -1076,7 +1092,8 @@ size_t decode_xs_bytes(const DevModel& M, int bt) {
 }
 
 // Stage region: the weight rows one CTA owns in the heaviest phase.
-size_t decode_stage_bytes(const DevModel& M, int n_ctas) {
+size_t decode_stage_bytes(const DevModel& M, int n_ctas, int bt) {
+    if (bt == 0) return (size_t)kRowsW;
     auto per = [&](long units, long slot) { return (size_t)((units + n_ctas - 1) / n_ctas) * (size_t)slot; };
     size_t m = 0;
     auto upd = [&](size_t v) { if (v > m) m = v; };
@@ -1091,6 +1108,49 @@ size_t decode_stage_bytes(const DevModel& M, int n_ctas) {
     upd(per(M.fdim, 2L * M.finter));
     upd(per(M.codebook_size, 2L * M.fdim));
     return (m + 127) / 128 * 128;
+}
+
+// Tile plan of the tensor-core variant's weight phases for `rows` activation rows: tiles per block and rows per group, by
+// a model of a CTA's clocks between two barriers -- L2 -> shared memory at 85 bytes per clock, RMSNorm and depth attention
+// repeated per tile block, MMAs at 0.5 clocks, weight fragments and partial sums through shared memory at 128 bytes per clock,
+// and a fixed part per row group (load latency, block barriers).
+void rows_plan(const DevModel& M, int rows, int n_ctas, RowsPlan (*plan)[6]) {
+    for (int f = 0; f < 2; ++f) {
+        const int D = f ? M.fdim : M.dim, F = f ? M.finter : M.inter, heads = f ? M.fn_head + 2 * M.fn_kv : M.n_head + 2 * M.n_kv;
+        for (int kind = 0; kind <= PH_HEAD; ++kind) {
+            RowsPlan& best = plan[f][kind];
+            best.mt = 1; best.n = 8;
+            if (kind == PH_ATTN) continue;
+            const bool wide = kind == PH_W2, attn = kind == PH_WO && f;
+            const int K = wide ? F : D;
+            const int tiles = kind == PH_QKV ? heads * kHeadDim / 16 : kind == PH_W13 ? F / 8 : kind == PH_HEAD ? ((f ? M.codebook_size : M.vocab) + 15) / 16 : D / 16;
+            const bool normed = kind == PH_QKV || kind == PH_W13 || kind == PH_HEAD;
+            double best_cost = 0.;
+            for (int n = 8; n <= (wide ? 24 : kRowsMax); n += wide ? 8 : n) {
+                const bool split = wide || kind == PH_WO;
+                const int kg = split ? (K % 256 == 0 ? 16 : K % 128 == 0 ? 8 : 4) : 4;    // chains, each with partial sums
+                const int mt_max = wide ? 1 : kind == PH_WO ? (f ? kRowsTilesWo : kRowsTilesSlowWo) : kRowsTiles;
+                const int groups = (rows + n - 1) / n;
+                const int live = (rows + groups - 1) / groups;     // rows of a group when they are shared out evenly
+                for (int mt = 1; mt <= mt_max && mt * 16 * (split ? 16 : 4) * n * 4 <= kRowsP && mt <= tiles; ++mt) {
+                    const int blocks = (tiles + mt - 1) / mt;
+                    const long share = blocks <= n_ctas ? n_ctas / blocks : 1;
+                    const long turns = blocks <= n_ctas ? (groups + share - 1) / share : (long)((blocks + n_ctas - 1) / n_ctas) * groups;
+                    double c = 1600. + live * K * 2 / 85.;
+                    if (normed) c += live * K / 32.;
+                    if (attn) c += 900. * ((live * M.fn_kv + 2 * kWarps - 1) / (2 * kWarps));
+                    // shared-memory reads: split chains read everything once, else the rows are read by four groups of warps
+                    c += (wide ? 0. : mt * (double)K * 32 / 128.) + (split ? 1. : 4.) * n * K * 2 / 128. + 200. * (split ? 1 : (mt + 3) / 4);
+                    c += mt * (double)live * 16 * kg * 4 * 2 / 128.;
+                    c *= turns;
+                    c += mt * K * 32 / 640.;                        // weights: hidden behind the barrier unless they are many
+                    if (best_cost == 0. || c < best_cost) { best_cost = c; best.mt = (uint8_t)mt; best.n = (uint8_t)n; }
+                }
+            }
+            const int groups = (rows + best.n - 1) / best.n;        // even groups: 212 rows are 4 x 53, not 3 x 64 + 20
+            best.n = (uint8_t)((rows + groups - 1) / groups);
+        }
+    }
 }
 
 // Kernel variant by batch tile (sequences whose activations share one pass over the weights).
@@ -1118,6 +1178,16 @@ cudaError_t decode_configure(int bt, size_t smem) {
 
 cudaError_t decode_max_ctas(int bt, size_t smem, int* per_sm) {
     return cudaOccupancyMaxActiveBlocksPerMultiprocessor(per_sm, decode_fn(bt), kThreads, smem);
+}
+
+size_t prompt_smem() { return (size_t)kPrSmem; }
+cudaError_t prompt_configure(int* per_sm) {
+    cudaError_t e = cudaFuncSetAttribute(smol_prompt_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kPrSmem);
+    return e != cudaSuccess ? e : cudaOccupancyMaxActiveBlocksPerMultiprocessor(per_sm, smol_prompt_kernel, kThreads, kPrSmem);
+}
+cudaError_t prompt_launch(const DevModel& M, const CallArgs& A, int n_ctas, cudaStream_t stream) {
+    void* args[2] = {(void*)&M, (void*)&A};
+    return cudaLaunchCooperativeKernel((const void*)smol_prompt_kernel, dim3(n_ctas), dim3(kThreads), args, kPrSmem, stream);
 }
 
 cudaError_t decode_launch(const DevModel& M, const CallArgs& A, int bt, int n_ctas, size_t smem, int xs_bytes,

@@ -61,6 +61,11 @@ struct DevLayer {
     const uint16_t* pk_wo;
     const uint16_t* pk_w13;
     const uint16_t* pk_w2;
+    // the same as plain mma.m16n8k16 A fragments (rows_phases.cuh; smol_rows_pack_kernel)
+    const uint16_t* pr_wqkv;
+    const uint16_t* pr_wo;
+    const uint16_t* pr_w13;
+    const uint16_t* pr_w2;
 };
 
 struct DevModel {
@@ -98,11 +103,11 @@ struct DevModel {
     uint16_t* q;        // rotated queries                 [B][max(n_head,fn_head)*64]
     uint16_t* attn;     // attention output                [B][max(dim,fdim)]
     uint16_t* act;      // silu(w1 x) * w3 x               [B][max(inter,finter)]
-    uint16_t* xn;       // tensor-core variant: RMSNorm output feeding the next weight phase  [B][max(dim,fdim)]
-    const uint16_t* silu_lut;  // bf16 silu of every bf16 input [65536] (exact expression, filled at bind time)
-    const unsigned char* tmaps;  // tensor-core variant: TMA tensor maps (128 B each, TensorMapSlot), in the workspace
-    float* kpart;       // tensor-core variant: split-K partial sums of the wo / w2 tiles  [kTcKSplit][ws_rows][max(dim,fdim)] fp32
+    uint16_t* xn;       // prompts: RMSNorm output feeding the next weight phase  [rows][dim]
+    const unsigned char* tmaps;  // prompts: TMA tensor maps (128 B each, TensorMapSlot), in the workspace
+    float* kpart;       // prompts: partial sums of the K slices of the wo / w2 tiles  [kTcKSplit][ws_rows][dim] fp32
     int ws_rows;        // rows of every workspace buffer
+    const uint16_t* silu_lut;  // bf16 silu of every bf16 input [65536] (exact expression, filled at bind time)
     uint16_t* fkv;      // fast KV  [B][n_flayer][2][depth][fn_kv*64]
     float* token_logits;  // [B][vocab]           (bf16-rounded values)
     float* depth_logits;  // [B][depth][codebook] (bf16-rounded values)
@@ -125,6 +130,8 @@ struct DevModel {
     uint32_t ll_off[kMaxProg];
     uint16_t ll_len[kMaxProg];
 
+    const uint16_t* pr_head;         // heads in the fragments of the batched decode
+    const uint16_t* pr_fast_output;
     const uint16_t* pk_head;         // packed LM head
     const uint16_t* pk_fast_output;  // packed depth heads (row groups in checkpoint order)
     unsigned long long* ll2_score;   // attention scores {fp32 bits, epoch} [teams][2][n_head][ll2_score_len] words
@@ -149,6 +156,11 @@ __host__ __device__ inline int ll_phase_words(int kind, int fast, int dim, int n
     return (n + 15) / 16 * 16;
 }
 
+// Tensor-core variant: 16-row weight tiles per block and activation rows per group of a weight phase (rows_phases.cuh).
+struct RowsPlan {
+    uint8_t mt, n;
+};
+
 // Per-launch arguments (passed by value).
 struct CallArgs {
     SmolBatch b;
@@ -166,13 +178,17 @@ struct CallArgs {
     int repeat;       // profiling only: run the body of every weight phase 1 + repeat times
     int tile_t;       // prefill: prompt positions handled per iteration (rows = real_batch * tile_t share the weight pass)
     int real_batch;   // prefill: sequences (rows / tile_t)
-    int tc_part;      // tensor-core variant, one phase per launch: 1 = only the phase's distributed pre-step, 2 = only its tiles,
-                      // 3 = only its post-step (0 = the whole phase: cooperative launches)
+    int tc_part;      // tensor-core variant, one phase per launch: 1 = only the phase's pre-step, 2 = only its tiles
+                      // (0 = the whole phase: cooperative launches)
     int tc_split;     // tensor-core variant: cached positions per attention split (0 = default)
     int team_ctas;    // second-generation data-flow kernel: CTAs per sequence (one team each); grid = batch * team_ctas
     const int32_t* prompt;      // prefill: [B][n_rows][s_max]
     const int32_t* prompt_len;  // prefill: [B]
     int s_max;
+    int whole_prompt; // prefill: cache all prompt_len positions (1) or all but the last, which stays pending (0)
+    int head_row;     // whole_prompt: row of the last prompt position in the last tile
+    RowsPlan rows_plan[2][6];   // tensor-core variant: [slow / depth transformer][phase kind]
+    alignas(64) unsigned char kv_map[128];   // ... tensor map of the paged pool: rows of 64 elements, boxes of 16 rows
 };
 
 // Phase kinds of one decode frame, in program order.
@@ -226,32 +242,21 @@ __host__ __device__ inline Phase decode_phase(int p, int n_layer, int n_flayer) 
     return ph;
 }
 
-// Tensor-core variant: phases that start with a grid-wide pre-step (embedding / input gather + RMSNorm into xn, or the
-// depth attention) -- every weight phase except the slow wo and the w2's, whose inputs the previous phase left in place.
-__host__ __device__ inline bool tc_has_prestep(const Phase& ph) {
-    if (ph.kind == PH_ATTN || ph.kind == PH_SAMPLE) return false;
-    return !(ph.kind == PH_W2 || (ph.kind == PH_WO && !ph.fast));
-}
+// Tensor-core variant: the phase that starts with a grid-wide pre-step (the token embedding of the slow transformer's input).
+__host__ __device__ inline bool tc_has_prestep(const Phase& ph) { return ph.kind == PH_QKV && !ph.fast && ph.layer == 0; }
 
-// Slots of the tensor-map table (DevModel.tmaps).  Activations: boxes of 128 rows (slots 0-5), 64 rows (6-11: batches of
-// at most 64 rows load half a tile) and 32 rows (12-17).  Weights: one map per matrix and box height 16 * (v + 1) rows,
-// v = 0..5, so that a tile's weight rows are ONE copy per stage (a TMA instruction costs its issuing thread ~60 ns).
-enum TensorMapSlot {
-    TM_XN_S = 0, TM_XN_F, TM_ATTN_S, TM_ATTN_F, TM_ACT_S, TM_ACT_F, TM_ACT_MAPS = 6, TM_WEIGHTS = 18
-};
+// Prompts (prompt_phases.cuh): slots of the tensor-map table (DevModel.tmaps).  Activations: boxes of 128 rows, of 64 and of 32;
+// weights of the slow transformer: one map per matrix and box height 16 * (v + 1) rows, v = 0..5, so that a tile's weight rows
+// are ONE copy per stage.
+enum TensorMapSlot { TM_XN = 0, TM_ATTN, TM_ACT, TM_ACT_MAPS = 3, TM_WEIGHTS = 9 };
 constexpr int kTmWeightBoxes = 6;
-constexpr int kTmWeightStride = 2 + 5 * (SMOL_MAX_LAYERS + SMOL_MAX_FAST_LAYERS);  // weight matrices a model can have
+constexpr int kTmWeightStride = 5 * SMOL_MAX_LAYERS;       // weight matrices a model can have
 constexpr int kTmTotal = TM_WEIGHTS + kTmWeightBoxes * kTmWeightStride;
-// weight index: 0 LM head, 1 depth heads, then 5 per layer (wqkv, wo, w1, w3, w2): slow layers first, fast layers after them
-__host__ __device__ inline int tm_weight_index(int n_layer, int fast, int layer, int which) {
-    return 2 + ((fast ? n_layer : 0) + layer) * 5 + which;
-}
-__host__ __device__ inline int tm_weight_slot(int weight_index, int box_rows) {
-    return TM_WEIGHTS + (box_rows / 16 - 1) * kTmWeightStride + weight_index;
-}
+// weight index: 5 per layer (wqkv, wo, w1, w3, w2)
+__host__ __device__ inline int tm_weight_index(int layer, int which) { return layer * 5 + which; }
+__host__ __device__ inline int tm_weight_slot(int weight_index, int box_rows) { return TM_WEIGHTS + (box_rows / 16 - 1) * kTmWeightStride + weight_index; }
 constexpr int kTensorMapBytes = 128;
-constexpr int kTcKSplit = 4;  // K slices of the wo / w2 tiles (their sum + residual + next RMSNorm is the phase's post-step)
-__host__ __device__ inline bool tc_has_poststep(const Phase& ph) { return ph.kind == PH_WO || ph.kind == PH_W2; }
+constexpr int kTcKSplit = 4;  // K slices of a prompt's wo / w2 tiles (their sum + residual + next RMSNorm is a step of its own)
 
 __host__ __device__ inline uint32_t pack_phase(const Phase& ph) {
     return (uint32_t)ph.kind | ((uint32_t)ph.fast << 4) | ((uint32_t)ph.layer << 8) | ((uint32_t)ph.depth_pos << 16);

@@ -38,4 +38,16 @@ inline bool make_tensor_map_2d(CUtensorMap* out, const void* base, uint64_t rows
                CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
+// A paged pool [page x layer][2][heads x positions][64] bf16: boxes of 16 rows of both halves (keys, values).
+inline bool make_tensor_map_kv(CUtensorMap* out, const void* base, uint64_t pages_layers, uint64_t head_rows) {
+    TensorMapEncodeTiledFn enc = tensor_map_encoder();
+    if (enc == nullptr) return false;
+    const cuuint64_t dims[4] = {64, (cuuint64_t)head_rows, 2, (cuuint64_t)pages_layers};
+    const cuuint64_t strides[3] = {128, (cuuint64_t)head_rows * 128, (cuuint64_t)head_rows * 256};
+    const cuuint32_t box[4] = {64u, 16u, 2u, 1u};
+    const cuuint32_t estr[4] = {1u, 1u, 1u, 1u};
+    return enc(out, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+               CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
 }  // namespace smol

@@ -392,6 +392,13 @@ class RQTransformer:
         return out
 
     @property
+    def _prompt_rows(self) -> int:
+        """Positions from which a prompt takes the tensor-core variant (0: never)."""
+        cfg = self.config
+        eligible = all(d % 64 == 0 for d in (cfg.dim, cfg.fast_dim, cfg.intermediate_size, cfg.fast_intermediate_size))
+        return self.get_option("tc_min_batch") if eligible else 0
+
+    @property
     def phase_count(self) -> int:
         return int(self.lib.smol_phase_count(self._h))
 
@@ -447,6 +454,14 @@ class RQTransformer:
         x = x.to(device=self.device, dtype=torch.int32).contiguous()
         S = x.shape[2]
         batch = cache.batch
+        if S > self._prompt_rows > 0:
+            # one pass: every position through the layers, the last one also through the LM head (the bits are those of a prefill
+            # of the first S - 1 positions, which is what the variant counts, and a step for the last)
+            if batch.host_len[0] + S > batch.capacity:
+                raise _capi.SmolError(_capi.SMOL_ERR_CAPACITY, "prompt (plus the positions already cached) exceeds the sequence's KV capacity")
+            _capi.check(self.lib.smol_prompt_logits(self._h, C.byref(batch.c), C.c_void_p(x.data_ptr()), S, self._stream()))
+            batch.host_len[0] += S
+            return self.debug_buffer("token_logits", 1).clone(), self.debug_buffer("x", 1).clone()
         if S > 1:
             self.prefill(batch, x, torch.tensor([S], dtype=torch.int32, device=self.device))
         else:

@@ -1,0 +1,127 @@
+"""The batched decode (csrc/rows_phases.cuh) and the prompt kernel (csrc/prompt_phases.cuh) at the sizes where they can go wrong:
+batches around the row groups, widths whose chains are long or cut unevenly, ragged heads, 16 depth positions, every group size of
+the attention, contexts around its splits, both page sizes.  The yardstick is the CUDA-core variant on the same inputs (itself held to
+the oracle): the two differ by the rounding of bf16 activations only, so their logits by a few bf16 ulps; bits that must not depend on
+the batch are compared as bits."""
+import pytest
+import torch
+
+from smoltts_b200.config import named_config
+from smoltts_b200.model import RQTransformer, make_prompt_cache
+from smoltts_b200.synth import byte_prompt, prompt_grid, state_dict_shapes
+
+pytestmark = pytest.mark.gpu
+
+CONFIGS = {
+    # w2 rows of 1600: 25 MMAs per chain, no K slices; 4 query heads per kv head
+    "long_chains": dict(base="smoltts_byte_tiny", dim=256, fast_dim=256, n_head=4, fast_n_head=4, n_local_heads=1, fast_n_local_heads=1, intermediate_size=1600, fast_intermediate_size=1600),
+    # two K slices in wo, heads that are not whole tiles, one kv head per query head
+    "ragged_heads": dict(base="smoltts_byte_tiny", dim=384, fast_dim=384, n_head=6, fast_n_head=6, n_local_heads=6, fast_n_local_heads=6, intermediate_size=640, fast_intermediate_size=640,
+                         vocab_size=2370, codebook_size=2050),
+    # positions 8 to 15 of the depth transformer
+    "deep": dict(base="smoltts_byte_tiny", num_codebooks=16),
+    "70m": dict(base="smoltts_byte_70m", n_layer=2, n_fast_layer=2),
+}
+
+
+def _model(name, max_batch, max_seq_len, page_size=32):
+    over = dict(CONFIGS[name])
+    cfg = named_config(over.pop("base"), **over)
+    g = torch.Generator(device="cuda").manual_seed(5)
+    w = {k: (1.0 + 0.05 * torch.randn(*s, generator=g, device="cuda") if k.endswith("norm.weight") else torch.randn(*s, generator=g, device="cuda") * cfg.initializer_range).to(torch.bfloat16)
+         for k, s in state_dict_shapes(cfg).items()}
+    model = RQTransformer(cfg, max_batch=max_batch, max_seq_len=max_seq_len, page_size=page_size)
+    model.load_state_dict(w)
+    return cfg, model
+
+
+def _frame(cfg, model, lens, rows, min_batch, frames=1):
+    """One forced frame of the sequences `rows` behind caches of the given lengths; (token logits, depth logits, cached pages)."""
+    g = torch.Generator(device="cuda").manual_seed(11)
+    n = len(lens)
+    codes = torch.randint(0, min(cfg.codebook_size, 1000), (2, n, cfg.n_rows), generator=g, device="cuda", dtype=torch.int32)
+    kv = torch.randn(n, max(lens), cfg.n_layer, 2, cfg.n_local_heads, 64, generator=g, device="cuda", dtype=torch.bfloat16)
+    batch = model.new_batch(len(rows), max_positions=model.max_seq_len, max_frames=frames)
+    try:
+        ps, pages = model.page_size, batch.block_table.long()
+        pad = torch.zeros(len(rows), pages.shape[1] * ps - max(lens), *kv.shape[2:], dtype=kv.dtype, device="cuda")
+        model.kv_view()[pages] = torch.cat([kv[rows], pad], 1).view(len(rows), -1, ps, *kv.shape[2:]).permute(0, 1, 3, 4, 5, 2, 6)
+        force = codes[1][rows].contiguous()
+        model.set_force(force)
+        batch.tokens.copy_(codes[0][rows])
+        batch.seq_len.copy_(torch.tensor([lens[r] for r in rows], dtype=torch.int32, device="cuda"))
+        batch.host_len = [lens[r] for r in rows]
+        model.set_option("tc_min_batch", min_batch)
+        model.set_option("ll_max_batch", 0)
+        model.decode_frames(batch, model.sampling(ignore_stop=True), frames)
+        torch.cuda.synchronize()
+        return model.debug_buffer("token_logits", len(rows)).clone(), model.debug_buffer("depth_logits", len(rows)).clone(), model.kv_view()[pages].clone()
+    finally:
+        model.set_force(None)
+        model.set_option("tc_min_batch", 9)
+        model.set_option("ll_max_batch", 8)
+        batch.release()
+
+
+def _close(a, b, what):
+    scale = b.float().pow(2).mean().sqrt()
+    d = (a.float() - b.float())
+    # two bf16 executions of a few layers: each rounding is 2^-9 of its value (rms 0.29 ulps), some thirty of them in a row
+    assert torch.isfinite(a).all() and d.pow(2).mean().sqrt() < 0.03 * scale and d.abs().max() < 0.25 * scale, (what, (d.pow(2).mean().sqrt() / scale).item(), (d.abs().max() / scale).item())
+
+
+@pytest.mark.parametrize("name,page_size", [("long_chains", 32), ("ragged_heads", 16), ("deep", 32), ("70m", 16)])
+@pytest.mark.parametrize("batch", [9, 17, 33, 65])
+def test_batched_decode_at_the_edges_of_its_row_groups(name, page_size, batch):
+    cfg, model = _model(name, 65, 200, page_size)
+    lens = [1 + (37 * b) % 170 for b in range(batch)]
+    every = list(range(batch))
+    tl, dl, kv = _frame(cfg, model, lens, every, 9)
+    assert model.get_option("tc_ready") == 1
+    tl0, dl0, kv0 = _frame(cfg, model, lens, every, 0)
+    _close(tl, tl0, "token logits")
+    _close(dl, dl0, "depth logits")
+    _close(kv, kv0, "keys and values")
+    some = every[-9:]                       # the smallest batch: the same bits
+    ts, ds, ks = _frame(cfg, model, lens, some, 9)
+    assert torch.equal(ts, tl[some]) and torch.equal(ds, dl[some]) and torch.equal(ks.view(torch.int16), kv[some].view(torch.int16))
+
+
+@pytest.mark.parametrize("name,longest,batch", [("70m", 127, 10), ("70m", 128, 10), ("70m", 129, 40), ("long_chains", 1030, 40), ("70m", 2300, 150), ("deep", 2300, 300)])
+def test_batch_attention_around_its_splits(name, longest, batch):
+    """Contexts below, at and above a split; more splits than a unit has warps (states through global memory); many units."""
+    cfg, model = _model(name, batch, longest + 4)
+    lens = [max(1, longest - (b * 131) % longest) for b in range(batch)]
+    tl, dl, _ = _frame(cfg, model, lens, list(range(batch)), 9)
+    tl0, dl0, _ = _frame(cfg, model, lens, list(range(batch)), 0)
+    _close(tl, tl0, "token logits")
+    _close(dl, dl0, "depth logits")
+    ts, ds, _ = _frame(cfg, model, lens, list(range(9)), 9)
+    assert torch.equal(ts, tl[:9]) and torch.equal(ds, dl[:9])
+
+
+@pytest.mark.parametrize("name,page_size", [("long_chains", 32), ("ragged_heads", 16), ("70m", 32)])
+@pytest.mark.parametrize("n,tile", [(9, 0), (10, 0), (16, 0), (65, 0), (130, 0), (130, 50), (301, 0)])
+def test_prompt_logits_equal_those_of_its_last_position_alone(name, page_size, n, tile):
+    """forward_generate of a prompt against the prefill of all but its last position and that position by itself: the same bits in
+    logits, hidden state and cache."""
+    cfg, model = _model(name, 1, 320, page_size)
+    prompt = prompt_grid(byte_prompt(max(1, n - 12), seed=n)[-n:], cfg)[None].to(device="cuda", dtype=torch.int32)
+    n = prompt.shape[2]
+    model.set_option("prefill_tile", tile)
+    cache = make_prompt_cache(model)
+    logits, hidden = model.forward_generate(prompt, cache)
+    pages = torch.tensor(cache.batch.pages, device="cuda")
+    assert int(cache.batch.seq_len[0]) == n and cache.batch.host_len == [n] and torch.equal(cache.batch.tokens[0], prompt[0, :, -1])
+    kv = model.kv_view()[pages].clone()
+    cache.batch.release()
+    model.kv_view().zero_()
+    cache = make_prompt_cache(model)
+    model.prefill(cache.batch, prompt, torch.tensor([n], dtype=torch.int32, device="cuda"))
+    model.slow_step(cache.batch, advance=True)
+    torch.cuda.synchronize()
+    assert torch.equal(logits, model.debug_buffer("token_logits", 1)) and torch.equal(hidden.view(torch.int16), model.debug_buffer("x", 1).view(torch.int16))
+    kv0 = model.kv_view()[torch.tensor(cache.batch.pages, device="cuda")]
+    flat = lambda t: t.permute(1, 2, 3, 0, 4, 5).flatten(3, 4)[..., :n, :].contiguous().view(torch.int16)  # noqa: E731
+    assert torch.equal(flat(kv), flat(kv0))
+    cache.batch.release()

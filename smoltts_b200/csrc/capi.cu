@@ -19,7 +19,7 @@ size_t decode_xs_bytes(const DevModel& M, int bt);
 size_t decode_stage_bytes(const DevModel& M, int n_ctas, int bt);
 void rows_plan(const DevModel& M, int rows, int n_ctas, RowsPlan (*plan)[6]);
 cudaError_t prompt_configure(int* per_sm);
-cudaError_t prompt_launch(const DevModel& M, const CallArgs& A, int n_ctas, cudaStream_t stream);
+cudaError_t prompt_launch(const DevModel& M, const CallArgs& A, bool wide, int n_ctas, cudaStream_t stream);
 int decode_batch_tile(int batch);
 cudaError_t decode_configure(int bt, size_t smem);
 cudaError_t decode_max_ctas(int bt, size_t smem, int* per_sm);
@@ -71,7 +71,7 @@ struct SmolModel {
                                // barrier kernel / its tcgen05 variant (measured at bs=8: 1.5 ms per frame step against 2.3 ms)
     smol::ll2::SmemPlan ll2_sp;
     size_t ll2_smem = 0;
-    bool tmaps_ready = false;  // tensor maps of the prompt kernel (rebuilt after a weight / workspace bind)
+    bool tmaps_ready = false;  // tensor maps of the 128-row tiles (rebuilt after a weight / workspace bind)
     bool prompt_ready = false; // its function attributes
     bool packed_ready = false; // tensor-core GEMV layout of the bound weights (rebuilt after a weight / workspace bind)
     int64_t launches = 0;
@@ -168,10 +168,10 @@ static WsLayout ws_layout(const SmolConfig& c, int depth) {
     L.q = take(B * imax(c.n_head, c.fast_n_head) * 64 * 2);
     L.attn = take(B * dmax * 2);
     L.act = take(B * imax(c.intermediate_size, c.fast_intermediate_size) * 2);
-    L.xn = take(B * c.dim * 2);
+    L.xn = take(B * dmax * 2);
     L.silu_lut = take(65536 * 2);
     L.tmaps = take((size_t)smol::kTmTotal * smol::kTensorMapBytes);
-    L.kpart = take((size_t)smol::kTcKSplit * B * c.dim * 4);
+    L.kpart = take((size_t)smol::kTcKSplit * B * dmax * 4);
     L.fkv = take(B * c.n_fast_layer * 2 * depth * c.fast_n_local_heads * 64 * 2);
     L.token_logits = take(B * c.vocab_size * 4);
     L.depth_logits = take(B * depth * c.codebook_size * 4);
@@ -379,8 +379,7 @@ static int ensure_configured(SmolModel* m) {
     return SMOL_OK;
 }
 
-
-// TMA tensor maps of the prompt kernel: encoded on the host and copied into the workspace once per bind (setup-time,
+// TMA tensor maps of the 128-row tiles: encoded on the host and copied into the workspace once per bind (setup-time,
 // synchronous; compute calls never come here again).
 static int ensure_tmaps(SmolModel* m) {
     if (m->tmaps_ready) return SMOL_OK;
@@ -400,18 +399,25 @@ static int ensure_tmaps(SmolModel* m) {
         for (int box = 16; box <= 16 * smol::kTmWeightBoxes; box += 16)
             ok = ok && smol::make_tensor_map_2d(&maps[smol::tm_weight_slot(index, box)], p, n, K, K, (uint32_t)box);
     };
-    act(smol::TM_XN, d.xn, c.dim);
-    act(smol::TM_ATTN, d.attn, c.dim);
-    act(smol::TM_ACT, d.act, c.intermediate_size);
-    for (int l = 0; l < c.n_layer; ++l) {
-        const smol::DevLayer& L = d.layers[l];
-        wgt(smol::tm_weight_index(l, 0), L.wqkv, (uint64_t)(c.n_head + 2 * c.n_local_heads) * 64, c.dim);
-        wgt(smol::tm_weight_index(l, 1), L.wo, c.dim, c.dim);
-        wgt(smol::tm_weight_index(l, 2), L.w1, c.intermediate_size, c.dim);
-        wgt(smol::tm_weight_index(l, 3), L.w3, c.intermediate_size, c.dim);
-        wgt(smol::tm_weight_index(l, 4), L.w2, c.dim, c.intermediate_size);
+    for (int f = 0; f < 2; ++f) {
+        const int nl = f ? c.n_fast_layer : c.n_layer, D = f ? c.fast_dim : c.dim, F = f ? c.fast_intermediate_size : c.intermediate_size;
+        const int qkv = ((f ? c.fast_n_head : c.n_head) + 2 * (f ? c.fast_n_local_heads : c.n_local_heads)) * 64;
+        act((f ? smol::TM_FAST : 0) + smol::TM_XN, d.xn, D);
+        act((f ? smol::TM_FAST : 0) + smol::TM_ATTN, d.attn, D);
+        act((f ? smol::TM_FAST : 0) + smol::TM_ACT, d.act, F);
+        for (int l = 0; l < nl; ++l) {
+            const smol::DevLayer& L = f ? d.fast_layers[l] : d.layers[l];
+            const int at = f ? c.n_layer + l : l;
+            wgt(smol::tm_weight_index(at, 0), L.wqkv, qkv, D);
+            wgt(smol::tm_weight_index(at, 1), L.wo, D, D);
+            wgt(smol::tm_weight_index(at, 2), L.w1, F, D);
+            wgt(smol::tm_weight_index(at, 3), L.w3, F, D);
+            wgt(smol::tm_weight_index(at, 4), L.w2, D, F);
+        }
     }
-    if (!ok) return fail(SMOL_ERR_CUDA, "cuTensorMapEncodeTiled failed for the prompt kernel's operands");
+    wgt(0, d.head, c.vocab_size, c.dim);
+    wgt(1, d.fast_output, (uint64_t)c.codebook_size * (c.depthwise_output ? d.depth : 1), c.fast_dim);
+    if (!ok) return fail(SMOL_ERR_CUDA, "cuTensorMapEncodeTiled failed for the tiles' operands");
     CU(cudaMemcpy(const_cast<unsigned char*>(d.tmaps), maps.data(), (size_t)smol::kTmTotal * smol::kTensorMapBytes, cudaMemcpyHostToDevice));
     m->tmaps_ready = true;
     return SMOL_OK;
@@ -446,16 +452,17 @@ static int ensure_packed(SmolModel* m) {
             const int qkv = ((f ? c.fast_n_head : c.n_head) + 2 * (f ? c.fast_n_local_heads : c.n_local_heads)) * 64;
             for (int l = 0; l < nl; ++l) {
                 smol::DevLayer& L = f ? d.fast_layers[l] : d.layers[l];
-                (form ? L.pr_wqkv : L.pk_wqkv) = put(L.wqkv, nullptr, qkv, D);
-                (form ? L.pr_wo : L.pk_wo) = put(L.wo, nullptr, D, D);
-                (form ? L.pr_w13 : L.pk_w13) = put(L.w1, L.w3, F, D);
-                (form ? L.pr_w2 : L.pk_w2) = put(L.w2, nullptr, D, F);
+                smol::RowsLayer& W = f ? d.rows_fast_layers[l] : d.rows_layers[l];
+                (form ? W.wqkv : L.pk_wqkv) = put(L.wqkv, nullptr, qkv, D);
+                (form ? W.wo : L.pk_wo) = put(L.wo, nullptr, D, D);
+                (form ? W.w13 : L.pk_w13) = put(L.w1, L.w3, F, D);
+                (form ? W.w2 : L.pk_w2) = put(L.w2, nullptr, D, F);
             }
         }
-        (form ? d.pr_head : d.pk_head) = put(d.head, nullptr, c.vocab_size, c.dim);
+        (form ? d.rows_head : d.pk_head) = put(d.head, nullptr, c.vocab_size, c.dim);
         for (int i = 0; i < (c.depthwise_output ? d.depth : 1); ++i) {   // one matrix per depth position, whole tiles each
             const uint16_t* q = put(d.fast_output + (size_t)i * c.codebook_size * c.fast_dim, nullptr, c.codebook_size, c.fast_dim);
-            if (i == 0) (form ? d.pr_fast_output : d.pk_fast_output) = q;
+            if (i == 0) (form ? d.rows_fast_output : d.pk_fast_output) = q;
         }
     }
     if (!ok) return fail(SMOL_ERR_CUDA, "packing the weights for the tensor-core kernels failed");
@@ -535,6 +542,28 @@ static bool use_tc(const SmolModel* m, int rows) {
     return m->tc_min_batch > 0 && rows >= m->tc_min_batch && tc_eligible(m->cfg);
 }
 
+// Rows of a decode batch up to which groups of 32 rows are faster than 128-row tiles (150m, us per frame): 128 rows 1986, 136
+// 2198 | 160 rows 2640, 256: 2699 on tiles (256 rows in groups 3380).
+constexpr int kWideRows = 144;
+
+// Tiles of 128 rows: a prompt (in every mode) or frames of a wide batch, one cooperative launch.
+static int enqueue_tiles(SmolModel* m, CallArgs A, bool wide, cudaStream_t stream) {
+    int rc = ensure_tmaps(m);
+    if (rc || (rc = ensure_kv_map(m))) return rc;
+    if (!m->prompt_ready) {
+        int per_sm = 0;
+        CU(smol::prompt_configure(&per_sm));
+        if (per_sm < 1) return fail(SMOL_ERR_UNSUPPORTED, "prompt kernel does not fit on an SM");
+        m->prompt_ready = true;
+    }
+    A.cooperative = 1;
+    A.tc_split = m->tc_attn_split;
+    std::memcpy(A.kv_map, m->kv_map, sizeof(A.kv_map));
+    CU(smol::prompt_launch(m->dm, A, wide, m->n_ctas, stream));
+    m->launches += 1;
+    return SMOL_OK;
+}
+
 static int enqueue(SmolModel* m, CallArgs A, cudaStream_t stream, bool whole_iters = false) {
     const int bt = use_tc(m, A.batch) ? 0 : smol::decode_batch_tile(A.batch);
     int rc;
@@ -555,7 +584,10 @@ static int enqueue(SmolModel* m, CallArgs A, cudaStream_t stream, bool whole_ite
     }
     rc = ensure_tile(m, bt);
     if (rc) return rc;
-    A.repeat = m->repeat;
+    if (bt == 0 && m->mode != 1 && A.mode == 0 && A.batch > kWideRows && A.phase_begin < A.phase_end) {
+        const smol::Phase first = smol::unpack_phase(m->dm.prog[A.phase_begin]);   // (launches begin where a transformer does)
+        if (first.kind == smol::PH_QKV && first.layer == 0) return enqueue_tiles(m, A, true, stream);
+    }
     if (bt == 0) {
         smol::rows_plan(m->dm, A.batch, m->n_ctas, A.rows_plan);
         std::memcpy(A.kv_map, m->kv_map, sizeof(A.kv_map));
@@ -605,24 +637,6 @@ static int enqueue(SmolModel* m, CallArgs A, cudaStream_t stream, bool whole_ite
     return SMOL_OK;
 }
 
-// A prompt on the tensor cores: one cooperative launch over all its tiles, in every mode.
-static int enqueue_prompt(SmolModel* m, CallArgs A, cudaStream_t stream) {
-    int rc = ensure_tmaps(m);
-    if (rc || (rc = ensure_kv_map(m))) return rc;
-    if (!m->prompt_ready) {
-        int per_sm = 0;
-        CU(smol::prompt_configure(&per_sm));
-        if (per_sm < 1) return fail(SMOL_ERR_UNSUPPORTED, "prompt kernel does not fit on an SM");
-        m->prompt_ready = true;
-    }
-    A.cooperative = 1;
-    A.tc_split = m->tc_attn_split;
-    std::memcpy(A.kv_map, m->kv_map, sizeof(A.kv_map));
-    CU(smol::prompt_launch(m->dm, A, m->n_ctas, stream));
-    m->launches += 1;
-    return SMOL_OK;
-}
-
 static CallArgs base_args(const SmolBatch* b, int batch, const SmolSampling* s) {
     CallArgs A;
     std::memset(&A, 0, sizeof(A));
@@ -666,7 +680,7 @@ int smol_prefill(SmolModel* m, const SmolBatch* b, int32_t batch, const int32_t*
     A.prompt = d_prompt;
     A.prompt_len = d_prompt_len;
     A.s_max = s_max;
-    if (use_tc(m, A.batch)) return enqueue_prompt(m, A, (cudaStream_t)stream);
+    if (use_tc(m, A.batch)) return enqueue_tiles(m, A, false, (cudaStream_t)stream);
     return enqueue(m, A, (cudaStream_t)stream, T == 1);  // tiled prefill runs on the barrier kernel
 }
 
@@ -689,7 +703,7 @@ int smol_prompt_logits(SmolModel* m, const SmolBatch* b, const int32_t* d_prompt
     A.whole_prompt = n;
     A.n_iter = (n + T - 1) / T;
     A.head_row = n - 1 - (A.n_iter - 1) * T;
-    return enqueue_prompt(m, A, (cudaStream_t)stream);
+    return enqueue_tiles(m, A, false, (cudaStream_t)stream);
 }
 
 int smol_slow_step(SmolModel* m, const SmolBatch* b, int32_t batch, int32_t advance, void* stream) {

@@ -125,9 +125,8 @@ __device__ __forceinline__ void bulk_g2s(void* dst, const void* src, uint32_t by
 }
 __device__ __forceinline__ void fence_proxy_async() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 
-// Generic-proxy writes (st.global of activations) <-> async-proxy reads (bulk copies of the same rows by other CTAs): fenced
-// on both sides of the grid barrier in the tensor-core variant.
-__device__ __forceinline__ void fence_proxy_async_all() { asm volatile("fence.proxy.async;" ::: "memory"); }
+// Generic-proxy writes (st.global of activations) <-> async-proxy reads (bulk copies of the same rows by other CTAs): fenced by the
+// threads that issue the copies, behind the grid barrier (the tensor-core variant).
 __device__ __forceinline__ void fence_proxy_async_global() { asm volatile("fence.proxy.async.global;" ::: "memory"); }
 
 struct Ctx {
@@ -1180,14 +1179,14 @@ cudaError_t decode_max_ctas(int bt, size_t smem, int* per_sm) {
     return cudaOccupancyMaxActiveBlocksPerMultiprocessor(per_sm, decode_fn(bt), kThreads, smem);
 }
 
-size_t prompt_smem() { return (size_t)kPrSmem; }
 cudaError_t prompt_configure(int* per_sm) {
-    cudaError_t e = cudaFuncSetAttribute(smol_prompt_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kPrSmem);
+    cudaError_t e = cudaFuncSetAttribute(smol_wide_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kPrSmem);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(smol_prompt_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kPrSmem);
     return e != cudaSuccess ? e : cudaOccupancyMaxActiveBlocksPerMultiprocessor(per_sm, smol_prompt_kernel, kThreads, kPrSmem);
 }
-cudaError_t prompt_launch(const DevModel& M, const CallArgs& A, int n_ctas, cudaStream_t stream) {
+cudaError_t prompt_launch(const DevModel& M, const CallArgs& A, bool wide, int n_ctas, cudaStream_t stream) {
     void* args[2] = {(void*)&M, (void*)&A};
-    return cudaLaunchCooperativeKernel((const void*)smol_prompt_kernel, dim3(n_ctas), dim3(kThreads), args, kPrSmem, stream);
+    return cudaLaunchCooperativeKernel(wide ? (const void*)smol_wide_kernel : (const void*)smol_prompt_kernel, dim3(n_ctas), dim3(kThreads), args, kPrSmem, stream);
 }
 
 cudaError_t decode_launch(const DevModel& M, const CallArgs& A, int bt, int n_ctas, size_t smem, int xs_bytes,

@@ -61,11 +61,12 @@ struct DevLayer {
     const uint16_t* pk_wo;
     const uint16_t* pk_w13;
     const uint16_t* pk_w2;
-    // the same as plain mma.m16n8k16 A fragments (rows_phases.cuh; smol_rows_pack_kernel)
-    const uint16_t* pr_wqkv;
-    const uint16_t* pr_wo;
-    const uint16_t* pr_w13;
-    const uint16_t* pr_w2;
+};
+
+// The same matrices as plain mma.m16n8k16 A fragments (rows_phases.cuh; smol_rows_pack_kernel).  (Not in DevLayer: the data-flow
+// kernel reads that from the constant bank in every phase.)
+struct RowsLayer {
+    const uint16_t *wqkv, *wo, *w13, *w2;
 };
 
 struct DevModel {
@@ -103,9 +104,9 @@ struct DevModel {
     uint16_t* q;        // rotated queries                 [B][max(n_head,fn_head)*64]
     uint16_t* attn;     // attention output                [B][max(dim,fdim)]
     uint16_t* act;      // silu(w1 x) * w3 x               [B][max(inter,finter)]
-    uint16_t* xn;       // prompts: RMSNorm output feeding the next weight phase  [rows][dim]
-    const unsigned char* tmaps;  // prompts: TMA tensor maps (128 B each, TensorMapSlot), in the workspace
-    float* kpart;       // prompts: partial sums of the K slices of the wo / w2 tiles  [kTcKSplit][ws_rows][dim] fp32
+    uint16_t* xn;       // tiles of 128 rows: RMSNorm output feeding the next weight phase  [rows][dim of the transformer]
+    const unsigned char* tmaps;  // ... TMA tensor maps (128 B each, TensorMapSlot), in the workspace
+    float* kpart;       // ... partial sums of the K slices of wo / w2  [kTcKSplit][ws_rows][dim of the transformer] fp32
     int ws_rows;        // rows of every workspace buffer
     const uint16_t* silu_lut;  // bf16 silu of every bf16 input [65536] (exact expression, filled at bind time)
     uint16_t* fkv;      // fast KV  [B][n_flayer][2][depth][fn_kv*64]
@@ -130,14 +131,15 @@ struct DevModel {
     uint32_t ll_off[kMaxProg];
     uint16_t ll_len[kMaxProg];
 
-    const uint16_t* pr_head;         // heads in the fragments of the batched decode
-    const uint16_t* pr_fast_output;
     const uint16_t* pk_head;         // packed LM head
     const uint16_t* pk_fast_output;  // packed depth heads (row groups in checkpoint order)
     unsigned long long* ll2_score;   // attention scores {fp32 bits, epoch} [teams][2][n_head][ll2_score_len] words
     unsigned long long* ll2_tok;     // sampled ids [teams][n_rows][kLLMaxCtas] words
     unsigned long long* ll2_cand;    // greedy candidates [teams][n_rows][kLLRep][kLLMaxCtas] words
     int ll2_score_len;
+
+    RowsLayer rows_layers[SMOL_MAX_LAYERS], rows_fast_layers[SMOL_MAX_FAST_LAYERS];   // batched decode: fragments
+    const uint16_t *rows_head, *rows_fast_output;
 };
 
 // Words (8 bytes, two bf16 + epoch) one sequence publishes in a phase; multiples of 16 words (128 B).
@@ -245,15 +247,15 @@ __host__ __device__ inline Phase decode_phase(int p, int n_layer, int n_flayer) 
 // Tensor-core variant: the phase that starts with a grid-wide pre-step (the token embedding of the slow transformer's input).
 __host__ __device__ inline bool tc_has_prestep(const Phase& ph) { return ph.kind == PH_QKV && !ph.fast && ph.layer == 0; }
 
-// Prompts (prompt_phases.cuh): slots of the tensor-map table (DevModel.tmaps).  Activations: boxes of 128 rows, of 64 and of 32;
-// weights of the slow transformer: one map per matrix and box height 16 * (v + 1) rows, v = 0..5, so that a tile's weight rows
-// are ONE copy per stage.
-enum TensorMapSlot { TM_XN = 0, TM_ATTN, TM_ACT, TM_ACT_MAPS = 3, TM_WEIGHTS = 9 };
+// Tiles of 128 rows (prompt_phases.cuh): slots of the tensor-map table (DevModel.tmaps).  Activations of the slow and (+ TM_FAST) the
+// depth transformer: boxes of 128 rows, of 64 and of 32; weights: one map per matrix and box height 16 * (v + 1) rows, v = 0..5, so
+// that a tile's weight rows are ONE copy per stage.
+enum TensorMapSlot { TM_XN = 0, TM_ATTN, TM_ACT, TM_FAST = 3, TM_ACT_MAPS = 6, TM_WEIGHTS = 18 };
 constexpr int kTmWeightBoxes = 6;
-constexpr int kTmWeightStride = 5 * SMOL_MAX_LAYERS;       // weight matrices a model can have
+constexpr int kTmWeightStride = 2 + 5 * (SMOL_MAX_LAYERS + SMOL_MAX_FAST_LAYERS);       // weight matrices a model can have
 constexpr int kTmTotal = TM_WEIGHTS + kTmWeightBoxes * kTmWeightStride;
-// weight index: 5 per layer (wqkv, wo, w1, w3, w2)
-__host__ __device__ inline int tm_weight_index(int layer, int which) { return layer * 5 + which; }
+// weight index: 0 LM head, 1 depth heads, then 5 per layer (wqkv, wo, w1, w3, w2); the depth transformer's layers follow the slow ones
+__host__ __device__ inline int tm_weight_index(int layer, int which) { return 2 + layer * 5 + which; }
 __host__ __device__ inline int tm_weight_slot(int weight_index, int box_rows) { return TM_WEIGHTS + (box_rows / 16 - 1) * kTmWeightStride + weight_index; }
 constexpr int kTensorMapBytes = 128;
 constexpr int kTcKSplit = 4;  // K slices of a prompt's wo / w2 tiles (their sum + residual + next RMSNorm is a step of its own)

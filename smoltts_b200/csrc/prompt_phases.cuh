@@ -1,5 +1,5 @@
-// Prompts: the slow transformer over hundreds of positions at once (rows = sequences x prompt positions), one persistent kernel
-// with the same phases and grid barrier as decoding.  Included by decode_kernel.cu after rows_phases.cuh (whose batch
+// Hundreds of rows at once: prompts (the slow transformer over sequences x positions) and the decode of wide batches, each one
+// persistent kernel with the same phases and grid barrier as decode_kernel.cu.  Included by decode_kernel.cu after rows_phases.cuh (whose batch
 // attention, split barrier and row bookkeeping it uses).
 //
 // A weight phase Y[rows][n_out] = X[rows][K] * W[n_out][K]^T is cut into units (128-row tile, block of `blk` weight rows; wo and
@@ -11,7 +11,7 @@
 // below its last place with every MMA, so chains are kept at 12.
 //
 // What needs whole rows happens in steps between: the sum of the K slices, the residual add and the next RMSNorm (five rows
-// per CTA and pass).  Measured (150m, device time of prompt -> logits, us): 40 positions 771, 212: 842, 800: 1608; one thread that issued
+// per CTA and pass).  Measured (150m, device time of prompt -> logits, us): 40 positions 743, 212: 835, 800: 1582; one thread that issued
 // loads and MMAs, no weights before the barrier, and a slow step behind it for the last position took 996, 1285 and 2090.
 #pragma once
 
@@ -262,13 +262,16 @@ __device__ __noinline__ void row_wide(const DevModel& M, int row, int layer, int
     }
 }
 
-// One weight phase; on return the CTA has finished its units, the barrier behind it is the caller's.
+// One weight phase; on return the CTA has finished its units, the barrier behind it is the caller's.  kWide: of a decode frame (the
+// depth transformer's phases and the heads exist, no row stands for a last position), else of a prompt.
+template <bool kWide>
 __device__ __noinline__ void prompt_gemm(const DevModel& M, const CallArgs& A, const Ctx& c, const Phase& ph, RowsSync& sy, uint32_t& chunk, uint32_t& tile, const int last_row) {
     const int kind = ph.kind;
-    const int D = M.dim, F = M.inter, Hq = M.n_head, Hkv = M.n_kv;
+    const bool fast = kWide && ph.fast != 0;
+    const int D = fast ? M.fdim : M.dim, F = fast ? M.finter : M.inter, Hq = fast ? M.fn_head : M.n_head, Hkv = fast ? M.fn_kv : M.n_kv;
     const int q_rows = Hq * kHeadDim, k_end = (Hq + Hkv) * kHeadDim;
     const int K = kind == PH_W2 ? F : D;
-    const int n_out = kind == PH_QKV ? (Hq + 2 * Hkv) * kHeadDim : kind == PH_W13 ? F : D;
+    const int n_out = kind == PH_QKV ? (Hq + 2 * Hkv) * kHeadDim : kind == PH_W13 ? F : kWide && kind == PH_HEAD ? (fast ? M.codebook_size : M.vocab) : D;
     const int rows = A.batch;
     unsigned char* ring = reinterpret_cast<unsigned char*>(c.xs);
     const int warp = c.warp, lane = c.lane;
@@ -276,9 +279,11 @@ __device__ __noinline__ void prompt_gemm(const DevModel& M, const CallArgs& A, c
     const unsigned char* tm = M.tmaps;
     const int box_idx = rows <= 32 ? 2 : rows <= 64 ? 1 : 0;   // activation box of 32 / 64 / 128 rows: the rest of a stage holds stale rows whose accumulator lanes nobody reads
     const int a_bytes = (umma::kM >> box_idx) * umma::kBK * 2;
-    const void* tm_a = tm + (size_t)kTensorMapBytes * (box_idx * TM_ACT_MAPS + (kind == PH_WO ? TM_ATTN : kind == PH_W2 ? TM_ACT : TM_XN));
+    const void* tm_a = tm + (size_t)kTensorMapBytes * (box_idx * TM_ACT_MAPS + (fast ? TM_FAST : 0) + (kind == PH_WO ? TM_ATTN : kind == PH_W2 ? TM_ACT : TM_XN));
     const int which = kind == PH_QKV ? 0 : kind == PH_WO ? 1 : kind == PH_W13 ? 2 : 4;
-    const int w0 = tm_weight_index(ph.layer, which), w1 = tm_weight_index(ph.layer, 3);
+    const int layer = fast ? M.n_layer + ph.layer : ph.layer;
+    const int w0 = kWide && kind == PH_HEAD ? (fast ? 1 : 0) : tm_weight_index(layer, which), w1 = tm_weight_index(layer, 3);
+    const int w_row = kWide && kind == PH_HEAD && fast && M.depthwise_output ? ph.depth_pos * n_out : 0;   // a depth position's own head
     const bool paired = kind == PH_W13;
     const int n_split = kind != PH_WO && kind != PH_W2 ? 1 : prompt_slices(K);
     const int nk = K / n_split / umma::kBK;
@@ -297,7 +302,7 @@ __device__ __noinline__ void prompt_gemm(const DevModel& M, const CallArgs& A, c
     auto load_w = [&](uint32_t g, int n0, int k0) {
         const uint32_t s = g % kPrStages, b = umma::s2u(ring + (size_t)s * umma::kStageBytes) + umma::kStageA;
         umma::bar_expect_tx(&g_pr.full[s], (uint32_t)(n_blk * umma::kBK * 2));
-        umma::tma_load_2d(b, tm + (size_t)kTensorMapBytes * tm_weight_slot(w0, blk), k0, n0, &g_pr.full[s]);
+        umma::tma_load_2d(b, tm + (size_t)kTensorMapBytes * tm_weight_slot(w0, blk), k0, w_row + n0, &g_pr.full[s]);
         if (paired) umma::tma_load_2d(b + blk * umma::kBK * 2, tm + (size_t)kTensorMapBytes * tm_weight_slot(w1, blk), k0, n0, &g_pr.full[s]);
     };
     // the first stages' weights do not wait for the phase before (the ring is empty: that phase's accumulators have been read)
@@ -370,7 +375,7 @@ __device__ __noinline__ void prompt_gemm(const DevModel& M, const CallArgs& A, c
             const int bg = m0 + quad * 32 + lane;
             const bool live = bg < rows && bg != last_row;
             int pos = 0, page = -1;
-            if (kind == PH_QKV && live) {      // cache slot of the row (-1: nothing is appended)
+            if (kind == PH_QKV && live && !fast) {      // cache slot of the row (-1: nothing is appended)
                 const int bs = row_seq(A, bg);
                 pos = ldcg_i32(A.b.seq_len + bs) + row_off(A, bg);
                 if (seq_active(M, A, c, bg) && pos < A.b.max_pages * M.page_size) page = ldcg_i32(A.b.block_table + (size_t)bs * A.b.max_pages + pos / M.page_size);
@@ -395,6 +400,19 @@ __device__ __noinline__ void prompt_gemm(const DevModel& M, const CallArgs& A, c
                     *reinterpret_cast<uint4*>(M.act + (size_t)bg * F + u0) = pack8(o);
                     continue;
                 }
+                if (kWide && kind == PH_HEAD) {
+                    float* out = (fast ? M.depth_logits + ((size_t)bg * M.depth + ph.depth_pos) * n_out : M.token_logits + (size_t)bg * n_out) + u0;
+#pragma unroll
+                    for (int e = 0; e < 8; ++e) acc[e] = bf16_round(acc[e]);
+                    if ((n_out & 7) == 0) {
+                        *reinterpret_cast<float4*>(out) = make_float4(acc[0], acc[1], acc[2], acc[3]);
+                        *reinterpret_cast<float4*>(out + 4) = make_float4(acc[4], acc[5], acc[6], acc[7]);
+                    } else {
+#pragma unroll
+                        for (int e = 0; e < 8; ++e) { if (u0 + e < n_out) out[e] = acc[e]; }
+                    }
+                    continue;
+                }
                 if (kind != PH_QKV) {
                     float* pp = M.kpart + ((size_t)ks * M.ws_rows + bg) * D + u0;
                     *reinterpret_cast<float4*>(pp) = make_float4(acc[0], acc[1], acc[2], acc[3]);
@@ -405,7 +423,7 @@ __device__ __noinline__ void prompt_gemm(const DevModel& M, const CallArgs& A, c
 #pragma unroll
                 for (int e = 0; e < 8; ++e) v[e] = bf16_round(acc[e]);
                 if (u0 < k_end) {  // q and k rows: interleaved-pair RoPE with the bf16 table (P:616-640); never past the table (host checks bound pos)
-                    const uint4 cs = __ldg(reinterpret_cast<const uint4*>(M.rope + (size_t)min(pos, M.max_seq_len - 1) * kHeadDim + (u0 & (kHeadDim - 1))));
+                    const uint4 cs = __ldg(reinterpret_cast<const uint4*>((fast ? M.fast_rope + (size_t)ph.depth_pos * kHeadDim : M.rope + (size_t)min(pos, M.max_seq_len - 1) * kHeadDim) + (u0 & (kHeadDim - 1))));
                     const uint32_t cw[4] = {cs.x, cs.y, cs.z, cs.w};
 #pragma unroll
                     for (int e = 0; e < 8; e += 2) {
@@ -416,8 +434,12 @@ __device__ __noinline__ void prompt_gemm(const DevModel& M, const CallArgs& A, c
                     }
                 }
                 if (u0 < q_rows) { *reinterpret_cast<uint4*>(M.q + (size_t)bg * q_rows + u0) = pack8(v); continue; }
-                if (page < 0) continue;
                 const int is_v = u0 >= k_end ? 1 : 0, n1 = u0 - (is_v ? k_end : q_rows), ps = M.page_size;
+                if (fast) {
+                    *reinterpret_cast<uint4*>(M.fkv + (((size_t)(bg * M.n_flayer + ph.layer) * 2 + is_v) * M.depth + ph.depth_pos) * (Hkv * kHeadDim) + n1) = pack8(v);
+                    continue;
+                }
+                if (page < 0) continue;
                 *reinterpret_cast<uint4*>(M.kv_pool + ((((size_t)page * M.n_layer + ph.layer) * 2 + is_v) * Hkv + n1 / kHeadDim) * ((size_t)ps * kHeadDim)
                                           + (size_t)(pos % ps) * kHeadDim + (n1 & (kHeadDim - 1))) = pack8(v);
             }
@@ -453,15 +475,10 @@ __device__ __forceinline__ void prompt_attn(const DevModel& M, const CallArgs& A
     }
 }
 
-__global__ void __launch_bounds__(kThreads, 1)
-smol_prompt_kernel(const __grid_constant__ DevModel Mp, const __grid_constant__ CallArgs Ap) {
-    extern __shared__ __align__(1024) unsigned char smem_dyn[];
+// What the kernels begin with: the arguments' copies, barriers, tensor memory.
+__device__ __forceinline__ void prompt_setup(const DevModel& Mp, const CallArgs& Ap, unsigned char* smem_dyn, Ctx& c, RowsSync& sy) {
     for (int i = threadIdx.x; i < (int)(sizeof(DevModel) / 4); i += kThreads) reinterpret_cast<uint32_t*>(smem_dyn + kPrData)[i] = reinterpret_cast<const uint32_t*>(&Mp)[i];
     for (int i = threadIdx.x; i < (int)(sizeof(CallArgs) / 4); i += kThreads) reinterpret_cast<uint32_t*>(smem_dyn + kPrData + kPrModel)[i] = reinterpret_cast<const uint32_t*>(&Ap)[i];
-    const DevModel& M = *reinterpret_cast<const DevModel*>(smem_dyn + kPrData);
-    const CallArgs& A = *reinterpret_cast<const CallArgs*>(smem_dyn + kPrData + kPrModel);
-    __syncthreads();
-    Ctx c;
     c.cta = blockIdx.x; c.n_ctas = gridDim.x; c.tid = threadIdx.x;
     c.warp = threadIdx.x >> 5; c.lane = threadIdx.x & 31;
     c.xs = reinterpret_cast<float*>(smem_dyn);
@@ -478,8 +495,17 @@ smol_prompt_kernel(const __grid_constant__ DevModel Mp, const __grid_constant__ 
     umma::fence_before_sync();
     __syncthreads();
     umma::fence_after_sync();
+    sy.target = ldcg_u32(Mp.barrier + 1); sy.par_w = 0; sy.par_x = 0; sy.pending = false; sy.phase = 0; sy.next = -1; sy.waits_for = 0;
+}
+
+__global__ void __launch_bounds__(kThreads, 1)
+smol_prompt_kernel(const __grid_constant__ DevModel Mp, const __grid_constant__ CallArgs Ap) {
+    extern __shared__ __align__(1024) unsigned char smem_dyn[];
+    const DevModel& M = *reinterpret_cast<const DevModel*>(smem_dyn + kPrData);
+    const CallArgs& A = *reinterpret_cast<const CallArgs*>(smem_dyn + kPrData + kPrModel);
+    Ctx c;
     RowsSync sy;
-    sy.target = ldcg_u32(M.barrier + 1); sy.par_w = 0; sy.par_x = 0; sy.pending = false; sy.phase = 0; sy.next = -1; sy.waits_for = 0;
+    prompt_setup(Mp, Ap, smem_dyn, c, sy);
     uint32_t chunk = 0, tile = 0;
     for (int it = 0; it < A.n_iter; ++it) {
         c.iter = it;
@@ -494,7 +520,7 @@ smol_prompt_kernel(const __grid_constant__ DevModel Mp, const __grid_constant__ 
                 rows_sync_in(M, sy);
                 prompt_attn(M, A, c, ph, sy, Ap.kv_map, last_row);
             } else {
-                prompt_gemm(M, A, c, ph, sy, chunk, tile, last_row);
+                prompt_gemm<false>(M, A, c, ph, sy, chunk, tile, last_row);
                 if (ph.kind == PH_WO || ph.kind == PH_W2) {   // h = stream + wo(attn) (P:499); stream = h + w2(act) (P:500); and the norm of the phase that reads it
                     rows_arrive(M, c, sy);
                     rows_sync_in(M, sy);
@@ -534,6 +560,94 @@ smol_prompt_kernel(const __grid_constant__ DevModel Mp, const __grid_constant__ 
         }
         if (c.tid == 0) M.barrier[1] = sy.target;
     }
+    umma::fence_before_sync();
+    __syncthreads();
+    if (c.warp == 0) umma::tmem_free(g_pr.tmem_base);
+}
+
+__device__ void phase_sample(const DevModel& M, const CallArgs& A, const Ctx& c, const Phase& ph);
+
+// ---- decode frames of wide batches ----------------------------------------------------------------------------------
+// From kWideRows rows on (host: wide_launch) a frame's weight phases are tiles of 128 rows instead of rows_phases.cuh's groups of 32,
+// which repeat the norm and the row copies per weight block and take several turns (150m, 256 rows: 2699 us per frame against 3380).  Sums are in the same order, so
+// a row's bits are the same on either side of the line.
+__device__ __noinline__ void wide_attn(const DevModel& M, const CallArgs& A, const Ctx& c, const Phase& ph, RowsSync& sy, const void* kv_map) { phase_attn_batch<false>(M, A, c, ph, sy, kv_map); }
+// Depth attention of all rows -> M.attn, the CTA's share of the rows in groups of one row per kv-head's warps.
+__device__ __noinline__ void wide_depth_attention(const DevModel& M, const CallArgs& A, const Ctx& c, int layer, int depth_pos) {
+    const int per = (A.batch + c.n_ctas - 1) / c.n_ctas, r0 = c.cta * per, n = min(per, A.batch - r0);
+    if (n <= 0) return;
+    unsigned char* out = reinterpret_cast<unsigned char*>(M.attn + (size_t)r0 * M.fdim);
+    if (depth_pos < 8) rows_depth_attention<false>(M, layer, depth_pos, r0, n, out, M.fdim * 2);
+    else rows_depth_attention<true>(M, layer, depth_pos, r0, n, out, M.fdim * 2);
+}
+// The input of the slow or the depth transformer -> its residual stream, and the first norm: the token embedding (P:205-221), the
+// slow hidden state or the previous depth code's embedding (G:136-140).
+__device__ __noinline__ void wide_input(const DevModel& M, const CallArgs& A, const Ctx& c, const Phase& ph) {
+    if (!ph.fast) {
+        prompt_row_step(M, A, c, M.dim, M.x, M.layers[0].attention_norm, [&](int bg, int ch, float (&x)[8]) { embed_chunk(M, A, c, bg, ch, x); });
+        return;
+    }
+    prompt_row_step(M, A, c, M.fdim, M.xf, M.fast_layers[0].attention_norm, [&](int bg, int ch, float (&x)[8]) {
+        const uint16_t* src = (A.fast_from_xf ? M.xf : M.x) + (size_t)bg * M.fdim;
+        if (!A.fast_from_xf && ph.depth_pos > 0) {
+            const int code = ldcg_i32(M.frame_tokens + (size_t)bg * M.n_rows + ph.depth_pos);
+            src = M.fast_embeddings + (size_t)(code + (M.depthwise_wte ? (M.dup0 ? ph.depth_pos - 1 : ph.depth_pos) * M.codebook_size : 0)) * M.fdim;
+        }
+        unpack8(ldcg_v4(src + ch * 8), x);
+    });
+}
+__device__ __noinline__ void wide_sample(const DevModel& M, const CallArgs& A, const Ctx& c, const Phase& ph) { phase_sample(M, A, c, ph); }
+
+__global__ void __launch_bounds__(kThreads, 1)
+smol_wide_kernel(const __grid_constant__ DevModel Mp, const __grid_constant__ CallArgs Ap) {
+    extern __shared__ __align__(1024) unsigned char smem_dyn[];
+    const DevModel& M = *reinterpret_cast<const DevModel*>(smem_dyn + kPrData);
+    const CallArgs& A = *reinterpret_cast<const CallArgs*>(smem_dyn + kPrData + kPrModel);
+    Ctx c;
+    RowsSync sy;
+    prompt_setup(Mp, Ap, smem_dyn, c, sy);
+    uint32_t chunk = 0, tile = 0;
+    const bool prof = M.prof != nullptr && c.cta == 0 && c.tid == 0;   // per phase: its time, and (in it) the wait for the one before
+    for (int it = 0; it < A.n_iter; ++it) {
+        c.iter = it;
+        for (int p = A.phase_begin; p < A.phase_end; ++p) {
+            const Phase ph = unpack_phase(M.prog[p]);
+            const bool fast = ph.fast != 0;
+            const unsigned long long t0 = prof ? globaltimer_ns() : 0ull;
+            if (ph.kind == PH_ATTN) {
+                wide_attn(M, A, c, ph, sy, Ap.kv_map);
+            } else if (ph.kind == PH_SAMPLE) {
+                rows_sync_in(M, sy);
+                wide_sample(M, A, c, ph);
+            } else {
+                const bool input = ph.kind == PH_QKV && ph.layer == 0, depth_attn = ph.kind == PH_WO && fast;
+                if (input || depth_attn) {
+                    rows_sync_in(M, sy);
+                    if (input) wide_input(M, A, c, ph);
+                    else wide_depth_attention(M, A, c, ph.layer, ph.depth_pos);
+                    rows_arrive(M, c, sy);
+                }
+                if (ph.kind == PH_QKV && !fast) attn_prefetch(M, A, c, ph.layer);
+                prompt_gemm<true>(M, A, c, ph, sy, chunk, tile, -1);
+                if (ph.kind == PH_WO || ph.kind == PH_W2) {
+                    rows_arrive(M, c, sy);
+                    rows_sync_in(M, sy);
+                    const bool wo = ph.kind == PH_WO;
+                    const DevLayer* L = fast ? M.fast_layers : M.layers;
+                    uint16_t* stream = fast ? M.xf : M.x;
+                    const uint16_t* norm = wo ? L[ph.layer].ffn_norm : ph.layer + 1 < (fast ? M.n_flayer : M.n_layer) ? L[ph.layer + 1].attention_norm : fast ? M.fast_norm : M.norm;
+                    const int D = fast ? M.fdim : M.dim;
+                    prompt_finish(M, A, c, wo ? stream : M.h, wo ? M.h : stream, D, prompt_slices(wo ? D : fast ? M.finter : M.inter), norm, -1);
+                }
+            }
+            if (c.cta == 0 && A.advance && p == A.phase_end - 1)
+                for (int b = c.tid; b < A.batch; b += kThreads) A.b.seq_len[b] = ldcg_i32(A.b.seq_len + b) + 1;
+            sy.waits_for = p;
+            if (prof) M.prof[2 * p] += globaltimer_ns() - t0;
+            if (!(it == A.n_iter - 1 && p == A.phase_end - 1)) rows_arrive(M, c, sy);
+        }
+    }
+    if (c.cta == 0 && c.tid == 0) M.barrier[1] = sy.target;
     umma::fence_before_sync();
     __syncthreads();
     if (c.warp == 0) umma::tmem_free(g_pr.tmem_base);

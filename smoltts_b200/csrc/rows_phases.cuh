@@ -10,7 +10,7 @@
 //   * weights never wait for activations: a CTA's weight tiles of the next phase (one bulk copy, packed fragments) land in
 //     shared memory while it finishes this phase and sits in the barrier; cached keys and values are fetched there, too;
 //   * rows come by bulk copies, and a phase's pointers and sizes from tables in shared memory.
-// Measured (150m, contexts of up to 471, us per frame): 9 rows 1255, 16: 1262, 32: 1330, 64: 1505; tcgen05 tiles (activation
+// Measured (150m, contexts of up to 471, us per frame): 9 rows 1188, 16: 1195, 32: 1266, 64: 1437; tcgen05 tiles (activation
 // rows as the 128 lanes of an accumulator, 16 .. 96 weight rows as its columns, row steps between the phases) took 2135 to 2226:
 // with so few columns an MMA is bound by the 4 KB of its A operand, wo and w2 had to be cut over CTAs and added in a step of
 // their own, and a frame had 380 barriers instead of 197.
@@ -77,7 +77,10 @@ __device__ __forceinline__ void rows_sync_in(const DevModel& M, RowsSync& sy) {
 }
 __device__ __forceinline__ void rows_arrive(const DevModel& M, const Ctx& c, RowsSync& sy) {
     rows_sync_in(M, sy);       // (every phase has waited already: a CTA never arrives twice in a row)
-    fence_proxy_async_all();   // rows written here are read by other CTAs' bulk copies; shared memory used here is overwritten by such copies
+    // Shared memory used here is overwritten by copies.  (Rows written here are read by other CTAs' copies: the threads that issue those
+    // fence global memory behind the barrier; a full fence.proxy.async here waits for
+    // the stores of every thread: frames of 9 / 64 rows 1263 / 1520 us with it, 1188 / 1437 without.)
+    fence_proxy_async();
     grid_arrive(M.barrier, sy.target, (uint32_t)c.n_ctas);
     sy.pending = true;
 }
@@ -180,7 +183,7 @@ __device__ __forceinline__ void phase_attn_batch(const DevModel& M, const CallAr
     const int wpt = attn_warps(n_units, c.n_ctas);
     const int per_cta = kWarps / wpt, slot = warp / wpt, wi = warp - slot * wpt;
     if (kPrompt) rows_sync_in(M, sy);
-    if (lane == 0) fence_proxy_async_global();               // keys and values written by other CTAs
+    if (kPrompt && lane == 0) fence_proxy_async_global();    // keys and values written by other CTAs
     constexpr float kScale = 0.125f * 1.4426950408889634f;   // 1/sqrt(64) * log2(e): softmax in base 2
 
     // neighbouring units on different SMs; the trip count is the same for all warps of the CTA
@@ -271,7 +274,10 @@ __device__ __forceinline__ void phase_attn_batch(const DevModel& M, const CallAr
                     for (int i = 0; i < depth && fetched + 16 <= min(pl, len0); ++i) fetch();
                     rows_sync_in(M, sy);
                 }
-                if (!kPrompt) load_q();
+                if (!kPrompt) {
+                    if (lane == 0) fence_proxy_async_global();   // the newest position was written by other CTAs
+                    load_q();
+                }
                 while (fetched < pl && fetched < p0 + 16 * depth) fetch();
                 for (int pb = p0; pb < pl; pb += 16) {
                     rows_wait(&g_kvbar[buf0 + at], __shfl_sync(0xffffffffu, par, at));
@@ -524,8 +530,9 @@ __device__ void rows_tables(const DevModel& M, const CallArgs& A, const Ctx& c, 
         if (ph.kind != PH_ATTN && ph.kind != PH_SAMPLE) {
             const RowsKind& r = g_rk[ph.fast][ph.kind];
             const DevLayer& L = ph.fast ? M.fast_layers[ph.layer] : M.layers[ph.layer];
-            s.w = ph.kind == PH_QKV ? L.pr_wqkv : ph.kind == PH_WO ? L.pr_wo : ph.kind == PH_W13 ? L.pr_w13 : ph.kind == PH_W2 ? L.pr_w2
-                : ph.fast ? M.pr_fast_output + (M.depthwise_output ? (size_t)ph.depth_pos * r.tiles * 16 * r.K : 0) : M.pr_head;
+            const RowsLayer& W = ph.fast ? M.rows_fast_layers[ph.layer] : M.rows_layers[ph.layer];
+            s.w = ph.kind == PH_QKV ? W.wqkv : ph.kind == PH_WO ? W.wo : ph.kind == PH_W13 ? W.w13 : ph.kind == PH_W2 ? W.w2
+                : ph.fast ? M.rows_fast_output + (M.depthwise_output ? (size_t)ph.depth_pos * r.tiles * 16 * r.K : 0) : M.rows_head;
             s.norm_w = ph.kind == PH_QKV ? L.attention_norm : ph.kind == PH_W13 ? L.ffn_norm : ph.fast ? M.fast_norm : M.norm;
             if (r.block0 >= 0) s.w += (size_t)r.block0 * r.mt * 16 * r.K;
         }

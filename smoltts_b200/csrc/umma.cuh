@@ -175,9 +175,7 @@ struct BSrc {
 };
 enum WeightPolicy { kWeightsDefault = 0, kWeightsStream = 1, kWeightsKeep = 2 };
 
-// The two TMA-issuing threads of a tile (warps 1 and 3).  decode_kernel.cu / tc_phases.cuh order the activations that other
-// CTAs wrote with st.global against these threads' async-proxy reads (fence.proxy.async after every grid barrier): the
-// fence predicates use the same constants.
+// The two TMA-issuing threads of a tile (warps 1 and 3) of tile_mma_tma.
 constexpr int kTmaProducerA = 32;   // activation boxes
 constexpr int kTmaProducerB = 96;   // weight boxes
 

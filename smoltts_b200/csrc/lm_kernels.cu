@@ -2442,6 +2442,126 @@ extern "C" int smol_lm_bind(SmolLm* m, const SmolLmGlobals* g, void* d_workspace
     return SMOL_OK;
 }
 
+namespace smol {
+namespace lm {
+// gemm_few_kernel for activations that a prologue makes (a form of its own: shared with the plain one it cost that 1.4 % in decoding).
+// begin(): the prologue; row(m, k): 8 elements of an activation row; part: [WARPS][few_out(NR, MT)], in the place of the activations.
+constexpr int few_out(int nr, int mt) { return nr * (nr == 16 ? 8 : 16) * mt; }     // outputs of a block
+template <int NR, int MT, int WARPS, class Begin, class Row>
+__device__ __forceinline__ void few_product(const bf16* __restrict__ w, float* __restrict__ y, int M, int N, int K, float* part, Begin begin, Row row) {
+    constexpr int WT = NR / 8, AT = NR == 16 ? MT : 2 * MT;      // 8-row pieces of weights and of activations per step
+    constexpr int U = WT + AT <= 3 ? 4 : 2;                      // steps of 32 whose loads are in flight together
+    constexpr int OUT = few_out(NR, MT);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, tq = lane & 3;
+    const int n0 = blockIdx.x * NR;
+    const bf16* wr[WT];
+#pragma unroll
+    for (int i = 0; i < WT; ++i) wr[i] = w + (size_t)min(n0 + i * 8 + g, N - 1) * K + tq * 8;
+    float acc[MT][4];
+#pragma unroll
+    for (int i = 0; i < MT; ++i)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) acc[i][e] = 0.0f;
+    const uint4 zero = make_uint4(0, 0, 0, 0);
+    uint4 p[U][WT];
+    auto load_weights = [&](int k0) {
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const int k = k0 + u * WARPS * 32;
+#pragma unroll
+            for (int i = 0; i < WT; ++i) p[u][i] = k + tq * 8 < K ? ldg_stream(wr[i] + k) : zero;
+        }
+    };
+    load_weights(warp * 32);             // no kernel of a step writes weights: the first ones are on their way before the wait (smol_lm_linear launches plainly)
+    begin();
+    for (int k0 = warp * 32; k0 < K; k0 += WARPS * 32 * U) {
+        uint4 x[U][AT];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const int k = k0 + u * WARPS * 32 + tq * 8;
+#pragma unroll
+            for (int i = 0; i < AT; ++i) {
+                const int m = i * 8 + g;
+                x[u][i] = (m < M && k < K) ? row(m, k) : zero;
+            }
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+#pragma unroll
+            for (int i = 0; i < MT; ++i) {
+                float lo[4] = {0.0f, 0.0f, 0.0f, 0.0f}, hi[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+                if constexpr (NR == 16) {
+                    mma_bf16_16816(lo, p[u][0].x, p[u][1].x, p[u][0].y, p[u][1].y, x[u][i].x, x[u][i].y);
+                    mma_bf16_16816(hi, p[u][0].z, p[u][1].z, p[u][0].w, p[u][1].w, x[u][i].z, x[u][i].w);
+                } else {
+                    mma_bf16_16816(lo, x[u][2 * i].x, x[u][2 * i + 1].x, x[u][2 * i].y, x[u][2 * i + 1].y, p[u][0].x, p[u][0].y);
+                    mma_bf16_16816(hi, x[u][2 * i].z, x[u][2 * i + 1].z, x[u][2 * i].w, x[u][2 * i + 1].w, p[u][0].z, p[u][0].w);
+                }
+#pragma unroll
+                for (int e = 0; e < 4; ++e) acc[i][e] += lo[e] + hi[e];
+            }
+        load_weights(k0 + WARPS * 32 * U);
+    }
+    __syncthreads();
+    // part[warp][m * NR + n]: neighbouring outputs of a row side by side.  acc[.][e]: tile row g + (e / 2) * 8, tile column 2 tq + e % 2
+#pragma unroll
+    for (int i = 0; i < MT; ++i)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            const int r = g + (e >> 1) * 8, c = tq * 2 + (e & 1);
+            part[warp * OUT + (NR == 16 ? (i * 8 + c) * NR + r : (i * 16 + r) * NR + c)] = acc[i][e];
+        }
+    __syncthreads();
+    for (int o = threadIdx.x; o < OUT; o += WARPS * 32) {
+        const int m = o / NR, n = n0 + o % NR;
+        double t = part[o];
+#pragma unroll
+        for (int x = 1; x < WARPS; ++x) t += part[x * OUT + o];
+        if (m < M && n < N) y[(size_t)m * N + n] = (float)t;
+    }
+}
+// Down-projection of one row with PolyNorm in its prologue: every block takes the row's activation into shared memory, behind its first
+// weights.  As a kernel of its own it is one more link of the step's chain, whatever it computes: one token through 10 layers of width 768,
+// 4 steps 1622 us -> 1589.  Two and more rows stay with two kernels: what the
+// blocks repeat costs more than the launch (2 rows 992 | 999, 4: 1042 | 1104, 8: 1097 | 1117 through 6 layers), as do gated units, whose input is twice as
+// long (5 rows of width 1536 990 | 1063).
+constexpr size_t kFewActSmem = 48 * 1024 - 512;
+template <int NR, int WARPS>
+__global__ void __launch_bounds__(WARPS * 32) gemm_polynorm_kernel(const float* __restrict__ z, const float* __restrict__ coef, float eps,
+                                                                   const bf16* __restrict__ w, float* __restrict__ y, int N, int K) {
+    extern __shared__ uint4 few_smem[];
+    __shared__ float red[3][33];
+    bf16* xs = reinterpret_cast<bf16*>(few_smem);
+    few_product<NR, 1, WARPS>(w, y, 1, N, K, reinterpret_cast<float*>(few_smem), [&] {
+        dep_wait();
+        dep_go();
+        float s2 = 0.0f, s4 = 0.0f, s6 = 0.0f;
+#pragma unroll 4
+        for (int c = threadIdx.x * 4; c < K; c += WARPS * 128) {
+            const float4 v = *reinterpret_cast<const float4*>(z + c);
+            const float e[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const float v2 = e[j] * e[j];
+                s2 += v2;
+                s4 += v2 * v2;
+                s6 += v2 * v2 * v2;
+            }
+        }
+        block_sum3(s2, s4, s6, red);
+        const float a = coef[0] / sqrtf(s2 / (float)K + eps), b = coef[1] / sqrtf(s4 / (float)K + eps), cc = coef[2] / sqrtf(s6 / (float)K + eps), e = coef[3];
+        auto f = [&](float v) { return a * v + b * v * v + cc * v * v * v + e; };
+#pragma unroll 4
+        for (int c = threadIdx.x * 4; c < K; c += WARPS * 128) {
+            const float4 v = *reinterpret_cast<const float4*>(z + c);
+            store4<bf16>(xs + c, f(v.x), f(v.y), f(v.z), f(v.w));
+        }
+        __syncthreads();
+    }, [&](int, int k) { return *reinterpret_cast<const uint4*>(xs + k); });
+}
+}  // namespace lm
+}  // namespace smol
+
 // The kernels of a step are launched with programmatic stream serialization and begin with dep_wait(): a kernel's blocks are set up while
 // the kernel before it drains, instead of after.  What bounds a decoding step is its chain of some hundred dependent kernels of two to ten
 // microseconds: 10 layers of width 768, one token against 2048 cached ones, 4 steps 1780 us -> 1615; 5 sequences of 700 through 4 layers of
@@ -2630,6 +2750,22 @@ cudaError_t linear<bf16>(SmolLm* m, const bf16* a, const bf16* w, float* y, int 
     }
     m->launches++;
     return cudaGetLastError();
+}
+
+// y [N] = polynorm(z [K]) . w^T in one kernel (gemm_polynorm_kernel); false: the row does not fit its shared memory or is not whole pieces.
+static bool linear_polynorm_row(SmolLm* m, const float* z, const float* coef, const bf16* w, float* y, int N, int K, cudaStream_t st) {
+    if (K % 8 != 0 || reinterpret_cast<uintptr_t>(w) % 16 != 0 || (size_t)K * 2 > kFewActSmem) return false;
+#define SMOL_FEW_POLY(NR, WARPS)                                                                                                           \
+    pdl_launch(gemm_polynorm_kernel<NR, WARPS>, (N + NR - 1) / NR, WARPS * 32, std::max((size_t)K * 2, (size_t)WARPS * few_out(NR, 1) * 4), st, \
+               z, coef, m->cfg.norm_eps, w, y, N, K)
+    if (N < kFewWideN) {
+        if (K >= kFewLongK) SMOL_FEW_POLY(8, 16);
+        else SMOL_FEW_POLY(8, 8);
+    } else if (K >= kFewLongK) SMOL_FEW_POLY(16, 16);
+    else SMOL_FEW_POLY(16, 8);
+#undef SMOL_FEW_POLY
+    m->launches++;
+    return true;
 }
 
 // Grouped product on the tcgen05 tile: a [rows, K] sorted by group, w [groups * N, K], the table cut into 128-row tiles.
@@ -3205,9 +3341,11 @@ static int step_impl(SmolLm* m, const SmolLmStep* s, cudaStream_t st) {
         auto feed_forward = [&](cudaStream_t st) -> int {
             if (L.mlp == SMOL_LM_MLP_POLYNORM) {
                 CU(linear<T>(m, hn, static_cast<const T*>(L.w_up), z, Tn, L.ff, D, st));
-                pdl_launch(polynorm_kernel<T>, Tn, 256, 0, st, z, L.act, c.norm_eps, L.ff, act);
-                CU(linear<T>(m, act, static_cast<const T*>(L.w_down), y, Tn, D, L.ff, st));
-                m->launches += 1;
+                if (kIsF32 || Tn != 1 || !linear_polynorm_row(m, z, L.act, static_cast<const bf16*>(L.w_down), y, D, L.ff, st)) {
+                    pdl_launch(polynorm_kernel<T>, Tn, 256, 0, st, z, L.act, c.norm_eps, L.ff, act);
+                    CU(linear<T>(m, act, static_cast<const T*>(L.w_down), y, Tn, D, L.ff, st));
+                    m->launches += 1;
+                }
             } else if (L.mlp == SMOL_LM_MLP_GATED) {
                 CU(linear<T>(m, hn, static_cast<const T*>(L.w_up), z, Tn, 2 * L.ff, D, st));
                 pdl_launch(gated_act_kernel<T>, cast_grid((size_t)Tn * L.ff / 4), 256, 0, st, z, L.ff, actp_of(L), (size_t)Tn, act);

@@ -218,6 +218,7 @@ template <> __device__ __forceinline__ void store4<bf16>(bf16* p, float a, float
 
 // PolyNorm: out = a z/rms(z) + b z^2/rms(z^2) + c z^3/rms(z^3) + e over a token's feed-forward vector.  The three sums
 // are taken in one pass and reduced together; rows whose length is a multiple of 4 move as 16-byte pieces.
+constexpr int kPolynormThreads = 256;
 template <class T>
 __global__ void polynorm_kernel(const float* __restrict__ z, const float* __restrict__ coef, float eps, int F, T* __restrict__ out) {
     dep_wait();
@@ -2536,16 +2537,19 @@ __global__ void __launch_bounds__(WARPS * 32) gemm_polynorm_kernel(const float* 
         dep_wait();
         dep_go();
         float s2 = 0.0f, s4 = 0.0f, s6 = 0.0f;
+        // the sums by polynorm_kernel's threads, each with the elements it has there: a row's bits do not depend on which form takes it
+        if (threadIdx.x < kPolynormThreads) {
 #pragma unroll 4
-        for (int c = threadIdx.x * 4; c < K; c += WARPS * 128) {
-            const float4 v = *reinterpret_cast<const float4*>(z + c);
-            const float e[4] = {v.x, v.y, v.z, v.w};
+            for (int c = threadIdx.x * 4; c < K; c += kPolynormThreads * 4) {
+                const float4 v = *reinterpret_cast<const float4*>(z + c);
+                const float e[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                const float v2 = e[j] * e[j];
-                s2 += v2;
-                s4 += v2 * v2;
-                s6 += v2 * v2 * v2;
+                for (int j = 0; j < 4; ++j) {
+                    const float v2 = e[j] * e[j];
+                    s2 += v2;
+                    s4 += v2 * v2;
+                    s6 += v2 * v2 * v2;
+                }
             }
         }
         block_sum3(s2, s4, s6, red);
@@ -3342,7 +3346,7 @@ static int step_impl(SmolLm* m, const SmolLmStep* s, cudaStream_t st) {
             if (L.mlp == SMOL_LM_MLP_POLYNORM) {
                 CU(linear<T>(m, hn, static_cast<const T*>(L.w_up), z, Tn, L.ff, D, st));
                 if (kIsF32 || Tn != 1 || !linear_polynorm_row(m, z, L.act, static_cast<const bf16*>(L.w_down), y, D, L.ff, st)) {
-                    pdl_launch(polynorm_kernel<T>, Tn, 256, 0, st, z, L.act, c.norm_eps, L.ff, act);
+                    pdl_launch(polynorm_kernel<T>, Tn, kPolynormThreads, 0, st, z, L.act, c.norm_eps, L.ff, act);
                     CU(linear<T>(m, act, static_cast<const T*>(L.w_down), y, Tn, D, L.ff, st));
                     m->launches += 1;
                 }

@@ -28,3 +28,23 @@ def test_one_row_against_two(width, ff):
     assert rel_err(alone, want) < TOL[torch.bfloat16]
     # the same roundings but for the order of PolyNorm's sums: a bf16 activation in some thousand moves by one place (2^-8 of it)
     assert rel_err(alone, both[:1]) < 2.0 ** -8
+
+
+@pytest.mark.parametrize("width,ff", [(64, 48), (64, 1000), (64, 2040), (96, 2048), (72, 4104), (64, 24312)])
+def test_one_row_has_the_bits_it_has_beside_another(width, ff):
+    """The sums of PolyNorm are taken in the same order whichever kernel takes the row: 8 warps of the down-projection (up to 2040
+    elements) or 16, or a kernel of its own."""
+    cfg = config([attn(ff=ff)], vocab=61, width=width)
+    model, _, _ = engine_and_oracle(cfg, seed=3, dtype=torch.bfloat16)
+    rows = [tokens(1, 61, seed=s) for s in range(1, 9)]
+    for i in range(0, 8, 2):
+        seqs = [model.open_sequence() for _ in range(2)]
+        both = model.forward([(q, t, [0]) for q, t in zip(seqs, rows[i:i + 2])]).clone()
+        for q in seqs:
+            model.close_sequence(q)
+        for j in range(2):
+            seq = model.open_sequence()
+            alone = model.forward([(seq, rows[i + j], [0])]).clone()
+            model.close_sequence(seq)
+            assert torch.equal(alone, both[j:j + 1])
+    model.check_device_errors()

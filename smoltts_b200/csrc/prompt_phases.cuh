@@ -577,8 +577,8 @@ __device__ __noinline__ void wide_depth_attention(const DevModel& M, const CallA
     const int per = (A.batch + c.n_ctas - 1) / c.n_ctas, r0 = c.cta * per, n = min(per, A.batch - r0);
     if (n <= 0) return;
     unsigned char* out = reinterpret_cast<unsigned char*>(M.attn + (size_t)r0 * M.fdim);
-    if (depth_pos < 8) rows_depth_attention<false>(M, layer, depth_pos, r0, n, out, M.fdim * 2);
-    else rows_depth_attention<true>(M, layer, depth_pos, r0, n, out, M.fdim * 2);
+    if (depth_pos < 8) rows_depth_attention<false>(M, layer, depth_pos, r0, n, out, M.fdim * 2, nullptr);
+    else rows_depth_attention<true>(M, layer, depth_pos, r0, n, out, M.fdim * 2, nullptr);
 }
 // The input of the slow or the depth transformer -> its residual stream, and the first norm: the token embedding (P:205-221), the
 // slow hidden state or the previous depth code's embedding (G:136-140).

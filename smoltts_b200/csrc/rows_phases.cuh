@@ -567,84 +567,93 @@ __device__ __noinline__ void rows_embed(const DevModel& M, const CallArgs& A, co
     }
 }
 
-// Depth attention of rows [r0, r0 + n_live), one warp per (row, kv head), two of them at a time: S = Q K^T with the kv head's
-// G query heads as the rows of the A operand and its <= 16 positions as columns, one softmax with the true maximum,
-// probabilities rounded to bf16 for P V while the row sum keeps the unrounded values (P:559-566), as fast_attention_rows.
-// The dims of Q K^T and the columns of P V are permuted as in phase_attn_batch, so that all loads are 16 bytes.  The result
-// goes to shared memory as bf16 rows (`stride` bytes apart), where the wo tiles of this CTA read it.  Every tile block of wo
-// repeats it: for 8 rows that is two tasks per warp, less than the barrier that a step of its own would need.
-template <bool deep>   // deep: positions 8 .. 15 exist (a form of its own: without the branch two tasks' chains interleave)
-__device__ __forceinline__ void rows_depth_attention(const DevModel& M, int layer, int depth_pos, int r0, int n_live, unsigned char* out, int stride) {
+// Depth attention of one query head by a warp, in the arithmetic and the order of additions of fast_attention_rows: fp32 FMAs, four lanes per
+// position with 16 dims each (position lane / 4, and + 8 where `deep`), one softmax with the true maximum, probabilities rounded to bf16 for
+// P V while the row sum keeps the unrounded values (P:559-566).  Returns dims 2 lane, 2 lane + 1.  q: the lane's 16 dims; k: of its
+// positions; v: its two dims of all positions (zeros past depth_pos).
+template <bool deep>
+__device__ __forceinline__ uint32_t depth_head(const uint4 (&q)[2], const uint4 (&k)[deep ? 2 : 1][2], const uint32_t (&v)[deep ? 16 : 8], int depth_pos, int lane) {
+    constexpr int H = deep ? 2 : 1;
+    const int jl = lane >> 2;
+    float qf[16], sc[H];
+    unpack8(q[0], *reinterpret_cast<float(*)[8]>(qf));
+    unpack8(q[1], *reinterpret_cast<float(*)[8]>(qf + 8));
+#pragma unroll
+    for (int h = 0; h < H; ++h) {
+        float k0[8], k1[8], s = 0.f;
+        unpack8(k[h][0], k0);
+        unpack8(k[h][1], k1);
+#pragma unroll
+        for (int e = 0; e < 8; ++e) s = fmaf(qf[e], k0[e], s);
+#pragma unroll
+        for (int e = 0; e < 8; ++e) s = fmaf(qf[8 + e], k1[e], s);
+        s += __shfl_xor_sync(0xffffffffu, s, 1);
+        s += __shfl_xor_sync(0xffffffffu, s, 2);
+        sc[h] = jl + 8 * h <= depth_pos ? s * 0.125f : -INFINITY;
+    }
+    float m = deep ? fmaxf(sc[0], sc[H - 1]) : sc[0];
+    asm volatile("redux.sync.max.f32 %0, %0, 0xffffffff;" : "+f"(m));
+    float pe[H], pb[H];
+#pragma unroll
+    for (int h = 0; h < H; ++h) { pe[h] = jl + 8 * h <= depth_pos ? expf(sc[h] - m) : 0.f; pb[h] = bf16_round(pe[h]); }
+    float l = deep ? pe[0] + pe[H - 1] : pe[0];
+    l += __shfl_xor_sync(0xffffffffu, l, 4);
+    l += __shfl_xor_sync(0xffffffffu, l, 8);
+    l += __shfl_xor_sync(0xffffffffu, l, 16);
+    float o0 = 0.f, o1 = 0.f;
+#pragma unroll
+    for (int j = 0; j < 8 * H; ++j) {
+        const float p = __shfl_sync(0xffffffffu, pb[j / 8], (j & 7) * 4);
+        o0 = fmaf(p, bf_lo(v[j]), o0);
+        o1 = fmaf(p, bf_hi(v[j]), o1);
+    }
+    const float inv = __frcp_rn(l);
+    return pack_bf16(o0 * inv, o1 * inv);
+}
+// kp: a kv head's first key; `kvw` elements from position to position, the values behind `depth` keys
+template <bool deep>
+__device__ __forceinline__ void depth_load(const uint16_t* kp, int kvw, int depth, int depth_pos, int lane, uint4 (&k)[deep ? 2 : 1][2], uint32_t (&v)[deep ? 16 : 8]) {
+    const uint4 z = make_uint4(0u, 0u, 0u, 0u);
+    const uint16_t* vp = kp + (size_t)depth * kvw + 2 * lane;
+#pragma unroll
+    for (int h = 0; h < (deep ? 2 : 1); ++h) {
+        const int j = (lane >> 2) + 8 * h;
+        const uint16_t* kr = kp + (size_t)j * kvw + (lane & 3) * 16;
+        k[h][0] = j <= depth_pos ? ldcg_v4(kr) : z;
+        k[h][1] = j <= depth_pos ? ldcg_v4(kr + 8) : z;
+    }
+#pragma unroll
+    for (int j = 0; j < (deep ? 16 : 8); ++j) v[j] = j <= depth_pos ? ldcg_u32(vp + (size_t)j * kvw) : 0u;
+}
+
+// Depth attention of rows [r0, r0 + n_live) by one CTA, a warp per (row, kv head), which goes through the kv head's G query heads.  The
+// result goes to shared memory as bf16 rows (`stride` bytes apart), where the wo tiles of this CTA read it, and, where `copy` is given,
+// to its rows of M.attn.  Every tile block of wo repeats it: for 8 rows that is two tasks per warp, less than the barrier that a
+// step of its own would need.  4.6 us of the 7.5 of such a phase at 64 rows (150m), a chain of loads, FMAs and shuffles per head; the heads side
+// by side, two tasks at once, or more loads ahead spill and take longer (frames of 64, us: 1456, and 1515 to 1720).
+template <bool deep>   // deep: positions 8 .. 15 exist
+__device__ __forceinline__ void rows_depth_attention(const DevModel& M, int layer, int depth_pos, int r0, int n_live, unsigned char* out, int stride, uint16_t* copy) {
     const int Hq = M.fn_head, Hkv = M.fn_kv, G = Hq / Hkv, kvw = Hkv * kHeadDim, depth = M.depth, n_flayer = M.n_flayer;
     const uint16_t* q0 = M.q;
     const uint16_t* kv0 = M.fkv;
-    const int tid = tid_here(), warp = tid >> 5, lane = tid & 31, g = lane >> 2, cc = lane & 3;
-    const uint4 z = make_uint4(0u, 0u, 0u, 0u);
-    constexpr int T = 2;
-    for (int t0 = warp; t0 < n_live * Hkv; t0 += T * kWarps) {
-        uint4 qv[T][2], kv[T][2], vv[T][2];
-        int row[T], kvh[T];
-#pragma unroll
-        for (int u = 0; u < T; ++u) {
-            const int task = min(t0 + u * kWarps, n_live * Hkv - 1);   // (a task twice: the same values to the same place)
-            row[u] = task / Hkv; kvh[u] = task - row[u] * Hkv;
-            const uint16_t* qp = q0 + (size_t)(r0 + row[u]) * Hq * kHeadDim + (kvh[u] * G + g) * kHeadDim + cc * 8;
-            const uint16_t* kp = kv0 + ((size_t)((r0 + row[u]) * n_flayer + layer) * 2) * depth * kvw + kvh[u] * kHeadDim;
-            const uint16_t* vp = kp + (size_t)depth * kvw + (size_t)(2 * cc) * kvw + g * 8;
-            kp += (size_t)g * kvw + cc * 8;
-            qv[u][0] = g < G ? ldcg_v4(qp) : z; qv[u][1] = g < G ? ldcg_v4(qp + 32) : z;
-            kv[u][0] = g <= depth_pos ? ldcg_v4(kp) : z; kv[u][1] = g <= depth_pos ? ldcg_v4(kp + 32) : z;
-            vv[u][0] = 2 * cc <= depth_pos ? ldcg_v4(vp) : z; vv[u][1] = 2 * cc + 1 <= depth_pos ? ldcg_v4(vp + kvw) : z;
-        }
-#pragma unroll
-        for (int u = 0; u < T; ++u) {
-            const uint4 a = qv[u][0], b = qv[u][1];
-            float s[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
-            auto scores = [&](float (&d)[4], uint4 ka, uint4 kb) {
-                mma_bf16_16816(d, a.x, 0u, a.y, 0u, ka.x, ka.y);
-                mma_bf16_16816(d, a.z, 0u, a.w, 0u, ka.z, ka.w);
-                mma_bf16_16816(d, b.x, 0u, b.y, 0u, kb.x, kb.y);
-                mma_bf16_16816(d, b.z, 0u, b.w, 0u, kb.z, kb.w);
-            };
-            scores(s[0], kv[u][0], kv[u][1]);
-            uint4 v2 = z, v3 = z;
-            if (deep) {
-                const uint16_t* kp = kv0 + ((size_t)((r0 + row[u]) * n_flayer + layer) * 2) * depth * kvw + kvh[u] * kHeadDim;
-                const uint16_t* vp = kp + (size_t)depth * kvw + (size_t)(2 * cc + 8) * kvw + g * 8;
-                kp += (size_t)(g + 8) * kvw + cc * 8;
-                const uint4 ka = g + 8 <= depth_pos ? ldcg_v4(kp) : z, kb = g + 8 <= depth_pos ? ldcg_v4(kp + 32) : z;
-                v2 = 2 * cc + 8 <= depth_pos ? ldcg_v4(vp) : z; v3 = 2 * cc + 9 <= depth_pos ? ldcg_v4(vp + kvw) : z;
-                scores(s[1], ka, kb);
-            }
-            // row g = query head g: positions 2 cc, 2 cc + 1 (and + 8)
-            float e[4];
-#pragma unroll
-            for (int i = 0; i < 4; ++i) e[i] = 2 * cc + (i & 1) + 8 * (i >> 1) <= depth_pos ? s[i >> 1][i & 1] * 0.125f : -INFINITY;
-            float m = fmaxf(fmaxf(e[0], e[1]), fmaxf(e[2], e[3]));
-            m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 1));
-            m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 2));
-            e[0] = expf(e[0] - m); e[1] = expf(e[1] - m);
-            if (deep) { e[2] = expf(e[2] - m); e[3] = expf(e[3] - m); } else { e[2] = 0.f; e[3] = 0.f; }
-            float l = (e[0] + e[1]) + (e[2] + e[3]);
-            l += __shfl_xor_sync(0xffffffffu, l, 1);
-            l += __shfl_xor_sync(0xffffffffu, l, 2);
-            const uint32_t pa = pack_bf16(e[0], e[1]), pb = pack_bf16(e[2], e[3]);
-            const float inv = 1.0f / l;
-            const uint32_t w0[4] = {vv[u][0].x, vv[u][0].y, vv[u][0].z, vv[u][0].w}, w1[4] = {vv[u][1].x, vv[u][1].y, vv[u][1].z, vv[u][1].w};
-            const uint32_t w2[4] = {v2.x, v2.y, v2.z, v2.w}, w3[4] = {v3.x, v3.y, v3.z, v3.w};
-            float x0[8], x1[8];
-#pragma unroll
-            for (int n = 0; n < 8; ++n) {   // columns 2 cc, 2 cc + 1 of n-tile n: dims 16 cc + n and 16 cc + 8 + n
-                const uint32_t sel = (n & 1) ? 0x7632u : 0x5410u;
-                float o[4] = {0.f, 0.f, 0.f, 0.f};
-                mma_bf16_16816(o, pa, 0u, pb, 0u, prmt(w0[n >> 1], w1[n >> 1], sel), prmt(w2[n >> 1], w3[n >> 1], sel));
-                x0[n] = o[0] * inv; x1[n] = o[1] * inv;
-            }
-            if (g < G) {
-                unsigned char* dst = out + (size_t)row[u] * stride + ((kvh[u] * G + g) * kHeadDim + 16 * cc) * 2;
-                *reinterpret_cast<uint4*>(dst) = pack8(x0);
-                *reinterpret_cast<uint4*>(dst + 16) = pack8(x1);
-            }
+    const int tid = tid_here(), warp = tid >> 5, lane = tid & 31;
+#pragma unroll 1
+    for (int task = warp; task < n_live * Hkv; task += kWarps) {
+        const int row = task / Hkv, kvh = task - row * Hkv;
+        const uint16_t* qp = q0 + ((size_t)(r0 + row) * Hq + kvh * G) * kHeadDim + (lane & 3) * 16;
+        uint4 k[deep ? 2 : 1][2], q[2] = {ldcg_v4(qp), ldcg_v4(qp + 8)};
+        uint32_t v[deep ? 16 : 8];
+        depth_load<deep>(kv0 + ((size_t)((r0 + row) * n_flayer + layer) * 2) * depth * kvw + kvh * kHeadDim, kvw, depth, depth_pos, lane, k, v);
+        int at = kvh * G * kHeadDim + 2 * lane;
+#pragma unroll 1
+        for (int g = 0; g < G; ++g, at += kHeadDim) {
+            uint4 next[2] = {q[0], q[1]};
+            qp += kHeadDim;
+            if (g + 1 < G) { next[0] = ldcg_v4(qp); next[1] = ldcg_v4(qp + 8); }
+            const uint32_t r = depth_head<deep>(q, k, v, depth_pos, lane);
+            *reinterpret_cast<uint32_t*>(out + (size_t)row * stride + at * 2) = r;
+            if (copy != nullptr) *reinterpret_cast<uint32_t*>(copy + (size_t)row * Hq * kHeadDim + at) = r;
+            q[0] = next[0]; q[1] = next[1];
         }
     }
 }
@@ -752,8 +761,9 @@ __device__ __forceinline__ void rows_gemm(const DevModel& M, const CallArgs& A, 
         // ---- the group's rows: bulk copies into shared memory (contiguous 16-byte loads take 3400 clocks for 96 KB on every SM
         // at once, loads straight into fragments -- 64 bytes of 8 rows each -- 7000, bulk copies 2000) ----
         if (kDepthAttn) {
-            if (ph.depth_pos < 8) rows_depth_attention<false>(M, ph.layer, ph.depth_pos, r0, n_live, rows_s, stride_s);
-            else rows_depth_attention<true>(M, ph.layer, ph.depth_pos, r0, n_live, rows_s, stride_s);
+            uint16_t* copy = block == 0 ? M.attn + (size_t)(uint32_t)(r0 * K) : nullptr;
+            if (ph.depth_pos < 8) rows_depth_attention<false>(M, ph.layer, ph.depth_pos, r0, n_live, rows_s, stride_s, copy);
+            else rows_depth_attention<true>(M, ph.layer, ph.depth_pos, r0, n_live, rows_s, stride_s, copy);
             __syncthreads();
         } else if (lane == 0) {
             if (warp < n_live) {

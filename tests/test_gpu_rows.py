@@ -127,3 +127,39 @@ def test_prompt_logits_equal_those_of_its_last_position_alone(name, page_size, n
     flat = lambda t: t.permute(1, 2, 3, 0, 4, 5).flatten(3, 4)[..., :n, :].contiguous().view(torch.int16)  # noqa: E731
     assert torch.equal(flat(kv), flat(kv0))
     cache.batch.release()
+
+
+def _depth_attention(q, kv, depth_pos):
+    """Attention of one depth position as the CUDA-core kernels add it up: q [B, Hq, 64], kv [B, 2, depth, Hkv, 64] bf16.  A product of
+    two bf16 numbers is exact in fp32, so an fp32 sum of products is a chain of FMAs."""
+    B, Hq, _ = q.shape
+    G = Hq // kv.shape[3]
+    q, kv = q.float(), kv.float().repeat_interleave(G, dim=3)
+    part = torch.zeros(B, Hq, depth_pos + 1, 4, device=q.device)
+    qd, kd = q.view(B, Hq, 1, 4, 16), kv[:, 0, :depth_pos + 1].transpose(1, 2).reshape(B, Hq, depth_pos + 1, 4, 16)
+    for e in range(16):
+        part = part + qd[..., e] * kd[..., e]
+    score = ((part[..., 0] + part[..., 1]) + (part[..., 2] + part[..., 3])) * 0.125
+    p = torch.exp(score - score.amax(-1, keepdim=True))
+    row = torch.zeros(B, Hq, 16, device=q.device)
+    row[..., :depth_pos + 1] = p
+    row = row[..., :8] + row[..., 8:]
+    for _ in range(3):
+        row = row[..., 0::2] + row[..., 1::2]
+    p = p.to(torch.bfloat16).float()
+    o = torch.zeros(B, Hq, 64, device=q.device)
+    for j in range(depth_pos + 1):
+        o = o + p[..., j, None] * kv[:, 1, j]
+    return (o * (1.0 / row)).to(torch.bfloat16)
+
+
+@pytest.mark.parametrize("name", ["long_chains", "ragged_heads", "deep", "70m"])    # 4, 1, 2 and 3 query heads per kv head
+@pytest.mark.parametrize("batch", [9, 40, 150])
+def test_depth_attention_adds_up_as_the_cuda_core_kernels_do(name, batch):
+    cfg, model = _model(name, batch, 64)
+    _frame(cfg, model, [1 + b % 50 for b in range(batch)], list(range(batch)), 9)
+    Hq, Hkv, last = cfg.fast_n_head, cfg.fast_n_local_heads, cfg.max_fast_seqlen - 1
+    q = model.debug_buffer("q", batch).view(batch, Hq, 64)
+    kv = model.debug_buffer("fkv", batch).view(batch, cfg.n_fast_layer, 2, -1, Hkv, 64)[:, -1]
+    got = model.debug_buffer("attn", batch).view(batch, Hq, 64)
+    assert torch.equal(got.view(torch.int16), _depth_attention(q, kv, last).view(torch.int16))

@@ -181,9 +181,11 @@ int smol_run_phases(SmolModel* m, const SmolBatch* b, int32_t batch, const SmolS
 int32_t smol_phase_count(const SmolModel* m);
 
 /* Per-phase timing (profiling aid): d_phase_ns [2 * 512 + 64] uint64 accumulators, zeroed by the
- * caller; CTA 0 adds [2p] = ns it spent inside phase p and [2p+1] = ns it then waited at the grid
- * barrier; [1024 + 4 * (kind + 8 * fast) + s] = ns in segment s (prologue, weight-stage wait,
- * GEMV + epilogue, closing block barrier) of the weight phases.  NULL switches it off. */
+ * caller; CTA 0 adds [2p] = ns it spent inside phase p, without its waits at grid barriers, and [2p+1] = ns of its arrival and
+ * wait at the barrier behind it and at those inside it; [1024 + 4 * (kind + 8 * fast) + s] = ns in segment s of the weight
+ * phases -- CUDA cores: prologue, weight-stage wait, GEMV + epilogue, closing block barrier; groups of rows: rows in place, norm,
+ * MMAs, sums + epilogue; 128-row tiles: row steps around them, a prompt's last position, copies + MMAs, epilogue.  A prompt's LM
+ * head is phase 5 * n_layer.  NULL switches it off. */
 int smol_set_profile(SmolModel* m, uint64_t* d_phase_ns);
 
 /* Per-frame clock (the "p50 per-frame latency at bs=1" of BASELINE.json): d_frame_ns [capacity] uint64; after frame f of

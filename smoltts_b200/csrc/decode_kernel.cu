@@ -849,7 +849,7 @@ __device__ void phase_sample(const DevModel& M, const CallArgs& A, const Ctx& c,
 }
 
 // BT == 0: the tensor-core variant (rows_phases.cuh) for 9 and more rows.
-template <int BT>
+template <int BT, bool kTimed>
 __device__ __forceinline__ void run_phase(const DevModel& M, const CallArgs& A, const Ctx& c, const Phase& ph,
                                           uint32_t& parity, RowsSync& sy, uint32_t packed_phase, const RowsStep* step) {
     if (BT == 0) {
@@ -859,7 +859,7 @@ __device__ __forceinline__ void run_phase(const DevModel& M, const CallArgs& A, 
             rows_sync_in(M, sy);
             phase_sample(M, A, c, ph);
         } else {
-            phase_rows(M, A, c, packed_phase, sy, step);
+            phase_rows<kTimed>(M, A, c, packed_phase, sy, step);
         }
         return;
     }
@@ -879,7 +879,8 @@ __device__ __forceinline__ bool next_weight_phase(const DevModel& M, const CallA
     }
 }
 
-template <int BT>
+// kTimed (BT 0): the build that a profiled launch takes.
+template <int BT, bool kTimed = false>
 __global__ void __launch_bounds__(kThreads, 1)
 smol_decode_kernel(const __grid_constant__ DevModel M, const __grid_constant__ CallArgs A, const int xs_bytes) {
     extern __shared__ __align__(1024) unsigned char smem_dyn[];
@@ -904,7 +905,7 @@ smol_decode_kernel(const __grid_constant__ DevModel M, const __grid_constant__ C
     uint32_t parity = 0;
     const int per_iter = (A.mode == 1) ? phases_per_prefill_step(M.n_layer)
                                        : phases_per_frame(M.n_layer, M.n_flayer, M.depth);
-    const bool prof_cta = (M.prof != nullptr) && c.cta == 0;  // CTA-uniform
+    const bool prof_cta = (BT == 0 ? kTimed : M.prof != nullptr) && c.cta == 0;  // CTA-uniform
     const bool prof = prof_cta && c.tid == 0;
     unsigned long long t0 = 0, t1 = 0;
     RowsSync sy;
@@ -931,13 +932,13 @@ smol_decode_kernel(const __grid_constant__ DevModel M, const __grid_constant__ C
                 }
                 st_it = it; st_p = p;
             }
+            if (BT == 0) sy.phase = p;
             if (BT == 0 && has_w) {   // the tiles of the next weight phase are fetched from inside this one
                 int nit = it, np = p;
-                sy.phase = p;
                 sy.next = next_weight_phase(M, A, nit, np) ? np : -1;
                 if (sy.next >= 0) { st_it = nit; st_p = np; }
             }
-            run_phase<BT>(M, A, c, ph, parity, sy, packed_phase, step);
+            run_phase<BT, kTimed>(M, A, c, ph, parity, sy, packed_phase, step);
             if (prof_cta) {
                 __syncthreads();
                 if (prof) t1 = globaltimer_ns();
@@ -959,8 +960,11 @@ smol_decode_kernel(const __grid_constant__ DevModel M, const __grid_constant__ C
             const bool last = (it == A.n_iter - 1) && (p == A.phase_end - 1);
             const bool sync = A.cooperative && !last;
             if (BT == 0) {
-                if (prof) { M.prof[2 * p] += t1 - t0; sy.waits_for = p; }
                 if (sync) rows_arrive(M, c, sy);
+                if (prof) {   // [2p]: rows_sync_in takes the waits inside the phase off; [2p + 1]: the arrival, then the wait, which the phase behind adds
+                    M.prof[2 * p] += t1 - t0;
+                    M.prof[2 * p + 1] += globaltimer_ns() - t1;
+                }
                 continue;
             }
             if (sync) grid_arrive(M.barrier, target, (uint32_t)c.n_ctas);
@@ -1154,9 +1158,9 @@ void rows_plan(const DevModel& M, int rows, int n_ctas, RowsPlan (*plan)[6]) {
 
 // Kernel variant by batch tile (sequences whose activations share one pass over the weights).
 static int tile_index(int bt) { return bt <= 0 ? 4 : bt <= 1 ? 0 : bt <= 2 ? 1 : bt <= 4 ? 2 : 3; }  // bt 0: tensor-core variant
-static const void* decode_fn(int bt) {
+static const void* decode_fn(int bt, bool timed = false) {
     switch (tile_index(bt)) {
-        case 4: return (const void*)smol_decode_kernel<0>;
+        case 4: return timed ? (const void*)smol_decode_kernel<0, true> : (const void*)smol_decode_kernel<0>;
         case 0: return (const void*)smol_decode_kernel<1>;
         case 1: return (const void*)smol_decode_kernel<2>;
         case 2: return (const void*)smol_decode_kernel<4>;
@@ -1171,6 +1175,7 @@ cudaError_t decode_configure(int bt, size_t smem) {
     size_t& cur = g_smem_configured[tile_index(bt)];
     if (smem <= cur) return cudaSuccess;
     cudaError_t e = cudaFuncSetAttribute(decode_fn(bt), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e == cudaSuccess && bt == 0) e = cudaFuncSetAttribute(decode_fn(bt, true), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e == cudaSuccess) cur = smem;
     return e;
 }
@@ -1179,22 +1184,29 @@ cudaError_t decode_max_ctas(int bt, size_t smem, int* per_sm) {
     return cudaOccupancyMaxActiveBlocksPerMultiprocessor(per_sm, decode_fn(bt), kThreads, smem);
 }
 
+static const void* prompt_fn(bool wide, bool timed) {
+    if (wide) return timed ? (const void*)smol_wide_kernel<true> : (const void*)smol_wide_kernel<false>;
+    return timed ? (const void*)smol_prompt_kernel<true> : (const void*)smol_prompt_kernel<false>;
+}
 cudaError_t prompt_configure(int* per_sm) {
-    cudaError_t e = cudaFuncSetAttribute(smol_wide_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kPrSmem);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(smol_prompt_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kPrSmem);
-    return e != cudaSuccess ? e : cudaOccupancyMaxActiveBlocksPerMultiprocessor(per_sm, smol_prompt_kernel, kThreads, kPrSmem);
+    for (int i = 0; i < 4; ++i) {
+        const cudaError_t e = cudaFuncSetAttribute(prompt_fn(i & 1, i >> 1), cudaFuncAttributeMaxDynamicSharedMemorySize, kPrSmem);
+        if (e != cudaSuccess) return e;
+    }
+    return cudaOccupancyMaxActiveBlocksPerMultiprocessor(per_sm, prompt_fn(false, false), kThreads, kPrSmem);
 }
 cudaError_t prompt_launch(const DevModel& M, const CallArgs& A, bool wide, int n_ctas, cudaStream_t stream) {
     void* args[2] = {(void*)&M, (void*)&A};
-    return cudaLaunchCooperativeKernel(wide ? (const void*)smol_wide_kernel : (const void*)smol_prompt_kernel, dim3(n_ctas), dim3(kThreads), args, kPrSmem, stream);
+    return cudaLaunchCooperativeKernel(prompt_fn(wide, M.prof != nullptr), dim3(n_ctas), dim3(kThreads), args, kPrSmem, stream);
 }
 
 cudaError_t decode_launch(const DevModel& M, const CallArgs& A, int bt, int n_ctas, size_t smem, int xs_bytes,
                           cudaStream_t stream) {
     void* args[3] = {(void*)&M, (void*)&A, (void*)&xs_bytes};
+    const void* fn = decode_fn(bt, M.prof != nullptr);
     if (A.cooperative)
-        return cudaLaunchCooperativeKernel(decode_fn(bt), dim3(n_ctas), dim3(kThreads), args, smem, stream);
-    return cudaLaunchKernel(decode_fn(bt), dim3(n_ctas), dim3(kThreads), args, smem, stream);
+        return cudaLaunchCooperativeKernel(fn, dim3(n_ctas), dim3(kThreads), args, smem, stream);
+    return cudaLaunchKernel(fn, dim3(n_ctas), dim3(kThreads), args, smem, stream);
 }
 
 }  // namespace smol

@@ -264,7 +264,7 @@ __device__ __noinline__ void row_wide(const DevModel& M, int row, int layer, int
 
 // One weight phase; on return the CTA has finished its units, the barrier behind it is the caller's.  kWide: of a decode frame (the
 // depth transformer's phases and the heads exist, no row stands for a last position), else of a prompt.
-template <bool kWide>
+template <bool kWide, bool kTimed>
 __device__ __noinline__ void prompt_gemm(const DevModel& M, const CallArgs& A, const Ctx& c, const Phase& ph, RowsSync& sy, uint32_t& chunk, uint32_t& tile, const int last_row) {
     const int kind = ph.kind;
     const bool fast = kWide && ph.fast != 0;
@@ -364,11 +364,15 @@ __device__ __noinline__ void prompt_gemm(const DevModel& M, const CallArgs& A, c
         constexpr int kParts = kWarps / 4 - 1;
         const uint32_t base = g_pr.tmem_base + ((uint32_t)(quad * 32) << 16);
         uint32_t t = tile;
+        const bool prof = kTimed && c.cta == 0 && c.tid == kPrEpilogueWarp * 32;   // segments: last position | copies and MMAs | accumulators
+        unsigned long long stamp = 0ull;
+        if (prof) stamp = globaltimer_ns();
         if (u_first < u_end) {
             if (kind == PH_W2) row_wide(M, last_row, ph.layer, u_first, u_step, u_end, lane);
             else row_narrow(M, A, kind, ph.layer, last_row, u_first, u_step, u_end, lane);
         }
         __syncwarp();
+        if (prof) rows_stamp(M, kind, ph.fast, 1, stamp);
         for (int u = c.cta; u < n_units; u += c.n_ctas, ++t) {
             int m0, ks, n0;
             place(u, m0, ks, n0);
@@ -383,6 +387,7 @@ __device__ __noinline__ void prompt_gemm(const DevModel& M, const CallArgs& A, c
             umma::bar_wait(&g_pr.acc_full, t & 1u);
             __syncwarp();
             umma::fence_after_sync();
+            if (prof) rows_stamp(M, kind, ph.fast, 2, stamp);
             for (int cg = part; cg * 8 < blk; cg += kParts) {
                 float acc[8], up[8];
                 __syncwarp();
@@ -446,6 +451,7 @@ __device__ __noinline__ void prompt_gemm(const DevModel& M, const CallArgs& A, c
             umma::fence_before_sync();
             __syncwarp();
             if (lane == 0) bar_arrive(&g_pr.acc_empty);
+            if (prof) rows_stamp(M, kind, ph.fast, 3, stamp);
         }
     }
     __syncwarp();
@@ -498,6 +504,20 @@ __device__ __forceinline__ void prompt_setup(const DevModel& Mp, const CallArgs&
     sy.target = ldcg_u32(Mp.barrier + 1); sy.par_w = 0; sy.par_x = 0; sy.pending = false; sy.phase = 0; sy.next = -1; sy.waits_for = 0;
 }
 
+// The phase recorder (thread 0 of CTA 0, profiling builds): a phase's time without its waits (rows_sync_in takes them off), the
+// arrival behind it, and the row steps around its tiles as segment 0.
+template <bool kTimed>
+struct PhaseTimer {
+    bool on;
+    unsigned long long t0, t1, ts;
+    __device__ __forceinline__ explicit PhaseTimer(const Ctx& c) : on(kTimed && c.cta == 0 && c.tid == 0) { if (on) t0 = globaltimer_ns(); }
+    __device__ __forceinline__ void rest() { if (on) ts = globaltimer_ns(); }
+    __device__ __forceinline__ void step(const DevModel& M, const Phase& ph) { if (on) rows_stamp(M, ph.kind, ph.fast, 0, ts); }
+    __device__ __forceinline__ void end(const DevModel& M, int p) { if (on) { t1 = globaltimer_ns(); M.prof[2 * p] += t1 - t0; } }
+    __device__ __forceinline__ void arrived(const DevModel& M, int p) { if (on) { t0 = globaltimer_ns(); M.prof[2 * p + 1] += t0 - t1; } }
+};
+
+template <bool kTimed>
 __global__ void __launch_bounds__(kThreads, 1)
 smol_prompt_kernel(const __grid_constant__ DevModel Mp, const __grid_constant__ CallArgs Ap) {
     extern __shared__ __align__(1024) unsigned char smem_dyn[];
@@ -511,22 +531,29 @@ smol_prompt_kernel(const __grid_constant__ DevModel Mp, const __grid_constant__ 
         c.iter = it;
         const bool last_iter = it == A.n_iter - 1;
         const int last_row = last_iter && A.whole_prompt > 0 ? A.head_row : -1;
+        sy.phase = 0;
+        PhaseTimer<kTimed> timer(c);
         rows_sync_in(M, sy);
+        timer.rest();
         prompt_row_step(M, A, c, M.dim, M.x, M.layers[0].attention_norm, [&](int bg, int ch, float (&x)[8]) { embed_chunk(M, A, c, bg, ch, x); });
+        timer.step(M, unpack_phase(M.prog[0]));
         rows_arrive(M, c, sy);
         for (int p = 0; p < phases_per_prefill_step(M.n_layer); ++p) {
             const Phase ph = unpack_phase(M.prog[p]);
+            sy.phase = p;
             if (ph.kind == PH_ATTN) {
                 rows_sync_in(M, sy);
                 prompt_attn(M, A, c, ph, sy, Ap.kv_map, last_row);
             } else {
-                prompt_gemm<false>(M, A, c, ph, sy, chunk, tile, last_row);
+                prompt_gemm<false, kTimed>(M, A, c, ph, sy, chunk, tile, last_row);
                 if (ph.kind == PH_WO || ph.kind == PH_W2) {   // h = stream + wo(attn) (P:499); stream = h + w2(act) (P:500); and the norm of the phase that reads it
                     rows_arrive(M, c, sy);
                     rows_sync_in(M, sy);
+                    timer.rest();
                     const bool wo = ph.kind == PH_WO;
                     const uint16_t* norm = wo ? M.layers[ph.layer].ffn_norm : ph.layer + 1 < M.n_layer ? M.layers[ph.layer + 1].attention_norm : M.norm;
                     prompt_finish(M, A, c, wo ? M.x : M.h, wo ? M.h : M.x, M.dim, prompt_slices(wo ? M.dim : M.inter), norm, last_row);
+                    timer.step(M, ph);
                 }
             }
             if (p == phases_per_prefill_step(M.n_layer) - 1 && c.cta == 0) {
@@ -538,10 +565,14 @@ smol_prompt_kernel(const __grid_constant__ DevModel Mp, const __grid_constant__ 
                     if (n_act) A.b.seq_len[b] = ldcg_i32(A.b.seq_len + b) + n_act;
                 }
             }
+            timer.end(M, p);
             if (!(last_iter && A.whole_prompt == 0 && p == phases_per_prefill_step(M.n_layer) - 1)) rows_arrive(M, c, sy);
+            timer.arrived(M, p);
         }
     }
     if (A.whole_prompt > 0) {
+        sy.phase = 5 * M.n_layer;        // the LM head's
+        PhaseTimer<kTimed> timer(c);
         rows_sync_in(M, sy);
         if (c.cta == 0 && A.head_row > 0)      // the last position's hidden state (pre-norm) -> row 0
             for (int i = c.tid; i < M.dim / 8; i += kThreads) *reinterpret_cast<uint4*>(M.x + i * 8) = ldcg_v4(M.x + (size_t)A.head_row * M.dim + i * 8);
@@ -551,6 +582,7 @@ smol_prompt_kernel(const __grid_constant__ DevModel Mp, const __grid_constant__ 
             row_fetch(M, PH_HEAD, 0, u, c.lane, w, w);
             row_finish(M, A, PH_HEAD, 0, A.head_row, u, c.lane, w, w, x, 0, -1, 0u);
         }
+        timer.end(M, sy.phase);
     }
     if (c.cta == 0) {
         // leave the last prompt column as the pending input of the first decode frame (G:66-73)
@@ -598,6 +630,7 @@ __device__ __noinline__ void wide_input(const DevModel& M, const CallArgs& A, co
 }
 __device__ __noinline__ void wide_sample(const DevModel& M, const CallArgs& A, const Ctx& c, const Phase& ph) { phase_sample(M, A, c, ph); }
 
+template <bool kTimed>
 __global__ void __launch_bounds__(kThreads, 1)
 smol_wide_kernel(const __grid_constant__ DevModel Mp, const __grid_constant__ CallArgs Ap) {
     extern __shared__ __align__(1024) unsigned char smem_dyn[];
@@ -607,13 +640,13 @@ smol_wide_kernel(const __grid_constant__ DevModel Mp, const __grid_constant__ Ca
     RowsSync sy;
     prompt_setup(Mp, Ap, smem_dyn, c, sy);
     uint32_t chunk = 0, tile = 0;
-    const bool prof = M.prof != nullptr && c.cta == 0 && c.tid == 0;   // per phase: its time, and (in it) the wait for the one before
+    PhaseTimer<kTimed> timer(c);
     for (int it = 0; it < A.n_iter; ++it) {
         c.iter = it;
         for (int p = A.phase_begin; p < A.phase_end; ++p) {
             const Phase ph = unpack_phase(M.prog[p]);
             const bool fast = ph.fast != 0;
-            const unsigned long long t0 = prof ? globaltimer_ns() : 0ull;
+            sy.phase = p;
             if (ph.kind == PH_ATTN) {
                 wide_attn(M, A, c, ph, sy, Ap.kv_map);
             } else if (ph.kind == PH_SAMPLE) {
@@ -623,28 +656,32 @@ smol_wide_kernel(const __grid_constant__ DevModel Mp, const __grid_constant__ Ca
                 const bool input = ph.kind == PH_QKV && ph.layer == 0, depth_attn = ph.kind == PH_WO && fast;
                 if (input || depth_attn) {
                     rows_sync_in(M, sy);
+                    timer.rest();
                     if (input) wide_input(M, A, c, ph);
                     else wide_depth_attention(M, A, c, ph.layer, ph.depth_pos);
+                    timer.step(M, ph);
                     rows_arrive(M, c, sy);
                 }
                 if (ph.kind == PH_QKV && !fast) attn_prefetch(M, A, c, ph.layer);
-                prompt_gemm<true>(M, A, c, ph, sy, chunk, tile, -1);
+                prompt_gemm<true, kTimed>(M, A, c, ph, sy, chunk, tile, -1);
                 if (ph.kind == PH_WO || ph.kind == PH_W2) {
                     rows_arrive(M, c, sy);
                     rows_sync_in(M, sy);
+                    timer.rest();
                     const bool wo = ph.kind == PH_WO;
                     const DevLayer* L = fast ? M.fast_layers : M.layers;
                     uint16_t* stream = fast ? M.xf : M.x;
                     const uint16_t* norm = wo ? L[ph.layer].ffn_norm : ph.layer + 1 < (fast ? M.n_flayer : M.n_layer) ? L[ph.layer + 1].attention_norm : fast ? M.fast_norm : M.norm;
                     const int D = fast ? M.fdim : M.dim;
                     prompt_finish(M, A, c, wo ? stream : M.h, wo ? M.h : stream, D, prompt_slices(wo ? D : fast ? M.finter : M.inter), norm, -1);
+                    timer.step(M, ph);
                 }
             }
             if (c.cta == 0 && A.advance && p == A.phase_end - 1)
                 for (int b = c.tid; b < A.batch; b += kThreads) A.b.seq_len[b] = ldcg_i32(A.b.seq_len + b) + 1;
-            sy.waits_for = p;
-            if (prof) M.prof[2 * p] += globaltimer_ns() - t0;
+            timer.end(M, p);
             if (!(it == A.n_iter - 1 && p == A.phase_end - 1)) rows_arrive(M, c, sy);
+            timer.arrived(M, p);
         }
     }
     if (c.cta == 0 && c.tid == 0) M.barrier[1] = sy.target;

@@ -64,7 +64,7 @@ struct RowsSync {
     uint32_t par_w, par_x;   // parities of the weight and the row copies
     bool pending;
     int phase, next;         // this phase; the launch's next weight phase (-1: none), whose tiles this one fetches
-    int waits_for;           // profiling: the phase whose barrier is pending
+    int waits_for;           // the phase whose barrier is pending
 };
 __device__ __forceinline__ void rows_sync_in(const DevModel& M, RowsSync& sy) {
     if (!sy.pending) return;
@@ -73,16 +73,27 @@ __device__ __forceinline__ void rows_sync_in(const DevModel& M, RowsSync& sy) {
     if (prof) t = globaltimer_ns();
     grid_wait(M.barrier, sy.target);
     sy.pending = false;
-    if (prof) M.prof[2 * sy.waits_for + 1] += globaltimer_ns() - t;
+    if (prof) {   // belongs to the phase in front of the barrier, not to the one that waits
+        t = globaltimer_ns() - t;
+        M.prof[2 * sy.waits_for + 1] += t;
+        M.prof[2 * sy.phase] -= t;
+    }
+}
+// Profiling: ns in segment s of a weight phase's body (CTA 0, one thread), from the last stamp on.
+__device__ __forceinline__ void rows_stamp(const DevModel& M, int kind, int fast, int s, unsigned long long& t) {
+    const unsigned long long now = globaltimer_ns();
+    M.prof[2 * kMaxProg + (kind + 8 * fast) * 4 + s] += now - t;
+    t = now;
 }
 __device__ __forceinline__ void rows_arrive(const DevModel& M, const Ctx& c, RowsSync& sy) {
-    rows_sync_in(M, sy);       // (every phase has waited already: a CTA never arrives twice in a row)
+    rows_sync_in(M, sy);       // (a phase in which this CTA has no work may not have waited yet)
     // Shared memory used here is overwritten by copies.  (Rows written here are read by other CTAs' copies: the threads that issue those
     // fence global memory behind the barrier; a full fence.proxy.async here waits for
     // the stores of every thread: frames of 9 / 64 rows 1263 / 1520 us with it, 1188 / 1437 without.)
     fence_proxy_async();
     grid_arrive(M.barrier, sy.target, (uint32_t)c.n_ctas);
     sy.pending = true;
+    sy.waits_for = sy.phase;
 }
 
 // ---- batch attention on the tensor cores -------------------------------------------------------------------------
@@ -700,7 +711,8 @@ constexpr int kNormSteps = 3;   // RMSNorm of a row by a warp: 256 elements per 
 // (K steps 0, 4, 8 .. of 16 elements; 1, 5, 9 ..; ..) for each K slice: one slice, or four for wo and w2.  Without slices the
 // warps are the four chains x 4, which take every fourth tile; with slices a warp is one chain and takes all tiles.  The one
 // tile of a w2 block sits in registers.
-template <int kind, bool kDepthAttn, int NT>
+// kTimed: the profiling build of the kernel, which stamps rows in place | normed | chains | sums and epilogue.
+template <int kind, bool kDepthAttn, int NT, bool kTimed>
 __device__ __forceinline__ void rows_gemm(const DevModel& M, const CallArgs& A, const int iter, const uint32_t packed_phase, const RowsStep* step,
                                           unsigned char* stage, float* P, RowsSync& sy) {
     constexpr bool wide = kind == PH_W2;
@@ -758,6 +770,9 @@ __device__ __forceinline__ void rows_gemm(const DevModel& M, const CallArgs& A, 
         }
         if (!wide && !landed) { rows_wait(&g_mbar[0], sy.par_w); sy.par_w ^= 1u; landed = true; }
         rows_sync_in(M, sy);
+        const bool timed = kTimed && blockIdx.x == 0 && tid == 0;
+        unsigned long long stamp = 0ull;
+        if (timed) stamp = globaltimer_ns();
         // ---- the group's rows: bulk copies into shared memory (contiguous 16-byte loads take 3400 clocks for 96 KB on every SM
         // at once, loads straight into fragments -- 64 bytes of 8 rows each -- 7000, bulk copies 2000) ----
         if (kDepthAttn) {
@@ -798,6 +813,7 @@ __device__ __forceinline__ void rows_gemm(const DevModel& M, const CallArgs& A, 
                 pre = ldcg_u32(rk.res + (size_t)(uint32_t)((r0 + row) * rk.n_out + ((block * rk.mt + t) * 16 + (item_w(tid) & ~1))));
         }
         if (!kDepthAttn) { rows_wait(&g_mbar[1], sy.par_x); sy.par_x ^= 1u; }
+        if (timed) rows_stamp(M, kind, ph.fast, 0, stamp);
         if (normed) {
             // a warp per row, two at a time: their chains of shuffles and divisions run side by side
             constexpr int NR = N > kWarps ? 2 : 1;
@@ -857,6 +873,7 @@ __device__ __forceinline__ void rows_gemm(const DevModel& M, const CallArgs& A, 
                     pre = __ldg(reinterpret_cast<const uint32_t*>((fast ? M.fast_rope : M.rope) + (size_t)(fast ? ph.depth_pos : min(g_rpos[row], M.max_seq_len - 1)) * kHeadDim + (u0 & (kHeadDim - 1))));
             }
         }
+        if (timed) rows_stamp(M, kind, ph.fast, 1, stamp);
         // ---- the warp's chains (columns past the group repeat its last row: nobody reads their sums) ----
         float acc[TW][NT][4];
 #pragma unroll
@@ -899,6 +916,7 @@ __device__ __forceinline__ void rows_gemm(const DevModel& M, const CallArgs& A, 
         const bool last_rows = r0 + rk.gstep * rk.n >= rk.rows;
         const int next_block = block + (rk.blocks <= (int)gridDim.x ? rk.blocks : (int)gridDim.x);
         __syncthreads();   // the rows have been read: their place takes the partial sums
+        if (timed) rows_stamp(M, kind, ph.fast, 2, stamp);
         if (!idle) {
 #pragma unroll
             for (int t = 0; t < TW; ++t) {
@@ -995,6 +1013,7 @@ __device__ __forceinline__ void rows_gemm(const DevModel& M, const CallArgs& A, 
                                              + (size_t)(p & (ps - 1)) * kHeadDim + d) = packed;
             }
         }
+        if (timed) rows_stamp(M, kind, ph.fast, 3, stamp);
         if (!last_rows || next_block < rk.blocks) {   // the partial sums are overwritten, by copies
             fence_proxy_async();
             __syncthreads();
@@ -1009,6 +1028,7 @@ __device__ __forceinline__ void rows_gemm(const DevModel& M, const CallArgs& A, 
 
 // One weight phase: the kernel form its plan names.  The CTA's first tiles are on their way (`step`); the tiles of
 // the launch's next weight phase are fetched as soon as these are used up.
+template <bool kTimed>
 __device__ __forceinline__ void phase_rows(const DevModel& M, const CallArgs& A, const Ctx& c, uint32_t packed_phase, RowsSync& sy, const RowsStep* step) {
     const Phase ph = unpack_phase(packed_phase);
     if (tc_has_prestep(ph)) {
@@ -1026,17 +1046,17 @@ __device__ __forceinline__ void phase_rows(const DevModel& M, const CallArgs& A,
     const int n = g_rk[ph.fast][ph.kind].n;
 #define ROWS_ARGS M, A, c.iter, packed_phase, step, c.stage, c.xs, sy
 #define ROWS_CASE(kind, attn) \
-    if (n <= 8) rows_gemm<kind, attn, 1>(ROWS_ARGS); \
-    else if (n <= 16) rows_gemm<kind, attn, 2>(ROWS_ARGS); \
-    else rows_gemm<kind, attn, 4>(ROWS_ARGS);
+    if (n <= 8) rows_gemm<kind, attn, 1, kTimed>(ROWS_ARGS); \
+    else if (n <= 16) rows_gemm<kind, attn, 2, kTimed>(ROWS_ARGS); \
+    else rows_gemm<kind, attn, 4, kTimed>(ROWS_ARGS);
     switch (ph.kind) {
         case PH_QKV: ROWS_CASE(PH_QKV, false) break;
         case PH_W13: ROWS_CASE(PH_W13, false) break;
         case PH_HEAD: ROWS_CASE(PH_HEAD, false) break;
         case PH_W2:
-            if (n <= 8) rows_gemm<PH_W2, false, 1>(ROWS_ARGS);
-            else if (n <= 16) rows_gemm<PH_W2, false, 2>(ROWS_ARGS);
-            else rows_gemm<PH_W2, false, 3>(ROWS_ARGS);
+            if (n <= 8) rows_gemm<PH_W2, false, 1, kTimed>(ROWS_ARGS);
+            else if (n <= 16) rows_gemm<PH_W2, false, 2, kTimed>(ROWS_ARGS);
+            else rows_gemm<PH_W2, false, 3, kTimed>(ROWS_ARGS);
             break;
         default:
             if (ph.fast) { ROWS_CASE(PH_WO, true) }

@@ -163,3 +163,44 @@ def test_depth_attention_adds_up_as_the_cuda_core_kernels_do(name, batch):
     kv = model.debug_buffer("fkv", batch).view(batch, cfg.n_fast_layer, 2, -1, Hkv, 64)[:, -1]
     got = model.debug_buffer("attn", batch).view(batch, Hq, 64)
     assert torch.equal(got.view(torch.int16), _depth_attention(q, kv, last).view(torch.int16))
+
+
+@pytest.mark.parametrize("what", ["frames of 12", "frames of 160", "prompt"])
+def test_phase_recorder_covers_the_launch_once(what):
+    """Work and waits are disjoint and belong to their own phases: together they are what the launch takes, and no phase in it is empty."""
+    n = 160 if what.endswith("160") else 12 if what.startswith("frames") else 1
+    cfg, model = _model("70m", n, 200)
+    batch = model.new_batch(n, max_positions=190, max_frames=4)
+    prompt = prompt_grid(byte_prompt(88, seed=1), cfg)[None].to(device="cuda", dtype=torch.int32)
+    model.set_option("ll_max_batch", 0)
+    frames = 4
+
+    def run():
+        batch.seq_len.zero_()
+        batch.step.zero_()
+        batch.host_len = [0] * n
+        if what == "prompt":
+            model.forward_generate(prompt, type("Cache", (), {"batch": batch}))
+        else:
+            model.decode_frames(batch, model.sampling(ignore_stop=True), frames)
+
+    run()
+    prof = model.set_profile(True)
+    run()
+    torch.cuda.synchronize()
+    prof.zero_()
+    begin, end = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+    begin.record()
+    run()
+    end.record()
+    torch.cuda.synchronize()
+    ns = prof[:1024].view(512, 2).cpu()
+    model.set_profile(False)
+    last = 5 * cfg.n_layer if what == "prompt" else model.phase_count - 1
+    first = [i for i in range(last + 1)]
+    assert (ns >= 0).all() and (ns[first, 0] > 0).all() and (ns[first[:-1], 1] > 0).all() and ns[last + 1:].sum() == 0
+    wall = begin.elapsed_time(end) * 1e6
+    # CTA 0's clock against events around the call's launches and copies: what is recorded twice or not at all would be a third of it
+    assert 0.6 * wall < ns.sum().item() < 1.02 * wall, (ns.sum().item(), wall)
+    # waits of many barriers, not of one
+    assert ns[:, 1].max() < 0.25 * ns[:, 1].sum()

@@ -1,8 +1,9 @@
 #!/usr/bin/env python
-"""Per-phase time breakdown of the persistent decode kernels: the barrier kernel accumulates %globaltimer per phase
-(CTA 0); the data-flow kernel (bs=1, default) records a %clock64 trace of the last frame (CTA 0 and CTA n/2).
+"""Per-phase time breakdown of the persistent decode kernels: the barrier kernel and its tensor-core variants accumulate
+%globaltimer per phase (CTA 0); the data-flow kernel (bs=1, default) records a %clock64 trace of the last frame (CTA 0 and CTA n/2).
 
 usage: python tools/phase_profile.py [--model smoltts_byte_150m] [--batch 1] [--frames 256] [--out profiles/x.json]
+       python tools/phase_profile.py --what prompt | prefill --prompt-bytes 200 [--batch 8]     (forward_generate | prefill, per call)
 """
 from __future__ import annotations
 
@@ -11,6 +12,7 @@ import collections
 import json
 import os
 import sys
+import types
 
 sys.path.insert(0, os.path.dirname(os.path.dirname(os.path.abspath(__file__))))
 
@@ -44,6 +46,7 @@ def main():
     ap.add_argument("--batch", type=int, default=1)
     ap.add_argument("--frames", type=int, default=256)
     ap.add_argument("--prompt-bytes", type=int, default=200)
+    ap.add_argument("--what", choices=["frames", "prompt", "prefill"], default="frames")
     ap.add_argument("--sampled", action="store_true")
     ap.add_argument("--out", default=None)
     ap.add_argument("--repeat", type=int, default=0, help="profiling: run every weight-phase body 1+repeat times")
@@ -62,18 +65,32 @@ def main():
     gs = (GenerationSettings(default_temp=0.7, default_fast_temp=0.7, top_k=50, top_p=0.9, seed=1234) if a.sampled
           else GenerationSettings(default_temp=0.0, default_fast_temp=0.0))
     s = _sampling(model, gs, True, ignore_stop=True)
+    calls = a.frames if a.what == "frames" else 8
+
+    def run(n):
+        if a.what == "frames":
+            model.decode_frames(batch, s, n)
+            return
+        for _ in range(n):
+            batch.seq_len.zero_()
+            batch.host_len = [0] * a.batch
+            if a.what == "prefill":
+                model.prefill(batch, padded, lens)
+            else:
+                model.forward_generate(padded[:1], types.SimpleNamespace(batch=batch))
+
     model.prefill(batch, padded, lens)
-    model.decode_frames(batch, s, 8)  # warm
+    run(min(8, calls))  # warm
     torch.cuda.synchronize()
     model.set_option("repeat", a.repeat)
     prof = model.set_profile(True)
     e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
     e0.record()
-    model.decode_frames(batch, s, a.frames)
+    run(calls)
     e1.record()
     torch.cuda.synchronize()
     model.set_profile(False)
-    raw = prof.cpu().numpy().astype(float) / a.frames  # per frame
+    raw = prof.cpu().numpy().astype(float) / calls  # per frame or call
     ns = raw[: 2 * model.phase_count].reshape(-1, 2)
     seg = raw[2 * 512: 2 * 512 + 64].reshape(16, 4)
     trace = prof.cpu().numpy()[2 * 512 + 64: 2 * 512 + 64 + 2 * 512 * 8].reshape(2, 512, 8)
@@ -84,15 +101,16 @@ def main():
         w, b, n = agg.get(k, (0.0, 0.0, 0))
         agg[k] = (w + ns[p, 0], b + ns[p, 1], n + 1)
     total = ns.sum()
-    print(f"{a.model} bs={a.batch} frames={a.frames}: {e0.elapsed_time(e1) * 1e3 / a.frames:.1f} us/frame by events"
-          + (f", {total / 1e3:.1f} us/frame by in-kernel timers (CTA 0)" if total > 0 else " (profiling build of the data-flow kernel)"))
+    print(f"{a.model} bs={a.batch} {a.what}={calls}: {e0.elapsed_time(e1) * 1e3 / calls:.1f} us each by events, recorded"
+          + (f", {total / 1e3:.1f} us by in-kernel timers (CTA 0)" if total > 0 else " (profiling build of the data-flow kernel)"))
     rows = {}
     if total > 0:  # barrier kernel: globaltimer accumulators (work, barrier wait) and sub-phase segments
         print(f"{'phase':14s} {'count':>5s} {'work us':>9s} {'wait us':>9s} {'per-phase work':>15s} {'per-phase wait':>15s}")
         for k, (w, b, n) in sorted(agg.items(), key=lambda kv: -(kv[1][0] + kv[1][1])):
             print(f"{k:14s} {n:5d} {w / 1e3:9.1f} {b / 1e3:9.1f} {w / n / 1e3:15.2f} {b / n / 1e3:15.2f}")
             rows[k] = {"count": n, "work_us": w / 1e3, "wait_us": b / 1e3}
-        print("sub-phase segments of the weight phases, us per frame (CTA 0 thread 0): prologue | stage wait | gemv+epilogue | final sync")
+        print("sub-phase segments of the weight phases, us (one thread of CTA 0): CUDA cores: prologue | stage wait | gemv + epilogue | final sync; "
+              "groups of rows: rows in place | norm | MMAs | sums + epilogue; 128-row tiles: row steps | last position | copies + MMAs | epilogue")
         for k in range(16):
             if seg[k].sum() > 0:
                 name = ("fast." if k >= 8 else "slow.") + KINDS[k % 8]
@@ -145,8 +163,8 @@ def main():
                   f"{(np.mean(gp2) if gp2 else float('nan')):7.0f} | most often last: {collections.Counter(late).most_common(5)}")
     if a.out:
         with open(a.out, "w") as f:
-            json.dump({"model": a.model, "batch": a.batch, "frames": a.frames,
-                       "us_per_frame_events": e0.elapsed_time(e1) * 1e3 / a.frames, "by_phase": rows}, f, indent=1)
+            json.dump({"model": a.model, "batch": a.batch, "what": a.what, "frames": calls,
+                       "us_per_frame_events": e0.elapsed_time(e1) * 1e3 / calls, "by_phase": rows}, f, indent=1)
 
 
 if __name__ == "__main__":

@@ -184,7 +184,8 @@ int32_t smol_phase_count(const SmolModel* m);
  * caller; CTA 0 adds [2p] = ns it spent inside phase p, without its waits at grid barriers, and [2p+1] = ns of its arrival and
  * wait at the barrier behind it and at those inside it; [1024 + 4 * (kind + 8 * fast) + s] = ns in segment s of the weight
  * phases -- CUDA cores: prologue, weight-stage wait, GEMV + epilogue, closing block barrier; groups of rows: rows in place, norm,
- * MMAs, sums + epilogue; 128-row tiles: row steps around them, a prompt's last position, copies + MMAs, epilogue.  A prompt's LM
+ * MMAs, sums + epilogue; prompts: row steps around the tiles, the last position, copies
+ * + MMAs, epilogue; 128-row tiles (barriers inside a phase count as work there): row steps, set-up, copies + MMAs, epilogue.  A prompt's LM
  * head is phase 5 * n_layer.  NULL switches it off. */
 int smol_set_profile(SmolModel* m, uint64_t* d_phase_ns);
 
@@ -200,8 +201,12 @@ int smol_set_frame_clock(SmolModel* m, uint64_t* d_frame_ns, int32_t capacity);
  * data-flow kernel used by tools/ll_ncu.py (0 = the shipped configuration);
  * "tc_min_batch" (default 9: the measured crossover) = rows (sequences of a decode call, sequences x prompt positions of a prefill iteration)
  * from which the tensor-core variant runs, 0 = never;  "prefill_tile" = cap on the prompt positions per prefill iteration
- * (0 = as many as fit: 1024 rows on the tensor-core variant, 8 on the CUDA-core variants).
- * smol_get_option also answers "n_sms", "smem_bytes", "ll_ready", "tc_ready" (1 once the tensor-core variant has been set up). */
+ * (0 = as many as fit: 1024 rows on the tensor-core variant, 8 on the CUDA-core variants);  "tc_group_rows" = rows of a decode call up to
+ * which the tensor-core variant works in groups of rows, above which on 128-row tiles (-1, the default: whichever is expected to be faster;
+ * the results have the same bits).
+ * smol_get_option also answers "n_sms", "smem_bytes", "ll_ready", "tc_ready" (1 once the tensor-core variant has been set up),
+ * "last_kernel" (SMOL_KERNEL_* of the last launch). */
+enum { SMOL_KERNEL_NONE = 0, SMOL_KERNEL_CUDA_CORES = 1, SMOL_KERNEL_DATAFLOW = 2, SMOL_KERNEL_GROUPS = 3, SMOL_KERNEL_TILES = 4, SMOL_KERNEL_PROMPT = 5 };
 int smol_set_option(SmolModel* m, const char* name, int64_t value);
 int64_t smol_get_option(const SmolModel* m, const char* name);
 

@@ -20,7 +20,7 @@ LIB_DIR = os.path.join(PKG, "_lib")
 LIB_PATH = os.path.join(LIB_DIR, "libsmoltts_b200.so")
 STAMP = os.path.join(LIB_DIR, "build.stamp")
 SOURCES = ["decode_kernel.cu", "ll2_kernel.cu", "capi.cu", "mimi_kernels.cu"]
-HEADERS = ["common.cuh", "dev_model.h", "f32_tile.cuh", "sampler.cuh", "umma.cuh", "rows_phases.cuh", "prompt_phases.cuh", "tmap_host.h", os.path.join("..", "..", "include", "smoltts_b200.h"),
+HEADERS = ["common.cuh", "dev_model.h", "f32_tile.cuh", "sampler.cuh", "umma.cuh", "rows_phases.cuh", "tile_phases.cuh", "prompt_phases.cuh", "tmap_host.h", os.path.join("..", "..", "include", "smoltts_b200.h"),
            os.path.join("..", "..", "include", "smoltts_b200_mimi.h")]
 LM_LIB_PATH = os.path.join(LIB_DIR, "libsmoltts_b200_lm.so")
 # target -> (library, stamp, sources, headers)

@@ -17,9 +17,12 @@
 namespace smol {
 size_t decode_xs_bytes(const DevModel& M, int bt);
 size_t decode_stage_bytes(const DevModel& M, int n_ctas, int bt);
-void rows_plan(const DevModel& M, int rows, int n_ctas, RowsPlan (*plan)[6]);
+double rows_plan(const DevModel& M, int rows, int n_ctas, RowsPlan (*plan)[6]);
+double tiles_time(const DevModel& M, int rows, int n_ctas);
 cudaError_t prompt_configure(int* per_sm);
-cudaError_t prompt_launch(const DevModel& M, const CallArgs& A, bool wide, int n_ctas, cudaStream_t stream);
+cudaError_t prompt_launch(const DevModel& M, const CallArgs& A, int n_ctas, cudaStream_t stream);
+cudaError_t tiles_configure(int* per_sm);
+cudaError_t tiles_launch(const DevModel& M, const CallArgs& A, int n_ctas, cudaStream_t stream);
 int decode_batch_tile(int batch);
 cudaError_t decode_configure(int bt, size_t smem);
 cudaError_t decode_max_ctas(int bt, size_t smem, int* per_sm);
@@ -71,8 +74,10 @@ struct SmolModel {
                                // barrier kernel / its tcgen05 variant (measured at bs=8: 1.5 ms per frame step against 2.3 ms)
     smol::ll2::SmemPlan ll2_sp;
     size_t ll2_smem = 0;
+    int tc_group_rows = -1;    // rows of a decode batch up to which it runs in groups of rows (-1: in_groups decides)
+    int last_kernel = 0;       // SMOL_KERNEL_* of the last launch
     bool tmaps_ready = false;  // tensor maps of the 128-row tiles (rebuilt after a weight / workspace bind)
-    bool prompt_ready = false; // its function attributes
+    bool tiles_ready = false, prompt_ready = false;   // the kernels' function attributes
     bool packed_ready = false; // tensor-core GEMV layout of the bound weights (rebuilt after a weight / workspace bind)
     int64_t launches = 0;
     alignas(64) unsigned char kv_map[128] = {0};   // tensor map of the bound KV pool (tensor-core variant)
@@ -542,12 +547,40 @@ static bool use_tc(const SmolModel* m, int rows) {
     return m->tc_min_batch > 0 && rows >= m->tc_min_batch && tc_eligible(m->cfg);
 }
 
-// Rows of a decode batch up to which groups of 32 rows are faster than 128-row tiles (150m, us per frame): 128 rows 1986, 136
-// 2198 | 160 rows 2640, 256: 2699 on tiles (256 rows in groups 3380).
-constexpr int kWideRows = 144;
+// A decode batch runs in groups of rows (rows_phases.cuh) or, where that is faster, on 128-row tiles (tile_phases.cuh): groups are taken in turns
+// once they are more than the CTAs that share a tile block, while a frame on tiles hardly depends on its rows.  Where the line lies
+// follows from the model's widths and the grid, so it is drawn by two models of a frame's time, fitted to 43 measured pairs (150m, 70m and
+// tiny; 40 to 148 CTAs; 9 to 512 rows; caches of <= 471 positions), all of which they order as measured.
+// us, groups | tiles: 150m 136 rows 2232 | 2321, 145: 2416 | 2323, 256: 3498 | 2435; 70m 200: 2004 | 2051, 256: 2126 | 2068; tiny 512: 714 | 802;
+// 150m on 40 CTAs 24: 1823 | 2388, 33: 2792 | 2402.  A row's bits are the same on either side.
+static bool in_groups(const SmolModel* m, int rows) {
+    if (m->tc_group_rows >= 0) return rows <= m->tc_group_rows;
+    smol::RowsPlan plan[2][6];
+    return smol::rows_plan(m->dm, rows, m->n_ctas, plan) <= smol::tiles_time(m->dm, rows, m->n_ctas);
+}
+// A prefill runs on tiles, too, unless its sequences have more positions per iteration than a row tile: the prompt kernel's attention is
+// faster with many positions of a sequence, but it takes longer from phase to phase.  us, tiles | prompt kernel (150m): 1 x 128 positions
+// 640 | 697, 1 x 140: 827 | 703, 1 x 1500: 4861 | 3524, 4 x 140: 1158 | 987, 8 x 100: 1114 | 1170, 64 x 60: 4235 | 4459.
+constexpr int kPromptRows = 129;
 
-// Tiles of 128 rows: a prompt (in every mode) or frames of a wide batch, one cooperative launch.
-static int enqueue_tiles(SmolModel* m, CallArgs A, bool wide, cudaStream_t stream) {
+// Tiles of 128 rows: frames of a wide batch, and prefills; one launch, or a phase of it.
+static int launch_tiles(SmolModel* m, const CallArgs& A, int n_ctas, cudaStream_t stream) {
+    if (!m->tiles_ready) {
+        const int rc = ensure_tmaps(m);
+        if (rc) return rc;
+        int per_sm = 0;
+        CU(smol::tiles_configure(&per_sm));
+        if (per_sm < 1) return fail(SMOL_ERR_UNSUPPORTED, "tile kernel does not fit on an SM");
+        m->tiles_ready = true;
+    }
+    CU(smol::tiles_launch(m->dm, A, n_ctas, stream));
+    m->launches += 1;
+    m->last_kernel = SMOL_KERNEL_TILES;
+    return SMOL_OK;
+}
+
+// The prompt of one sequence as one cooperative launch (in every mode).
+static int enqueue_prompt(SmolModel* m, CallArgs A, cudaStream_t stream) {
     int rc = ensure_tmaps(m);
     if (rc || (rc = ensure_kv_map(m))) return rc;
     if (!m->prompt_ready) {
@@ -559,13 +592,15 @@ static int enqueue_tiles(SmolModel* m, CallArgs A, bool wide, cudaStream_t strea
     A.cooperative = 1;
     A.tc_split = m->tc_attn_split;
     std::memcpy(A.kv_map, m->kv_map, sizeof(A.kv_map));
-    CU(smol::prompt_launch(m->dm, A, wide, m->n_ctas, stream));
+    CU(smol::prompt_launch(m->dm, A, m->n_ctas, stream));
     m->launches += 1;
+    m->last_kernel = SMOL_KERNEL_PROMPT;
     return SMOL_OK;
 }
 
 static int enqueue(SmolModel* m, CallArgs A, cudaStream_t stream, bool whole_iters = false) {
-    const int bt = use_tc(m, A.batch) ? 0 : smol::decode_batch_tile(A.batch);
+    const bool tc = use_tc(m, A.batch), tiles = tc && (A.mode == 1 || !in_groups(m, A.batch));
+    const int bt = tc ? 0 : smol::decode_batch_tile(A.batch);
     int rc;
     A.repeat = m->repeat;
     A.tc_split = m->tc_attn_split;
@@ -579,33 +614,34 @@ static int enqueue(SmolModel* m, CallArgs A, cudaStream_t stream, bool whole_ite
             m->ll2_sp.flags = m->ll_flags;
             CU(smol::ll2_launch(m->dm, A, m->ll2_sp, m->ll2_smem, A.team_ctas * A.batch, stream));
             m->launches += 1;
+            m->last_kernel = SMOL_KERNEL_DATAFLOW;
             return SMOL_OK;
         }
     }
-    rc = ensure_tile(m, bt);
-    if (rc) return rc;
-    if (bt == 0 && m->mode != 1 && A.mode == 0 && A.batch > kWideRows && A.phase_begin < A.phase_end) {
-        const smol::Phase first = smol::unpack_phase(m->dm.prog[A.phase_begin]);   // (launches begin where a transformer does)
-        if (first.kind == smol::PH_QKV && first.layer == 0) return enqueue_tiles(m, A, true, stream);
+    if (!tiles) {
+        if ((rc = ensure_tile(m, bt))) return rc;
+        if (bt == 0) {
+            smol::rows_plan(m->dm, A.batch, m->n_ctas, A.rows_plan);
+            std::memcpy(A.kv_map, m->kv_map, sizeof(A.kv_map));
+        }
     }
-    if (bt == 0) {
-        smol::rows_plan(m->dm, A.batch, m->n_ctas, A.rows_plan);
-        std::memcpy(A.kv_map, m->kv_map, sizeof(A.kv_map));
-    }
+    auto launch = [&](int n_ctas) -> int {
+        if (tiles) return launch_tiles(m, A, n_ctas, stream);
+        CU(smol::decode_launch(m->dm, A, bt, n_ctas, m->smem[bt], (int)m->xs_bytes[bt], stream));
+        m->launches += 1;
+        m->last_kernel = bt == 0 ? SMOL_KERNEL_GROUPS : SMOL_KERNEL_CUDA_CORES;
+        return SMOL_OK;
+    };
     if (m->mode != 1) {
         A.cooperative = 1;
-        CU(smol::decode_launch(m->dm, A, bt, m->n_ctas, m->smem[bt], (int)m->xs_bytes[bt], stream));
-        m->launches += 1;
-        return SMOL_OK;
+        return launch(m->n_ctas);
     }
     const int n_iter = A.n_iter, begin = A.phase_begin, end = A.phase_end;
     const int finalize = A.finalize, advance = A.advance, base = A.iter_base;
     A.cooperative = 0;
     if (n_iter == 0 && finalize) {
         A.n_iter = 0;
-        CU(smol::decode_launch(m->dm, A, bt, 1, m->smem[bt], (int)m->xs_bytes[bt], stream));
-        m->launches += 1;
-        return SMOL_OK;
+        return launch(1);
     }
     for (int it = 0; it < n_iter; ++it) {
         for (int p = begin; p < end; ++p) {
@@ -619,19 +655,21 @@ static int enqueue(SmolModel* m, CallArgs A, cudaStream_t stream, bool whole_ite
             A.tc_part = 0;
             const smol::Phase ph = smol::unpack_phase(m->dm.prog[p]);
             const bool weights = ph.kind != smol::PH_ATTN && ph.kind != smol::PH_SAMPLE;
-            if (bt == 0 && weights) {
-                // the grid barrier between a phase's pre-step and its tiles becomes a launch boundary
-                if (smol::tc_has_prestep(ph)) {
+            if (tc && weights) {
+                // the grid barriers between a phase's pre-step, tiles and post-step become launch boundaries
+                if (tiles ? smol::tile_has_prestep(ph) : smol::tc_has_prestep(ph)) {
                     A.tc_part = 1;
-                    CU(smol::decode_launch(m->dm, A, bt, m->n_ctas, m->smem[bt], (int)m->xs_bytes[bt], stream));
-                    m->launches += 1;
+                    if ((rc = launch(m->n_ctas))) return rc;
                 }
                 A.tc_part = 2;
+                if (tiles && smol::tile_has_poststep(ph)) {
+                    if ((rc = launch(m->n_ctas))) return rc;
+                    A.tc_part = 3;
+                }
             }
             A.finalize = last ? finalize : 0;
             A.advance = (p == end - 1) ? advance : 0;
-            CU(smol::decode_launch(m->dm, A, bt, m->n_ctas, m->smem[bt], (int)m->xs_bytes[bt], stream));
-            m->launches += 1;
+            if ((rc = launch(m->n_ctas))) return rc;
         }
     }
     return SMOL_OK;
@@ -680,7 +718,7 @@ int smol_prefill(SmolModel* m, const SmolBatch* b, int32_t batch, const int32_t*
     A.prompt = d_prompt;
     A.prompt_len = d_prompt_len;
     A.s_max = s_max;
-    if (use_tc(m, A.batch)) return enqueue_tiles(m, A, false, (cudaStream_t)stream);
+    if (use_tc(m, A.batch) && m->mode != 1 && T >= kPromptRows) return enqueue_prompt(m, A, (cudaStream_t)stream);
     return enqueue(m, A, (cudaStream_t)stream, T == 1);  // tiled prefill runs on the barrier kernel
 }
 
@@ -703,7 +741,7 @@ int smol_prompt_logits(SmolModel* m, const SmolBatch* b, const int32_t* d_prompt
     A.whole_prompt = n;
     A.n_iter = (n + T - 1) / T;
     A.head_row = n - 1 - (A.n_iter - 1) * T;
-    return enqueue_tiles(m, A, false, (cudaStream_t)stream);
+    return enqueue_prompt(m, A, (cudaStream_t)stream);
 }
 
 int smol_slow_step(SmolModel* m, const SmolBatch* b, int32_t batch, int32_t advance, void* stream) {
@@ -872,6 +910,11 @@ int smol_set_option(SmolModel* m, const char* name, int64_t value) {
         m->frame_key_valid = false;  // a cached frame graph was captured for the other kernel variant
         return SMOL_OK;
     }
+    if (!std::strcmp(name, "tc_group_rows")) {
+        m->tc_group_rows = value < 0 ? -1 : value > 0x7fffffff ? 0x7fffffff : (int)value;
+        m->frame_key_valid = false;
+        return SMOL_OK;
+    }
     if (!std::strcmp(name, "ll_flags")) {
         m->ll_flags = (int)value;
         return SMOL_OK;
@@ -903,7 +946,9 @@ int64_t smol_get_option(const SmolModel* m, const char* name) {
     if (!std::strcmp(name, "n_sms")) return m->n_sms;
     if (!std::strcmp(name, "smem_bytes")) return (int64_t)m->smem[1];
     if (!std::strcmp(name, "tc_min_batch")) return m->tc_min_batch;
-    if (!std::strcmp(name, "tc_ready")) return m->tile_ready[0] ? 1 : 0;
+    if (!std::strcmp(name, "tc_ready")) return m->tile_ready[0] || m->tiles_ready || m->prompt_ready ? 1 : 0;
+    if (!std::strcmp(name, "tc_group_rows")) return m->tc_group_rows;
+    if (!std::strcmp(name, "last_kernel")) return m->last_kernel;
     if (!std::strcmp(name, "ll_smem_bytes")) return (int64_t)m->ll2_smem;
     if (!std::strcmp(name, "ll_ready")) return (int64_t)m->ll2_state;
     if (!std::strcmp(name, "ll_max_batch")) return (int64_t)m->ll2_max_batch;

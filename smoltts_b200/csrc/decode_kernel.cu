@@ -125,8 +125,9 @@ __device__ __forceinline__ void bulk_g2s(void* dst, const void* src, uint32_t by
 }
 __device__ __forceinline__ void fence_proxy_async() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 
-// Generic-proxy writes (st.global of activations) <-> async-proxy reads (bulk copies of the same rows by other CTAs): fenced by the
-// threads that issue the copies, behind the grid barrier (the tensor-core variant).
+// Generic-proxy writes (st.global of activations) <-> async-proxy reads of the same rows by other CTAs: fenced by the threads that issue
+// the copies, behind the grid barrier (groups of rows, prompts), or on both sides of it (128-row tiles).
+__device__ __forceinline__ void fence_proxy_async_all() { asm volatile("fence.proxy.async;" ::: "memory"); }
 __device__ __forceinline__ void fence_proxy_async_global() { asm volatile("fence.proxy.async.global;" ::: "memory"); }
 
 struct Ctx {
@@ -668,6 +669,7 @@ __device__ void phase_attn(const DevModel& M, const CallArgs& A, const Ctx& c, c
 
 }  // namespace smol
 #include "rows_phases.cuh"
+#include "tile_phases.cuh"
 #include "prompt_phases.cuh"
 namespace smol {
 
@@ -807,7 +809,11 @@ __device__ void phase_gemv(const DevModel& M, const CallArgs& A, const Ctx& c, c
 
 // Sampling of one id per sequence (G:88-99 slow, G:118-132 depth) and, after the last depth code,
 // frame assembly and the stop rule (G:143-166).
-__device__ void phase_sample(const DevModel& M, const CallArgs& A, const Ctx& c, const Phase& ph) {
+// feed (tiles of 128 rows, cooperative launch, a depth step follows in the launch): the CTA that chose row b's id also
+// writes the next depth step's input -- the slow hidden state after the slow id, the embedding of the code after a depth
+// code (G:136-140) -- to the fast residual stream and its RMSNorm to M.xn, exactly as that step's own pre-step would
+// (tile_row_step: same chunks per warp, same order of additions), which then is skipped.
+__device__ void phase_sample(const DevModel& M, const CallArgs& A, const Ctx& c, const Phase& ph, bool feed) {
     const bool fast = ph.fast != 0;
     const int N = fast ? M.codebook_size : M.vocab;
     const int r = fast ? 1 + ph.depth_pos : 0;
@@ -844,11 +850,47 @@ __device__ void phase_sample(const DevModel& M, const CallArgs& A, const Ctx& c,
                 }
             }
         }
+        if (feed) {
+            const int D = M.fdim, nch = D >> 3, ch = c.tid;
+            const int next_pos = fast ? ph.depth_pos + 1 : 0;
+            const uint16_t* row = !fast ? M.x + (size_t)b * D
+                                        : M.fast_embeddings + (size_t)(tok + (M.depthwise_wte ? (M.dup0 ? next_pos - 1 : next_pos) * M.codebook_size : 0)) * D;
+            const uint16_t* norm_w = M.fast_layers[0].attention_norm;
+            float x[8];
+            float ss = 0.f;
+            uint4 wv = make_uint4(0u, 0u, 0u, 0u);
+            if (ch < nch) {
+                wv = __ldg(reinterpret_cast<const uint4*>(norm_w + ch * 8));
+                unpack8(ldcg_v4(row + ch * 8), x);
+#pragma unroll
+                for (int e = 0; e < 8; ++e) ss = fmaf(x[e], x[e], ss);
+            }
+            ss = warp_sum(ss);
+            if (c.lane == 0) g_part[c.warp] = ss;
+            __syncthreads();
+            if (ch < nch) {
+                float t = 0.f;
+                for (int i = 0; i < 3; ++i) t += g_part[i];
+                const float mean = __fdiv_rn(t, (float)D);
+                const float rs = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(mean, M.eps)));
+                uint4 raw;
+                raw.x = pack_bf16(x[0], x[1]); raw.y = pack_bf16(x[2], x[3]); raw.z = pack_bf16(x[4], x[5]); raw.w = pack_bf16(x[6], x[7]);
+                *reinterpret_cast<uint4*>(M.xf + (size_t)b * D + ch * 8) = raw;
+                float wf[8];
+                unpack8(wv, wf);
+                uint4 o;
+                o.x = pack_bf16(__fmul_rn(bf16_round(__fmul_rn(x[0], rs)), wf[0]), __fmul_rn(bf16_round(__fmul_rn(x[1], rs)), wf[1]));
+                o.y = pack_bf16(__fmul_rn(bf16_round(__fmul_rn(x[2], rs)), wf[2]), __fmul_rn(bf16_round(__fmul_rn(x[3], rs)), wf[3]));
+                o.z = pack_bf16(__fmul_rn(bf16_round(__fmul_rn(x[4], rs)), wf[4]), __fmul_rn(bf16_round(__fmul_rn(x[5], rs)), wf[5]));
+                o.w = pack_bf16(__fmul_rn(bf16_round(__fmul_rn(x[6], rs)), wf[6]), __fmul_rn(bf16_round(__fmul_rn(x[7], rs)), wf[7]));
+                *reinterpret_cast<uint4*>(M.xn + (size_t)b * D + ch * 8) = o;
+            }
+        }
         __syncthreads();
     }
 }
 
-// BT == 0: the tensor-core variant (rows_phases.cuh) for 9 and more rows.
+// BT == 0: decoding of 9 and more sequences in groups of rows (rows_phases.cuh).
 template <int BT, bool kTimed>
 __device__ __forceinline__ void run_phase(const DevModel& M, const CallArgs& A, const Ctx& c, const Phase& ph,
                                           uint32_t& parity, RowsSync& sy, uint32_t packed_phase, const RowsStep* step) {
@@ -943,9 +985,7 @@ smol_decode_kernel(const __grid_constant__ DevModel M, const __grid_constant__ C
                 __syncthreads();
                 if (prof) t1 = globaltimer_ns();
             }
-            // (tensor-core variant, one phase per launch: a phase may take two launches; bookkeeping runs in the last)
-            const bool final_part = A.tc_part != 1;
-            if (c.cta == 0 && p == per_iter - 1 && A.mode == 1 && final_part) {
+            if (BT != 0 && c.cta == 0 && p == per_iter - 1 && A.mode == 1) {
                 // prefill bookkeeping: every sequence advances by the positions of this tile that lie inside its prompt
                 const int T = A.tile_t > 1 ? A.tile_t : 1;
                 for (int b = c.tid; b < A.real_batch; b += kThreads) {
@@ -960,7 +1000,7 @@ smol_decode_kernel(const __grid_constant__ DevModel M, const __grid_constant__ C
             const bool last = (it == A.n_iter - 1) && (p == A.phase_end - 1);
             const bool sync = A.cooperative && !last;
             if (BT == 0) {
-                if (sync) rows_arrive(M, c, sy);
+                if (sync) rows_arrive<kTimed>(M, c, sy);
                 if (prof) {   // [2p]: rows_sync_in takes the waits inside the phase off; [2p + 1]: the arrival, then the wait, which the phase behind adds
                     M.prof[2 * p] += t1 - t0;
                     M.prof[2 * p + 1] += globaltimer_ns() - t1;
@@ -987,7 +1027,7 @@ smol_decode_kernel(const __grid_constant__ DevModel M, const __grid_constant__ C
             }
         }
     }
-    if (A.mode == 1 && A.finalize && c.cta == 0) {
+    if (BT != 0 && A.mode == 1 && A.finalize && c.cta == 0) {
         // leave the last prompt column as the pending input of the first decode frame (G:66-73)
         for (int i = c.tid; i < A.real_batch * M.n_rows; i += kThreads) {
             const int b = i / M.n_rows, r = i - b * M.n_rows;
@@ -1113,11 +1153,16 @@ size_t decode_stage_bytes(const DevModel& M, int n_ctas, int bt) {
     return (m + 127) / 128 * 128;
 }
 
+// Phases of a kind in a frame.
+static int frame_phases(const DevModel& M, int fast, int kind) {
+    return kind == PH_HEAD ? (fast ? M.depth : 1) : fast ? M.n_flayer * M.depth : M.n_layer;
+}
 // Tile plan of the tensor-core variant's weight phases for `rows` activation rows: tiles per block and rows per group, by
 // a model of a CTA's clocks between two barriers -- L2 -> shared memory at 85 bytes per clock, RMSNorm and depth attention
 // repeated per tile block, MMAs at 0.5 clocks, weight fragments and partial sums through shared memory at 128 bytes per clock,
-// and a fixed part per row group (load latency, block barriers).
-void rows_plan(const DevModel& M, int rows, int n_ctas, RowsPlan (*plan)[6]) {
+// and a fixed part per row group (load latency, block barriers).  Returns the time of a frame by that model (us).
+double rows_plan(const DevModel& M, int rows, int n_ctas, RowsPlan (*plan)[6]) {
+    double clocks = 0.;
     for (int f = 0; f < 2; ++f) {
         const int D = f ? M.fdim : M.dim, F = f ? M.finter : M.inter, heads = f ? M.fn_head + 2 * M.fn_kv : M.n_head + 2 * M.n_kv;
         for (int kind = 0; kind <= PH_HEAD; ++kind) {
@@ -1150,10 +1195,35 @@ void rows_plan(const DevModel& M, int rows, int n_ctas, RowsPlan (*plan)[6]) {
                     if (best_cost == 0. || c < best_cost) { best_cost = c; best.mt = (uint8_t)mt; best.n = (uint8_t)n; }
                 }
             }
-            const int groups = (rows + best.n - 1) / best.n;        // even groups: 212 rows are 4 x 53, not 3 x 64 + 20
+            const int groups = (rows + best.n - 1) / best.n;        // even groups: 68 rows are 3 x 23, not 2 x 32 + 4
             best.n = (uint8_t)((rows + groups - 1) / groups);
+            clocks += best_cost * frame_phases(M, f, kind);
         }
     }
+    const int phases = phases_per_frame(M.n_layer, M.n_flayer, M.depth);
+    return 0.92e-3 * clocks + 2.66 * phases + 4.6 * (1 + M.depth) * ((rows + n_ctas - 1) / n_ctas) + 6.6 * M.n_layer * ((rows * M.n_kv + 4 * n_ctas - 1) / (4 * n_ctas));
+}
+// The time of a frame on 128-row tiles (us): ring stages of the fullest CTA, steps between two barriers, row tiles, sampling.
+double tiles_time(const DevModel& M, int rows, int n_ctas) {
+    const int m_tiles = (rows + umma::kM - 1) / umma::kM;
+    int stages = 0, steps = 0, phases = 0;
+    for (int f = 0; f < 2; ++f) {
+        const int D = f ? M.fdim : M.dim, F = f ? M.finter : M.inter, heads = f ? M.fn_head + 2 * M.fn_kv : M.n_head + 2 * M.n_kv;
+        for (int kind = 0; kind <= PH_HEAD; ++kind) {
+            if (kind == PH_ATTN) continue;
+            const int K = kind == PH_W2 ? F : D, cap = kind == PH_W13 ? umma::kMaxN / 2 : umma::kMaxN;
+            const int n_out = kind == PH_QKV ? heads * kHeadDim : kind == PH_W13 ? F : kind == PH_HEAD ? (f ? M.codebook_size : M.vocab) : D;
+            const int split = kind != PH_WO && kind != PH_W2 ? 1 : K % (4 * umma::kBK) == 0 ? 4 : K % (2 * umma::kBK) == 0 ? 2 : 1;
+            int blk = 16;
+            while (blk < cap && m_tiles * ((n_out + blk - 1) / blk) * split > n_ctas) blk += 16;
+            const int units = m_tiles * ((n_out + blk - 1) / blk) * split, n = frame_phases(M, f, kind);
+            stages += n * ((units + n_ctas - 1) / n_ctas) * (K / split / umma::kBK);
+            steps += n * (kind == PH_WO ? 2 + f : kind == PH_W2 ? 2 : 1);
+            phases += kind == PH_HEAD ? 0 : n;
+        }
+    }
+    return 0.665 * stages + 2.7 * steps * ((rows + kRowsPerPass * n_ctas - 1) / (kRowsPerPass * n_ctas)) + 0.74 * phases * m_tiles
+           + 3.0 * (1 + M.depth) * ((rows + n_ctas - 1) / n_ctas);
 }
 
 // Kernel variant by batch tile (sequences whose activations share one pass over the weights).
@@ -1184,20 +1254,28 @@ cudaError_t decode_max_ctas(int bt, size_t smem, int* per_sm) {
     return cudaOccupancyMaxActiveBlocksPerMultiprocessor(per_sm, decode_fn(bt), kThreads, smem);
 }
 
-static const void* prompt_fn(bool wide, bool timed) {
-    if (wide) return timed ? (const void*)smol_wide_kernel<true> : (const void*)smol_wide_kernel<false>;
-    return timed ? (const void*)smol_prompt_kernel<true> : (const void*)smol_prompt_kernel<false>;
-}
+static const void* prompt_fn(bool timed) { return timed ? (const void*)smol_prompt_kernel<true> : (const void*)smol_prompt_kernel<false>; }
 cudaError_t prompt_configure(int* per_sm) {
-    for (int i = 0; i < 4; ++i) {
-        const cudaError_t e = cudaFuncSetAttribute(prompt_fn(i & 1, i >> 1), cudaFuncAttributeMaxDynamicSharedMemorySize, kPrSmem);
+    for (int i = 0; i < 2; ++i) {
+        const cudaError_t e = cudaFuncSetAttribute(prompt_fn(i), cudaFuncAttributeMaxDynamicSharedMemorySize, kPrSmem);
         if (e != cudaSuccess) return e;
     }
-    return cudaOccupancyMaxActiveBlocksPerMultiprocessor(per_sm, prompt_fn(false, false), kThreads, kPrSmem);
+    return cudaOccupancyMaxActiveBlocksPerMultiprocessor(per_sm, prompt_fn(false), kThreads, kPrSmem);
 }
-cudaError_t prompt_launch(const DevModel& M, const CallArgs& A, bool wide, int n_ctas, cudaStream_t stream) {
+cudaError_t prompt_launch(const DevModel& M, const CallArgs& A, int n_ctas, cudaStream_t stream) {
     void* args[2] = {(void*)&M, (void*)&A};
-    return cudaLaunchCooperativeKernel(prompt_fn(wide, M.prof != nullptr), dim3(n_ctas), dim3(kThreads), args, kPrSmem, stream);
+    return cudaLaunchCooperativeKernel(prompt_fn(M.prof != nullptr), dim3(n_ctas), dim3(kThreads), args, kPrSmem, stream);
+}
+
+constexpr int kTilesSmem = umma::kRingBytes + 2048 + umma::kM * 4;   // 1024-aligned ring and the RoPE positions of the tile's rows
+cudaError_t tiles_configure(int* per_sm) {
+    const cudaError_t e = cudaFuncSetAttribute(smol_tiles_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kTilesSmem);
+    return e != cudaSuccess ? e : cudaOccupancyMaxActiveBlocksPerMultiprocessor(per_sm, smol_tiles_kernel, kThreads, kTilesSmem);
+}
+cudaError_t tiles_launch(const DevModel& M, const CallArgs& A, int n_ctas, cudaStream_t stream) {
+    void* args[2] = {(void*)&M, (void*)&A};
+    if (A.cooperative) return cudaLaunchCooperativeKernel((const void*)smol_tiles_kernel, dim3(n_ctas), dim3(kThreads), args, kTilesSmem, stream);
+    return cudaLaunchKernel((const void*)smol_tiles_kernel, dim3(n_ctas), dim3(kThreads), args, kTilesSmem, stream);
 }
 
 cudaError_t decode_launch(const DevModel& M, const CallArgs& A, int bt, int n_ctas, size_t smem, int xs_bytes,

@@ -180,8 +180,8 @@ struct CallArgs {
     int repeat;       // profiling only: run the body of every weight phase 1 + repeat times
     int tile_t;       // prefill: prompt positions handled per iteration (rows = real_batch * tile_t share the weight pass)
     int real_batch;   // prefill: sequences (rows / tile_t)
-    int tc_part;      // tensor-core variant, one phase per launch: 1 = only the phase's pre-step, 2 = only its tiles
-                      // (0 = the whole phase: cooperative launches)
+    int tc_part;      // tensor-core variants, one phase per launch: 1 = only the phase's pre-step, 2 = only its tiles,
+                      // 3 = only its post-step (0 = the whole phase: cooperative launches)
     int tc_split;     // tensor-core variant: cached positions per attention split (0 = default)
     int team_ctas;    // second-generation data-flow kernel: CTAs per sequence (one team each); grid = batch * team_ctas
     const int32_t* prompt;      // prefill: [B][n_rows][s_max]
@@ -246,8 +246,16 @@ __host__ __device__ inline Phase decode_phase(int p, int n_layer, int n_flayer) 
 
 // Tensor-core variant: the phase that starts with a grid-wide pre-step (the token embedding of the slow transformer's input).
 __host__ __device__ inline bool tc_has_prestep(const Phase& ph) { return ph.kind == PH_QKV && !ph.fast && ph.layer == 0; }
+// Tiles of 128 rows: phases that start with a grid-wide pre-step (embedding / input gather + RMSNorm into xn, or the depth attention) --
+// every weight phase except the slow wo and the w2's, whose inputs the previous phase left in place -- and those whose K slices meet
+// in a post-step.
+__host__ __device__ inline bool tile_has_prestep(const Phase& ph) {
+    if (ph.kind == PH_ATTN || ph.kind == PH_SAMPLE) return false;
+    return !(ph.kind == PH_W2 || (ph.kind == PH_WO && !ph.fast));
+}
+__host__ __device__ inline bool tile_has_poststep(const Phase& ph) { return ph.kind == PH_WO || ph.kind == PH_W2; }
 
-// Tiles of 128 rows (prompt_phases.cuh): slots of the tensor-map table (DevModel.tmaps).  Activations of the slow and (+ TM_FAST) the
+// Tiles of 128 rows (tile_phases.cuh, prompt_phases.cuh): slots of the tensor-map table (DevModel.tmaps).  Activations of the slow and (+ TM_FAST) the
 // depth transformer: boxes of 128 rows, of 64 and of 32; weights: one map per matrix and box height 16 * (v + 1) rows, v = 0..5, so
 // that a tile's weight rows are ONE copy per stage.
 enum TensorMapSlot { TM_XN = 0, TM_ATTN, TM_ACT, TM_FAST = 3, TM_ACT_MAPS = 6, TM_WEIGHTS = 18 };
@@ -258,7 +266,7 @@ constexpr int kTmTotal = TM_WEIGHTS + kTmWeightBoxes * kTmWeightStride;
 __host__ __device__ inline int tm_weight_index(int layer, int which) { return 2 + layer * 5 + which; }
 __host__ __device__ inline int tm_weight_slot(int weight_index, int box_rows) { return TM_WEIGHTS + (box_rows / 16 - 1) * kTmWeightStride + weight_index; }
 constexpr int kTensorMapBytes = 128;
-constexpr int kTcKSplit = 4;  // K slices of a prompt's wo / w2 tiles (their sum + residual + next RMSNorm is a step of its own)
+constexpr int kTcKSplit = 4;  // K slices of the wo / w2 tiles (their sum + residual + next RMSNorm is a step of its own)
 
 __host__ __device__ inline uint32_t pack_phase(const Phase& ph) {
     return (uint32_t)ph.kind | ((uint32_t)ph.fast << 4) | ((uint32_t)ph.layer << 8) | ((uint32_t)ph.depth_pos << 16);

@@ -1,6 +1,6 @@
-// Hundreds of rows at once: prompts (the slow transformer over sequences x positions) and the decode of wide batches, each one
-// persistent kernel with the same phases and grid barrier as decode_kernel.cu.  Included by decode_kernel.cu after rows_phases.cuh (whose batch
-// attention, split barrier and row bookkeeping it uses).
+// The prompt of one sequence: the slow transformer over its positions as one persistent kernel with the same phases and grid barrier as
+// decode_kernel.cu.  Included by decode_kernel.cu after rows_phases.cuh and tile_phases.cuh (whose batch attention, split barrier and row
+// steps it uses).
 //
 // A weight phase Y[rows][n_out] = X[rows][K] * W[n_out][K]^T is cut into units (128-row tile, block of `blk` weight rows; wo and
 // w2 also into K slices, so that a unit's chain is K = 768 long and the SMs are full); blk is the smallest multiple of 16 that
@@ -55,77 +55,8 @@ __device__ __forceinline__ void bar_arrive(uint64_t* bar) {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(umma::s2u(bar)) : "memory");
 }
 
-// Row steps.  Three warps per row (one 16-byte chunk per lane: every load of a row is in flight at once), five rows per CTA and
-// pass.  load(bg, ch, x) produces chunk ch of row bg; the row goes to `raw` as it is and, if norm_w is given, through RMSNorm
-// (P:601-613: fp32 normalise, round to bf16, multiply by the bf16 weight, round again) to M.xn.
-constexpr int kRowWarps = 3;
-constexpr int kRowsPerPass = kWarps / kRowWarps;
-
-template <class Load>
-__device__ __forceinline__ void prompt_row_step(const DevModel& M, const CallArgs& A, const Ctx& c, int D, uint16_t* raw, const uint16_t* norm_w, Load load) {
-    const int nch = D >> 3;
-    const int slot = c.warp / kRowWarps, wi = c.warp - slot * kRowWarps;
-    const int ch = wi * 32 + c.lane;
-    for (int row0 = c.cta * kRowsPerPass; row0 < A.batch; row0 += c.n_ctas * kRowsPerPass) {
-        const int bg = row0 + slot;
-        const bool act = slot < kRowsPerPass && bg < A.batch && ch < nch;
-        float x[8];
-        float ss = 0.f;
-        uint4 wv = make_uint4(0u, 0u, 0u, 0u);
-        if (act) {
-            if (norm_w != nullptr) wv = __ldg(reinterpret_cast<const uint4*>(norm_w + ch * 8));
-            load(bg, ch, x);
-#pragma unroll
-            for (int e = 0; e < 8; ++e) ss = fmaf(x[e], x[e], ss);
-        }
-        ss = warp_sum(ss);
-        if (c.lane == 0) g_part[c.warp] = ss;
-        __syncthreads();
-        if (act) {
-            *reinterpret_cast<uint4*>(raw + (size_t)bg * D + ch * 8) = pack8(x);
-            if (norm_w != nullptr) {
-                float t = 0.f;
-                for (int i = 0; i < kRowWarps; ++i) t += g_part[slot * kRowWarps + i];
-                const float mean = __fdiv_rn(t, (float)D);
-                const float r = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(mean, M.eps)));
-                float wf[8], o[8];
-                unpack8(wv, wf);
-#pragma unroll
-                for (int e = 0; e < 8; ++e) o[e] = __fmul_rn(bf16_round(__fmul_rn(x[e], r)), wf[e]);
-                *reinterpret_cast<uint4*>(M.xn + (size_t)bg * D + ch * 8) = pack8(o);
-            }
-        }
-        __syncthreads();
-    }
-}
-
-// dst = res + bf16(sum of the K slices' partial sums, in slice order): the Linear's bf16 output plus the residual (P:499-500).
 __device__ __noinline__ void prompt_finish(const DevModel& M, const CallArgs& A, const Ctx& c, const uint16_t* res, uint16_t* dst, int D, int slices, const uint16_t* norm_w, int last_row) {
-    prompt_row_step(M, A, c, D, dst, norm_w, [&](int bg, int ch, float (&x)[8]) {
-        const int n_split = bg == last_row ? 1 : slices;
-        const uint4 rv = ldcg_v4(res + (size_t)bg * D + ch * 8);
-        float4 pa[kTcKSplit], pb[kTcKSplit];
-#pragma unroll
-        for (int sp = 0; sp < kTcKSplit; ++sp) {
-            const float* pp = M.kpart + ((size_t)min(sp, n_split - 1) * M.ws_rows + bg) * D + ch * 8;
-            pa[sp] = __ldcg(reinterpret_cast<const float4*>(pp));
-            pb[sp] = __ldcg(reinterpret_cast<const float4*>(pp + 4));
-        }
-        float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-#pragma unroll
-        for (int sp = 0; sp < kTcKSplit; ++sp) {
-            if (sp < n_split) {
-                acc[0] = __fadd_rn(acc[0], pa[sp].x); acc[1] = __fadd_rn(acc[1], pa[sp].y);
-                acc[2] = __fadd_rn(acc[2], pa[sp].z); acc[3] = __fadd_rn(acc[3], pa[sp].w);
-                acc[4] = __fadd_rn(acc[4], pb[sp].x); acc[5] = __fadd_rn(acc[5], pb[sp].y);
-                acc[6] = __fadd_rn(acc[6], pb[sp].z); acc[7] = __fadd_rn(acc[7], pb[sp].w);
-            }
-        }
-        float rf[8];
-        unpack8(rv, rf);
-#pragma unroll
-        for (int e = 0; e < 8; ++e) x[e] = bf16_round(__fadd_rn(rf[e], bf16_round(acc[e])));
-    });
+    tile_finish(M, A, c, res, dst, D, slices, norm_w, last_row);
 }
 
 // The last position of a prompt whose logits are wanted, row `row` of the tile: its dot products in the order of the one-row
@@ -262,16 +193,14 @@ __device__ __noinline__ void row_wide(const DevModel& M, int row, int layer, int
     }
 }
 
-// One weight phase; on return the CTA has finished its units, the barrier behind it is the caller's.  kWide: of a decode frame (the
-// depth transformer's phases and the heads exist, no row stands for a last position), else of a prompt.
-template <bool kWide, bool kTimed>
+// One weight phase; on return the CTA has finished its units, the barrier behind it is the caller's.
+template <bool kTimed>
 __device__ __noinline__ void prompt_gemm(const DevModel& M, const CallArgs& A, const Ctx& c, const Phase& ph, RowsSync& sy, uint32_t& chunk, uint32_t& tile, const int last_row) {
     const int kind = ph.kind;
-    const bool fast = kWide && ph.fast != 0;
-    const int D = fast ? M.fdim : M.dim, F = fast ? M.finter : M.inter, Hq = fast ? M.fn_head : M.n_head, Hkv = fast ? M.fn_kv : M.n_kv;
+    const int D = M.dim, F = M.inter, Hq = M.n_head, Hkv = M.n_kv;
     const int q_rows = Hq * kHeadDim, k_end = (Hq + Hkv) * kHeadDim;
     const int K = kind == PH_W2 ? F : D;
-    const int n_out = kind == PH_QKV ? (Hq + 2 * Hkv) * kHeadDim : kind == PH_W13 ? F : kWide && kind == PH_HEAD ? (fast ? M.codebook_size : M.vocab) : D;
+    const int n_out = kind == PH_QKV ? (Hq + 2 * Hkv) * kHeadDim : kind == PH_W13 ? F : D;
     const int rows = A.batch;
     unsigned char* ring = reinterpret_cast<unsigned char*>(c.xs);
     const int warp = c.warp, lane = c.lane;
@@ -279,11 +208,9 @@ __device__ __noinline__ void prompt_gemm(const DevModel& M, const CallArgs& A, c
     const unsigned char* tm = M.tmaps;
     const int box_idx = rows <= 32 ? 2 : rows <= 64 ? 1 : 0;   // activation box of 32 / 64 / 128 rows: the rest of a stage holds stale rows whose accumulator lanes nobody reads
     const int a_bytes = (umma::kM >> box_idx) * umma::kBK * 2;
-    const void* tm_a = tm + (size_t)kTensorMapBytes * (box_idx * TM_ACT_MAPS + (fast ? TM_FAST : 0) + (kind == PH_WO ? TM_ATTN : kind == PH_W2 ? TM_ACT : TM_XN));
+    const void* tm_a = tm + (size_t)kTensorMapBytes * (box_idx * TM_ACT_MAPS + (kind == PH_WO ? TM_ATTN : kind == PH_W2 ? TM_ACT : TM_XN));
     const int which = kind == PH_QKV ? 0 : kind == PH_WO ? 1 : kind == PH_W13 ? 2 : 4;
-    const int layer = fast ? M.n_layer + ph.layer : ph.layer;
-    const int w0 = kWide && kind == PH_HEAD ? (fast ? 1 : 0) : tm_weight_index(layer, which), w1 = tm_weight_index(layer, 3);
-    const int w_row = kWide && kind == PH_HEAD && fast && M.depthwise_output ? ph.depth_pos * n_out : 0;   // a depth position's own head
+    const int w0 = tm_weight_index(ph.layer, which), w1 = tm_weight_index(ph.layer, 3);
     const bool paired = kind == PH_W13;
     const int n_split = kind != PH_WO && kind != PH_W2 ? 1 : prompt_slices(K);
     const int nk = K / n_split / umma::kBK;
@@ -302,7 +229,7 @@ __device__ __noinline__ void prompt_gemm(const DevModel& M, const CallArgs& A, c
     auto load_w = [&](uint32_t g, int n0, int k0) {
         const uint32_t s = g % kPrStages, b = umma::s2u(ring + (size_t)s * umma::kStageBytes) + umma::kStageA;
         umma::bar_expect_tx(&g_pr.full[s], (uint32_t)(n_blk * umma::kBK * 2));
-        umma::tma_load_2d(b, tm + (size_t)kTensorMapBytes * tm_weight_slot(w0, blk), k0, w_row + n0, &g_pr.full[s]);
+        umma::tma_load_2d(b, tm + (size_t)kTensorMapBytes * tm_weight_slot(w0, blk), k0, n0, &g_pr.full[s]);
         if (paired) umma::tma_load_2d(b + blk * umma::kBK * 2, tm + (size_t)kTensorMapBytes * tm_weight_slot(w1, blk), k0, n0, &g_pr.full[s]);
     };
     // the first stages' weights do not wait for the phase before (the ring is empty: that phase's accumulators have been read)
@@ -379,7 +306,7 @@ __device__ __noinline__ void prompt_gemm(const DevModel& M, const CallArgs& A, c
             const int bg = m0 + quad * 32 + lane;
             const bool live = bg < rows && bg != last_row;
             int pos = 0, page = -1;
-            if (kind == PH_QKV && live && !fast) {      // cache slot of the row (-1: nothing is appended)
+            if (kind == PH_QKV && live) {      // cache slot of the row (-1: nothing is appended)
                 const int bs = row_seq(A, bg);
                 pos = ldcg_i32(A.b.seq_len + bs) + row_off(A, bg);
                 if (seq_active(M, A, c, bg) && pos < A.b.max_pages * M.page_size) page = ldcg_i32(A.b.block_table + (size_t)bs * A.b.max_pages + pos / M.page_size);
@@ -405,19 +332,6 @@ __device__ __noinline__ void prompt_gemm(const DevModel& M, const CallArgs& A, c
                     *reinterpret_cast<uint4*>(M.act + (size_t)bg * F + u0) = pack8(o);
                     continue;
                 }
-                if (kWide && kind == PH_HEAD) {
-                    float* out = (fast ? M.depth_logits + ((size_t)bg * M.depth + ph.depth_pos) * n_out : M.token_logits + (size_t)bg * n_out) + u0;
-#pragma unroll
-                    for (int e = 0; e < 8; ++e) acc[e] = bf16_round(acc[e]);
-                    if ((n_out & 7) == 0) {
-                        *reinterpret_cast<float4*>(out) = make_float4(acc[0], acc[1], acc[2], acc[3]);
-                        *reinterpret_cast<float4*>(out + 4) = make_float4(acc[4], acc[5], acc[6], acc[7]);
-                    } else {
-#pragma unroll
-                        for (int e = 0; e < 8; ++e) { if (u0 + e < n_out) out[e] = acc[e]; }
-                    }
-                    continue;
-                }
                 if (kind != PH_QKV) {
                     float* pp = M.kpart + ((size_t)ks * M.ws_rows + bg) * D + u0;
                     *reinterpret_cast<float4*>(pp) = make_float4(acc[0], acc[1], acc[2], acc[3]);
@@ -428,7 +342,7 @@ __device__ __noinline__ void prompt_gemm(const DevModel& M, const CallArgs& A, c
 #pragma unroll
                 for (int e = 0; e < 8; ++e) v[e] = bf16_round(acc[e]);
                 if (u0 < k_end) {  // q and k rows: interleaved-pair RoPE with the bf16 table (P:616-640); never past the table (host checks bound pos)
-                    const uint4 cs = __ldg(reinterpret_cast<const uint4*>((fast ? M.fast_rope + (size_t)ph.depth_pos * kHeadDim : M.rope + (size_t)min(pos, M.max_seq_len - 1) * kHeadDim) + (u0 & (kHeadDim - 1))));
+                    const uint4 cs = __ldg(reinterpret_cast<const uint4*>(M.rope + (size_t)min(pos, M.max_seq_len - 1) * kHeadDim + (u0 & (kHeadDim - 1))));
                     const uint32_t cw[4] = {cs.x, cs.y, cs.z, cs.w};
 #pragma unroll
                     for (int e = 0; e < 8; e += 2) {
@@ -440,10 +354,6 @@ __device__ __noinline__ void prompt_gemm(const DevModel& M, const CallArgs& A, c
                 }
                 if (u0 < q_rows) { *reinterpret_cast<uint4*>(M.q + (size_t)bg * q_rows + u0) = pack8(v); continue; }
                 const int is_v = u0 >= k_end ? 1 : 0, n1 = u0 - (is_v ? k_end : q_rows), ps = M.page_size;
-                if (fast) {
-                    *reinterpret_cast<uint4*>(M.fkv + (((size_t)(bg * M.n_flayer + ph.layer) * 2 + is_v) * M.depth + ph.depth_pos) * (Hkv * kHeadDim) + n1) = pack8(v);
-                    continue;
-                }
                 if (page < 0) continue;
                 *reinterpret_cast<uint4*>(M.kv_pool + ((((size_t)page * M.n_layer + ph.layer) * 2 + is_v) * Hkv + n1 / kHeadDim) * ((size_t)ps * kHeadDim)
                                           + (size_t)(pos % ps) * kHeadDim + (n1 & (kHeadDim - 1))) = pack8(v);
@@ -481,7 +391,7 @@ __device__ __forceinline__ void prompt_attn(const DevModel& M, const CallArgs& A
     }
 }
 
-// What the kernels begin with: the arguments' copies, barriers, tensor memory.
+// What the kernel begins with: the arguments' copies, barriers, tensor memory.
 __device__ __forceinline__ void prompt_setup(const DevModel& Mp, const CallArgs& Ap, unsigned char* smem_dyn, Ctx& c, RowsSync& sy) {
     for (int i = threadIdx.x; i < (int)(sizeof(DevModel) / 4); i += kThreads) reinterpret_cast<uint32_t*>(smem_dyn + kPrData)[i] = reinterpret_cast<const uint32_t*>(&Mp)[i];
     for (int i = threadIdx.x; i < (int)(sizeof(CallArgs) / 4); i += kThreads) reinterpret_cast<uint32_t*>(smem_dyn + kPrData + kPrModel)[i] = reinterpret_cast<const uint32_t*>(&Ap)[i];
@@ -531,23 +441,23 @@ smol_prompt_kernel(const __grid_constant__ DevModel Mp, const __grid_constant__ 
         c.iter = it;
         const bool last_iter = it == A.n_iter - 1;
         const int last_row = last_iter && A.whole_prompt > 0 ? A.head_row : -1;
-        sy.phase = 0;
+        if (kTimed) sy.phase = 0;
         PhaseTimer<kTimed> timer(c);
         rows_sync_in(M, sy);
         timer.rest();
-        prompt_row_step(M, A, c, M.dim, M.x, M.layers[0].attention_norm, [&](int bg, int ch, float (&x)[8]) { embed_chunk(M, A, c, bg, ch, x); });
+        tile_row_step(M, A, c, M.dim, M.x, M.layers[0].attention_norm, [&](int bg, int ch, float (&x)[8]) { embed_chunk(M, A, c, bg, ch, x); });
         timer.step(M, unpack_phase(M.prog[0]));
-        rows_arrive(M, c, sy);
+        rows_arrive<kTimed>(M, c, sy);
         for (int p = 0; p < phases_per_prefill_step(M.n_layer); ++p) {
             const Phase ph = unpack_phase(M.prog[p]);
-            sy.phase = p;
+            if (kTimed) sy.phase = p;
             if (ph.kind == PH_ATTN) {
                 rows_sync_in(M, sy);
                 prompt_attn(M, A, c, ph, sy, Ap.kv_map, last_row);
             } else {
-                prompt_gemm<false, kTimed>(M, A, c, ph, sy, chunk, tile, last_row);
+                prompt_gemm<kTimed>(M, A, c, ph, sy, chunk, tile, last_row);
                 if (ph.kind == PH_WO || ph.kind == PH_W2) {   // h = stream + wo(attn) (P:499); stream = h + w2(act) (P:500); and the norm of the phase that reads it
-                    rows_arrive(M, c, sy);
+                    rows_arrive<kTimed>(M, c, sy);
                     rows_sync_in(M, sy);
                     timer.rest();
                     const bool wo = ph.kind == PH_WO;
@@ -566,12 +476,12 @@ smol_prompt_kernel(const __grid_constant__ DevModel Mp, const __grid_constant__ 
                 }
             }
             timer.end(M, p);
-            if (!(last_iter && A.whole_prompt == 0 && p == phases_per_prefill_step(M.n_layer) - 1)) rows_arrive(M, c, sy);
+            if (!(last_iter && A.whole_prompt == 0 && p == phases_per_prefill_step(M.n_layer) - 1)) rows_arrive<kTimed>(M, c, sy);
             timer.arrived(M, p);
         }
     }
     if (A.whole_prompt > 0) {
-        sy.phase = 5 * M.n_layer;        // the LM head's
+        if (kTimed) sy.phase = 5 * M.n_layer;        // the LM head's
         PhaseTimer<kTimed> timer(c);
         rows_sync_in(M, sy);
         if (c.cta == 0 && A.head_row > 0)      // the last position's hidden state (pre-norm) -> row 0
@@ -582,7 +492,7 @@ smol_prompt_kernel(const __grid_constant__ DevModel Mp, const __grid_constant__ 
             row_fetch(M, PH_HEAD, 0, u, c.lane, w, w);
             row_finish(M, A, PH_HEAD, 0, A.head_row, u, c.lane, w, w, x, 0, -1, 0u);
         }
-        timer.end(M, sy.phase);
+        timer.end(M, 5 * M.n_layer);
     }
     if (c.cta == 0) {
         // leave the last prompt column as the pending input of the first decode frame (G:66-73)
@@ -592,99 +502,6 @@ smol_prompt_kernel(const __grid_constant__ DevModel Mp, const __grid_constant__ 
         }
         if (c.tid == 0) M.barrier[1] = sy.target;
     }
-    umma::fence_before_sync();
-    __syncthreads();
-    if (c.warp == 0) umma::tmem_free(g_pr.tmem_base);
-}
-
-__device__ void phase_sample(const DevModel& M, const CallArgs& A, const Ctx& c, const Phase& ph);
-
-// ---- decode frames of wide batches ----------------------------------------------------------------------------------
-// From kWideRows rows on (host: wide_launch) a frame's weight phases are tiles of 128 rows instead of rows_phases.cuh's groups of 32,
-// which repeat the norm and the row copies per weight block and take several turns (150m, 256 rows: 2699 us per frame against 3380).  Sums are in the same order, so
-// a row's bits are the same on either side of the line.
-__device__ __noinline__ void wide_attn(const DevModel& M, const CallArgs& A, const Ctx& c, const Phase& ph, RowsSync& sy, const void* kv_map) { phase_attn_batch<false>(M, A, c, ph, sy, kv_map); }
-// Depth attention of all rows -> M.attn, the CTA's share of the rows in groups of one row per kv-head's warps.
-__device__ __noinline__ void wide_depth_attention(const DevModel& M, const CallArgs& A, const Ctx& c, int layer, int depth_pos) {
-    const int per = (A.batch + c.n_ctas - 1) / c.n_ctas, r0 = c.cta * per, n = min(per, A.batch - r0);
-    if (n <= 0) return;
-    unsigned char* out = reinterpret_cast<unsigned char*>(M.attn + (size_t)r0 * M.fdim);
-    if (depth_pos < 8) rows_depth_attention<false>(M, layer, depth_pos, r0, n, out, M.fdim * 2, nullptr);
-    else rows_depth_attention<true>(M, layer, depth_pos, r0, n, out, M.fdim * 2, nullptr);
-}
-// The input of the slow or the depth transformer -> its residual stream, and the first norm: the token embedding (P:205-221), the
-// slow hidden state or the previous depth code's embedding (G:136-140).
-__device__ __noinline__ void wide_input(const DevModel& M, const CallArgs& A, const Ctx& c, const Phase& ph) {
-    if (!ph.fast) {
-        prompt_row_step(M, A, c, M.dim, M.x, M.layers[0].attention_norm, [&](int bg, int ch, float (&x)[8]) { embed_chunk(M, A, c, bg, ch, x); });
-        return;
-    }
-    prompt_row_step(M, A, c, M.fdim, M.xf, M.fast_layers[0].attention_norm, [&](int bg, int ch, float (&x)[8]) {
-        const uint16_t* src = (A.fast_from_xf ? M.xf : M.x) + (size_t)bg * M.fdim;
-        if (!A.fast_from_xf && ph.depth_pos > 0) {
-            const int code = ldcg_i32(M.frame_tokens + (size_t)bg * M.n_rows + ph.depth_pos);
-            src = M.fast_embeddings + (size_t)(code + (M.depthwise_wte ? (M.dup0 ? ph.depth_pos - 1 : ph.depth_pos) * M.codebook_size : 0)) * M.fdim;
-        }
-        unpack8(ldcg_v4(src + ch * 8), x);
-    });
-}
-__device__ __noinline__ void wide_sample(const DevModel& M, const CallArgs& A, const Ctx& c, const Phase& ph) { phase_sample(M, A, c, ph); }
-
-template <bool kTimed>
-__global__ void __launch_bounds__(kThreads, 1)
-smol_wide_kernel(const __grid_constant__ DevModel Mp, const __grid_constant__ CallArgs Ap) {
-    extern __shared__ __align__(1024) unsigned char smem_dyn[];
-    const DevModel& M = *reinterpret_cast<const DevModel*>(smem_dyn + kPrData);
-    const CallArgs& A = *reinterpret_cast<const CallArgs*>(smem_dyn + kPrData + kPrModel);
-    Ctx c;
-    RowsSync sy;
-    prompt_setup(Mp, Ap, smem_dyn, c, sy);
-    uint32_t chunk = 0, tile = 0;
-    PhaseTimer<kTimed> timer(c);
-    for (int it = 0; it < A.n_iter; ++it) {
-        c.iter = it;
-        for (int p = A.phase_begin; p < A.phase_end; ++p) {
-            const Phase ph = unpack_phase(M.prog[p]);
-            const bool fast = ph.fast != 0;
-            sy.phase = p;
-            if (ph.kind == PH_ATTN) {
-                wide_attn(M, A, c, ph, sy, Ap.kv_map);
-            } else if (ph.kind == PH_SAMPLE) {
-                rows_sync_in(M, sy);
-                wide_sample(M, A, c, ph);
-            } else {
-                const bool input = ph.kind == PH_QKV && ph.layer == 0, depth_attn = ph.kind == PH_WO && fast;
-                if (input || depth_attn) {
-                    rows_sync_in(M, sy);
-                    timer.rest();
-                    if (input) wide_input(M, A, c, ph);
-                    else wide_depth_attention(M, A, c, ph.layer, ph.depth_pos);
-                    timer.step(M, ph);
-                    rows_arrive(M, c, sy);
-                }
-                if (ph.kind == PH_QKV && !fast) attn_prefetch(M, A, c, ph.layer);
-                prompt_gemm<true, kTimed>(M, A, c, ph, sy, chunk, tile, -1);
-                if (ph.kind == PH_WO || ph.kind == PH_W2) {
-                    rows_arrive(M, c, sy);
-                    rows_sync_in(M, sy);
-                    timer.rest();
-                    const bool wo = ph.kind == PH_WO;
-                    const DevLayer* L = fast ? M.fast_layers : M.layers;
-                    uint16_t* stream = fast ? M.xf : M.x;
-                    const uint16_t* norm = wo ? L[ph.layer].ffn_norm : ph.layer + 1 < (fast ? M.n_flayer : M.n_layer) ? L[ph.layer + 1].attention_norm : fast ? M.fast_norm : M.norm;
-                    const int D = fast ? M.fdim : M.dim;
-                    prompt_finish(M, A, c, wo ? stream : M.h, wo ? M.h : stream, D, prompt_slices(wo ? D : fast ? M.finter : M.inter), norm, -1);
-                    timer.step(M, ph);
-                }
-            }
-            if (c.cta == 0 && A.advance && p == A.phase_end - 1)
-                for (int b = c.tid; b < A.batch; b += kThreads) A.b.seq_len[b] = ldcg_i32(A.b.seq_len + b) + 1;
-            timer.end(M, p);
-            if (!(it == A.n_iter - 1 && p == A.phase_end - 1)) rows_arrive(M, c, sy);
-            timer.arrived(M, p);
-        }
-    }
-    if (c.cta == 0 && c.tid == 0) M.barrier[1] = sy.target;
     umma::fence_before_sync();
     __syncthreads();
     if (c.warp == 0) umma::tmem_free(g_pr.tmem_base);

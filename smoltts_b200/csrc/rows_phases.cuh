@@ -85,6 +85,7 @@ __device__ __forceinline__ void rows_stamp(const DevModel& M, int kind, int fast
     M.prof[2 * kMaxProg + (kind + 8 * fast) * 4 + s] += now - t;
     t = now;
 }
+template <bool kTimed>
 __device__ __forceinline__ void rows_arrive(const DevModel& M, const Ctx& c, RowsSync& sy) {
     rows_sync_in(M, sy);       // (a phase in which this CTA has no work may not have waited yet)
     // Shared memory used here is overwritten by copies.  (Rows written here are read by other CTAs' copies: the threads that issue those
@@ -93,7 +94,7 @@ __device__ __forceinline__ void rows_arrive(const DevModel& M, const Ctx& c, Row
     fence_proxy_async();
     grid_arrive(M.barrier, sy.target, (uint32_t)c.n_ctas);
     sy.pending = true;
-    sy.waits_for = sy.phase;
+    if (kTimed) sy.waits_for = sy.phase;
 }
 
 // ---- batch attention on the tensor cores -------------------------------------------------------------------------
@@ -1034,7 +1035,7 @@ __device__ __forceinline__ void phase_rows(const DevModel& M, const CallArgs& A,
     if (tc_has_prestep(ph)) {
         rows_sync_in(M, sy);
         if (A.tc_part == 0 || A.tc_part == 1) rows_embed(M, A, c);
-        if (A.cooperative) rows_arrive(M, c, sy);
+        if (A.cooperative) rows_arrive<kTimed>(M, c, sy);
         if (A.tc_part == 1) return;
     }
     if (ph.kind == PH_QKV && !ph.fast) attn_prefetch(M, A, c, ph.layer);

@@ -1,4 +1,4 @@
-"""The batched decode (csrc/rows_phases.cuh) and the prompt kernel (csrc/prompt_phases.cuh) at the sizes where they can go wrong:
+"""The batched decode (csrc/rows_phases.cuh, csrc/tile_phases.cuh) and the prompt kernel (csrc/prompt_phases.cuh) at the sizes where they can go wrong:
 batches around the row groups, widths whose chains are long or cut unevenly, ragged heads, 16 depth positions, every group size of
 the attention, contexts around its splits, both page sizes.  The yardstick is the CUDA-core variant on the same inputs (itself held to
 the oracle): the two differ by the rounding of bf16 activations only, so their logits by a few bf16 ulps; bits that must not depend on
@@ -204,3 +204,58 @@ def test_phase_recorder_covers_the_launch_once(what):
     assert 0.6 * wall < ns.sum().item() < 1.02 * wall, (ns.sum().item(), wall)
     # waits of many barriers, not of one
     assert ns[:, 1].max() < 0.25 * ns[:, 1].sum()
+
+
+KERNEL = {"groups": 3, "tiles": 4, "prompt": 5}     # SMOL_KERNEL_*
+
+
+@pytest.mark.parametrize("name,batch", [("70m", 9), ("ragged_heads", 40), ("deep", 33), ("long_chains", 130)])
+@pytest.mark.parametrize("mode", [0, 1])
+def test_groups_and_tiles_give_the_same_bits(name, batch, mode):
+    cfg, model = _model(name, batch, 300)
+    model.set_option("mode", mode)
+    lens = [1 + (37 * b) % 280 for b in range(batch)]
+    out = {}
+    for kernel, rows in (("groups", 100000), ("tiles", 0)):
+        model.set_option("tc_group_rows", rows)
+        out[kernel] = _frame(cfg, model, lens, list(range(batch)), 9, frames=2)[:2]
+        assert model.get_option("last_kernel") == KERNEL[kernel]
+    assert all(torch.equal(a, b) for a, b in zip(out["groups"], out["tiles"]))
+
+
+@pytest.mark.parametrize("name", ["long_chains", "70m"])
+@pytest.mark.parametrize("batch,rows", [(9, 100000), (33, 100000), (65, 100000), (65, 0), (160, 0)])
+def test_small_grids_give_the_bits_of_the_whole_one(name, batch, rows):
+    """Fewer CTAs than tile blocks: a CTA walks several blocks of a phase, in groups of rows and on tiles."""
+    cfg, model = _model(name, batch, 150)
+    model.set_option("tc_group_rows", rows)
+    lens = [1 + (37 * b) % 130 for b in range(batch)]
+    want = _frame(cfg, model, lens, list(range(batch)), 9)
+    for n_ctas in (40, 7):
+        model.set_option("n_ctas", n_ctas)
+        got = _frame(cfg, model, lens, list(range(batch)), 9)
+        assert model.get_option("n_ctas") == n_ctas and model.get_option("last_kernel") == KERNEL["groups" if rows else "tiles"]
+        assert all(torch.equal(a.view(torch.int16 if a.dtype == torch.bfloat16 else a.dtype), b.view(torch.int16 if b.dtype == torch.bfloat16 else b.dtype))
+                   for a, b in zip(got, want))
+    model.set_option("n_ctas", 0)
+
+
+@pytest.mark.parametrize("seqs,n,kernel", [(1, 129, "tiles"), (1, 130, "prompt"), (3, 40, "tiles"), (2, 200, "prompt"), (9, 2, "tiles")])
+def test_prefills_have_the_same_bits_in_either_kernel(seqs, n, kernel):
+    """A prefill against the same one cut into tiles of 100 positions: on either side of the line between the kernels."""
+    cfg, model = _model("70m", seqs, 260)
+    prompts = torch.stack([prompt_grid(byte_prompt(max(1, n - 12), seed=s)[-n:], cfg)[:, -n:] for s in range(seqs)]).to(device="cuda", dtype=torch.int32).contiguous()
+    n = prompts.shape[2]
+    lens = torch.tensor([n - (s % 3 if n > 8 else 0) for s in range(seqs)], dtype=torch.int32, device="cuda")
+    out = []
+    for tile in (0, 100):
+        model.set_option("prefill_tile", tile)
+        model.kv_view().zero_()
+        batch = model.new_batch(seqs, max_positions=250)
+        model.prefill(batch, prompts, lens)
+        if tile == 0:
+            assert model.get_option("last_kernel") == KERNEL[kernel]
+        out.append((model.kv_view()[batch.block_table.long()].clone().view(torch.int16), batch.tokens.clone(), batch.seq_len.clone()))
+        batch.release()
+    model.set_option("prefill_tile", 0)
+    assert all(torch.equal(a, b) for a, b in zip(*out))

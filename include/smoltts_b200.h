@@ -136,7 +136,8 @@ int smol_prefill(SmolModel* m, const SmolBatch* b, int32_t batch, const int32_t*
                  const int32_t* d_prompt_len, int32_t s_max, void* stream);
 /* The prompt of ONE sequence and the logits of its last position (batch slot 0): d_prompt [R, n] ids; all n columns are
  * cached (n positions on top of what the sequence holds), the last one also stays in SmolBatch.tokens.  Writes
- * "token_logits" row 0 and "x" row 0.  n must reach option "tc_min_batch" (SMOL_ERR_UNSUPPORTED otherwise). */
+ * "token_logits" row 0 and "x" row 0.  n must reach option "tc_min_batch" (SMOL_ERR_UNSUPPORTED otherwise).
+ * One cooperative launch in every "mode"; iterations of up to 1024 positions, or "prefill_tile" of them. */
 int smol_prompt_logits(SmolModel* m, const SmolBatch* b, const int32_t* d_prompt, int32_t n, void* stream);
 
 /* forward_generate with S == 1 (M:173-192): embed(tokens) -> slow layers (KV append at
@@ -205,7 +206,8 @@ int smol_set_frame_clock(SmolModel* m, uint64_t* d_frame_ns, int32_t capacity);
  * which the tensor-core variant works in groups of rows, above which on 128-row tiles (-1, the default: whichever is expected to be faster;
  * the results have the same bits).
  * smol_get_option also answers "n_sms", "smem_bytes", "ll_ready", "tc_ready" (1 once the tensor-core variant has been set up),
- * "last_kernel" (SMOL_KERNEL_* of the last launch). */
+ * "last_kernel" (SMOL_KERNEL_* of the last launch), "prompt_min_rows" (a prompt of MORE positions whose prefill would take the tensor-core
+ * variant goes through smol_prompt_logits in forward_generate; 0: none, as in "mode" 1 or with a "prefill_tile" below "tc_min_batch"). */
 enum { SMOL_KERNEL_NONE = 0, SMOL_KERNEL_CUDA_CORES = 1, SMOL_KERNEL_DATAFLOW = 2, SMOL_KERNEL_GROUPS = 3, SMOL_KERNEL_TILES = 4, SMOL_KERNEL_PROMPT = 5 };
 int smol_set_option(SmolModel* m, const char* name, int64_t value);
 int64_t smol_get_option(const SmolModel* m, const char* name);

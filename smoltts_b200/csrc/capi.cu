@@ -579,6 +579,9 @@ static int launch_tiles(SmolModel* m, const CallArgs& A, int n_ctas, cudaStream_
     return SMOL_OK;
 }
 
+// Positions of one sequence that a prompt iteration takes at most: the workspace's rows, or the caller's cap.
+static int prompt_cap(const SmolModel* m) { return m->prefill_tile > 0 && m->prefill_tile < kPrefillRows ? m->prefill_tile : kPrefillRows; }
+
 // The prompt of one sequence as one cooperative launch (in every mode).
 static int enqueue_prompt(SmolModel* m, CallArgs A, cudaStream_t stream) {
     int rc = ensure_tmaps(m);
@@ -731,9 +734,7 @@ int smol_prompt_logits(SmolModel* m, const SmolBatch* b, const int32_t* d_prompt
     if (!use_tc(m, n)) return fail(SMOL_ERR_UNSUPPORTED, "smol_prompt_logits: fewer positions than option \"tc_min_batch\", or a model outside the tensor-core variant");
     CallArgs A = base_args(b, 1, nullptr);
     A.mode = 1;
-    int T = n < kPrefillRows ? n : kPrefillRows;
-    if (m->prefill_tile > 0 && m->prefill_tile < T) T = m->prefill_tile;
-    if (!use_tc(m, T)) T = m->tc_min_batch;
+    const int T = n < prompt_cap(m) ? n : prompt_cap(m);
     A.tile_t = T;
     A.batch = T;
     A.prompt = d_prompt;
@@ -946,6 +947,8 @@ int64_t smol_get_option(const SmolModel* m, const char* name) {
     if (!std::strcmp(name, "n_sms")) return m->n_sms;
     if (!std::strcmp(name, "smem_bytes")) return (int64_t)m->smem[1];
     if (!std::strcmp(name, "tc_min_batch")) return m->tc_min_batch;
+    if (!std::strcmp(name, "prefill_tile")) return m->prefill_tile;
+    if (!std::strcmp(name, "prompt_min_rows")) return m->mode != 1 && use_tc(m, prompt_cap(m)) ? m->tc_min_batch : 0;
     if (!std::strcmp(name, "tc_ready")) return m->tile_ready[0] || m->tiles_ready || m->prompt_ready ? 1 : 0;
     if (!std::strcmp(name, "tc_group_rows")) return m->tc_group_rows;
     if (!std::strcmp(name, "last_kernel")) return m->last_kernel;

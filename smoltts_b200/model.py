@@ -392,13 +392,6 @@ class RQTransformer:
         return out
 
     @property
-    def _prompt_rows(self) -> int:
-        """Positions from which a prompt takes the tensor-core variant (0: never)."""
-        cfg = self.config
-        eligible = all(d % 64 == 0 for d in (cfg.dim, cfg.fast_dim, cfg.intermediate_size, cfg.fast_intermediate_size))
-        return self.get_option("tc_min_batch") if eligible else 0
-
-    @property
     def phase_count(self) -> int:
         return int(self.lib.smol_phase_count(self._h))
 
@@ -454,7 +447,7 @@ class RQTransformer:
         x = x.to(device=self.device, dtype=torch.int32).contiguous()
         S = x.shape[2]
         batch = cache.batch
-        if S > self._prompt_rows > 0:
+        if S > self.get_option("prompt_min_rows") > 0:
             # one pass: every position through the layers, the last one also through the LM head (the bits are those of a prefill
             # of the first S - 1 positions, which is what the variant counts, and a step for the last)
             if batch.host_len[0] + S > batch.capacity:

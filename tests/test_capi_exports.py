@@ -123,3 +123,26 @@ def test_mimi_create_validates_shapes_without_a_gpu():
     assert lib.smol_mimi_create(ctypes.byref(make(head_dim=48)), ctypes.byref(h2)) == _capi.SMOL_ERR_INVALID
     assert lib.smol_mimi_create(ctypes.byref(make(max_positions=7)), ctypes.byref(h2)) == _capi.SMOL_ERR_INVALID
     assert lib.smol_mimi_create(ctypes.byref(make(max_positions=4000000)), ctypes.byref(h2)) == _capi.SMOL_ERR_CAPACITY
+
+
+def test_prompts_go_in_one_pass_only_where_a_prefill_iteration_takes_the_tensor_core_variant():
+    """The rule that forward_generate asks for: a workspace holds 1024 rows of a prompt (and the caller may cap them), so a larger
+    tc_min_batch, which no iteration reaches, leaves prompts to the prefill."""
+    from smoltts_b200 import _capi
+    from smoltts_b200.config import named_config
+
+    cfg = named_config("smoltts_byte_tiny")
+    c = _capi.SmolConfig(**{n: int(getattr(cfg, n)) for n, _ in _capi.SmolConfig._fields_ if hasattr(cfg, n) and n not in ("norm_eps",)})
+    c.norm_eps, c.max_batch, c.page_size, c.head_dim, c.fast_head_dim = 1e-5, 1, 32, 64, 64
+    lib, h = _capi.load(), ctypes.c_void_p()
+    assert lib.smol_create(ctypes.byref(c), ctypes.byref(h)) == 0
+
+    def rows(**options):
+        for name in ("mode", "tc_min_batch", "prefill_tile"):
+            assert lib.smol_set_option(h, name.encode(), options.get(name, {"mode": 2, "tc_min_batch": 9, "prefill_tile": 0}[name])) == 0
+        return lib.smol_get_option(h, b"prompt_min_rows")
+
+    assert rows() == 9 and rows(mode=0) == 9 and rows(tc_min_batch=30) == 30 and rows(tc_min_batch=1024) == 1024 and rows(prefill_tile=9) == 9
+    assert rows(tc_min_batch=1025) == 0 and rows(tc_min_batch=1 << 30) == 0
+    assert rows(tc_min_batch=0) == 0 and rows(prefill_tile=8) == 0 and rows(mode=1) == 0
+    lib.smol_destroy(h)

@@ -259,3 +259,40 @@ def test_prefills_have_the_same_bits_in_either_kernel(seqs, n, kernel):
         batch.release()
     model.set_option("prefill_tile", 0)
     assert all(torch.equal(a, b) for a, b in zip(*out))
+
+
+def _prompt_logits(model, cache, prompt):
+    import ctypes
+
+    from smoltts_b200 import _capi
+
+    _capi.check(model.lib.smol_prompt_logits(model._h, ctypes.byref(cache.batch.c), ctypes.c_void_p(prompt.data_ptr()), prompt.shape[2], model._stream()))
+    torch.cuda.synchronize()
+    return model.debug_buffer("token_logits", 1).clone()
+
+
+def test_prompt_iterations_stay_within_the_workspace_and_the_callers_cap():
+    """A tc_min_batch above the workspace's 1024 rows, and caps below tc_min_batch: the iterations follow the workspace and the cap, the
+    logits stay; forward_generate then leaves the prompt to prefill and step."""
+    cfg, model = _model("70m", 1, 1400)
+    prompt = prompt_grid(byte_prompt(1288, seed=4), cfg)[None].to(device="cuda", dtype=torch.int32)
+    cache = make_prompt_cache(model)
+    want, _ = model.forward_generate(prompt, cache)
+    assert model.get_option("last_kernel") == KERNEL["prompt"]
+    cache.batch.release()
+    for options in (dict(tc_min_batch=1200), dict(prefill_tile=5), dict(prefill_tile=1)):
+        for name, value in options.items():
+            model.set_option(name, value)
+        cache = make_prompt_cache(model)
+        assert torch.equal(_prompt_logits(model, cache, prompt), want) and int(cache.batch.seq_len[0]) == 1300
+        cache.batch.release()
+        assert model.get_option("prompt_min_rows") == 0
+        model.set_option("tc_min_batch", 9)
+        model.set_option("prefill_tile", 0)
+    model.set_option("tc_min_batch", 1200)
+    cache = make_prompt_cache(model)
+    logits, _ = model.forward_generate(prompt, cache)
+    assert model.get_option("last_kernel") == 1 and cache.batch.host_len == [1300]      # CUDA cores
+    _close(logits, want, "token logits")
+    cache.batch.release()
+    model.set_option("tc_min_batch", 9)

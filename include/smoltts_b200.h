@@ -37,7 +37,8 @@ enum {
     SMOL_ERR_UNBOUND = -2,     /* weights / workspace / KV pool not bound yet */
     SMOL_ERR_CUDA = -3,        /* a CUDA runtime call failed (message has the reason) */
     SMOL_ERR_UNSUPPORTED = -4, /* config feature outside the decode path built so far */
-    SMOL_ERR_CAPACITY = -5     /* batch / context exceeds what was configured */
+    SMOL_ERR_CAPACITY = -5,    /* batch / context exceeds what was configured */
+    SMOL_ERR_TIMEOUT = -6      /* a wait inside an earlier launch ran out (option "wait_ms"): results since then are not valid */
 };
 
 /* Model shape: RQTransformerModelArgs (P:25-114; M:10-48) + token ids (TokenConfig M:51-89). */
@@ -205,6 +206,9 @@ int smol_set_frame_clock(SmolModel* m, uint64_t* d_frame_ns, int32_t capacity);
  * (0 = as many as fit: 1024 rows on the tensor-core variant, 8 on the CUDA-core variants);  "tc_group_rows" = rows of a decode call up to
  * which the tensor-core variant works in groups of rows, above which on 128-row tiles (-1, the default: whichever is expected to be faster;
  * the results have the same bits).
+ * "wait_ms" (default 2000) = how long a wait inside the batched decode and the prompt kernel may take before the launch gives up: it
+ * ends, and the model's next compute call returns SMOL_ERR_TIMEOUT, once ("device_status" answers 1 until then);  "wait_probe" 1 = the next
+ * such launch waits for something that never happens (a test of that report).
  * smol_get_option also answers "n_sms", "smem_bytes", "ll_ready", "tc_ready" (1 once the tensor-core variant has been set up),
  * "last_kernel" (SMOL_KERNEL_* of the last launch), "prompt_min_rows" (a prompt of MORE positions whose prefill would take the tensor-core
  * variant goes through smol_prompt_logits in forward_generate; 0: none, as in "mode" 1 or with a "prefill_tile" below "tc_min_batch"). */

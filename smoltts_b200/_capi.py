@@ -15,7 +15,7 @@ SMOL_ABI_VERSION = 1
 SMOL_MAX_LAYERS = 64
 SMOL_MAX_FAST_LAYERS = 16
 
-from ._errors import (SMOL_ERR_CAPACITY, SMOL_ERR_CUDA, SMOL_ERR_INVALID, SMOL_ERR_UNBOUND, SMOL_ERR_UNSUPPORTED, SMOL_OK,  # noqa: F401
+from ._errors import (SMOL_ERR_CAPACITY, SMOL_ERR_CUDA, SMOL_ERR_INVALID, SMOL_ERR_TIMEOUT, SMOL_ERR_UNBOUND, SMOL_ERR_UNSUPPORTED, SMOL_OK,  # noqa: F401
                       SmolError)
 
 

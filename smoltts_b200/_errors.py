@@ -5,6 +5,7 @@ SMOL_ERR_UNBOUND = -2
 SMOL_ERR_CUDA = -3
 SMOL_ERR_UNSUPPORTED = -4
 SMOL_ERR_CAPACITY = -5
+SMOL_ERR_TIMEOUT = -6
 
 
 class SmolError(RuntimeError):

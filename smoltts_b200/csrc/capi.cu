@@ -76,6 +76,8 @@ struct SmolModel {
     size_t ll2_smem = 0;
     int tc_group_rows = -1;    // rows of a decode batch up to which it runs in groups of rows (-1: in_groups decides)
     int last_kernel = 0;       // SMOL_KERNEL_* of the last launch
+    uint32_t* status = nullptr;    // the kernels' status word (DevModel.status), in mapped host memory
+    int wait_probe = 0;        // launches whose first block waits for something that never happens
     bool tmaps_ready = false;  // tensor maps of the 128-row tiles (rebuilt after a weight / workspace bind)
     bool tiles_ready = false, prompt_ready = false;   // the kernels' function attributes
     bool packed_ready = false; // tensor-core GEMV layout of the bound weights (rebuilt after a weight / workspace bind)
@@ -242,6 +244,7 @@ int smol_create(const SmolConfig* cfg, SmolModel** out) {
     d.codebook_size = c.codebook_size; d.num_codebooks = c.num_codebooks; d.depth = depth; d.n_rows = 1 + depth;
     d.dup0 = c.duplicate_code_0; d.depthwise_wte = c.depthwise_wte; d.depthwise_output = c.depthwise_output;
     d.max_seq_len = c.max_seq_len; d.max_batch = c.max_batch; d.page_size = c.page_size;
+    d.wait_ms = 2000;
     d.semantic_start = c.semantic_start_id; d.semantic_end = c.semantic_end_id; d.im_end = c.im_end_id;
     d.mlx_embed_mask = c.mlx_embed_mask; d.eps = c.norm_eps;
     const int n_prog = smol::phases_per_frame(d.n_layer, d.n_flayer, d.depth);
@@ -259,6 +262,7 @@ int smol_create(const SmolConfig* cfg, SmolModel** out) {
 
 void smol_destroy(SmolModel* m) {
     if (!m) return;
+    if (m->status) cudaFreeHost(m->status);
     if (m->frame_graph) cudaGraphExecDestroy(m->frame_graph);
     if (m->capture_stream) cudaStreamDestroy(m->capture_stream);
     delete m;
@@ -322,6 +326,11 @@ int smol_bind_workspace(SmolModel* m, void* d_workspace, size_t bytes) {
     d.x = (uint16_t*)(base + L.x); d.h = (uint16_t*)(base + L.h); d.xf = (uint16_t*)(base + L.xf);
     d.q = (uint16_t*)(base + L.q); d.attn = (uint16_t*)(base + L.attn); d.act = (uint16_t*)(base + L.act);
     d.fkv = (uint16_t*)(base + L.fkv);
+    if (!m->status) {
+        CU(cudaHostAlloc((void**)&m->status, sizeof(uint32_t), cudaHostAllocMapped | cudaHostAllocPortable));
+        *m->status = 0u;
+    }
+    CU(cudaHostGetDevicePointer((void**)&d.status, m->status, 0));
     d.xn = (uint16_t*)(base + L.xn); d.tmaps = (const unsigned char*)(base + L.tmaps);
     d.kpart = (float*)(base + L.kpart); d.ws_rows = ws_rows(m->cfg);
     m->tmaps_ready = false;
@@ -370,6 +379,12 @@ int smol_kv_bind(SmolModel* m, void* d_kv_pool, int32_t n_pages) {
 static int ensure_configured(SmolModel* m) {
     if (!m->weights_bound || !m->ws_bound || !m->kv_bound)
         return fail(SMOL_ERR_UNBOUND, "weights, workspace and KV pool must be bound before compute calls");
+    if (*reinterpret_cast<volatile uint32_t*>(m->status) != 0u) {
+        CU(cudaDeviceSynchronize());
+        CU(cudaMemset(m->dm.barrier, 0, 256));     // (its counter is poisoned)
+        *m->status = 0u;
+        return fail(SMOL_ERR_TIMEOUT, "a wait inside an earlier launch ran out: the results since then are not valid");
+    }
     if (m->configured) return SMOL_OK;
     CU(cudaGetDevice(&m->device));
     int coop = 0;
@@ -594,6 +609,7 @@ static int enqueue_prompt(SmolModel* m, CallArgs A, cudaStream_t stream) {
     }
     A.cooperative = 1;
     A.tc_split = m->tc_attn_split;
+    if (m->wait_probe > 0) { A.wait_probe = 1; --m->wait_probe; }
     std::memcpy(A.kv_map, m->kv_map, sizeof(A.kv_map));
     CU(smol::prompt_launch(m->dm, A, m->n_ctas, stream));
     m->launches += 1;
@@ -625,6 +641,7 @@ static int enqueue(SmolModel* m, CallArgs A, cudaStream_t stream, bool whole_ite
         if ((rc = ensure_tile(m, bt))) return rc;
         if (bt == 0) {
             smol::rows_plan(m->dm, A.batch, m->n_ctas, A.rows_plan);
+            if (m->wait_probe > 0 && m->mode != 1) { A.wait_probe = 1; --m->wait_probe; }
             std::memcpy(A.kv_map, m->kv_map, sizeof(A.kv_map));
         }
     }
@@ -911,6 +928,16 @@ int smol_set_option(SmolModel* m, const char* name, int64_t value) {
         m->frame_key_valid = false;  // a cached frame graph was captured for the other kernel variant
         return SMOL_OK;
     }
+    if (!std::strcmp(name, "wait_ms")) {
+        if (value < 1 || value > 60000) return fail(SMOL_ERR_INVALID, "wait_ms must be in [1, 60000]");
+        m->dm.wait_ms = (uint32_t)value;
+        m->frame_key_valid = false;
+        return SMOL_OK;
+    }
+    if (!std::strcmp(name, "wait_probe")) {
+        m->wait_probe = value > 0 ? 1 : 0;
+        return SMOL_OK;
+    }
     if (!std::strcmp(name, "tc_group_rows")) {
         m->tc_group_rows = value < 0 ? -1 : value > 0x7fffffff ? 0x7fffffff : (int)value;
         m->frame_key_valid = false;
@@ -952,6 +979,8 @@ int64_t smol_get_option(const SmolModel* m, const char* name) {
     if (!std::strcmp(name, "tc_ready")) return m->tile_ready[0] || m->tiles_ready || m->prompt_ready ? 1 : 0;
     if (!std::strcmp(name, "tc_group_rows")) return m->tc_group_rows;
     if (!std::strcmp(name, "last_kernel")) return m->last_kernel;
+    if (!std::strcmp(name, "wait_ms")) return m->dm.wait_ms;
+    if (!std::strcmp(name, "device_status")) return m->status ? (int64_t)*reinterpret_cast<volatile uint32_t*>(m->status) : 0;
     if (!std::strcmp(name, "ll_smem_bytes")) return (int64_t)m->ll2_smem;
     if (!std::strcmp(name, "ll_ready")) return (int64_t)m->ll2_state;
     if (!std::strcmp(name, "ll_max_batch")) return (int64_t)m->ll2_max_batch;

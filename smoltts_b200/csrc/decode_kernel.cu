@@ -100,6 +100,40 @@ __device__ __forceinline__ void grid_wait(uint32_t* ctr, uint32_t target) {
     __syncthreads();
 }
 
+// ---- a launch that gives up ------------------------------------------------------------------------
+// The waits of groups of rows and of prompts are bounded (DevModel.wait_ms).  Where one runs out, its block poisons the grid barrier's counter:
+// every barrier of the launch is complete for everybody from then on, and a block that passes one leaves its phase loop.  The
+// status word lies in host memory: the model's next call reports it and puts the barrier right.
+constexpr uint32_t kPoison = 0x40000000u;      // (more than a launch's arrivals, less than the wrap-safe compare allows)
+constexpr unsigned long long kWaitOver = ~0ull;
+__shared__ uint32_t g_gave_up;
+// t0: when this wait was first found long (0: not yet); returns that, or kWaitOver.
+__device__ __noinline__ unsigned long long wait_over(uint32_t* barrier, uint32_t* status, unsigned long long ms, unsigned long long t0) {
+    if (*reinterpret_cast<volatile uint32_t*>(&g_gave_up) != 0u) return kWaitOver;
+    const unsigned long long now = globaltimer_ns();
+    if (t0 == 0ull) return now;
+    if (now - t0 < ms * 1000000ull) return t0;
+    *reinterpret_cast<volatile uint32_t*>(&g_gave_up) = 1u;
+    if (atomicExch(barrier + 2, 1u) == 0u) atomicAdd(barrier, kPoison);
+    *reinterpret_cast<volatile uint32_t*>(status) = 1u;
+    __threadfence_system();
+    return kWaitOver;
+}
+// One thread: until `target` arrivals; true: the launch is given up.
+__device__ __forceinline__ bool grid_poll(uint32_t* ctr, uint32_t* status, uint32_t ms, uint32_t target) {
+    uint32_t v;
+    unsigned long long t0 = 0ull;
+    for (uint32_t spin = 1;; ++spin) {
+        asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(ctr) : "memory");
+        if ((int32_t)(v - target) >= 0) break;
+        if ((spin & 1023u) == 0u) {
+            t0 = wait_over(ctr, status, 4ull * ms, t0);     // (the others' waits run out first)
+            if (t0 == kWaitOver) return true;
+        }
+    }
+    return v - target >= kPoison / 2;
+}
+
 // ---- mbarrier + TMA bulk copy (global -> shared) ---------------------------------------------------
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 __device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) {
@@ -107,6 +141,15 @@ __device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) {
 }
 __device__ __forceinline__ void mbar_expect_tx(uint64_t* bar, uint32_t bytes) {
     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ bool mbar_try(uint64_t* bar, uint32_t parity) {
+    uint32_t ok;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}\n"
+        : "=r"(ok) : "r"(smem_u32(bar)), "r"(parity) : "memory");
+    return ok != 0u;
 }
 __device__ __forceinline__ void mbar_wait(uint64_t* bar, uint32_t parity) {
     asm volatile(
@@ -939,8 +982,10 @@ smol_decode_kernel(const __grid_constant__ DevModel M, const __grid_constant__ C
             if (BT == 0) { for (int i = 2 * w; i < 2 * w + 2; ++i) { mbar_init(&g_kvbar[i], 1u); g_kvpar[i] = 0u; } }
         }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        if (BT == 0) g_gave_up = 0u;
     }
     __syncthreads();
+    if (BT == 0 && A.wait_probe && c.cta == 0 && c.tid == 0) rows_wait(M, &g_kvbar[2 * kWarps - 1], 0u);   // (nothing completes it)
 
     uint32_t target = 0;
     if (A.cooperative) target = ldcg_u32(M.barrier + 1);
@@ -951,16 +996,16 @@ smol_decode_kernel(const __grid_constant__ DevModel M, const __grid_constant__ C
     const bool prof = prof_cta && c.tid == 0;
     unsigned long long t0 = 0, t1 = 0;
     RowsSync sy;
-    sy.target = target; sy.par_w = 0; sy.par_x = 0; sy.pending = false; sy.phase = 0; sy.next = -1; sy.waits_for = 0;
+    sy.target = target; sy.par_w = 0; sy.par_x = 0; sy.pending = false; sy.failed = false; sy.phase = 0; sy.next = -1; sy.waits_for = 0;
     RowsStep* steps = reinterpret_cast<RowsStep*>(smem_dyn);   // tensor-core variant: phase table | rows, partial sums | weights
     if (BT == 0) {
         c.xs = reinterpret_cast<float*>(smem_dyn + xs_bytes - kRowsP);
         rows_tables(M, A, c, steps);
     }
     int st_it = -1, st_p = -1;  // (iteration, phase) whose weights are staged / in flight
-    for (int it = 0; it < A.n_iter; ++it) {
+    for (int it = 0; it < A.n_iter && !(BT == 0 && sy.failed); ++it) {
         c.iter = it;
-        for (int p = A.phase_begin; p < A.phase_end; ++p) {
+        for (int p = A.phase_begin; p < A.phase_end && !(BT == 0 && sy.failed); ++p) {
             const uint32_t packed_phase = M.prog[p];
             const Phase ph = unpack_phase(packed_phase);
             const bool has_w = ph.kind != PH_ATTN && ph.kind != PH_SAMPLE;  // weights are staged a phase ahead
@@ -1000,7 +1045,7 @@ smol_decode_kernel(const __grid_constant__ DevModel M, const __grid_constant__ C
             const bool last = (it == A.n_iter - 1) && (p == A.phase_end - 1);
             const bool sync = A.cooperative && !last;
             if (BT == 0) {
-                if (sync) rows_arrive<kTimed>(M, c, sy);
+                if (sync && !sy.failed) rows_arrive<kTimed>(M, c, sy);
                 if (prof) {   // [2p]: rows_sync_in takes the waits inside the phase off; [2p + 1]: the arrival, then the wait, which the phase behind adds
                     M.prof[2 * p] += t1 - t0;
                     M.prof[2 * p + 1] += globaltimer_ns() - t1;
@@ -1033,6 +1078,15 @@ smol_decode_kernel(const __grid_constant__ DevModel M, const __grid_constant__ C
             const int b = i / M.n_rows, r = i - b * M.n_rows;
             A.b.tokens[i] = ldcg_i32(A.prompt + ((size_t)b * M.n_rows + r) * A.s_max + prompt_last(A, b));
         }
+    }
+    if (BT == 0 && sy.failed) {     // the next phase's tiles may still be landing
+        if (c.tid == 0 && sy.next >= 0) {
+            const Phase ph = unpack_phase(M.prog[sy.next]);
+            const unsigned long long t0 = globaltimer_ns();
+            if (g_rk[ph.fast][ph.kind].bytes != 0u) while (!mbar_try(&g_mbar[0], sy.par_w) && globaltimer_ns() - t0 < (unsigned long long)M.wait_ms * 1000000ull) {}
+        }
+        __syncthreads();
+        return;
     }
     if (A.cooperative && c.cta == 0 && c.tid == 0) M.barrier[1] = BT == 0 ? sy.target : target;
 }

@@ -140,6 +140,9 @@ struct DevModel {
 
     RowsLayer rows_layers[SMOL_MAX_LAYERS], rows_fast_layers[SMOL_MAX_FAST_LAYERS];   // batched decode: fragments
     const uint16_t *rows_head, *rows_fast_output;
+
+    uint32_t* status;    // host memory: 1 = a wait of a launch ran out
+    uint32_t wait_ms;    // how long a wait may take
 };
 
 // Words (8 bytes, two bf16 + epoch) one sequence publishes in a phase; multiples of 16 words (128 B).
@@ -188,6 +191,7 @@ struct CallArgs {
     const int32_t* prompt_len;  // prefill: [B]
     int s_max;
     int whole_prompt; // prefill: cache all prompt_len positions (1) or all but the last, which stays pending (0)
+    int wait_probe;   // wait for something that never happens (tests of the report)
     int head_row;     // whole_prompt: row of the last prompt position in the last tile
     RowsPlan rows_plan[2][6];   // tensor-core variant: [slow / depth transformer][phase kind]
     alignas(64) unsigned char kv_map[128];   // ... tensor map of the paged pool: rows of 64 elements, boxes of 16 rows

@@ -406,12 +406,13 @@ __device__ __forceinline__ void prompt_setup(const DevModel& Mp, const CallArgs&
         mbar_init(&g_pr.acc_empty, (uint32_t)(kWarps - kPrEpilogueWarp));
         for (int i = 0; i < 2 * kWarps; ++i) { mbar_init(&g_kvbar[i], 1u); g_kvpar[i] = 0u; }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        g_gave_up = 0u;
     }
     if (c.warp == 0) umma::tmem_alloc(&g_pr.tmem_base);
     umma::fence_before_sync();
     __syncthreads();
     umma::fence_after_sync();
-    sy.target = ldcg_u32(Mp.barrier + 1); sy.par_w = 0; sy.par_x = 0; sy.pending = false; sy.phase = 0; sy.next = -1; sy.waits_for = 0;
+    sy.target = ldcg_u32(Mp.barrier + 1); sy.par_w = 0; sy.par_x = 0; sy.pending = false; sy.failed = false; sy.phase = 0; sy.next = -1; sy.waits_for = 0;
 }
 
 // The phase recorder (thread 0 of CTA 0, profiling builds): a phase's time without its waits (rows_sync_in takes them off), the
@@ -437,7 +438,8 @@ smol_prompt_kernel(const __grid_constant__ DevModel Mp, const __grid_constant__ 
     RowsSync sy;
     prompt_setup(Mp, Ap, smem_dyn, c, sy);
     uint32_t chunk = 0, tile = 0;
-    for (int it = 0; it < A.n_iter; ++it) {
+    if (A.wait_probe && c.cta == 0 && c.tid == 0) rows_wait(M, &g_kvbar[2 * kWarps - 1], 0u);   // (nothing completes it)
+    for (int it = 0; it < A.n_iter && !sy.failed; ++it) {
         c.iter = it;
         const bool last_iter = it == A.n_iter - 1;
         const int last_row = last_iter && A.whole_prompt > 0 ? A.head_row : -1;
@@ -448,7 +450,7 @@ smol_prompt_kernel(const __grid_constant__ DevModel Mp, const __grid_constant__ 
         tile_row_step(M, A, c, M.dim, M.x, M.layers[0].attention_norm, [&](int bg, int ch, float (&x)[8]) { embed_chunk(M, A, c, bg, ch, x); });
         timer.step(M, unpack_phase(M.prog[0]));
         rows_arrive<kTimed>(M, c, sy);
-        for (int p = 0; p < phases_per_prefill_step(M.n_layer); ++p) {
+        for (int p = 0; p < phases_per_prefill_step(M.n_layer) && !sy.failed; ++p) {
             const Phase ph = unpack_phase(M.prog[p]);
             if (kTimed) sy.phase = p;
             if (ph.kind == PH_ATTN) {
@@ -476,11 +478,11 @@ smol_prompt_kernel(const __grid_constant__ DevModel Mp, const __grid_constant__ 
                 }
             }
             timer.end(M, p);
-            if (!(last_iter && A.whole_prompt == 0 && p == phases_per_prefill_step(M.n_layer) - 1)) rows_arrive<kTimed>(M, c, sy);
+            if (!sy.failed && !(last_iter && A.whole_prompt == 0 && p == phases_per_prefill_step(M.n_layer) - 1)) rows_arrive<kTimed>(M, c, sy);
             timer.arrived(M, p);
         }
     }
-    if (A.whole_prompt > 0) {
+    if (A.whole_prompt > 0 && !sy.failed) {
         if (kTimed) sy.phase = 5 * M.n_layer;        // the LM head's
         PhaseTimer<kTimed> timer(c);
         rows_sync_in(M, sy);
@@ -494,7 +496,7 @@ smol_prompt_kernel(const __grid_constant__ DevModel Mp, const __grid_constant__ 
         }
         timer.end(M, 5 * M.n_layer);
     }
-    if (c.cta == 0) {
+    if (c.cta == 0 && !sy.failed) {
         // leave the last prompt column as the pending input of the first decode frame (G:66-73)
         for (int i = c.tid; i < A.real_batch * M.n_rows; i += kThreads) {
             const int b = i / M.n_rows, r = i - b * M.n_rows;

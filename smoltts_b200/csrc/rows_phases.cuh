@@ -43,17 +43,14 @@ __device__ __forceinline__ uint4 pack8(const float (&f)[8]) {
     return v;
 }
 
-// Bounded wait: a copy that never lands ends the launch with wrong results instead of a hung GPU.
-__device__ __forceinline__ void rows_wait(uint64_t* bar, uint32_t parity) {
-    const uint32_t a = smem_u32(bar);
-    for (uint32_t spin = 0; spin < (1u << 24); ++spin) {
-        uint32_t ok;
-        asm volatile(
-            "{\n\t.reg .pred p;\n\t"
-            "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-            "selp.u32 %0, 1, 0, p;\n\t}\n"
-            : "=r"(ok) : "r"(a), "r"(parity) : "memory");
-        if (ok) return;
+// A wait that runs out ends the launch and is reported by the model's next call (wait_over).
+__device__ __forceinline__ void rows_wait(const DevModel& M, uint64_t* bar, uint32_t parity) {
+    unsigned long long t0 = 0ull;
+    for (uint32_t spin = 1; !mbar_try(bar, parity); ++spin) {
+        if ((spin & 255u) == 0u) {
+            t0 = wait_over(M.barrier, M.status, M.wait_ms, t0);
+            if (t0 == kWaitOver) return;
+        }
     }
 }
 
@@ -62,7 +59,7 @@ __device__ __forceinline__ void rows_wait(uint64_t* bar, uint32_t parity) {
 struct RowsSync {
     uint32_t target;         // arrivals the barrier completes at
     uint32_t par_w, par_x;   // parities of the weight and the row copies
-    bool pending;
+    bool pending, failed;    // failed: the launch was given up (the same in all threads)
     int phase, next;         // this phase; the launch's next weight phase (-1: none), whose tiles this one fetches
     int waits_for;           // the phase whose barrier is pending
 };
@@ -71,7 +68,7 @@ __device__ __forceinline__ void rows_sync_in(const DevModel& M, RowsSync& sy) {
     const bool prof = M.prof != nullptr && blockIdx.x == 0 && threadIdx.x == 0;
     unsigned long long t = 0;
     if (prof) t = globaltimer_ns();
-    grid_wait(M.barrier, sy.target);
+    sy.failed = __syncthreads_or(threadIdx.x == 0 && grid_poll(M.barrier, M.status, M.wait_ms, sy.target)) != 0;
     sy.pending = false;
     if (prof) {   // belongs to the phase in front of the barrier, not to the one that waits
         t = globaltimer_ns() - t;
@@ -292,7 +289,7 @@ __device__ __forceinline__ void phase_attn_batch(const DevModel& M, const CallAr
                 }
                 while (fetched < pl && fetched < p0 + 16 * depth) fetch();
                 for (int pb = p0; pb < pl; pb += 16) {
-                    rows_wait(&g_kvbar[buf0 + at], __shfl_sync(0xffffffffu, par, at));
+                    rows_wait(M, &g_kvbar[buf0 + at], __shfl_sync(0xffffffffu, par, at));
                     const unsigned char* kt = stage + at * 4096;
                     if (lane == at) par ^= 1u;
                     at = at + 1 < depth ? at + 1 : 0;
@@ -769,7 +766,7 @@ __device__ __forceinline__ void rows_gemm(const DevModel& M, const CallArgs& A, 
                 page = ldcg_i32(A.b.block_table + (size_t)bs * A.b.max_pages + p / M.page_size);
             g_rpos[i] = p; g_rpage[i] = page;
         }
-        if (!wide && !landed) { rows_wait(&g_mbar[0], sy.par_w); sy.par_w ^= 1u; landed = true; }
+        if (!wide && !landed) { rows_wait(M, &g_mbar[0], sy.par_w); sy.par_w ^= 1u; landed = true; }
         rows_sync_in(M, sy);
         const bool timed = kTimed && blockIdx.x == 0 && tid == 0;
         unsigned long long stamp = 0ull;
@@ -813,7 +810,7 @@ __device__ __forceinline__ void rows_gemm(const DevModel& M, const CallArgs& A, 
             if (t < nt && row < n_live)
                 pre = ldcg_u32(rk.res + (size_t)(uint32_t)((r0 + row) * rk.n_out + ((block * rk.mt + t) * 16 + (item_w(tid) & ~1))));
         }
-        if (!kDepthAttn) { rows_wait(&g_mbar[1], sy.par_x); sy.par_x ^= 1u; }
+        if (!kDepthAttn) { rows_wait(M, &g_mbar[1], sy.par_x); sy.par_x ^= 1u; }
         if (timed) rows_stamp(M, kind, ph.fast, 0, stamp);
         if (normed) {
             // a warp per row, two at a time: their chains of shuffles and divisions run side by side

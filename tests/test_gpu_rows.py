@@ -296,3 +296,34 @@ def test_prompt_iterations_stay_within_the_workspace_and_the_callers_cap():
     _close(logits, want, "token logits")
     cache.batch.release()
     model.set_option("tc_min_batch", 9)
+
+
+@pytest.mark.parametrize("what", ["frames", "prompt"])
+def test_a_wait_that_runs_out_ends_the_launch_and_the_next_call_reports_it(what):
+    """One block waits for something that nothing completes: the launch ends by itself, without a CUDA error; the next call says so, and the
+    call after that works, with the bits of one that never failed."""
+    from smoltts_b200 import _capi
+
+    cfg, model = _model("70m", 12, 200)
+    lens = [1 + (37 * b) % 170 for b in range(12)]
+    prompt = prompt_grid(byte_prompt(88, seed=1), cfg)[None].to(device="cuda", dtype=torch.int32)
+
+    def run():
+        if what == "frames":
+            return _frame(cfg, model, lens, list(range(12)), 9, frames=3)[:2]
+        cache = make_prompt_cache(model)
+        out = tuple(t.clone() for t in model.forward_generate(prompt, cache))
+        torch.cuda.synchronize()
+        cache.batch.release()
+        return out
+
+    want = run()
+    model.set_option("wait_ms", 20)
+    model.set_option("wait_probe", 1)
+    run()
+    assert model.get_option("device_status") == 1
+    with pytest.raises(_capi.SmolError) as e:
+        run()
+    assert e.value.code == _capi.SMOL_ERR_TIMEOUT and model.get_option("device_status") == 0
+    model.set_option("wait_ms", 2000)
+    assert all(torch.equal(a, b) for a, b in zip(run(), want))

@@ -565,8 +565,9 @@ static bool use_tc(const SmolModel* m, int rows) {
 // A decode batch runs in groups of rows (rows_phases.cuh) or, where that is faster, on 128-row tiles (tile_phases.cuh): groups are taken in turns
 // once they are more than the CTAs that share a tile block, while a frame on tiles hardly depends on its rows.  Where the line lies
 // follows from the model's widths and the grid, so it is drawn by two models of a frame's time, fitted to 43 measured pairs (150m, 70m and
-// tiny; 40 to 148 CTAs; 9 to 512 rows; caches of <= 471 positions), all of which they order as measured.
-// us, groups | tiles: 150m 136 rows 2232 | 2321, 145: 2416 | 2323, 256: 3498 | 2435; 70m 200: 2004 | 2051, 256: 2126 | 2068; tiny 512: 714 | 802;
+// tiny; 40 to 148 CTAs; 9 to 512 rows; caches of <= 471 positions), of which they order all but one (70m, 256
+// rows: 2126 | 2068); of 21 pairs of three other models, of 64 + 5 layers and widths of 128 to 768, all but two (by 2 and 6 %).
+// us, groups | tiles: 150m 136 rows 2232 | 2321, 145: 2416 | 2323, 256: 3498 | 2435; 70m 200: 2004 | 2051, 288: 2556 | 2166; tiny 512: 714 | 802;
 // 150m on 40 CTAs 24: 1823 | 2388, 33: 2792 | 2402.  A row's bits are the same on either side.
 static bool in_groups(const SmolModel* m, int rows) {
     if (m->tc_group_rows >= 0) return rows <= m->tc_group_rows;

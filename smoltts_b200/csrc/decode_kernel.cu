@@ -1255,9 +1255,9 @@ double rows_plan(const DevModel& M, int rows, int n_ctas, RowsPlan (*plan)[6]) {
         }
     }
     const int phases = phases_per_frame(M.n_layer, M.n_flayer, M.depth);
-    return 0.92e-3 * clocks + 2.66 * phases + 4.6 * (1 + M.depth) * ((rows + n_ctas - 1) / n_ctas) + 6.6 * M.n_layer * ((rows * M.n_kv + 4 * n_ctas - 1) / (4 * n_ctas));
+    return 0.97e-3 * clocks + 2.2 * phases + 4.9 * (1 + M.depth) * ((rows + n_ctas - 1) / n_ctas) + 7.5 * M.n_layer * ((rows * M.n_kv + 4 * n_ctas - 1) / (4 * n_ctas));
 }
-// The time of a frame on 128-row tiles (us): ring stages of the fullest CTA, steps between two barriers, row tiles, sampling.
+// The time of a frame on 128-row tiles (us): ring stages of the fullest CTA, steps between two barriers, row tiles, sampling, attention.
 double tiles_time(const DevModel& M, int rows, int n_ctas) {
     const int m_tiles = (rows + umma::kM - 1) / umma::kM;
     int stages = 0, steps = 0, phases = 0;
@@ -1276,8 +1276,8 @@ double tiles_time(const DevModel& M, int rows, int n_ctas) {
             phases += kind == PH_HEAD ? 0 : n;
         }
     }
-    return 0.665 * stages + 2.7 * steps * ((rows + kRowsPerPass * n_ctas - 1) / (kRowsPerPass * n_ctas)) + 0.74 * phases * m_tiles
-           + 3.0 * (1 + M.depth) * ((rows + n_ctas - 1) / n_ctas);
+    return 0.56 * stages + 3.15 * steps * ((rows + kRowsPerPass * n_ctas - 1) / (kRowsPerPass * n_ctas)) + 0.91 * phases * m_tiles
+           + 0.9 * (1 + M.depth) * ((rows + n_ctas - 1) / n_ctas) + 8.5 * M.n_layer;
 }
 
 // Kernel variant by batch tile (sequences whose activations share one pass over the weights).

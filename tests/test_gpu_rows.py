@@ -327,3 +327,17 @@ def test_a_wait_that_runs_out_ends_the_launch_and_the_next_call_reports_it(what)
     assert e.value.code == _capi.SMOL_ERR_TIMEOUT and model.get_option("device_status") == 0
     model.set_option("wait_ms", 2000)
     assert all(torch.equal(a, b) for a, b in zip(run(), want))
+
+
+def test_the_longest_program_fits_beside_the_tiles():
+    """498 of at most 512 phases: their table lies in shared memory beside the weight tiles."""
+    over = dict(base="smoltts_byte_tiny", n_layer=64, n_fast_layer=5)
+    CONFIGS["long_program"] = over
+    cfg, model = _model("long_program", 12, 64)
+    assert model.phase_count == 5 * 64 + 2 + 8 * (4 * 5 + 2) == 498
+    lens = [1 + b for b in range(12)]
+    out = [_frame(cfg, model, lens, list(range(12)), 9)[:2]]
+    assert model.get_option("last_kernel") == KERNEL["groups"]
+    model.set_option("tc_group_rows", 0)
+    out.append(_frame(cfg, model, lens, list(range(12)), 9)[:2])
+    assert all(torch.equal(a, b) for a, b in zip(*out))

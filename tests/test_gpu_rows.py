@@ -329,6 +329,48 @@ def test_a_wait_that_runs_out_ends_the_launch_and_the_next_call_reports_it(what)
     assert all(torch.equal(a, b) for a, b in zip(run(), want))
 
 
+def _prompt_against_prefill_and_step(cfg, model, n, cached=0):
+    """forward_generate of n columns (behind `cached` positions) against the prefill of all but the last and that one alone: bits."""
+    grid = prompt_grid(byte_prompt(max(1, n + cached - 12), seed=n)[-(n + cached):], cfg)[None].to(device="cuda", dtype=torch.int32)
+    grid = torch.cat([grid, grid], 2)[:, :, :n + cached].contiguous()
+    before, prompt = grid[:, :, :cached + 1].contiguous(), grid[:, :, cached:].contiguous()
+    out = []
+    for one_pass in (True, False):
+        model.kv_view().zero_()
+        cache = make_prompt_cache(model)
+        if cached:
+            model.prefill(cache.batch, before, torch.tensor([cached + 1], dtype=torch.int32, device="cuda"))
+        if one_pass:
+            logits, hidden = model.forward_generate(prompt, cache)
+            assert model.get_option("last_kernel") == KERNEL["prompt"]
+        else:
+            model.prefill(cache.batch, prompt, torch.tensor([n], dtype=torch.int32, device="cuda"))
+            model.slow_step(cache.batch, advance=True)
+            logits, hidden = model.debug_buffer("token_logits", 1).clone(), model.debug_buffer("x", 1).clone()
+        assert int(cache.batch.seq_len[0]) == n + cached and cache.batch.host_len == [n + cached]
+        kv = model.kv_view()[torch.tensor(cache.batch.pages, device="cuda")].permute(1, 2, 3, 0, 4, 5).flatten(3, 4)[..., :n + cached, :]
+        out.append((logits, hidden.view(torch.int16), kv.contiguous().view(torch.int16)))
+        cache.batch.release()
+    assert all(torch.equal(a, b) for a, b in zip(*out))
+
+
+@pytest.mark.parametrize("name,page_size", [("long_chains", 32), ("70m", 16)])
+@pytest.mark.parametrize("n,cached", [(10, 1), (17, 31), (130, 300), (1024, 0), (1025, 0), (1100, 3), (1990, 0)])
+def test_prompt_logits_behind_a_cache_and_over_several_iterations(name, page_size, n, cached):
+    """On top of what the sequence holds; a last iteration of a single row (1025 positions); the last position's attention over up to 32
+    splits of 64 positions, and over longer ones."""
+    cfg, model = _model(name, 1, 2040, page_size)
+    _prompt_against_prefill_and_step(cfg, model, n, cached)
+
+
+def test_a_prompt_alone_sets_the_variant_up():
+    cfg, model = _model("70m", 1, 64)
+    assert model.get_option("tc_ready") == 0 and model.get_option("last_kernel") == 0
+    cache = make_prompt_cache(model)
+    model.forward_generate(prompt_grid(byte_prompt(20, seed=1), cfg)[None].to(device="cuda", dtype=torch.int32), cache)
+    assert model.get_option("tc_ready") == 1
+
+
 def test_the_longest_program_fits_beside_the_tiles():
     """498 of at most 512 phases: their table lies in shared memory beside the weight tiles."""
     over = dict(base="smoltts_byte_tiny", n_layer=64, n_fast_layer=5)

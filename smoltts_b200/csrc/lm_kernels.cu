@@ -2445,24 +2445,22 @@ extern "C" int smol_lm_bind(SmolLm* m, const SmolLmGlobals* g, void* d_workspace
 
 namespace smol {
 namespace lm {
-// gemm_few_kernel for activations that a prologue makes (a form of its own: shared with the plain one it cost that 1.4 % in decoding).
-// begin(): the prologue; row(m, k): 8 elements of an activation row; part: [WARPS][few_out(NR, MT)], in the place of the activations.
-constexpr int few_out(int nr, int mt) { return nr * (nr == 16 ? 8 : 16) * mt; }     // outputs of a block
-template <int NR, int MT, int WARPS, class Begin, class Row>
-__device__ __forceinline__ void few_product(const bf16* __restrict__ w, float* __restrict__ y, int M, int N, int K, float* part, Begin begin, Row row) {
-    constexpr int WT = NR / 8, AT = NR == 16 ? MT : 2 * MT;      // 8-row pieces of weights and of activations per step
+// gemm_few_kernel of one row that a prologue makes (a form of its own: shared with the plain one it cost that 1.4 % in decoding).
+// begin(): the prologue; row(k): 8 elements of the row; part: [WARPS][few_out(NR)], in the place of the row.
+constexpr int few_out(int nr) { return nr * (nr == 16 ? 8 : 16); }     // outputs of a block (those of one activation row count)
+template <int NR, int WARPS, class Begin, class Row>
+__device__ __forceinline__ void few_product(const bf16* __restrict__ w, float* __restrict__ y, int N, int K, float* part, Begin begin, Row row) {
+    constexpr int WT = NR / 8, AT = NR == 16 ? 1 : 2;            // 8-row pieces of weights and of activations per step
     constexpr int U = WT + AT <= 3 ? 4 : 2;                      // steps of 32 whose loads are in flight together
-    constexpr int OUT = few_out(NR, MT);
+    constexpr int OUT = few_out(NR);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, tq = lane & 3;
     const int n0 = blockIdx.x * NR;
     const bf16* wr[WT];
 #pragma unroll
     for (int i = 0; i < WT; ++i) wr[i] = w + (size_t)min(n0 + i * 8 + g, N - 1) * K + tq * 8;
-    float acc[MT][4];
+    float acc[4];
 #pragma unroll
-    for (int i = 0; i < MT; ++i)
-#pragma unroll
-        for (int e = 0; e < 4; ++e) acc[i][e] = 0.0f;
+    for (int e = 0; e < 4; ++e) acc[e] = 0.0f;
     const uint4 zero = make_uint4(0, 0, 0, 0);
     uint4 p[U][WT];
     auto load_weights = [&](int k0) {
@@ -2483,42 +2481,38 @@ __device__ __forceinline__ void few_product(const bf16* __restrict__ w, float* _
 #pragma unroll
             for (int i = 0; i < AT; ++i) {
                 const int m = i * 8 + g;
-                x[u][i] = (m < M && k < K) ? row(m, k) : zero;
+                x[u][i] = (m < 1 && k < K) ? row(k) : zero;
             }
         }
 #pragma unroll
-        for (int u = 0; u < U; ++u)
-#pragma unroll
-            for (int i = 0; i < MT; ++i) {
-                float lo[4] = {0.0f, 0.0f, 0.0f, 0.0f}, hi[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-                if constexpr (NR == 16) {
-                    mma_bf16_16816(lo, p[u][0].x, p[u][1].x, p[u][0].y, p[u][1].y, x[u][i].x, x[u][i].y);
-                    mma_bf16_16816(hi, p[u][0].z, p[u][1].z, p[u][0].w, p[u][1].w, x[u][i].z, x[u][i].w);
-                } else {
-                    mma_bf16_16816(lo, x[u][2 * i].x, x[u][2 * i + 1].x, x[u][2 * i].y, x[u][2 * i + 1].y, p[u][0].x, p[u][0].y);
-                    mma_bf16_16816(hi, x[u][2 * i].z, x[u][2 * i + 1].z, x[u][2 * i].w, x[u][2 * i + 1].w, p[u][0].z, p[u][0].w);
-                }
-#pragma unroll
-                for (int e = 0; e < 4; ++e) acc[i][e] += lo[e] + hi[e];
+        for (int u = 0; u < U; ++u) {
+            float lo[4] = {0.0f, 0.0f, 0.0f, 0.0f}, hi[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+            if constexpr (NR == 16) {
+                mma_bf16_16816(lo, p[u][0].x, p[u][1].x, p[u][0].y, p[u][1].y, x[u][0].x, x[u][0].y);
+                mma_bf16_16816(hi, p[u][0].z, p[u][1].z, p[u][0].w, p[u][1].w, x[u][0].z, x[u][0].w);
+            } else {
+                mma_bf16_16816(lo, x[u][0].x, x[u][1].x, x[u][0].y, x[u][1].y, p[u][0].x, p[u][0].y);
+                mma_bf16_16816(hi, x[u][0].z, x[u][1].z, x[u][0].w, x[u][1].w, p[u][0].z, p[u][0].w);
             }
+#pragma unroll
+            for (int e = 0; e < 4; ++e) acc[e] += lo[e] + hi[e];
+        }
         load_weights(k0 + WARPS * 32 * U);
     }
     __syncthreads();
-    // part[warp][m * NR + n]: neighbouring outputs of a row side by side.  acc[.][e]: tile row g + (e / 2) * 8, tile column 2 tq + e % 2
+    // part[warp][m * NR + n]: neighbouring outputs of a row side by side.  acc[e]: tile row g + (e / 2) * 8, tile column 2 tq + e % 2
 #pragma unroll
-    for (int i = 0; i < MT; ++i)
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-            const int r = g + (e >> 1) * 8, c = tq * 2 + (e & 1);
-            part[warp * OUT + (NR == 16 ? (i * 8 + c) * NR + r : (i * 16 + r) * NR + c)] = acc[i][e];
-        }
+    for (int e = 0; e < 4; ++e) {
+        const int r = g + (e >> 1) * 8, c = tq * 2 + (e & 1);
+        part[warp * OUT + (NR == 16 ? c * NR + r : r * NR + c)] = acc[e];
+    }
     __syncthreads();
     for (int o = threadIdx.x; o < OUT; o += WARPS * 32) {
         const int m = o / NR, n = n0 + o % NR;
         double t = part[o];
 #pragma unroll
         for (int x = 1; x < WARPS; ++x) t += part[x * OUT + o];
-        if (m < M && n < N) y[(size_t)m * N + n] = (float)t;
+        if (m < 1 && n < N) y[n] = (float)t;
     }
 }
 // Down-projection of one row with PolyNorm in its prologue: every block takes the row's activation into shared memory, behind its first
@@ -2533,7 +2527,7 @@ __global__ void __launch_bounds__(WARPS * 32) gemm_polynorm_kernel(const float* 
     extern __shared__ uint4 few_smem[];
     __shared__ float red[3][33];
     bf16* xs = reinterpret_cast<bf16*>(few_smem);
-    few_product<NR, 1, WARPS>(w, y, 1, N, K, reinterpret_cast<float*>(few_smem), [&] {
+    few_product<NR, WARPS>(w, y, N, K, reinterpret_cast<float*>(few_smem), [&] {
         dep_wait();
         dep_go();
         float s2 = 0.0f, s4 = 0.0f, s6 = 0.0f;
@@ -2561,7 +2555,7 @@ __global__ void __launch_bounds__(WARPS * 32) gemm_polynorm_kernel(const float* 
             store4<bf16>(xs + c, f(v.x), f(v.y), f(v.z), f(v.w));
         }
         __syncthreads();
-    }, [&](int, int k) { return *reinterpret_cast<const uint4*>(xs + k); });
+    }, [&](int k) { return *reinterpret_cast<const uint4*>(xs + k); });
 }
 }  // namespace lm
 }  // namespace smol
@@ -2760,7 +2754,7 @@ cudaError_t linear<bf16>(SmolLm* m, const bf16* a, const bf16* w, float* y, int 
 static bool linear_polynorm_row(SmolLm* m, const float* z, const float* coef, const bf16* w, float* y, int N, int K, cudaStream_t st) {
     if (K % 8 != 0 || reinterpret_cast<uintptr_t>(w) % 16 != 0 || (size_t)K * 2 > kFewActSmem) return false;
 #define SMOL_FEW_POLY(NR, WARPS)                                                                                                           \
-    pdl_launch(gemm_polynorm_kernel<NR, WARPS>, (N + NR - 1) / NR, WARPS * 32, std::max((size_t)K * 2, (size_t)WARPS * few_out(NR, 1) * 4), st, \
+    pdl_launch(gemm_polynorm_kernel<NR, WARPS>, (N + NR - 1) / NR, WARPS * 32, std::max((size_t)K * 2, (size_t)WARPS * few_out(NR) * 4), st, \
                z, coef, m->cfg.norm_eps, w, y, N, K)
     if (N < kFewWideN) {
         if (K >= kFewLongK) SMOL_FEW_POLY(8, 16);

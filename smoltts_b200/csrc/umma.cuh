@@ -1,4 +1,5 @@
-// tcgen05 / TMEM building blocks for the batched decode path (sm_100a only).
+// tcgen05 / TMEM building blocks (sm_100a only): of the batched engine's 128-row tiles (tile_phases.cuh), of its prompts
+// (prompt_phases.cuh) and of the language models' products (lm_gemm_tc.cuh, lm_flash_tc.cuh).
 //
 // One output tile = 128 sequences (TMEM lanes) x n_blk weight rows (TMEM columns, fp32), accumulated by
 // tcgen05.mma.cta_group::1.kind::f16 over K in ring stages of 64 elements.  Both operands are K-major
@@ -23,7 +24,6 @@ constexpr int kMaxN = 96;                    // widest tile (w1|w3: 48 + 48 rows
 #define UMMA_STAGES 5
 #endif
 constexpr int kStages = UMMA_STAGES;
-constexpr int kAhead = 3;                    // stages in flight ahead of the MMA
 constexpr int kStageA = kM * kBK * 2;        // 16 KB
 constexpr int kStageB = kMaxN * kBK * 2;     // 12 KB
 constexpr int kStageBytes = kStageA + kStageB;
@@ -82,11 +82,6 @@ __device__ __forceinline__ void fence_before_sync() { asm volatile("tcgen05.fenc
 __device__ __forceinline__ void fence_after_sync() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void fence_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 
-// K-major, no swizzle (layout type 0), descriptor version 1 (sm_100).
-__device__ __forceinline__ uint64_t smem_desc(uint32_t addr, uint32_t lbo, uint32_t sbo) {
-    return (uint64_t)((addr & 0x3FFFFu) >> 4) | ((uint64_t)((lbo >> 4) & 0x3FFFu) << 16) |
-           ((uint64_t)((sbo >> 4) & 0x3FFFu) << 32) | (1ull << 46);
-}
 // D fp32, A/B bf16, both K-major, M = 128, N = n.
 __device__ __forceinline__ uint32_t instr_desc(int n) {
     return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(kM >> 4) << 24);
@@ -101,17 +96,6 @@ __device__ __forceinline__ void mma_bf16(uint32_t d_tmem, uint64_t a_desc, uint6
 __device__ __forceinline__ void commit(uint64_t* bar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(s2u(bar)) : "memory");
 }
-// 8 consecutive fp32 columns of this thread's lane (lane quadrant = warp % 4).
-__device__ __forceinline__ void tmem_ld8(uint32_t taddr, float (&v)[8]) {
-    uint32_t r[8];
-    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
-                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
-                 : "r"(taddr) : "memory");
-    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-#pragma unroll
-    for (int i = 0; i < 8; ++i) v[i] = __uint_as_float(r[i]);
-}
-
 
 // Called once per kernel by all threads (before any tile): barriers + TMEM allocation by warp 0.
 __device__ __forceinline__ void setup(Bars* bars, Pipe& pipe, uint32_t issuers = 1u, uint32_t producers = 1u) {
@@ -147,22 +131,6 @@ __device__ __forceinline__ void tma_load_2d(uint32_t dst, const void* tmap, int 
     asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
                  ::"r"(dst), "l"(tmap), "r"(s2u(bar)), "r"(c0), "r"(c1) : "memory");
 }
-// The same with an L2 eviction policy (createpolicy): weights that are read once per frame leave L2 first, weights that
-// every depth step re-reads stay.
-__device__ __forceinline__ void tma_load_2d_hint(uint32_t dst, const void* tmap, int c0, int c1, uint64_t* bar, uint64_t policy) {
-    asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes.L2::cache_hint [%0], [%1, {%3, %4}], [%2], %5;"
-                 ::"r"(dst), "l"(tmap), "r"(s2u(bar)), "r"(c0), "r"(c1), "l"(policy) : "memory");
-}
-__device__ __forceinline__ uint64_t l2_policy_evict_first() {
-    uint64_t p;
-    asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(p));
-    return p;
-}
-__device__ __forceinline__ uint64_t l2_policy_evict_last() {
-    uint64_t p;
-    asm volatile("createpolicy.fractional.L2::evict_last.b64 %0, 1.0;" : "=l"(p));
-    return p;
-}
 // K-major, 128-byte swizzle (layout type 2), 8-row groups 1024 B apart, descriptor version 1.
 __device__ __forceinline__ uint64_t smem_desc_sw128(uint32_t addr) {
     return (uint64_t)((addr & 0x3FFFFu) >> 4) | ((uint64_t)1 << 16) | ((uint64_t)(1024 >> 4) << 32) | (1ull << 46) | (2ull << 61);
@@ -173,9 +141,9 @@ struct BSrc {
     const void* tm;   // map whose box is `box` rows high
     int row0, n, box;
 };
-enum WeightPolicy { kWeightsDefault = 0, kWeightsStream = 1, kWeightsKeep = 2 };
 
-// The two TMA-issuing threads of a tile (warps 1 and 3) of tile_mma_tma.
+// The two TMA-issuing threads of a tile (warps 1 and 3).  tile_phases.cuh orders the activations that other CTAs wrote with st.global against
+// these threads' async-proxy reads (fence.proxy.async around every grid barrier).
 constexpr int kTmaProducerA = 32;   // activation boxes
 constexpr int kTmaProducerB = 96;   // weight boxes
 
@@ -183,7 +151,7 @@ constexpr int kTmaProducerB = 96;   // weight boxes
 // arguments; `ring` is 1024-byte aligned.  K elements starting at column k0 of both operands (split-K units).
 template <int NT>
 __device__ __forceinline__ void tile_mma_tma(unsigned char* ring, Bars* bars, Pipe& pipe, int K, const void* tm_a, int a_row0,
-                                             BSrc b0, BSrc b1, int k0 = 0, int a_rows = kM, int weight_policy = kWeightsDefault) {
+                                             BSrc b0, BSrc b1, int k0 = 0, int a_rows = kM) {
     const int nk = K / kBK;
     const int tid = threadIdx.x;
     const int n_blk = b0.n + b1.n;
@@ -192,7 +160,6 @@ __device__ __forceinline__ void tile_mma_tma(unsigned char* ring, Bars* bars, Pi
     const uint32_t g0 = pipe.chunk;
     // a_rows: rows of the activation box behind tm_a (fewer than 128 when the batch is small: the MMA still spans 128
     // rows, the rest of the stage holds stale rows whose accumulator lanes nobody reads)
-    const uint64_t w_policy = weight_policy == kWeightsKeep ? l2_policy_evict_last() : l2_policy_evict_first();
     // Two producing threads (a TMA instruction costs its issuing thread ~60 ns: measured 285 / 341 / 655 ns per stage with
     // 2 / 3 / 7 copies): `part` 0 = the activation box, 1 = the weight boxes.  Each part arrives on `full` with its own
     // byte count.
@@ -207,16 +174,9 @@ __device__ __forceinline__ void tile_mma_tma(unsigned char* ring, Bars* bars, Pi
             return;
         }
         bar_expect_tx(&bars->full_[s], (uint32_t)(n_blk * kBK * 2));
-        if (weight_policy == kWeightsDefault) {
-            for (int j = 0; j < b0.n; j += b0.box) tma_load_2d(b + j * (kBK * 2), b0.tm, k0 + kc * kBK, b0.row0 + j, &bars->full_[s]);
-            for (int j = 0; j < b1.n; j += b1.box)
-                tma_load_2d(b + (b0.n + j) * (kBK * 2), b1.tm, k0 + kc * kBK, b1.row0 + j, &bars->full_[s]);
-        } else {
-            for (int j = 0; j < b0.n; j += b0.box)
-                tma_load_2d_hint(b + j * (kBK * 2), b0.tm, k0 + kc * kBK, b0.row0 + j, &bars->full_[s], w_policy);
-            for (int j = 0; j < b1.n; j += b1.box)
-                tma_load_2d_hint(b + (b0.n + j) * (kBK * 2), b1.tm, k0 + kc * kBK, b1.row0 + j, &bars->full_[s], w_policy);
-        }
+        for (int j = 0; j < b0.n; j += b0.box) tma_load_2d(b + j * (kBK * 2), b0.tm, k0 + kc * kBK, b0.row0 + j, &bars->full_[s]);
+        for (int j = 0; j < b1.n; j += b1.box)
+            tma_load_2d(b + (b0.n + j) * (kBK * 2), b1.tm, k0 + kc * kBK, b1.row0 + j, &bars->full_[s]);
     };
     // six working threads; everybody else sleeps in the block barrier below instead of polling `done` (512 polling
     // threads take issue slots from the producers' and the MMA threads' dependent chains)

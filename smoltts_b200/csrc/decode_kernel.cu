@@ -939,9 +939,9 @@ __device__ __forceinline__ void run_phase(const DevModel& M, const CallArgs& A, 
                                           uint32_t& parity, RowsSync& sy, uint32_t packed_phase, const RowsStep* step) {
     if (BT == 0) {
         if (ph.kind == PH_ATTN) {
-            phase_attn_batch<false>(M, A, c, ph, sy, A.kv_map);
+            phase_attn_batch<false, kTimed>(M, A, c, ph, sy, A.kv_map);
         } else if (ph.kind == PH_SAMPLE) {
-            rows_sync_in(M, sy);
+            rows_sync_in<kTimed>(M, sy);
             phase_sample(M, A, c, ph);
         } else {
             phase_rows<kTimed>(M, A, c, packed_phase, sy, step);

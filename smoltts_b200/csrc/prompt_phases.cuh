@@ -21,8 +21,9 @@ constexpr int kPrStages = 7;                                   // 28 KB each: 12
 constexpr int kPrRing = kPrStages * umma::kStageBytes;
 constexpr int kPrEpilogueWarp = 4;                             // first of the warps that read accumulators
 constexpr int kPrData = kPrRing > kWarps * kAttnStage ? kPrRing : kWarps * kAttnStage;
-// behind the ring: copies of the kernel's arguments.  The phases are functions of their own (inlined into one kernel their registers
-// would not suffice), and reading an argument through a reference there is a load from the parameter space: several hundred clocks.
+// behind the ring: copies of the kernel's arguments.  The last position's products, the attentions and the row steps are functions of their own
+// (the weight phases are not: calls, and arguments through a stack that the L1 beside the ring does not hold, cost 5 % of a prompt of 212
+// positions, 844 us against 801), and reading an argument through a reference there is a load from the parameter space: several hundred clocks.
 constexpr int kPrModel = (sizeof(DevModel) + 127) / 128 * 128, kPrArgs = (sizeof(CallArgs) + 127) / 128 * 128;
 constexpr int kPrSmem = kPrData + kPrModel + kPrArgs;
 static_assert(kPrSmem <= 226 * 1024, "ring and arguments");
@@ -195,7 +196,7 @@ __device__ __noinline__ void row_wide(const DevModel& M, int row, int layer, int
 
 // One weight phase; on return the CTA has finished its units, the barrier behind it is the caller's.
 template <bool kTimed>
-__device__ __noinline__ void prompt_gemm(const DevModel& M, const CallArgs& A, const Ctx& c, const Phase& ph, RowsSync& sy, uint32_t& chunk, uint32_t& tile, const int last_row) {
+__device__ __forceinline__ void prompt_gemm(const DevModel& M, const CallArgs& A, const Ctx& c, const Phase& ph, RowsSync& sy, uint32_t& chunk, uint32_t& tile, const int last_row) {
     const int kind = ph.kind;
     const int D = M.dim, F = M.inter, Hq = M.n_head, Hkv = M.n_kv;
     const int q_rows = Hq * kHeadDim, k_end = (Hq + Hkv) * kHeadDim;
@@ -243,7 +244,7 @@ __device__ __noinline__ void prompt_gemm(const DevModel& M, const CallArgs& A, c
     const bool dots = last_row >= 0 && warp >= kPrEpilogueWarp;
     const int u_first = dots ? (warp - kPrEpilogueWarp) * c.n_ctas + c.cta : 0, u_step = (kWarps - kPrEpilogueWarp) * c.n_ctas, u_end = dots ? row_units(M, kind) : 0;
     for (int u = u_first; u < u_end; u += u_step) row_prefetch(M, kind, ph.layer, u, lane);
-    rows_sync_in(M, sy);
+    rows_sync_in<kTimed>(M, sy);
     if (warp == 0 && lane == 0) {
         fence_proxy_async_global();      // rows written by st.global in other CTAs
         uint32_t g = chunk;
@@ -370,11 +371,13 @@ __device__ __noinline__ void prompt_gemm(const DevModel& M, const CallArgs& A, c
     tile += (uint32_t)my_units;
 }
 
-__device__ __noinline__ void prompt_attn_rows(const DevModel& M, const CallArgs& A, const Ctx& c, const Phase& ph, RowsSync& sy, const void* kv_map, int last_row) { phase_attn_batch<true>(M, A, c, ph, sy, kv_map, last_row); }
+template <bool kTimed>
+__device__ __noinline__ void prompt_attn_rows(const DevModel& M, const CallArgs& A, const Ctx& c, const Phase& ph, RowsSync& sy, const void* kv_map, int last_row) { phase_attn_batch<true, kTimed>(M, A, c, ph, sy, kv_map, last_row); }
 __device__ __noinline__ void prompt_attn_alone(const DevModel& M, const CallArgs& A, const Ctx& c, const Phase& ph, int splits, int row) { phase_attn_g(M, A, c, ph, splits, row, 1); }
+template <bool kTimed>
 __device__ __forceinline__ void prompt_attn(const DevModel& M, const CallArgs& A, const Ctx& c, const Phase& ph, RowsSync& sy, const void* kv_map, int last_row) {
     if (last_row < 0) {
-        prompt_attn_rows(M, A, c, ph, sy, kv_map, -1);
+        prompt_attn_rows<kTimed>(M, A, c, ph, sy, kv_map, -1);
         return;
     }
     // the last row as decoded alone, on a few CTAs of its own
@@ -382,7 +385,7 @@ __device__ __forceinline__ void prompt_attn(const DevModel& M, const CallArgs& A
     const int n_alone = min(min(M.n_kv * ns, 20), c.n_ctas / 4);
     Ctx cs = c;
     cs.n_ctas = c.n_ctas - n_alone;
-    if (c.cta < cs.n_ctas) prompt_attn_rows(M, A, cs, ph, sy, kv_map, last_row);
+    if (c.cta < cs.n_ctas) prompt_attn_rows<kTimed>(M, A, cs, ph, sy, kv_map, last_row);
     if (c.cta >= cs.n_ctas || n_alone == 0) {
         cs.cta = c.cta - (n_alone ? cs.n_ctas : 0);
         cs.n_ctas = n_alone ? n_alone : c.n_ctas;
@@ -445,7 +448,7 @@ smol_prompt_kernel(const __grid_constant__ DevModel Mp, const __grid_constant__ 
         const int last_row = last_iter && A.whole_prompt > 0 ? A.head_row : -1;
         if (kTimed) sy.phase = 0;
         PhaseTimer<kTimed> timer(c);
-        rows_sync_in(M, sy);
+        rows_sync_in<kTimed>(M, sy);
         timer.rest();
         tile_row_step(M, A, c, M.dim, M.x, M.layers[0].attention_norm, [&](int bg, int ch, float (&x)[8]) { embed_chunk(M, A, c, bg, ch, x); });
         timer.step(M, unpack_phase(M.prog[0]));
@@ -454,13 +457,13 @@ smol_prompt_kernel(const __grid_constant__ DevModel Mp, const __grid_constant__ 
             const Phase ph = unpack_phase(M.prog[p]);
             if (kTimed) sy.phase = p;
             if (ph.kind == PH_ATTN) {
-                rows_sync_in(M, sy);
-                prompt_attn(M, A, c, ph, sy, Ap.kv_map, last_row);
+                rows_sync_in<kTimed>(M, sy);
+                prompt_attn<kTimed>(M, A, c, ph, sy, Ap.kv_map, last_row);
             } else {
                 prompt_gemm<kTimed>(M, A, c, ph, sy, chunk, tile, last_row);
                 if (ph.kind == PH_WO || ph.kind == PH_W2) {   // h = stream + wo(attn) (P:499); stream = h + w2(act) (P:500); and the norm of the phase that reads it
                     rows_arrive<kTimed>(M, c, sy);
-                    rows_sync_in(M, sy);
+                    rows_sync_in<kTimed>(M, sy);
                     timer.rest();
                     const bool wo = ph.kind == PH_WO;
                     const uint16_t* norm = wo ? M.layers[ph.layer].ffn_norm : ph.layer + 1 < M.n_layer ? M.layers[ph.layer + 1].attention_norm : M.norm;
@@ -485,7 +488,7 @@ smol_prompt_kernel(const __grid_constant__ DevModel Mp, const __grid_constant__ 
     if (A.whole_prompt > 0 && !sy.failed) {
         if (kTimed) sy.phase = 5 * M.n_layer;        // the LM head's
         PhaseTimer<kTimed> timer(c);
-        rows_sync_in(M, sy);
+        rows_sync_in<kTimed>(M, sy);
         if (c.cta == 0 && A.head_row > 0)      // the last position's hidden state (pre-norm) -> row 0
             for (int i = c.tid; i < M.dim / 8; i += kThreads) *reinterpret_cast<uint4*>(M.x + i * 8) = ldcg_v4(M.x + (size_t)A.head_row * M.dim + i * 8);
         uint4 x[kRowCh], w[kRowCh];

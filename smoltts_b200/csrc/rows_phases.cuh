@@ -63,9 +63,10 @@ struct RowsSync {
     int phase, next;         // this phase; the launch's next weight phase (-1: none), whose tiles this one fetches
     int waits_for;           // the phase whose barrier is pending
 };
+template <bool kTimed>
 __device__ __forceinline__ void rows_sync_in(const DevModel& M, RowsSync& sy) {
     if (!sy.pending) return;
-    const bool prof = M.prof != nullptr && blockIdx.x == 0 && threadIdx.x == 0;
+    const bool prof = kTimed && blockIdx.x == 0 && threadIdx.x == 0;
     unsigned long long t = 0;
     if (prof) t = globaltimer_ns();
     sy.failed = __syncthreads_or(threadIdx.x == 0 && grid_poll(M.barrier, M.status, M.wait_ms, sy.target)) != 0;
@@ -84,7 +85,7 @@ __device__ __forceinline__ void rows_stamp(const DevModel& M, int kind, int fast
 }
 template <bool kTimed>
 __device__ __forceinline__ void rows_arrive(const DevModel& M, const Ctx& c, RowsSync& sy) {
-    rows_sync_in(M, sy);       // (a phase in which this CTA has no work may not have waited yet)
+    rows_sync_in<kTimed>(M, sy);       // (a phase in which this CTA has no work may not have waited yet)
     // Shared memory used here is overwritten by copies.  (Rows written here are read by other CTAs' copies: the threads that issue those
     // fence global memory behind the barrier; a full fence.proxy.async here waits for
     // the stores of every thread: frames of 9 / 64 rows 1263 / 1520 us with it, 1188 / 1437 without.)
@@ -176,7 +177,7 @@ __device__ __forceinline__ void tma_kv(uint32_t dst, const void* map, int row, i
 // they are combined in split order, relative to the largest maximum, so the result does not depend on wpt.
 // Decoding (kPrompt false): one position per unit, so only the fragments' first eight rows are in use, and a unit's cached keys and
 // values are fetched before the barrier in front of the phase (all but the step that holds the newest position).
-template <bool kPrompt>
+template <bool kPrompt, bool kTimed>
 __device__ __forceinline__ void phase_attn_batch(const DevModel& M, const CallArgs& A, const Ctx& c, const Phase& ph, RowsSync& sy, const void* kv_map,
                                                  const int skip_row = -1) {   // kv_map: the pool's tensor map; skip_row: left alone
     const int tid = tid_here(), warp = tid >> 5, lane = tid & 31;
@@ -191,7 +192,7 @@ __device__ __forceinline__ void phase_attn_batch(const DevModel& M, const CallAr
     const int n_units = n_groups * Hkv;
     const int wpt = attn_warps(n_units, c.n_ctas);
     const int per_cta = kWarps / wpt, slot = warp / wpt, wi = warp - slot * wpt;
-    if (kPrompt) rows_sync_in(M, sy);
+    if (kPrompt) rows_sync_in<kTimed>(M, sy);
     if (kPrompt && lane == 0) fence_proxy_async_global();    // keys and values written by other CTAs
     constexpr float kScale = 0.125f * 1.4426950408889634f;   // 1/sqrt(64) * log2(e): softmax in base 2
 
@@ -281,7 +282,7 @@ __device__ __forceinline__ void phase_attn_batch(const DevModel& M, const CallAr
                 };
                 if (!kPrompt && sy.pending) {
                     for (int i = 0; i < depth && fetched + 16 <= min(pl, len0); ++i) fetch();
-                    rows_sync_in(M, sy);
+                    rows_sync_in<kTimed>(M, sy);
                 }
                 if (!kPrompt) {
                     if (lane == 0) fence_proxy_async_global();   // the newest position was written by other CTAs
@@ -405,7 +406,7 @@ __device__ __forceinline__ void phase_attn_batch(const DevModel& M, const CallAr
                 }
             }
         }
-        rows_sync_in(M, sy);   // (warps without a split come by here)
+        rows_sync_in<kTimed>(M, sy);   // (warps without a split come by here)
         if (ns > 0) {
             asm volatile("bar.sync %0, %1;" ::"r"(1 + slot), "r"(wpt * 32) : "memory");
             if (one_round && wi < 4) {
@@ -767,7 +768,7 @@ __device__ __forceinline__ void rows_gemm(const DevModel& M, const CallArgs& A, 
             g_rpos[i] = p; g_rpage[i] = page;
         }
         if (!wide && !landed) { rows_wait(M, &g_mbar[0], sy.par_w); sy.par_w ^= 1u; landed = true; }
-        rows_sync_in(M, sy);
+        rows_sync_in<kTimed>(M, sy);
         const bool timed = kTimed && blockIdx.x == 0 && tid == 0;
         unsigned long long stamp = 0ull;
         if (timed) stamp = globaltimer_ns();
@@ -1030,7 +1031,7 @@ template <bool kTimed>
 __device__ __forceinline__ void phase_rows(const DevModel& M, const CallArgs& A, const Ctx& c, uint32_t packed_phase, RowsSync& sy, const RowsStep* step) {
     const Phase ph = unpack_phase(packed_phase);
     if (tc_has_prestep(ph)) {
-        rows_sync_in(M, sy);
+        rows_sync_in<kTimed>(M, sy);
         if (A.tc_part == 0 || A.tc_part == 1) rows_embed(M, A, c);
         if (A.cooperative) rows_arrive<kTimed>(M, c, sy);
         if (A.tc_part == 1) return;
@@ -1038,7 +1039,7 @@ __device__ __forceinline__ void phase_rows(const DevModel& M, const CallArgs& A,
     if (ph.kind == PH_QKV && !ph.fast) attn_prefetch(M, A, c, ph.layer);
     if (g_rk[ph.fast][ph.kind].block0 < 0) {   // no unit here: the weight region is free for the phase that follows
         if (c.tid == kThreads - 32) rows_issue_next(M, sy, step, c.stage);
-        rows_sync_in(M, sy);
+        rows_sync_in<kTimed>(M, sy);
         return;
     }
     const int n = g_rk[ph.fast][ph.kind].n;

@@ -65,14 +65,14 @@ struct SmolModel {
     int repeat = 0;
     int prefill_tile = 0;  // option: cap of prompt positions per prefill iteration (0 = as many as fit)
     int tc_attn_split = 0;  // option: cached positions per split of the batch attention (0 = the kernel's default)
-    int tc_min_batch = 9;  // rows (sequences, or prompt positions of a prefill tile) from which the tcgen05 variant runs:
+    int tc_min_batch = 9;  // rows (sequences, or prompt positions of a prefill tile) from which the tensor-core variant runs:
                            // measured crossover (150m, us per frame): bs 8: 2276 CUDA-core vs 2566 tensor-core; bs 12: 3642 vs 2577
     int ll_flags = 0;  // data-flow kernel: A/B switches and hold-off override (tools/ll_ncu.py)
     // data-flow kernel
     int ll2_state = 0;         // 0 unknown, 1 ready, -1 does not fit this model
     int ll2_holdoff = 400;     // option "ll_holdoff": cycles between the end of a phase and the first poll of the next
     int ll2_max_batch = 8;     // option: sequences (teams of CTAs) the kernel carries per launch; larger batches go to the
-                               // barrier kernel / its tcgen05 variant (measured at bs=8: 1.5 ms per frame step against 2.3 ms)
+                               // barrier kernel / its tensor-core variant (measured at bs=8: 1.5 ms per frame step against 2.3 ms)
     smol::ll2::SmemPlan ll2_sp;
     size_t ll2_smem = 0;
     int tc_group_rows = -1;    // rows of a decode batch up to which it runs in groups of rows (-1: in_groups decides)
@@ -233,7 +233,7 @@ static WsLayout ws_layout(const SmolConfig& c, int depth) {
 
 static int depth_of(const SmolConfig& c) { return c.num_codebooks - (c.duplicate_code_0 ? 0 : 1); }
 
-static bool tc_eligible(const SmolConfig& c) {   // whole 32-element blocks of K for every slice
+static bool tc_eligible(const SmolConfig& c) {   // whole 64-element blocks of K
     return (c.dim % 64) == 0 && (c.fast_dim % 64) == 0 && (c.intermediate_size % 64) == 0 && (c.fast_intermediate_size % 64) == 0;
 }
 static int ensure_tmaps(SmolModel* m);

@@ -11,8 +11,8 @@
 // below its last place with every MMA, so chains are kept at 12.
 //
 // What needs whole rows happens in steps between: the sum of the K slices, the residual add and the next RMSNorm (five rows
-// per CTA and pass).  Measured (150m, device time of prompt -> logits, us): 40 positions 743, 212: 835, 800: 1582; one thread that issued
-// loads and MMAs, no weights before the barrier, and a slow step behind it for the last position took 996, 1285 and 2090.
+// per CTA and pass).  Measured (150m, prompt -> logits, us): 40 positions 623, 212: 706, 800: 1467; one thread that issued
+// loads and MMAs, no weights before the barrier, and a slow step behind it for the last position took 917, 1219 and 2017.
 #pragma once
 
 namespace smol {

@@ -10,14 +10,14 @@
 //   * weights never wait for activations: a CTA's weight tiles of the next phase (one bulk copy, packed fragments) land in
 //     shared memory while it finishes this phase and sits in the barrier; cached keys and values are fetched there, too;
 //   * rows come by bulk copies, and a phase's pointers and sizes from tables in shared memory.
-// Measured (150m, contexts of up to 471, us per frame): 9 rows 1188, 16: 1195, 32: 1266, 64: 1437; tcgen05 tiles (activation
-// rows as the 128 lanes of an accumulator, 16 .. 96 weight rows as its columns, row steps between the phases) took 2135 to 2226:
-// with so few columns an MMA is bound by the 4 KB of its A operand, wo and w2 had to be cut over CTAs and added in a step of
-// their own, and a frame had 380 barriers instead of 197.
+// Measured (150m, us per frame): 9 rows (contexts of up to 100) 1093, 33: 1288, 64 (up to 471): 1411; tcgen05 tiles (tile_phases.cuh:
+// activation rows as the 128 lanes of an accumulator, 16 .. 96 weight rows as its columns, row steps between the phases) take 2024, 2094
+// and 2216: with so few columns an MMA is bound by the 4 KB of its A operand, wo and w2 are cut over CTAs and added in a step of their
+// own, and a frame has 380 barriers instead of 197.  Wide batches take several turns here and go there (in_groups, capi.cu).
 //
 // Summation order: four chains of MMAs per dot product (K steps 0, 4, 8 .. of 16 elements; 1, 5, 9 ..; ..), for wo and w2 per K
 // slice, added in order: a function of K alone, so a row's bits depend neither on the number of rows nor on the tile plan.  (The
-// tcgen05 tiles of the prompt kernel sum in the same order, and mma.sync and tcgen05 turn out to round alike: to the bit the same.)
+// tcgen05 tiles sum in the same order, and mma.sync and tcgen05 turn out to round alike: to the bit the same.)
 #pragma once
 
 namespace smol {
@@ -639,8 +639,8 @@ __device__ __forceinline__ void depth_load(const uint16_t* kp, int kvw, int dept
 // Depth attention of rows [r0, r0 + n_live) by one CTA, a warp per (row, kv head), which goes through the kv head's G query heads.  The
 // result goes to shared memory as bf16 rows (`stride` bytes apart), where the wo tiles of this CTA read it, and, where `copy` is given,
 // to its rows of M.attn.  Every tile block of wo repeats it: for 8 rows that is two tasks per warp, less than the barrier that a
-// step of its own would need.  4.6 us of the 7.5 of such a phase at 64 rows (150m), a chain of loads, FMAs and shuffles per head; the heads side
-// by side, two tasks at once, or more loads ahead spill and take longer (frames of 64, us: 1456, and 1515 to 1720).
+// step of its own would need.  4.0 us of the 6.9 of such a phase at 64 rows (150m), a chain of loads, FMAs and shuffles per head; the heads side
+// by side, two tasks at once, or more loads ahead spill and take longer (frames of 64, us: 1451, and 1513 to 1717).
 template <bool deep>   // deep: positions 8 .. 15 exist
 __device__ __forceinline__ void rows_depth_attention(const DevModel& M, int layer, int depth_pos, int r0, int n_live, unsigned char* out, int stride, uint16_t* copy) {
     const int Hq = M.fn_head, Hkv = M.fn_kv, G = Hq / Hkv, kvw = Hkv * kHeadDim, depth = M.depth, n_flayer = M.n_flayer;

@@ -158,7 +158,7 @@ def test_greedy_vs_literal_reference_goldens(size):
 def test_modes_and_batch_composition_are_bit_identical():
     """mode 0 (one persistent kernel) == mode 1 (per-phase launches in a CUDA graph), and a sequence
     decodes to the same ids alone, inside a batch of 3, and inside a batch of 11 (two batch tiles) -- on the GEMV variants
-    (the tcgen05 variant, which would take the batch of 11 and every prefill, is switched off here: it is bit-identical
+    (the tensor-core variant, which would take the batch of 11 and every prefill, is switched off here: it is bit-identical
     with itself, tests/test_gpu_tc.py, not with the GEMV kernels)."""
     from smoltts_b200 import GenerationSettings, generate_batch
 

@@ -2,7 +2,7 @@
 (smol_run_phases) on inputs copied bit-for-bit from the CPU oracle's trace, and its output is
 compared with the oracle's next tensor.  With identical inputs only the fp32 summation order
 differs, so the bar is: every element within 2 bf16 ulps and >= 98% of elements bit-identical.
-Batches of 9+ rows go through the tcgen05 tiles (tc_phases.cuh) and are held to the same bar."""
+Batches of 9+ rows go through the tensor-core tiles (rows_phases.cuh) and are held to the same bar."""
 import numpy as np
 import pytest
 import torch

@@ -90,8 +90,8 @@ def test_batched_decode_at_the_edges_of_its_row_groups(name, page_size, batch):
 @pytest.mark.parametrize("name,longest,batch", [("70m", 127, 10), ("70m", 128, 10), ("70m", 129, 40), ("long_chains", 1030, 40), ("70m", 2300, 150), ("deep", 2300, 300),
                                                 ("70m", 40, 145), ("ragged_heads", 200, 160), ("long_chains", 100, 290)])
 def test_batch_attention_around_its_splits(name, longest, batch):
-    """Contexts below, at and above a split; more splits than a unit has warps (states through global memory); many units.  Batches of
-    more than 144 rows take the tiles of 128 rows: the bits stay those of nine sequences."""
+    """Contexts below, at and above a split; more splits than a unit has warps (states through global memory); many units.  Wide
+    batches take the tiles of 128 rows: the bits stay those of nine sequences."""
     cfg, model = _model(name, batch, longest + 4)
     lens = [max(1, longest - (b * 131) % longest) for b in range(batch)]
     tl, dl, _ = _frame(cfg, model, lens, list(range(batch)), 9)

@@ -1,12 +1,12 @@
 """Oracle parity at the sizes BASELINE.json's configurations run at (150m), through the C-ABI:
 
-  * the tcgen05 variant at bs=64 and bs=256: two teacher-forced frames for every row of the
+  * the tensor-core variant at bs=64 and bs=256: two teacher-forced frames for every row of the
     batch against the CPU oracle (bf16) and its fp32 twin, under the calibrated bars of test_gpu_decode.py
     (our error against the fp32 logits <= 1.3x rms / 1.6x max of the bf16 oracle's own error; argmax = fp32 argmax
     wherever its margin exceeds TAU);
   * long contexts: prefill of 2100 and 4300 positions (> 128 KV pages, RoPE rows beyond 4096, up to 9
     attention blocks of 512 positions), then two teacher-forced frames, at bs=1 (data-flow kernel) and as rows of a
-    ragged batch of 32 (tcgen05 variant, batch attention), against the CPU oracle's bf16 logits.
+    ragged batch of 32 (tensor-core variant, batch attention), against the CPU oracle's bf16 logits.
 
 The oracle runs on the box's host cores inside the test (results cached per prompt), sized to finish in about a minute.
 """
@@ -77,7 +77,7 @@ def test_tensor_core_batches_vs_oracle_150m(B):
     assert B >= model.get_option("tc_min_batch") > 0
     grid = teacher_grid(cfg, n_text=14, n_audio=4 + N_FRAMES, batch=B, seed=300 + B, zero_code_at=2)   # [B, R, 20]
     tok, cb = _gpu_teacher_forced(model, [grid[b] for b in range(B)])
-    assert model.get_option("tc_ready") == 1, "the tcgen05 variant did not run"
+    assert model.get_option("tc_ready") == 1, "the tensor-core variant did not run"
     rbf_t, rbf_c = _oracle_teacher_forced(orc, grid)
     orc32 = DualAROracle(cfg, sd, dtype=torch.float32, max_seq_len=256)
     rf_t, rf_c = _oracle_teacher_forced(orc32, grid)
@@ -139,7 +139,7 @@ def test_long_context_bs1_dataflow_vs_oracle_150m(total):
 
 @pytest.mark.timeout(1200)
 def test_long_context_bs32_tensor_core_vs_oracle_150m():
-    """A ragged batch of 32 on the tcgen05 variant: rows 0 and 31 carry the 4300- and 2100-position probes (same prompts as
+    """A ragged batch of 32 on the tensor-core variant: rows 0 and 31 carry the 4300- and 2100-position probes (same prompts as
     the bs=1 test, so the oracle's results are shared), the other rows random contexts of 40..3000 positions."""
     cfg, sd, model, orc = model_and_oracle(SIZE, max_batch=32, max_seq_len=4352)
     gen = torch.Generator().manual_seed(77)

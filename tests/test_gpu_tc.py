@@ -1,4 +1,4 @@
-"""The tcgen05 variant of the decode kernel (batches / prefill tiles of 9+ rows, csrc/tc_phases.cuh + umma.cuh).
+"""The tensor-core variant of the decode kernel (batches / prefill tiles of 9+ rows: csrc/rows_phases.cuh, tile_phases.cuh, prompt_phases.cuh).
 
 Its dot products are summed by the tensor core, so it is not bit-identical to the CUDA-core variants; it is held to
   * the oracle's greedy ids up to near-tie decisions (greedy-with-resync, same rule and TAU as tests/test_gpu_decode.py);

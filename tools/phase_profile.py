@@ -107,10 +107,12 @@ def main():
     if total > 0:  # barrier kernel: globaltimer accumulators (work, barrier wait) and sub-phase segments
         print(f"{'phase':14s} {'count':>5s} {'work us':>9s} {'wait us':>9s} {'per-phase work':>15s} {'per-phase wait':>15s}")
         for k, (w, b, n) in sorted(agg.items(), key=lambda kv: -(kv[1][0] + kv[1][1])):
+            if w + b == 0:
+                continue
             print(f"{k:14s} {n:5d} {w / 1e3:9.1f} {b / 1e3:9.1f} {w / n / 1e3:15.2f} {b / n / 1e3:15.2f}")
             rows[k] = {"count": n, "work_us": w / 1e3, "wait_us": b / 1e3}
         print("sub-phase segments of the weight phases, us (one thread of CTA 0): CUDA cores: prologue | stage wait | gemv + epilogue | final sync; "
-              "groups of rows: rows in place | norm | MMAs | sums + epilogue; 128-row tiles: row steps | last position | copies + MMAs | epilogue")
+              "groups of rows: rows in place | norm | MMAs | sums + epilogue; prompts: row steps | last position | copies + MMAs | epilogue; 128-row tiles: row steps | set-up | copies + MMAs | epilogue")
         for k in range(16):
             if seg[k].sum() > 0:
                 name = ("fast." if k >= 8 else "slow.") + KINDS[k % 8]

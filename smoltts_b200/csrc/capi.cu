@@ -122,7 +122,7 @@ struct StatusWords {
         unused.push_back(w);
     }
 };
-StatusWords g_status_words;
+StatusWords& g_status_words = *new StatusWords;    // (never destroyed: models may be, at the end of the process)
 }  // namespace
 
 static thread_local std::string g_err;

@@ -1827,6 +1827,7 @@ __global__ void __launch_bounds__(kThreads) lm_sample_kernel(const float* __rest
 #include "lm_sigmoid_linear.cuh"
 #include "lm_delta_mlstm.cuh"
 #include "lm_quad_scan.cuh"
+#include "lm_chunk_scan.cuh"
 
 // =====================================================================================================================
 // Host side
@@ -1862,7 +1863,7 @@ struct SmolLm {
     std::vector<RunInfo> side_runs;       // the cache / state placement of a run's side mixer
     size_t o_conv = 0, o_head = 0;        // state-space: convolved channels [T][channels], per-head decay and step [2][T][heads]
     int max_conv = 0, max_ssd_heads = 0;
-    size_t o_rec = 0, max_rec = 0;        // prompts' four-token scan: records of a group over all heads [floats]
+    size_t o_rec = 0, max_rec = 0, max_quad = 0;      // prompts' scans: records of a chunk, of a group over all heads [floats]
     size_t o_pairs = 0;                   // four-token scan: products between a group's queries and keys
     int max_pair_heads = 0;
     SmolLmGlobals g{};
@@ -2268,14 +2269,15 @@ extern "C" int smol_lm_create(const SmolLmConfig* cfg, const SmolLmLayer* layers
     for (const RunInfo& r : m->runs)
         for (const SmolLmLayer* L : {(const SmolLmLayer*)&m->layers[r.layer], m->layers[r.layer].side}) {
             if (!L) continue;
-            const bool ssd = L->mixer == SMOL_LM_MIX_STATE_SPACE;
-            int form = -1;
-            if (L->mixer == SMOL_LM_MIX_GENERAL_DELTA) form = kFormGeneral;
-            else if (ssd || L->mixer == SMOL_LM_MIX_GATED_LINEAR || L->mixer == SMOL_LM_MIX_LIGHTNING || L->mixer == SMOL_LM_MIX_HGRN2 ||
-                     L->mixer == SMOL_LM_MIX_RETENTION) form = kFormAdd;
-            if (form >= 0) m->max_rec = std::max(m->max_rec, (size_t)L->heads * quad_record(form, quad_pad(ssd ? L->n_state : L->dim)));
+            const bool ssd = L->mixer == SMOL_LM_MIX_STATE_SPACE, general = L->mixer == SMOL_LM_MIX_GENERAL_DELTA, unit = L->mixer == SMOL_LM_MIX_MLSTM;
+            const bool removes = general || L->mixer == SMOL_LM_MIX_GATED_DELTA;
+            if (removes || ssd || unit || L->mixer == SMOL_LM_MIX_GATED_LINEAR || L->mixer == SMOL_LM_MIX_LIGHTNING || L->mixer == SMOL_LM_MIX_HGRN2 ||
+                L->mixer == SMOL_LM_MIX_RETENTION)
+                m->max_rec = std::max(m->max_rec, (size_t)L->heads * chunk_record(removes, chunk_pad(ssd ? L->n_state : L->dim), general ? L->dim : L->vdim + (unit ? 1 : 0)));
+            if (general || (!removes && !unit)) m->max_quad = std::max(m->max_quad, (size_t)L->heads * quad_record(general ? kFormGeneral : kFormAdd, quad_pad(ssd ? L->n_state : L->dim)));
         }
-    if (m->max_rec > 0 && cfg->max_step_tokens >= kQuadMinTokens) m->o_rec = carve((T / kQuad + cfg->max_step_seqs + 1) * m->max_rec * 4);
+    if (m->max_rec > 0 && cfg->max_step_tokens >= kQuadMinTokens)
+        m->o_rec = carve(std::max((T / kChunk + cfg->max_step_seqs + 1) * m->max_rec, (T / kQuad + cfg->max_step_seqs + 1) * m->max_quad) * 4);
     if (m->max_pair_heads > 0) m->o_pairs = carve(T * (size_t)m->max_pair_heads * kPairFloats * 4);
     if (m->max_top > 0) {
         const size_t pairs = T * (size_t)m->max_top;
@@ -2326,6 +2328,22 @@ static cudaError_t quad_attribute() {
     if (e == cudaSuccess) e = cudaFuncSetAttribute(quad_scan_kernel<DK, kFormGeneral>, cudaFuncAttributeMaxDynamicSharedMemorySize, std::max(kScanSpread, (int)quad_smem(kFormGeneral, DK)));
     return e;
 }
+template <int DK>
+static cudaError_t chunk_attributes() {
+    const auto allow = [](auto kernel, size_t bytes) { return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes); };
+    cudaError_t e = allow(chunk_scan_kernel<DK, true, 1>, std::max((size_t)kScanSpread, chunk_smem(true, DK, 1)));
+    if (e == cudaSuccess) e = allow(chunk_scan_kernel<DK, false, 1>, std::max((size_t)kScanSpread, chunk_smem(false, DK, 1)));
+    if constexpr (DK > 64) {
+        if (e == cudaSuccess) e = allow(chunk_scan_kernel<DK, true, 2>, chunk_smem(true, DK, 2));
+        if (e == cudaSuccess) e = allow(chunk_scan_kernel<DK, false, 2>, chunk_smem(false, DK, 2));
+    }
+    const size_t with = chunk_prep_floats(true, DK) * sizeof(float), without = chunk_prep_floats(false, DK) * sizeof(float);
+    if (e == cudaSuccess) e = allow(chunk_prep_kernel<kScanGeneralDelta, DK>, with);
+    if (e == cudaSuccess) e = allow(chunk_prep_kernel<kScanGatedDelta, DK>, with);
+    if (e == cudaSuccess) e = allow(chunk_prep_kernel<kScanChannelDecay, DK>, without);
+    if (e == cudaSuccess) e = allow(chunk_prep_kernel<kScanHeadDecay, DK>, without);
+    return e;
+}
 static constexpr int flash_smem_bytes(int DK, int DV, bool vk, int maps = 1) { return 2 * 64 * (maps * (DK + 8) + (vk ? 0 : DV + 8)) * (int)sizeof(bf16); }
 
 template <int DK, int HPW>
@@ -2343,9 +2361,13 @@ static cudaError_t set_kernel_attributes() {
     if (e == cudaSuccess) e = scan_attribute<128>();
     if (e == cudaSuccess) e = scan_attribute<256>();
     if (e == cudaSuccess) e = quad_attribute<32>();
+    if (e == cudaSuccess) e = chunk_attributes<32>();
     if (e == cudaSuccess) e = quad_attribute<64>();
+    if (e == cudaSuccess) e = chunk_attributes<64>();
     if (e == cudaSuccess) e = quad_attribute<128>();
+    if (e == cudaSuccess) e = chunk_attributes<128>();
     if (e == cudaSuccess) e = quad_attribute<256>();
+    if (e == cudaSuccess) e = chunk_attributes<256>();
     if (e == cudaSuccess) e = cudaFuncSetAttribute(attn_split_kernel<T, 8, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, kAttnSplitSmemMax);
     if (e == cudaSuccess) e = cudaFuncSetAttribute(attn_split_kernel<T, 8, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, kAttnSplitWideSmem);
     if (e == cudaSuccess) e = cudaFuncSetAttribute(attn_split_kernel<T, 16, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, kAttnSplitSmemMax);
@@ -2812,6 +2834,48 @@ static cudaError_t launch_quad(SmolLm* m, const QuadSource& Q, const QuadArgs& A
     }
 }
 
+// The scan by chunks where some sequence is long enough; shorter ones lose by the records what the chain saves.  One layer's recurrence as a whole, by chunks and
+// four tokens at a time: generalized delta rule, 12 x 64 x 64, 128 / 260 / 1100 tokens 37 / 39 / 84 us against 41 / 49 / 146, 4 x 40 and 4 x 150 40 and 48 against
+// 31 and 48; 12 x 128 x 128, 128 / 260 / 1100 69 / 68 / 158 against 86 / 96 / 282; gated linear recurrence, 128 / 300 / 1100 26 / 27 / 63 against 26 / 36 / 95.
+static bool chunks_pay(int n_seqs, int n_tokens, int max_n, int d) { return max_n >= (d <= 64 ? kChunkMinTokens : kChunkMinTokensWide) && n_tokens >= kQuadMeanTokens * n_seqs; }
+// The same for the gated delta rule and the mLSTM, whose other form has no records to make: with many heads of up to 64 channels the SMs are full either way and
+// that form has less to do (gated delta rule, 12 heads, 1 / 4 / 7 / 16 x 260 tokens: 35 / 54 / 82 / 162 us against 45 / 60 / 78 / 147; 3 x 1000: 128 against 155; heads of
+// 128, 1 x 150 / 1 x 260 / 16 x 260: 80 / 61 / 351 against 76 / 74 / 391).
+static bool chunks_pay_beside_groups(int n_seqs, int heads, int n_tokens, int max_n, int d) {
+    return (d <= 64 ? max_n >= kChunkMinTokens && max_n >= 5 * n_seqs * heads : max_n >= kChunkMinTokensWideGroups) && n_tokens >= kQuadMeanTokens * n_seqs;
+}
+template <int KIND, int DK>
+static cudaError_t launch_chunks_sized(SmolLm* m, ChunkSource Q, ChunkArgs A, int n_seqs, int max_n, float* o_raw, cudaStream_t st, size_t min_smem) {
+    constexpr bool REM = scan_removes(KIND);
+    float* rec = reinterpret_cast<float*>(m->ws + m->o_rec);
+    Q.cap = A.cap = m->cfg.max_step_tokens / kChunk + m->cfg.max_step_seqs + 1;
+    pdl_launch(chunk_prep_kernel<KIND, DK>, dim3((max_n + kChunk - 1) / kChunk, n_seqs, Q.H), 128, chunk_prep_floats(REM, DK) * sizeof(float), st, Q, rec);
+    A.rec = rec;
+    // Above 64 channels a block has an SM to itself.  Where single blocks of columns would not all run at once, it takes two, whose products share the
+    // records' fragments (12 heads of 128, 1801 tokens: 140 us for 96 blocks of two, 144 for 192 single ones with half the ring, two to an SM; 3 x 12 heads of
+    // 64, 1000 tokens: 57 in twos, 46 single).
+    const int parts = chunk_blocks(Q.columns), threads = chunk_warps(DK) * 64 + 32;
+    if constexpr (DK > 64) {
+        if (n_seqs * A.H * parts > m->n_sms) {
+            plain_launch(chunk_scan_kernel<DK, REM, 2>, n_seqs * A.H * ((parts + 1) / 2), threads, std::max(chunk_smem(REM, DK, 2), min_smem), st, A, m->slots, o_raw);
+            m->launches += 1;
+            return cudaGetLastError();
+        }
+    }
+    plain_launch(chunk_scan_kernel<DK, REM, 1>, n_seqs * A.H * parts, threads, std::max(chunk_smem(REM, DK, 1), min_smem), st, A, m->slots, o_raw);
+    m->launches += 1;
+    return cudaGetLastError();
+}
+template <int KIND>
+static cudaError_t launch_chunks(SmolLm* m, const ChunkSource& Q, const ChunkArgs& A, int n_seqs, int max_n, float* o_raw, cudaStream_t st, size_t min_smem = 0) {
+    switch (chunk_pad(A.d)) {
+        case 32: return launch_chunks_sized<KIND, 32>(m, Q, A, n_seqs, max_n, o_raw, st, min_smem);
+        case 64: return launch_chunks_sized<KIND, 64>(m, Q, A, n_seqs, max_n, o_raw, st, min_smem);
+        case 128: return launch_chunks_sized<KIND, 128>(m, Q, A, n_seqs, max_n, o_raw, st, min_smem);
+        default: return launch_chunks_sized<KIND, 256>(m, Q, A, n_seqs, max_n, o_raw, st, min_smem);
+    }
+}
+
 template <int DK>
 static cudaError_t launch_gla_scan(const GlaArgs& A, int n_seqs, const float* dec, float* pool, float* o_raw, cudaStream_t st, size_t min_smem) {
     constexpr int CB = gla_block_cols(DK), threads = CB * gla_lanes(DK);
@@ -2824,6 +2888,13 @@ static cudaError_t launch_gla_scan(const GlaArgs& A, int n_seqs, const float* de
 // the scan over key sizes up to 256: the smallest built size that holds A.d
 static cudaError_t launch_gla_scan_any(SmolLm* m, const GlaArgs& A, int n_seqs, int n_tokens, int max_n, const float* dec, float* pool, float* o_raw, cudaStream_t st,
                                         size_t min_smem = 0) {
+    if (chunks_pay(n_seqs, n_tokens, max_n, A.d)) {
+        const ChunkSource Q{A.H, A.qk_share, A.d, A.dv, A.dv, A.q_src, A.k_src, A.q_ld, A.k_ld, A.v_src, A.v_ld, dec, A.head_decay, A.head_step, A.head_ld, 1,
+                            nullptr, nullptr, 0.0f, A.seq_start, 0};
+        const ChunkArgs S{A.H, A.d, A.dv, nullptr, 0, A.q_scale, A.seq_start, A.seq_pos0, A.seq_slot, A.slot_floats, A.state_off, A.n_slots, A.err, nullptr, 0, ConvIo{}};
+        if (A.head_decay) return launch_chunks<kScanHeadDecay>(m, Q, S, n_seqs, max_n, o_raw, st, min_smem);
+        return launch_chunks<kScanChannelDecay>(m, Q, S, n_seqs, max_n, o_raw, st, min_smem);
+    }
     if (quad_pays(n_seqs, n_tokens, max_n)) {
         QuadSource Q{A.H, A.qk_share, A.d, A.q_src, A.k_src, A.q_ld, A.k_ld, dec, A.head_decay, A.head_step, A.head_ld, 1, nullptr, nullptr, 0.0f, A.seq_start, 0};
         QuadArgs S{A.H, A.d, A.dv, nullptr, 0, A.v_src, A.v_ld, A.q_scale, A.seq_start, A.seq_pos0, A.seq_slot, A.slot_floats, A.state_off, A.n_slots, A.err};
@@ -2844,10 +2915,18 @@ static cudaError_t launch_group_scan(const GroupScanArgs& A, int n_seqs, float* 
     plain_launch(group_scan_kernel<DK, DELTA>, n_seqs * A.H * parts, threads, std::max(2 * group_scan_buf_floats(DK) * sizeof(float), min_smem), st, A, pool, o_raw);
     return cudaGetLastError();
 }
-// The four-token scan: the group's products (not needed where every sequence brings one token), then the recurrence itself.
+// The gated delta rule's and the mLSTM's scan: by chunks, or four tokens at a time -- the group's products (not needed where every sequence brings one
+// token), then the recurrence itself.
 template <bool DELTA>
-static cudaError_t launch_group_scan_any(SmolLm* m, const GroupScanArgs& A, float* pairs, int n_seqs, int max_n, float* pool, float* o_raw, cudaStream_t st,
+static cudaError_t launch_group_scan_any(SmolLm* m, const GroupScanArgs& A, float* pairs, int n_seqs, int n_tokens, int max_n, float* pool, float* o_raw, cudaStream_t st,
                                          size_t min_smem = 0) {
+    if (chunks_pay_beside_groups(n_seqs, A.H, n_tokens, max_n, A.d)) {
+        const ChunkSource Q{A.H, A.H / A.G, A.d, A.dv, A.dv + (A.unit_out ? 1 : 0), A.q_src, A.k_src, A.q_ld, A.k_ld, A.v_src, A.v_ld, nullptr, A.head, A.head + 1, 2 * A.H, 2,
+                            nullptr, nullptr, 0.0f, A.seq_start, 0};
+        const ChunkArgs S{A.H, A.d, A.dv, nullptr, 0, A.q_scale, A.seq_start, A.seq_pos0, A.seq_slot, A.slot_floats, A.state_off, A.n_slots, A.err, A.unit_out, A.unit_off, A.conv};
+        m->launches += 1;
+        return launch_chunks<DELTA ? kScanGatedDelta : kScanHeadDecay>(m, Q, S, n_seqs, max_n, o_raw, st, min_smem);
+    }
     if (max_n > 1) {
         pdl_launch(scan_pairs_kernel<DELTA>, dim3((max_n + kScanGroup - 1) / kScanGroup, n_seqs, (A.G + 3) / 4), 128, 0, st, A, pairs);
         m->launches++;
@@ -3287,7 +3366,7 @@ static int step_impl(SmolLm* m, const SmolLmStep* s, cudaStream_t st) {
             S.q_src = conv; S.k_src = conv + gd; S.v_src = conv + 2 * gd;
             S.q_ld = S.k_ld = S.v_ld = ch;
             S.conv = P.conv;
-            CU(launch_group_scan_any<true>(m, S, pairs, s->n_seqs, max_n, m->slots, oraw, ms));
+            CU(launch_group_scan_any<true>(m, S, pairs, s->n_seqs, Tn, max_n, m->slots, oraw, ms));
             GlaArgs A = scan_args(M, Ri, pj);
             A.out_norm = M.out_norm; A.gate_off = ch; A.out_ld = ld; A.out_scale = M.mix_scale;
             pdl_launch(gla_out_kernel<T>, (Tn * M.heads + 3) / 4, 128, 0, ms, A, oraw, mix_at);
@@ -3311,7 +3390,7 @@ static int step_impl(SmolLm* m, const SmolLmStep* s, cudaStream_t st) {
             S.q_ld = S.k_ld = S.v_ld = n_in;
             S.q_scale = M.score_scale;
             S.unit_out = den; S.unit_off = Ri.unit_off;
-            CU(launch_group_scan_any<false>(m, S, pairs, s->n_seqs, max_n, m->slots, oraw, ms, ms != st && Tn > kGraphMaxTokens ? kScanSpread : 0));
+            CU(launch_group_scan_any<false>(m, S, pairs, s->n_seqs, Tn, max_n, m->slots, oraw, ms, ms != st && Tn > kGraphMaxTokens ? kScanSpread : 0));
             GlaArgs A = scan_args(M, Ri, pj);
             A.den = den; A.den_floor = floor_at; A.den_eps = M.den_eps;
             A.out_norm = M.out_norm; A.norm_own = 1; A.gate_sigmoid = 1; A.out_ld = ld; A.out_scale = M.mix_scale;
@@ -3576,15 +3655,21 @@ static int step_impl(SmolLm* m, const SmolLmStep* s, cudaStream_t st) {
             A.rate_bias = L.rate_bias; A.decay_w2 = L.decay_w2; A.decay_bias = L.decay_bias; A.out_norm = L.out_norm;
             A.seq_start = s->seq_start; A.seq_pos0 = s->seq_pos0; A.seq_slot = s->seq_slot;
             A.slot_floats = m->slot_floats; A.state_off = R.state_off; A.n_slots = m->n_slots; A.err = err;
-            const bool quad = quad_pays(s->n_seqs, Tn, max_n);
-            float *u_to = quad ? nullptr : uk, *au_to = quad ? nullptr : auk;
+            const bool chunks = chunks_pay(s->n_seqs, Tn, max_n, L.dim), quad = !chunks && quad_pays(s->n_seqs, Tn, max_n);
+            float *u_to = chunks || quad ? nullptr : uk, *au_to = chunks || quad ? nullptr : auk;
             const size_t prep_smem = (size_t)(L.rank + L.heads) * sizeof(float);
             const int slices = (L.heads * L.dim + 127) / 128;
             if (Tn >= kDecayMinTokens && kDecayTokens * prep_smem <= 48 * 1024)
                 pdl_launch(delta_prep_kernel<kDecayTokens>, dim3((Tn + kDecayTokens - 1) / kDecayTokens, slices), 128, kDecayTokens * prep_smem, st, A, dec, u_to, au_to);
             else pdl_launch(delta_prep_kernel<1>, dim3(Tn, slices), 128, prep_smem, st, A, dec, u_to, au_to);
             cudaError_t e;
-            if (quad) {
+            if (chunks) {
+                const int HD = L.heads * L.dim;
+                const ChunkSource Q{L.heads, 1, L.dim, L.dim, L.dim, proj, proj + HD, n_in, n_in, proj + 2 * HD, n_in, dec, nullptr, nullptr, 0, 0,
+                                    proj + 4 * HD, L.rate_bias, L.unit_eps, s->seq_start, 0};
+                const ChunkArgs S{L.heads, L.dim, L.dim, nullptr, 0, 1.0f, s->seq_start, s->seq_pos0, s->seq_slot, m->slot_floats, R.state_off, m->n_slots, err, nullptr, 0, ConvIo{}};
+                e = launch_chunks<kScanGeneralDelta>(m, Q, S, s->n_seqs, max_n, oraw, st);
+            } else if (quad) {
                 const int HD = L.heads * L.dim;
                 QuadSource Q{L.heads, 1, L.dim, proj, proj + HD, n_in, n_in, dec, nullptr, nullptr, 0, 0, proj + 4 * HD, L.rate_bias, L.unit_eps, s->seq_start, 0};
                 QuadArgs S{L.heads, L.dim, L.dim, nullptr, 0, proj + 2 * HD, n_in, 1.0f, s->seq_start, s->seq_pos0, s->seq_slot, m->slot_floats, R.state_off, m->n_slots, err};

@@ -1,4 +1,4 @@
-// The recurrences' scan for prompts, four tokens at a time (included by lm_kernels.cu after lm_delta_mlstm.cuh).  Everything is fp32.
+// The recurrences' scan for short prompts, four tokens at a time (included by lm_kernels.cu after lm_delta_mlstm.cuh; long ones: lm_chunk_scan.cuh).  Everything is fp32.
 //
 // The generalized delta rule and the linear attentions act on a head's state S [d, dv] as
 //     S <- diag(w) S - a (u^T S) + k v^T,     o = S^T r

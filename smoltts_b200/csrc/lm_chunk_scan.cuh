@@ -80,15 +80,9 @@ __host__ __device__ constexpr int chunk_prep_floats(bool removes, int DK) {
     return kChunk * ((removes ? 2 : 1) * (DK + 4 + DK + 8) + DK + 4) + 4 * DK + (removes ? 4 : 1) * kChunk * kChunk;
 }
 
-// x = hi + lo + less than the last place, both within tf32's 11 bits (the MMA ignores what lo has behind them)
-__device__ __forceinline__ void tf32_parts(float x, uint32_t& hi, uint32_t& lo) {
-    hi = (__float_as_uint(x) + 0x1000u) & 0xffffe000u;
-    lo = __float_as_uint(x - __uint_as_float(hi));
-}
-__device__ __forceinline__ void mma_tf32(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
-    asm("mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-        : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
-}
+__device__ __forceinline__ void tf32_parts(float x, uint32_t& hi, uint32_t& lo) { f32t::tf32_parts(__float_as_uint(x), hi, lo); }
+using f32t::mma_tf32;
+// The two tf32 parts of fp32 fragments (f32_tile.cuh)
 struct PartsA {
     uint32_t hi[4], lo[4];
     __device__ __forceinline__ void set(float x, float y, float z, float w) {

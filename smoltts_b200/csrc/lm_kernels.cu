@@ -284,11 +284,11 @@ static GemmIo plain_io(int K, int N) {
 // (f32_tile.cuh), K shared by a cluster of CTAs along grid.x where the output has too few tiles to fill the GPU.
 // 300 rows, 768 to 4608 columns and k: 65 us a product against 331 on the form below, which stages element by element and is bound by
 // instruction issue.
-template <int BM, int BN, int TM, int TN>
-__global__ void __launch_bounds__(f32t::Tile<BM, BN, TM, TN>::NT) gemm_f32_tile_kernel(const float* __restrict__ a, const float* __restrict__ w,
+template <int BM, int BN, int WM, int WN>
+__global__ void __launch_bounds__(f32t::MmaTile<BM, BN, WM, WN>::NT) gemm_f32_tile_kernel(const float* __restrict__ a, const float* __restrict__ w,
                                                                                        float* __restrict__ y, int M, int N, int K, const GemmIo io) {
     dep_wait();      // (and no early dep_go: the next kernel's blocks would take room from the CTAs that are still to come)
-    using T = f32t::Tile<BM, BN, TM, TN>;
+    using T = f32t::MmaTile<BM, BN, WM, WN>;
     extern __shared__ __align__(16) float f32_sm[];
     __shared__ long long arow[BM];
     int m0 = blockIdx.y * BM;
@@ -309,9 +309,9 @@ __global__ void __launch_bounds__(f32t::Tile<BM, BN, TM, TN>::NT) gemm_f32_tile_
     }
     __syncthreads();
     int k_lo, k_hi;
-    T::range(K, k_lo, k_hi);
-    float out[TM][TN];
-    T::template product<0>(f32_sm, k_lo, k_hi, [&](int r) { return arow[r] >= 0 ? a + arow[r] : nullptr; }, [](int k) -> long long { return k; },
+    f32t::rank_range(K, k_lo, k_hi);
+    typename T::Out out;
+    T::product(f32_sm, k_lo, k_hi, [&](int r) { return arow[r] >= 0 ? a + arow[r] : nullptr; }, [](int k) -> long long { return k; },
                            [&](int r) { return n0 + r < N ? w + (size_t)(n0 + r) * K : nullptr; }, [] {}, out);
     const bool whole = io.ldy % 4 == 0 && reinterpret_cast<uintptr_t>(y) % 16 == 0;
     T::finish(f32_sm, out, [&](int r, int c, float4 v) {
@@ -2627,9 +2627,9 @@ template <class T>
 static cudaError_t linear_ex(SmolLm* m, const T* a, const T* w, float* y, int M, int N, int K, const GemmIo& io, int batch, int tiles,
                              cudaStream_t st);
 
-template <int BM, int BN, int TM, int TN>
+template <int BM, int BN, int WM, int WN>
 static cudaError_t launch_f32_tile(const float* a, const float* w, float* y, int M, int N, int K, const GemmIo& io, int batch, int row_tiles, cudaStream_t st) {
-    using T = smol::f32t::Tile<BM, BN, TM, TN>;
+    using T = smol::f32t::MmaTile<BM, BN, WM, WN>;
     const int cols = (N + BN - 1) / BN;
     // CTAs per tile: as many as bring the grid of a single row of tiles to about four per SM, each with at least 128 k.  From N, K and the
     // batch alone: a row's sums must not depend on how many rows the step holds.  (With S from the rows as well 1024 rows of 4608 x 768 took 179 us, 201 now,
@@ -2648,7 +2648,7 @@ static cudaError_t launch_f32_tile(const float* a, const float* w, float* y, int
     cfg.attrs = at;
     cfg.numAttrs = 1;
     t_plain_next = false;      // launched plainly, as plain_launch does
-    return cudaLaunchKernelEx(&cfg, gemm_f32_tile_kernel<BM, BN, TM, TN>, a, w, y, M, N, K, io);
+    return cudaLaunchKernelEx(&cfg, gemm_f32_tile_kernel<BM, BN, WM, WN>, a, w, y, M, N, K, io);
 }
 
 template <>
@@ -2657,9 +2657,9 @@ cudaError_t linear_ex<float>(SmolLm* m, const float* a, const float* w, float* y
     m->launches++;
     // whole 16-byte pieces in every row of both operands
     if (K % 4 == 0 && io.lda % 4 == 0 && io.sa % 4 == 0 && io.sw % 4 == 0 && (reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(w)) % 16 == 0) {
-        if (io.tile_group) return launch_f32_tile<kGroupTile, 64, 8, 8>(a, w, y, M, N, K, io, 1, tiles, st);
-        if (M <= 16) return launch_f32_tile<16, 64, 4, 4>(a, w, y, M, N, K, io, batch, (M + 15) / 16, st);
-        return launch_f32_tile<64, 64, 8, 8>(a, w, y, M, N, K, io, batch, (M + 63) / 64, st);
+        if (io.tile_group) return launch_f32_tile<kGroupTile, 64, 16, 32>(a, w, y, M, N, K, io, 1, tiles, st);
+        if (M <= 16) return launch_f32_tile<16, 64, 16, 16>(a, w, y, M, N, K, io, batch, (M + 15) / 16, st);
+        return launch_f32_tile<64, 64, 32, 32>(a, w, y, M, N, K, io, batch, (M + 63) / 64, st);
     }
     if (io.tile_group) {
         dim3 grid((N + 63) / 64, tiles, 1);

@@ -367,9 +367,8 @@ __global__ void __launch_bounds__(kThreads) lin_kernel(const RowOp op) {
 // Bound by the FMAs and, with them in balance, shared-memory loads (f32_tile.cuh): 48 streams, 4 frames at once, 3.59 ms for 83 GFLOP (23
 // TFLOP/s; 64 x 64 plain-FMA tiles of 4 x 4 outputs and a warp per weight row before: 1.75 ms per single frame).  128 x 128 tiles of
 // 256 threads, ELU and LayerNorm applied by every block that reads the rows: 5.9 ms.
-template <int BM, int BN, int TM, int TN, int RUN>
-__global__ void __launch_bounds__(f32t::Tile<BM, BN, TM, TN>::NT) tile_kernel(const RowOp op) {
-    using T = f32t::Tile<BM, BN, TM, TN>;
+template <int BM, int BN, class T>
+__global__ void __launch_bounds__(T::NT) tile_kernel(const RowOp op) {
     extern __shared__ __align__(16) float tile_sm[];
     __shared__ int s_slot[BM], s_t[BM], s_b[BM];
     const int tid = threadIdx.x, rows = op.batch * op.T;
@@ -383,9 +382,9 @@ __global__ void __launch_bounds__(f32t::Tile<BM, BN, TM, TN>::NT) tile_kernel(co
     __syncthreads();
     const int turn = op.tapstep < 0 ? op.in_c : op.K;      // transposed convolution: from here on the previous row's channels
     int k_lo, k_hi;
-    T::range(op.K, k_lo, k_hi);
-    float out[TM][TN];
-    T::template product<RUN>(tile_sm, k_lo, k_hi,
+    f32t::rank_range(op.K, k_lo, k_hi);
+    typename T::Out out;
+    T::product(tile_sm, k_lo, k_hi,
                              [&](int r) -> const float* {
                                  return s_slot[r] < 0 ? nullptr : op.in + (long long)s_slot[r] * op.in_stride + (long long)(op.in_hs + s_t[r] + op.tap0) * op.in_c;
                              },
@@ -1014,9 +1013,8 @@ static bool use_tile(const RowOp& op) {
     return (op.batch >= kTileMinBatch || rows_per_frame(op) >= 16) && op.N >= 16 && op.N % 4 == 0 && op.bias_mod % (op.bias ? 4 : 1) == 0 && op.K % 4 == 0 && op.in_c % 4 == 0 &&
            (op.tapstep > 0 || op.K == 2 * op.in_c) && (op.pro == PRO_NONE || (op.norm_at && op.K <= 32 * kNormRegs));
 }
-template <int BM, int BN, int TM, int TN, int RUN>
-static cudaError_t launch_tile_run(const RowOp& op, int split, cudaStream_t st) {
-    using T = smol::f32t::Tile<BM, BN, TM, TN>;
+template <int BM, int BN, class T>
+static cudaError_t launch_tile_of(const RowOp& op, int split, cudaStream_t st) {
     static_assert(T::kSmemBytes <= 48 * 1024, "no attribute needed");
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3((op.N + BN - 1) / BN * split, (op.batch * op.T + BM - 1) / BM);
@@ -1030,11 +1028,12 @@ static cudaError_t launch_tile_run(const RowOp& op, int split, cudaStream_t st) 
     at[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = at;
     cfg.numAttrs = g_pdl ? 2 : 1;
-    return cudaLaunchKernelEx(&cfg, tile_kernel<BM, BN, TM, TN, RUN>, op);
+    return cudaLaunchKernelEx(&cfg, tile_kernel<BM, BN, T>, op);
 }
 template <int BM, int BN, int TM, int TN>
 static cudaError_t launch_tile(const RowOp& op, int split, cudaStream_t st) {
-    return op.batch >= kTileMinBatch ? launch_tile_run<BM, BN, TM, TN, 0>(op, split, st) : launch_tile_run<BM, BN, TM, TN, kFewStreamRun>(op, split, st);
+    if (op.batch >= kTileMinBatch) return launch_tile_of<BM, BN, smol::f32t::Tile<BM, BN, TM, TN, 0>>(op, split, st);
+    return launch_tile_of<BM, BN, smol::f32t::Tile<BM, BN, TM, TN, kFewStreamRun>>(op, split, st);
 }
 static cudaError_t launch_tiles(const RowOp& op, cudaStream_t st) {
     const int rows = op.batch * op.T;

@@ -1022,6 +1022,150 @@ __device__ __forceinline__ float2 load_pair(const bf16* p) {
 // row stride of the staged values: an even number of elements
 template <class T> __host__ __device__ constexpr int split_value_ld(int dv) { return (dv + 16 / (int)sizeof(T) + 1) / 2 * 2; }
 
+// Prompts without a tensor-core form (float32; bf16 heads above 128): a block takes 4 R neighbouring rows of a sequence and one head, a warp R of them, 32 keys and
+// values at a time in shared memory.  A lane scores one key for the warp's R rows, so a key's 16-byte loads and a value's are shared by R rows; a row's sums are
+// those of a warp of its own: it takes nothing from a key or value that it does not see.
+// What bounds it is shared memory: a 16-byte load of a key and one of each query for 4 R multiply-adds.  300 rows of 12 heads of 64, float32: 60 us
+// (1100: 332) against 230 (2237) for a warp per row that reads its keys from global memory, a row per lane (attn_kernel, which stays for rows that leave no room
+// for the tiles); 9 rows 5.7 against 8.8, 7 x 170 76 against 249; two maps of 64 and values of 128, 300 rows 91 against 330; a latent of 160, 79 against 431.
+constexpr int kRowsKeys = 32, kRowsWarps = 4, kRowsSmemMax = 100 * 1024;
+template <class T> __host__ __device__ constexpr int rows_ld(int d) { return (d * (int)sizeof(T) + 15) / 16 * 16 / (int)sizeof(T) + 16 / (int)sizeof(T); }      // 16-byte rows, an odd number of them
+template <class T> static constexpr size_t rows_smem(int R, int d, int dv, bool v_in_k) {
+    return (size_t)kRowsWarps * R * ((d + 3) / 4 * 4 + kRowsKeys) * 4 + (size_t)kRowsKeys * (rows_ld<T>(d) + (v_in_k ? 0 : rows_ld<T>(dv))) * sizeof(T);
+}
+template <class T, int MAXV, int MAPS, int R>
+__global__ void __launch_bounds__(kRowsWarps * 32) attn_rows_kernel(const AttnArgs A, const T* __restrict__ qbuf, const T* __restrict__ pool, T* __restrict__ out) {
+    dep_wait();
+    dep_go();
+    extern __shared__ __align__(16) unsigned char sm_raw[];
+    constexpr int kPad = 16 / (int)sizeof(T), KEYS = kRowsKeys, RB = kRowsWarps * R;
+    const int h = blockIdx.y, s = blockIdx.z, t0 = A.seq_start[s], n = A.seq_start[s + 1] - t0, r0 = blockIdx.x * RB;
+    if (r0 >= n) return;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = h / (A.H / A.G), rows = min(RB, n - r0);
+    const int pos0 = A.tok_pos[t0 + r0], mine = min(R, max(0, rows - warp * R)), my_pos = pos0 + warp * R;      // (a sequence's tokens of a step are neighbours)
+    const int qd = (A.d + 3) / 4 * 4, ldk = rows_ld<T>(A.d), ldv = A.v_in_k ? ldk : rows_ld<T>(A.dv);
+    float* qs = reinterpret_cast<float*>(sm_raw) + warp * R * qd;
+    float* ps = reinterpret_cast<float*>(sm_raw) + RB * qd + warp * R * KEYS;      // [KEYS][R]
+    T* Ks = reinterpret_cast<T*>(sm_raw + (size_t)RB * (qd + KEYS) * 4);
+    T* Vs = A.v_in_k ? Ks : Ks + KEYS * ldk;
+    const int32_t* bt = A.block_table + (size_t)s * A.max_pages;
+    const float r1 = A.r1 ? A.r1[h] : 0.0f, r2 = A.r1 ? A.r2[h] : 0.0f, slope = A.slope ? A.slope[h] : 0.0f;
+    const bool kvec = (A.d * sizeof(T)) % 16 == 0 && (A.k_ld * sizeof(T)) % 16 == 0 && (A.k_off * sizeof(T)) % 16 == 0;
+    const bool vvec = (A.dv * sizeof(T)) % 16 == 0 && (A.v_ld * sizeof(T)) % 16 == 0 && (A.v_off * sizeof(T)) % 16 == 0;
+    const int kchunks = kvec ? A.d / kPad : A.d, vchunks = A.v_in_k ? 0 : vvec ? A.dv / kPad : A.dv;
+    const int j_first = attn_first_key(A, pos0), j_last = pos0 + rows - 1;
+    float sum[R][MAXV];                    // the maps' joined results
+#pragma unroll
+    for (int map = 0; map < MAPS; ++map) {
+        __syncwarp();
+        for (int i = 0; i < mine; ++i)
+            for (int c = lane; c < qd; c += 32) qs[i * qd + c] = c < A.d ? to_f<T>(qbuf[(((size_t)(t0 + r0 + warp * R + i) * A.H + h) * MAPS + map) * A.d + c]) : 0.0f;
+        float m[R], l[R], o[R][MAXV];
+#pragma unroll
+        for (int i = 0; i < R; ++i) {
+            m[i] = A.sink ? A.sink[h] : -INFINITY;
+            l[i] = A.sink ? 1.0f : 0.0f;
+#pragma unroll
+            for (int e = 0; e < MAXV; ++e) o[i][e] = 0.0f;
+        }
+        for (int j0 = j_first; j0 <= j_last; j0 += KEYS) {
+            const int cnt = min(KEYS, j_last - j0 + 1);
+            __syncthreads();
+            {
+                const int jr = min(j0 + lane, j_last), page = bt[jr / A.page_size], place = jr % A.page_size;
+                for (int c = lane; c - lane < kchunks + vchunks; c += 32) {
+                    const bool key = c < kchunks, live = c < kchunks + vchunks;
+                    const int piece = key ? c : c - kchunks, step = (key ? kvec : vvec) ? kPad : 1, ld = key ? A.k_ld : A.v_ld, dst_ld = key ? ldk : ldv;
+                    const T* src0 = pool + (key ? A.k_off + (size_t)(g * MAPS + map) * A.page_size * ld : A.v_off + (size_t)g * A.page_size * ld) + piece * step;
+                    T* dst0 = (key ? Ks : Vs) + piece * step;
+#pragma unroll 4
+                    for (int r = warp; r < cnt; r += kRowsWarps) {
+                        const int pg = __shfl_sync(0xffffffffu, page, r), at = __shfl_sync(0xffffffffu, place, r);
+                        const T* src = src0 + (size_t)pg * A.page_elems + (size_t)at * ld;
+                        T* dst = dst0 + r * dst_ld;
+                        if (!live) continue;
+                        if (step == kPad) cp_async16(dst, src);
+                        else *dst = *src;
+                    }
+                }
+                cp_async_commit_group();
+                cp_async_wait_group<0>();
+            }
+            __syncthreads();
+            if (mine == 0 || j0 > my_pos + mine - 1) continue;
+            float dot[R];
+#pragma unroll
+            for (int i = 0; i < R; ++i) dot[i] = 0.0f;
+            const T* kr = Ks + lane * ldk;
+            int c = 0;
+            if (sizeof(T) == 4) {
+#pragma unroll 4
+                for (; c + 4 <= A.d; c += 4) {
+                    const float4 k = *reinterpret_cast<const float4*>(kr + c);
+#pragma unroll
+                    for (int i = 0; i < R; ++i) {
+                        const float4 q = *reinterpret_cast<const float4*>(qs + i * qd + c);
+                        dot[i] = fmaf(q.x, k.x, fmaf(q.y, k.y, fmaf(q.z, k.z, fmaf(q.w, k.w, dot[i]))));
+                    }
+                }
+            }
+            for (; c < A.d; ++c) {
+                const float k = to_f<T>(kr[c]);
+#pragma unroll
+                for (int i = 0; i < R; ++i) dot[i] = fmaf(qs[i * qd + c], k, dot[i]);
+            }
+            const int j = j0 + lane;
+            int lo[R], hi[R], all_lo = 0, all_hi = KEYS - 1;      // the tile's keys that a row sees; that every row sees
+#pragma unroll
+            for (int i = 0; i < R; ++i) {
+                const int pos = my_pos + i;
+                lo[i] = max(0, attn_first_key(A, pos) - j0);
+                hi[i] = i < mine ? min(cnt - 1, pos - j0) : -1;
+                all_lo = max(all_lo, lo[i]);
+                all_hi = min(all_hi, hi[i]);
+                const bool seen = lane >= lo[i] && lane <= hi[i];
+                const float sc = seen ? attn_score<false>(A, dot[i], pos - j, r1, r2, slope) : -INFINITY;
+                const float mn = fmaxf(m[i], warp_max(sc));
+                const float p = seen ? expf(sc - mn) : 0.0f, corr = mn == -INFINITY ? 1.0f : expf(m[i] - mn);
+                l[i] = l[i] * corr + warp_sum(p);
+                m[i] = mn;
+                ps[lane * R + i] = p;
+#pragma unroll
+                for (int e = 0; e < MAXV; ++e) o[i][e] *= corr;
+            }
+            __syncwarp();
+            auto add = [&](int jj, bool every) {
+                float p[R];
+#pragma unroll
+                for (int i = 0; i < R; ++i) p[i] = ps[jj * R + i];
+#pragma unroll
+                for (int e = 0; e < MAXV; ++e) {
+                    const int c2 = lane + 32 * e;
+                    if (c2 >= A.dv) continue;
+                    const float v = to_f<T>(Vs[jj * ldv + c2]);
+#pragma unroll
+                    for (int i = 0; i < R; ++i)
+                        if (every || (jj >= lo[i] && jj <= hi[i])) o[i][e] = fmaf(p[i], v, o[i][e]);
+                }
+            };
+            for (int jj = 0; jj < min(all_lo, cnt); ++jj) add(jj, false);
+#pragma unroll 4
+            for (int jj = all_lo; jj <= all_hi; ++jj) add(jj, true);
+            for (int jj = max(all_lo, all_hi + 1); jj < cnt; ++jj) add(jj, false);
+            __syncwarp();
+        }
+#pragma unroll
+        for (int i = 0; i < R; ++i) {
+            const float inv = 1.0f / l[i];
+#pragma unroll
+            for (int e = 0; e < MAXV; ++e) sum[i][e] = map == 0 ? o[i][e] * inv : fmaf(-A.diff_lambda, o[i][e] * inv, sum[i][e]);
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < R; ++i)
+        if (i < mine) attn_finish<T, MAXV, MAPS>(A, t0 + r0 + warp * R + i, h, lane, sum[i], out);
+}
+
 template <class T, int MAXV, int KPL>
 __global__ void __launch_bounds__(256) attn_split_kernel(const AttnArgs A, const T* __restrict__ qbuf, const T* __restrict__ pool) {
     dep_wait();
@@ -2368,6 +2512,11 @@ static cudaError_t set_kernel_attributes() {
     if (e == cudaSuccess) e = chunk_attributes<128>();
     if (e == cudaSuccess) e = quad_attribute<256>();
     if (e == cudaSuccess) e = chunk_attributes<256>();
+    const auto rows = [&](auto kernel) {
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kRowsSmemMax);
+    };
+    rows(attn_rows_kernel<T, 8, 1, 1>); rows(attn_rows_kernel<T, 8, 2, 1>); rows(attn_rows_kernel<T, 16, 1, 1>); rows(attn_rows_kernel<T, 16, 2, 1>);
+    rows(attn_rows_kernel<T, 8, 1, 4>); rows(attn_rows_kernel<T, 8, 2, 4>); rows(attn_rows_kernel<T, 16, 1, 4>); rows(attn_rows_kernel<T, 16, 2, 4>);
     if (e == cudaSuccess) e = cudaFuncSetAttribute(attn_split_kernel<T, 8, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, kAttnSplitSmemMax);
     if (e == cudaSuccess) e = cudaFuncSetAttribute(attn_split_kernel<T, 8, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, kAttnSplitWideSmem);
     if (e == cudaSuccess) e = cudaFuncSetAttribute(attn_split_kernel<T, 16, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, kAttnSplitSmemMax);
@@ -3019,7 +3168,13 @@ static void launch_attention(SmolLm* m, const SmolLmStep* s, AttnArgs& A, bool f
         } else {
             // every row, also those of short sequences
             const int au = Tn * A.H;
-            plain_launch(attn_kernel<T, MAXV, MAPS>, (au + kAttnWarps - 1) / kAttnWarps, kAttnWarps * 32, kAttnWarps * A.d * sizeof(float), st, A, qbuf, pool, mix);
+            // four rows of a warp where that still fills the SMs
+            const int R = s->n_seqs * A.H * ((max_n + 15) / 16) >= m->n_sms ? 4 : 1;
+            const size_t smem = rows_smem<T>(R, A.d, A.dv, A.v_in_k);
+            if (smem > (size_t)kRowsSmemMax)
+                plain_launch(attn_kernel<T, MAXV, MAPS>, (au + kAttnWarps - 1) / kAttnWarps, kAttnWarps * 32, kAttnWarps * A.d * sizeof(float), st, A, qbuf, pool, mix);
+            else if (R == 4) plain_launch(attn_rows_kernel<T, MAXV, MAPS, 4>, dim3((max_n + 15) / 16, A.H, s->n_seqs), kRowsWarps * 32, smem, st, A, qbuf, pool, mix);
+            else plain_launch(attn_rows_kernel<T, MAXV, MAPS, 1>, dim3((max_n + 3) / 4, A.H, s->n_seqs), kRowsWarps * 32, smem, st, A, qbuf, pool, mix);
         }
         m->launches += 1;
     }

@@ -56,6 +56,44 @@ __device__ __forceinline__ float block_sum(float v, float* red) {
     return red[32];
 }
 
+// A row in registers as 16-byte pieces, V per thread.  LONE: the row has a block of its own, a piece per thread, and the warps' sums meet behind one barrier;
+// otherwise the row has one warp and needs none.
+template <int V, bool LONE>
+struct RowPieces {
+    __device__ static __forceinline__ int row() { return LONE ? (int)blockIdx.x : (int)(blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)); }
+    __device__ static __forceinline__ int column(int i) { return 4 * (LONE ? (int)threadIdx.x : (int)(threadIdx.x & 31) + 32 * i); }
+    // `red`: 16 floats that no other sum of the kernel uses
+    __device__ static __forceinline__ float sum(float v, float* red) {
+        v = warp_sum(v);
+        if (!LONE) return v;
+        const int nw = (int)blockDim.x >> 5;
+        if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
+        __syncthreads();
+        float t = red[0];
+        for (int i = 1; i < nw; ++i) t += red[i];
+        return t;
+    }
+};
+__device__ __forceinline__ float4 load4(const float* p) { return *reinterpret_cast<const float4*>(p); }
+__device__ __forceinline__ float4 load4(const bf16* p) {
+    const uint2 v = *reinterpret_cast<const uint2*>(p);
+    return make_float4(bf_lo(v.x), bf_hi(v.x), bf_lo(v.y), bf_hi(v.y));
+}
+__device__ __forceinline__ float squares(const float4 v) { return fmaf(v.x, v.x, fmaf(v.y, v.y, fmaf(v.z, v.z, v.w * v.w))); }
+template <class T> __device__ __forceinline__ void store4(T* p, float a, float b, float c, float d);
+template <> __device__ __forceinline__ void store4<float>(float* p, float a, float b, float c, float d) {
+    *reinterpret_cast<float4*>(p) = make_float4(a, b, c, d);
+}
+template <> __device__ __forceinline__ void store4<bf16>(bf16* p, float a, float b, float c, float d) {
+    const __nv_bfloat162 lo = __floats2bfloat162_rn(a, b), hi = __floats2bfloat162_rn(c, d);
+    *reinterpret_cast<uint2*>(p) = make_uint2(*reinterpret_cast<const uint32_t*>(&lo), *reinterpret_cast<const uint32_t*>(&hi));
+}
+// v * r * (off + w)
+template <class T>
+__device__ __forceinline__ void store_normed(T* p, const float4 v, float r, float off, const float4 w) {
+    store4<T>(p, v.x * r * (off + w.x), v.y * r * (off + w.y), v.z * r * (off + w.z), v.w * r * (off + w.w));
+}
+
 // ---------------------------------------------------------------------------------------------------------------------
 // Embedding: x[t] = embed[token[t]] * scale, then the first layer's norm -> hn.  The norms of the sandwich block multiply
 // by woff + w: woff = 1 for one-plus weight vectors, 0 for plain ones.
@@ -80,6 +118,36 @@ __global__ void embed_norm_kernel(const int32_t* __restrict__ tokens, const T* _
     for (int c = threadIdx.x; c < D; c += blockDim.x) hn[(size_t)t * D + c] = from_f<T>(x[(size_t)t * D + c] * r * (woff + wn[c]));
 }
 
+// The same with the row in registers (D a multiple of 4, aligned rows): see add_norm_vec_kernel.  (2048 rows of 768: 6 us as against 11.)
+template <class T, int V, bool LONE>
+__global__ void __launch_bounds__(LONE ? 512 : 128) embed_norm_vec_kernel(const int32_t* __restrict__ tokens, const T* __restrict__ embed, float scale, int D, int vocab,
+                                                                          const float* __restrict__ wn, float eps, float* __restrict__ x, T* __restrict__ hn, const float woff, int rows) {
+    dep_wait();
+    dep_go();
+    using R = RowPieces<V, LONE>;
+    __shared__ float red[16];
+    const int t = R::row();
+    if (t >= rows) return;
+    int tok = tokens[t];
+    tok = tok < 0 ? 0 : (tok >= vocab ? vocab - 1 : tok);
+    const T* e = embed + (size_t)tok * D;
+    const size_t o = (size_t)t * D;
+    float4 v[V];
+    float ss = 0.0f;
+#pragma unroll
+    for (int i = 0; i < V; ++i) v[i] = R::column(i) < D ? load4(e + R::column(i)) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+#pragma unroll
+    for (int i = 0; i < V; ++i) {
+        v[i] = make_float4(v[i].x * scale, v[i].y * scale, v[i].z * scale, v[i].w * scale);
+        if (R::column(i) < D) *reinterpret_cast<float4*>(x + o + R::column(i)) = v[i];
+        ss += squares(v[i]);
+    }
+    const float r = 1.0f / sqrtf(R::sum(ss, red) / (float)D + eps);
+#pragma unroll
+    for (int i = 0; i < V; ++i)
+        if (R::column(i) < D) store_normed<T>(hn + o + R::column(i), v[i], r, woff, load4(wn + R::column(i)));
+}
+
 // RMS norm of selected rows -> T.  rows == nullptr: row r of the output is row r of the input.
 template <class T>
 __global__ void norm_rows_kernel(const float* __restrict__ x, const int32_t* __restrict__ rows, const float* __restrict__ w, float eps,
@@ -94,6 +162,28 @@ __global__ void norm_rows_kernel(const float* __restrict__ x, const int32_t* __r
     ss = block_sum(ss, red);
     const float s = 1.0f / sqrtf(ss / (float)D + eps);
     for (int c = threadIdx.x; c < D; c += blockDim.x) out[(size_t)r * D + c] = from_f<T>(xr[c] * s * (woff + w[c]));
+}
+
+template <class T, int V, bool LONE>
+__global__ void __launch_bounds__(LONE ? 512 : 128) norm_rows_vec_kernel(const float* __restrict__ x, const int32_t* __restrict__ rows, const float* __restrict__ w, float eps,
+                                                                         int D, T* __restrict__ out, const float woff, int n_rows) {
+    dep_wait();
+    dep_go();
+    using R = RowPieces<V, LONE>;
+    __shared__ float red[16];
+    const int r = R::row();
+    if (r >= n_rows) return;
+    const float* xr = x + (size_t)(rows ? rows[r] : r) * D;
+    float4 v[V];
+    float ss = 0.0f;
+#pragma unroll
+    for (int i = 0; i < V; ++i) v[i] = R::column(i) < D ? load4(xr + R::column(i)) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+#pragma unroll
+    for (int i = 0; i < V; ++i) ss += squares(v[i]);
+    const float f = 1.0f / sqrtf(R::sum(ss, red) / (float)D + eps);
+#pragma unroll
+    for (int i = 0; i < V; ++i)
+        if (R::column(i) < D) store_normed<T>(out + (size_t)r * D + R::column(i), v[i], f, woff, load4(w + R::column(i)));
 }
 
 // End of a sublayer fused with the start of the next one:
@@ -188,6 +278,87 @@ __global__ void add_norm_kernel(float* __restrict__ x, const float* __restrict__
     for (int c = threadIdx.x; c < D; c += blockDim.x) hn[o + c] = from_f<T>(row[c] * r2 * (woff + wn[c]));
 }
 
+// The same with the rows as 16-byte pieces in registers (D a multiple of 4 up to 2048, aligned rows).  What bounds it is waiting: for the rows (one round of loads),
+// then for the two sums.  Many rows: a warp per row, so that a row's sums are shuffles and an SM's rows are all in flight at once (2048 rows of 768: 7 us as against
+// 13 for a block of 128 threads per row, 4-byte loads and six barriers).  Few rows: a block per row, a piece per thread, one barrier per sum, and the weights -- no
+// kernel of a step writes them, and the step's first kernel has waited for what did -- loaded before the wait for the kernel in front (one row: 1.7 as against 4.5).
+template <class T, int V, bool LONE>
+__global__ void __launch_bounds__(LONE ? 512 : 128) add_norm_vec_kernel(float* __restrict__ x, const float* __restrict__ y, const float* __restrict__ wb, const float* __restrict__ ls,
+                                                                        const float* __restrict__ wn, float eps, int D, T* __restrict__ hn, const float woff,
+                                                                        const float* __restrict__ yb, const RoutedSum rs, const T* hin, int rows) {
+    using R = RowPieces<V, LONE>;
+    const float4 none = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    float4 early[4] = {none, none, none, none};
+    if (LONE && R::column(0) < D) {
+        early[0] = load4(ls + R::column(0));
+        early[1] = load4(wb + R::column(0));
+        if (wn) early[2] = load4(wn + R::column(0));
+        if (yb) early[3] = load4(yb + R::column(0));
+    }
+    dep_wait();
+    dep_go();
+    __shared__ float red[2][16];
+    const int t = R::row();
+    if (t >= rows) return;
+    const size_t o = (size_t)t * D;
+    float4 xv[V], yv[V];
+    float ss = 0.0f;
+#pragma unroll
+    for (int i = 0; i < V; ++i) {
+        const int c = R::column(i);
+        const bool in = c < D;
+        xv[i] = in ? load4(x + o + c) : none;
+        yv[i] = none;
+        if (!in) continue;
+        if (!rs.yp) yv[i] = load4(y + o + c);
+    }
+    if (rs.yp) {
+        for (int k = 0; k < rs.top; ++k) {
+            const int slot = rs.slot_of[(size_t)t * rs.top + k];
+            const float w = rs.sel_w ? rs.sel_w[(size_t)t * rs.top + k] : 1.0f;
+#pragma unroll
+            for (int i = 0; i < V; ++i) {
+                const int c = R::column(i);
+                if (c >= D) continue;
+                const float4 v = slot >= 0 ? load4(rs.yp + (size_t)slot * D + c) : load4(hin + o + c);
+                yv[i] = make_float4(fmaf(w, v.x, yv[i].x), fmaf(w, v.y, yv[i].y), fmaf(w, v.z, yv[i].z), fmaf(w, v.w, yv[i].w));
+            }
+        }
+    } else if (yb) {
+#pragma unroll
+        for (int i = 0; i < V; ++i) {
+            const float4 v = LONE ? early[3] : R::column(i) < D ? load4(yb + R::column(i)) : none;
+            yv[i] = make_float4(yv[i].x + v.x, yv[i].y + v.y, yv[i].z + v.z, yv[i].w + v.w);
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < V; ++i) ss += squares(yv[i]);
+    const float r = 1.0f / sqrtf(R::sum(ss, red[0]) / (float)D + eps);
+    float s2 = 0.0f;
+#pragma unroll
+    for (int i = 0; i < V; ++i) {
+        const int c = R::column(i);
+        if (c >= D) continue;
+        const float4 l = LONE ? early[0] : load4(ls + c), b = LONE ? early[1] : load4(wb + c), u = yv[i];
+        float4& v = xv[i];
+        v.x += l.x * (u.x * r * (woff + b.x));
+        v.y += l.y * (u.y * r * (woff + b.y));
+        v.z += l.z * (u.z * r * (woff + b.z));
+        v.w += l.w * (u.w * r * (woff + b.w));
+        *reinterpret_cast<float4*>(x + o + c) = v;
+        s2 += squares(v);
+    }
+    if (!wn) return;
+    const float r2 = 1.0f / sqrtf(R::sum(s2, red[1]) / (float)D + eps);
+#pragma unroll
+    for (int i = 0; i < V; ++i) {
+        const int c = R::column(i);
+        if (c < D) store_normed<T>(hn + o + c, xv[i], r2, woff, LONE ? early[2] : load4(wn + c));
+    }
+}
+constexpr int kRowPiecesMax = 2048;      // widths up to which rows stay in registers
+constexpr int kWarpRows = 512;           // rows from which a warp has a row of its own
+
 // Three sums over the block at once; every thread gets the results.  `red` holds 3 x 33 floats.
 __device__ __forceinline__ void block_sum3(float& a, float& b, float& c, float (*red)[33]) {
     a = warp_sum(a);
@@ -205,15 +376,6 @@ __device__ __forceinline__ void block_sum3(float& a, float& b, float& c, float (
     a = red[0][32];
     b = red[1][32];
     c = red[2][32];
-}
-
-template <class T> __device__ __forceinline__ void store4(T* p, float a, float b, float c, float d);
-template <> __device__ __forceinline__ void store4<float>(float* p, float a, float b, float c, float d) {
-    *reinterpret_cast<float4*>(p) = make_float4(a, b, c, d);
-}
-template <> __device__ __forceinline__ void store4<bf16>(bf16* p, float a, float b, float c, float d) {
-    const __nv_bfloat162 lo = __floats2bfloat162_rn(a, b), hi = __floats2bfloat162_rn(c, d);
-    *reinterpret_cast<uint2*>(p) = make_uint2(*reinterpret_cast<const uint32_t*>(&lo), *reinterpret_cast<const uint32_t*>(&hi));
 }
 
 // PolyNorm: out = a z/rms(z) + b z^2/rms(z^2) + c z^3/rms(z^3) + e over a token's feed-forward vector.  The three sums
@@ -1923,25 +2085,6 @@ __global__ void __launch_bounds__(delta_block_cols(DK) * delta_lanes(DK)) delta_
         }
 }
 
-// End of the recurrent mixer: each head's o divided by its root mean square, times the plain weight, times the sigmoid
-// gate, written in T.  One warp per (token, head).
-template <class T>
-__global__ void delta_out_kernel(const DeltaArgs A, const float* __restrict__ o_raw, T* __restrict__ out) {
-    dep_wait();
-    dep_go();
-    const int lane = threadIdx.x & 31;
-    const int unit = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-    if (unit >= A.n_tokens * A.H) return;
-    const int t = unit / A.H, h = unit % A.H, d = A.d, HD = A.H * d;
-    const float* o = o_raw + (size_t)t * HD + h * d;
-    const float* gate = A.proj + (size_t)t * A.n_in + 3 * HD + h * d;
-    float ss = 0.0f;
-    for (int c = lane; c < d; c += 32) ss = fmaf(o[c], o[c], ss);
-    ss = warp_sum(ss);
-    const float rs = 1.0f / sqrtf(ss / (float)d + A.eps);
-    for (int c = lane; c < d; c += 32) out[(size_t)t * HD + h * d + c] = from_f<T>(o[c] * rs * A.out_norm[h * d + c] * sigmoidf_(gate[c]));
-}
-
 // ---------------------------------------------------------------------------------------------------------------------
 // Sampling: the library's integer-weight sampler, one block per row.
 template <int PER>
@@ -2766,6 +2909,20 @@ static cudaError_t plain_launch(void (*kernel)(P...), dim3 grid, dim3 block, siz
     return pdl_launch(kernel, grid, block, smem, st, std::forward<X>(args)...);
 }
 
+// Launches the form of a row kernel for `rows` rows of D: go(V, LONE, blocks, threads).  False: the rows are not whole 16-byte pieces, or too wide.
+template <class Go>
+static bool row_pieces(int rows, int D, uintptr_t addresses, Go go) {
+    if (D % 4 != 0 || D > kRowPiecesMax || addresses % 16 != 0) return false;
+    using std::integral_constant;
+    if (rows < kWarpRows) go(integral_constant<int, 1>{}, TrueType{}, rows, (D / 4 + 31) / 32 * 32);
+    else if (D <= 768) go(integral_constant<int, 6>{}, FalseType{}, (rows + 3) / 4, 128);
+    else if (D <= 1536) go(integral_constant<int, 12>{}, FalseType{}, (rows + 3) / 4, 128);
+    else go(integral_constant<int, 16>{}, FalseType{}, (rows + 3) / 4, 128);
+    return true;
+}
+template <class... P>
+static uintptr_t addresses_of(const P*... p) { return (reinterpret_cast<uintptr_t>(p) | ...); }
+
 // y fp32 [M, N] = a [M, K] . w [N, K]^T
 template <class T>
 static cudaError_t linear(SmolLm* m, const T* a, const T* w, float* y, int M, int N, int K, cudaStream_t st);
@@ -3265,6 +3422,17 @@ static void launch_residual_norm(const ResidualArgs& A, int rows, int threads, T
 }
 
 template <class T>
+static void launch_gla_out(const GlaArgs& A, const float* o_raw, T* out, cudaStream_t st) {
+    const int units = A.n_tokens * A.H;
+    const size_t gate_at = A.gate_off >= 0 ? (size_t)A.gate_off : (size_t)2 * A.H * A.d + (size_t)A.H * A.dv;
+    // whole 16-byte pieces of every row
+    const bool vec = A.dv % 4 == 0 && A.n_in % 4 == 0 && gate_at % 4 == 0 && A.out_ld % 4 == 0 && addresses_of(A.proj, A.out_norm, o_raw) % 16 == 0 && addresses_of(out) % 8 == 0;
+    if (vec && A.dv == 64) pdl_launch(gla_out_vec_kernel<T, 16>, (units + 7) / 8, 128, 0, st, A, o_raw, out);
+    else if (vec && A.dv == 128) pdl_launch(gla_out_vec_kernel<T, 32>, (units + 3) / 4, 128, 0, st, A, o_raw, out);
+    else pdl_launch(gla_out_kernel<T>, (units + 3) / 4, 128, 0, st, A, o_raw, out);
+}
+
+template <class T>
 static int step_impl(SmolLm* m, const SmolLmStep* s, cudaStream_t st) {
     const SmolLmConfig& c = m->cfg;
     const int Tn = s->n_tokens, D = c.width;
@@ -3311,10 +3479,20 @@ static int step_impl(SmolLm* m, const SmolLmStep* s, cudaStream_t st) {
         pdl_launch(embed_prenorm_kernel<T>, Tn, nthr, 0, st, s->tokens, static_cast<const T*>(m->g.embed), c.embed_scale, D, c.vocab,
                                                      merge ? no_norm : norm_of(L0.norm1, L0.norm1_shift, L0.norm1_alpha), x, x0, hn, cat);
     } else {
-        pdl_launch(embed_norm_kernel<T>, Tn, nthr, 0, st, s->tokens, static_cast<const T*>(m->g.embed), c.embed_scale, D, c.vocab,
-                                                  m->layers[m->runs[0].layer].norm1, c.norm_eps, x, hn, woff);
+        const T* table = static_cast<const T*>(m->g.embed);
+        const float* w = m->layers[m->runs[0].layer].norm1;
+        if (!row_pieces(Tn, D, addresses_of(table, w, x, hn), [&](auto v, auto lone, int blocks, int threads) {
+                pdl_launch(embed_norm_vec_kernel<T, decltype(v)::value, decltype(lone)::value>, blocks, threads, 0, st, s->tokens, table, c.embed_scale, D, c.vocab, w, c.norm_eps, x, hn, woff, Tn);
+            }))
+            pdl_launch(embed_norm_kernel<T>, Tn, nthr, 0, st, s->tokens, table, c.embed_scale, D, c.vocab, w, c.norm_eps, x, hn, woff);
     }
     m->launches++;
+    auto add_norm = [&](const float* wb, const float* ls, const float* wn, const float* yb, const RoutedSum& rs) {
+        if (!row_pieces(Tn, D, addresses_of(x, y, wb, ls, wn, yb, hn, rs.yp), [&](auto v, auto lone, int blocks, int threads) {
+                pdl_launch(add_norm_vec_kernel<T, decltype(v)::value, decltype(lone)::value>, blocks, threads, 0, st, x, y, wb, ls, wn, c.norm_eps, D, hn, woff, yb, rs, hn, Tn);
+            }))
+            pdl_launch(add_norm_kernel<T>, Tn, nthr, D * sizeof(float), st, x, y, wb, ls, wn, c.norm_eps, D, hn, woff, yb, rs, hn);
+    };
     for (size_t n = 0; n < m->runs.size(); ++n) {
         const RunInfo& R = m->runs[n];
         const SmolLmLayer& L = m->layers[R.layer];
@@ -3491,7 +3669,7 @@ static int step_impl(SmolLm* m, const SmolLmStep* s, cudaStream_t st) {
             A.head_decay = M.head_decay; A.head_ld = 0;
             CU(launch_gla_scan_any(m, A, s->n_seqs, Tn, max_n, nullptr, m->slots, oraw, ms, parallel && Tn > kGraphMaxTokens ? kScanSpread : 0));
             A.out_ld = ld; A.out_scale = M.mix_scale;
-            pdl_launch(gla_out_kernel<T>, (Tn * M.heads + 3) / 4, 128, 0, ms, A, oraw, mix_at);
+            launch_gla_out<T>(A, oraw, mix_at, ms);
             m->launches += 3;
             return SMOL_OK;
         };
@@ -3524,7 +3702,7 @@ static int step_impl(SmolLm* m, const SmolLmStep* s, cudaStream_t st) {
             CU(launch_group_scan_any<true>(m, S, pairs, s->n_seqs, Tn, max_n, m->slots, oraw, ms));
             GlaArgs A = scan_args(M, Ri, pj);
             A.out_norm = M.out_norm; A.gate_off = ch; A.out_ld = ld; A.out_scale = M.mix_scale;
-            pdl_launch(gla_out_kernel<T>, (Tn * M.heads + 3) / 4, 128, 0, ms, A, oraw, mix_at);
+            launch_gla_out<T>(A, oraw, mix_at, ms);
             m->launches += 2;
             return SMOL_OK;
         };
@@ -3549,7 +3727,7 @@ static int step_impl(SmolLm* m, const SmolLmStep* s, cudaStream_t st) {
             GlaArgs A = scan_args(M, Ri, pj);
             A.den = den; A.den_floor = floor_at; A.den_eps = M.den_eps;
             A.out_norm = M.out_norm; A.norm_own = 1; A.gate_sigmoid = 1; A.out_ld = ld; A.out_scale = M.mix_scale;
-            pdl_launch(gla_out_kernel<T>, (Tn * M.heads + 3) / 4, 128, 0, ms, A, oraw, mix_at);
+            launch_gla_out<T>(A, oraw, mix_at, ms);
             m->launches += 2;
             return SMOL_OK;
         };
@@ -3800,7 +3978,7 @@ static int step_impl(SmolLm* m, const SmolLmStep* s, cudaStream_t st) {
                 pdl_launch(gla_prep_kernel<kDecayTokens>, dim3((Tn + kDecayTokens - 1) / kDecayTokens, slices), 128, kDecayTokens * L.rank * sizeof(float), st, A, dec);
             else pdl_launch(gla_prep_kernel<1>, dim3(Tn, slices), 128, L.rank * sizeof(float), st, A, dec);
             CU(launch_gla_scan_any(m, A, s->n_seqs, Tn, max_n, dec, m->slots, oraw, st));
-            pdl_launch(gla_out_kernel<T>, (Tn * L.heads + 3) / 4, 128, 0, st, A, oraw, mix);
+            launch_gla_out<T>(A, oraw, mix, st);
             m->launches += 3;
             mix_cols = L.heads * L.vdim;
         } else {
@@ -3835,7 +4013,9 @@ static int step_impl(SmolLm* m, const SmolLmStep* s, cudaStream_t st) {
             else if (L.dim <= 128) e = launch_scan<128>(A, s->n_seqs, dec, uk, auk, m->slots, oraw, st);
             else e = launch_scan<256>(A, s->n_seqs, dec, uk, auk, m->slots, oraw, st);
             CU(e);
-            pdl_launch(delta_out_kernel<T>, (Tn * L.heads + 3) / 4, 128, 0, st, A, oraw, mix);
+            GlaArgs O = scan_args(L, R, proj);
+            O.dv = L.dim; O.out_norm = L.out_norm; O.norm_own = 1; O.gate_off = 3LL * L.heads * L.dim; O.gate_sigmoid = 1; O.out_ld = L.heads * L.dim;
+            launch_gla_out<T>(O, oraw, mix, st);
             m->launches += 3;
             mix_cols = L.heads * L.dim;
         }
@@ -3922,13 +4102,13 @@ static int step_impl(SmolLm* m, const SmolLmStep* s, cudaStream_t st) {
                 m->launches += 1;
             }
         } else if (L.mlp != SMOL_LM_MLP_NONE) {
-            pdl_launch(add_norm_kernel<T>, Tn, nthr, D * sizeof(float), st, x, y, L.norm1b, L.ls1, L.norm2, c.norm_eps, D, hn, woff, L.out_bias, no_sum, hn);
+            add_norm(L.norm1b, L.ls1, L.norm2, L.out_bias, no_sum);
             const int rc = feed_forward(st);
             if (rc != SMOL_OK) return rc;
-            pdl_launch(add_norm_kernel<T>, Tn, nthr, D * sizeof(float), st, x, y, L.norm2b, L.ls2, next_norm1, c.norm_eps, D, hn, woff, nullptr, routed, hn);
+            add_norm(L.norm2b, L.ls2, next_norm1, nullptr, routed);
             m->launches += 2;
         } else {
-            pdl_launch(add_norm_kernel<T>, Tn, nthr, D * sizeof(float), st, x, y, L.norm1b, L.ls1, next_norm1, c.norm_eps, D, hn, woff, L.out_bias, no_sum, hn);
+            add_norm(L.norm1b, L.ls1, next_norm1, L.out_bias, no_sum);
             m->launches += 1;
         }
         if (s->trace && !prenorm && !parallel && !outnorm) CU(cudaMemcpyAsync(s->trace + n * (size_t)Tn * D, x, (size_t)Tn * D * 4, cudaMemcpyDeviceToDevice, st));
@@ -3937,7 +4117,10 @@ static int step_impl(SmolLm* m, const SmolLmStep* s, cudaStream_t st) {
         if (postnorm) pdl_launch(post_norm_kernel<T>, s->n_want, nthr, 2 * D * sizeof(float), st, x, nullptr, c.logit_scale, m->g.final_norm, c.norm_eps, D, nullptr, 0, 0,
                                                                                       nullptr, s->want_rows, hw, RoutedSum{nullptr, nullptr, nullptr, 0});
         else if (prenorm || parallel || outnorm) pdl_launch(prenorm_rows_kernel<T>, s->n_want, nthr, 0, st, x, s->want_rows, norm_of(m->g.final_norm, m->g.final_norm_shift, m->g.final_norm_alpha), D, hw);
-        else pdl_launch(norm_rows_kernel<T>, s->n_want, nthr, 0, st, x, s->want_rows, m->g.final_norm, c.norm_eps, D, hw, woff);
+        else if (!row_pieces(s->n_want, D, addresses_of(x, m->g.final_norm, hw), [&](auto v, auto lone, int blocks, int threads) {
+                     pdl_launch(norm_rows_vec_kernel<T, decltype(v)::value, decltype(lone)::value>, blocks, threads, 0, st, x, s->want_rows, m->g.final_norm, c.norm_eps, D, hw, woff, s->n_want);
+                 }))
+            pdl_launch(norm_rows_kernel<T>, s->n_want, nthr, 0, st, x, s->want_rows, m->g.final_norm, c.norm_eps, D, hw, woff);
         m->launches++;
         CU(linear<T>(m, hw, static_cast<const T*>(m->g.head), s->logits, s->n_want, c.vocab, D, st));
         const float lscale = postnorm ? 1.0f : c.logit_scale;      // the post-norm block scales inside the final norm

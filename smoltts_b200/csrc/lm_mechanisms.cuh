@@ -578,6 +578,31 @@ __global__ void gla_out_kernel(const GlaArgs A, const float* __restrict__ o_raw,
     for (int c = lane; c < dv; c += 32) out[(size_t)t * A.out_ld + h * dv + c] = finish(o[c] * inv, rs, weight ? weight[c] : 1.0f, gate[c]);
 }
 
+// The same for rows of exactly 4 L columns, a piece per lane, L lanes per unit: 24 000 units of 64 columns 5.3 us as against 10.2 (four units of 4-byte loads per warp: 11.7).
+template <class T, int L>
+__global__ void __launch_bounds__(128) gla_out_vec_kernel(const GlaArgs A, const float* __restrict__ o_raw, T* __restrict__ out) {
+    dep_wait();
+    dep_go();
+    constexpr int DV = 4 * L;
+    const int unit = (blockIdx.x * blockDim.x + threadIdx.x) / L, q = threadIdx.x % L;
+    if (unit >= A.n_tokens * A.H) return;
+    const int t = unit / A.H, h = unit - t * A.H;
+    const size_t gate_at = A.gate_off >= 0 ? (size_t)A.gate_off : (size_t)2 * A.H * A.d + (size_t)A.H * DV;
+    float4 v = load4(o_raw + (size_t)unit * DV + 4 * q);
+    const float4 g = load4(A.proj + (size_t)t * A.n_in + gate_at + h * DV + 4 * q);
+    const float4 w = A.out_norm ? load4(A.out_norm + (A.norm_own ? h * DV : 0) + 4 * q) : make_float4(1.0f, 1.0f, 1.0f, 1.0f);
+    if (A.den) {
+        const float inv = 1.0f / (fmaxf(fabsf(A.den[unit]), A.den_floor[unit]) + A.den_eps);
+        v = make_float4(v.x * inv, v.y * inv, v.z * inv, v.w * inv);
+    }
+    float ss = squares(v);
+#pragma unroll
+    for (int x = L / 2; x > 0; x >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, x);
+    const float rs = 1.0f / sqrtf(ss / (float)DV + A.eps);
+    auto finish = [&](float x, float y, float z) { return x * rs * y * (A.gate_sigmoid ? sigmoidf_(z) : silu_(z)) * A.out_scale; };
+    store4<T>(out + (size_t)t * A.out_ld + h * DV + 4 * q, finish(v.x, w.x, g.x), finish(v.y, w.y, g.y), finish(v.z, w.z, g.z), finish(v.w, w.w, g.w));
+}
+
 // ---------------------------------------------------------------------------------------------------------------------
 // Short causal convolution over a sequence's positions: channel c of a token is silu(b[c] + sum_k w[c][k] * input at k - (taps - 1)
 // positions from it), zeros before position 0; the inputs are columns of the fused projection.  The last taps - 1 inputs live

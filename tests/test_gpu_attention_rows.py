@@ -58,7 +58,7 @@ def test_rows_take_nothing_from_keys_they_do_not_see(name):
 
     def logits(row):
         seq = model.open_sequence()
-        out = model.forward([(seq, row, list(range(len(row))))]).clone()
+        out = model.forward([(seq, row, list(range(len(row))))])[:, :BAD].clone()      # (a tied head has that token's column)
         model.close_sequence(seq)
         return out
 

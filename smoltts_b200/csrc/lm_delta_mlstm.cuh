@@ -111,8 +111,6 @@ __device__ __forceinline__ void group_scan_stage(const GroupScanArgs& A, float* 
 
 template <int DK, bool DELTA>
 __global__ void __launch_bounds__(gla_block_cols(DK) * gla_lanes(DK)) group_scan_kernel(const GroupScanArgs A, float* state_pool, float* __restrict__ o_raw) {
-    dep_wait();
-    dep_go();
     constexpr int L = gla_lanes(DK), CB = gla_block_cols(DK), RV = DK / L / 4, CH = group_scan_chunk(DK), PL = CH * DK;
     constexpr int kBuf = group_scan_buf_floats(DK), GS = kScanGroup;
     static_assert(L >= GS && kBuf % 4 == 0, "a lane per token of a group stores its result; 16-byte buffers");
@@ -126,6 +124,7 @@ __global__ void __launch_bounds__(gla_block_cols(DK) * gla_lanes(DK)) group_scan
     const int slot = A.seq_slot[seq];
     if (slot < 0 || slot >= A.n_slots) {
         if (threadIdx.x == 0) atomicExch(A.err, 2);
+        dep_wait();
         return;
     }
     // 16-byte copies need every source to start on a 16-byte boundary: d, dv and the row lengths multiples of 4
@@ -137,9 +136,6 @@ __global__ void __launch_bounds__(gla_block_cols(DK) * gla_lanes(DK)) group_scan
         for (int i = threadIdx.x; i < 2 * CH; i += blockDim.x) sh[(i / CH) * kBuf + 2 * PL + (i % CH) * CB + dv - j0] = 1.0f;
     }
     __syncthreads();
-    if (vec) group_scan_stage<DK, 4>(A, sh, t0, min(CH, t1 - t0), h, j0, nc);
-    else group_scan_stage<DK, 1>(A, sh, t0, min(CH, t1 - t0), h, j0, nc);
-    cp_async_commit();
     // element i of this thread's column: st[i * st_ld]
     const bool unit = j == dv && dvs > dv;
     float* st = state_pool + (size_t)slot * A.slot_floats + (unit ? A.unit_off + (size_t)h * d : A.state_off + (size_t)h * d * dv + j);
@@ -153,6 +149,11 @@ __global__ void __launch_bounds__(gla_block_cols(DK) * gla_lanes(DK)) group_scan
             const int i = 4 * (e * L + q) + x;
             S[e][x] = (!fresh && i < d && j < dvs) ? st[(size_t)i * st_ld] : 0.0f;
         }
+    dep_wait();
+    dep_go();
+    if (vec) group_scan_stage<DK, 4>(A, sh, t0, min(CH, t1 - t0), h, j0, nc);
+    else group_scan_stage<DK, 1>(A, sh, t0, min(CH, t1 - t0), h, j0, nc);
+    cp_async_commit();
     if (A.conv.taps > 1)
         for (int c = part * blockDim.x + threadIdx.x; c < A.conv.ch; c += A.H * NS * blockDim.x) conv_state_update(A.conv, state_pool, seq, c);
     // this lane's output: token q of a group (q < GS)
@@ -276,17 +277,18 @@ struct GatedDeltaArgs {
 constexpr int kGatedDeltaCols = 64;
 __global__ void __launch_bounds__(128) gated_delta_prep_kernel(const GatedDeltaArgs A, const float* __restrict__ slots, float* __restrict__ qkv,
                                                                float* __restrict__ head, float* __restrict__ pairs) {
-    dep_wait();
-    dep_go();
     const int t = blockIdx.x, warp = blockIdx.y * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
     const ConvIo& C = A.conv;
     const int s = A.tok_seq[t], r = t - C.seq_start[s], pos0 = C.seq_pos0[s], slot = C.seq_slot[s];
     if (slot < 0 || slot >= C.n_slots) {
         if (threadIdx.x == 0) atomicExch(A.err, 2);
+        dep_wait();
         return;
     }
     const float* before = slots + (size_t)slot * C.slot_floats + C.conv_off;
     const int gd = A.G * A.d;
+    dep_wait();
+    dep_go();
     float* row = qkv + (size_t)t * C.ch;
     for (int h = threadIdx.x; blockIdx.y == 0 && h < A.H; h += blockDim.x) {
         const float* p = A.proj + (size_t)t * A.n_in + C.ch + A.H * A.dv + h;

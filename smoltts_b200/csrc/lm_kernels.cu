@@ -874,13 +874,15 @@ __device__ __forceinline__ float attn_score(const AttnArgs& A, float dot, int di
 // q_norm / k_norm == nullptr: no norm.
 template <class T>
 __global__ void attn_prep_kernel(const AttnArgs A, T* __restrict__ qbuf, T* __restrict__ pool) {
-    dep_wait();
-    dep_go();
     const int lane = threadIdx.x & 31;
     const int unit = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     const int HQ = A.H * A.maps, GK = A.G * A.maps, slots = HQ + (A.own_kv ? GK + A.G : 0);
-    if (unit >= A.n_tokens * slots) return;
-    const int t = unit / slots, s = unit % slots;
+    if (unit >= A.n_tokens * slots) { dep_wait(); return; }
+    const int t = unit / slots, s = unit % slots, pos = A.tok_pos[t];
+    const int pg = pos / A.page_size, in_pg = pos % A.page_size;
+    const int page = s >= HQ && pg < A.max_pages ? A.block_table[(size_t)A.tok_seq[t] * A.max_pages + pg] : -1;
+    dep_wait();
+    dep_go();
     const float* row = A.proj + (size_t)t * A.n_in;
     if (s < HQ) {
         const float* q = row + s * A.d;
@@ -888,14 +890,11 @@ __global__ void attn_prep_kernel(const AttnArgs A, T* __restrict__ qbuf, T* __re
         float ss = 0.0f;
         for (int c = lane; c < A.d; c += 32) { const float v = q[c] + (qb ? qb[c] : 0.0f); ss += v * v; }
         ss = warp_sum(ss);
-        const float r = (A.q_norm ? 1.0f / sqrtf(ss / (float)A.d + A.eps) : 1.0f) * attn_temperature(A, A.tok_pos[t]);
+        const float r = (A.q_norm ? 1.0f / sqrtf(ss / (float)A.d + A.eps) : 1.0f) * attn_temperature(A, pos);
         for (int c = lane; c < A.d; c += 32)
             qbuf[((size_t)t * HQ + s) * A.d + c] = from_f<T>((q[c] + (qb ? qb[c] : 0.0f)) * r * (A.q_norm ? A.q_norm[c] : 1.0f));
         return;
     }
-    const int pos = A.tok_pos[t];
-    const int pg = pos / A.page_size, in_pg = pos % A.page_size;
-    int page = pg < A.max_pages ? A.block_table[(size_t)A.tok_seq[t] * A.max_pages + pg] : -1;
     if (page < 0 || page >= A.n_pages) {
         if (lane == 0) atomicExch(A.err, 1);
         return;
@@ -920,6 +919,42 @@ __global__ void attn_prep_kernel(const AttnArgs A, T* __restrict__ qbuf, T* __re
     }
 }
 
+// The same for heads of up to 4 L elements whose rows are whole 16-byte pieces: a piece per lane, L lanes per unit.  Nearly all of it is waiting for loads: 2048 tokens of 20
+// heads of 64 PLACEHOLDER us as against 13.8 with 4-byte loads and a warp per unit (24 with four units per warp).
+template <class T, int L>
+__global__ void __launch_bounds__(128) attn_prep_vec_kernel(const AttnArgs A, T* __restrict__ qbuf, T* __restrict__ pool) {
+    const int unit = (int)(blockIdx.x * blockDim.x + threadIdx.x) / L, c = 4 * (threadIdx.x % L);
+    const int HQ = A.H * A.maps, GK = A.G * A.maps, slots = HQ + (A.own_kv ? GK + A.G : 0);
+    const bool live = unit < A.n_tokens * slots;
+    const int t = live ? unit / slots : 0, s = unit - t * slots, pos = A.tok_pos[t];
+    const int pg = pos / A.page_size, in_pg = pos - pg * A.page_size;
+    const int page = s >= HQ && pg < A.max_pages ? A.block_table[(size_t)A.tok_seq[t] * A.max_pages + pg] : -1;
+    const bool key = s >= HQ && s < HQ + GK, in = live && c < (s < HQ + GK ? A.d : A.dv);
+    const int at = (s < HQ + GK ? s * A.d : (HQ + GK) * A.d + (s - HQ - GK) * A.dv) + c;
+    const float* norm = s < HQ ? A.q_norm : key ? A.k_norm : nullptr;
+    const float4 none = make_float4(0.0f, 0.0f, 0.0f, 0.0f), w = in && norm ? load4(norm + c) : make_float4(1.0f, 1.0f, 1.0f, 1.0f), b = in && A.bias ? load4(A.bias + at) : none;
+    dep_wait();
+    dep_go();
+    float4 v = in ? load4(A.proj + (size_t)t * A.n_in + at) : none;
+    v = make_float4(v.x + b.x, v.y + b.y, v.z + b.z, v.w + b.w);
+    float ss = squares(v);
+#pragma unroll
+    for (int x = L / 2; x > 0; x >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, x);
+    float r = norm ? 1.0f / sqrtf(ss / (float)A.d + A.eps) : 1.0f;
+    T* to;
+    if (s < HQ) {
+        r *= attn_temperature(A, pos);
+        to = qbuf + ((size_t)t * HQ + s) * A.d + c;
+    } else {
+        if (live && (page < 0 || page >= A.n_pages)) {
+            if (c == 0) atomicExch(A.err, 1);
+            return;
+        }
+        to = pool + (size_t)page * A.page_elems + (key ? A.k_off + ((size_t)(s - HQ) * A.page_size + in_pg) * A.d : A.v_off + ((size_t)(s - HQ - GK) * A.page_size + in_pg) * A.dv) + c;
+    }
+    if (in) store4<T>(to, v.x * r * w.x, v.y * r * w.y, v.z * r * w.z, v.w * r * w.w);
+}
+
 // The same preparation with query and key norms over the WHOLE projection: one root mean square for all query heads of a
 // token (weights q_norm [H*d]) and one for all key heads (k_norm [G*d]).  One block per token.  Loads go out kPrepBatch
 // at a time before their first use: a lone token (decoding) waits for memory a few times, not once per element.
@@ -929,8 +964,6 @@ constexpr int kMaxRotPairs = 256;
 
 template <class T, bool ROT>
 __global__ void __launch_bounds__(256) attn_prep_whole_kernel(const AttnArgs A, T* __restrict__ qbuf, T* __restrict__ pool) {
-    dep_wait();
-    dep_go();
     __shared__ float red[2][33];
     __shared__ float turn[2][ROT ? kMaxRotPairs : 1];
     const int t = blockIdx.x, nq = A.H * A.d, nk = A.G * A.d, nv = A.G * A.dv;
@@ -961,6 +994,8 @@ __global__ void __launch_bounds__(256) attn_prep_whole_kernel(const AttnArgs A, 
             turn[0][i] = cs * A.rot_mult;
             turn[1][i] = sn * A.rot_mult;
         }
+    dep_wait();
+    dep_go();
     float sq = sum_sq(0, nq), sk = sum_sq(nq, nk);
     sq = warp_sum(sq);
     sk = warp_sum(sk);
@@ -1329,9 +1364,7 @@ __global__ void __launch_bounds__(kRowsWarps * 32) attn_rows_kernel(const AttnAr
 }
 
 template <class T, int MAXV, int KPL>
-__global__ void __launch_bounds__(256) attn_split_kernel(const AttnArgs A, const T* __restrict__ qbuf, const T* __restrict__ pool) {
-    dep_wait();
-    dep_go();
+__global__ void __launch_bounds__(256) attn_split_kernel(const AttnArgs A, const T* __restrict__ qbuf, const T* pool) {
     // One block per (row, key/value head x group of up to 8 of its query rows, key range); one warp per query row (a query
     // head, or one of its maps: the block then stages every map's keys beside the values they share).
     // 32 * KPL keys and values at a time (KPL keys per lane) are staged in shared memory (rows padded by 16 bytes: conflict-free
@@ -1340,12 +1373,12 @@ __global__ void __launch_bounds__(256) attn_split_kernel(const AttnArgs A, const
     constexpr int kPad = 16 / (int)sizeof(T), KEYS = 32 * KPL;
     const int s = blockIdx.x / kShortSeq, r = blockIdx.x % kShortSeq;
     const int t0 = A.seq_start[s], n = A.seq_start[s + 1] - t0;
-    if (n > kShortSeq || r >= n) return;
+    if (n > kShortSeq || r >= n) { dep_wait(); return; }
     const int t = t0 + r, pos = A.tok_pos[t];
     // with a window the ranges are counted from the one that holds the row's first visible key
     const int j_first = attn_first_key(A, pos);
     const int range = j_first / A.split_len + blockIdx.z;
-    if (range * A.split_len > pos) return;
+    if (range * A.split_len > pos) { dep_wait(); return; }
     const int j_lo = max(range * A.split_len, j_first);
     const int j_hi = min(pos, (range + 1) * A.split_len - 1);
     const int Gq = A.H / A.G * A.maps, nwarp = blockDim.x >> 5;
@@ -1360,7 +1393,6 @@ __global__ void __launch_bounds__(256) attn_split_kernel(const AttnArgs A, const
     T* Ks = reinterpret_cast<T*>(sm_raw + (((size_t)nwarp * (A.d + KEYS) * 4 + 15) / 16) * 16);
     T* Vs = A.v_in_k ? Ks : Ks + KEYS * ldk * A.maps;
     const int32_t* bt = A.block_table + (size_t)s * A.max_pages;
-    for (int c = lane; c < A.d; c += 32) qs[c] = to_f<T>(qbuf[((size_t)t * A.H * A.maps + h) * A.d + c]);
     const float r1 = A.r1 ? A.r1[head] : 0.0f, r2 = A.r1 ? A.r2[head] : 0.0f, slope = A.slope ? A.slope[head] : 0.0f;
     float m = -INFINITY, l = 0.0f;
     float o[MAXV];                       // columns 2 lane + 64 (e / 2) + e % 2
@@ -1370,9 +1402,8 @@ __global__ void __launch_bounds__(256) attn_split_kernel(const AttnArgs A, const
     const bool kvec = (A.d * sizeof(T)) % 16 == 0 && (A.k_ld * sizeof(T)) % 16 == 0 && (A.k_off * sizeof(T)) % 16 == 0;
     const bool vvec = (A.dv * sizeof(T)) % 16 == 0 && (A.v_ld * sizeof(T)) % 16 == 0 && (A.v_off * sizeof(T)) % 16 == 0;
     const int kchunk1 = kvec ? A.d / kPad : A.d, kchunks = kchunk1 * A.maps, vchunks = A.v_in_k ? 0 : (vvec ? A.dv / kPad : A.dv);
-    for (int j0 = j_lo; j0 <= j_hi; j0 += KEYS) {
-        const int cnt = min(KEYS, j_hi - j0 + 1);
-        __syncthreads();
+    // rows [from, to) of the round that starts at j0, on their way
+    auto stage = [&](int j0, int from, int to) {
         // Where the round's rows are cached: lane r looks rows r, r + 32 up.  Then a warp per row, its lanes side by side over the
         // row's pieces (a lane keeps its piece over the rows, so that nothing is divided inside the loop).
         int page[KPL], place[KPL];
@@ -1392,7 +1423,7 @@ __global__ void __launch_bounds__(256) attn_split_kernel(const AttnArgs A, const
 #pragma unroll
             for (int x = 0; x < KPL; ++x)
 #pragma unroll 4
-                for (int r = warp; r < min(32, cnt - 32 * x); r += nwarp) {
+                for (int r = warp + (max(0, from - 32 * x) + nwarp - 1 - warp) / nwarp * nwarp; r < min(32, to - 32 * x); r += nwarp) {
                     const int pg = __shfl_sync(0xffffffffu, page[x], r), in_pg = __shfl_sync(0xffffffffu, place[x], r);
                     const T* src = src0 + (size_t)pg * A.page_elems + (size_t)in_pg * ld;
                     T* dst = dst0 + (r + 32 * x) * dst_ld;
@@ -1401,6 +1432,17 @@ __global__ void __launch_bounds__(256) attn_split_kernel(const AttnArgs A, const
                     else *dst = *src;
                 }
         }
+    };
+    // The first round's rows of earlier steps do not wait for the kernel in front, which caches this step's.
+    const int old = min(max(A.tok_pos[t0] - j_lo, 0), min(KEYS, j_hi - j_lo + 1));
+    stage(j_lo, 0, old);
+    dep_wait();
+    dep_go();
+    for (int c = lane; c < A.d; c += 32) qs[c] = to_f<T>(qbuf[((size_t)t * A.H * A.maps + h) * A.d + c]);
+    for (int j0 = j_lo; j0 <= j_hi; j0 += KEYS) {
+        const int cnt = min(KEYS, j_hi - j0 + 1);
+        if (j0 > j_lo) __syncthreads();
+        if (j0 > j_lo || old < cnt) stage(j0, j0 > j_lo ? 0 : old, cnt);
         cp_async_commit_group();
         cp_async_wait_group<0>();
         __syncthreads();
@@ -1461,20 +1503,20 @@ __global__ void __launch_bounds__(256) attn_split_kernel(const AttnArgs A, const
 constexpr int kMergeWarps = 8;      // per map
 template <class T, int MAXV, int MAPS>
 __global__ void __launch_bounds__(kMergeWarps * MAPS * 32) attn_merge_kernel(const AttnArgs A, T* __restrict__ out) {
-    dep_wait();
-    dep_go();
     constexpr int PER = kMergeWarps, ALL = PER * MAPS;   // warps per map, of the block
     extern __shared__ float share[];                    // [ALL][dv], then [ALL] denominators
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int x = blockIdx.x / A.H, h = blockIdx.x % A.H;
     const int s = x / kShortSeq, r = x % kShortSeq;
     const int t0 = A.seq_start[s], n = A.seq_start[s + 1] - t0;
-    if (n > kShortSeq || r >= n) return;
+    if (n > kShortSeq || r >= n) { dep_wait(); return; }
     const int t = t0 + r, pos = A.tok_pos[t];
     const int ns = pos / A.split_len - attn_first_key(A, pos) / A.split_len + 1;
     const int map = warp / PER, w0 = warp % PER;
     const float* src = A.part + (((size_t)x * A.H + h) * MAPS + map) * A.n_splits * (A.dv + 2);
     const float sink = A.sink ? A.sink[h] : -INFINITY;
+    dep_wait();
+    dep_go();
     float M = sink;
     for (int z = lane; z < ns; z += 32) M = fmaxf(M, src[(size_t)z * (A.dv + 2)]);
     M = warp_max(M);
@@ -1851,10 +1893,19 @@ struct DeltaArgs {
 // One token per block made 2048 tokens of 12 x 64 channels and rank 64 read 400 MB of it: 84 us; eight: 27 us.
 template <int TT>
 __global__ void __launch_bounds__(128) delta_prep_kernel(const DeltaArgs A, float* __restrict__ decay, float* __restrict__ ukey, float* __restrict__ aukey) {
-    dep_wait();
-    dep_go();
     extern __shared__ float th[];   // tanh(inner) [rank][TT], then 1/|k| [TT][H]
     const int t0 = blockIdx.x * TT, nt = min(TT, A.n_tokens - t0), HD = A.H * A.d;      // blockIdx.y: a slice of blockDim.x channels
+    const int c = blockIdx.y * blockDim.x + threadIdx.x;
+    // a lone token's share of W2 comes while the kernel in front ends: its products would wait for it eight rows at a time (6 us, PLACEHOLDER now)
+    constexpr int EARLY = TT == 1 ? 64 : 1;
+    float early[EARLY];
+    const float bias = c < HD ? A.decay_bias[c] : 0.0f, rb = c < HD ? A.rate_bias[c] : 0.0f;
+    if (TT == 1) {
+#pragma unroll
+        for (int r = 0; r < EARLY; ++r) early[r] = r < A.rank && c < HD ? A.decay_w2[(size_t)r * HD + c] : 0.0f;
+    }
+    dep_wait();
+    dep_go();
     float* inv = th + A.rank * TT;
     for (int i = threadIdx.x; i < A.rank * TT; i += blockDim.x) {
         const int tt = i / A.rank, r = i - tt * A.rank;
@@ -1873,19 +1924,21 @@ __global__ void __launch_bounds__(128) delta_prep_kernel(const DeltaArgs A, floa
         if (lane == 0) inv[tt * A.H + h] = 1.0f / sqrtf(ss + A.unit_eps);
     }
     __syncthreads();
-    const int c = c_lo + threadIdx.x;
     if (c >= c_hi) return;
     float lo[TT];
-    const float bias = A.decay_bias[c];
 #pragma unroll
     for (int tt = 0; tt < TT; ++tt) lo[tt] = bias;
+    if (TT == 1) {
+#pragma unroll
+        for (int r = 0; r < EARLY; ++r)
+            if (r < A.rank) lo[0] = fmaf(early[r], th[r], lo[0]);
+    }
 #pragma unroll 8
-    for (int r = 0; r < A.rank; ++r) {
+    for (int r = TT == 1 ? EARLY : 0; r < A.rank; ++r) {
         const float wv = A.decay_w2[(size_t)r * HD + c];
 #pragma unroll
         for (int tt = 0; tt < TT; ++tt) lo[tt] = fmaf(wv, th[r * TT + tt], lo[tt]);
     }
-    const float rb = A.rate_bias[c];
 #pragma unroll
     for (int tt = 0; tt < TT; ++tt)
         if (tt < nt) {
@@ -1977,8 +2030,6 @@ __global__ void __launch_bounds__(delta_block_cols(DK) * delta_lanes(DK)) delta_
                                                                                            const float* __restrict__ ukey,
                                                                                            const float* __restrict__ aukey,
                                                                                            float* __restrict__ state_pool, float* __restrict__ o_raw) {
-    dep_wait();
-    dep_go();
     constexpr int L = delta_lanes(DK), CB = delta_block_cols(DK), NS = DK / CB, RV = DK / L / 4, PL = kDeltaChunk * DK;
     constexpr int kBuf = delta_buf_floats(DK);
     static_assert(DK % (4 * L) == 0, "every lane owns whole 16-byte pieces");
@@ -1987,21 +2038,19 @@ __global__ void __launch_bounds__(delta_block_cols(DK) * delta_lanes(DK)) delta_
     const int group = blockIdx.x % NS, sh_id = blockIdx.x / NS;
     const int seq = sh_id / A.H, h = sh_id % A.H;
     const int j0 = group * CB;
-    if (j0 >= d) return;                          // a group of padded columns only
+    if (j0 >= d) { dep_wait(); return; }          // a group of padded columns only
     const int nc = min(CB, d - j0);
     const int col = threadIdx.x / L, q = threadIdx.x % L, j = j0 + col;
     const int t0 = A.seq_start[seq], t1 = A.seq_start[seq + 1];
     const int slot = A.seq_slot[seq];
     if (slot < 0 || slot >= A.n_slots) {
         if (threadIdx.x == 0) atomicExch(A.err, 2);
+        dep_wait();
         return;
     }
     const bool vec = (d % 4 == 0) && (A.n_in % 4 == 0);
     for (int i = threadIdx.x; i < 2 * kBuf; i += blockDim.x) sh[i] = 0.0f;      // padded channels and columns stay zero for good
     __syncthreads();
-    if (vec) delta_stage<DK, 4>(A, sh, t0, min(kDeltaChunk, t1 - t0), h, j0, nc, decay, ukey, aukey);
-    else delta_stage<DK, 1>(A, sh, t0, min(kDeltaChunk, t1 - t0), h, j0, nc, decay, ukey, aukey);
-    cp_async_commit();
     float* st = state_pool + (size_t)slot * A.slot_floats + A.state_off + (size_t)h * d * d;
     float S[RV][4];
     const bool fresh = A.seq_pos0[seq] == 0;
@@ -2012,6 +2061,11 @@ __global__ void __launch_bounds__(delta_block_cols(DK) * delta_lanes(DK)) delta_
             const int i = 4 * (e * L + q) + x;
             S[e][x] = (!fresh && i < d && j < d) ? st[(size_t)i * d + j] : 0.0f;
         }
+    dep_wait();
+    dep_go();
+    if (vec) delta_stage<DK, 4>(A, sh, t0, min(kDeltaChunk, t1 - t0), h, j0, nc, decay, ukey, aukey);
+    else delta_stage<DK, 1>(A, sh, t0, min(kDeltaChunk, t1 - t0), h, j0, nc, decay, ukey, aukey);
+    cp_async_commit();
     float po = 0.0f;                              // this lane's share of the previous token's o
     int cur = 0;
     for (int c0 = t0; c0 < t1; c0 += kDeltaChunk, cur ^= 1) {
@@ -2878,6 +2932,10 @@ __global__ void __launch_bounds__(WARPS * 32) gemm_polynorm_kernel(const float* 
 // the kernel before it drains, instead of after.  What bounds a decoding step is its chain of some hundred dependent kernels of two to ten
 // microseconds: 10 layers of width 768, one token against 2048 cached ones, 4 steps 1780 us -> 1615; 5 sequences of 700 through 4 layers of
 // width 1536, 1024 -> 940.  A launch right after a wait for another stream's event goes out plainly.
+// What no kernel of the step writes -- weights, the step's index arrays, cached rows of earlier steps, slots' states that only the kernel itself writes -- is read before
+// dep_wait(): a kernel's blocks start when every block of the one in front has passed its own dep_wait(), so all before that one has completed and is visible.  (The
+// step's first kernel reads nothing before it: in front of it may be anything.  And no block leaves without it: a kernel of blocks that all left at once would be
+// complete before the one in front of it.)
 static thread_local bool t_plain_next = false;
 static cudaError_t wait_event(cudaStream_t st, cudaEvent_t e) {
     t_plain_next = true;
@@ -3536,7 +3594,12 @@ static int step_impl(SmolLm* m, const SmolLmStep* s, cudaStream_t st) {
                 else pdl_launch(attn_prep_whole_kernel<T, false>, Tn, threads, 0, ms, A, qbuf, pool);
             } else {
                 const int units = Tn * (M.heads * A.maps + (A.own_kv ? M.kv_heads * (A.maps + 1) : 0));
-                pdl_launch(attn_prep_kernel<T>, (units + 3) / 4, 128, 0, ms, A, qbuf, pool);
+                // whole 16-byte pieces of every row read, 4-element pieces of every row written
+                const bool vec = M.dim % 4 == 0 && M.vdim % 4 == 0 && n_in % 4 == 0 && Ri.k_off % 4 == 0 && Ri.v_off % 4 == 0 && m->page_elems % 4 == 0 &&
+                                 addresses_of(pj, bias, M.q_norm, M.k_norm, qbuf, pool) % 16 == 0;
+                if (vec && std::max(M.dim, M.vdim) <= 64) pdl_launch(attn_prep_vec_kernel<T, 16>, (units + 7) / 8, 128, 0, ms, A, qbuf, pool);
+                else if (vec && std::max(M.dim, M.vdim) <= 128) pdl_launch(attn_prep_vec_kernel<T, 32>, (units + 3) / 4, 128, 0, ms, A, qbuf, pool);
+                else pdl_launch(attn_prep_kernel<T>, (units + 3) / 4, 128, 0, ms, A, qbuf, pool);
             }
             m->launches += 1;
             const bool flash = sizeof(T) == 2 && std::max(M.dim, M.vdim) <= 128;

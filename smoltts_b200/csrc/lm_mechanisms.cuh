@@ -581,16 +581,16 @@ __global__ void gla_out_kernel(const GlaArgs A, const float* __restrict__ o_raw,
 // The same for rows of exactly 4 L columns, a piece per lane, L lanes per unit: 24 000 units of 64 columns 5.3 us as against 10.2 (four units of 4-byte loads per warp: 11.7).
 template <class T, int L>
 __global__ void __launch_bounds__(128) gla_out_vec_kernel(const GlaArgs A, const float* __restrict__ o_raw, T* __restrict__ out) {
-    dep_wait();
-    dep_go();
     constexpr int DV = 4 * L;
     const int unit = (blockIdx.x * blockDim.x + threadIdx.x) / L, q = threadIdx.x % L;
-    if (unit >= A.n_tokens * A.H) return;
+    if (unit >= A.n_tokens * A.H) { dep_wait(); return; }
     const int t = unit / A.H, h = unit - t * A.H;
     const size_t gate_at = A.gate_off >= 0 ? (size_t)A.gate_off : (size_t)2 * A.H * A.d + (size_t)A.H * DV;
+    const float4 w = A.out_norm ? load4(A.out_norm + (A.norm_own ? h * DV : 0) + 4 * q) : make_float4(1.0f, 1.0f, 1.0f, 1.0f);
+    dep_wait();
+    dep_go();
     float4 v = load4(o_raw + (size_t)unit * DV + 4 * q);
     const float4 g = load4(A.proj + (size_t)t * A.n_in + gate_at + h * DV + 4 * q);
-    const float4 w = A.out_norm ? load4(A.out_norm + (A.norm_own ? h * DV : 0) + 4 * q) : make_float4(1.0f, 1.0f, 1.0f, 1.0f);
     if (A.den) {
         const float inv = 1.0f / (fmaxf(fabsf(A.den[unit]), A.den_floor[unit]) + A.den_eps);
         v = make_float4(v.x * inv, v.y * inv, v.z * inv, v.w * inv);

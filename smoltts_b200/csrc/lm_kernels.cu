@@ -920,7 +920,7 @@ __global__ void attn_prep_kernel(const AttnArgs A, T* __restrict__ qbuf, T* __re
 }
 
 // The same for heads of up to 4 L elements whose rows are whole 16-byte pieces: a piece per lane, L lanes per unit.  Nearly all of it is waiting for loads: 2048 tokens of 20
-// heads of 64 PLACEHOLDER us as against 13.8 with 4-byte loads and a warp per unit (24 with four units per warp).
+// heads of 64 6.9 us as against 13.8 with 4-byte loads and a warp per unit (24 with four units per warp).
 template <class T, int L>
 __global__ void __launch_bounds__(128) attn_prep_vec_kernel(const AttnArgs A, T* __restrict__ qbuf, T* __restrict__ pool) {
     const int unit = (int)(blockIdx.x * blockDim.x + threadIdx.x) / L, c = 4 * (threadIdx.x % L);
@@ -1363,14 +1363,17 @@ __global__ void __launch_bounds__(kRowsWarps * 32) attn_rows_kernel(const AttnAr
         if (i < mine) attn_finish<T, MAXV, MAPS>(A, t0 + r0 + warp * R + i, h, lane, sum[i], out);
 }
 
-template <class T, int MAXV, int KPL>
-__global__ void __launch_bounds__(256) attn_split_kernel(const AttnArgs A, const T* __restrict__ qbuf, const T* pool) {
+// PARTS 2: a query row has two warps, half of the round's keys each, whose states are joined at the end.  A warp's own chain of shared-memory loads and sums bounds the
+// kernel where every block has an SM to itself: one row at 2048 positions of 12 heads of 64 8.2 us, with one warp per query row 9.5; with more blocks than SMs
+// the smaller ones win (5 rows at 700, two maps of 6 heads: 16.2 against 12.4).
+template <class T, int MAXV, int KPL, int PARTS>
+__global__ void __launch_bounds__(256 * PARTS) attn_split_kernel(const AttnArgs A, const T* __restrict__ qbuf, const T* pool) {
     // One block per (row, key/value head x group of up to 8 of its query rows, key range); one warp per query row (a query
     // head, or one of its maps: the block then stages every map's keys beside the values they share).
     // 32 * KPL keys and values at a time (KPL keys per lane) are staged in shared memory (rows padded by 16 bytes: conflict-free
     // row-per-lane reads), so that no global load sits inside the softmax / value loops.
     extern __shared__ __align__(16) unsigned char sm_raw[];
-    constexpr int kPad = 16 / (int)sizeof(T), KEYS = 32 * KPL;
+    constexpr int kPad = 16 / (int)sizeof(T), KEYS = 32 * KPL, KP = KPL / PARTS, OWN = 32 * KP;      // keys of a round, of a lane, of a warp
     const int s = blockIdx.x / kShortSeq, r = blockIdx.x % kShortSeq;
     const int t0 = A.seq_start[s], n = A.seq_start[s + 1] - t0;
     if (n > kShortSeq || r >= n) { dep_wait(); return; }
@@ -1381,16 +1384,16 @@ __global__ void __launch_bounds__(256) attn_split_kernel(const AttnArgs A, const
     if (range * A.split_len > pos) { dep_wait(); return; }
     const int j_lo = max(range * A.split_len, j_first);
     const int j_hi = min(pos, (range + 1) * A.split_len - 1);
-    const int Gq = A.H / A.G * A.maps, nwarp = blockDim.x >> 5;
-    const int groups = (Gq + nwarp - 1) / nwarp;
-    const int g = blockIdx.y / groups, hq = (blockIdx.y % groups) * nwarp + (threadIdx.x >> 5);
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int Gq = A.H / A.G * A.maps, nwarp = blockDim.x >> 5, nrow = nwarp / PARTS;
+    const int groups = (Gq + nrow - 1) / nrow;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, own = warp % nrow, key0 = warp / nrow * OWN;
+    const int g = blockIdx.y / groups, hq = (blockIdx.y % groups) * nrow + own;
     const bool active = hq < Gq;
     const int h = g * Gq + (active ? hq : 0), map = h % A.maps, head = h / A.maps;      // h: query row
     const int ldk = A.v_in_k ? (A.d + kPad + 1) / 2 * 2 : A.d + kPad, ldv = A.v_in_k ? ldk : split_value_ld<T>(A.dv);
     float* qs = reinterpret_cast<float*>(sm_raw) + warp * A.d;
-    float* ps = reinterpret_cast<float*>(sm_raw) + nwarp * A.d + warp * KEYS;
-    T* Ks = reinterpret_cast<T*>(sm_raw + (((size_t)nwarp * (A.d + KEYS) * 4 + 15) / 16) * 16);
+    float* ps = reinterpret_cast<float*>(sm_raw) + nwarp * A.d + warp * OWN;
+    T* Ks = reinterpret_cast<T*>(sm_raw + (((size_t)nwarp * (A.d + OWN) * 4 + 15) / 16) * 16);
     T* Vs = A.v_in_k ? Ks : Ks + KEYS * ldk * A.maps;
     const int32_t* bt = A.block_table + (size_t)s * A.max_pages;
     const float r1 = A.r1 ? A.r1[head] : 0.0f, r2 = A.r1 ? A.r2[head] : 0.0f, slope = A.slope ? A.slope[head] : 0.0f;
@@ -1447,18 +1450,19 @@ __global__ void __launch_bounds__(256) attn_split_kernel(const AttnArgs A, const
         cp_async_wait_group<0>();
         __syncthreads();
         if (!active) continue;
-        float sc[KPL], mx = -INFINITY, pl = 0.0f;
+        if (key0 >= cnt) continue;
+        float sc[KP], mx = -INFINITY, pl = 0.0f;
 #pragma unroll
-        for (int x = 0; x < KPL; ++x) {
-            const int row = lane + 32 * x;
+        for (int x = 0; x < KP; ++x) {
+            const int row = key0 + lane + 32 * x;
             sc[x] = row < cnt ? attn_score<false>(A, key_dot<T>(qs, Ks + (map * KEYS + row) * ldk, A.d), pos - (j0 + row), r1, r2, slope) : -INFINITY;
             mx = fmaxf(mx, sc[x]);
         }
-        const float mn = fmaxf(m, warp_max(mx));          // finite: lane 0 of every round holds a valid key
+        const float mn = fmaxf(m, warp_max(mx));          // finite: lane 0 holds a valid key
         const float corr = expf(m - mn);
 #pragma unroll
-        for (int x = 0; x < KPL; ++x) {
-            const float p = lane + 32 * x < cnt ? expf(sc[x] - mn) : 0.0f;
+        for (int x = 0; x < KP; ++x) {
+            const float p = key0 + lane + 32 * x < cnt ? expf(sc[x] - mn) : 0.0f;
             ps[lane + 32 * x] = p;
             pl += p;
         }
@@ -1468,7 +1472,7 @@ __global__ void __launch_bounds__(256) attn_split_kernel(const AttnArgs A, const
 #pragma unroll
         for (int e = 0; e < MAXV; ++e) o[e] *= corr;
         auto add_value = [&](int jj) {
-            const float pj = ps[jj];
+            const float pj = ps[jj - key0];
 #pragma unroll
             for (int e = 0; e < MAXV; e += 2) {
                 const int c = 2 * lane + e * 32;
@@ -1479,13 +1483,31 @@ __global__ void __launch_bounds__(256) attn_split_kernel(const AttnArgs A, const
                 }
             }
         };
-        int jj = 0;
-        for (; jj + 8 <= cnt; jj += 8) {
+        int jj = key0;
+        const int end = min(cnt, key0 + OWN);
+        for (; jj + 8 <= end; jj += 8) {
 #pragma unroll
             for (int x = 0; x < 8; ++x) add_value(jj + x);      // the next keys' loads go out under the current products
         }
-        for (; jj < cnt; ++jj) add_value(jj);
+        for (; jj < end; ++jj) add_value(jj);
         __syncwarp();
+    }
+    if (PARTS == 2) {
+        // the second warp's state joins the first's (the first has seen a key; the second perhaps none)
+        float* other = reinterpret_cast<float*>(sm_raw) + nwarp * (A.d + OWN) + own * (MAXV * 32 + 2);      // over the staged keys
+        __syncthreads();
+        if (key0 > 0) {
+            if (lane == 0) { other[0] = m; other[1] = l; }
+#pragma unroll
+            for (int e = 0; e < MAXV; ++e) other[2 + e * 32 + lane] = o[e];
+        }
+        __syncthreads();
+        if (key0 > 0) return;
+        const float m2 = other[0], mn = fmaxf(m, m2), w1 = expf(m - mn), w2 = m2 == -INFINITY ? 0.0f : expf(m2 - mn);
+        l = l * w1 + (w2 > 0.0f ? other[1] * w2 : 0.0f);
+        m = mn;
+#pragma unroll
+        for (int e = 0; e < MAXV; ++e) o[e] = o[e] * w1 + (w2 > 0.0f ? other[2 + e * 32 + lane] * w2 : 0.0f);
     }
     if (!active) return;
     float* dst = A.part + (((size_t)blockIdx.x * A.H * A.maps + h) * A.n_splits + blockIdx.z) * (A.dv + 2);
@@ -1893,19 +1915,19 @@ struct DeltaArgs {
 // One token per block made 2048 tokens of 12 x 64 channels and rank 64 read 400 MB of it: 84 us; eight: 27 us.
 template <int TT>
 __global__ void __launch_bounds__(128) delta_prep_kernel(const DeltaArgs A, float* __restrict__ decay, float* __restrict__ ukey, float* __restrict__ aukey) {
-    extern __shared__ float th[];   // tanh(inner) [rank][TT], then 1/|k| [TT][H]
-    const int t0 = blockIdx.x * TT, nt = min(TT, A.n_tokens - t0), HD = A.H * A.d;      // blockIdx.y: a slice of blockDim.x channels
-    const int c = blockIdx.y * blockDim.x + threadIdx.x;
-    // a lone token's share of W2 comes while the kernel in front ends: its products would wait for it eight rows at a time (6 us, PLACEHOLDER now)
+    // a lone token's share of W2 comes while the kernel in front ends: its products would wait for it eight rows at a time (6 us, 3.7 now)
     constexpr int EARLY = TT == 1 ? 64 : 1;
-    float early[EARLY];
-    const float bias = c < HD ? A.decay_bias[c] : 0.0f, rb = c < HD ? A.rate_bias[c] : 0.0f;
+    float early[EARLY], early_bias = 0.0f;
     if (TT == 1) {
+        const int HD = A.H * A.d, c = blockIdx.y * blockDim.x + threadIdx.x;
+        if (c < HD) early_bias = A.decay_bias[c];
 #pragma unroll
         for (int r = 0; r < EARLY; ++r) early[r] = r < A.rank && c < HD ? A.decay_w2[(size_t)r * HD + c] : 0.0f;
     }
     dep_wait();
     dep_go();
+    extern __shared__ float th[];   // tanh(inner) [rank][TT], then 1/|k| [TT][H]
+    const int t0 = blockIdx.x * TT, nt = min(TT, A.n_tokens - t0), HD = A.H * A.d;      // blockIdx.y: a slice of blockDim.x channels
     float* inv = th + A.rank * TT;
     for (int i = threadIdx.x; i < A.rank * TT; i += blockDim.x) {
         const int tt = i / A.rank, r = i - tt * A.rank;
@@ -1924,8 +1946,10 @@ __global__ void __launch_bounds__(128) delta_prep_kernel(const DeltaArgs A, floa
         if (lane == 0) inv[tt * A.H + h] = 1.0f / sqrtf(ss + A.unit_eps);
     }
     __syncthreads();
+    const int c = c_lo + threadIdx.x;
     if (c >= c_hi) return;
     float lo[TT];
+    const float bias = TT == 1 ? early_bias : A.decay_bias[c];
 #pragma unroll
     for (int tt = 0; tt < TT; ++tt) lo[tt] = bias;
     if (TT == 1) {
@@ -1939,6 +1963,7 @@ __global__ void __launch_bounds__(128) delta_prep_kernel(const DeltaArgs A, floa
 #pragma unroll
         for (int tt = 0; tt < TT; ++tt) lo[tt] = fmaf(wv, th[r * TT + tt], lo[tt]);
     }
+    const float rb = A.rate_bias[c];
 #pragma unroll
     for (int tt = 0; tt < TT; ++tt)
         if (tt < nt) {
@@ -2714,9 +2739,10 @@ static cudaError_t set_kernel_attributes() {
     };
     rows(attn_rows_kernel<T, 8, 1, 1>); rows(attn_rows_kernel<T, 8, 2, 1>); rows(attn_rows_kernel<T, 16, 1, 1>); rows(attn_rows_kernel<T, 16, 2, 1>);
     rows(attn_rows_kernel<T, 8, 1, 4>); rows(attn_rows_kernel<T, 8, 2, 4>); rows(attn_rows_kernel<T, 16, 1, 4>); rows(attn_rows_kernel<T, 16, 2, 4>);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(attn_split_kernel<T, 8, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, kAttnSplitSmemMax);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(attn_split_kernel<T, 8, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, kAttnSplitWideSmem);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(attn_split_kernel<T, 16, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, kAttnSplitSmemMax);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(attn_split_kernel<T, 8, 1, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, kAttnSplitSmemMax);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(attn_split_kernel<T, 8, 2, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, kAttnSplitWideSmem);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(attn_split_kernel<T, 8, 2, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, kAttnSplitWideSmem);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(attn_split_kernel<T, 16, 1, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, kAttnSplitSmemMax);
     if (e == cudaSuccess) e = cudaFuncSetAttribute(sigmoid_attn_kernel<T, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize, 96 * 1024);
     if (e == cudaSuccess) e = cudaFuncSetAttribute(sigmoid_attn_kernel<T, 16>, cudaFuncAttributeMaxDynamicSharedMemorySize, 96 * 1024);
     if (e == cudaSuccess) e = cudaFuncSetAttribute(sigmoid_split_kernel<T, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSigmoidSmemMax);
@@ -3396,16 +3422,20 @@ static void launch_attention(SmolLm* m, const SmolLmStep* s, AttnArgs& A, bool f
     if (min_n <= kShortSeq && (flash || max_n <= kShortSeq)) {
         const int Gq = A.H / A.G * MAPS, nwarp = std::min(Gq, 8), groups = (Gq + nwarp - 1) / nwarp;
         const int pad = 16 / (int)sizeof(T);
-        auto smem_of = [&](int keys) {
-            return ((size_t)nwarp * (A.d + keys) * 4 + 15) / 16 * 16 + (size_t)keys * (MAPS * (A.d + pad + 1) + (A.v_in_k ? 0 : split_value_ld<T>(A.dv))) * sizeof(T);
+        // queries and weights of every warp, then the staged keys and values or, afterwards, the states to be joined
+        auto smem_of = [&](int keys, int parts) {
+            const size_t staged = (size_t)keys * (MAPS * (A.d + pad + 1) + (A.v_in_k ? 0 : split_value_ld<T>(A.dv))) * sizeof(T), joined = parts == 2 ? (size_t)nwarp * (MAXV * 32 + 2) * 4 : 0;
+            return ((size_t)nwarp * (parts * A.d + keys) * 4 + 15) / 16 * 16 + std::max(staged, joined);
         };
         dim3 grid(A.short_rows, A.G * groups, A.n_splits);
+        const bool alone = (long long)std::min(Tn, A.short_rows) * A.G * groups * A.n_splits <= m->n_sms;
         bool wide = false;
         if constexpr (MAXV == 8) {
-            wide = smem_of(64) <= (size_t)kAttnSplitWideSmem;
-            if (wide) pdl_launch(attn_split_kernel<T, MAXV, 2>, grid, nwarp * 32, smem_of(64), st, A, qbuf, pool);
+            wide = smem_of(64, 2) <= (size_t)kAttnSplitWideSmem;
+            if (wide && alone) pdl_launch(attn_split_kernel<T, MAXV, 2, 2>, grid, nwarp * 64, smem_of(64, 2), st, A, qbuf, pool);
+            else if (wide) pdl_launch(attn_split_kernel<T, MAXV, 2, 1>, grid, nwarp * 32, smem_of(64, 1), st, A, qbuf, pool);
         }
-        if (!wide) pdl_launch(attn_split_kernel<T, MAXV, 1>, grid, nwarp * 32, smem_of(32), st, A, qbuf, pool);
+        if (!wide) pdl_launch(attn_split_kernel<T, MAXV, 1, 1>, grid, nwarp * 32, smem_of(32, 1), st, A, qbuf, pool);
         pdl_launch(attn_merge_kernel<T, MAXV, MAPS>, A.short_rows * A.H, kMergeWarps * MAPS * 32, kMergeWarps * MAPS * (A.dv + 1) * sizeof(float), st, A, mix);
         m->launches += 2;
     }

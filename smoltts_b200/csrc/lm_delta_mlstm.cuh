@@ -130,7 +130,18 @@ __global__ void __launch_bounds__(gla_block_cols(DK) * gla_lanes(DK)) group_scan
     // 16-byte copies need every source to start on a 16-byte boundary: d, dv and the row lengths multiples of 4
     const bool vec = (d % 4 == 0) && (dv % 4 == 0) && (A.q_ld % 4 == 0) && (A.k_ld % 4 == 0) && (A.v_ld % 4 == 0) &&
                      ((reinterpret_cast<uintptr_t>(A.q_src) | reinterpret_cast<uintptr_t>(A.k_src) | reinterpret_cast<uintptr_t>(A.v_src)) % 16 == 0);
-    for (int i = threadIdx.x; i < 2 * kBuf; i += blockDim.x) sh[i] = 0.0f;      // padded channels and columns stay zero for good
+    // Padded channels and columns stay zero for good; without any, only the rows behind the last token of its group need to be finite (a lone token pays for
+    // 17 000 zeros: 13.4 us for 5 tokens of 12 x 128 x 128, 11.8 without).
+    if (d < DK || nc < CB || dvs > dv) {
+        for (int i = threadIdx.x; i < 2 * kBuf; i += blockDim.x) sh[i] = 0.0f;
+    } else {
+        const int n = min(CH, t1 - t0), rows = (n + GS - 1) / GS * GS - n;
+        for (int i = threadIdx.x; i < rows * DK; i += blockDim.x) sh[n * DK + i] = sh[PL + n * DK + i] = 0.0f;
+        for (int i = threadIdx.x; i < rows * CB; i += blockDim.x) sh[2 * PL + n * CB + i] = 0.0f;
+        float* sc = sh + 2 * PL + CH * CB;
+        for (int i = threadIdx.x; i < rows * kPairFloats; i += blockDim.x) sc[n * kPairFloats + i] = 0.0f;
+        for (int i = threadIdx.x; i < rows * 2; i += blockDim.x) sc[CH * kPairFloats + 2 * n + i] = 0.0f;
+    }
     if (dvs > dv && dv >= j0 && dv < j0 + CB) {                                 // ... and the unit column one
         __syncthreads();
         for (int i = threadIdx.x; i < 2 * CH; i += blockDim.x) sh[(i / CH) * kBuf + 2 * PL + (i % CH) * CB + dv - j0] = 1.0f;
@@ -275,6 +286,7 @@ struct GatedDeltaArgs {
 // their product; the others take 64 value channels each.  qkv [T][2 G d + H dv]: unit q (scaled) | unit k | v;
 // head: (decay, step) [T][H]; pairs: the token's own k.q where group_scan_kernel expects it.
 constexpr int kGatedDeltaCols = 64;
+template <bool FEW>
 __global__ void __launch_bounds__(128) gated_delta_prep_kernel(const GatedDeltaArgs A, const float* __restrict__ slots, float* __restrict__ qkv,
                                                                float* __restrict__ head, float* __restrict__ pairs) {
     const int t = blockIdx.x, warp = blockIdx.y * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
@@ -287,8 +299,45 @@ __global__ void __launch_bounds__(128) gated_delta_prep_kernel(const GatedDeltaA
     }
     const float* before = slots + (size_t)slot * C.slot_floats + C.conv_off;
     const int gd = A.G * A.d;
+    // FEW tokens, four taps: a channel's weights are one 16-byte piece, and its inputs of earlier steps are loaded before the wait, every channel of the thread at once (5
+    // tokens of 12 heads of 128 6.5 us, with the loads of a channel behind those of the one before 11.4).  That takes 93 registers, which prompts pay for in blocks
+    // per SM (2250 tokens of heads of 64: 43 us against 25).
+    constexpr int EARLY = 8;
+    const bool four = FEW && C.taps == 4 && !C.b && !C.bias && reinterpret_cast<uintptr_t>(C.w) % 16 == 0 && (warp >= A.G || A.d <= 32 * EARLY / 2);
+    float4 w4[EARLY], x4[EARLY];
+    int ch[EARLY];
+    if (four) {
+#pragma unroll
+        for (int e = 0; e < EARLY; ++e) {
+            // a key head's warp: channels of q, then of k; a value warp: its two
+            const int half = e / (EARLY / 2), c = lane + 32 * (e % (EARLY / 2));
+            ch[e] = warp < A.G ? (c < A.d ? half * gd + warp * A.d + c : -1)
+                               : (e < kGatedDeltaCols / 32 && (warp - A.G) * kGatedDeltaCols + lane + 32 * e < A.H * A.dv ? 2 * gd + (warp - A.G) * kGatedDeltaCols + lane + 32 * e : -1);
+            if (ch[e] < 0) continue;
+            w4[e] = load4(C.w + (size_t)ch[e] * 4);
+            float* x = reinterpret_cast<float*>(&x4[e]);
+#pragma unroll
+            for (int k = 0; k < 3; ++k) {
+                const int back = 3 - k;
+                x[k] = back > r && pos0 + r - back >= 0 ? before[(size_t)(3 - (back - r)) * C.ch + ch[e]] : 0.0f;
+            }
+        }
+    }
     dep_wait();
     dep_go();
+    float cv[EARLY];
+    if (four) {
+#pragma unroll
+        for (int e = 0; e < EARLY; ++e) {
+            if (ch[e] < 0) continue;
+            float* x = reinterpret_cast<float*>(&x4[e]);
+#pragma unroll
+            for (int k = 0; k < 4; ++k)
+                if (3 - k <= r) x[k] = C.src[(size_t)(t - (3 - k)) * C.ld + ch[e]];
+        }
+#pragma unroll
+        for (int e = 0; e < EARLY; ++e) cv[e] = ch[e] < 0 ? 0.0f : silu_(fmaf(w4[e].w, x4[e].w, fmaf(w4[e].z, x4[e].z, fmaf(w4[e].y, x4[e].y, w4[e].x * x4[e].x))));
+    }
     float* row = qkv + (size_t)t * C.ch;
     for (int h = threadIdx.x; blockIdx.y == 0 && h < A.H; h += blockDim.x) {
         const float* p = A.proj + (size_t)t * A.n_in + C.ch + A.H * A.dv + h;
@@ -303,7 +352,9 @@ __global__ void __launch_bounds__(128) gated_delta_prep_kernel(const GatedDeltaA
         for (int e = 0; e < R; ++e) {
             const int c = lane + 32 * e;
             q[e] = k[e] = 0.0f;
-            if (c < A.d) {
+            if (four) {
+                if (e < EARLY / 2) { q[e] = cv[e]; k[e] = cv[e + EARLY / 2]; }
+            } else if (c < A.d) {
                 q[e] = conv_channel(C, before, t, r, pos0, warp * A.d + c);
                 k[e] = conv_channel(C, before, t, r, pos0, gd + warp * A.d + c);
             }
@@ -333,7 +384,7 @@ __global__ void __launch_bounds__(128) gated_delta_prep_kernel(const GatedDeltaA
 #pragma unroll
     for (int e = 0; e < kGatedDeltaCols / 32; ++e) {
         const int c = c0 + lane + 32 * e;
-        if (c < A.H * A.dv) row[2 * gd + c] = conv_channel(C, before, t, r, pos0, 2 * gd + c);
+        if (c < A.H * A.dv) row[2 * gd + c] = four ? cv[e] : conv_channel(C, before, t, r, pos0, 2 * gd + c);
     }
 }
 

@@ -2074,8 +2074,10 @@ __global__ void __launch_bounds__(delta_block_cols(DK) * delta_lanes(DK)) delta_
         return;
     }
     const bool vec = (d % 4 == 0) && (A.n_in % 4 == 0);
-    for (int i = threadIdx.x; i < 2 * kBuf; i += blockDim.x) sh[i] = 0.0f;      // padded channels and columns stay zero for good
-    __syncthreads();
+    if (d < DK || nc < CB) {                      // padded channels and columns stay zero for good
+        for (int i = threadIdx.x; i < 2 * kBuf; i += blockDim.x) sh[i] = 0.0f;
+        __syncthreads();
+    }
     float* st = state_pool + (size_t)slot * A.slot_floats + A.state_off + (size_t)h * d * d;
     float S[RV][4];
     const bool fresh = A.seq_pos0[seq] == 0;
@@ -3787,7 +3789,8 @@ static int step_impl(SmolLm* m, const SmolLmStep* s, cudaStream_t st) {
             P.tok_seq = s->tok_seq; P.err = err;
             P.conv = ConvIo{pj, nullptr, n_in, ch, M.conv_taps, M.conv_w, nullptr, s->seq_start, s->seq_pos0, s->seq_slot, m->slot_floats, Ri.conv_off, m->n_slots};
             const int warps = M.kv_heads + (hv + kGatedDeltaCols - 1) / kGatedDeltaCols;
-            pdl_launch(gated_delta_prep_kernel, dim3(Tn, (warps + 3) / 4), 128, 0, ms, P, m->slots, conv, head, pairs);
+            if (Tn <= kGraphMaxTokens) pdl_launch(gated_delta_prep_kernel<true>, dim3(Tn, (warps + 3) / 4), 128, 0, ms, P, m->slots, conv, head, pairs);
+            else pdl_launch(gated_delta_prep_kernel<false>, dim3(Tn, (warps + 3) / 4), 128, 0, ms, P, m->slots, conv, head, pairs);
             GroupScanArgs S = group_args(M, Ri, M.kv_heads);
             S.q_src = conv; S.k_src = conv + gd; S.v_src = conv + 2 * gd;
             S.q_ld = S.k_ld = S.v_ld = ch;

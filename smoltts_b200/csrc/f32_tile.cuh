@@ -5,7 +5,8 @@
 //
 // MmaTile (the language models' float32 engine): a warp takes WM x WN outputs and multiplies with mma.sync m16n8k8 on tf32 parts: every fp32 operand is hi + lo,
 // 11 bits each and the sign of lo, made from the fragments that ldmatrix brings, and a product is lo hi + hi lo + hi hi (lo lo lies below the last place).  The
-// tensor core drops what its sum has below the last place, so a sum runs over 8 k, smallest parts first, and is added in fp32.
+// tensor core drops what its sum has below the last place, so a sum runs over 8 k, smallest parts first, and is added in fp32.  (Operands below 2^-115, whose lo is
+// denormal, keep 11 bits; the lo of an infinity is no number.)
 // What bounds it is the MMAs, 170 multiply-adds per clock and SM after the three parts, and the instructions that split operands and add sums beside them:
 // 300 x 4608 x 768 56 us (38 TFLOP/s), 1024 x 4608 x 768 137 (53); Tile, which reads 16 bytes of shared memory (four clocks of the SM) for every 16 multiply-adds, 77
 // and 201.  Without splitting and adding 3072 x 1536 x 1024 takes 142 us instead of 181.  Warps of 64 x 32 in tiles of 64 x 64 or 128 x 64: 174 there, but 20 to 40 %

@@ -442,9 +442,9 @@ static GemmIo plain_io(int K, int N) {
     return io;
 }
 
-// Matrix product, fp32, operands whose rows are whole 16-byte pieces: y[M, N] = a[M, K] . w[N, K]^T on the packed-FMA tile
+// Matrix product, fp32, operands whose rows are whole 16-byte pieces: y[M, N] = a[M, K] . w[N, K]^T on the tensor-core tile
 // (f32_tile.cuh), K shared by a cluster of CTAs along grid.x where the output has too few tiles to fill the GPU.
-// 300 rows, 768 to 4608 columns and k: 65 us a product against 331 on the form below, which stages element by element and is bound by
+// 300 rows, 768 to 4608 columns and k: 57 us a product against 331 on the form below, which stages element by element and is bound by
 // instruction issue.
 template <int BM, int BN, int WM, int WN>
 __global__ void __launch_bounds__(f32t::MmaTile<BM, BN, WM, WN>::NT) gemm_f32_tile_kernel(const float* __restrict__ a, const float* __restrict__ w,
@@ -1988,7 +1988,7 @@ constexpr int kDecayMinTokens = 128;     // fewer: a token per block (more block
 // Everything a token needs (r, k, u, a u, w over the key channels; v over the block's columns) is brought into shared
 // memory kDeltaChunk tokens at a time with cp.async, the next chunk while the current one is computed; inside a chunk
 // the next token's vectors are read into registers before the current token is computed, so the token loop waits for
-// neither global nor shared memory.  The raw o goes to global memory; delta_out_kernel finishes it.
+// neither global nor shared memory.  The raw o goes to global memory; the kernels of lm_mechanisms.cuh that end a recurrence finish it.
 constexpr int kDeltaChunk = 16;
 
 __host__ __device__ constexpr int delta_lanes(int DK) { return DK >= 256 ? 16 : DK >= 64 ? 8 : 4; }
@@ -3024,8 +3024,8 @@ static cudaError_t launch_f32_tile(const float* a, const float* w, float* y, int
     using T = smol::f32t::MmaTile<BM, BN, WM, WN>;
     const int cols = (N + BN - 1) / BN;
     // CTAs per tile: as many as bring the grid of a single row of tiles to about four per SM, each with at least 128 k.  From N, K and the
-    // batch alone: a row's sums must not depend on how many rows the step holds.  (With S from the rows as well 1024 rows of 4608 x 768 took 179 us, 201 now,
-    // and 343 without a split; 300 rows 74 either way.)
+    // batch alone: a row's sums must not depend on how many rows the step holds.  (K shared by 1 / 2 / 4: 300 rows of 4608 x 768 60 / 50 / 54 us, 1024 rows 137 / 139 /
+    // 150; of 768 x 4608 by 2 / 4 / 8: 76 / 66 / 59 and 166 / 158 / 154.)
     int S = 1;
     while (S < 8 && (long long)cols * batch * S < 4 * 148 && K / (2 * S) >= 128) S *= 2;
     static_assert(T::kSmemBytes <= 48 * 1024, "no attribute needed");

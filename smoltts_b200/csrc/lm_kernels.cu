@@ -1363,17 +1363,19 @@ __global__ void __launch_bounds__(kRowsWarps * 32) attn_rows_kernel(const AttnAr
         if (i < mine) attn_finish<T, MAXV, MAPS>(A, t0 + r0 + warp * R + i, h, lane, sum[i], out);
 }
 
-// PARTS 2: a query row has two warps, half of the round's keys each, whose states are joined at the end.  A warp's own chain of shared-memory loads and sums bounds the
-// kernel where every block has an SM to itself: one row at 2048 positions of 12 heads of 64 8.2 us, with one warp per query row 9.5; with more blocks than SMs
-// the smaller ones win (5 rows at 700, two maps of 6 heads: 16.2 against 12.4).
+// KPL 2: a round's 64 keys are two halves, and all first halves of the range make one softmax state, all second halves another; the two are joined at the end.
+// PARTS 2: a query row has two warps, a half each.  PARTS 1: one warp takes both, side by side.  The arithmetic is the same: which of the two forms a step takes
+// does not show in the result.  A warp's own chain of shared-memory loads and sums bounds the kernel where every block has an SM to itself: one row at 2048
+// positions of 12 heads of 64 8.2 us with two warps, 9.5 with one; with more blocks than SMs the smaller ones win (5 rows at 700, two maps of 6 heads: 16.2 against 12.4).
 template <class T, int MAXV, int KPL, int PARTS>
 __global__ void __launch_bounds__(256 * PARTS) attn_split_kernel(const AttnArgs A, const T* __restrict__ qbuf, const T* pool) {
-    // One block per (row, key/value head x group of up to 8 of its query rows, key range); one warp per query row (a query
+    // One block per (row, key/value head x group of up to 8 of its query rows, key range); PARTS warps per query row (a query
     // head, or one of its maps: the block then stages every map's keys beside the values they share).
     // 32 * KPL keys and values at a time (KPL keys per lane) are staged in shared memory (rows padded by 16 bytes: conflict-free
     // row-per-lane reads), so that no global load sits inside the softmax / value loops.
     extern __shared__ __align__(16) unsigned char sm_raw[];
-    constexpr int kPad = 16 / (int)sizeof(T), KEYS = 32 * KPL, KP = KPL / PARTS, OWN = 32 * KP;      // keys of a round, of a lane, of a warp
+    static_assert(KPL % PARTS == 0 && KPL <= 2, "one or two states per query row");
+    constexpr int kPad = 16 / (int)sizeof(T), KEYS = 32 * KPL, HV = KPL / PARTS, OWN = 32 * HV;      // keys of a round; halves, keys of a warp
     const int s = blockIdx.x / kShortSeq, r = blockIdx.x % kShortSeq;
     const int t0 = A.seq_start[s], n = A.seq_start[s + 1] - t0;
     if (n > kShortSeq || r >= n) { dep_wait(); return; }
@@ -1397,10 +1399,15 @@ __global__ void __launch_bounds__(256 * PARTS) attn_split_kernel(const AttnArgs 
     T* Vs = A.v_in_k ? Ks : Ks + KEYS * ldk * A.maps;
     const int32_t* bt = A.block_table + (size_t)s * A.max_pages;
     const float r1 = A.r1 ? A.r1[head] : 0.0f, r2 = A.r1 ? A.r2[head] : 0.0f, slope = A.slope ? A.slope[head] : 0.0f;
-    float m = -INFINITY, l = 0.0f;
-    float o[MAXV];                       // columns 2 lane + 64 (e / 2) + e % 2
+    float m[HV], l[HV];
+    float o[HV][MAXV];                   // columns 2 lane + 64 (e / 2) + e % 2
 #pragma unroll
-    for (int e = 0; e < MAXV; ++e) o[e] = 0.0f;
+    for (int x = 0; x < HV; ++x) {
+        m[x] = -INFINITY;
+        l[x] = 0.0f;
+#pragma unroll
+        for (int e = 0; e < MAXV; ++e) o[x][e] = 0.0f;
+    }
     // whole 16-byte pieces when every cached row starts on a 16-byte boundary (pages are 16-byte aligned)
     const bool kvec = (A.d * sizeof(T)) % 16 == 0 && (A.k_ld * sizeof(T)) % 16 == 0 && (A.k_off * sizeof(T)) % 16 == 0;
     const bool vvec = (A.dv * sizeof(T)) % 16 == 0 && (A.v_ld * sizeof(T)) % 16 == 0 && (A.v_off * sizeof(T)) % 16 == 0;
@@ -1451,71 +1458,86 @@ __global__ void __launch_bounds__(256 * PARTS) attn_split_kernel(const AttnArgs 
         __syncthreads();
         if (!active) continue;
         if (key0 >= cnt) continue;
-        float sc[KP], mx = -INFINITY, pl = 0.0f;
 #pragma unroll
-        for (int x = 0; x < KP; ++x) {
+        for (int x = 0; x < HV; ++x) {
             const int row = key0 + lane + 32 * x;
-            sc[x] = row < cnt ? attn_score<false>(A, key_dot<T>(qs, Ks + (map * KEYS + row) * ldk, A.d), pos - (j0 + row), r1, r2, slope) : -INFINITY;
-            mx = fmaxf(mx, sc[x]);
-        }
-        const float mn = fmaxf(m, warp_max(mx));          // finite: lane 0 holds a valid key
-        const float corr = expf(m - mn);
-#pragma unroll
-        for (int x = 0; x < KP; ++x) {
-            const float p = key0 + lane + 32 * x < cnt ? expf(sc[x] - mn) : 0.0f;
+            const float sc = row < cnt ? attn_score<false>(A, key_dot<T>(qs, Ks + (map * KEYS + row) * ldk, A.d), pos - (j0 + row), r1, r2, slope) : -INFINITY;
+            const float mn = fmaxf(m[x], warp_max(sc)), base = mn == -INFINITY ? 0.0f : mn;      // (a half with no key yet: weights of 0)
+            const float p = row < cnt ? expf(sc - base) : 0.0f, corr = expf(m[x] - base);
             ps[lane + 32 * x] = p;
-            pl += p;
+            l[x] = fmaf(l[x], corr, warp_sum(p));
+            m[x] = mn;
+#pragma unroll
+            for (int e = 0; e < MAXV; ++e) o[x][e] *= corr;
         }
-        l = l * corr + warp_sum(pl);
-        m = mn;
         __syncwarp();
+        auto add_value = [&](int x, int jj) {
+            const float pj = ps[32 * x + jj];
+            const T* row = Vs + (key0 + 32 * x + jj) * ldv + 2 * lane;
 #pragma unroll
-        for (int e = 0; e < MAXV; ++e) o[e] *= corr;
-        auto add_value = [&](int jj) {
-            const float pj = ps[jj - key0];
-#pragma unroll
-            for (int e = 0; e < MAXV; e += 2) {
-                const int c = 2 * lane + e * 32;
-                if (c < A.dv) {               // an odd last column's neighbour is padding and is not stored
-                    const float2 v = load_pair(Vs + jj * ldv + c);
-                    o[e] = fmaf(pj, v.x, o[e]);
-                    o[e + 1] = fmaf(pj, v.y, o[e + 1]);
+            for (int e = 0; e < MAXV; e += 2)
+                if (2 * lane + e * 32 < A.dv) {      // an odd last column's neighbour is padding and is not stored
+                    const float2 v = load_pair(row + e * 32);
+                    o[x][e] = fmaf(pj, v.x, o[x][e]);
+                    o[x][e + 1] = fmaf(pj, v.y, o[x][e + 1]);
                 }
-            }
         };
-        int jj = key0;
-        const int end = min(cnt, key0 + OWN);
-        for (; jj + 8 <= end; jj += 8) {
+        // keys that all of the warp's halves have, then those of the first alone; the next keys' loads go out under the current products
+        const int every = min(32, max(0, cnt - key0 - 32 * (HV - 1))), first = min(32, cnt - key0);
+        int jj = 0;
+        for (; jj + 8 / HV <= every; jj += 8 / HV) {
 #pragma unroll
-            for (int x = 0; x < 8; ++x) add_value(jj + x);      // the next keys' loads go out under the current products
+            for (int u = 0; u < 8 / HV; ++u)
+#pragma unroll
+                for (int x = 0; x < HV; ++x) add_value(x, jj + u);
         }
-        for (; jj < end; ++jj) add_value(jj);
+        for (; jj < every; ++jj)
+#pragma unroll
+            for (int x = 0; x < HV; ++x) add_value(x, jj);
+        if (HV > 1) {
+            for (; jj + 8 <= first; jj += 8) {
+#pragma unroll
+                for (int u = 0; u < 8; ++u) add_value(0, jj + u);
+            }
+            for (; jj < first; ++jj) add_value(0, jj);
+        }
         __syncwarp();
     }
-    if (PARTS == 2) {
-        // the second warp's state joins the first's (the first has seen a key; the second perhaps none)
-        float* other = reinterpret_cast<float*>(sm_raw) + nwarp * (A.d + OWN) + own * (MAXV * 32 + 2);      // over the staged keys
-        __syncthreads();
-        if (key0 > 0) {
-            if (lane == 0) { other[0] = m; other[1] = l; }
+    if (KPL == 2) {
+        float m2 = m[HV - 1], l2 = l[HV - 1], o2[MAXV];
 #pragma unroll
-            for (int e = 0; e < MAXV; ++e) other[2 + e * 32 + lane] = o[e];
+        for (int e = 0; e < MAXV; ++e) o2[e] = o[HV - 1][e];
+        if (PARTS == 2) {
+            float* other = reinterpret_cast<float*>(sm_raw) + nwarp * (A.d + OWN) + own * (MAXV * 32 + 2);      // over the staged keys
+            __syncthreads();
+            if (key0 > 0) {
+                if (lane == 0) { other[0] = m2; other[1] = l2; }
+#pragma unroll
+                for (int e = 0; e < MAXV; ++e) other[2 + e * 32 + lane] = o2[e];
+            }
+            __syncthreads();
+            if (key0 > 0) return;
+            m2 = other[0];
+            l2 = other[1];
+#pragma unroll
+            for (int e = 0; e < MAXV; ++e) o2[e] = other[2 + e * 32 + lane];
         }
-        __syncthreads();
-        if (key0 > 0) return;
-        const float m2 = other[0], mn = fmaxf(m, m2), w1 = expf(m - mn), w2 = m2 == -INFINITY ? 0.0f : expf(m2 - mn);
-        l = l * w1 + (w2 > 0.0f ? other[1] * w2 : 0.0f);
-        m = mn;
+        // the range has keys for its second halves: not to be read off their largest score, which passes over what is not a number
+        if (j_hi - j_lo >= 32) {
+            const float mn = fmaxf(m[0], m2), base = mn == -INFINITY ? 0.0f : mn, w1 = expf(m[0] - base), w2 = expf(m2 - base);
+            l[0] = fmaf(l2, w2, l[0] * w1);
+            m[0] = mn;
 #pragma unroll
-        for (int e = 0; e < MAXV; ++e) o[e] = o[e] * w1 + (w2 > 0.0f ? other[2 + e * 32 + lane] * w2 : 0.0f);
+            for (int e = 0; e < MAXV; ++e) o[0][e] = fmaf(o2[e], w2, o[0][e] * w1);
+        }
     }
     if (!active) return;
     float* dst = A.part + (((size_t)blockIdx.x * A.H * A.maps + h) * A.n_splits + blockIdx.z) * (A.dv + 2);
-    if (lane == 0) { dst[0] = m; dst[1] = l; }
+    if (lane == 0) { dst[0] = m[0]; dst[1] = l[0]; }
 #pragma unroll
     for (int e = 0; e < MAXV; ++e) {
         const int c = 2 * lane + e / 2 * 64 + e % 2;
-        if (c < A.dv) dst[2 + c] = o[e];
+        if (c < A.dv) dst[2 + c] = o[0][e];
     }
 }
 

@@ -12,17 +12,21 @@
 // (without a and u: X_o = W(0, t] r_t, O' = R V, no X_w, V', Y_a).  The decays are at most one, so nothing is divided and nothing grows; the inverse is a
 // forward substitution.
 //
-// chunk_prep_kernel makes X, Y, V' and O' of a (chunk, head) in one block; it is parallel over the whole prompt.  chunk_scan_kernel is what is left to do in
-// order: two small matrix products per sixteen tokens.  A head's value columns never mix, so a block takes eight of them, and its four warps share
-// the key channels.  Both products run on mma.sync m16n8k8: every fp32 operand as two tf32 parts, three MMAs (the fourth product lies below the last place),
-// 170 multiply-adds per clock and SM against 128 on the FMA pipe, and without the shared-memory traffic and shuffles that those need for 16 x 8 results.
+// (The chunk-wise form of the delta rule: the triangular inverse is that of a product of Householder-like updates, its WY representation.)
+//
+// chunk_prep_kernel (one decay per head: chunk_prep_head_kernel) makes X, Y, V' and O' of a (chunk, head) in one block; it is parallel over the whole prompt.
+// chunk_scan_kernel is what is left to do in order: two small matrix products per sixteen tokens.  A head's value columns never mix, so a block takes eight of them,
+// and its four warps share the key channels.  Both products run on mma.sync m16n8k16: every fp32 operand as three bf16 parts, which hold all of its 24 bits, and the
+// six products of parts that reach the last place (the split of a product over pieces of a shorter format): 170 multiply-adds per clock and SM against 128 on the FMA
+// pipe, and without the shared-memory traffic and shuffles that those need for 16 x 8 results.
 // The state's accumulator fragments become operand fragments through a patch of shared memory of the warp's own; the warps' shares of `seen` and o meet
-// in shared memory, one barrier per chunk.  X and Y lie in the order of the fragments, so a lane's share is one 16-byte load.
-// What bounds the scan is the instructions of that chain (some 220 of a warp and chunk, one warp per scheduler), no longer a chain per four tokens.
-// 2048 tokens, 12 heads of 64 x 64, generalized delta rule: 64 us (and 30 for the records) against 192 (25) four tokens at a time; 1801 tokens of 128 x 128: 140 (53)
-// against 358 (45); gated linear recurrence, 1024 tokens of 64 x 64: 30 (10) against 66 (5); gated delta rule and mLSTM, 3 x 1000 tokens of 64 x 64: 46 and 57 against 101
-// and 122.  The models' fp32 outputs stay as close to 64 bits as they were (generalized delta rule 3.54e-7 | 3.53e-7, gated linear recurrence 4.13e-7 | 4.20e-7, gated
-// delta rule 3.12e-7 | 3.09e-7, mLSTM 5.43e-7 | 5.42e-7; no more than two MMAs' sums in one accumulator: with four and eight 3.56e-7 and 3.14e-7).
+// in shared memory, one barrier per chunk.  X, Y and V lie as the parts of their fragments, so a lane's share is three 16-byte (V: 8-byte) loads.
+// What bounds the scan is the instructions of that chain (one warp per scheduler), no longer a chain per four tokens.
+// Records and scan, 2048 tokens, 12 heads of 64 x 64: generalized delta rule 109 us (four tokens at a time 211), decay per channel 79 (135), gated delta rule 92 (207),
+// mLSTM 76 (181); 1801 tokens of 128 x 128: 196 (408), 149 (220), 177 (307), 140 (266); 3 x 1000 of 64 x 64: 103 (172), 68 (84), 83 (107), 96 (140).
+// Error of the outputs | of the state against 64 bits, 1100 tokens of 12 heads of 64 x 64 (four tokens at a time): generalized delta rule 1.16e-7 (1.36) | 0.90e-7 (1.17), decay
+// per channel 1.08 (1.13) | 0.84 (0.90), gated delta rule 1.06 (1.18) | 0.81 (1.07), mLSTM 1.02 (1.16) | 0.80 (1.15); 9 to 256 channels, 210 to 2000 tokens: never above.
+// With two tf32 parts per operand (three MMAs of 8, 99 us where it is 109 now) the outputs were at 1.62, 1.49, 1.63 and 1.53e-7.
 #pragma once
 
 namespace smol {
@@ -34,13 +38,19 @@ constexpr int kChunkMinTokens = 256, kChunkMinTokensWide = 144, kChunkMinTokensW
 enum { kScanGeneralDelta = 0, kScanChannelDecay = 1, kScanHeadDecay = 2, kScanGatedDelta = 3 };
 constexpr bool scan_removes(int kind) { return kind == kScanGeneralDelta || kind == kScanGatedDelta; }      // has a and u
 __host__ __device__ constexpr int chunk_pad(int d) { return d <= 32 ? 32 : d <= 64 ? 64 : d <= 128 ? 128 : 256; }
-// A record holds the key side: X fragments [k-step of 8 channels][seen, o][32 lanes][4] | Y fragments [16 channels][k-step of 8 tokens: V, then seen]
-// [32 lanes][4] | W(0, 16]; the value side follows, per block of columns V' [16][8] (with removal) | O' [16][8] | V [16][8].
-__host__ __device__ constexpr int chunk_rows(bool removes) { return removes ? 2 * kChunk : kChunk; }
-__host__ __device__ constexpr int chunk_key_floats(bool removes, int DK) { return (2 * chunk_rows(removes) + 1) * DK; }
-__host__ __device__ constexpr int chunk_col_floats(bool removes) { return (removes ? 3 : 2) * kChunk * kChunkCols; }
+// Fragments of 16 x 16 lie as their three bf16 parts, made once beside the records instead of by every block that reads them; above 128 channels, where two such
+// records do not fit an SM, as fp32.
+__host__ __device__ constexpr bool chunk_split(int DK) { return DK <= 128; }
+__host__ __device__ constexpr int chunk_frag(int DK) { return chunk_split(DK) ? 384 : 256; }      // words of a fragment
+// A record holds the key side: X fragments [16 channels][seen, o] | Y fragments [16 channels][V, then seen] | W(0, 16]; the value side follows, per block of
+// columns V' [16][8] (with removal; rows in the order of chunk_place) | O' [16][8] | V's three parts, an operand fragment each [32 lanes][2].
+constexpr int kChunkVals = 3 * 64;
+__host__ __device__ constexpr int chunk_key_floats(bool removes, int DK) { return (removes ? 4 : 2) * DK / 16 * chunk_frag(DK) + DK; }
+__host__ __device__ constexpr int chunk_col_floats(bool removes) { return (removes ? 2 : 1) * kChunk * kChunkCols + kChunkVals; }
 __host__ __device__ constexpr int chunk_blocks(int columns) { return (columns + kChunkCols - 1) / kChunkCols; }
 __host__ __device__ constexpr int chunk_record(bool removes, int DK, int columns) { return chunk_key_floats(removes, DK) + chunk_blocks(columns) * chunk_col_floats(removes); }
+// Where row k of a 16 x 8 operand lies in shared memory: lane (g, q) reads rows 2 q + b + 8 r of column g, and so finds them in banks of its own
+__host__ __device__ constexpr int chunk_place(int k) { return (k >> 3) * 8 + (k & 1) * 4 + ((k >> 1) & 3); }
 // The records of a head follow one another: record (head, chunk) is head * cap + chunk.  Number of the first chunk of sequence `seq`, whose first row is t0
 // (sequences' records never overlap: floor(t0 / 16) + seq grows by at least a sequence's number of chunks)
 __host__ __device__ constexpr int chunk_first(int t0, int seq) { return t0 / kChunk + seq; }
@@ -76,76 +86,179 @@ __device__ __forceinline__ void scatter_sum8(float (&v)[N], int sub) {
     if (N == 4) v[0] += __shfl_xor_sync(0xffffffffu, v[0], 1);
 }
 
-__host__ __device__ constexpr int chunk_prep_floats(bool removes, int DK) {
-    return kChunk * ((removes ? 2 : 1) * (DK + 4 + DK + 8) + DK + 4) + 4 * DK + (removes ? 4 : 1) * kChunk * kChunk;
+// floats between the tokens' rows: r and u are gathered as operands whose rows are tokens, k and a as operands whose columns are; decays are read in pieces only
+__host__ __device__ constexpr int chunk_xl(int DK) { return DK + 8; }
+__host__ __device__ constexpr int chunk_yl(int DK) { return DK + 4; }
+constexpr int kDecayLd = kChunk + 4;      // W(s, t] of a head: [16 tokens t][s = -1 .. 15], here and there four more
+__host__ __device__ constexpr int chunk_prep_floats(int kind, int DK) {
+    const int xl = chunk_xl(DK), yl = chunk_yl(DK);
+    return kind == kScanGeneralDelta ? kChunk * (2 * xl + 2 * yl + DK + 4) + 4 * DK + 4 * kChunk * kChunk
+           : kind == kScanChannelDecay ? kChunk * (xl + yl + DK + 4) + 4 * DK + kChunk * kChunk
+           : kind == kScanGatedDelta ? kChunk * (2 * xl + yl + kDecayLd) + 2 * kChunk * kChunk
+                                     : kChunk * (xl + yl + kDecayLd) + kChunk * kChunk;
 }
 
-__device__ __forceinline__ void tf32_parts(float x, uint32_t& hi, uint32_t& lo) { f32t::tf32_parts(__float_as_uint(x), hi, lo); }
-using f32t::mma_tf32;
-// The two tf32 parts of fp32 fragments (f32_tile.cuh)
-struct PartsA {
-    uint32_t hi[4], lo[4];
-    __device__ __forceinline__ void set(float x, float y, float z, float w) {
-        tf32_parts(x, hi[0], lo[0]);
-        tf32_parts(y, hi[1], lo[1]);
-        tf32_parts(z, hi[2], lo[2]);
-        tf32_parts(w, hi[3], lo[3]);
+__device__ __forceinline__ void mma_bf16(float (&d)[4], const uint32_t (&a)[4], const uint32_t (&b)[2]) {
+    asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+        : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b[0]), "r"(b[1]));
+}
+// Two fp32 numbers as three pairs of bf16, eight bits each and cut off, so that nothing of the 24 is lost: x = p[0] + p[1] + p[2].
+__device__ __forceinline__ void bf16_parts(float x, float y, uint32_t (&p)[3]) {
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+        const uint32_t a = __float_as_uint(x), b = __float_as_uint(y);
+        p[i] = __byte_perm(a, b, 0x7632);
+        x -= __uint_as_float(a & 0xffff0000u);
+        y -= __uint_as_float(b & 0xffff0000u);
     }
+}
+// Operands of mma.sync m16n8k16 in their three parts
+struct PartsA {
+    uint32_t p[3][4];
+    // rows g, g + 8, g, g + 8; columns 2 q, 2 q + 1 (the last two: + 8)
+    __device__ __forceinline__ void set(int i, float x, float y) {
+        uint32_t z[3];
+        bf16_parts(x, y, z);
+#pragma unroll
+        for (int k = 0; k < 3; ++k) p[k][i] = z[k];
+    }
+    template <bool SPLIT>
     __device__ __forceinline__ void load(const float* frag, int lane) {
-        const float4 v = reinterpret_cast<const float4*>(frag)[lane];
-        set(v.x, v.y, v.z, v.w);
+        if (SPLIT) {
+#pragma unroll
+            for (int k = 0; k < 3; ++k) {
+                const uint4 v = reinterpret_cast<const uint4*>(frag)[k * 32 + lane];
+                p[k][0] = v.x; p[k][1] = v.y; p[k][2] = v.z; p[k][3] = v.w;
+            }
+        } else {
+#pragma unroll
+            for (int k = 0; k < 2; ++k) {
+                const float4 v = reinterpret_cast<const float4*>(frag)[k * 32 + lane];
+                set(2 * k, v.x, v.y);
+                set(2 * k + 1, v.z, v.w);
+            }
+        }
+    }
+    template <bool SPLIT>
+    __device__ static __forceinline__ void store(float* frag, int lane, const float (&v)[8]) {
+        if (SPLIT) {
+            PartsA a;
+#pragma unroll
+            for (int i = 0; i < 4; ++i) a.set(i, v[2 * i], v[2 * i + 1]);
+#pragma unroll
+            for (int k = 0; k < 3; ++k) reinterpret_cast<uint4*>(frag)[k * 32 + lane] = make_uint4(a.p[k][0], a.p[k][1], a.p[k][2], a.p[k][3]);
+        } else {
+#pragma unroll
+            for (int k = 0; k < 2; ++k) reinterpret_cast<float4*>(frag)[k * 32 + lane] = make_float4(v[4 * k], v[4 * k + 1], v[4 * k + 2], v[4 * k + 3]);
+        }
     }
 };
 struct PartsB {
-    uint32_t hi[2], lo[2];
-    __device__ __forceinline__ void set(float x, float y) {
-        tf32_parts(x, hi[0], lo[0]);
-        tf32_parts(y, hi[1], lo[1]);
-    }
-};
-// The three products that count, in accumulators of their own: one after the other they would wait 20 clocks for each other.
-struct Acc3 {
-    float big[4], s1[4], s2[4];
-    __device__ __forceinline__ void zero() {
+    uint32_t p[3][2];
+    // rows 2 q, 2 q + 1 (the second: + 8) of column g
+    __device__ __forceinline__ void set(int i, float x, float y) {
+        uint32_t z[3];
+        bf16_parts(x, y, z);
 #pragma unroll
-        for (int e = 0; e < 4; ++e) big[e] = s1[e] = s2[e] = 0.0f;
+        for (int k = 0; k < 3; ++k) p[k][i] = z[k];
     }
-    __device__ __forceinline__ void mma(const PartsA& a, const PartsB& b) {
-        mma_tf32(s1, a.hi, b.lo[0], b.lo[1]);
-        mma_tf32(s2, a.lo, b.hi[0], b.hi[1]);
-        mma_tf32(big, a.hi, b.hi[0], b.hi[1]);
+    __device__ __forceinline__ void load(const float* parts, int lane) {
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+            const uint2 v = reinterpret_cast<const uint2*>(parts)[k * 32 + lane];
+            p[k][0] = v.x; p[k][1] = v.y;
+        }
     }
-    __device__ __forceinline__ float sum(int e) const { return big[e] + (s1[e] + s2[e]); }
 };
-// sum += a b over N k-steps: the tensor core drops what lies below its accumulator's last place, so no more than two of its sums follow one another
+// sum = a b over N steps of 16: six of the nine products of parts (the others lie below the last place), those of one size in accumulators of their own, no more than
+// two MMAs behind one another.  The tensor core cuts its sums off instead of rounding them; what the largest one loses by that in the mean is given back.
+constexpr float kCutOff = 0.85f * 0x1p-24f;
 template <int N>
 __device__ __forceinline__ void mma_sum(float (&sum)[4], const PartsA (&a)[N], const PartsB (&b)[N]) {
 #pragma unroll
-    for (int k = 0; k < N; k += 2) {
-        Acc3 acc;
-        acc.zero();
-        acc.mma(a[k], b[k]);
-        if (k + 1 < N) acc.mma(a[k + 1 < N ? k + 1 : k], b[k + 1 < N ? k + 1 : k]);
+    for (int k = 0; k < N; ++k) {
+        float big[4], s1[4], s2[4], s3[4];
 #pragma unroll
-        for (int e = 0; e < 4; ++e) sum[e] = k == 0 ? acc.sum(e) : sum[e] + acc.sum(e);
+        for (int e = 0; e < 4; ++e) big[e] = s1[e] = s2[e] = s3[e] = 0.0f;
+        mma_bf16(s1, a[k].p[0], b[k].p[2]);
+        mma_bf16(s2, a[k].p[2], b[k].p[0]);
+        mma_bf16(s3, a[k].p[1], b[k].p[1]);
+        mma_bf16(big, a[k].p[0], b[k].p[0]);
+        mma_bf16(s1, a[k].p[0], b[k].p[1]);
+        mma_bf16(s2, a[k].p[1], b[k].p[0]);
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            const float t = big[e] + (fmaf(big[e], kCutOff, s3[e]) + (s1[e] + s2[e]));
+            sum[e] = k == 0 ? t : sum[e] + t;
+        }
     }
 }
 
-// One block per (chunk, sequence, head); a warp has four tokens, the chunk four such quads.  The vectors lie in shared memory [16][DK].  Within a quad a warp
+// acc += sign * sum_(s < upto) p[s] z[s] over the quad s = 4 i .., which is added up by itself
+__device__ __forceinline__ void chunk_take(float& acc, const float4 p, const float (&z)[kChunk], int i, int upto, float sign) {
+    float part = 0.0f;
+    if (4 * i < upto) part = p.x * z[4 * i];
+    if (4 * i + 1 < upto) part = fmaf(p.y, z[4 * i + 1], part);
+    if (4 * i + 2 < upto) part = fmaf(p.z, z[4 * i + 2], part);
+    if (4 * i + 3 < upto) part = fmaf(p.w, z[4 * i + 3], part);
+    acc = fmaf(sign, part, acc);
+}
+__device__ __forceinline__ float2 two(const float* p) { return *reinterpret_cast<const float2*>(p); }
+// value column j of a chunk's rows (a unit column is behind the value columns); V's parts of that column in its block's record
+__device__ __forceinline__ void chunk_values(const ChunkSource& A, size_t row, int n, int h, int j, float (&v)[kChunk]) {
+    const float* at = A.v + row * A.v_ld + h * A.dv + j;
+#pragma unroll
+    for (int t = 0; t < kChunk; ++t, at += A.v_ld) v[t] = t < n && j < A.columns ? (j < A.dv ? *at : 1.0f) : 0.0f;
+}
+template <bool REM>
+__device__ __forceinline__ void chunk_value_parts(float* cols, int j, const float (&v)[kChunk]) {
+    uint2* parts = reinterpret_cast<uint2*>(cols + (j / kChunkCols) * chunk_col_floats(REM) + (REM ? 2 : 1) * kChunk * kChunkCols) + j % kChunkCols * 4;
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+        PartsB b;
+        b.set(0, v[2 * q], v[2 * q + 1]);
+        b.set(1, v[2 * q + 8], v[2 * q + 9]);
+#pragma unroll
+        for (int k = 0; k < 3; ++k) parts[k * 32 + q] = make_uint2(b.p[k][0], b.p[k][1]);
+    }
+}
+// The key side's fragments: X from rows of tokens, Y from columns of tokens (`removed`: the sign of the writes along a: 1, or -1 where a is k itself)
+template <int DK, bool REM>
+__device__ __forceinline__ void chunk_fragments(float* out, const float* s_u, const float* s_r, const float* s_k, const float* s_a, float removed) {
+    constexpr int MX = REM ? 2 : 1, FR = chunk_frag(DK), XL = chunk_xl(DK), YL = chunk_yl(DK);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, gq = lane >> 2, q = lane & 3;
+#pragma unroll 2
+    for (int i = warp; i < DK / 16 * MX; i += 4) {
+        const float* p = (REM && i % MX == 0 ? s_u : s_r) + gq * XL + i / MX * 16 + 2 * q;
+        const float2 a = two(p), b = two(p + 8 * XL), c = two(p + 8), e = two(p + 8 * XL + 8);
+        PartsA::store<chunk_split(DK)>(out + i * FR, lane, {a.x, a.y, b.x, b.y, c.x, c.y, e.x, e.y});
+    }
+#pragma unroll 2
+    for (int i = warp; i < DK / 16 * MX; i += 4) {
+        const bool of_a = i % MX != 0;
+        const float* p = (of_a ? s_a : s_k) + 2 * q * YL + i / MX * 16 + gq;
+        const float f = of_a ? removed : 1.0f;
+        PartsA::store<chunk_split(DK)>(out + (DK / 16 * MX + i) * FR, lane,
+                                       {f * p[0], f * p[YL], f * p[8], f * p[YL + 8], f * p[8 * YL], f * p[9 * YL], f * p[8 * YL + 8], f * p[9 * YL + 8]});
+    }
+}
+
+// Decays per channel.  One block per (chunk, sequence, head); a warp has four tokens, the chunk four such quads.  The vectors lie in shared memory [16][DK].  Within a quad a warp
 // makes the products on the FMA pipe, eight lanes per token, the decays multiplied in on the way back from token to token; products between two quads
-// are made by MMAs (three tf32 parts of fp32 operands, as in the scan) from what each side is at the border: the later one's vectors decayed back to the
+// are made by MMAs (operands in three bf16 parts, as in the scan) from what each side is at the border: the later one's vectors decayed back to the
 // start of its quad, the earlier one's writes decayed up to there.  Then a thread per column runs the substitutions, and the results leave as fragments.
 template <int KIND, int DK>
 __global__ void __launch_bounds__(128, DK <= 64 ? 5 : DK <= 128 ? 4 : 1) chunk_prep_kernel(const ChunkSource A, float* __restrict__ rec) {
     dep_wait();
     dep_go();
     using f32t::fma2;
-    constexpr bool REM = scan_removes(KIND), CHANNEL = KIND == kScanGeneralDelta || KIND == kScanChannelDecay;
-    constexpr int XL = DK + 4, YL = DK + 8, NM = REM ? 4 : 1, E = DK / 32;       // row strides free of bank conflicts where fragments are gathered
+    constexpr bool REM = scan_removes(KIND);
+    static_assert(KIND == kScanGeneralDelta || KIND == kScanChannelDecay, "one decay per head: chunk_prep_head_kernel");
+    constexpr int XL = chunk_xl(DK), YL = chunk_yl(DK), WL = DK + 4, NM = REM ? 4 : 1, E = DK / 32;
     constexpr int kR = NM - 1, kM = NM > 1 ? 1 : 0, kA = NM > 1 ? 2 : 0;         // products: L, M, A, R, or R alone
     extern __shared__ __align__(16) float sh[];
     float *s_r = sh, *s_u = s_r + kChunk * XL, *s_k = s_u + (REM ? kChunk * XL : 0), *s_a = s_k + kChunk * YL, *s_w = s_a + (REM ? kChunk * YL : 0);
-    float *s_q = s_w + kChunk * XL, *s_m = s_q + 4 * DK;                         // a quad's decay [4][DK]; products [NM][16][16]
+    float *s_q = s_w + kChunk * WL, *s_m = s_q + 4 * DK;                         // a quad's decay [4][DK]; products [NM][16][16]
     const int h = blockIdx.z, seq = blockIdx.y, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int t0 = A.seq_start[seq], n_all = A.seq_start[seq + 1] - t0, r0 = blockIdx.x * kChunk;
     if (r0 >= n_all) return;
@@ -155,44 +268,31 @@ __global__ void __launch_bounds__(128, DK <= 64 ? 5 : DK <= 128 ? 4 : 1) chunk_p
     // value column j of the rows, every load on its way before the products are made (DK 64: on the threads that will have no key channel)
     const int j_first = DK <= 64 ? (int)(threadIdx.x + 128 - DK) % 128 : (int)threadIdx.x;
     float v[kChunk];
-    auto load_values = [&](int j) {
-        const float* at = A.v + (size_t)(t0 + r0) * A.v_ld + h * A.dv + j;
-#pragma unroll
-        for (int t = 0; t < kChunk; ++t, at += A.v_ld) v[t] = t < n && j < A.columns ? (j < A.dv ? *at : 1.0f) : 0.0f;
-    };
     constexpr bool EARLY = DK <= 64 && REM;
-    if (EARLY) load_values(j_first);
+    if (EARLY) chunk_values(A, t0 + r0, n, h, j_first, v);
     // ---- the tokens' vectors ----
     {
-        float kv[4][E], qv[4][E], wv[4][E], rv[4][E], bias[E], hw[4], hs[4];
+        float kv[4][E], qv[4][E], wv[4][E], rv[4][E], bias[E];
 #pragma unroll
         for (int e = 0; e < E; ++e) bias[e] = KIND == kScanGeneralDelta && lane + 32 * e < d ? A.rate_bias[h * d + lane + 32 * e] : 0.0f;
         const size_t row = t0 + r0 + warp * 4;
         const float *pk = A.k + row * A.k_ld + g * d + lane, *pq = A.q + row * A.q_ld + g * d + lane;
-        const float* pw = CHANNEL ? A.decay + row * A.H * d + h * d + lane : A.head_decay + row * A.head_ld + h * A.head_el;
-        const float* pr = KIND == kScanGeneralDelta ? A.rate + row * A.k_ld + h * d + lane : A.head_step ? A.head_step + row * A.head_ld + h * A.head_el : nullptr;
+        const float *pw = A.decay + row * A.H * d + h * d + lane, *pr = KIND == kScanGeneralDelta ? A.rate + row * A.k_ld + h * d + lane : nullptr;
 #pragma unroll
         for (int x = 0; x < 4; ++x) {
             const bool on = warp * 4 + x < n;
-            hw[x] = 1.0f;
-            hs[x] = 0.0f;
-            if (!CHANNEL && on) {
-                hw[x] = *pw;
-                hs[x] = pr ? *pr : 1.0f;
-            }
 #pragma unroll
             for (int e = 0; e < E; ++e) {
                 const bool in = on && lane + 32 * e < d;
                 kv[x][e] = in ? pk[32 * e] : 0.0f;
                 qv[x][e] = in ? pq[32 * e] : 0.0f;
-                wv[x][e] = CHANNEL && in ? pw[32 * e] : 1.0f;
+                wv[x][e] = in ? pw[32 * e] : 1.0f;
                 rv[x][e] = KIND == kScanGeneralDelta && in ? pr[32 * e] : 0.0f;
             }
             pk += A.k_ld;
             pq += A.q_ld;
-            pw += CHANNEL ? A.H * d : A.head_ld;
+            pw += A.H * d;
             if (KIND == kScanGeneralDelta) pr += A.k_ld;
-            else if (pr) pr += A.head_ld;
         }
 #pragma unroll
         for (int x = 0; x < 4; ++x) {
@@ -208,17 +308,13 @@ __global__ void __launch_bounds__(128, DK <= 64 ? 5 : DK <= 128 ? 4 : 1) chunk_p
             for (int e = 0; e < E; ++e) {
                 const int c = lane + 32 * e;
                 s_r[t * XL + c] = qv[x][e];
-                s_w[t * XL + c] = CHANNEL ? wv[x][e] : hw[x];
-                float u = 0.0f, a = 0.0f, k = kv[x][e];
-                if (KIND == kScanGeneralDelta) {
-                    u = k * inv;
-                    a = t < n && c < d ? sigmoidf_(rv[x][e] + bias[e]) * u : 0.0f;
-                } else if (KIND == kScanGatedDelta) {      // S <- w S; S <- S + b k (v - k^T S): what is removed reads the state before the decay
-                    u = hw[x] * k;
-                    a = k = hs[x] * k;
-                } else if (KIND == kScanHeadDecay) k = hs[x] * k;
-                s_k[t * YL + c] = k;
-                if (REM) { s_u[t * XL + c] = u; s_a[t * YL + c] = a; }
+                s_w[t * WL + c] = wv[x][e];
+                s_k[t * YL + c] = kv[x][e];
+                if (REM) {
+                    const float u = kv[x][e] * inv;
+                    s_u[t * XL + c] = u;
+                    s_a[t * YL + c] = t < n && c < d ? sigmoidf_(rv[x][e] + bias[e]) * u : 0.0f;
+                }
             }
         }
     }
@@ -244,7 +340,7 @@ __global__ void __launch_bounds__(128, DK <= 64 ? 5 : DK <= 128 ? 4 : 1) chunk_p
             for (int m = 0; m < NM; ++m) p[m] = 0ull;
 #pragma unroll
             for (int e = 0; e < E; ++e) {
-                const ulonglong2 kk = piece(s_k + s * YL, e), ww = piece(s_w + s * XL, e);
+                const ulonglong2 kk = piece(s_k + s * YL, e), ww = piece(s_w + s * WL, e);
                 p[kR] = fma2(y[e].x, kk.x, p[kR]); p[kR] = fma2(y[e].y, kk.y, p[kR]);
                 if (REM) {
                     const ulonglong2 aa = piece(s_a + s * YL, e);
@@ -276,7 +372,7 @@ __global__ void __launch_bounds__(128, DK <= 64 ? 5 : DK <= 128 ? 4 : 1) chunk_p
             ulonglong2 all = one, mine = one;
 #pragma unroll
             for (int i = 3; i >= 0; --i) {
-                const ulonglong2 ww = piece(s_w + (warp * 4 + i) * XL, e);
+                const ulonglong2 ww = piece(s_w + (warp * 4 + i) * WL, e);
                 if (i == tg) mine = all;
                 all = {mul2(all.x, ww.x), mul2(all.y, ww.y)};
             }
@@ -306,22 +402,24 @@ __global__ void __launch_bounds__(128, DK <= 64 ? 5 : DK <= 128 ? 4 : 1) chunk_p
             const float *col = REM && gq < 4 ? s_a + (4 * j + gq) * YL : s_k + (4 * j + (gq & 3)) * YL;
             float sum[2] = {0.0f, 0.0f};
 #pragma unroll 4
-            for (int k = 0; k < DK / 8; k += 2) {
-                PartsA a[2];
-                PartsB z[2];
+            for (int k = 0; k < DK / 16; ++k) {
+                PartsA a[1];
+                PartsB z[1];
 #pragma unroll
                 for (int x = 0; x < 2; ++x) {
-                    const int c = 8 * (k + x) + q;
-                    float z0 = col[c], z1 = col[c + 4];                    // ... times the decay of the quads between
-                    if (i - j > 1) { z0 *= s_q[(i - 1) * DK + c]; z1 *= s_q[(i - 1) * DK + c + 4]; }
-                    if (i - j > 2) { z0 *= s_q[(i - 2) * DK + c]; z1 *= s_q[(i - 2) * DK + c + 4]; }
-                    a[x].set(row[c], 0.0f, row[c + 4], 0.0f);
-                    z[x].set(z0, z1);
+                    const int c = 16 * k + 8 * x + 2 * q;
+                    const float2 r2 = two(row + c);
+                    float2 z2 = two(col + c);                              // ... times the decay of the quads between
+                    if (i - j > 1) { const float2 w2 = two(s_q + (i - 1) * DK + c); z2.x *= w2.x; z2.y *= w2.y; }
+                    if (i - j > 2) { const float2 w2 = two(s_q + (i - 2) * DK + c); z2.x *= w2.x; z2.y *= w2.y; }
+                    a[0].set(2 * x, r2.x, r2.y);
+                    a[0].set(2 * x + 1, 0.0f, 0.0f);
+                    z[0].set(x, z2.x, z2.y);
                 }
-                float two[4];
-                mma_sum<2>(two, a, z);
-                sum[0] += two[0];
-                sum[1] += two[1];
+                float part[4];
+                mma_sum<1>(part, a, z);
+                sum[0] += part[0];
+                sum[1] += part[1];
             }
             // row gq, columns 2 q, 2 q + 1
 #pragma unroll
@@ -335,12 +433,6 @@ __global__ void __launch_bounds__(128, DK <= 64 ? 5 : DK <= 128 ? 4 : 1) chunk_p
     __syncthreads();
     // ---- columns: key channels first, then value columns; row t of a product, elements 4 i .. + 3 ----
     auto row4 = [&](int m, int t, int i) { return *reinterpret_cast<const float4*>(s_m + m * kChunk * kChunk + t * kChunk + 4 * i); };
-    auto take = [&](float& acc, const float4 p, const float (&z)[kChunk], int i, int upto, float sign) {      // acc += sign * sum_(s < upto) p[s] z[s]
-        if (4 * i < upto) acc = fmaf(sign * p.x, z[4 * i], acc);
-        if (4 * i + 1 < upto) acc = fmaf(sign * p.y, z[4 * i + 1], acc);
-        if (4 * i + 2 < upto) acc = fmaf(sign * p.z, z[4 * i + 2], acc);
-        if (4 * i + 3 < upto) acc = fmaf(sign * p.w, z[4 * i + 3], acc);
-    };
     for (int c = threadIdx.x; c < DK; c += 128) {
         float xw[kChunk], p = 1.0f;
 #pragma unroll
@@ -349,15 +441,15 @@ __global__ void __launch_bounds__(128, DK <= 64 ? 5 : DK <= 128 ? 4 : 1) chunk_p
             if (REM) {
                 xw[t] = p * s_u[t * XL + c];
 #pragma unroll
-                for (int i = 0; 4 * i < t; ++i) take(xw[t], row4(0, t, i), xw, i, t, -1.0f);
+                for (int i = 0; 4 * i < t; ++i) chunk_take(xw[t], row4(0, t, i), xw, i, t, -1.0f);
 #pragma unroll
-                for (int i = 0; 4 * i <= t; ++i) take(o, row4(kA, t, i), xw, i, t + 1, -1.0f);
+                for (int i = 0; 4 * i <= t; ++i) chunk_take(o, row4(kA, t, i), xw, i, t + 1, -1.0f);
                 s_u[t * XL + c] = xw[t];
             }
             s_r[t * XL + c] = o;
             if (t % 4 == 3) p *= s_q[t / 4 * DK + c];
         }
-        out[2 * chunk_rows(REM) * DK + c] = p;
+        out[chunk_key_floats(REM, DK) - DK + c] = p;
         p = 1.0f;
 #pragma unroll
         for (int s = kChunk - 1; s >= 0; --s) {
@@ -369,7 +461,7 @@ __global__ void __launch_bounds__(128, DK <= 64 ? 5 : DK <= 128 ? 4 : 1) chunk_p
     asm volatile("" ::: "memory");               // the products are read again: kept for both loops they do not fit the registers (DK 128)
     float* cols = out + chunk_key_floats(REM, DK);
     for (int j = j_first; j < n_cols; j += 128) {
-        if (!EARLY || j != j_first) load_values(j);
+        if (!EARLY || j != j_first) chunk_values(A, t0 + r0, n, h, j, v);
         float seen[kChunk];
         float* to = cols + (j / kChunkCols) * chunk_col_floats(REM) + j % kChunkCols;
 #pragma unroll
@@ -380,37 +472,167 @@ __global__ void __launch_bounds__(128, DK <= 64 ? 5 : DK <= 128 ? 4 : 1) chunk_p
                 seen[t] = 0.0f;
 #pragma unroll
                 for (int i = 0; 4 * i < t; ++i) {
-                    take(seen[t], row4(kM, t, i), v, i, t, 1.0f);
-                    take(seen[t], row4(0, t, i), seen, i, t, -1.0f);
+                    chunk_take(seen[t], row4(kM, t, i), v, i, t, 1.0f);
+                    chunk_take(seen[t], row4(0, t, i), seen, i, t, -1.0f);
                 }
-                to[t * kChunkCols] = seen[t];
+                to[chunk_place(t) * kChunkCols] = seen[t];
             }
 #pragma unroll
             for (int i = 0; 4 * i <= t; ++i) {
-                take(o, row4(kR, t, i), v, i, t + 1, 1.0f);
-                if (REM) take(o, row4(kA, t, i), seen, i, t + 1, -1.0f);
+                chunk_take(o, row4(kR, t, i), v, i, t + 1, 1.0f);
+                if (REM) chunk_take(o, row4(kA, t, i), seen, i, t + 1, -1.0f);
             }
             to[(REM ? kChunk + t : t) * kChunkCols] = o;
-            to[((REM ? 2 : 1) * kChunk + t) * kChunkCols] = v[t];
         }
+        chunk_value_parts<REM>(cols, j, v);
     }
     __syncthreads();
     // ---- fragments ----
-    float4* frag = reinterpret_cast<float4*>(out);
-    constexpr int MX = REM ? 2 : 1;
-#pragma unroll 4
-    for (int i = threadIdx.x; i < DK / 8 * MX * 32; i += 128) {
-        const int l = i & 31, m = i / 32 % MX, c = i / 32 / MX * 8 + (l & 3);
-        const float* p = (REM && m == 0 ? s_u : s_r) + (l >> 2) * XL + c;
-        frag[i] = make_float4(p[0], p[8 * XL], p[4], p[8 * XL + 4]);
+    chunk_fragments<DK, REM>(out, s_u, s_r, s_k, s_a, 1.0f);
+}
+
+// One decay per head and token: it leaves the products of vectors alone and multiplies them afterwards.  W(s, t] is a product of at most sixteen numbers in fp64,
+// rounded once (multiplied up along the vectors, its roundings would be the same in all of a head's channels).  The gated delta rule, S <- w S + b k (v - k^T (w S))^T,
+// removes along what it writes along: with L = W(s, t] (k_t . b_s k_s) and R likewise of r, and u_t = v_t - sum_(s < t) L u_s what a token writes,
+//     X_w = W(0, t] k_t - L X_w      V' = L u      X_o = W(0, t] r_t - R X_w      O' = R u      Y_v = W(s, 16] b_s k_s = -Y_a.
+// One block per (chunk, sequence, head).  All products are MMAs, a warp a triangle's half (eight columns; without removal two of the warps).
+template <int KIND, int DK>
+__global__ void __launch_bounds__(128, DK <= 64 ? 5 : DK <= 128 ? 4 : 1) chunk_prep_head_kernel(const ChunkSource A, float* __restrict__ rec) {
+    dep_wait();
+    dep_go();
+    constexpr bool REM = scan_removes(KIND);
+    constexpr int XL = chunk_xl(DK), YL = chunk_yl(DK), NM = REM ? 2 : 1, E = DK / 32, kR = NM - 1;
+    extern __shared__ __align__(16) float sh[];
+    float *s_r = sh, *s_u = s_r + kChunk * XL, *s_k = s_u + (REM ? kChunk * XL : 0), *s_m = s_k + kChunk * YL, *s_w = s_m + NM * kChunk * kChunk;
+    const int h = blockIdx.z, seq = blockIdx.y, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int t0 = A.seq_start[seq], n_all = A.seq_start[seq + 1] - t0, r0 = blockIdx.x * kChunk;
+    if (r0 >= n_all) return;
+    const int n = min(kChunk, n_all - r0), g = h / A.share, d = A.d;
+    const int nb = chunk_blocks(A.columns), n_cols = nb * kChunkCols;
+    float* out = rec + ((size_t)h * A.cap + chunk_first(t0, seq) + blockIdx.x) * (chunk_key_floats(REM, DK) + nb * chunk_col_floats(REM));
+    // value column j of the rows, every load on its way before the products are made (DK 64: on the threads that will have no key channel)
+    const int j_first = DK <= 64 ? (int)(threadIdx.x + 128 - DK) % 128 : (int)threadIdx.x;
+    float v[kChunk];
+    constexpr bool EARLY = DK <= 64 && REM;
+    if (EARLY) chunk_values(A, t0 + r0, n, h, j_first, v);
+    // ---- the tokens' vectors, four tokens a warp; the decays ----
+    {
+        float kv[4][E], qv[4][E], hs[4];
+        const size_t row = t0 + r0 + warp * 4;
+        const float *pk = A.k + row * A.k_ld + g * d + lane, *pq = A.q + row * A.q_ld + g * d + lane, *ps = A.head_step ? A.head_step + row * A.head_ld + h * A.head_el : nullptr;
+        float w = 1.0f;
+        if (warp == 3 && lane < n) w = A.head_decay[(size_t)(t0 + r0 + lane) * A.head_ld + h * A.head_el];
+#pragma unroll
+        for (int x = 0; x < 4; ++x) {
+            const bool on = warp * 4 + x < n;
+            hs[x] = on && ps ? *ps : 1.0f;
+#pragma unroll
+            for (int e = 0; e < E; ++e) {
+                const bool in = on && lane + 32 * e < d;
+                kv[x][e] = in ? pk[32 * e] : 0.0f;
+                qv[x][e] = in ? pq[32 * e] : 0.0f;
+            }
+            pk += A.k_ld;
+            pq += A.q_ld;
+            if (ps) ps += A.head_ld;
+        }
+        if (warp == 3) {
+            // lane t: W(s, t] for s = t down to -1, at s + 1
+            double p = 1.0;
+#pragma unroll
+            for (int s = kChunk - 1; s >= 0; --s) {
+                const float ws = __shfl_sync(0xffffffffu, w, s);
+                if (s > lane || lane >= kChunk) continue;
+                s_w[lane * kDecayLd + s + 1] = (float)p;
+                p *= (double)ws;
+            }
+            if (lane < kChunk) s_w[lane * kDecayLd] = (float)p;
+        }
+#pragma unroll
+        for (int x = 0; x < 4; ++x)
+#pragma unroll
+            for (int e = 0; e < E; ++e) {
+                const int t = warp * 4 + x, c = lane + 32 * e;
+                s_r[t * XL + c] = qv[x][e];
+                if (REM) s_u[t * XL + c] = kv[x][e];
+                s_k[t * YL + c] = hs[x] * kv[x][e];
+            }
     }
-    frag += DK / 8 * MX * 32;
+    __syncthreads();
+    // ---- products: rows 16 tokens t, columns eight tokens s ----
+    if (warp < 2 * NM) {
+        const int gq = lane >> 2, q = lane & 3, m = warp >> 1, s0 = (warp & 1) * 8;
+        const float *row = (REM && m == 0 ? s_u : s_r) + gq * XL + 2 * q, *col = s_k + (s0 + gq) * YL + 2 * q;
+        float sum[4];
 #pragma unroll 4
-    for (int i = threadIdx.x; i < DK / 16 * 2 * MX * 32; i += 128) {
-        const int l = i & 31, ks = i / 32 % (2 * MX), c = i / 32 / (2 * MX) * 16 + (l >> 2);
-        const float* p = (ks < 2 ? s_k : s_a) + (8 * (ks & 1) + (l & 3)) * YL + c;
-        frag[i] = make_float4(p[0], p[8], p[4 * YL], p[4 * YL + 8]);
+        for (int k = 0; k < DK / 16; ++k) {
+            PartsA a[1];
+            PartsB z[1];
+#pragma unroll
+            for (int x = 0; x < 2; ++x) {
+                const float2 lo = two(row + 16 * k + 8 * x), hi = two(row + 8 * XL + 16 * k + 8 * x), b2 = two(col + 16 * k + 8 * x);
+                a[0].set(2 * x, lo.x, lo.y);
+                a[0].set(2 * x + 1, hi.x, hi.y);
+                z[0].set(x, b2.x, b2.y);
+            }
+            float part[4];
+            mma_sum<1>(part, a, z);
+#pragma unroll
+            for (int e = 0; e < 4; ++e) sum[e] = k == 0 ? part[e] : sum[e] + part[e];
+        }
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            const int t = gq + 8 * (e >> 1), s = s0 + 2 * q + (e & 1);
+            // what lies behind the diagonal is dropped, also where it is not finite
+            s_m[m * kChunk * kChunk + t * kChunk + s] = (REM && m == 0 ? s < t : s <= t) ? sum[e] * s_w[t * kDecayLd + s + 1] : 0.0f;
+        }
     }
+    __syncthreads();
+    // ---- columns: key channels first, then value columns; row t of a product, elements 4 i .. + 3 ----
+    auto row4 = [&](int m, int t, int i) { return *reinterpret_cast<const float4*>(s_m + m * kChunk * kChunk + t * kChunk + 4 * i); };
+    for (int c = threadIdx.x; c < DK; c += 128) {
+        float xw[kChunk];
+#pragma unroll
+        for (int t = 0; t < kChunk; ++t) {
+            const float w = s_w[t * kDecayLd];
+            float o = w * s_r[t * XL + c];
+            if (REM) {
+                xw[t] = w * s_u[t * XL + c];
+#pragma unroll
+                for (int i = 0; 4 * i < t; ++i) chunk_take(xw[t], row4(0, t, i), xw, i, t, -1.0f);
+#pragma unroll
+                for (int i = 0; 4 * i <= t; ++i) chunk_take(o, row4(kR, t, i), xw, i, t + 1, -1.0f);
+                s_u[t * XL + c] = xw[t];
+            }
+            s_r[t * XL + c] = o;
+            s_k[t * YL + c] *= s_w[(kChunk - 1) * kDecayLd + t + 1];
+        }
+        out[chunk_key_floats(REM, DK) - DK + c] = s_w[(kChunk - 1) * kDecayLd];
+    }
+    asm volatile("" ::: "memory");               // the products are read again: kept for both loops they do not fit the registers (DK 128)
+    float* cols = out + chunk_key_floats(REM, DK);
+    for (int j = j_first; j < n_cols; j += 128) {
+        if (!EARLY || j != j_first) chunk_values(A, t0 + r0, n, h, j, v);
+        chunk_value_parts<REM>(cols, j, v);
+        float* to = cols + (j / kChunkCols) * chunk_col_floats(REM) + j % kChunkCols;
+#pragma unroll
+        for (int t = 0; t < kChunk; ++t) {
+            if (t % 4 == 0) asm volatile("" ::: "memory");      // (all rows read ahead would not fit either)
+            float o = 0.0f;
+            if (REM) {
+                float seen = 0.0f;
+#pragma unroll
+                for (int i = 0; 4 * i < t; ++i) chunk_take(seen, row4(0, t, i), v, i, t, 1.0f);
+                to[chunk_place(t) * kChunkCols] = seen;
+                v[t] -= seen;                    // what the token writes
+            }
+#pragma unroll
+            for (int i = 0; 4 * i <= t; ++i) chunk_take(o, row4(kR, t, i), v, i, t + 1, 1.0f);
+            to[(REM ? kChunk + t : t) * kChunkCols] = o;
+        }
+    }
+    __syncthreads();
+    chunk_fragments<DK, REM>(out, s_u, s_r, s_k, s_k, -1.0f);
 }
 
 struct ChunkArgs {
@@ -438,11 +660,12 @@ __host__ __device__ constexpr size_t chunk_smem(bool removes, int DK, int NT) {
 // Warps 0 .. NW - 1 carry the state from chunk to chunk, DK / NW channels each; warps NW .. 2 NW - 1 do for the same channels what that chain need not wait for
 // -- V's writes of the next chunk, the outputs of this one --; the last warp copies records.  NT blocks of eight columns.
 template <int DK, bool REM, int NT>
-__global__ void __launch_bounds__(chunk_warps(DK) * 64 + 32, DK <= 64 ? 2 : 1) chunk_scan_kernel(const ChunkArgs A, float* state_pool, float* __restrict__ o_raw) {
+__global__ void __launch_bounds__(chunk_warps(DK) * 64 + 32, DK <= 32 ? 4 : DK <= 64 ? 2 : 1) chunk_scan_kernel(const ChunkArgs A, float* state_pool, float* __restrict__ o_raw) {
     dep_wait();
     dep_go();
-    constexpr int NW = chunk_warps(DK), CW = DK / NW, MT = CW / 16, KS = CW / 8, NB = chunk_ring(DK), KF = chunk_key_floats(REM, DK), CF = chunk_col_floats(REM);
-    constexpr int MX = REM ? 2 : 1, ROWS = chunk_rows(REM), CB = kChunkCols, SH = kChunk * CB, SLOT = KF + NT * CF;
+    constexpr int NW = chunk_warps(DK), CW = DK / NW, MT = CW / 16, KS = CW / 16, NB = chunk_ring(DK), KF = chunk_key_floats(REM, DK), CF = chunk_col_floats(REM);
+    constexpr int MX = REM ? 2 : 1, CB = kChunkCols, SH = kChunk * CB, SLOT = KF + NT * CF, FR = chunk_frag(DK), YF = DK / 16 * MX * FR;
+    constexpr bool SPLIT = chunk_split(DK);
     extern __shared__ __align__(16) float sh[];
     __shared__ uint64_t full[NB], empty[NB];
     float* state = sh + NB * SLOT;                      // [2][NT][DK][CB]: the state before a chunk, on its way from result to operand
@@ -483,14 +706,17 @@ __global__ void __launch_bounds__(chunk_warps(DK) * 64 + 32, DK <= 64 ? 2 : 1) c
         return;
     }
     auto all_barrier = [&] { asm volatile("bar.sync 1, %0;" ::"n"(NW * 64) : "memory"); };
-    // operand fragments of the state before a chunk, this warp's channels
+    // operands whose rows lie in the order of chunk_place: of the state before a chunk, this warp's channels
     auto state_parts = [&](const float* at, PartsB (&sb)[KS]) {
 #pragma unroll
-        for (int k = 0; k < KS; ++k) sb[k].set(at[(8 * k + q) * CB + gq], at[(8 * k + q + 4) * CB + gq]);
+        for (int k = 0; k < KS; ++k)
+#pragma unroll
+            for (int x = 0; x < 2; ++x) sb[k].set(x, at[(16 * k + 8 * x + q) * CB + gq], at[(16 * k + 8 * x + 4 + q) * CB + gq]);
     };
-    auto put_share = [&](float* to, const float (&sum)[4]) {
-        *reinterpret_cast<float2*>(to + gq * CB + 2 * q) = make_float2(sum[0], sum[1]);
-        *reinterpret_cast<float2*>(to + (gq + 8) * CB + 2 * q) = make_float2(sum[2], sum[3]);
+    const int g_at = chunk_place(gq);
+    auto put_share = [&](float* to, int row, const float (&sum)[4]) {
+        *reinterpret_cast<float2*>(to + row * CB + 2 * q) = make_float2(sum[0], sum[1]);
+        *reinterpret_cast<float2*>(to + (row + 8) * CB + 2 * q) = make_float2(sum[2], sum[3]);
     };
     int b = 0;                                          // the chunk's slot in the ring, and the parity of its round
     uint32_t parity = 0;
@@ -499,19 +725,17 @@ __global__ void __launch_bounds__(chunk_warps(DK) * 64 + 32, DK <= 64 ? 2 : 1) c
     };
     if (role == 1) {
         auto make_writes = [&](const float* R, float* to) {
+            PartsB vb[NT][1];
+#pragma unroll
+            for (int n = 0; n < NT; ++n) vb[n][0].load(R + KF + n * CF + MX * SH, lane);
 #pragma unroll
             for (int m = 0; m < MT; ++m) {
-                PartsA y[2];
-#pragma unroll
-                for (int k = 0; k < 2; ++k) y[k].load(R + ROWS * DK + ((warp * MT + m) * 2 * MX + k) * 128, lane);
+                PartsA y[1];
+                y[0].load<SPLIT>(R + YF + (warp * MT + m) * MX * FR, lane);
 #pragma unroll
                 for (int n = 0; n < NT; ++n) {
-                    const float* V = R + KF + n * CF + MX * SH;
-                    PartsB vb[2];
-#pragma unroll
-                    for (int k = 0; k < 2; ++k) vb[k].set(V[(8 * k + q) * CB + gq], V[(8 * k + q + 4) * CB + gq]);
                     float sum[4];
-                    mma_sum<2>(sum, y, vb);
+                    mma_sum<1>(sum, y, vb[n]);
                     reinterpret_cast<float4*>(to + ((warp * NT + n) * MT + m) * 128)[lane] = make_float4(sum[0], sum[1], sum[2], sum[3]);
                 }
             }
@@ -526,7 +750,7 @@ __global__ void __launch_bounds__(chunk_warps(DK) * 64 + 32, DK <= 64 ? 2 : 1) c
             const int now = b;
             PartsA X[KS];
 #pragma unroll
-            for (int k = 0; k < KS; ++k) X[k].load(R + ((warp * KS + k) * MX + MX - 1) * 128, lane);
+            for (int k = 0; k < KS; ++k) X[k].load<SPLIT>(R + ((warp * KS + k) * MX + MX - 1) * FR, lane);
             all_barrier();                               // the state before chunk i is there, V's writes of chunk i are
             float* part = share_o + (i & 1) * NT * NW * SH;
 #pragma unroll
@@ -535,16 +759,17 @@ __global__ void __launch_bounds__(chunk_warps(DK) * 64 + 32, DK <= 64 ? 2 : 1) c
                 state_parts(state + ((i & 1) * NT + n) * DK * CB + c0 * CB, sb);
                 float sum[4];
                 mma_sum<KS>(sum, X, sb);
-                put_share(part + (n * NW + warp) * SH, sum);
+                put_share(part + (n * NW + warp) * SH, gq, sum);
             }
             asm volatile("bar.sync 2, %0;" ::"n"(NW * 32) : "memory");
 #pragma unroll
             for (int n = 0; n < NT; ++n)
 #pragma unroll
                 for (int x = first; x < SH; x += NW * 32) {
-                    float o = R[KF + n * CF + (MX - 1) * SH + x];
+                    float p[NW];
 #pragma unroll
-                    for (int p = 0; p < NW; ++p) o += part[(n * NW + p) * SH + x];
+                    for (int w = 0; w < NW; ++w) p[w] = part[(n * NW + w) * SH + x];
+                    const float o = (NW == 4 ? (p[0] + p[1]) + (p[NW - 2] + p[NW - 1]) : p[0] + p[NW - 1]) + R[KF + n * CF + (MX - 1) * SH + x];
                     const int t = t0 + i * kChunk + x / CB, j = j0 + n * CB + x % CB;
                     if (t < t1 && j < columns) (j < dv ? o_raw[((size_t)t * A.H + h) * dv + j] : A.unit_out[(size_t)t * A.H + h]) = o * A.q_scale;
                 }
@@ -576,20 +801,20 @@ __global__ void __launch_bounds__(chunk_warps(DK) * 64 + 32, DK <= 64 ? 2 : 1) c
     auto load_x = [&](const float* R) {
         if (REM) {
 #pragma unroll
-            for (int k = 0; k < KS; ++k) X[k].load(R + (warp * KS + k) * MX * 128, lane);
+            for (int k = 0; k < KS; ++k) X[k].load<SPLIT>(R + (warp * KS + k) * MX * FR, lane);
         }
     };
     umma::bar_wait(&full[0], 0);
     load_x(sh);
     for (int i = 0; i < chunks; ++i) {
-        const float *R = sh + b * SLOT, *W = R + 2 * ROWS * DK + c0;
+        const float *R = sh + b * SLOT, *W = R + KF - DK + c0;
         const int now = b;
         float *at = state + (i & 1) * NT * DK * CB + c0 * CB, *part = share_s + (i & 1) * NT * NW * SH;
 #pragma unroll
         for (int n = 0; n < NT; ++n)
 #pragma unroll
             for (int m = 0; m < MT; ++m) {
-                float* to = at + n * DK * CB + (16 * m + gq) * CB + 2 * q;
+                float* to = at + n * DK * CB + (16 * m + g_at) * CB + 2 * q;
                 *reinterpret_cast<float2*>(to) = make_float2(S[n][m][0], S[n][m][1]);
                 *reinterpret_cast<float2*>(to + 8 * CB) = make_float2(S[n][m][2], S[n][m][3]);
             }
@@ -601,7 +826,7 @@ __global__ void __launch_bounds__(chunk_warps(DK) * 64 + 32, DK <= 64 ? 2 : 1) c
                 state_parts(at + n * DK * CB, sb);
                 float sum[4];
                 mma_sum<KS>(sum, X, sb);
-                put_share(part + (n * NW + warp) * SH, sum);
+                put_share(part + (n * NW + warp) * SH, g_at, sum);
             }
         }
         // what does not wait for the other warps' shares
@@ -613,12 +838,10 @@ __global__ void __launch_bounds__(chunk_warps(DK) * 64 + 32, DK <= 64 ? 2 : 1) c
 #pragma unroll
                 for (int e = 0; e < 4; ++e) S[n][m][e] *= e < 2 ? w0 : w1;
         }
-        PartsA Y[REM ? MT : 1][2];
+        PartsA Y[REM ? MT : 1][1];
         if (REM) {
 #pragma unroll
-            for (int m = 0; m < MT; ++m)
-#pragma unroll
-                for (int k = 0; k < 2; ++k) Y[m][k].load(R + ROWS * DK + ((warp * MT + m) * 2 * MX + 2 + k) * 128, lane);
+            for (int m = 0; m < MT; ++m) Y[m][0].load<SPLIT>(R + YF + ((warp * MT + m) * MX + MX - 1) * FR, lane);
         }
         next_slot();
         if (i + 1 < chunks) {
@@ -629,7 +852,7 @@ __global__ void __launch_bounds__(chunk_warps(DK) * 64 + 32, DK <= 64 ? 2 : 1) c
 #pragma unroll
         for (int n = 0; n < NT; ++n) {
             if (REM) {
-                PartsB seen[2];
+                PartsB seen[1];
 #pragma unroll
                 for (int k = 0; k < 2; ++k) {
                     float z[2];
@@ -641,12 +864,12 @@ __global__ void __launch_bounds__(chunk_warps(DK) * 64 + 32, DK <= 64 ? 2 : 1) c
                         for (int w = 0; w < NW; ++w) p[w] = part[(n * NW + w) * SH + e];
                         z[x] = (NW == 4 ? (p[0] + p[1]) + (p[NW - 2] + p[NW - 1]) : p[0] + p[NW - 1]) + R[KF + n * CF + e];
                     }
-                    seen[k].set(z[0], z[1]);
+                    seen[0].set(k, z[0], z[1]);
                 }
 #pragma unroll
                 for (int m = 0; m < MT; ++m) {
                     float sum[4];
-                    mma_sum<2>(sum, Y[m], seen);
+                    mma_sum<1>(sum, Y[m], seen);
 #pragma unroll
                     for (int e = 0; e < 4; ++e) S[n][m][e] += sum[e];
                 }

@@ -2727,11 +2727,10 @@ static cudaError_t chunk_attributes() {
         if (e == cudaSuccess) e = allow(chunk_scan_kernel<DK, true, 2>, chunk_smem(true, DK, 2));
         if (e == cudaSuccess) e = allow(chunk_scan_kernel<DK, false, 2>, chunk_smem(false, DK, 2));
     }
-    const size_t with = chunk_prep_floats(true, DK) * sizeof(float), without = chunk_prep_floats(false, DK) * sizeof(float);
-    if (e == cudaSuccess) e = allow(chunk_prep_kernel<kScanGeneralDelta, DK>, with);
-    if (e == cudaSuccess) e = allow(chunk_prep_kernel<kScanGatedDelta, DK>, with);
-    if (e == cudaSuccess) e = allow(chunk_prep_kernel<kScanChannelDecay, DK>, without);
-    if (e == cudaSuccess) e = allow(chunk_prep_kernel<kScanHeadDecay, DK>, without);
+    if (e == cudaSuccess) e = allow(chunk_prep_kernel<kScanGeneralDelta, DK>, chunk_prep_floats(kScanGeneralDelta, DK) * sizeof(float));
+    if (e == cudaSuccess) e = allow(chunk_prep_kernel<kScanChannelDecay, DK>, chunk_prep_floats(kScanChannelDecay, DK) * sizeof(float));
+    if (e == cudaSuccess) e = allow(chunk_prep_head_kernel<kScanGatedDelta, DK>, chunk_prep_floats(kScanGatedDelta, DK) * sizeof(float));
+    if (e == cudaSuccess) e = allow(chunk_prep_head_kernel<kScanHeadDecay, DK>, chunk_prep_floats(kScanHeadDecay, DK) * sizeof(float));
     return e;
 }
 static constexpr int flash_smem_bytes(int DK, int DV, bool vk, int maps = 1) { return 2 * 64 * (maps * (DK + 8) + (vk ? 0 : DV + 8)) * (int)sizeof(bf16); }
@@ -3263,7 +3262,10 @@ static cudaError_t launch_chunks_sized(SmolLm* m, ChunkSource Q, ChunkArgs A, in
     constexpr bool REM = scan_removes(KIND);
     float* rec = reinterpret_cast<float*>(m->ws + m->o_rec);
     Q.cap = A.cap = m->cfg.max_step_tokens / kChunk + m->cfg.max_step_seqs + 1;
-    pdl_launch(chunk_prep_kernel<KIND, DK>, dim3((max_n + kChunk - 1) / kChunk, n_seqs, Q.H), 128, chunk_prep_floats(REM, DK) * sizeof(float), st, Q, rec);
+    const dim3 grid((max_n + kChunk - 1) / kChunk, n_seqs, Q.H);
+    constexpr size_t prep_smem = chunk_prep_floats(KIND, DK) * sizeof(float);
+    if constexpr (KIND == kScanGeneralDelta || KIND == kScanChannelDecay) pdl_launch(chunk_prep_kernel<KIND, DK>, grid, 128, prep_smem, st, Q, rec);
+    else pdl_launch(chunk_prep_head_kernel<KIND, DK>, grid, 128, prep_smem, st, Q, rec);
     A.rec = rec;
     // Above 64 channels a block has an SM to itself.  Where single blocks of columns would not all run at once, it takes two, whose products share the
     // records' fragments (12 heads of 128, 1801 tokens: 140 us for 96 blocks of two, 144 for 192 single ones with half the ring, two to an SM; 3 x 12 heads of

@@ -34,7 +34,6 @@ namespace lm {
 
 constexpr int kChunk = 16;               // tokens of a chunk
 constexpr int kChunkCols = 8;            // value columns of a block
-constexpr int kChunkMinTokens = 256, kChunkMinTokensWide = 144, kChunkMinTokensWideGroups = 208;      // the longest sequence of a step, up to 64 channels and above (beside group_scan_kernel): shorter ones go four at a time
 enum { kScanGeneralDelta = 0, kScanChannelDecay = 1, kScanHeadDecay = 2, kScanGatedDelta = 3 };
 constexpr bool scan_removes(int kind) { return kind == kScanGeneralDelta || kind == kScanGatedDelta; }      // has a and u
 __host__ __device__ constexpr int chunk_pad(int d) { return d <= 32 ? 32 : d <= 64 ? 64 : d <= 128 ? 128 : 256; }

@@ -3247,15 +3247,28 @@ static cudaError_t launch_quad(SmolLm* m, const QuadSource& Q, const QuadArgs& A
     }
 }
 
-// The scan by chunks where some sequence is long enough; shorter ones lose by the records what the chain saves.  One layer's recurrence as a whole, by chunks and
-// four tokens at a time: generalized delta rule, 12 x 64 x 64, 128 / 260 / 1100 tokens 37 / 39 / 84 us against 41 / 49 / 146, 4 x 40 and 4 x 150 40 and 48 against
-// 31 and 48; 12 x 128 x 128, 128 / 260 / 1100 69 / 68 / 158 against 86 / 96 / 282; gated linear recurrence, 128 / 300 / 1100 26 / 27 / 63 against 26 / 36 / 95.
-static bool chunks_pay(int n_seqs, int n_tokens, int max_n, int d) { return max_n >= (d <= 64 ? kChunkMinTokens : kChunkMinTokensWide) && n_tokens >= kQuadMeanTokens * n_seqs; }
-// The same for the gated delta rule and the mLSTM, whose other form has no records to make: with many heads of up to 64 channels the SMs are full either way and
-// that form has less to do (gated delta rule, 12 heads, 1 / 4 / 7 / 16 x 260 tokens: 35 / 54 / 82 / 162 us against 45 / 60 / 78 / 147; 3 x 1000: 128 against 155; heads of
-// 128, 1 x 150 / 1 x 260 / 16 x 260: 80 / 61 / 351 against 76 / 74 / 391).
-static bool chunks_pay_beside_groups(int n_seqs, int heads, int n_tokens, int max_n, int d) {
-    return (d <= 64 ? max_n >= kChunkMinTokens && max_n >= 5 * n_seqs * heads : max_n >= kChunkMinTokensWideGroups) && n_tokens >= kQuadMeanTokens * n_seqs;
+// The scan by chunks, or one of those that go four tokens at a time.  By chunks a sequence must be long enough to pay for its records, and a step's blocks of eight
+// columns must not be many more than the SMs run at once: then either form fills them, and the one with less to do wins -- the more so the fewer channels a head has,
+// since chunks pad to 32.  Times by chunks / four at a time, records included, over 1 to 64 heads, 1 to 16 sequences, 144 to 1000 tokens (us):
+//   generalized delta rule, 12 x 64 x 64, 1 x 260 / 3 x 1000 tokens: 25 / 35, 103 / 172; 8 x 128 x 128, 144 / 160 tokens 1.04 / 0.95 of the other's time;
+//     16 channels, 222 / 256 blocks 0.93 / 1.03
+//   decay per channel or head, 64 x 64: 288 / 384 blocks 0.95 / 1.13; 48 x 24: 222 / 288 blocks 1.00 / 1.10; 32: 222 / 296 blocks 0.96 / 1.05; 16: 148 / 192 blocks 0.99 / 1.08;
+//     12 heads of 96, 176 / 208 tokens 1.07 / 0.96
+//   gated delta rule, 64 x 64: 512 / 768 blocks 0.95 / 1.07; 48 x 24: 288 / 384 blocks 0.87 / 1.13; 32: 384 / 480 blocks 0.94 / 1.11; 16: 148 / 192 blocks 0.92 / 1.08; heads of 128, 176 / 208
+//     tokens 1.06 / 0.99; of 256, 256 / 320 tokens 1.03 / 0.96, but 384 blocks, of which two at a time fill one SM and a third of them again, 1.20 / 1.14
+//   mLSTM, 64 x 64: 0.40 to 0.95 everywhere; 48 x 24: 612 / 768 blocks 0.79 / 1.06; 32: 1224 blocks 0.99; 16: 288 / 384 blocks 0.92 / 1.08
+static bool chunks_pay(int kind, bool unit, int n_seqs, int heads, int n_tokens, int max_n, int d, int columns, int n_sms) {
+    const int min_n = d <= 64 ? 256 : kind == kScanGeneralDelta ? 160 : kind == kScanGatedDelta && d > 128 ? 320 : 208;
+    if (max_n < min_n || n_tokens < kQuadMeanTokens * n_seqs) return false;
+    const double blocks = (double)n_seqs * heads * chunk_blocks(columns) / n_sms, any = 1e30;      // per SM
+    double most = any;
+    if (kind == kScanGeneralDelta) most = d <= 16 ? 1.5 : any;
+    else if (kind == kScanGatedDelta) {
+        if (d > 128) return blocks <= 2.0 || blocks >= 5.0;
+        most = d <= 16 ? 1.0 : d < 64 ? 2.0 : d == 64 ? 3.5 : any;
+    } else if (unit) most = d <= 16 ? 2.0 : d < 64 ? 4.0 : any;
+    else most = d <= 16 ? 1.0 : d < 64 ? 1.5 : d == 64 ? 2.0 : any;
+    return blocks <= most;
 }
 template <int KIND, int DK>
 static cudaError_t launch_chunks_sized(SmolLm* m, ChunkSource Q, ChunkArgs A, int n_seqs, int max_n, float* o_raw, cudaStream_t st, size_t min_smem) {
@@ -3304,7 +3317,7 @@ static cudaError_t launch_gla_scan(const GlaArgs& A, int n_seqs, const float* de
 // the scan over key sizes up to 256: the smallest built size that holds A.d
 static cudaError_t launch_gla_scan_any(SmolLm* m, const GlaArgs& A, int n_seqs, int n_tokens, int max_n, const float* dec, float* pool, float* o_raw, cudaStream_t st,
                                         size_t min_smem = 0) {
-    if (chunks_pay(n_seqs, n_tokens, max_n, A.d)) {
+    if (chunks_pay(A.head_decay ? kScanHeadDecay : kScanChannelDecay, false, n_seqs, A.H, n_tokens, max_n, A.d, A.dv, m->n_sms)) {
         const ChunkSource Q{A.H, A.qk_share, A.d, A.dv, A.dv, A.q_src, A.k_src, A.q_ld, A.k_ld, A.v_src, A.v_ld, dec, A.head_decay, A.head_step, A.head_ld, 1,
                             nullptr, nullptr, 0.0f, A.seq_start, 0};
         const ChunkArgs S{A.H, A.d, A.dv, nullptr, 0, A.q_scale, A.seq_start, A.seq_pos0, A.seq_slot, A.slot_floats, A.state_off, A.n_slots, A.err, nullptr, 0, ConvIo{}};
@@ -3336,7 +3349,7 @@ static cudaError_t launch_group_scan(const GroupScanArgs& A, int n_seqs, float* 
 template <bool DELTA>
 static cudaError_t launch_group_scan_any(SmolLm* m, const GroupScanArgs& A, float* pairs, int n_seqs, int n_tokens, int max_n, float* pool, float* o_raw, cudaStream_t st,
                                          size_t min_smem = 0) {
-    if (chunks_pay_beside_groups(n_seqs, A.H, n_tokens, max_n, A.d)) {
+    if (chunks_pay(DELTA ? kScanGatedDelta : kScanHeadDecay, A.unit_out != nullptr, n_seqs, A.H, n_tokens, max_n, A.d, A.dv + (A.unit_out ? 1 : 0), m->n_sms)) {
         const ChunkSource Q{A.H, A.H / A.G, A.d, A.dv, A.dv + (A.unit_out ? 1 : 0), A.q_src, A.k_src, A.q_ld, A.k_ld, A.v_src, A.v_ld, nullptr, A.head, A.head + 1, 2 * A.H, 2,
                             nullptr, nullptr, 0.0f, A.seq_start, 0};
         const ChunkArgs S{A.H, A.d, A.dv, nullptr, 0, A.q_scale, A.seq_start, A.seq_pos0, A.seq_slot, A.slot_floats, A.state_off, A.n_slots, A.err, A.unit_out, A.unit_off, A.conv};
@@ -4108,7 +4121,7 @@ static int step_impl(SmolLm* m, const SmolLmStep* s, cudaStream_t st) {
             A.rate_bias = L.rate_bias; A.decay_w2 = L.decay_w2; A.decay_bias = L.decay_bias; A.out_norm = L.out_norm;
             A.seq_start = s->seq_start; A.seq_pos0 = s->seq_pos0; A.seq_slot = s->seq_slot;
             A.slot_floats = m->slot_floats; A.state_off = R.state_off; A.n_slots = m->n_slots; A.err = err;
-            const bool chunks = chunks_pay(s->n_seqs, Tn, max_n, L.dim), quad = !chunks && quad_pays(s->n_seqs, Tn, max_n);
+            const bool chunks = chunks_pay(kScanGeneralDelta, false, s->n_seqs, L.heads, Tn, max_n, L.dim, L.dim, m->n_sms), quad = !chunks && quad_pays(s->n_seqs, Tn, max_n);
             float *u_to = chunks || quad ? nullptr : uk, *au_to = chunks || quad ? nullptr : auk;
             const size_t prep_smem = (size_t)(L.rank + L.heads) * sizeof(float);
             const int slices = (L.heads * L.dim + 127) / 128;

@@ -67,3 +67,27 @@ def test_rows_take_nothing_from_keys_they_do_not_see(name):
         got = logits(toks[:at] + [BAD] + toks[at + 1:])
         assert torch.equal(got[:at], want[:at])
         assert not bool(got[at].isfinite().any())
+
+
+@pytest.mark.parametrize("window", [20, 32, 37])
+def test_window_rows_do_not_depend_on_their_block(window):
+    """The same bits whatever the portions a prompt comes in, and so wherever a row lies in its block, and for both block heights (beside three long ones)."""
+    cfg = su.config([su.layer(su.left(heads=12, kv_heads=4, dim=24, vdim=20, window=window))], vocab=61, width=48)
+    model, orc, _ = su.engine_and_oracle(cfg, seed=13, max_tokens=4096, max_seqs=4, page_size=16, max_step_tokens=1024)
+    toks, beside = pu.tokens(231, 61, window), pu.tokens(231, 61, 1)
+
+    def logits(sizes, others):
+        seqs, at, out = [model.open_sequence() for _ in range(1 + others)], 0, []
+        for n in sizes:
+            got = model.forward([(seqs[0], toks[at:at + n], list(range(n)))] + [(s, beside[at:at + n], []) for s in seqs[1:]]).clone()
+            out.append(got)
+            at += n
+        for s in seqs:
+            model.close_sequence(s)
+        return torch.cat(out)
+
+    want = logits([231], 0)
+    assert pu.rel_err(want, orc.forward(toks)) < pu.TOL[torch.float32]
+    for sizes, others in (([9, 222], 0), ([103, 11, 117], 0), ([231], 3), ([50, 181], 3)):
+        assert torch.equal(logits(sizes, others), want)
+    model.check_device_errors()

@@ -1,4 +1,5 @@
-"""The recurrences' scan by chunks of sixteen tokens (prompts of 256 tokens and more, of 144 with more than 64 key channels)."""
+"""The recurrences' scan by chunks of sixteen tokens (prompts of 256 tokens and more; with more than 64 key channels of 160 or 208, the gated delta rule above
+128 channels of 320)."""
 from __future__ import annotations
 
 import pytest
@@ -28,8 +29,8 @@ def test_scan_by_chunks(dim, form):
     """Padded key channels, last chunks of any size, a sequence shorter than a chunk and a single token beside long ones; then a second long portion on the
     state left behind, then a short one that the four-token scan takes on; against the oracles."""
     cfg, make = layers_of(dim)[form]
-    lens, second, third = (273, 256, 19, 1), (257, 3, 260, 31), (20, 1, 5, 33)
-    model, orc, _ = make(cfg, seed=4, max_tokens=4096, max_seqs=4, page_size=16, max_step_tokens=640)
+    lens, second, third = ((273, 256, 19, 1), (257, 3, 260, 31), (20, 1, 5, 33)) if dim <= 128 else ((337, 320, 19, 1), (321, 3, 324, 31), (20, 1, 5, 33))
+    model, orc, _ = make(cfg, seed=4, max_tokens=4096, max_seqs=4, page_size=16, max_step_tokens=704)
     toks = [pu.tokens(a + b + c, 61, a) for a, b, c in zip(lens, second, third)]
     want = [orc.forward(t) for t in toks]
     seqs, at = [model.open_sequence() for _ in lens], [0] * 4
@@ -47,7 +48,7 @@ def test_scan_by_chunks(dim, form):
     model.check_device_errors()
 
 
-@pytest.mark.parametrize("n", [150, 161])
+@pytest.mark.parametrize("n", [215, 225])
 def test_two_blocks_of_columns_per_block(n):
     """More blocks of columns than SMs above 64 channels: two per block of threads, the last one alone (13 blocks of columns of 12 heads)."""
     for cfg, make in ((pu.config([pu.delta(heads=12, dim=104, ff=0, rank=5)], vocab=61, width=48), pu.engine_and_oracle),
@@ -83,3 +84,22 @@ def test_tokens_take_nothing_from_later_ones_of_their_chunk(form):
 
 def spoil(w):
     w["embed"][60] = float("nan")
+
+
+def test_both_forms_on_either_side_of_the_rule():
+    """Sixteen channels take chunks while a step has few blocks of columns: one sequence by chunks, four together four tokens at a time, alike beyond rounding."""
+    for form in (1, 2, 3):
+        cfg, make = layers_of(16)[form]
+        wide = {"heads": 12, "vdim": 16}
+        layer = cfg["layers"][0]["mixer"]
+        (layer["right"] if "right" in layer else layer).update(wide, **({"kv_heads": 12} if "kv_heads" in layer else {}))
+        model, orc, _ = make(cfg, seed=8, max_tokens=8192, max_seqs=16, page_size=16, max_step_tokens=16 * 264)
+        toks = pu.tokens(264, 61, form)
+        want = orc.forward(toks)
+        for many in (1, 16):
+            seqs = [model.open_sequence() for _ in range(many)]
+            got = model.forward([(s, toks, list(range(264)) if s is seqs[-1] else []) for s in seqs]).clone()
+            assert pu.rel_err(got[1:], want[1:]) < TOL
+            for s in seqs:
+                model.close_sequence(s)
+        model.check_device_errors()

@@ -35,3 +35,17 @@ def test_ends_of_recurrences(vdim):
         got = model.forward([(seq, toks, list(range(37)))]).clone()
         model.close_sequence(seq)
         assert rel_err(got, orc.forward(toks)) < TOL[torch.float32]
+
+
+@pytest.mark.parametrize("width", [4, 128, 132, 764, 768, 1540, 2048])
+def test_a_row_does_not_depend_on_the_number_of_rows(width):
+    """A sequence alone, whose rows have a block each, and beside another, where they have a warp each: the same bits."""
+    cfg = config([attn(heads=1, kv_heads=1, dim=8, vdim=8, ff=16)], vocab=33, width=width)
+    model, _, _ = engine_and_oracle(cfg, seed=9, max_step_tokens=520)
+    toks, other = tokens(300, 33, width), tokens(215, 33, 1)
+    seqs = [model.open_sequence() for _ in range(3)]
+    alone = model.forward([(seqs[0], toks, list(range(300)))]).clone()
+    both = model.forward([(seqs[1], toks, list(range(300))), (seqs[2], other, list(range(215)))]).clone()      # all rows through the final norm as well
+    assert torch.equal(alone, both[:300])
+    for s in seqs:
+        model.close_sequence(s)

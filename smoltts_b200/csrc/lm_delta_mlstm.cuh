@@ -88,7 +88,7 @@ __global__ void __launch_bounds__(128) scan_pairs_kernel(const GroupScanArgs A, 
 }
 
 template <int DK, int VEC>
-__device__ __forceinline__ void group_scan_stage(const GroupScanArgs& A, float* buf, int c0, int n, int h, int j0, int nc) {
+__device__ __forceinline__ void group_scan_stage(const GroupScanArgs& A, float* buf, int c0, int n, int h, int j0, int nc, bool cleared) {
     constexpr int CB = gla_block_cols(DK), CH = group_scan_chunk(DK), PL = CH * DK;
     const int d = A.d, dq = d / VEC, ncq = (nc + VEC - 1) / VEC, g = h / (A.H / A.G);
     for (int idx = threadIdx.x; idx < n * dq; idx += blockDim.x) {
@@ -109,7 +109,7 @@ __device__ __forceinline__ void group_scan_stage(const GroupScanArgs& A, float* 
         cp_async_f<1>(sc + CH * kPairFloats + idx, A.head + ((size_t)(c0 + idx / 2) * A.H + h) * 2 + idx % 2);
     // The tokens that the last group lacks: their step is taken as 0, and 0 times what a buffer was left with need not be 0.  (Only a sequence's last
     // chunk of the step has any, in whichever buffer it lies; nothing reads these rows as real tokens afterwards.)
-    const int gap = (n + kScanGroup - 1) / kScanGroup * kScanGroup - n;
+    const int gap = cleared ? 0 : (n + kScanGroup - 1) / kScanGroup * kScanGroup - n;
     for (int i = threadIdx.x; i < gap * DK; i += blockDim.x) buf[n * DK + i] = buf[PL + n * DK + i] = 0.0f;
     for (int i = threadIdx.x; i < gap * CB; i += blockDim.x) buf[2 * PL + n * CB + i] = 0.0f;
     for (int i = threadIdx.x; i < gap * kPairFloats; i += blockDim.x) sc[n * kPairFloats + i] = 0.0f;
@@ -118,7 +118,6 @@ __device__ __forceinline__ void group_scan_stage(const GroupScanArgs& A, float* 
 template <int DK, bool DELTA>
 __global__ void __launch_bounds__(gla_block_cols(DK) * gla_lanes(DK)) group_scan_kernel(const GroupScanArgs A, float* state_pool, float* __restrict__ o_raw) {
     dep_wait();      // (launched plainly: nothing comes before it)
-    dep_go();
     constexpr int L = gla_lanes(DK), CB = gla_block_cols(DK), RV = DK / L / 4, CH = group_scan_chunk(DK), PL = CH * DK;
     constexpr int kBuf = group_scan_buf_floats(DK), GS = kScanGroup;
     static_assert(L >= GS && kBuf % 4 == 0, "a lane per token of a group stores its result; 16-byte buffers");
@@ -139,16 +138,14 @@ __global__ void __launch_bounds__(gla_block_cols(DK) * gla_lanes(DK)) group_scan
                      ((reinterpret_cast<uintptr_t>(A.q_src) | reinterpret_cast<uintptr_t>(A.k_src) | reinterpret_cast<uintptr_t>(A.v_src)) % 16 == 0);
     // Padded channels and columns stay zero for good; without any, nothing is cleared (a lone token pays for 17 000 zeros: 13.4 us for 5 tokens of
     // 12 x 128 x 128, 11.8 without).
-    if (d < DK || nc < CB || dvs > dv)
+    const bool clear = d < DK || nc < CB || dvs > dv;
+    if (clear)
         for (int i = threadIdx.x; i < 2 * kBuf; i += blockDim.x) sh[i] = 0.0f;
     if (dvs > dv && dv >= j0 && dv < j0 + CB) {                                 // ... and the unit column one
         __syncthreads();
         for (int i = threadIdx.x; i < 2 * CH; i += blockDim.x) sh[(i / CH) * kBuf + 2 * PL + (i % CH) * CB + dv - j0] = 1.0f;
     }
     __syncthreads();
-    if (vec) group_scan_stage<DK, 4>(A, sh, t0, min(CH, t1 - t0), h, j0, nc);
-    else group_scan_stage<DK, 1>(A, sh, t0, min(CH, t1 - t0), h, j0, nc);
-    cp_async_commit();
     // element i of this thread's column: st[i * st_ld]
     const bool unit = j == dv && dvs > dv;
     float* st = state_pool + (size_t)slot * A.slot_floats + (unit ? A.unit_off + (size_t)h * d : A.state_off + (size_t)h * d * dv + j);
@@ -160,8 +157,12 @@ __global__ void __launch_bounds__(gla_block_cols(DK) * gla_lanes(DK)) group_scan
 #pragma unroll
         for (int x = 0; x < 4; ++x) {
             const int i = 4 * (e * L + q) + x;
-            S[e][x] = (!fresh && i < d && j < dvs) ? st[(size_t)i * st_ld] : 0.0f;
+            S[e][x] = (!fresh && i < d && j < dvs) ? st[(size_t)i * st_ld] : 0.0f;      // on their way while the copies are issued
         }
+    dep_go();
+    if (vec) group_scan_stage<DK, 4>(A, sh, t0, min(CH, t1 - t0), h, j0, nc, clear);
+    else group_scan_stage<DK, 1>(A, sh, t0, min(CH, t1 - t0), h, j0, nc, clear);
+    cp_async_commit();
     if (A.conv.taps > 1)
         for (int c = part * blockDim.x + threadIdx.x; c < A.conv.ch; c += A.H * NS * blockDim.x) conv_state_update(A.conv, state_pool, seq, c);
     // this lane's output: token q of a group (q < GS)
@@ -174,8 +175,8 @@ __global__ void __launch_bounds__(gla_block_cols(DK) * gla_lanes(DK)) group_scan
         __syncthreads();                          // this chunk has landed; every thread is done with the other buffer
         if (c0 + CH < t1) {
             const int nn = min(CH, t1 - c0 - CH);
-            if (vec) group_scan_stage<DK, 4>(A, sh + (cur ^ 1) * kBuf, c0 + CH, nn, h, j0, nc);
-            else group_scan_stage<DK, 1>(A, sh + (cur ^ 1) * kBuf, c0 + CH, nn, h, j0, nc);
+            if (vec) group_scan_stage<DK, 4>(A, sh + (cur ^ 1) * kBuf, c0 + CH, nn, h, j0, nc, false);
+            else group_scan_stage<DK, 1>(A, sh + (cur ^ 1) * kBuf, c0 + CH, nn, h, j0, nc, false);
             cp_async_commit();
         }
         const float* b = sh + cur * kBuf;

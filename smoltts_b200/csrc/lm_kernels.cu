@@ -1250,7 +1250,7 @@ __global__ void __launch_bounds__(kRowsWarps * 32) attn_rows_kernel(const AttnAr
     const bool kvec = (A.d * sizeof(T)) % 16 == 0 && (A.k_ld * sizeof(T)) % 16 == 0 && (A.k_off * sizeof(T)) % 16 == 0;
     const bool vvec = (A.dv * sizeof(T)) % 16 == 0 && (A.v_ld * sizeof(T)) % 16 == 0 && (A.v_off * sizeof(T)) % 16 == 0;
     const int kchunks = kvec ? A.d / kPad : A.d, vchunks = A.v_in_k ? 0 : vvec ? A.dv / kPad : A.dv;
-    const int j_first = attn_first_key(A, pos0), j_last = pos0 + rows - 1;
+    const int j_first = attn_first_key(A, pos0), j_last = pos0 + rows - 1;      // keys that some row of the block sees
     float sum[R][MAXV];                    // the maps' joined results
 #pragma unroll
     for (int map = 0; map < MAPS; ++map) {
@@ -1265,18 +1265,19 @@ __global__ void __launch_bounds__(kRowsWarps * 32) attn_rows_kernel(const AttnAr
 #pragma unroll
             for (int e = 0; e < MAXV; ++e) o[i][e] = 0.0f;
         }
-        for (int j0 = j_first; j0 <= j_last; j0 += KEYS) {
-            const int cnt = min(KEYS, j_last - j0 + 1);
+        // Tiles begin at multiples of KEYS: a row's sums depend neither on its place in the block nor on what the block's first row sees of a window.
+        for (int j0 = j_first / KEYS * KEYS; j0 <= j_last; j0 += KEYS) {
+            const int skip = max(0, j_first - j0), cnt = min(KEYS, j_last - j0 + 1);
             __syncthreads();
             {
-                const int jr = min(j0 + lane, j_last), page = bt[jr / A.page_size], place = jr % A.page_size;
+                const int jr = min(max(j0 + lane, j_first), j_last), page = bt[jr / A.page_size], place = jr % A.page_size;      // (pages in front of the window may be gone)
                 for (int c = lane; c - lane < kchunks + vchunks; c += 32) {
                     const bool key = c < kchunks, live = c < kchunks + vchunks;
                     const int piece = key ? c : c - kchunks, step = (key ? kvec : vvec) ? kPad : 1, ld = key ? A.k_ld : A.v_ld, dst_ld = key ? ldk : ldv;
                     const T* src0 = pool + (key ? A.k_off + (size_t)(g * MAPS + map) * A.page_size * ld : A.v_off + (size_t)g * A.page_size * ld) + piece * step;
                     T* dst0 = (key ? Ks : Vs) + piece * step;
 #pragma unroll 4
-                    for (int r = warp; r < cnt; r += kRowsWarps) {
+                    for (int r = skip + warp; r < cnt; r += kRowsWarps) {
                         const int pg = __shfl_sync(0xffffffffu, page, r), at = __shfl_sync(0xffffffffu, place, r);
                         const T* src = src0 + (size_t)pg * A.page_elems + (size_t)at * ld;
                         T* dst = dst0 + r * dst_ld;
@@ -1345,7 +1346,7 @@ __global__ void __launch_bounds__(kRowsWarps * 32) attn_rows_kernel(const AttnAr
                         if (every || (jj >= lo[i] && jj <= hi[i])) o[i][e] = fmaf(p[i], v, o[i][e]);
                 }
             };
-            for (int jj = 0; jj < min(all_lo, cnt); ++jj) add(jj, false);
+            for (int jj = skip; jj < min(all_lo, cnt); ++jj) add(jj, false);
 #pragma unroll 4
             for (int jj = all_lo; jj <= all_hi; ++jj) add(jj, true);
             for (int jj = max(all_lo, all_hi + 1); jj < cnt; ++jj) add(jj, false);

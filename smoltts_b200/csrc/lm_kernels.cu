@@ -57,17 +57,25 @@ __device__ __forceinline__ float block_sum(float v, float* red) {
 }
 
 // A row in registers as 16-byte pieces, V per thread.  LONE: the row has a block of its own, a piece per thread, and the warps' sums meet behind one barrier;
-// otherwise the row has one warp and needs none.
+// otherwise the row has one warp and needs none.  Both add in the same order -- the sums of 32 pieces side by side, one after the other --, so a row's bits do not
+// depend on how many rows a step has.
 template <int V, bool LONE>
 struct RowPieces {
     __device__ static __forceinline__ int row() { return LONE ? (int)blockIdx.x : (int)(blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)); }
     __device__ static __forceinline__ int column(int i) { return 4 * (LONE ? (int)threadIdx.x : (int)(threadIdx.x & 31) + 32 * i); }
     // `red`: 16 floats that no other sum of the kernel uses
-    __device__ static __forceinline__ float sum(float v, float* red) {
-        v = warp_sum(v);
-        if (!LONE) return v;
+    __device__ static __forceinline__ float sum(float (&v)[V], float* red) {
+#pragma unroll
+        for (int x = 16; x > 0; x >>= 1)
+#pragma unroll
+            for (int i = 0; i < V; ++i) v[i] += __shfl_xor_sync(0xffffffffu, v[i], x);
+        if (!LONE) {
+#pragma unroll
+            for (int i = 1; i < V; ++i) v[0] += v[i];
+            return v[0];
+        }
         const int nw = (int)blockDim.x >> 5;
-        if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
+        if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v[0];
         __syncthreads();
         float t = red[0];
         for (int i = 1; i < nw; ++i) t += red[i];
@@ -133,14 +141,14 @@ __global__ void __launch_bounds__(LONE ? 512 : 128) embed_norm_vec_kernel(const 
     const T* e = embed + (size_t)tok * D;
     const size_t o = (size_t)t * D;
     float4 v[V];
-    float ss = 0.0f;
+    float ss[V];
 #pragma unroll
     for (int i = 0; i < V; ++i) v[i] = R::column(i) < D ? load4(e + R::column(i)) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
 #pragma unroll
     for (int i = 0; i < V; ++i) {
         v[i] = make_float4(v[i].x * scale, v[i].y * scale, v[i].z * scale, v[i].w * scale);
         if (R::column(i) < D) *reinterpret_cast<float4*>(x + o + R::column(i)) = v[i];
-        ss += squares(v[i]);
+        ss[i] = squares(v[i]);
     }
     const float r = 1.0f / sqrtf(R::sum(ss, red) / (float)D + eps);
 #pragma unroll
@@ -175,11 +183,11 @@ __global__ void __launch_bounds__(LONE ? 512 : 128) norm_rows_vec_kernel(const f
     if (r >= n_rows) return;
     const float* xr = x + (size_t)(rows ? rows[r] : r) * D;
     float4 v[V];
-    float ss = 0.0f;
+    float ss[V];
 #pragma unroll
     for (int i = 0; i < V; ++i) v[i] = R::column(i) < D ? load4(xr + R::column(i)) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
 #pragma unroll
-    for (int i = 0; i < V; ++i) ss += squares(v[i]);
+    for (int i = 0; i < V; ++i) ss[i] = squares(v[i]);
     const float f = 1.0f / sqrtf(R::sum(ss, red) / (float)D + eps);
 #pragma unroll
     for (int i = 0; i < V; ++i)
@@ -302,7 +310,7 @@ __global__ void __launch_bounds__(LONE ? 512 : 128) add_norm_vec_kernel(float* _
     if (t >= rows) return;
     const size_t o = (size_t)t * D;
     float4 xv[V], yv[V];
-    float ss = 0.0f;
+    float ss[V], s2[V];
 #pragma unroll
     for (int i = 0; i < V; ++i) {
         const int c = R::column(i);
@@ -332,12 +340,12 @@ __global__ void __launch_bounds__(LONE ? 512 : 128) add_norm_vec_kernel(float* _
         }
     }
 #pragma unroll
-    for (int i = 0; i < V; ++i) ss += squares(yv[i]);
+    for (int i = 0; i < V; ++i) ss[i] = squares(yv[i]);
     const float r = 1.0f / sqrtf(R::sum(ss, red[0]) / (float)D + eps);
-    float s2 = 0.0f;
 #pragma unroll
     for (int i = 0; i < V; ++i) {
         const int c = R::column(i);
+        s2[i] = 0.0f;
         if (c >= D) continue;
         const float4 l = LONE ? early[0] : load4(ls + c), b = LONE ? early[1] : load4(wb + c), u = yv[i];
         float4& v = xv[i];
@@ -346,7 +354,7 @@ __global__ void __launch_bounds__(LONE ? 512 : 128) add_norm_vec_kernel(float* _
         v.z += l.z * (u.z * r * (woff + b.z));
         v.w += l.w * (u.w * r * (woff + b.w));
         *reinterpret_cast<float4*>(x + o + c) = v;
-        s2 += squares(v);
+        s2[i] = squares(v);
     }
     if (!wn) return;
     const float r2 = 1.0f / sqrtf(R::sum(s2, red[1]) / (float)D + eps);

@@ -10,8 +10,8 @@
  * decoded token), against the pages and the state slot the caller's scheduler gave it.
  *
  * Element type: `dtype` 0 = bfloat16 matrices, GEMM inputs and key/value pool (fp32 accumulation), 1 = float32
- * everywhere (matrix products on the tensor cores, every operand as two tf32 parts: fp32 results,
- * as close to 64 bits as FMAs; operands below 2^-115 keep 11 bits, infinities give NaN).  In both, the residual stream, every norm, the
+ * everywhere (matrix products of 72 k and more on the tensor cores, every operand as two tf32 parts, outputs that parts cannot make -- infinite or
+ * very large operands, very small outputs -- on FMAs: fp32 results, as close to 64 bits as FMAs throughout).  In both, the residual stream, every norm, the
  * attention scores and weights, and everything inside the recurrence are fp32; long prompts' recurrences multiply on the tensor cores, every
  * operand as three bf16 parts that hold all of its bits (an infinity inside a recurrence gives NaN), and are closer to 64 bits than FMAs.
  */

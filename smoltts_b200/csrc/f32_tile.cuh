@@ -3,18 +3,22 @@
 // out[BM rows][BN columns] = A . W^T over a range of k, both operands k-contiguous.  cp.async brings BK = 16 k at a time into a ring
 // of row-major stages (rows of 20 floats: eight neighbouring rows start in eight different 16-byte bank groups).
 //
-// MmaTile (the language models' float32 engine): a warp takes WM x WN outputs and multiplies with mma.sync m16n8k8 on tf32 parts: every fp32 operand is hi + lo,
-// 11 bits each and the sign of lo, made from the fragments that ldmatrix brings, and a product is lo hi + hi lo + hi hi (lo lo lies below the last place).  The
-// tensor core drops what its sum has below the last place, so a sum runs over 8 k, smallest parts first, and is added in fp32.  (Operands below 2^-115, whose lo is
-// denormal, keep 11 bits; the lo of an infinity is no number.)
+// MmaTile (the language models' float32 engine, sums of 72 k and more): a warp takes WM x WN outputs and multiplies with mma.sync m16n8k8 on tf32 parts: every fp32 operand is hi + lo,
+// 11 bits each and the sign of lo, made from the fragments that ldmatrix brings, and a product is lo hi + hi lo + hi hi.  (Left out: lo lo, at most 2^-22 of the product,
+// and the last bit, 2^-23, of an operand whose lo needs twelve; the errors below have both in them.)  The
+// tensor core drops what its sum has below the last place, so a sum runs over 8 k, smallest parts first, and is added in fp32.
+// Parts cannot hold everything that fp32 holds: the lo of an infinity is no number, an operand in the last half step of tf32 below the largest float has an infinite
+// hi, and operands below 2^-115 have a denormal lo.  So an output that comes out not finite, or below 2^-80 and not zero, is made once more from the operands
+// themselves, on FMAs: whatever is wrong with the parts of a finite product's operands shows in one of the two, except where an operand below 2^-115 meets one
+// above 2^35, or its product vanishes beside larger ones.
 // What bounds it is the MMAs, 170 multiply-adds per clock and SM after the three parts, and the instructions that split operands and add sums beside them:
 // 300 x 4608 x 768 56 us (38 TFLOP/s), 1024 x 4608 x 768 137 (53); Tile, which reads 16 bytes of shared memory (four clocks of the SM) for every 16 multiply-adds, 77
 // and 201.  Without splitting and adding 3072 x 1536 x 1024 takes 142 us instead of 181.  Warps of 64 x 32 in tiles of 64 x 64 or 128 x 64: 174 there, but 20 to 40 %
 // slower on a few hundred rows; sums over 16 k 174 as well, but further from 64 bits where all products have one sign (8.0e-8 against 6.7e-8).
-// Errors against 64 bits (rows x columns x K, MmaTile | Tile): 300 x 4608 x 768 1.37e-7 | 1.83e-7, 300 x 768 x 4608 1.89e-7 | 3.10e-7, 64 x 64 x 8192 2.4e-7 | 4.2e-7;
+// Errors against 64 bits (rows x columns x K, MmaTile | Tile; shorter sums than 72 k go to Tile, see lm_kernels.cu): 300 x 4608 x 768 1.37e-7 | 1.83e-7, 300 x 768 x 4608 1.89e-7 | 3.10e-7, 64 x 64 x 8192 2.4e-7 | 4.2e-7;
 // values in [0, 1): 6.7e-8 | 6.7e-8, 7.7e-8 | 8.1e-8, 8.0e-8 | 9.1e-8.
 //
-// Tile (the codec): a thread owns TM x TN outputs and multiplies k-pairs with fma.rn.f32x2: each accumulator is a pair (sum over even k, sum over odd k), so the
+// Tile (the codec, and the engine's shorter sums): a thread owns TM x TN outputs and multiplies k-pairs with fma.rn.f32x2: each accumulator is a pair (sum over even k, sum over odd k), so the
 // pairs come straight from 16-byte shared-memory loads, with nothing to duplicate or transpose, and one instruction does two
 // multiply-adds (at the rate of two: measured 72 TFLOP/s either way, but half the issue slots).  What bounds it is shared memory: a
 // warp's 16-byte load takes four clocks of the SM, however many lanes share an address, so 8 x 8 outputs per thread just balance the FMAs
@@ -240,6 +244,29 @@ struct MmaTile {
             }
         }
         wait<0>();
+        // outputs that parts cannot make
+        static_assert(MF * NF * 4 <= 32, "a bit per output");
+        uint32_t again = 0;
+#pragma unroll
+        for (int i = 0; i < MF * NF * 4; ++i) {
+            const float x = fabsf(out[i / (NF * 4)][i / 4 % NF][i % 4]);
+            if (!(x >= 0x1p-80f && x <= 0x1.fffffep127f) && x != 0.0f) again |= 1u << i;
+        }
+        while (again) {
+            const int i = __ffs((int)again) - 1, n = i / 4 % NF, e = i % 4;
+            again &= again - 1;
+            const float* ar = a_row(warp / WARPS_N * WM + i / (NF * 4) * 16 + lane / 4 + 8 * (e >> 1));
+            const float* wr = w_row(column_at(warp % WARPS_N * WN + n * 8 + 2 * (lane & 3) + (e & 1)));
+            float sum = 0.0f;
+            if (ar && wr)
+                for (int k = k_lo; k < k_hi; k += 4) {
+                    const float4 x = *reinterpret_cast<const float4*>(ar + a_at(k)), y = *reinterpret_cast<const float4*>(wr + k);
+                    sum = fmaf(x.w, y.w, fmaf(x.z, y.z, fmaf(x.y, y.y, fmaf(x.x, y.x, sum))));
+                }
+#pragma unroll
+            for (int z = 0; z < MF * NF * 4; ++z)
+                if (z == i) out[z / (NF * 4)][z / 4 % NF][z % 4] = sum;
+        }
     }
 
     template <class Done>

@@ -450,15 +450,13 @@ static GemmIo plain_io(int K, int N) {
     return io;
 }
 
-// Matrix product, fp32, operands whose rows are whole 16-byte pieces: y[M, N] = a[M, K] . w[N, K]^T on the tensor-core tile
-// (f32_tile.cuh), K shared by a cluster of CTAs along grid.x where the output has too few tiles to fill the GPU.
+// Matrix product, fp32, operands whose rows are whole 16-byte pieces: y[M, N] = a[M, K] . w[N, K]^T on a tile of f32_tile.cuh (tensor cores; FMAs for the shortest
+// sums), K shared by a cluster of CTAs along grid.x where the output has too few tiles to fill the GPU.
 // 300 rows, 768 to 4608 columns and k: 57 us a product against 331 on the form below, which stages element by element and is bound by
 // instruction issue.
-template <int BM, int BN, int WM, int WN>
-__global__ void __launch_bounds__(f32t::MmaTile<BM, BN, WM, WN>::NT) gemm_f32_tile_kernel(const float* __restrict__ a, const float* __restrict__ w,
-                                                                                       float* __restrict__ y, int M, int N, int K, const GemmIo io) {
+template <int BM, int BN, class T>
+__global__ void __launch_bounds__(T::NT) gemm_f32_tile_kernel(const float* __restrict__ a, const float* __restrict__ w, float* __restrict__ y, int M, int N, int K, const GemmIo io) {
     dep_wait();      // (and no early dep_go: the next kernel's blocks would take room from the CTAs that are still to come)
-    using T = f32t::MmaTile<BM, BN, WM, WN>;
     extern __shared__ __align__(16) float f32_sm[];
     __shared__ long long arow[BM];
     int m0 = blockIdx.y * BM;
@@ -3049,9 +3047,11 @@ template <class T>
 static cudaError_t linear_ex(SmolLm* m, const T* a, const T* w, float* y, int M, int N, int K, const GemmIo& io, int batch, int tiles,
                              cudaStream_t st);
 
-template <int BM, int BN, int WM, int WN>
+// Sums of fewer k stay on FMAs: what an operand's two parts leave out then weighs more than the roundings of the longer chain (error against 64 bits, parts | FMAs, K
+// 16: 0.97e-7 | 0.61e-7, 64: 1.06 | 1.05, 100: 1.15 | 1.30, 256: 1.22 | 1.49).  The times are alike, some 10 us with the launch.
+constexpr int kPartsMinK = 72;
+template <int BM, int BN, class T>
 static cudaError_t launch_f32_tile(const float* a, const float* w, float* y, int M, int N, int K, const GemmIo& io, int batch, int row_tiles, cudaStream_t st) {
-    using T = smol::f32t::MmaTile<BM, BN, WM, WN>;
     const int cols = (N + BN - 1) / BN;
     // CTAs per tile: as many as bring the grid of a single row of tiles to about four per SM, each with at least 128 k.  From N, K and the
     // batch alone: a row's sums must not depend on how many rows the step holds.  (K shared by 1 / 2 / 4: 300 rows of 4608 x 768 60 / 50 / 54 us, 1024 rows 137 / 139 /
@@ -3070,7 +3070,7 @@ static cudaError_t launch_f32_tile(const float* a, const float* w, float* y, int
     cfg.attrs = at;
     cfg.numAttrs = 1;
     t_plain_next = false;      // launched plainly, as plain_launch does
-    return cudaLaunchKernelEx(&cfg, gemm_f32_tile_kernel<BM, BN, WM, WN>, a, w, y, M, N, K, io);
+    return cudaLaunchKernelEx(&cfg, gemm_f32_tile_kernel<BM, BN, T>, a, w, y, M, N, K, io);
 }
 
 template <>
@@ -3079,9 +3079,14 @@ cudaError_t linear_ex<float>(SmolLm* m, const float* a, const float* w, float* y
     m->launches++;
     // whole 16-byte pieces in every row of both operands
     if (K % 4 == 0 && io.lda % 4 == 0 && io.sa % 4 == 0 && io.sw % 4 == 0 && (reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(w)) % 16 == 0) {
-        if (io.tile_group) return launch_f32_tile<kGroupTile, 64, 16, 32>(a, w, y, M, N, K, io, 1, tiles, st);
-        if (M <= 16) return launch_f32_tile<16, 64, 16, 16>(a, w, y, M, N, K, io, batch, (M + 15) / 16, st);
-        return launch_f32_tile<64, 64, 32, 32>(a, w, y, M, N, K, io, batch, (M + 63) / 64, st);
+        using namespace smol::f32t;
+        const auto on = [&](auto group, auto few, auto many) {
+            if (io.tile_group) return launch_f32_tile<kGroupTile, 64, decltype(group)>(a, w, y, M, N, K, io, 1, tiles, st);
+            if (M <= 16) return launch_f32_tile<16, 64, decltype(few)>(a, w, y, M, N, K, io, batch, (M + 15) / 16, st);
+            return launch_f32_tile<64, 64, decltype(many)>(a, w, y, M, N, K, io, batch, (M + 63) / 64, st);
+        };
+        if (K < kPartsMinK) return on(Tile<kGroupTile, 64, 8, 8, 0>{}, Tile<16, 64, 4, 4, 0>{}, Tile<64, 64, 8, 8, 0>{});
+        return on(MmaTile<kGroupTile, 64, 16, 32>{}, MmaTile<16, 64, 16, 16>{}, MmaTile<64, 64, 32, 32>{});
     }
     if (io.tile_group) {
         dim3 grid((N + 63) / 64, tiles, 1);

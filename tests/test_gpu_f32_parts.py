@@ -16,8 +16,8 @@ def engine():
     return model
 
 
-# rows: a tile of 16 and of 64 rows, with remainders; few columns and a long sum: K shared by a cluster
-@pytest.mark.parametrize("m,n,k", [(1, 40, 36), (17, 72, 64), (65, 130, 4100), (16, 64, 1536)])
+# rows: a tile of 16 and of 64 rows, with remainders; few columns and a long sum: K shared by a cluster; sums of fewer than 72 k: on FMAs
+@pytest.mark.parametrize("m,n,k", [(1, 40, 36), (17, 72, 68), (1, 33, 72), (33, 65, 76), (65, 130, 4100), (16, 64, 1536)])
 def test_infinities_and_numbers_next_to_them(engine, m, n, k):
     g = torch.Generator().manual_seed(m)
     a, w = torch.randn(m, k, generator=g), torch.randn(n, k, generator=g)
@@ -45,8 +45,8 @@ def test_infinities_and_numbers_next_to_them(engine, m, n, k):
 def test_small_operands_keep_their_bits(engine, size):
     """Products that nothing larger hides: operands whose lower part would be denormal."""
     g = torch.Generator().manual_seed(3)
-    a, w = torch.randn(20, 64, generator=g) * size, torch.randn(40, 64, generator=g)
+    a, w = torch.randn(20, 96, generator=g) * size, torch.randn(40, 96, generator=g)
     got = engine.linear(a.cuda(), w.cuda()).cpu().double()
     want = a.double() @ w.double().T
-    bound = (a.double().abs() @ w.double().abs().T) * 64 * 2.0 ** -24 + 64 * 2.0 ** -150
+    bound = (a.double().abs() @ w.double().abs().T) * 96 * 2.0 ** -24 + 96 * 2.0 ** -150
     assert bool(((got - want).abs() <= bound).all())

@@ -2375,6 +2375,35 @@ extern "C" size_t smol_lm_struct_bytes(int which) {
 }
 extern "C" const char* smol_lm_last_error(void) { return g_err.c_str(); }
 
+// The four-token scan over a step in which some sequence brings at least kQuadMinTokens tokens, kQuadMeanTokens in the mean (fewer: its two
+// launches and the records of single tokens cost more than the chain they shorten).  One layer of 12 x 64 x 64 as a whole, generalized delta rule,
+// 16 / 24 / 40 / 300 / 1200 tokens: 61 / 68 / 166 / 142 / 275 us against 56 / 65 / 165 / 166 / 370; the two scans alone, 17 tokens
+// beside 15 / 63 single ones: 28 / 67 us against 11 / 20.
+static bool quad_pays(int n_seqs, int n_tokens, int max_n) { return max_n >= kQuadMinTokens && n_tokens >= kQuadMeanTokens * n_seqs; }
+// The scan by chunks, or one of those that go four tokens at a time.  By chunks a sequence must be long enough to pay for its records, and a step's blocks of eight
+// columns must not be many more than the SMs run at once: then either form fills them, and the one with less to do wins -- the more so the fewer channels a head has,
+// since chunks pad to 32.  Times by chunks / four at a time, records included, over 1 to 64 heads, 1 to 16 sequences, 144 to 1000 tokens (us):
+//   generalized delta rule, 12 x 64 x 64, 1 x 260 / 3 x 1000 tokens: 25 / 35, 103 / 172; 8 x 128 x 128, 144 / 160 tokens 1.04 / 0.95 of the other's time;
+//     16 channels, 222 / 256 blocks 0.93 / 1.03
+//   decay per channel or head, 64 x 64: 288 / 384 blocks 0.95 / 1.13; 48 x 24: 222 / 288 blocks 1.00 / 1.10; 32: 222 / 296 blocks 0.96 / 1.05; 16: 148 / 192 blocks 0.99 / 1.08;
+//     12 heads of 96, 176 / 208 tokens 1.07 / 0.96
+//   gated delta rule, 64 x 64: 512 / 768 blocks 0.95 / 1.07; 48 x 24: 288 / 384 blocks 0.87 / 1.13; 32: 384 / 480 blocks 0.94 / 1.11; 16: 148 / 192 blocks 0.92 / 1.08; heads of 128, 176 / 208
+//     tokens 1.06 / 0.99; of 256, 256 / 320 tokens 1.03 / 0.96, but 384 blocks, of which two at a time fill one SM and a third of them again, 1.20 / 1.14
+//   mLSTM, 64 x 64: 0.40 to 0.95 everywhere; 48 x 24: 612 / 768 blocks 0.79 / 1.06; 32: 1224 blocks 0.99; 16: 288 / 384 blocks 0.92 / 1.08
+static bool chunks_pay(int kind, bool unit, int n_seqs, int heads, int n_tokens, int max_n, int d, int columns, int n_sms) {
+    const int min_n = d <= 64 ? 256 : kind == kScanGeneralDelta ? 160 : kind == kScanGatedDelta && d > 128 ? 320 : 208;
+    if (max_n < min_n || n_tokens < kQuadMeanTokens * n_seqs) return false;
+    const double blocks = (double)n_seqs * heads * chunk_blocks(columns) / n_sms, any = 1e30;      // per SM
+    double most = any;
+    if (kind == kScanGeneralDelta) most = d <= 16 ? 1.5 : any;
+    else if (kind == kScanGatedDelta) {
+        if (d > 128) return blocks <= 2.0 || blocks >= 5.0;
+        most = d <= 16 ? 1.0 : d < 64 ? 2.0 : d == 64 ? 3.5 : any;
+    } else if (unit) most = d <= 16 ? 2.0 : d < 64 ? 4.0 : any;
+    else most = d <= 16 ? 1.0 : d < 64 ? 1.5 : d == 64 ? 2.0 : any;
+    return blocks <= most;
+}
+
 extern "C" int smol_lm_create(const SmolLmConfig* cfg, const SmolLmLayer* layers, const int32_t* run_layer, SmolLm** out) {
     if (!cfg || !layers || !run_layer || !out) return fail(SMOL_ERR_INVALID, "smol_lm_create: null argument");
     if (cfg->dtype != SMOL_LM_BF16 && cfg->dtype != SMOL_LM_F32) return fail(SMOL_ERR_INVALID, "dtype must be 0 (bf16) or 1 (f32)");
@@ -2667,13 +2696,16 @@ extern "C" int smol_lm_create(const SmolLmConfig* cfg, const SmolLmLayer* layers
         for (const SmolLmLayer* L : {(const SmolLmLayer*)&m->layers[r.layer], m->layers[r.layer].side}) {
             if (!L) continue;
             const bool ssd = L->mixer == SMOL_LM_MIX_STATE_SPACE, general = L->mixer == SMOL_LM_MIX_GENERAL_DELTA, unit = L->mixer == SMOL_LM_MIX_MLSTM;
-            const bool removes = general || L->mixer == SMOL_LM_MIX_GATED_DELTA;
-            if (removes || ssd || unit || L->mixer == SMOL_LM_MIX_GATED_LINEAR || L->mixer == SMOL_LM_MIX_LIGHTNING || L->mixer == SMOL_LM_MIX_HGRN2 ||
-                L->mixer == SMOL_LM_MIX_RETENTION)
-                m->max_rec = std::max(m->max_rec, (size_t)L->heads * chunk_record(removes, chunk_pad(ssd ? L->n_state : L->dim), general ? L->dim : L->vdim + (unit ? 1 : 0)));
-            if (general || (!removes && !unit)) m->max_quad = std::max(m->max_quad, (size_t)L->heads * quad_record(general ? kFormGeneral : kFormAdd, quad_pad(ssd ? L->n_state : L->dim)));
+            const bool gated = L->mixer == SMOL_LM_MIX_GATED_DELTA, channel = L->mixer == SMOL_LM_MIX_GATED_LINEAR || L->mixer == SMOL_LM_MIX_HGRN2;
+            if (!general && !gated && !unit && !channel && !ssd && L->mixer != SMOL_LM_MIX_LIGHTNING && L->mixer != SMOL_LM_MIX_RETENTION) continue;
+            // records of the forms that a step of this engine can take, on however many SMs
+            const int kind = general ? kScanGeneralDelta : gated ? kScanGatedDelta : channel ? kScanChannelDecay : kScanHeadDecay;
+            const int d = ssd ? L->n_state : L->dim, columns = general ? L->dim : L->vdim + (unit ? 1 : 0), n = cfg->max_step_tokens;
+            if (chunks_pay(kind, unit, 1, L->heads, n, n, d, columns, 1 << 20))
+                m->max_rec = std::max(m->max_rec, (size_t)L->heads * chunk_record(scan_removes(kind), chunk_pad(d), columns));
+            if (!gated && !unit && quad_pays(1, n, n)) m->max_quad = std::max(m->max_quad, (size_t)L->heads * quad_record(general ? kFormGeneral : kFormAdd, quad_pad(d)));
         }
-    if (m->max_rec > 0 && cfg->max_step_tokens >= kQuadMinTokens)
+    if (m->max_rec + m->max_quad > 0)
         m->o_rec = carve(std::max((T / kChunk + cfg->max_step_seqs + 1) * m->max_rec, (T / kQuad + cfg->max_step_seqs + 1) * m->max_quad) * 4);
     if (m->max_pair_heads > 0) m->o_pairs = carve(T * (size_t)m->max_pair_heads * kPairFloats * 4);
     if (m->max_top > 0) {
@@ -3234,11 +3266,6 @@ static cudaError_t launch_scan(const DeltaArgs& A, int n_seqs, const float* dec,
     return cudaGetLastError();
 }
 
-// The four-token scan over a step in which some sequence brings at least kQuadMinTokens tokens, kQuadMeanTokens in the mean (fewer: its two
-// launches and the records of single tokens cost more than the chain they shorten).  One layer of 12 x 64 x 64 as a whole, generalized delta rule,
-// 16 / 24 / 40 / 300 / 1200 tokens: 61 / 68 / 166 / 142 / 275 us against 56 / 65 / 165 / 166 / 370; the two scans alone, 17 tokens
-// beside 15 / 63 single ones: 28 / 67 us against 11 / 20.
-static bool quad_pays(int n_seqs, int n_tokens, int max_n) { return max_n >= kQuadMinTokens && n_tokens >= kQuadMeanTokens * n_seqs; }
 template <int KIND, int DK>
 static cudaError_t launch_quad_sized(SmolLm* m, QuadSource Q, QuadArgs A, int n_seqs, int max_n, float* o_raw, cudaStream_t st, size_t min_smem) {
     constexpr int FORM = quad_form(KIND);
@@ -3261,29 +3288,6 @@ static cudaError_t launch_quad(SmolLm* m, const QuadSource& Q, const QuadArgs& A
     }
 }
 
-// The scan by chunks, or one of those that go four tokens at a time.  By chunks a sequence must be long enough to pay for its records, and a step's blocks of eight
-// columns must not be many more than the SMs run at once: then either form fills them, and the one with less to do wins -- the more so the fewer channels a head has,
-// since chunks pad to 32.  Times by chunks / four at a time, records included, over 1 to 64 heads, 1 to 16 sequences, 144 to 1000 tokens (us):
-//   generalized delta rule, 12 x 64 x 64, 1 x 260 / 3 x 1000 tokens: 25 / 35, 103 / 172; 8 x 128 x 128, 144 / 160 tokens 1.04 / 0.95 of the other's time;
-//     16 channels, 222 / 256 blocks 0.93 / 1.03
-//   decay per channel or head, 64 x 64: 288 / 384 blocks 0.95 / 1.13; 48 x 24: 222 / 288 blocks 1.00 / 1.10; 32: 222 / 296 blocks 0.96 / 1.05; 16: 148 / 192 blocks 0.99 / 1.08;
-//     12 heads of 96, 176 / 208 tokens 1.07 / 0.96
-//   gated delta rule, 64 x 64: 512 / 768 blocks 0.95 / 1.07; 48 x 24: 288 / 384 blocks 0.87 / 1.13; 32: 384 / 480 blocks 0.94 / 1.11; 16: 148 / 192 blocks 0.92 / 1.08; heads of 128, 176 / 208
-//     tokens 1.06 / 0.99; of 256, 256 / 320 tokens 1.03 / 0.96, but 384 blocks, of which two at a time fill one SM and a third of them again, 1.20 / 1.14
-//   mLSTM, 64 x 64: 0.40 to 0.95 everywhere; 48 x 24: 612 / 768 blocks 0.79 / 1.06; 32: 1224 blocks 0.99; 16: 288 / 384 blocks 0.92 / 1.08
-static bool chunks_pay(int kind, bool unit, int n_seqs, int heads, int n_tokens, int max_n, int d, int columns, int n_sms) {
-    const int min_n = d <= 64 ? 256 : kind == kScanGeneralDelta ? 160 : kind == kScanGatedDelta && d > 128 ? 320 : 208;
-    if (max_n < min_n || n_tokens < kQuadMeanTokens * n_seqs) return false;
-    const double blocks = (double)n_seqs * heads * chunk_blocks(columns) / n_sms, any = 1e30;      // per SM
-    double most = any;
-    if (kind == kScanGeneralDelta) most = d <= 16 ? 1.5 : any;
-    else if (kind == kScanGatedDelta) {
-        if (d > 128) return blocks <= 2.0 || blocks >= 5.0;
-        most = d <= 16 ? 1.0 : d < 64 ? 2.0 : d == 64 ? 3.5 : any;
-    } else if (unit) most = d <= 16 ? 2.0 : d < 64 ? 4.0 : any;
-    else most = d <= 16 ? 1.0 : d < 64 ? 1.5 : d == 64 ? 2.0 : any;
-    return blocks <= most;
-}
 template <int KIND, int DK>
 static cudaError_t launch_chunks_sized(SmolLm* m, ChunkSource Q, ChunkArgs A, int n_seqs, int max_n, float* o_raw, cudaStream_t st, size_t min_smem) {
     constexpr bool REM = scan_removes(KIND);

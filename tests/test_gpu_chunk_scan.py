@@ -103,3 +103,12 @@ def test_both_forms_on_either_side_of_the_rule():
             for s in seqs:
                 model.close_sequence(s)
         model.check_device_errors()
+
+
+@pytest.mark.parametrize("make", [lambda n: vu.engine_and_oracle(vu.config([vu.delta(heads=4, kv_heads=2, dim=128, vdim=128)], vocab=61, width=48), seed=4, max_step_tokens=n),
+                                  lambda n: vu.engine_and_oracle(vu.config([vu.par(b=vu.right(heads=4, dim=128, vdim=128))], vocab=61, width=48), seed=4, max_step_tokens=n)])
+def test_no_room_for_records_that_no_step_makes(make):
+    """The gated delta rule's and the mLSTM's scan of shorter prompts has none: an engine for 192 tokens a step keeps none, one for 224 does."""
+    size = {n: make(n)[0]._workspace.numel() for n in (160, 192, 224, 256)}
+    assert size[224] - size[192] > 2 * (size[192] - size[160])
+    assert size[256] - size[224] < size[224] - size[192]

@@ -1225,12 +1225,12 @@ __device__ __forceinline__ float2 load_pair(const bf16* p) {
 // row stride of the staged values: an even number of elements
 template <class T> __host__ __device__ constexpr int split_value_ld(int dv) { return (dv + 16 / (int)sizeof(T) + 1) / 2 * 2; }
 
-// Prompts without a tensor-core form (float32; bf16 heads above 128): a block takes 4 R neighbouring rows of a sequence and one head, a warp R of them, 32 keys and
+// Prompts without a tensor-core form (float32; bf16 heads above 128 whose rows are whole 16-byte pieces): a block takes 4 R neighbouring rows of a sequence and one head, a warp R of them, 32 keys and
 // values at a time in shared memory.  A lane scores one key for the warp's R rows, so a key's 16-byte loads and a value's are shared by R rows; a row's sums are
 // those of a warp of its own: it takes nothing from a key or value that it does not see.
 // What bounds it is shared memory: a 16-byte load of a key and one of each query for 4 R multiply-adds.  300 rows of 12 heads of 64, float32: 60 us
 // (1100: 332) against 230 (2237) for a warp per row that reads its keys from global memory, a row per lane (attn_kernel, which stays for rows that leave no room
-// for the tiles); 9 rows 5.7 against 8.8, 7 x 170 76 against 249; two maps of 64 and values of 128, 300 rows 91 against 330; a latent of 160, 79 against 431.
+// for the tiles and for most that are no whole pieces); 9 rows 5.7 against 8.8, 7 x 170 76 against 249; two maps of 64 and values of 128, 300 rows 91 against 330; a latent of 160, 79 against 431.
 constexpr int kRowsKeys = 32, kRowsWarps = 4, kRowsSmemMax = 100 * 1024;
 template <class T> __host__ __device__ constexpr int rows_ld(int d) { return (d * (int)sizeof(T) + 15) / 16 * 16 / (int)sizeof(T) + 16 / (int)sizeof(T); }      // 16-byte rows, an odd number of them
 template <class T> static constexpr size_t rows_smem(int R, int d, int dv, bool v_in_k) {
@@ -3469,7 +3469,13 @@ static void launch_attention(SmolLm* m, const SmolLmStep* s, AttnArgs& A, bool f
             // four rows of a warp where that still fills the SMs
             const int R = s->n_seqs * A.H * ((max_n + 15) / 16) >= m->n_sms ? 4 : 1;
             const size_t smem = rows_smem<T>(R, A.d, A.dv, A.v_in_k);
-            if (smem > (size_t)kRowsSmemMax)
+            // Rows that are not whole 16-byte pieces are staged an element at a time: in bf16 2.4 and 2.2 times as long as reading them where they lie (keys of 20, values of
+            // 300, 1 x 300 and 7 x 170 tokens; whole pieces of 136 to 320 0.2 to 0.8), in float32 (heads of 130; of 33: 0.63 to 0.89) 1.14 for 1 x 300 tokens, 152 blocks
+            // of 16 rows, 0.99 for 7 x 170, 616, 0.85 for 1 x 1100, 552.
+            const int e = 16 / (int)sizeof(T);
+            const bool pieces = A.d % e == 0 && A.k_ld % e == 0 && A.k_off % e == 0 && (A.v_in_k || (A.dv % e == 0 && A.v_ld % e == 0 && A.v_off % e == 0));
+            const bool rows = pieces || (sizeof(T) == 4 && (std::max(A.d, A.dv) <= 64 || s->n_seqs * A.H * ((max_n + 15) / 16) >= 3 * m->n_sms));
+            if (smem > (size_t)kRowsSmemMax || !rows)
                 plain_launch(attn_kernel<T, MAXV, MAPS>, (au + kAttnWarps - 1) / kAttnWarps, kAttnWarps * 32, kAttnWarps * A.d * sizeof(float), st, A, qbuf, pool, mix);
             else if (R == 4) plain_launch(attn_rows_kernel<T, MAXV, MAPS, 4>, dim3((max_n + 15) / 16, A.H, s->n_seqs), kRowsWarps * 32, smem, st, A, qbuf, pool, mix);
             else plain_launch(attn_rows_kernel<T, MAXV, MAPS, 1>, dim3((max_n + 3) / 4, A.H, s->n_seqs), kRowsWarps * 32, smem, st, A, qbuf, pool, mix);

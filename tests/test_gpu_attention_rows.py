@@ -90,3 +90,19 @@ def test_window_rows_do_not_depend_on_their_block(sizes, window):
     assert pu.rel_err(alone, orc.forward(toks)) < pu.TOL[torch.float32]
     assert torch.equal(logits(3), alone)
     model.check_device_errors()
+
+
+@pytest.mark.parametrize("dim,vdim", [(20, 300), (130, 130), (136, 144), (160, 20)])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32], ids=["bf16", "f32"])
+def test_wide_heads_of_whole_pieces_and_others(dim, vdim, dtype):
+    """Both kernels of prompts' attention without a tensor-core form, on either side of their rule: whole 16-byte pieces or not, few blocks and many."""
+    cfg = pu.config([pu.attn(heads=12, kv_heads=2, dim=dim, vdim=vdim, scale=dim ** -0.5, ff=0)], vocab=61, width=48)
+    model, orc, _ = pu.engine_and_oracle(cfg, seed=14, dtype=dtype, max_tokens=4096, max_seqs=4, page_size=16, max_step_tokens=1024)
+    for lens in ((9,), (181, 33), (250, 240, 230, 210)):
+        toks = [pu.tokens(n, 61, n) for n in lens]
+        seqs = [model.open_sequence() for _ in lens]
+        got = model.forward([(s, t, list(range(n))) for s, t, n in zip(seqs, toks, lens)]).cpu()
+        assert pu.rel_err(got, torch.cat([orc.forward(t) for t in toks])) < pu.TOL[dtype]
+        for s in seqs:
+            model.close_sequence(s)
+    model.check_device_errors()

@@ -49,3 +49,18 @@ def test_a_row_does_not_depend_on_the_number_of_rows(width):
     assert torch.equal(alone, both[:300])
     for s in seqs:
         model.close_sequence(s)
+
+
+@pytest.mark.parametrize("dim,vdim", [(4, 4), (60, 64), (64, 60), (68, 4), (128, 124), (132, 8), (6, 8), (8, 6), (62, 64)])
+def test_preparation_of_attention_rows(dim, vdim):
+    """Heads of whole 16-byte pieces up to 128 elements, sixteen and thirty-two pieces a unit, and those that are not: a prompt, then tokens behind it."""
+    cfg = config([attn(heads=3, kv_heads=1, dim=dim, vdim=vdim, ff=0)], vocab=61, width=48)
+    model, orc, _ = engine_and_oracle(cfg, seed=15)
+    toks = tokens(26, 61, dim)
+    seq, at, got = model.open_sequence(), 0, []
+    for n in (21, 3, 1, 1):
+        got.append(model.forward([(seq, toks[at:at + n], list(range(n)))]).clone())
+        at += n
+    model.close_sequence(seq)
+    assert rel_err(torch.cat(got), orc.forward(toks)) < TOL[torch.float32]
+    model.check_device_errors()

@@ -626,3 +626,29 @@ def test_a_step_that_only_ends_a_request():
         assert rel_err(got, want) < TOL[F32]
     assert len(model.page_pool) == 4 and len(model.slot_pool) == 1
     tb.close()
+
+
+@pytest.mark.parametrize("dim,vdim", [(12, 16), (64, 64), (128, 40), (136, 16)])
+def test_four_taps_of_few_tokens_are_those_of_any_number(dim, vdim):
+    """Few tokens bring a channel's four weights as one piece and all its inputs at once; five taps whose first is zero go one by one: the same bits."""
+    def one(taps):
+        return config([delta(heads=4, kv_heads=2, dim=dim, vdim=vdim, conv=taps)], vocab=61, width=48)
+
+    four, _, w4 = engine_and_oracle(one(4), seed=21)
+
+    def padded(w):
+        for name, value in w4.items():
+            w[name] = torch.cat([torch.zeros_like(value[:, :1]), value], 1) if name.endswith(".conv") else value
+
+    five, _, _ = engine_and_oracle(one(5), seed=21, edit=padded)
+    rows = [tokens(20, 61, i) for i in range(3)]
+    both_seqs = [[m.open_sequence() for _ in rows] for m in (four, five)]
+    at = [0, 0, 0]
+    for part in ((1, 2, 3), (1, 1, 1), (5, 1, 9), (1, 4, 1), (1, 1, 1)):
+        got = [m.forward([(s, r[a:a + n], list(range(n))) for s, r, a, n in zip(seqs, rows, at, part)]).clone() for m, seqs in zip((four, five), both_seqs)]
+        assert torch.equal(got[0], got[1])
+        at = [a + n for a, n in zip(at, part)]
+    for m, seqs in zip((four, five), both_seqs):
+        for s in seqs:
+            m.close_sequence(s)
+        m.check_device_errors()

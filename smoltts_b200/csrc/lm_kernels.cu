@@ -3299,8 +3299,8 @@ static cudaError_t launch_chunks_sized(SmolLm* m, ChunkSource Q, ChunkArgs A, in
     else pdl_launch(chunk_prep_head_kernel<KIND, DK>, grid, 128, prep_smem, st, Q, rec);
     A.rec = rec;
     // Above 64 channels a block has an SM to itself.  Where single blocks of columns would not all run at once, it takes two, whose products share the
-    // records' fragments (12 heads of 128, 1801 tokens: 140 us for 96 blocks of two, 144 for 192 single ones with half the ring, two to an SM; 3 x 12 heads of
-    // 64, 1000 tokens: 57 in twos, 46 single).
+    // records' fragments (measured with operands in two parts: 12 heads of 128, 1801 tokens 140 us for 96 blocks of two, 144 for 192 single ones with half the ring, two
+    // to an SM; 3 x 12 heads of 64, 1000 tokens 57 in twos, 46 single).
     const int parts = chunk_blocks(Q.columns), threads = chunk_warps(DK) * 64 + 32;
     if constexpr (DK > 64) {
         if (n_seqs * A.H * parts > m->n_sms) {

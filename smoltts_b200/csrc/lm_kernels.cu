@@ -1225,12 +1225,12 @@ __device__ __forceinline__ float2 load_pair(const bf16* p) {
 // row stride of the staged values: an even number of elements
 template <class T> __host__ __device__ constexpr int split_value_ld(int dv) { return (dv + 16 / (int)sizeof(T) + 1) / 2 * 2; }
 
-// Prompts without a tensor-core form (float32; bf16 heads above 128 whose rows are whole 16-byte pieces): a block takes 4 R neighbouring rows of a sequence and one head, a warp R of them, 32 keys and
+// Prompts without a tensor-core form (float32; bf16 heads above 128): a block takes 4 R neighbouring rows of a sequence and one head, a warp R of them, 32 keys and
 // values at a time in shared memory.  A lane scores one key for the warp's R rows, so a key's 16-byte loads and a value's are shared by R rows; a row's sums are
 // those of a warp of its own: it takes nothing from a key or value that it does not see.
 // What bounds it is shared memory: a 16-byte load of a key and one of each query for 4 R multiply-adds.  300 rows of 12 heads of 64, float32: 60 us
 // (1100: 332) against 230 (2237) for a warp per row that reads its keys from global memory, a row per lane (attn_kernel, which stays for rows that leave no room
-// for the tiles and for most that are no whole pieces); 9 rows 5.7 against 8.8, 7 x 170 76 against 249; two maps of 64 and values of 128, 300 rows 91 against 330; a latent of 160, 79 against 431.
+// for the tiles and for some that are no whole pieces); 9 rows 5.7 against 8.8, 7 x 170 76 against 249; two maps of 64 and values of 128, 300 rows 91 against 330; a latent of 160, 79 against 431.
 constexpr int kRowsKeys = 32, kRowsWarps = 4, kRowsSmemMax = 100 * 1024;
 template <class T> __host__ __device__ constexpr int rows_ld(int d) { return (d * (int)sizeof(T) + 15) / 16 * 16 / (int)sizeof(T) + 16 / (int)sizeof(T); }      // 16-byte rows, an odd number of them
 template <class T> static constexpr size_t rows_smem(int R, int d, int dv, bool v_in_k) {
@@ -2382,26 +2382,33 @@ extern "C" const char* smol_lm_last_error(void) { return g_err.c_str(); }
 static bool quad_pays(int n_seqs, int n_tokens, int max_n) { return max_n >= kQuadMinTokens && n_tokens >= kQuadMeanTokens * n_seqs; }
 // The scan by chunks, or one of those that go four tokens at a time.  By chunks a sequence must be long enough to pay for its records, and a step's blocks of eight
 // columns must not be many more than the SMs run at once: then either form fills them, and the one with less to do wins -- the more so the fewer channels a head has,
-// since chunks pad to 32.  Times by chunks / four at a time, records included, over 1 to 64 heads, 1 to 16 sequences, 144 to 1000 tokens (us):
-//   generalized delta rule, 12 x 64 x 64, 1 x 260 / 3 x 1000 tokens: 25 / 35, 103 / 172; 8 x 128 x 128, 144 / 160 tokens 1.04 / 0.95 of the other's time;
-//     16 channels, 222 / 256 blocks 0.93 / 1.03
-//   decay per channel or head, 64 x 64: 288 / 384 blocks 0.95 / 1.13; 48 x 24: 222 / 288 blocks 1.00 / 1.10; 32: 222 / 296 blocks 0.96 / 1.05; 16: 148 / 192 blocks 0.99 / 1.08;
-//     12 heads of 96, 176 / 208 tokens 1.07 / 0.96
-//   gated delta rule, 64 x 64: 512 / 768 blocks 0.95 / 1.07; 48 x 24: 288 / 384 blocks 0.87 / 1.13; 32: 384 / 480 blocks 0.94 / 1.11; 16: 148 / 192 blocks 0.92 / 1.08; heads of 128, 176 / 208
-//     tokens 1.06 / 0.99; of 256, 256 / 320 tokens 1.03 / 0.96, but 384 blocks, of which two at a time fill one SM and a third of them again, 1.20 / 1.14
-//   mLSTM, 64 x 64: 0.40 to 0.95 everywhere; 48 x 24: 612 / 768 blocks 0.79 / 1.06; 32: 1224 blocks 0.99; 16: 288 / 384 blocks 0.92 / 1.08
+// since chunks pad to 32; just above what runs at once a nearly empty second wave costs most.  Time by chunks over the other form's, records included, from 1 to 128
+// heads, 1 to 16 sequences, 144 to 1000 tokens (blocks per SM in brackets):
+//   generalized delta rule: 0.45 to 0.79 with 64 channels; 16 [1.5] 0.82, [1.7] 1.03; 128, 144 / 160 tokens [0.9] 1.04 / 0.95, otherwise 0.60 to 0.83
+//   one decay per head: 64 [2.0] 0.92, [2.6] 1.06, [3] and more 0.66 to 0.98; 48 x 24 [1.9] 0.92, [2.4] 1.19; 32 x 32 [5.2] 0.97, [13.8] 1.14; 16 [1.5] 0.88, [1.6] 1.04; above 64, 144 tokens 0.64 to 1.00
+//   decays per channel: 64 [1.9] 0.95, [2.6] 1.13, [4] 1.10, 64 x 128 [5] and more 0.80 to 1.00; 48 x 24 [1.5] 1.00, [1.9] 1.10; 32 x 32 [1.5] 0.96, [2.0] 1.05, 32 x 128 0.79 to 0.99; 16 [1.0] 0.99,
+//     [1.3] 1.08; 128, 144 / 176 / 208 tokens [0.9] 1.18 / 1.10 / 0.99, otherwise 0.75 to 1.01
+//   gated delta rule: 64 [3.5] 0.95, [5.2] 1.07; 48 x 24 [1.9] 0.87, [2.6] 1.13; 32 [2.6] 0.94, [3.2] 1.11; 16 [1.0] 0.92, [1.3] 1.08; 128, 176 / 208 tokens 1.06 / 0.99; 256, 256 / 320
+//     tokens 1.03 / 0.96, but [2.6], where blocks of two leave a third of them for a second wave, 1.20 / 1.14
+//   mLSTM: 64 0.40 to 0.95; 48 x 24 [4.1] 0.79, [5.2] 1.06; 32 [8.3] 0.99; 16 [1.9] 0.92, [2.6] 1.08
 static bool chunks_pay(int kind, bool unit, int n_seqs, int heads, int n_tokens, int max_n, int d, int columns, int n_sms) {
-    const int min_n = d <= 64 ? 256 : kind == kScanGeneralDelta ? 160 : kind == kScanGatedDelta && d > 128 ? 320 : 208;
-    if (max_n < min_n || n_tokens < kQuadMeanTokens * n_seqs) return false;
-    const double blocks = (double)n_seqs * heads * chunk_blocks(columns) / n_sms, any = 1e30;      // per SM
-    double most = any;
-    if (kind == kScanGeneralDelta) most = d <= 16 ? 1.5 : any;
-    else if (kind == kScanGatedDelta) {
-        if (d > 128) return blocks <= 2.0 || blocks >= 5.0;
-        most = d <= 16 ? 1.0 : d < 64 ? 2.0 : d == 64 ? 3.5 : any;
-    } else if (unit) most = d <= 16 ? 2.0 : d < 64 ? 4.0 : any;
-    else most = d <= 16 ? 1.0 : d < 64 ? 1.5 : d == 64 ? 2.0 : any;
-    return blocks <= most;
+    if (n_tokens < kQuadMeanTokens * n_seqs) return false;
+    const double blocks = (double)n_seqs * heads * chunk_blocks(columns) / n_sms;      // per SM
+    const bool wave = blocks <= 2.0 || blocks > 3.0;                                   // (64 channels: an SM runs two)
+    if (kind == kScanGeneralDelta) {
+        const int min_n = d <= 64 ? 256 : blocks > 0.8 && blocks <= 0.9 ? 160 : 144;
+        return max_n >= min_n && (d > 16 || blocks <= 1.5);
+    }
+    if (kind == kScanGatedDelta) {
+        if (max_n < (d <= 64 ? 256 : d <= 128 ? 208 : 320)) return false;
+        return d > 128 ? blocks <= 2.0 || blocks >= 5.0 : d > 64 || blocks <= (d <= 16 ? 1.0 : d < 64 ? 2.0 : 3.5);
+    }
+    if (unit) return max_n >= (d <= 64 ? 256 : 208) && (d >= 64 || blocks <= (d <= 16 ? 2.0 : 4.0));
+    if (kind == kScanHeadDecay) return max_n >= (d <= 64 ? 256 : 144) && (d > 64 || (d == 64 ? wave : blocks <= (d <= 16 ? 1.5 : d <= 32 ? 5.0 : 2.0)));
+    if (d > 64) return max_n >= (blocks > 0.75 && blocks <= 1.2 ? 208 : 144);
+    if (max_n < 256) return false;
+    if (d > 16 && columns >= 2 * d) return d <= 32 || wave;
+    return blocks <= (d <= 16 ? 1.0 : d < 64 ? 1.5 : 2.0);
 }
 
 extern "C" int smol_lm_create(const SmolLmConfig* cfg, const SmolLmLayer* layers, const int32_t* run_layer, SmolLm** out) {
@@ -3466,15 +3473,17 @@ static void launch_attention(SmolLm* m, const SmolLmStep* s, AttnArgs& A, bool f
         } else {
             // every row, also those of short sequences
             const int au = Tn * A.H;
-            // four rows of a warp where that still fills the SMs
-            const int R = s->n_seqs * A.H * ((max_n + 15) / 16) >= m->n_sms ? 4 : 1;
+            // Rows that are not whole 16-byte pieces are staged an element at a time, which a block of four rows a warp pays for once per sixteen rows.  A layer of 8 heads as a
+            // whole against one that reads keys and values where they lie (attn_kernel): bf16, keys or values of whole pieces 0.44 to 0.88; neither, heads of 130: 1 x 300 tokens (152
+            // blocks of 16 rows) 1.10, 1 x 64 (32) 1.07, 1 x 150 (80) 0.92, 1 x 1100 (552) 0.70; keys of 20 and values of 140, 7 x 170 1.40, 4 x 40 (96) 0.81, of 300 1.51 and 0.86.  float32, heads of 33 0.63
+            // to 0.89, of 130 1 x 300 1.14, 7 x 170 (616) 0.99, 1 x 1100 0.85.  Whole pieces: 0.2 to 0.8.
+            const int e = 16 / (int)sizeof(T), blocks = s->n_seqs * A.H * ((max_n + 15) / 16);
+            const bool k_pieces = A.d % e == 0 && A.k_ld % e == 0 && A.k_off % e == 0, v_pieces = A.v_in_k ? k_pieces : A.dv % e == 0 && A.v_ld % e == 0 && A.v_off % e == 0;
+            const bool many = blocks >= 3 * m->n_sms, wave = blocks < m->n_sms && blocks * 5 >= 2 * m->n_sms;      // (wave: of blocks of four rows)
+            const bool rows = (k_pieces && v_pieces) || (sizeof(T) == 4 ? std::max(A.d, A.dv) <= 64 || many
+                              : wave || (A.dv <= 256 && (k_pieces || v_pieces || (A.d >= 64 && many))));
+            const int R = blocks >= m->n_sms ? 4 : 1;      // four rows of a warp where that still fills the SMs
             const size_t smem = rows_smem<T>(R, A.d, A.dv, A.v_in_k);
-            // Rows that are not whole 16-byte pieces are staged an element at a time: in bf16 2.4 and 2.2 times as long as reading them where they lie (keys of 20, values of
-            // 300, 1 x 300 and 7 x 170 tokens; whole pieces of 136 to 320 0.2 to 0.8), in float32 (heads of 130; of 33: 0.63 to 0.89) 1.14 for 1 x 300 tokens, 152 blocks
-            // of 16 rows, 0.99 for 7 x 170, 616, 0.85 for 1 x 1100, 552.
-            const int e = 16 / (int)sizeof(T);
-            const bool pieces = A.d % e == 0 && A.k_ld % e == 0 && A.k_off % e == 0 && (A.v_in_k || (A.dv % e == 0 && A.v_ld % e == 0 && A.v_off % e == 0));
-            const bool rows = pieces || (sizeof(T) == 4 && (std::max(A.d, A.dv) <= 64 || s->n_seqs * A.H * ((max_n + 15) / 16) >= 3 * m->n_sms));
             if (smem > (size_t)kRowsSmemMax || !rows)
                 plain_launch(attn_kernel<T, MAXV, MAPS>, (au + kAttnWarps - 1) / kAttnWarps, kAttnWarps * 32, kAttnWarps * A.d * sizeof(float), st, A, qbuf, pool, mix);
             else if (R == 4) plain_launch(attn_rows_kernel<T, MAXV, MAPS, 4>, dim3((max_n + 15) / 16, A.H, s->n_seqs), kRowsWarps * 32, smem, st, A, qbuf, pool, mix);

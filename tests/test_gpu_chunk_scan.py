@@ -1,4 +1,4 @@
-"""The recurrences' scan by chunks of sixteen tokens (prompts of 256 tokens and more; with more than 64 key channels of 160 or 208, the gated delta rule above
+"""The recurrences' scan by chunks of sixteen tokens (prompts of 256 tokens and more; with more than 64 key channels of 144 to 208, the gated delta rule above
 128 channels of 320)."""
 from __future__ import annotations
 
@@ -48,7 +48,7 @@ def test_scan_by_chunks(dim, form):
     model.check_device_errors()
 
 
-@pytest.mark.parametrize("n", [215, 225])
+@pytest.mark.parametrize("n", [150, 161, 225])
 def test_two_blocks_of_columns_per_block(n):
     """More blocks of columns than SMs above 64 channels: two per block of threads, the last one alone (13 blocks of columns of 12 heads)."""
     for cfg, make in ((pu.config([pu.delta(heads=12, dim=104, ff=0, rank=5)], vocab=61, width=48), pu.engine_and_oracle),

@@ -170,7 +170,8 @@ struct PartsB {
     }
 };
 // sum = a b over N steps of 16: six of the nine products of parts (the others lie below the last place), those of one size in accumulators of their own, no more than
-// two MMAs behind one another.  The tensor core cuts its sums off instead of rounding them; what the largest one loses by that in the mean is given back.
+// two MMAs behind one another.  The tensor core cuts its sums off instead of rounding them; what the largest one loses by that in the mean, half a unit of its last place
+// (0.5 to 1 x 2^-24 of it), is given back (outputs of the generalized delta rule with 0 / 0.72 / 1.0: 1.48, 1.32 and 1.31e-7 off, all else alike).
 constexpr float kCutOff = 0.85f * 0x1p-24f;
 template <int N>
 __device__ __forceinline__ void mma_sum(float (&sum)[4], const PartsA (&a)[N], const PartsB (&b)[N]) {
@@ -749,7 +750,7 @@ __global__ void __launch_bounds__(chunk_warps(DK) * 64 + 32, DK <= 32 ? 4 : DK <
             const int now = b;
             PartsA X[KS];
 #pragma unroll
-            for (int k = 0; k < KS; ++k) X[k].load<SPLIT>(R + ((warp * KS + k) * MX + MX - 1) * FR, lane);
+            for (int k = 0; k < KS; ++k) X[k].template load<SPLIT>(R + ((warp * KS + k) * MX + MX - 1) * FR, lane);
             all_barrier();                               // the state before chunk i is there, V's writes of chunk i are
             float* part = share_o + (i & 1) * NT * NW * SH;
 #pragma unroll
@@ -800,7 +801,7 @@ __global__ void __launch_bounds__(chunk_warps(DK) * 64 + 32, DK <= 32 ? 4 : DK <
     auto load_x = [&](const float* R) {
         if (REM) {
 #pragma unroll
-            for (int k = 0; k < KS; ++k) X[k].load<SPLIT>(R + (warp * KS + k) * MX * FR, lane);
+            for (int k = 0; k < KS; ++k) X[k].template load<SPLIT>(R + (warp * KS + k) * MX * FR, lane);
         }
     };
     umma::bar_wait(&full[0], 0);
@@ -840,7 +841,7 @@ __global__ void __launch_bounds__(chunk_warps(DK) * 64 + 32, DK <= 32 ? 4 : DK <
         PartsA Y[REM ? MT : 1][1];
         if (REM) {
 #pragma unroll
-            for (int m = 0; m < MT; ++m) Y[m][0].load<SPLIT>(R + YF + ((warp * MT + m) * MX + MX - 1) * FR, lane);
+            for (int m = 0; m < MT; ++m) Y[m][0].template load<SPLIT>(R + YF + ((warp * MT + m) * MX + MX - 1) * FR, lane);
         }
         next_slot();
         if (i + 1 < chunks) {
